@@ -347,13 +347,12 @@ int splatad_isect_lidar_tiles_fill(
     int32_t *tile_offsets, int64_t *host_counts, void *stream);
 
 /* No counterpart in the reference. Arms a one-shot request for the NEXT _plan call of the calling
- * thread: when the lists will be built by the row / column split (sorted output, at most 128 tile
- * rows and 16384 tiles), a kernel stores host_pair[0] = n_isects, host_pair[2] = status bits and
+ * thread: a kernel stores host_pair[0] = n_isects, host_pair[2] = status bits and
  * then host_pair[1] = sequence into host_pair, four int64 of pinned (mapped) host memory, as soon
  * as they are known - before the depth order is built, with no copy in the stream. A host that only
  * needs the count polls host_pair[1] for `sequence` (a number it has not used for this triple
- * before) instead of waiting for the end of the plan. Otherwise (other list construction, memory not mapped for the
- * device) nothing is written and the host waits for host_counts as usual. NULL disarms. */
+ * before) instead of waiting for the end of the plan. With memory that is not mapped for the
+ * device nothing is written and the host waits for host_counts as usual. NULL disarms. */
 int splatad_isect_set_early_count(int64_t *host_pair, int64_t sequence);
 
 /* No counterpart in the reference. Arms a one-shot hint for the NEXT _plan call of the calling
