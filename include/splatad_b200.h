@@ -304,7 +304,7 @@ int splatad_compute_lidar_velocity_bwd(uint32_t C, uint32_t N, const float *p_vi
  *          plan, fill and compositing without waiting for the count.
  * `sort`: 0 = lists in flatten-index order; 1 = sorted, with the depth order of the visible
  * Gaussians built by buckets (four kernels: count, scan, scatter, per-bucket order) - if more than
- * 1024 depths fall into one of the 65536 buckets that span the scene's depth range, the plan sets
+ * 1024 depths of a sensor fall into one of the buckets that span the scene's depth range, the plan sets
  * status bit 4 in host_counts[2] and the order is not final: call _plan again with sort = 2;
  * 2 = sorted, depth order by four radix passes (twelve kernels, any depth distribution). Pass the
  * same value to _fill. Both give the same lists.

@@ -8,18 +8,17 @@
 //
 // What this file does instead, with bit-identical results: because a stable sort of the
 // emitted keys orders each tile's list by (depth bits, flatten index), the same lists are
-// obtained by
-//   1. a stable radix sort of the *visible Gaussians* by their 32 depth bits (4 passes over
-//      at most C*N 8-byte pairs - small, L2 resident),
-//   2. emitting (sensor*n_tiles + tile, flatten index) pairs in that depth order, and
-//   3. a stable radix split of those 8-byte pairs by the compact tile key only
-//      (ceil(bits/8) passes: 2 for every configuration up to 65536 sensor-tiles),
-// the last pass writing the 64-bit isect_ids and int32 flatten_ids directly. Offsets are a
-// binary search per tile.
+// obtained by ordering the *visible elements* by (sensor, depth bits, flatten index) with depth
+// buckets - at most C*N 8-byte pairs, L2 resident - and splitting their rectangles stably by blocks of
+// tiles and then by tile (the block split below). Offsets fall out of the split.
 //
-// All kernels run on a fixed grid (a multiple of the 148 SMs) and read problem sizes from
-// device memory, so the whole sequence can be enqueued without a host round trip; the only
-// device->host traffic is the (n_isects, n_visible, status) triple.
+// Grids beyond the block split's tables and depths too crowded for the buckets take the radix split: the
+// elements ordered by depth alone, (sensor*n_tiles + tile, flatten index) pairs emitted in that order,
+// and a stable radix split of those 8-byte pairs by the compact tile key (ceil(bits/8) passes), the last
+// pass writing the 64-bit isect_ids and int32 flatten_ids directly; offsets by a binary search per tile.
+//
+// All kernels read problem sizes from device memory, so the whole sequence can be enqueued without a
+// host round trip; the only device->host traffic is the (n_isects, n_visible, status) triple.
 #include "common.cuh"
 
 namespace splatad {
@@ -196,40 +195,57 @@ __device__ __forceinline__ void stage_boundaries(GridArgs<kLidar> &a, float *sb)
 // (depths that agree to within half a millimetre by the thousand) are passed through unordered and reported
 // with status bit ST_DEPTH_BUCKETS: the caller repeats the plan with the radix sort (sort = 2).
 // ---------------------------------------------------------------------------------------
-constexpr uint32_t kDepthBuckets = 262144;
+constexpr uint32_t kDepthBucketsMax = 262144, kDepthBucketsMin = 8192;
 constexpr uint32_t kBucketMax = 1024;
-constexpr uint32_t kBucketScanBlocks = kDepthBuckets / 1024;   // 256
-static_assert(kBucketScanBlocks % 32 == 0 && kBucketScanBlocks <= 1024, "block totals are scanned by one warp");
+
+// One bucket per element, rounded up to a power of two within the limits above: a frame of 20,000
+// Gaussians scans 32,768 buckets, not 262,144 (bucket scan 13 -> 5 us).
+__host__ __device__ inline uint32_t depth_bucket_count(uint64_t total) {
+    uint32_t n = kDepthBucketsMin;
+    while (n < kDepthBucketsMax && n < total) n *= 2;
+    return n;
+}
+
+// How the elements are grouped before their depths order them: by sensor for the block split (every
+// sensor then owns `per` consecutive buckets and its entries are consecutive), not at all otherwise.
+struct BucketLayout {
+    const int64_t *camera_ids;   // packed: sensor of each row, else nullptr
+    uint32_t N;                  // Gaussians per sensor ([C, N] layout)
+    uint32_t groups;             // sensors, or 1
+    uint32_t per;                // buckets per group
+    __device__ __forceinline__ uint32_t group(uint32_t idx) const {
+        if (groups == 1u) return 0u;
+        return camera_ids ? (uint32_t)__ldg(camera_ids + idx) : idx / N;
+    }
+};
 
 struct DepthBuckets {
     float dmin, scale;
+    uint32_t per;
     __device__ __forceinline__ uint32_t operator()(uint32_t bits) const {
         const float d = __uint_as_float(bits);
-        if (!(d == d)) return kDepthBuckets - 1;   // NaN patterns sort behind +infinity
+        if (!(d == d)) return per - 1;             // NaN patterns sort behind +infinity
         const float x = (d - dmin) * scale;        // weakly monotone in d for finite dmin, scale >= 0
         if (!(x > 0.f)) return 0u;                 // depths below a range given by the caller
-        return x >= (float)(kDepthBuckets - 1) ? kDepthBuckets - 1 : (uint32_t)x;
+        return x >= (float)(per - 1) ? per - 1 : (uint32_t)x;
     }
 };
 
 // The buckets span the range the caller gave for this frame (its last frame's, widened: depths
 // outside it fall into the end buckets, which keeps the bucket index monotone in depth, and the
 // ranks inside a bucket go by the full key) or, without one, the measured range of this frame.
-__device__ __forceinline__ DepthBuckets depth_buckets(const int64_t *counters) {
+__device__ __forceinline__ DepthBuckets depth_buckets(const int64_t *counters, uint32_t per) {
     const bool given = (uint32_t)counters[CNT_BHI] >= (uint32_t)counters[CNT_BLO];
     const uint32_t lo = (uint32_t)counters[given ? CNT_BLO : CNT_DMIN];
     const uint32_t hi = min((uint32_t)counters[given ? CNT_BHI : CNT_DMAX], 0x7f800000u);   // a NaN maximum counts as +infinity
     DepthBuckets b;
+    b.per = per;
     b.dmin = __uint_as_float(min(lo, hi));
     const float range = __uint_as_float(hi) - b.dmin;
-    b.scale = (range > 0.f) ? (float)(kDepthBuckets - 1) / range : 0.f;   // infinite range: scale 0, one bucket
+    b.scale = (range > 0.f) ? (float)(per - 1) / range : 0.f;   // infinite range: scale 0, one bucket
     return b;
 }
 
-// tiles_per_gauss[idx] for every (sensor, Gaussian) / packed row. With rect_xw / rect_yh the
-// rectangle is also stored, packed into two words per element (x0 | width << 16, first grid row |
-// height << 16 with grid row = sensor * tile rows + y; 16-bit fields, used only when
-// the geometry is within its limits) for the row / column split, and the total is added to *n_isects.
 // {count, sequence number, status bits} for a polling host, stored by whichever kernel knows them first
 // into mapped pinned memory: count and status, a system-wide fence, then the sequence number.
 __device__ __forceinline__ void tell_host(volatile int64_t *early_host, int64_t seq, int64_t n_isects,
@@ -242,13 +258,16 @@ __device__ __forceinline__ void tell_host(volatile int64_t *early_host, int64_t 
     __threadfence_system();
 }
 
+// tiles_per_gauss[idx] for every (sensor, Gaussian) / packed row. With `rect` the rectangle is also
+// stored for the block split, packed into two words per element ({x0 | width << 16, y0 | height << 16},
+// the first column wrapped into the row; used only when the geometry is within its limits), and the
+// total is added to *n_isects.
 constexpr int kCountThreads = 1024;   // few, large blocks: every block ends with a handful of same-address atomics
 
 template <bool kLidar>
 __global__ void __launch_bounds__(kCountThreads)
 isect_count_kernel(GridArgs<kLidar> a, uint32_t total, int32_t *__restrict__ tiles_per_gauss,
-                   const int64_t *__restrict__ camera_ids, uint32_t N, uint32_t *__restrict__ rect_xw,
-                   uint32_t *__restrict__ rect_yh, int64_t *__restrict__ n_isects,
+                   BucketLayout layout, uint2 *__restrict__ rect, int64_t *__restrict__ n_isects,
                    int64_t *__restrict__ ticket /* with early_host: a zeroed counter */,
                    volatile int64_t *early_host /* optional, host-mapped: {count, sequence number, status} */,
                    int64_t early_seq,
@@ -256,39 +275,42 @@ isect_count_kernel(GridArgs<kLidar> a, uint32_t total, int32_t *__restrict__ til
                    int64_t *__restrict__ counters /* with depth_bits: CNT_DMIN / CNT_DMAX / CNT_NVIS */,
                    uint32_t *__restrict__ bcount /* optional, with a given bucket range: the bucket counts */) {
     chain_enter();
-    DepthBuckets bucket{0.f, 0.f};
-    if (bcount != nullptr) bucket = depth_buckets(counters);
+    DepthBuckets bucket{0.f, 0.f, 1u};
+    if (bcount != nullptr) bucket = depth_buckets(counters, layout.per);
     __shared__ float sb[kLidar ? kMaxElevSmem : 1];
     __shared__ unsigned long long wsum[kCountThreads / 32];
     stage_boundaries<kLidar>(a, sb);
-    const uint32_t tile_rows = kLidar ? a.lidar.n_tiles_elev : a.cam.tile_height;
     unsigned long long sum = 0;
     uint32_t dmin = 0xffffffffu, dmax = 0u, nvis = 0u;
     for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += gridDim.x * blockDim.x) {
         Rect r;
         int32_t cnt = 0;
-        uint32_t xw = 0, yh = 0;
+        uint2 packed = make_uint2(0u, 0u);
         if (elem_rect<kLidar>(a, idx, r)) {
             cnt = rect_count(r);
-            if (rect_xw != nullptr && cnt > 0) {
-                const uint32_t sensor = camera_ids ? (uint32_t)camera_ids[idx] : idx / N;
-                xw = ((uint32_t)r.x0 & 0xffffu) | ((uint32_t)(r.x1 - r.x0) << 16);
-                yh = (sensor * tile_rows + (uint32_t)r.y0) | ((uint32_t)(r.y1 - r.y0) << 16);
+            if (rect != nullptr && cnt > 0) {
+                int32_t x0 = r.x0;
+                if (kLidar) {
+                    const int32_t n = (int32_t)a.lidar.n_tiles_azim;
+                    if (x0 < 0 || x0 >= n) {
+                        x0 %= n;
+                        if (x0 < 0) x0 += n;
+                    }
+                }
+                packed = make_uint2((uint32_t)x0 | ((uint32_t)(r.x1 - r.x0) << 16),
+                                    (uint32_t)r.y0 | ((uint32_t)(r.y1 - r.y0) << 16));
             }
         }
         tiles_per_gauss[idx] = cnt;
-        if (rect_xw != nullptr) {
-            rect_xw[idx] = xw;
-            rect_yh[idx] = yh;
-        }
+        if (rect != nullptr) rect[idx] = packed;
         sum += (unsigned long long)(cnt > 0 ? cnt : 0);
         if (depth_bits != nullptr && cnt > 0) {
             const uint32_t d = __ldg(depth_bits + idx);
             dmin = min(dmin, d);
             dmax = max(dmax, d);
             ++nvis;
-            if (bcount != nullptr) atomicAdd(&bcount[bucket(d)], 1u);
+            if (bcount != nullptr) atomicAdd(&bcount[layout.group(idx) * layout.per + bucket(d)], 1u);
         }
     }
     if (depth_bits != nullptr) {
@@ -591,23 +613,29 @@ radix_downsweep_kernel(PassSrc s, int shift, int nbits, uint32_t mask, const uin
 
 __global__ void __launch_bounds__(kThreads)
 depth_bucket_count_kernel(const uint32_t *__restrict__ depth_bits, const int32_t *__restrict__ tiles_per_gauss,
-                          uint32_t total, const int64_t *__restrict__ counters, uint32_t *__restrict__ bcount) {
+                          uint32_t total, BucketLayout layout, const int64_t *__restrict__ counters,
+                          uint32_t *__restrict__ bcount) {
     chain_enter();
-    const DepthBuckets bucket = depth_buckets(counters);
+    const DepthBuckets bucket = depth_buckets(counters, layout.per);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
-        if (tiles_per_gauss[i] > 0) atomicAdd(&bcount[bucket(__ldg(depth_bits + i))], 1u);
+        if (tiles_per_gauss[i] > 0)
+            atomicAdd(&bcount[layout.group(i) * layout.per + bucket(__ldg(depth_bits + i))], 1u);
 }
 
 // Blocks of 1024 threads, one bucket per thread: starts within the block's 1024 buckets, counts
 // back to zero (they become the scatter's cursors), the block's total. The block that finishes
 // last turns the block totals into block offsets (a bucket's start = bstart[b] + boff[b >> 10]), sets
-// the status bit for oversized buckets and - when asked - tells the polling host.
+// the status bit for oversized buckets, tells the polling host when asked, and - for a grouped order -
+// notes where every group's entries and its chunks of `chunk` entries start.
 __global__ void __launch_bounds__(1024)
 depth_bucket_scan_kernel(uint32_t *__restrict__ bcount, uint32_t *__restrict__ bstart, uint32_t *__restrict__ boff,
-                         int64_t *__restrict__ counters, volatile int64_t *early_host, int64_t early_seq) {
+                         int64_t *__restrict__ counters, volatile int64_t *early_host, int64_t early_seq,
+                         uint32_t groups, uint32_t per, uint32_t chunk, uint32_t *__restrict__ group_start,
+                         uint32_t *__restrict__ group_chunk /* both [groups + 1]; nullptr: not asked for */) {
     chain_enter();
     __shared__ uint32_t wt[33];
     __shared__ bool s_last;
+    const uint32_t n_scan = gridDim.x;
     const uint32_t b = blockIdx.x * 1024 + threadIdx.x;
     const uint32_t c = bcount[b];
     bcount[b] = 0u;
@@ -615,7 +643,7 @@ depth_bucket_scan_kernel(uint32_t *__restrict__ bcount, uint32_t *__restrict__ b
     bstart[b] = block_excl_scan(c, wt, total);
     const bool big = __syncthreads_or(c > kBucketMax);
     if (threadIdx.x == 0) {
-        boff[kBucketScanBlocks + 1 + blockIdx.x] = total;
+        boff[n_scan + 1 + blockIdx.x] = total;
         if (big) atomicOr((unsigned long long *)&counters[CNT_STATUS], (unsigned long long)ST_DEPTH_BUCKETS);
         __threadfence();
         s_last = atomicAdd((unsigned long long *)&counters[CNT_TICKET], 1ull) + 1ull == (unsigned long long)gridDim.x;
@@ -624,13 +652,14 @@ depth_bucket_scan_kernel(uint32_t *__restrict__ bcount, uint32_t *__restrict__ b
     if (!s_last) return;
     __threadfence();
     if (threadIdx.x < 32) {
-        // the block totals: kBucketScanBlocks / 32 consecutive ones per lane
-        constexpr uint32_t per = kBucketScanBlocks / 32;
-        const volatile uint32_t *tot = boff + kBucketScanBlocks + 1;
-        uint32_t v[per], sum = 0;
+        // the block totals: kScanPerLane consecutive ones per lane
+        constexpr uint32_t kScanPerLane = kDepthBucketsMax / 1024 / 32;
+        const volatile uint32_t *tot = boff + n_scan + 1;
+        uint32_t v[kScanPerLane], sum = 0;
 #pragma unroll
-        for (uint32_t k = 0; k < per; ++k) {
-            v[k] = tot[per * threadIdx.x + k];
+        for (uint32_t k = 0; k < kScanPerLane; ++k) {
+            const uint32_t i = kScanPerLane * threadIdx.x + k;
+            v[k] = i < n_scan ? tot[i] : 0u;
             sum += v[k];
         }
         uint32_t inc = sum;
@@ -641,12 +670,13 @@ depth_bucket_scan_kernel(uint32_t *__restrict__ bcount, uint32_t *__restrict__ b
         }
         uint32_t run = inc - sum;
 #pragma unroll
-        for (uint32_t k = 0; k < per; ++k) {
-            boff[per * threadIdx.x + k] = run;
+        for (uint32_t k = 0; k < kScanPerLane; ++k) {
+            const uint32_t i = kScanPerLane * threadIdx.x + k;
+            if (i < n_scan) boff[i] = run;
             run += v[k];
         }
         if (threadIdx.x == 31) {
-            boff[kBucketScanBlocks] = inc;
+            boff[n_scan] = inc;
             counters[CNT_TICKET] = 0;
             __threadfence();
             if (early_host != nullptr)
@@ -656,19 +686,44 @@ depth_bucket_scan_kernel(uint32_t *__restrict__ bcount, uint32_t *__restrict__ b
                                     (unsigned long long)(uint32_t)counters[CNT_DMIN]));
         }
     }
+    if (group_start == nullptr) return;
+    __syncthreads();
+    const uint32_t n = boff[n_scan];
+    uint32_t chunks = 0;
+    for (uint32_t g0 = 0; g0 < groups; g0 += 1024) {
+        const uint32_t g = g0 + threadIdx.x;
+        uint32_t lo = 0, mine = 0;
+        if (g < groups) {
+            const uint32_t first = g * per, next = first + per;   // next <= buckets
+            lo = __ldcg(bstart + first) + boff[first >> 10];
+            const uint32_t hi = (next >> 10) < n_scan ? __ldcg(bstart + next) + boff[next >> 10] : n;
+            mine = (hi - lo + chunk - 1) / chunk;
+        }
+        uint32_t round;
+        const uint32_t ex = block_excl_scan(mine, wt, round);
+        if (g < groups) {
+            group_start[g] = lo;
+            group_chunk[g] = chunks + ex;
+        }
+        chunks += round;
+    }
+    if (threadIdx.x == 0) {
+        group_start[groups] = n;
+        group_chunk[groups] = chunks;
+    }
 }
 
 __global__ void __launch_bounds__(kThreads)
 depth_bucket_scatter_kernel(const uint32_t *__restrict__ depth_bits, const int32_t *__restrict__ tiles_per_gauss,
-                            uint32_t total, const int64_t *__restrict__ counters,
+                            uint32_t total, BucketLayout layout, const int64_t *__restrict__ counters,
                             const uint32_t *__restrict__ bstart, const uint32_t *__restrict__ boff,
                             uint32_t *__restrict__ bcursor, uint2 *__restrict__ pairs /* {bits, flatten index} */) {
     chain_enter();
-    const DepthBuckets bucket = depth_buckets(counters);
+    const DepthBuckets bucket = depth_buckets(counters, layout.per);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         if (tiles_per_gauss[i] <= 0) continue;
         const uint32_t d = __ldg(depth_bits + i);
-        const uint32_t b = bucket(d);
+        const uint32_t b = layout.group(i) * layout.per + bucket(d);
         const uint32_t pos = bstart[b] + boff[b >> 10] + atomicAdd(&bcursor[b], 1u);
         pairs[pos] = make_uint2(d, i);
     }
@@ -678,19 +733,20 @@ depth_bucket_scatter_kernel(const uint32_t *__restrict__ depth_bits, const int32
 // index) order, by counting, and the move to its final place. Neighbouring threads hold neighbouring
 // elements, almost always of the same bucket: the loads of the loop are broadcasts.
 __global__ void __launch_bounds__(kThreads)
-depth_bucket_rank_kernel(const int64_t *__restrict__ counters, const uint32_t *__restrict__ bstart,
-                         const uint32_t *__restrict__ boff, const uint2 *__restrict__ pairs,
-                         uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out) {
+depth_bucket_rank_kernel(BucketLayout layout, uint32_t n_buckets, const int64_t *__restrict__ counters,
+                         const uint32_t *__restrict__ bstart, const uint32_t *__restrict__ boff,
+                         const uint2 *__restrict__ pairs, const uint2 *__restrict__ rect,
+                         uint2 *__restrict__ sorted_pair /* with rect: {depth bits, flatten index} */,
+                         uint2 *__restrict__ sorted_rect, uint32_t *__restrict__ order /* without rect */) {
     chain_enter();
-    const DepthBuckets bucket = depth_buckets(counters);
-    const uint32_t n = boff[kBucketScanBlocks];
+    const DepthBuckets bucket = depth_buckets(counters, layout.per);
+    const uint32_t n = boff[n_buckets >> 10];
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const uint2 mine = __ldg(pairs + p);
         const uint32_t key = mine.x, val = mine.y;
-        const uint32_t b = bucket(key);
+        const uint32_t b = layout.group(val) * layout.per + bucket(key);
         const uint32_t lo = bstart[b] + boff[b >> 10];
-        const uint32_t hi = (b + 1 < kDepthBuckets && ((b + 1) & 1023u)) ? bstart[b + 1] + boff[b >> 10]
-                            : (b + 1 < kDepthBuckets ? boff[(b + 1) >> 10] : n);
+        const uint32_t hi = ((b + 1) & 1023u) ? bstart[b + 1] + boff[b >> 10] : boff[(b + 1) >> 10];   // boff ends with n
         uint32_t rank = p - lo;                      // crowded bucket: passed through as it is
         if (hi - lo <= kBucketMax) {
             rank = 0;
@@ -701,8 +757,12 @@ depth_bucket_rank_kernel(const int64_t *__restrict__ counters, const uint32_t *_
                 rank += ((((unsigned long long)o.x << 32) | o.y) < me) ? 1u : 0u;
             }
         }
-        keys_out[lo + rank] = key;
-        vals_out[lo + rank] = val;
+        if (rect != nullptr) {
+            sorted_pair[lo + rank] = mine;
+            sorted_rect[lo + rank] = __ldg(rect + val);
+        } else {
+            order[lo + rank] = val;
+        }
     }
 }
 
@@ -962,675 +1022,537 @@ emit_kernel(GridArgs<kLidar> a, EmitArgs e, const uint32_t *__restrict__ eoff,
 }
 
 // ---------------------------------------------------------------------------------------
-// Row / column split (at most 128 tile rows and 16384 tiles over all sensors, rows of at most
-// 1024 tiles: a lidar with 57 x 16 tiles, a 1920 x 1080 camera with 120 x 68): builds the
-// per-tile lists without ever writing the emission out.
+// Block split (sorted output, any number of sensors): builds the per-tile lists of a sensor from its
+// depth-ordered rectangles without ever writing the emission out, in two stable steps.
 //
-// A rectangle is a stack of `h` row runs, each `w` tiles wide. The tile lists of grid row r are
-// made of the row runs of the rectangles that cover r, in depth order, so the split is done in
-// two stable steps that both write long contiguous runs:
-//   A. rows:    every depth-ordered entry appends one record (run start, width, flatten index,
-//               depth bits, running output offset) to the bucket of each grid row it covers.
-//               Ranks inside a bucket come from one ballot per (32 entries, row); the offsets
-//               from a warp prefix sum of the widths. ~0.4 records per intersection.
-//   B. columns: the records of a row, expanded to their `w` outputs, are cut into units of
-//               4096 consecutive outputs (one block each, 512 per warp). The number of outputs
-//               per column of a piece comes from +1 / -1 updates of a difference row; inside a
-//               piece the warp walks 32 outputs at a time: the records that start inside the
-//               32 outputs set one bit each, which tells every lane its record, and lanes that
-//               hit the same column are ranked in lane order (one ballot per column bit). The
-//               4096 outputs are put in tile order in shared memory and leave as ~70-entry
-//               runs per tile.
-// Positions are exclusive sums over (earlier tiles, earlier units, earlier warps), all of
-// them plain scans: the result is the same for any scheduling.
+//   A. blocks: the tile grid is cut into blocks of 4 x 8 tiles. Every depth-ordered entry appends one
+//              record - the 32-bit mask of the block's tiles it covers, its depth bits and flatten
+//              index - to the list of each block it touches (2.3 records per entry for the lidar
+//              benchmark, 3.1 for the camera's, against 5.9 and 5.2 for whole tile rows). A CTA takes
+//              512 consecutive entries; its warps mark their lanes' blocks in one word per (warp,
+//              block), so that an entry's rank in a block's list is a population count.
+//   B. tiles:  a warp takes 256 records of a block, 32 at a time, one record per lane. A 32 x 32 bit
+//              transpose of the masks gives every lane the records that cover ITS tile: that is the
+//              count. To write, the lanes whose record covers tile t store their entry to consecutive
+//              places of t's list.
+//
+// Per intersection this costs 2 warp instructions per 32 lanes' worth of output at the lidar
+// benchmark's density (a fifth of a block per record) and 0.5 at the camera rig's (three fifths);
+// walking the row runs of a rectangle output by output, which it replaces, took 6, and the radix
+// passes over (tile, entry) pairs that grids of more than 128 tile rows took before move 44 B per
+// intersection. What bounds it now is the 12 B of every list entry.
+// Positions are exclusive sums over (earlier tiles, earlier units, earlier CTAs, lower lanes), all of
+// them plain scans: the result is the same for any scheduling, and no block waits for another.
 // ---------------------------------------------------------------------------------------
-constexpr uint32_t kSplitMaxRows = 128;                    // grid rows over all sensors
-constexpr uint32_t kSplitMaxWidth = 1024;                  // tiles per row
-constexpr uint32_t kSplitMaxTiles = 16384;
-constexpr uint32_t kSplitMaxSlots = kSplitMaxTiles + kSplitMaxRows;   // rows * (row_width + 1)
-constexpr uint32_t kSplitWarps = 8;
-// Entries per warp in step A, chosen per call: 128 for grids of up to 32 rows, 32 above (a warp walks
-// its entries 32 at a time and loops over the rows for each window: with many rows that chain gets
-// long and short pieces keep more warps in flight; config 1, 68 rows: step A 119 -> 71 us).
-constexpr uint32_t kSplitWarpEntriesMin = 32, kSplitWarpEntriesMax = 128;
-constexpr uint32_t kSplitSub = 512;                        // outputs per warp in step B
-constexpr uint32_t kSplitUnit = kSplitWarps * kSplitSub;   // outputs per block in step B
-constexpr uint32_t kSplitColBits = 11;
+constexpr uint32_t kBlkW = 4, kBlkH = 8;                   // tiles per block: one per lane
+static_assert(kBlkW * kBlkH == 32, "one lane per tile of a block");
+constexpr uint32_t kBlkThreads = 512, kBlkWarps = kBlkThreads / 32;   // step A: one entry per thread
+constexpr uint32_t kBlkUnit = 128;                         // step B: records per warp
+constexpr uint32_t kBlkMaxPerSensor = 1024;                // blocks per sensor (32768 tiles)
+constexpr uint32_t kBlkMaxPerRow = 256;                    // block columns: shared-memory tables of step A
+constexpr uint32_t kBlkRows = 2;                           // block rows per CTA of step A's scatter
+constexpr uint32_t kBlkMaxBlocks = 16384;                  // blocks over all sensors
+constexpr uint32_t kBlkMaxSensors = 4096;
+constexpr uint32_t kBlkMaxExtent = 8192;                   // tiles per row / rows: the packed rectangle's 16-bit fields
+constexpr uint32_t kBlkGridB = 8 * kNumSMs;                // persistent grid of step B: counting
+constexpr uint32_t kBlkOutThreads = 128;                   // step B, writing: 37 KB of staging per CTA
+constexpr uint32_t kBlkGridOut = 6 * kNumSMs;
 
-struct SplitArgs {
-    uint32_t warp_entries;       // step A: entries per warp (a multiple of 32)
-    // entries: rectangles by flatten index, visited in depth order
-    const uint32_t *rect_xw;     // [total] x0 | width << 16
-    const uint32_t *rect_yh;     // [total] first grid row | height << 16
-    const uint32_t *order;       // [n_entries] flatten index, depth order
-    const uint32_t *depth_key;   // [n_entries] depth bits
-    const int64_t *n_entries_ptr;
-    const int64_t *counters;     // CNT_NISECT
+struct BlkArgs {
+    // entries in (sensor, depth bits, flatten index) order
+    const uint2 *rect;            // {x0 | width << 16, y0 | height << 16}
+    const uint2 *pair;            // {depth bits, flatten index}
+    const uint32_t *sensor_start; // [C + 1] first entry of every sensor
+    const uint32_t *sensor_cta;   // [C + 1] first step-A CTA of every sensor
+    const int64_t *counters;      // CNT_NISECT
     int64_t capacity;
-    uint32_t rows;               // grid rows over all sensors
-    uint32_t tile_rows;          // rows per sensor
-    uint32_t row_width, stride;  // tiles per row, row_width + 1
-    uint32_t tile_n_bits, col_bits, wrap;
+    uint32_t C, n_tiles;          // sensors, tiles per sensor
+    uint32_t width, height;       // tile grid of a sensor
+    uint32_t bx, by, blocks;      // blocks per row, per column, per sensor
+    uint32_t tile_n_bits;
     // workspace
-    uint32_t *ha_cnt, *ha_out;   // [blocks][rows]: records / outputs per (1024 entries, row); scanned
-    uint32_t *hw_cnt, *hw_out;   // [blocks][warps][rows]: the same per warp (128 entries), as counted
-    uint32_t *row_rec, *row_out, *row_unit;   // [rows + 1] exclusive starts
-    uint4 *rec;                  // records {run start | width << 16, output offset, flatten index,
-                                 // depth bits}, row bucket after row bucket
-    uint32_t *hb;                // [units_b][stride] outputs per (unit, column); after the scan:
-                                 // outputs of the column in earlier units of the row
-    uint32_t *hw;                // [units_b][warps][stride] outputs per (unit, warp, column)
-    uint32_t *hb_first;          // [units_b][warps] record owning the first output of the warp
-    uint32_t *slot_tot, *slot_base;           // [rows * stride]
+    uint32_t total, ctas;         // elements (>= entries), step-A CTAs launched
+    uint32_t *table;              // [blocks][ctas] records per (block, step-A CTA); scanned in place
+    uint32_t *rec_start;          // [C * blocks + 1] first record of every block (totals before the scan)
+    uint32_t *unit_start;         // [C * blocks + 1] first step-B unit of every block
+    uint2 *rec;                   // [capacity] {tiles covered, entry}
+    uint32_t *unit_cnt;           // [units][32] list entries per (unit, tile); scanned per block in place
+    uint32_t *tile_base;          // [C * n_tiles] totals, then first list position of every tile
 };
 
-// Warp-cooperative search: last record p in [lo, hi] whose output offset is <= q (offsets are
-// non-decreasing, that of lo is <= q). 32 probes per round.
-__device__ __forceinline__ uint32_t rec_off(const SplitArgs &a, uint32_t p) {
-    return __ldg(reinterpret_cast<const uint32_t *>(a.rec + p) + 1);
+// More intersections than output slots: the split is skipped altogether (the record arrays are sized
+// by the capacity) and only the status bit is raised.
+__device__ __forceinline__ bool blk_overflow(const BlkArgs &a) { return a.counters[CNT_NISECT] > a.capacity; }
+
+// last i in [0, n) with start[i] <= v (start ascending, start[0] <= v), by one warp: 32 probes per round
+__device__ __forceinline__ uint32_t warp_find(const uint32_t *__restrict__ start, uint32_t n, uint32_t v,
+                                              uint32_t lane) {
+    uint32_t lo = 0;
+    while (n > 1) {
+        const uint32_t step = (n + 31) / 32;
+        const uint32_t at = lane * step;
+        const uint32_t m = __ballot_sync(0xffffffffu, at < n && __ldg(start + lo + at) <= v);
+        const uint32_t k = 31u - __clz(m | 1u);
+        lo += k * step;
+        n = min(step, n - k * step);
+    }
+    return lo;
 }
 
-// ---- step A: rows -----------------------------------------------------------------------
-struct SplitEntry {
-    uint32_t xw, row0, h, idx;
-    bool valid;
+struct BlkCta { uint32_t sensor, first, n; bool live; };
+
+// Which entries a step-A CTA takes: every sensor's are cut into chunks of kBlkThreads.
+__device__ __forceinline__ BlkCta blk_cta(const BlkArgs &a) {
+    BlkCta c{};
+    if (a.C == 1) {   // nothing to look up but the number of entries
+        const uint32_t n = __ldg(a.sensor_start + 1);
+        c.first = blockIdx.x * kBlkThreads;
+        c.live = c.first < n;
+        c.n = c.live ? min(kBlkThreads, n - c.first) : 0u;
+        return c;
+    }
+    if (blockIdx.x >= a.sensor_cta[a.C]) return c;
+    c.sensor = warp_find(a.sensor_cta, a.C, blockIdx.x, threadIdx.x & 31);
+    c.first = a.sensor_start[c.sensor] + (blockIdx.x - a.sensor_cta[c.sensor]) * kBlkThreads;
+    c.n = min(kBlkThreads, a.sensor_start[c.sensor + 1] - c.first);
+    c.live = true;
+    return c;
+}
+
+// rectangle of the thread's entry, loaded before anything says whether there is one
+__device__ __forceinline__ uint2 blk_load_rect(const BlkArgs &a, uint32_t entry) {
+    return __ldg(a.rect + min(entry, a.total - 1));
+}
+
+// A rectangle as the blocks it touches. Columns may run on past the last tile column to the first
+// (lidar grids) and, for Gaussians next to the sensor, cover the turn more than once: `layers` runs
+// of at most one turn each, every one inside the one before.
+struct BlkRect {
+    uint32_t x0, w, y0, h;   // w may exceed the grid's width
+    uint32_t sx, nx, sy, ny; // first block column, columns touched (wrapping), first block row, rows
+    uint32_t layers;
 };
 
-__device__ __forceinline__ SplitEntry split_load_entry(const SplitArgs &a, uint32_t p, uint32_t n_entries) {
-    SplitEntry e{0u, 0u, 0u, 0u, p < n_entries};
-    if (e.valid) {
-        e.idx = __ldg(a.order + p);
-        e.xw = __ldg(a.rect_xw + e.idx);
-        const uint32_t yh = __ldg(a.rect_yh + e.idx);
-        e.row0 = yh & 0xffffu;
-        e.h = yh >> 16;
+__device__ __forceinline__ BlkRect blk_rect(const BlkArgs &a, uint2 r, bool live) {
+    BlkRect b;
+    b.x0 = r.x & 0xffffu; b.w = live ? r.x >> 16 : 0u;
+    b.y0 = r.y & 0xffffu; b.h = live ? r.y >> 16 : 0u;
+    b.layers = 1; b.nx = 0; b.ny = 0; b.sx = b.x0 / kBlkW; b.sy = b.y0 / kBlkH;
+    if (b.w == 0u || b.h == 0u) return b;
+    b.ny = (b.y0 + b.h - 1) / kBlkH - b.sy + 1;
+    const uint32_t end = b.x0 + b.w;
+    if (end <= a.width) {
+        b.nx = (end - 1) / kBlkW - b.sx + 1;
+    } else {
+        const uint32_t over = min(end - a.width, b.x0);   // columns [0, over) after the wrap
+        const uint32_t tail = over ? (over - 1) / kBlkW + 1 : 0u;
+        b.nx = min(a.bx, a.bx - b.sx + tail);
+        b.layers = (b.w + a.width - 1) / a.width;
     }
-    return e;
+    return b;
 }
 
-// Records and outputs per grid row of the a.warp_entries entries starting at `first`, for the
-// 32 rows starting at `row_lo`; lane l holds row row_lo + l.
-__device__ __forceinline__ void split_rows_of_warp(const SplitArgs &a, uint32_t first, uint32_t n_entries,
-                                                   uint32_t lane, uint32_t row_lo, uint32_t &cnt,
-                                                   uint32_t &out) {
-    cnt = 0;
-    out = 0;
-    const uint32_t row_hi = min(a.rows, row_lo + 32u);
-    for (uint32_t win = 0; win < a.warp_entries / 32; ++win) {
-        const uint32_t base = first + win * 32;
-        if (base >= n_entries) break;
-        const SplitEntry e = split_load_entry(a, base + lane, n_entries);
-        const uint32_t w = e.xw >> 16;
-        for (uint32_t r = row_lo; r < row_hi; ++r) {
-            const bool hit = e.valid && (r - e.row0) < e.h;
-            const uint32_t bal = __ballot_sync(0xffffffffu, hit);
-            if (bal == 0u) continue;
-            const uint32_t s = __reduce_add_sync(0xffffffffu, hit ? w : 0u);
-            if (row_lo + lane == r) {
-                cnt += __popc(bal);
-                out += s;
-            }
-        }
-    }
+// columns [lo, hi) of the grid as bits of block column s (lo, hi may lie outside the block)
+__device__ __forceinline__ uint32_t blk_span(uint32_t lo, uint32_t hi, uint32_t first, uint32_t n) {
+    const int32_t l = max((int32_t)(lo - first), 0), h = min((int32_t)(hi - first), (int32_t)n);
+    return h > l ? (1u << h) - (1u << l) : 0u;
 }
 
-// More intersections than output slots: the split is skipped altogether (the record arrays are
-// sized by the capacity) and only the status bit is raised.
-__device__ __forceinline__ bool split_overflow(const SplitArgs &a) {
-    return a.counters[CNT_NISECT] > a.capacity;
+// The mask over a block's 32 tiles (bit y * 4 + x) of one layer of a rectangle is the product of the
+// two: its rows as bits four apart, its columns as a nibble.
+__device__ __forceinline__ uint32_t blk_row_bits(const BlkRect &b, uint32_t r) {
+    const uint32_t rows = blk_span(b.y0, b.y0 + b.h, r * kBlkH, kBlkH);
+    uint32_t m = (rows | (rows << 12)) & 0x000f000fu;
+    m = (m | (m << 6)) & 0x03030303u;
+    return (m | (m << 3)) & 0x11111111u;
 }
 
-__global__ void __launch_bounds__(kSplitWarps * 32)
-rowsplit_count_kernel(SplitArgs a) {
+__device__ __forceinline__ uint32_t blk_col_bits(const BlkArgs &a, const BlkRect &b, uint32_t s, uint32_t layer) {
+    const uint32_t end = b.x0 + min(b.w - layer * a.width, a.width);
+    uint32_t cols = blk_span(b.x0, min(end, a.width), s * kBlkW, kBlkW);
+    if (end > a.width) cols |= blk_span(0u, end - a.width, s * kBlkW, kBlkW);
+    return cols;
+}
+
+// records a rectangle leaves in a touched block of block column s: one per layer that covers part of it
+__device__ __forceinline__ uint32_t blk_records(const BlkArgs &a, const BlkRect &b, uint32_t s) {
+    uint32_t n = 1;
+    for (uint32_t j = 1; j < b.layers; ++j) n += blk_col_bits(a, b, s, j) ? 1u : 0u;
+    return n;
+}
+
+// ---- step A -----------------------------------------------------------------------------
+// block columns of a rectangle in block row r
+__device__ __forceinline__ uint32_t blk_row_cols(const BlkRect &b, uint32_t r) {
+    return (r - b.sy) < b.ny ? b.nx : 0u;
+}
+
+template <bool kWrap>
+__global__ void __launch_bounds__(kBlkThreads)
+blk_count_kernel(BlkArgs a) {
     chain_enter();
-    __shared__ uint32_t s_cnt[kSplitMaxRows], s_out[kSplitMaxRows];
-    if (split_overflow(a)) return;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t n_entries = (uint32_t)(*a.n_entries_ptr);
-    const uint32_t first = blockIdx.x * kSplitWarps * a.warp_entries;
-    if (first >= n_entries) return;
-    if (threadIdx.x < kSplitMaxRows) {
-        s_cnt[threadIdx.x] = 0;
-        s_out[threadIdx.x] = 0;
-    }
+    extern __shared__ uint32_t s_cnt[];   // [blocks]
+    const bool overflow = blk_overflow(a);
+    const BlkCta c = blk_cta(a);
+    const uint2 rect = blk_load_rect(a, c.first + threadIdx.x);
+    for (uint32_t k = threadIdx.x; k < a.blocks; k += kBlkThreads) s_cnt[k] = 0u;
+    if (overflow || !c.live) return;
     __syncthreads();
-    const uint32_t wu = blockIdx.x * kSplitWarps + warp;
-    for (uint32_t row_lo = 0; row_lo < a.rows; row_lo += 32) {
-        uint32_t cnt, out;
-        split_rows_of_warp(a, first + warp * a.warp_entries, n_entries, lane, row_lo, cnt, out);
-        const uint32_t r = row_lo + lane;
-        if (r < a.rows) {
-            // kept per warp too, so that the scatter does not have to count again
-            a.hw_cnt[wu * a.rows + r] = cnt;
-            a.hw_out[wu * a.rows + r] = out;
-            if (cnt) {
-                atomicAdd(&s_cnt[r], cnt);
-                atomicAdd(&s_out[r], out);
-            }
+    const BlkRect b = blk_rect(a, rect, threadIdx.x < c.n);
+    for (uint32_t j = 0; j < b.ny; ++j) {
+        uint32_t *row = s_cnt + (b.sy + j) * a.bx;
+        for (uint32_t i = 0, s = b.sx; i < b.nx; ++i) {
+            atomicAdd(&row[s], kWrap && b.layers > 1 ? blk_records(a, b, s) : 1u);
+            if (++s == a.bx) s = 0;
         }
     }
     __syncthreads();
-    if (threadIdx.x < a.rows) {
-        a.ha_cnt[blockIdx.x * a.rows + threadIdx.x] = s_cnt[threadIdx.x];
-        a.ha_out[blockIdx.x * a.rows + threadIdx.x] = s_out[threadIdx.x];
-    }
+    for (uint32_t k = threadIdx.x; k < a.blocks; k += kBlkThreads) a.table[(size_t)k * a.ctas + blockIdx.x] = s_cnt[k];
 }
 
-// Block r: exclusive scan over the entry blocks of grid row r (in place). The block that
-// finishes last turns the row totals into the row starts of records, outputs and step-B units.
+// One CTA per (sensor, block): exclusive scan over the sensor's step-A CTAs, in place. The CTA that
+// finishes last (a ticket, nobody waits) turns the totals into record and unit starts.
 __global__ void __launch_bounds__(1024)
-rowsplit_scan_kernel(SplitArgs a, unsigned long long *__restrict__ ticket) {
+blk_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket) {
     chain_enter();
     __shared__ uint32_t wt[33];
     __shared__ bool s_last;
-    const uint32_t r = blockIdx.x, tid = threadIdx.x;
-    if (split_overflow(a)) return;
-    const uint32_t n_entries = (uint32_t)(*a.n_entries_ptr);
-    const uint32_t block_entries = kSplitWarps * a.warp_entries;
-    const uint32_t n_units = (n_entries + block_entries - 1) / block_entries;
-    uint32_t carry_c = 0, carry_o = 0;
-    for (uint32_t u0 = 0; u0 < n_units; u0 += 1024) {
-        const uint32_t u = u0 + tid;
-        const bool live = u < n_units;
-        const uint32_t vc = live ? a.ha_cnt[u * a.rows + r] : 0u;
-        const uint32_t vo = live ? a.ha_out[u * a.rows + r] : 0u;
-        uint32_t tc, to;
-        const uint32_t ec = block_excl_scan(vc, wt, tc);
-        const uint32_t eo = block_excl_scan(vo, wt, to);
-        if (live) {
-            a.ha_cnt[u * a.rows + r] = carry_c + ec;
-            a.ha_out[u * a.rows + r] = carry_o + eo;
-        }
-        carry_c += tc;
-        carry_o += to;
+    if (blk_overflow(a)) return;
+    const uint32_t tid = threadIdx.x, sensor = blockIdx.x / a.blocks, k = blockIdx.x - sensor * a.blocks;
+    const uint32_t cta0 = a.sensor_cta[sensor], n = a.sensor_cta[sensor + 1] - cta0;
+    uint32_t *row = a.table + (size_t)k * a.ctas + cta0;
+    uint32_t carry = 0;
+    for (uint32_t i0 = 0; i0 < n; i0 += blockDim.x) {
+        const uint32_t i = i0 + tid;
+        const uint32_t v = i < n ? row[i] : 0u;
+        uint32_t tot;
+        const uint32_t ex = block_excl_scan(v, wt, tot);
+        if (i < n) row[i] = carry + ex;
+        carry += tot;
     }
-    // row totals, parked in the upper half of the row tables until the last block arrives
     if (tid == 0) {
-        a.row_rec[kSplitMaxRows + 1 + r] = carry_c;
-        a.row_out[kSplitMaxRows + 1 + r] = carry_o;
+        a.rec_start[blockIdx.x] = carry;
         __threadfence();
         s_last = atomicAdd(ticket, 1ull) + 1ull == (unsigned long long)gridDim.x;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // exclusive scans over the rows (rows <= 128 <= blockDim)
-    const uint32_t vc = tid < a.rows ? a.row_rec[kSplitMaxRows + 1 + tid] : 0u;
-    const uint32_t vo = tid < a.rows ? a.row_out[kSplitMaxRows + 1 + tid] : 0u;
-    const uint32_t vu = (vo + kSplitUnit - 1) / kSplitUnit;
-    uint32_t tc, to, tu;
-    const uint32_t ec = block_excl_scan(vc, wt, tc);
-    const uint32_t eo = block_excl_scan(vo, wt, to);
-    const uint32_t eu = block_excl_scan(vu, wt, tu);
-    if (tid < a.rows) {
-        a.row_rec[tid] = ec;
-        a.row_out[tid] = eo;
-        a.row_unit[tid] = eu;
+    const uint32_t n_blocks = a.C * a.blocks;
+    uint32_t recs = 0, units = 0;
+    for (uint32_t i0 = 0; i0 < n_blocks; i0 += blockDim.x) {
+        const uint32_t i = i0 + tid;
+        const uint32_t v = i < n_blocks ? __ldcg(a.rec_start + i) : 0u;
+        uint32_t tr, tu;
+        const uint32_t er = block_excl_scan(v, wt, tr);
+        const uint32_t eu = block_excl_scan((v + kBlkUnit - 1) / kBlkUnit, wt, tu);
+        if (i < n_blocks) {
+            a.rec_start[i] = recs + er;
+            a.unit_start[i] = units + eu;
+        }
+        recs += tr;
+        units += tu;
     }
     if (tid == 0) {
-        a.row_rec[a.rows] = tc;
-        a.row_out[a.rows] = to;
-        a.row_unit[a.rows] = tu;
+        a.rec_start[n_blocks] = recs;
+        a.unit_start[n_blocks] = units;
         *ticket = 0ull;
     }
 }
 
-// kOneGroup: at most 32 grid rows, so the loop over groups of 32 rows runs once from row 0.
-template <bool kOneGroup>
-__global__ void __launch_bounds__(kSplitWarps * 32)
-rowsplit_scatter_kernel(SplitArgs a) {
+// blockIdx.x: 512 entries of a sensor, blockIdx.y: two block rows. Few rows per CTA, because the entries
+// come in depth order and the nearest ones cover the whole image: the CTA that holds them walks 60 blocks
+// per lane of a 1920 x 1080 grid instead of 270 (70 -> 39 us for the camera benchmark's frame).
+// kWrap: rectangles may cover the turn more than once and then leave several records in a block (a
+// rectangle spans less than five turns): three more mask words per (warp, block) hold the bits of their
+// lanes' surplus.
+template <bool kWrap>
+__global__ void __launch_bounds__(kBlkThreads)
+blk_scatter_kernel(BlkArgs a) {
     chain_enter();
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t lt = (1u << lane) - 1u;
-    if (split_overflow(a)) return;
-    const uint32_t n_entries = (uint32_t)(*a.n_entries_ptr);
-    const uint32_t wu = blockIdx.x * kSplitWarps + warp;
-    const uint32_t first = wu * a.warp_entries;
-    if (first >= n_entries) return;
-    const uint32_t cap = (uint32_t)(a.capacity < 0x7fffffffll ? a.capacity : 0x7fffffffll);
-    for (uint32_t row_lo = 0; row_lo < (kOneGroup ? 1u : a.rows); row_lo += 32) {
-        // lane l: where this warp's records / outputs of row row_lo + l start: row start, earlier
-        // blocks (scanned), earlier warps of this block (as counted)
-        const uint32_t row_hi = min(a.rows, row_lo + 32u);
-        const uint32_t my_row = row_lo + lane;
-        uint32_t rec_at = 0, out_at = 0, row_start = 0, row_piece0 = 0;
-        if (my_row < a.rows) {
-            row_start = a.row_out[my_row];
-            row_piece0 = a.row_unit[my_row] * kSplitWarps;   // first step-B piece of the row
-            rec_at = a.row_rec[my_row] + a.ha_cnt[blockIdx.x * a.rows + my_row];
-            out_at = row_start + a.ha_out[blockIdx.x * a.rows + my_row];
-            for (uint32_t w2 = blockIdx.x * kSplitWarps; w2 < wu; ++w2) {
-                rec_at += a.hw_cnt[w2 * a.rows + my_row];
-                out_at += a.hw_out[w2 * a.rows + my_row];
-            }
-        }
-        for (uint32_t win = 0; win < a.warp_entries / 32; ++win) {
-            const uint32_t base = first + win * 32;
-            if (base >= n_entries) break;
-            const uint32_t p = base + lane;
-            const SplitEntry e = split_load_entry(a, p, n_entries);
-            const uint32_t w = e.xw >> 16;
-            uint32_t xs = 0, idx = 0, depth = 0;
-            if (e.valid) {
-                int32_t x0 = (int32_t)(int16_t)(e.xw & 0xffffu);
-                if (a.wrap) {
-                    x0 %= (int32_t)a.row_width;
-                    if (x0 < 0) x0 += (int32_t)a.row_width;
-                }
-                xs = (uint32_t)x0;
-                idx = e.idx;
-                depth = __ldg(a.depth_key + p);
-            }
-            for (uint32_t r = row_lo; r < row_hi; ++r) {
-                const bool hit = e.valid && (r - e.row0) < e.h;
-                const uint32_t bal = __ballot_sync(0xffffffffu, hit);
-                if (bal == 0u) continue;
-                // exclusive prefix of the widths of the hit lanes
-                const uint32_t v = hit ? w : 0u;
-                uint32_t inc = v;
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const uint32_t o = __shfl_up_sync(0xffffffffu, inc, off);
-                    if (lane >= (uint32_t)off) inc += o;
-                }
-                const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-                const uint32_t rbase = __shfl_sync(0xffffffffu, rec_at, r - row_lo);
-                const uint32_t obase = __shfl_sync(0xffffffffu, out_at, r - row_lo);
-                const uint32_t rstart = __shfl_sync(0xffffffffu, row_start, r - row_lo);
-                const uint32_t rpiece0 = __shfl_sync(0xffffffffu, row_piece0, r - row_lo);
-                if (hit) {
-                    const uint32_t pos = rbase + __popc(bal & lt);
-                    const uint32_t s0 = obase + inc - v;
-                    if (pos < cap) {
-                        a.rec[pos] = make_uint4(xs | (w << 16), s0, idx, depth);
-                        // step B cuts the row's outputs into pieces of kSplitSub: the record that
-                        // holds the first output of a piece is noted for it
-                        const uint32_t rel = s0 - rstart;
-                        for (uint32_t m = (rel + kSplitSub - 1) / kSplitSub; m * kSplitSub < rel + w; ++m)
-                            a.hb_first[rpiece0 + m] = pos;
-                    }
-                }
-                if (my_row == r) {
-                    rec_at += __popc(bal);
-                    out_at += total;
-                }
-            }
-        }
-    }
-}
-
-// ---- step B: columns --------------------------------------------------------------------
-struct SplitUnit {
-    uint32_t row, q_lo, q_hi;   // grid row and output range
-    uint32_t n_rec, n_out;      // records / outputs in all rows
-    bool live;
-};
-
-__device__ __forceinline__ SplitUnit split_unit(const SplitArgs &a, uint32_t u, uint32_t lane) {
-    SplitUnit s{};
-    const uint32_t n_units = a.row_unit[a.rows];
-    s.n_rec = a.row_rec[a.rows];
-    s.n_out = a.row_out[a.rows];
-    s.live = u < n_units;
-    if (!s.live) return s;
-    // last row whose first unit is <= u (rows without outputs own no unit and are passed over)
-    if (a.rows <= 32) {   // one probe per lane
-        const uint32_t m = __ballot_sync(0xffffffffu, lane < a.rows && a.row_unit[lane] <= u);
-        s.row = 31u - __clz(m);
-    } else {
-        uint32_t lo = 0, hi = a.rows - 1;
-        while (lo < hi) {
-            const uint32_t m = (lo + hi + 1) >> 1;
-            if (a.row_unit[m] <= u) lo = m; else hi = m - 1;
-        }
-        s.row = lo;
-    }
-    const uint32_t k = u - a.row_unit[s.row];
-    const uint32_t row_end = a.row_out[s.row + 1];
-    s.q_lo = min(row_end, a.row_out[s.row] + k * kSplitUnit);
-    s.q_hi = min(row_end, s.q_lo + kSplitUnit);
-    return s;
-}
-
-// Adds the outputs [q_lo, q_hi) to a difference row (one record per lane), starting at the record
-// `first` that owns output q_lo (noted by step A's scatter).
-__device__ __forceinline__ void split_count_cols(int32_t *d, const SplitArgs &a, uint32_t q_lo,
-                                                 uint32_t q_hi, uint32_t n_rec, uint32_t n_out,
-                                                 uint32_t first, uint32_t lane) {
-    if (q_lo >= q_hi || n_rec == 0) return;
-    const uint32_t rw = a.row_width;
-    uint32_t base = first;
-    while (true) {
-        const uint32_t p = base + lane;
-        uint32_t s1 = 0u;
-        if (p < n_rec) {
-            const uint2 xo = __ldg(reinterpret_cast<const uint2 *>(a.rec + p));
-            const uint32_t s0 = xo.y;
-            s1 = (p + 1 < n_rec) ? rec_off(a, p + 1) : n_out;
-            if (s0 < q_hi && s1 > q_lo) {
-                const uint32_t xw = xo.x;
-                const uint32_t k_lo = max(s0, q_lo) - s0, k_hi = min(s1, q_hi) - s0;
-                uint32_t start = (xw & 0xffffu) + k_lo;
-                uint32_t len = k_hi - k_lo;
-                if (a.wrap) {
-                    if (len >= rw) {   // the run covers every tile of the row `full` times
-                        const int32_t full = (int32_t)(len / rw);
-                        atomicAdd(d, full);
-                        atomicAdd(d + rw, -full);
-                        len -= (uint32_t)full * rw;
-                    }
-                    if (len) {
-                        if (start >= rw) start %= rw;
-                        const uint32_t end = start + len;
-                        atomicAdd(d + start, 1);
-                        if (end <= rw) {
-                            atomicAdd(d + end, -1);
-                        } else {
-                            atomicAdd(d + rw, -1);
-                            atomicAdd(d, 1);
-                            atomicAdd(d + (end - rw), -1);
-                        }
-                    }
-                } else if (start + len <= rw) {
-                    atomicAdd(d + start, 1);
-                    atomicAdd(d + start + len, -1);
-                }
-            }
-        }
-        const uint32_t last_s1 = __shfl_sync(0xffffffffu, s1, 31);
-        if (base + 32 >= n_rec || last_s1 >= q_hi) break;
-        base += 32;
-    }
-}
-
-// In-place inclusive prefix sum of d[0 .. n) by one warp.
-__device__ __forceinline__ void warp_prefix_inplace(int32_t *d, uint32_t n, uint32_t lane) {
-    int32_t carry = 0;
-    for (uint32_t i0 = 0; i0 < n; i0 += 32) {
-        const uint32_t i = i0 + lane;
-        int32_t v = i < n ? d[i] : 0;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int32_t o = __shfl_up_sync(0xffffffffu, v, off);
-            if (lane >= (uint32_t)off) v += o;
-        }
-        v += carry;
-        if (i < n) d[i] = v;
-        carry = __shfl_sync(0xffffffffu, v, 31);
-    }
-}
-
-__global__ void __launch_bounds__(kSplitWarps * 32)
-colsplit_count_kernel(SplitArgs a) {
-    chain_enter();
-    extern __shared__ int32_t s_d[];   // [kSplitWarps][stride]
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (split_overflow(a)) return;
-    const SplitUnit u = split_unit(a, blockIdx.x, lane);
-    if (!u.live) return;
-    int32_t *wd = s_d + warp * a.stride;
-    for (uint32_t i = lane; i < a.stride; i += 32) wd[i] = 0;
-    __syncwarp();
-    const uint32_t q_lo = min(u.q_hi, u.q_lo + warp * kSplitSub);
-    const uint32_t q_hi = min(u.q_hi, q_lo + kSplitSub);
-    const size_t piece = (size_t)blockIdx.x * kSplitWarps + warp;
-    const uint32_t first = q_lo < q_hi ? min(a.hb_first[piece], u.n_rec ? u.n_rec - 1 : 0u) : 0u;
-    split_count_cols(wd, a, q_lo, q_hi, u.n_rec, u.n_out, first, lane);
-    __syncwarp();
-    warp_prefix_inplace(wd, a.stride, lane);
+    extern __shared__ uint32_t s_dyn[];
+    const uint32_t r0 = blockIdx.y * kBlkRows, n_cols = min(kBlkRows, a.by - r0) * a.bx, plane = kBlkWarps * n_cols;
+    uint32_t *s_base = s_dyn;              // [warps][rows][bx] position of the warp's first record
+    uint32_t *s_mask = s_base + plane;     // (kWrap: 4 planes of) [warps][rows][bx] lanes with a record
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lt = (1u << lane) - 1u;
+    const bool overflow = blk_overflow(a);
+    const BlkCta c = blk_cta(a);
+    const uint32_t entry = c.first + tid;
+    const uint2 rect = blk_load_rect(a, entry);
+    // the CTA's first record of the block of this thread: block start, earlier CTAs of the sensor
+    uint32_t first = 0;
+    if (tid < n_cols)
+        first = __ldg(a.rec_start + c.sensor * a.blocks + r0 * a.bx + tid) +
+                __ldg(a.table + (size_t)(r0 * a.bx + tid) * a.ctas + blockIdx.x);
+    for (uint32_t k = tid; k < plane; k += kBlkThreads) s_mask[k] = 0u;
+    if (overflow || !c.live) return;
+    const BlkRect b = blk_rect(a, rect, tid < c.n);
+    const bool layered = kWrap && __syncthreads_or(b.layers > 1);
+    if (kWrap && layered)
+        for (uint32_t k = plane + tid; k < 4 * plane; k += kBlkThreads) s_mask[k] = 0u;
     __syncthreads();
-    // per warp (so that the scatter does not have to count again) and per unit (to be scanned)
-    uint32_t *prow = a.hw + piece * a.stride;
-    for (uint32_t i = lane; i < a.stride; i += 32) prow[i] = (uint32_t)wd[i];
-    uint32_t *row = a.hb + (size_t)blockIdx.x * a.stride;
-    for (uint32_t i = tid; i < a.stride; i += blockDim.x) {
-        uint32_t tot = 0;
+    uint32_t *mask = s_mask + warp * n_cols;
+    for (uint32_t j = 0; j < kBlkRows; ++j) {
+        const uint32_t n = blk_row_cols(b, r0 + j);
+        uint32_t *row = mask + j * a.bx;
+        for (uint32_t i = 0, s = b.sx; i < n; ++i) {
+            atomicOr(&row[s], 1u << lane);
+            if (kWrap && b.layers > 1) {
+                const uint32_t more = blk_records(a, b, s) - 1u;
+                for (uint32_t q = 0; q < 3; ++q)
+                    if ((more >> q) & 1u) atomicOr(&row[(q + 1) * plane + s], 1u << lane);
+            }
+            if (++s == a.bx) s = 0;
+        }
+    }
+    __syncthreads();
+    if (tid < n_cols) {
+        uint32_t run = first;
 #pragma unroll
-        for (uint32_t w2 = 0; w2 < kSplitWarps; ++w2) tot += (uint32_t)s_d[w2 * a.stride + i];
-        row[i] = tot;
+        for (uint32_t w = 0; w < kBlkWarps; ++w) {
+            s_base[w * n_cols + tid] = run;
+            run += __popc(s_mask[w * n_cols + tid]);
+            if (kWrap && layered)
+                for (uint32_t q = 0; q < 3; ++q) run += __popc(s_mask[(q + 1) * plane + w * n_cols + tid]) << q;
+        }
+    }
+    __syncthreads();
+    const uint32_t cap = (uint32_t)min(a.capacity, (int64_t)0x7fffffff);
+    for (uint32_t j = 0; j < kBlkRows; ++j) {
+        const uint32_t n = blk_row_cols(b, r0 + j);
+        if (n == 0u) continue;
+        const uint32_t *row = mask + j * a.bx, *base = s_base + warp * n_cols + j * a.bx;
+        const uint32_t rows = blk_row_bits(b, r0 + j);
+        for (uint32_t i = 0, s = b.sx; i < n; ++i) {
+            uint32_t pos = base[s] + __popc(row[s] & lt);
+            if (kWrap && layered)
+                for (uint32_t q = 0; q < 3; ++q) pos += __popc(row[(q + 1) * plane + s] & lt) << q;
+            if (pos < cap) a.rec[pos] = make_uint2(rows * blk_col_bits(a, b, s, 0u), entry);
+            if (kWrap)
+                for (uint32_t l = 1; l < b.layers; ++l) {
+                    const uint32_t m = blk_col_bits(a, b, s, l);
+                    if (m != 0u && ++pos < cap) a.rec[pos] = make_uint2(rows * m, entry);
+                }
+            if (++s == a.bx) s = 0;
+        }
     }
 }
 
-// One block per grid row and group of 32 columns: exclusive scan over the units of the row for
-// those columns (in place); the column totals go to slot_tot[r][col]. The block that finishes last (an atomic ticket, nobody waits)
-// scans the totals into slot_base and, when asked, writes the tile offsets - the slot starts
-// without the closing column of every row - followed by the total.
+// ---- step B -----------------------------------------------------------------------------
+struct BlkUnit { uint32_t block, lo, hi; };
+
+__device__ __forceinline__ BlkUnit blk_unit(const BlkArgs &a, uint32_t u, uint32_t lane) {
+    BlkUnit v;
+    // blocks without records own no unit: the search ends at the last of equal starts, which has one
+    v.block = warp_find(a.unit_start, a.C * a.blocks, u, lane);
+    const uint32_t cap = (uint32_t)min(a.capacity, (int64_t)0x7fffffff);
+    v.lo = min(cap, __ldg(a.rec_start + v.block) + (u - __ldg(a.unit_start + v.block)) * kBlkUnit);
+    v.hi = min(min(cap, __ldg(a.rec_start + v.block + 1)), v.lo + kBlkUnit);
+    return v;
+}
+
+// Tile of lane l of a block, as (sensor, x, y); tiles beyond the grid's edges are in no record.
+struct BlkTile { uint32_t sensor, x, y; };
+
+__device__ __forceinline__ BlkTile blk_tile(const BlkArgs &a, uint32_t block, uint32_t l) {
+    BlkTile t;
+    t.sensor = block / a.blocks;
+    const uint32_t k = block - t.sensor * a.blocks, r = k / a.bx;
+    t.x = (k - r * a.bx) * kBlkW + (l & (kBlkW - 1));
+    t.y = r * kBlkH + l / kBlkW;
+    return t;
+}
+
+// 32 x 32 bit transpose across a warp: lane l comes with row l and leaves with column l.
+__device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, uint32_t lane) {
+#pragma unroll
+    for (int j = 16; j >= 1; j >>= 1) {
+        const uint32_t m = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu
+                         : j == 2 ? 0x33333333u : 0x55555555u;
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & (uint32_t)j) ? ((x & ~m) | ((y & ~m) >> j)) : ((x & m) | ((y & m) << j));
+    }
+    return x;
+}
+
+__global__ void __launch_bounds__(kThreads)
+tile_count_kernel(BlkArgs a) {
+    chain_enter();
+    if (blk_overflow(a)) return;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t n_units = a.unit_start[a.C * a.blocks];
+    for (uint32_t u = (blockIdx.x * kThreads + threadIdx.x) >> 5; u < n_units; u += gridDim.x * (kThreads / 32)) {
+        const BlkUnit v = blk_unit(a, u, lane);
+        uint32_t m[kBlkUnit / 32], cnt = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kBlkUnit / 32; ++j) {
+            const uint32_t p = v.lo + 32 * j + lane;
+            m[j] = p < v.hi ? __ldg(&a.rec[p].x) : 0u;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kBlkUnit / 32; ++j) cnt += __popc(warp_transpose_bits(m[j], lane));
+        a.unit_cnt[(size_t)u * 32 + lane] = cnt;
+    }
+}
+
+// One CTA per block: exclusive scan over its units for each of the 32 tiles (one lane each), the units
+// cut into one segment per warp. The CTA that finishes last scans the totals over all tiles: list starts.
 __global__ void __launch_bounds__(1024)
-colsplit_scan_kernel(SplitArgs a, unsigned long long *__restrict__ ticket, int32_t *__restrict__ offsets) {
+tile_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket, int32_t *__restrict__ offsets) {
     chain_enter();
     __shared__ uint32_t seg_sum[32][33];
     __shared__ uint32_t wt[33];
     __shared__ bool s_last;
-    const uint32_t lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
-    // one block per (grid row, group of 32 columns)
-    const uint32_t n_groups = (a.stride + 31) / 32;
-    const uint32_t r = blockIdx.x / n_groups, c_first = (blockIdx.x - r * n_groups) * 32;
-    const uint32_t n_tiles = a.rows * a.row_width;
-    if (split_overflow(a)) {
-        // the split is skipped for lack of room: every offset 0, so that compositing enqueued
-        // behind it finds empty tiles instead of stale numbers
+    const uint32_t tid = threadIdx.x, lane = tid & 31, seg = tid >> 5, n_seg = blockDim.x >> 5;
+    const uint32_t n_tiles = a.C * a.n_tiles;
+    if (blk_overflow(a)) {
+        // the split is skipped for lack of room: every offset 0, so that compositing enqueued behind it
+        // finds empty tiles instead of stale numbers
         if (offsets != nullptr)
-            for (uint32_t t = blockIdx.x * 1024 + threadIdx.x; t <= n_tiles; t += gridDim.x * 1024) offsets[t] = 0;
+            for (uint32_t t = blockIdx.x * blockDim.x + tid; t <= n_tiles; t += gridDim.x * blockDim.x) offsets[t] = 0;
         return;
     }
-    const uint32_t ub0 = a.row_unit[r], n_units = a.row_unit[r + 1] - ub0;
-    const uint32_t per = (n_units + 31) / 32;
-    const uint32_t u_lo = min(n_units, seg * per), u_hi = min(n_units, u_lo + per);
-    const size_t S = a.stride;
-    {
-        const uint32_t c = c_first + lane;
-        const bool live = c < a.stride;
-        uint32_t *col = a.hb + (size_t)ub0 * S + c;
-        uint32_t sum = 0;
-        if (live) {
-            uint32_t u = u_lo;
-            for (; u + 4 <= u_hi; u += 4) {
-                const uint32_t *h = col + (size_t)u * S;
-                const uint32_t v0 = h[0], v1 = h[S], v2 = h[2 * S], v3 = h[3 * S];
-                sum += v0 + v1 + v2 + v3;
-            }
-            for (; u < u_hi; ++u) sum += col[(size_t)u * S];
-        }
-        __syncthreads();
-        seg_sum[seg][lane] = sum;
-        __syncthreads();
-        uint32_t prefix = 0, total = 0;
-        for (uint32_t s2 = 0; s2 < 32; ++s2) {
-            const uint32_t v = seg_sum[s2][lane];
-            if (s2 < seg) prefix += v;
-            total += v;
-        }
-        if (live) {
-            uint32_t run = prefix;
-            for (uint32_t u = u_lo; u < u_hi; ++u) {
-                uint32_t *h = col + (size_t)u * S;
-                const uint32_t v = *h;
-                *h = run;
-                run += v;
-            }
-            if (seg == 0) a.slot_tot[r * a.stride + c] = total;
-        }
-    }
-    __threadfence();   // the writers of slot_tot publish before the ticket is taken
+    const uint32_t u0 = a.unit_start[blockIdx.x], n_units = a.unit_start[blockIdx.x + 1] - u0;
+    const uint32_t per = (n_units + n_seg - 1) / n_seg;
+    const uint32_t lo = min(n_units, seg * per), hi = min(n_units, lo + per);
+    uint32_t *col = a.unit_cnt + (size_t)u0 * 32 + lane;
+    uint32_t sum = 0;
+#pragma unroll 8
+    for (uint32_t u = lo; u < hi; ++u) sum += col[(size_t)u * 32];
+    seg_sum[seg][lane] = sum;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    uint32_t run = 0, total = 0;
+    for (uint32_t s = 0; s < n_seg; ++s) {
+        const uint32_t v = seg_sum[s][lane];
+        if (s < seg) run += v;
+        total += v;
+    }
+#pragma unroll 8
+    for (uint32_t u = lo; u < hi; ++u) {
+        const uint32_t v = col[(size_t)u * 32];
+        col[(size_t)u * 32] = run;
+        run += v;
+    }
+    if (seg == 0) {
+        const BlkTile t = blk_tile(a, blockIdx.x, lane);
+        if (t.x < a.width && t.y < a.height) a.tile_base[t.sensor * a.n_tiles + t.y * a.width + t.x] = total;
         __threadfence();
-        s_last = atomicAdd(ticket, 1ull) + 1ull == (unsigned long long)gridDim.x;
+        __syncwarp();
+        if (lane == 0) s_last = atomicAdd(ticket, 1ull) + 1ull == (unsigned long long)gridDim.x;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // slot_base = exclusive scan of slot_tot, two slots per thread and 2048 per round
-    const uint32_t n_slots = a.rows * a.stride;
-    uint32_t total = 0;
-    for (uint32_t s0 = 0; s0 < n_slots; s0 += 2048) {
-        const uint32_t i0 = s0 + 2 * threadIdx.x, i1 = i0 + 1;
-        const uint32_t v0 = i0 < n_slots ? a.slot_tot[i0] : 0u;
-        const uint32_t v1 = i1 < n_slots ? a.slot_tot[i1] : 0u;
-        uint32_t round_total;
-        const uint32_t ex = block_excl_scan(v0 + v1, wt, round_total);
-        if (i0 < n_slots) a.slot_base[i0] = total + ex;
-        if (i1 < n_slots) a.slot_base[i1] = total + ex + v0;
-        total += round_total;
+    uint32_t carry = 0;
+    for (uint32_t t0 = 0; t0 < n_tiles; t0 += 4 * blockDim.x) {
+        const uint32_t t = t0 + 4 * tid;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (t < n_tiles) v = __ldcg(reinterpret_cast<const uint4 *>(a.tile_base + t));   // room for whole fours
+        if (t + 1 >= n_tiles) v.y = 0u;
+        if (t + 2 >= n_tiles) v.z = 0u;
+        if (t + 3 >= n_tiles) v.w = 0u;
+        uint32_t round;
+        const uint32_t at = carry + block_excl_scan(v.x + v.y + v.z + v.w, wt, round);
+        const uint4 s = make_uint4(at, at + v.x, at + v.x + v.y, at + v.x + v.y + v.z);
+        if (t < n_tiles) *reinterpret_cast<uint4 *>(a.tile_base + t) = s;
+        if (offsets != nullptr) {
+            if (t < n_tiles) offsets[t] = (int32_t)s.x;
+            if (t + 1 < n_tiles) offsets[t + 1] = (int32_t)s.y;
+            if (t + 2 < n_tiles) offsets[t + 2] = (int32_t)s.z;
+            if (t + 3 < n_tiles) offsets[t + 3] = (int32_t)s.w;
+        }
+        carry += round;
     }
-    if (threadIdx.x == 0) *ticket = 0ull;
-    if (offsets == nullptr) return;
-    __syncthreads();
-    for (uint32_t t = threadIdx.x; t <= n_tiles; t += 1024) {
-        const uint32_t rr = t / a.row_width, c = t - rr * a.row_width;
-        offsets[t] = (t == n_tiles) ? (int32_t)total : (int32_t)a.slot_base[rr * a.stride + c];
+    if (tid == 0) {
+        *ticket = 0ull;
+        if (offsets != nullptr) offsets[n_tiles] = (int32_t)carry;
     }
 }
 
-struct SplitWindow {
-    uint32_t xw, s0, s1, idx, depth;
-};
-
-__device__ __forceinline__ SplitWindow split_load_window(const SplitArgs &a, uint32_t base, uint32_t lane,
-                                                         uint32_t n_rec, uint32_t n_out) {
-    SplitWindow win{0u, 0u, 0u, 0u, 0u};
-    const uint32_t p = base + lane;
-    if (p < n_rec) {
-        const uint4 r = __ldg(a.rec + p);
-        win.xw = r.x;
-        win.s0 = r.y;
-        win.s1 = (p + 1 < n_rec) ? rec_off(a, p + 1) : n_out;
-        win.idx = r.z;
-        win.depth = r.w;
-    }
-    return win;
-}
-
-__global__ void __launch_bounds__(kSplitWarps * 32)
-colsplit_scatter_kernel(SplitArgs a, int64_t *__restrict__ isect_ids, int32_t *__restrict__ flatten_ids,
-                        int64_t *__restrict__ counters) {
+// Every warp puts its unit's list entries in tile order in shared memory first - as (record, tile), two
+// bytes each - and then writes them out 32 at a time. (Storing straight from the lanes whose record
+// covers a tile needs no staging, but a store instruction costs the SM about eight cycles of moving
+// addresses and data however few of its lanes are active, and a fifth were: 180 us for the lidar
+// benchmark's 15.3 M entries.)
+__global__ void __launch_bounds__(kBlkOutThreads)
+tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restrict__ flatten_ids,
+                    int64_t *__restrict__ counters) {
     chain_enter();
-    extern __shared__ int32_t s_dyn[];
-    // [kSplitWarps][stride] column tables, [stride] global - local start, staged outputs
-    int32_t *s_tab = s_dyn;
-    int32_t *s_shift = s_tab + kSplitWarps * a.stride;
-    uint32_t *st_depth = reinterpret_cast<uint32_t *>(s_shift + a.stride);
-    uint32_t *st_idx = st_depth + kSplitUnit;
-    uint16_t *st_col = reinterpret_cast<uint16_t *>(st_idx + kSplitUnit);
-    __shared__ uint32_t wt[33];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t lt = (1u << lane) - 1u, le = 0xffffffffu >> (31 - lane);
-    if (split_overflow(a)) {
-        if (blockIdx.x == 0 && tid == 0)
+    constexpr uint32_t kWords = kBlkUnit / 32;
+    __shared__ uint16_t s_out[kBlkOutThreads / 32][kBlkUnit * 32];
+    __shared__ uint2 s_pair[kBlkOutThreads / 32][kBlkUnit];
+    if (blk_overflow(a)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0)
             atomicOr((unsigned long long *)&counters[CNT_STATUS], (unsigned long long)ST_OVERFLOW_CAPACITY);
         return;
     }
-    const SplitUnit u = split_unit(a, blockIdx.x, lane);
-    if (!u.live) return;
-    const uint32_t cap = (uint32_t)(a.capacity < 0x7fffffffll ? a.capacity : 0x7fffffffll);
-    const uint32_t q_lo = min(u.q_hi, u.q_lo + warp * kSplitSub);
-    const uint32_t q_hi = min(u.q_hi, q_lo + kSplitSub);
-    int32_t *wd = s_tab + warp * a.stride;
-    uint32_t *hist = reinterpret_cast<uint32_t *>(wd);
-
-    // Local start of every (warp, column) inside the unit, and the shift to global positions: the
-    // per-warp counts come from the count kernel, the unit's global starts from the scans.
-    const size_t piece0 = (size_t)blockIdx.x * kSplitWarps;
-    const uint32_t *hrow = a.hb + (size_t)blockIdx.x * a.stride;
-    const uint32_t *sbase = a.slot_base + u.row * a.stride;
-    uint32_t carry = 0;
-    for (uint32_t c0 = 0; c0 < a.stride; c0 += blockDim.x) {
-        const uint32_t c = c0 + tid;
-        uint32_t cnt[kSplitWarps], tot = 0;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t n_units = a.unit_start[a.C * a.blocks];
+    const uint32_t cap = (uint32_t)min(a.capacity, (int64_t)0x7fffffff);
+    uint16_t *out = s_out[warp];
+    uint2 *pair = s_pair[warp];
+    for (uint32_t u = blockIdx.x * (kBlkOutThreads / 32) + warp; u < n_units; u += gridDim.x * (kBlkOutThreads / 32)) {
+        const BlkUnit v = blk_unit(a, u, lane);
+        const BlkTile t = blk_tile(a, v.block, lane);
+        const bool in_grid = t.x < a.width && t.y < a.height;
+        const uint32_t tile = t.y * a.width + t.x;
+        uint32_t at = 0;   // lane l: list position of the unit's first entry of tile l
+        if (in_grid) at = __ldg(a.tile_base + t.sensor * a.n_tiles + tile) + __ldg(a.unit_cnt + (size_t)u * 32 + lane);
+        uint2 rec[kWords];
 #pragma unroll
-        for (uint32_t w2 = 0; w2 < kSplitWarps; ++w2) {
-            cnt[w2] = c < a.stride ? a.hw[(piece0 + w2) * a.stride + c] : 0u;
-            tot += cnt[w2];
+        for (uint32_t j = 0; j < kWords; ++j) {
+            const uint32_t p = v.lo + 32 * j + lane;
+            rec[j] = p < v.hi ? __ldg(a.rec + p) : make_uint2(0u, 0u);
         }
-        uint32_t chunk_total;
-        const uint32_t ex = block_excl_scan(tot, wt, chunk_total);
-        if (c < a.stride) {
-            uint32_t run = carry + ex;
-            s_shift[c] = (int32_t)(hrow[c] + sbase[c] - run);
+        uint32_t word[kWords], n = 0;   // lane l: which records cover tile l, how many
 #pragma unroll
-            for (uint32_t w2 = 0; w2 < kSplitWarps; ++w2) {
-                s_tab[w2 * a.stride + c] = (int32_t)run;
-                run += cnt[w2];
+        for (uint32_t j = 0; j < kWords; ++j) {
+            if (v.lo + 32 * j + lane < v.hi) pair[32 * j + lane] = __ldg(a.pair + rec[j].y);
+            word[j] = warp_transpose_bits(rec[j].x, lane);
+            n += __popc(word[j]);
+        }
+        uint32_t inc = n;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= (uint32_t)off) inc += o;
+        }
+        const uint32_t n_out = __shfl_sync(0xffffffffu, inc, 31);
+        uint32_t local = inc - n;
+        at -= local;                    // list position of local place 0 as seen by tile l
+#pragma unroll
+        for (uint32_t j = 0; j < kWords; ++j) {
+            uint32_t w = word[j];
+            while (w) {
+                const uint32_t r = __ffs(w) - 1;
+                w &= w - 1;
+                out[local++] = (uint16_t)((32 * j + r) | (lane << 8));
             }
         }
-        carry += chunk_total;
-    }
-    const uint32_t first_rec = a.hb_first[piece0 + warp];
-    __syncthreads();
-
-    // walk the piece, 32 outputs at a time
-    const uint32_t sensor = u.row / a.tile_rows, y = u.row - sensor * a.tile_rows;
-    const uint32_t hi_row = (sensor << a.tile_n_bits) | (y * a.row_width);
-    if (q_lo < q_hi && u.n_rec > 0) {
-        uint32_t base = first_rec;
-        uint32_t q = q_lo;
-        SplitWindow win = split_load_window(a, base, lane, u.n_rec, u.n_out);
-        while (q < q_hi && base < u.n_rec) {
-            const SplitWindow nxt = split_load_window(a, base + 32, lane, u.n_rec, u.n_out);
-            const uint32_t n_in = min(32u, u.n_rec - base);
-            const uint32_t w_end = min(__shfl_sync(0xffffffffu, win.s1, n_in - 1), q_hi);
-            uint32_t cur = 0;   // window lane of the record owning output q
-            while (q < w_end) {
-                // records after `cur` that start inside this chunk (one may start exactly at q)
-                const bool starts = lane > cur && lane < n_in && win.s0 >= q && (win.s0 - q) < 32u;
-                const uint32_t B = __reduce_or_sync(0xffffffffu, starts ? (1u << (win.s0 - q)) : 0u);
-                const uint32_t o = q + lane;
-                const uint32_t rel = __popc(B & le);
-                const uint32_t own = (cur + rel) & 31u;
-                const uint32_t jxw = __shfl_sync(0xffffffffu, win.xw, own);
-                const uint32_t e0 = __shfl_sync(0xffffffffu, win.s0, own);
-                const uint32_t idx = __shfl_sync(0xffffffffu, win.idx, own);
-                const uint32_t depth = __shfl_sync(0xffffffffu, win.depth, own);
-                uint32_t col = (jxw & 0xffffu) + (o - e0);
-                if (a.wrap && col >= a.row_width) {
-                    col -= a.row_width;
-                    if (col >= a.row_width) col %= a.row_width;
-                }
-                // a column outside the row cannot come from a consistent record
-                const bool active = o < w_end && col < a.row_width;
-                if (!active) col = 0;
-                // Rank among the outputs of this chunk in the same column: lanes with equal
-                // columns are matched with one ballot per column bit and ranked in lane order.
-                // (Letting the records of a chunk take turns instead - the columns of one run are
-                // distinct - measured the same.)
-                // (one match.any per step in place of the ballots measured 18 % slower for this kernel)
-                uint32_t peers = __ballot_sync(0xffffffffu, active);
+        __syncwarp();
+        // four steps of 32 entries in flight per warp: the shared-memory loads and shuffles of one step
+        // follow each other, and 37 KB per CTA leave a scheduler six warps to fill the waits
+        const uint32_t hi0 = (t.sensor << a.tile_n_bits) | (__shfl_sync(0xffffffffu, tile, 0));
+        for (uint32_t i0 = lane; i0 < n_out + lane; i0 += 4 * 32) {
+            uint32_t o[4], pos[4];
+            uint2 e[4];
 #pragma unroll
-                for (uint32_t bit = 0; bit < kSplitColBits; ++bit) {
-                    if (bit >= a.col_bits) break;
-                    const bool one = (col >> bit) & 1u;
-                    const uint32_t bal = __ballot_sync(0xffffffffu, one);
-                    peers &= one ? bal : ~bal;
-                }
-                const uint32_t rank = __popc(peers & lt), cnt = __popc(peers);
-                uint32_t v = 0;
-                if (active) v = hist[col];
-                __syncwarp();
-                if (active && rank + 1 == cnt) hist[col] = v + cnt;   // one lane per column
-                __syncwarp();
-                const uint32_t lpos = v + rank;
-                if (active && lpos < kSplitUnit) {
-                    st_col[lpos] = (uint16_t)col;
-                    st_depth[lpos] = depth;
-                    st_idx[lpos] = idx;
-                }
-                cur += __popc(B);
-                q = min(q + 32u, w_end);
+            for (uint32_t q = 0; q < 4; ++q) o[q] = i0 + 32 * q < n_out ? out[i0 + 32 * q] : 0u;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                pos[q] = i0 + 32 * q + __shfl_sync(0xffffffffu, at, o[q] >> 8);
+                e[q] = pair[o[q] & 0xffu];
             }
-            base += 32;
-            win = nxt;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t l = o[q] >> 8, id = hi0 + (l / kBlkW) * a.width + (l & (kBlkW - 1));
+                if (i0 + 32 * q < n_out && pos[q] < cap) {
+                    isect_ids[pos[q]] = (int64_t)(((uint64_t)id << 32) | e[q].x);
+                    flatten_ids[pos[q]] = (int32_t)e[q].y;
+                }
+            }
         }
-    }
-    __syncthreads();
-    // the unit's outputs now sit in tile order: consecutive threads write consecutive entries
-    const uint32_t n_unit = u.q_hi - u.q_lo;
-    for (uint32_t i = tid; i < n_unit; i += blockDim.x) {
-        const uint32_t col = st_col[i];
-        const uint32_t pos = i + (uint32_t)s_shift[col < a.stride ? col : 0];
-        if (pos < cap) {
-            isect_ids[pos] = ((int64_t)(hi_row + col) << 32) | (int64_t)st_depth[i];
-            flatten_ids[pos] = (int32_t)st_idx[i];
-        }
+        __syncwarp();
     }
 }
 
@@ -1655,15 +1577,16 @@ offset_encode_kernel(const int64_t *__restrict__ isect_ids, const int64_t *n_ptr
     offsets[t] = (int32_t)l;
 }
 
-// counters back to zero (depth range: empty) and, for the bucket depth sort, its 65536 cursors
-__global__ void init_counters_kernel(int64_t *counters, uint32_t *bcount, uint32_t bucket_lo, uint32_t bucket_hi) {
+// counters back to zero (depth range: empty) and, for the bucket depth sort, its cursors
+__global__ void init_counters_kernel(int64_t *counters, uint32_t *bcount, uint32_t n_buckets, uint32_t bucket_lo,
+                                     uint32_t bucket_hi) {
     chain_enter();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < CNT_DEV_SLOTS)
         counters[t] = (t == CNT_DMIN) ? 0xffffffffll : (t == CNT_BLO) ? (int64_t)bucket_lo
                                                      : (t == CNT_BHI) ? (int64_t)bucket_hi : 0;
     if (bcount != nullptr)
-        for (uint32_t i = t; i < kDepthBuckets; i += gridDim.x * blockDim.x) bcount[i] = 0u;
+        for (uint32_t i = t; i < n_buckets; i += gridDim.x * blockDim.x) bcount[i] = 0u;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1679,11 +1602,12 @@ struct PlanWs {
     unsigned long long *block_offs;
     uint32_t *keyA, *valA, *keyB, *valB;
     uint32_t *eoff;
-    uint32_t *ha_cnt, *ha_out;   // row split: per (block of entries, grid row)
-    uint32_t *hw_cnt, *hw_out;   // row split: per (warp of a block, grid row)
-    uint32_t *rect_xw, *rect_yh; // row split: packed rectangles by flatten index
-    uint32_t *bcount, *bstart;   // bucket depth sort: [65536] counts / cursors, [65536] starts in their scan block
-    uint32_t *boff;              // [256] offsets of the scan blocks, [1] total, [256] block totals
+    uint2 *rect, *sorted_rect;   // block split: packed rectangles by flatten index, and in depth order
+    uint32_t *blk_table;         // block split: records per (block, step-A CTA)
+    uint32_t *group_start, *group_chunk;   // block split: first entry / first step-A CTA of every sensor
+    uint32_t n_buckets;
+    uint32_t *bcount, *bstart;   // bucket depth sort: counts / cursors, starts in their scan block
+    uint32_t *boff;              // offsets of the scan blocks, total, block totals
     size_t bytes;
 };
 
@@ -1702,17 +1626,16 @@ static PlanWs carve_plan(void *ws, uint64_t total) {
     p.keyB = (uint32_t *)take(sizeof(uint32_t) * total);
     p.valB = (uint32_t *)take(sizeof(uint32_t) * total);
     p.eoff = (uint32_t *)take(sizeof(uint32_t) * total);
-    const uint64_t smallest_block = kSplitWarps * kSplitWarpEntriesMin;
-    const size_t n_ha = (size_t)((total + smallest_block - 1) / smallest_block) * kSplitMaxRows;
-    p.ha_cnt = (uint32_t *)take(sizeof(uint32_t) * n_ha);
-    p.ha_out = (uint32_t *)take(sizeof(uint32_t) * n_ha);
-    p.hw_cnt = (uint32_t *)take(sizeof(uint32_t) * n_ha * kSplitWarps);
-    p.hw_out = (uint32_t *)take(sizeof(uint32_t) * n_ha * kSplitWarps);
-    p.rect_xw = (uint32_t *)take(sizeof(uint32_t) * total);
-    p.rect_yh = (uint32_t *)take(sizeof(uint32_t) * total);
-    p.bcount = (uint32_t *)take(sizeof(uint32_t) * kDepthBuckets);
-    p.bstart = (uint32_t *)take(sizeof(uint32_t) * kDepthBuckets);
-    p.boff = (uint32_t *)take(sizeof(uint32_t) * (2 * kBucketScanBlocks + 1));
+    p.rect = (uint2 *)take(sizeof(uint2) * total);
+    p.sorted_rect = (uint2 *)take(sizeof(uint2) * total);
+    // blocks * (ceil(total / kBlkThreads) + sensors)
+    p.blk_table = (uint32_t *)take(sizeof(uint32_t) * (kBlkMaxPerSensor * (total / kBlkThreads + 1) + kBlkMaxBlocks));
+    p.group_start = (uint32_t *)take(sizeof(uint32_t) * (kBlkMaxSensors + 1));
+    p.group_chunk = (uint32_t *)take(sizeof(uint32_t) * (kBlkMaxSensors + 1));
+    p.n_buckets = depth_bucket_count(total);
+    p.bcount = (uint32_t *)take(sizeof(uint32_t) * p.n_buckets);
+    p.bstart = (uint32_t *)take(sizeof(uint32_t) * p.n_buckets);
+    p.boff = (uint32_t *)take(sizeof(uint32_t) * (2 * (p.n_buckets / 1024) + 1));
     p.bytes = off;
     return p;
 }
@@ -1735,31 +1658,23 @@ static FillWs carve_fill(void *ws, uint64_t cap) {
     return f;
 }
 
-struct SplitWs {
-    uint32_t *row_rec, *row_out, *row_unit;
-    uint4 *rec;
-    uint32_t *hb, *hw, *hb_first, *slot_tot, *slot_base;
-    uint32_t units_b_cap;
+struct BlkWs {
+    uint32_t *rec_start, *unit_start, *unit_cnt, *tile_base;
+    uint2 *rec;
     size_t bytes;
 };
 
-static SplitWs carve_split(void *ws, uint64_t cap, uint32_t rows, uint32_t stride) {
-    SplitWs w;
+static BlkWs carve_blocks(void *ws, uint64_t cap) {
+    BlkWs w;
     char *c = (char *)ws;
     size_t off = 0;
     auto take = [&](size_t n) { char *r = c ? c + off : nullptr; off += align256(n); return r; };
-    // [0 .. rows] exclusive starts; the second half parks the row totals during the scan
-    w.row_rec = (uint32_t *)take(sizeof(uint32_t) * 2 * (kSplitMaxRows + 1));
-    w.row_out = (uint32_t *)take(sizeof(uint32_t) * 2 * (kSplitMaxRows + 1));
-    w.row_unit = (uint32_t *)take(sizeof(uint32_t) * (kSplitMaxRows + 1));
-    w.rec = (uint4 *)take(sizeof(uint4) * cap);
-    // every grid row rounds its outputs up to whole units
-    w.units_b_cap = (uint32_t)((cap + kSplitUnit - 1) / kSplitUnit) + rows;
-    w.hb = (uint32_t *)take(sizeof(uint32_t) * (size_t)w.units_b_cap * stride);
-    w.hw = (uint32_t *)take(sizeof(uint32_t) * (size_t)w.units_b_cap * kSplitWarps * stride);
-    w.hb_first = (uint32_t *)take(sizeof(uint32_t) * (size_t)w.units_b_cap * kSplitWarps);
-    w.slot_tot = (uint32_t *)take(sizeof(uint32_t) * kSplitMaxSlots);
-    w.slot_base = (uint32_t *)take(sizeof(uint32_t) * kSplitMaxSlots);
+    w.rec_start = (uint32_t *)take(sizeof(uint32_t) * (kBlkMaxBlocks + 1));
+    w.unit_start = (uint32_t *)take(sizeof(uint32_t) * (kBlkMaxBlocks + 1));
+    w.tile_base = (uint32_t *)take(sizeof(uint32_t) * kBlkMaxBlocks * 32);
+    // a record stands for at least one list entry; every block rounds its records up to whole units
+    w.unit_cnt = (uint32_t *)take(sizeof(uint32_t) * 32 * (cap / kBlkUnit + kBlkMaxBlocks));
+    w.rec = (uint2 *)take(sizeof(uint2) * cap);
     w.bytes = off;
     return w;
 }
@@ -1779,14 +1694,21 @@ struct IsectGeom {
     const uint32_t *depth_bits;
 };
 
-// The row / column split applies to sorted output with at most 128 grid rows and 16384 tiles over
-// all sensors and rows of at most 1024 tiles (every field of the packed rectangle record then fits
-// 16 bits, the column tables fit shared memory).
-static bool use_split(const IsectGeom &g, int sort) {
-    if (!sort || (uint64_t)g.C * g.n_tiles > kSplitMaxTiles) return false;
-    const uint64_t rw = g.lidar ? g.lid.lidar.n_tiles_azim : g.cam.cam.tile_width;
-    const uint64_t rows = (uint64_t)g.C * (g.n_tiles / rw);
-    return rows <= kSplitMaxRows && rw <= kSplitMaxWidth;
+// The block split applies to sorted output whose depth order is built by buckets, within the limits
+// of its tables (six 1920 x 1080 cameras have 1620 blocks, a 128-beam lidar 30); larger grids and the
+// radix depth order take the radix split.
+static bool use_blocks(const IsectGeom &g, int sort) {
+    if (sort != 1 || g.C > kBlkMaxSensors) return false;
+    const uint64_t width = g.lidar ? g.lid.lidar.n_tiles_azim : g.cam.cam.tile_width, height = g.n_tiles / width;
+    if (width > kBlkMaxExtent || height > kBlkMaxExtent) return false;
+    const uint64_t bx = (width + kBlkW - 1) / kBlkW, blocks = bx * ((height + kBlkH - 1) / kBlkH);
+    return bx <= kBlkMaxPerRow && blocks <= kBlkMaxPerSensor && blocks * g.C <= kBlkMaxBlocks &&
+           g.C <= depth_bucket_count(g.total);
+}
+
+static BucketLayout bucket_layout(const IsectGeom &g, bool grouped) {
+    const uint32_t groups = grouped ? g.C : 1u;
+    return BucketLayout{g.camera_ids, g.N, groups, depth_bucket_count(g.total) / groups};
 }
 
 // One-shot request of the calling thread's next plan (splatad_isect_set_early_count): where the
@@ -1817,13 +1739,15 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
     {
         SPL_PROF("init_counters_kernel", st);
         if (buckets)
-            launch_chained(init_counters_kernel, kDepthBuckets / 1024, 1024, 0, st, p.counters, p.bcount, range_lo, range_hi);
+            launch_chained(init_counters_kernel, p.n_buckets / 1024, 1024, 0, st, p.counters, p.bcount, p.n_buckets,
+                           range_lo, range_hi);
         else
-            launch_chained(init_counters_kernel, 1, 32, 0, st, p.counters, (uint32_t *)nullptr, 1u, 0u);
+            launch_chained(init_counters_kernel, 1, 32, 0, st, p.counters, (uint32_t *)nullptr, 0u, 1u, 0u);
     }
-    // with few enough sensor-tiles the fill uses the row / column split: it wants the packed
-    // rectangles and needs neither the emission offsets nor their block sums
-    const bool split = use_split(g, sort);
+    // the block split wants the packed rectangles and the order grouped by sensor; it needs neither the
+    // emission offsets nor their block sums
+    const bool blocks = use_blocks(g, sort);
+    const BucketLayout layout = bucket_layout(g, blocks);
     const uint32_t cgrid = min(div_up(g.total, kCountThreads), (uint32_t)(2 * kNumSMs));
     // the intersection count is known when the rectangle count ends: a host that has asked for it (to
     // size or cut its lists) gets it from a kernel - the rectangle count itself, or the bucket scan right
@@ -1840,18 +1764,18 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
     t_early_host = nullptr;
     {
         SPL_PROF("isect_count_kernel", st);
-        uint32_t *rx = split ? p.rect_xw : nullptr, *ry = split ? p.rect_yh : nullptr;
+        uint2 *rect = blocks ? p.rect : nullptr;
         int64_t *tot = p.counters + CNT_NISECT;
         int64_t *ticket = p.counters + CNT_TICKET;
         int64_t *early_here = buckets ? nullptr : early;
         const uint32_t *db = buckets ? g.depth_bits : nullptr;
         if (g.lidar)
             launch_chained(isect_count_kernel<true>, cgrid, kCountThreads, 0, st, g.lid, g.total, tiles_per_gauss,
-                           g.camera_ids, g.N, rx, ry, tot, ticket, early_here, seq, db, p.counters,
+                           layout, rect, tot, ticket, early_here, seq, db, p.counters,
                            ranged ? p.bcount : (uint32_t *)nullptr);
         else
             launch_chained(isect_count_kernel<false>, cgrid, kCountThreads, 0, st, g.cam, g.total, tiles_per_gauss,
-                           g.camera_ids, g.N, rx, ry, tot, ticket, early_here, seq, db, p.counters,
+                           layout, rect, tot, ticket, early_here, seq, db, p.counters,
                            ranged ? p.bcount : (uint32_t *)nullptr);
     }
 
@@ -1866,26 +1790,29 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
         // {bits, flatten index} pairs in bucket order: keyA and valA lie back to back in the workspace
         // (each g.total words, 256-byte aligned), together room for g.total 8-byte pairs
         uint2 *pairs = reinterpret_cast<uint2 *>(p.keyA);
+        uint2 *sorted_pair = reinterpret_cast<uint2 *>(p.keyB);   // the same with keyB and valB
         if (!ranged) {
             SPL_PROF("depth_bucket_count_kernel", st);
             launch_chained(depth_bucket_count_kernel, bgrid, kThreads, 0, st, g.depth_bits,
-                           (const int32_t *)tiles_per_gauss, g.total, (const int64_t *)p.counters, p.bcount);
+                           (const int32_t *)tiles_per_gauss, g.total, layout, (const int64_t *)p.counters, p.bcount);
         }
         {
             SPL_PROF("depth_bucket_scan_kernel", st);
-            launch_chained(depth_bucket_scan_kernel, kBucketScanBlocks, 1024, 0, st, p.bcount, p.bstart, p.boff,
-                           p.counters, (volatile int64_t *)early, seq);
+            launch_chained(depth_bucket_scan_kernel, p.n_buckets / 1024, 1024, 0, st, p.bcount, p.bstart, p.boff,
+                           p.counters, (volatile int64_t *)early, seq, layout.groups, layout.per, kBlkThreads,
+                           blocks ? p.group_start : (uint32_t *)nullptr, p.group_chunk);
         }
         {
             SPL_PROF("depth_bucket_scatter_kernel", st);
             launch_chained(depth_bucket_scatter_kernel, bgrid, kThreads, 0, st, g.depth_bits,
-                           (const int32_t *)tiles_per_gauss, g.total, (const int64_t *)p.counters,
+                           (const int32_t *)tiles_per_gauss, g.total, layout, (const int64_t *)p.counters,
                            (const uint32_t *)p.bstart, (const uint32_t *)p.boff, p.bcount, pairs);
         }
         {
             SPL_PROF("depth_bucket_rank_kernel", st);
-            launch_chained(depth_bucket_rank_kernel, bgrid, kThreads, 0, st, (const int64_t *)p.counters,
-                           (const uint32_t *)p.bstart, (const uint32_t *)p.boff, (const uint2 *)pairs, p.keyB, p.valB);
+            launch_chained(depth_bucket_rank_kernel, bgrid, kThreads, 0, st, layout, p.n_buckets,
+                           (const int64_t *)p.counters, (const uint32_t *)p.bstart, (const uint32_t *)p.boff, (const uint2 *)pairs,
+                           blocks ? (const uint2 *)p.rect : (const uint2 *)nullptr, sorted_pair, p.sorted_rect, p.valB);
         }
         e.order = p.valB;
         e.n_order_ptr = p.counters + CNT_NVIS;
@@ -1939,7 +1866,7 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
         e.order = va;
         e.n_order_ptr = p.counters + CNT_NVIS;
     }
-    if (!split) {
+    if (!blocks) {
         {
             SPL_PROF("emit_blocksum_kernel", st);
             emit_blocksum_kernel<<<kSortGrid, kThreads, 0, st>>>(e, p.block_sums);
@@ -1991,69 +1918,67 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
                     g.cam, e, p.eoff, p.counters, nullptr, nullptr, isect_ids, flatten_ids, p.counters);
             }
         }
-    } else if (use_split(g, sort)) {
-        SplitArgs a{};
-        a.rect_xw = p.rect_xw;
-        a.rect_yh = p.rect_yh;
-        a.order = p.valB;
-        a.depth_key = p.keyB;
-        a.n_entries_ptr = p.counters + CNT_NVIS;
-        a.counters = p.counters;
-        a.capacity = capacity;
-        a.row_width = g.lidar ? g.lid.lidar.n_tiles_azim : g.cam.cam.tile_width;
-        a.stride = a.row_width + 1;
-        a.tile_rows = g.n_tiles / a.row_width;
-        a.rows = g.C * a.tile_rows;
-        a.tile_n_bits = g.tile_n_bits;
-        a.col_bits = max(1u, bit_length((uint64_t)a.row_width - 1));
-        a.wrap = g.lidar ? 1u : 0u;
-        SplitWs w = carve_split(fill_workspace, (uint64_t)capacity, a.rows, a.stride);
+    } else if (use_blocks(g, sort)) {
+        BlkWs w = carve_blocks(fill_workspace, (uint64_t)capacity);
         SPL_REQUIRE(fill_workspace != nullptr && fill_workspace_bytes >= w.bytes,
                     SPLATAD_ERR_WORKSPACE, "isect fill: workspace too small (%zu < %zu)",
                     fill_workspace_bytes, w.bytes);
-        a.ha_cnt = p.ha_cnt;
-        a.ha_out = p.ha_out;
-        a.hw_cnt = p.hw_cnt;
-        a.hw_out = p.hw_out;
-        a.row_rec = w.row_rec; a.row_out = w.row_out; a.row_unit = w.row_unit;
+        BlkArgs a{};
+        a.rect = p.sorted_rect;
+        a.pair = (const uint2 *)p.keyB;
+        a.sensor_start = p.group_start;
+        a.sensor_cta = p.group_chunk;
+        a.counters = p.counters;
+        a.capacity = capacity;
+        a.C = g.C;
+        a.n_tiles = g.n_tiles;
+        a.width = g.lidar ? g.lid.lidar.n_tiles_azim : g.cam.cam.tile_width;
+        a.height = g.n_tiles / a.width;
+        a.bx = div_up(a.width, kBlkW);
+        a.by = div_up(a.height, kBlkH);
+        a.blocks = a.bx * a.by;
+        a.tile_n_bits = g.tile_n_bits;
+        a.table = p.blk_table;
+        a.total = g.total;
+        a.rec_start = w.rec_start; a.unit_start = w.unit_start;
         a.rec = w.rec;
-        a.hb = w.hb; a.hw = w.hw; a.hb_first = w.hb_first; a.slot_tot = w.slot_tot; a.slot_base = w.slot_base;
-        a.warp_entries = a.rows > 32 ? kSplitWarpEntriesMin : kSplitWarpEntriesMax;
-        const uint32_t units_a = div_up(g.total, kSplitWarps * a.warp_entries);
-        const size_t smem_count = sizeof(int32_t) * kSplitWarps * a.stride;
-        const size_t smem_scatter = sizeof(int32_t) * ((kSplitWarps + 1) * a.stride + 2 * kSplitUnit) +
-                                    sizeof(uint16_t) * kSplitUnit;
-        if (smem_scatter > 32 * 1024)   // the 48 KB default also has to hold static shared memory
-            cudaFuncSetAttribute(colsplit_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_scatter);
+        a.unit_cnt = w.unit_cnt; a.tile_base = w.tile_base;
+        const uint32_t ctas_a = div_up(g.total, kBlkThreads) + (g.C > 1 ? g.C : 0u);
+        a.ctas = ctas_a;
+        const uint32_t n_blocks = a.C * a.blocks;
+        const uint32_t units_max = div_up((uint64_t)capacity, kBlkUnit) + n_blocks;
+        const uint32_t ctas_b = min(div_up(units_max, kThreads / 32), kBlkGridB);
+        const size_t smem_count = sizeof(uint32_t) * a.blocks;
+        const size_t smem_scatter = sizeof(uint32_t) * kBlkWarps * min(kBlkRows, a.by) * a.bx * (g.lidar ? 5 : 2);
+        auto count = g.lidar ? blk_count_kernel<true> : blk_count_kernel<false>;
+        auto scatter = g.lidar ? blk_scatter_kernel<true> : blk_scatter_kernel<false>;
+        if (smem_scatter > 48 * 1024)
+            cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_scatter);
+        unsigned long long *ticket = (unsigned long long *)(p.counters + CNT_TICKET);
         {
-            SPL_PROF("rowsplit_count_kernel", st);
-            launch_chained(rowsplit_count_kernel, units_a, kSplitWarps * 32, 0, st, a);
+            SPL_PROF("blk_count_kernel", st);
+            launch_chained(count, ctas_a, kBlkThreads, smem_count, st, a);
         }
         {
-            SPL_PROF("rowsplit_scan_kernel", st);
-            launch_chained(rowsplit_scan_kernel, a.rows, 1024, 0, st, a,
-                           (unsigned long long *)(p.counters + CNT_TICKET));
+            SPL_PROF("blk_scan_kernel", st);
+            launch_chained(blk_scan_kernel, n_blocks, 1024, 0, st, a, ticket);
         }
         {
-            SPL_PROF("rowsplit_scatter_kernel", st);
-            if (a.rows <= 32) launch_chained(rowsplit_scatter_kernel<true>, units_a, kSplitWarps * 32, 0, st, a);
-            else launch_chained(rowsplit_scatter_kernel<false>, units_a, kSplitWarps * 32, 0, st, a);
+            SPL_PROF("blk_scatter_kernel", st);
+            launch_chained(scatter, dim3(ctas_a, div_up(a.by, kBlkRows)), kBlkThreads, smem_scatter, st, a);
         }
         {
-            SPL_PROF("colsplit_count_kernel", st);
-            launch_chained(colsplit_count_kernel, w.units_b_cap, kSplitWarps * 32, smem_count, st, a);
+            SPL_PROF("tile_count_kernel", st);
+            launch_chained(tile_count_kernel, ctas_b, kThreads, 0, st, a);
         }
         {
-            SPL_PROF("colsplit_scan_kernel", st);
-            launch_chained(colsplit_scan_kernel, a.rows * ((a.stride + 31) / 32), 1024, 0, st, a,
-                           (unsigned long long *)(p.counters + CNT_TICKET), tile_offsets);
+            SPL_PROF("tile_scan_kernel", st);
+            launch_chained(tile_scan_kernel, n_blocks, n_blocks < kNumSMs ? 1024 : 256, 0, st, a, ticket, tile_offsets);
             tile_offsets = nullptr;   // done
         }
         {
-            SPL_PROF("colsplit_scatter_kernel", st);
-            launch_chained(colsplit_scatter_kernel, w.units_b_cap, kSplitWarps * 32, smem_scatter, st, a,
-                           isect_ids, flatten_ids, p.counters);
+            SPL_PROF("tile_scatter_kernel", st);
+            launch_chained(tile_scatter_kernel, min(div_up(units_max, kBlkOutThreads / 32), kBlkGridOut), kBlkOutThreads, 0, st, a, isect_ids, flatten_ids, p.counters);
         }
     } else {
         FillWs f = carve_fill(fill_workspace, (uint64_t)capacity);
@@ -2261,10 +2186,9 @@ extern "C" size_t splatad_isect_plan_workspace_bytes(uint64_t total_elems) {
 }
 
 extern "C" size_t splatad_isect_fill_workspace_bytes(uint64_t capacity) {
-    // the larger of the radix buffers and the split's records + tables; the widest rows and the
-    // most rows together bound (units + rows) * stride of every geometry the split accepts
+    // the larger of the radix buffers and the block split's records + tables
     const size_t a = carve_fill(nullptr, capacity).bytes;
-    const size_t b = carve_split(nullptr, capacity, kSplitMaxRows, kSplitMaxWidth + 1).bytes;
+    const size_t b = carve_blocks(nullptr, capacity).bytes;
     return a > b ? a : b;
 }
 

@@ -260,3 +260,58 @@ def test_depth_range_hint_never_changes_the_lists(lo, hi):
     # a hint is consumed by one plan: the next call measures its own range again
     _check(_run_lidar(means2d, radii, depths, eb, res, -180.0), want, "lidar, after the hint")
     ops._depth_sort_mode.clear()   # an overflow above made this shape take the radix passes: not for other tests
+
+
+@pytest.mark.parametrize("C,N,tw,th", [(1, 1, 1, 1), (1, 127, 3, 7), (1, 512, 4, 8), (2, 513, 5, 9), (3, 1500, 31, 17),
+                                       (5, 300, 64, 40), (2, 1025, 1, 70), (130, 64, 9, 3)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_block_split_at_the_edges_of_its_blocks(C, N, tw, th, packed):
+    """The lists are built over blocks of 4 x 8 tiles, 512 entries per step-A block and 128 records per
+    unit: grids one tile short of, at and beyond a block's edges, entry counts around the chunk sizes,
+    sensors without a single entry, more sensors than a warp has lanes. Bit for bit the oracle's lists."""
+    from oracle import isect
+    from splatad_b200 import ops
+    g = torch.Generator().manual_seed(C * 1000 + N)
+    ts = 16
+    m2 = (torch.rand(C, N, 2, generator=g) * 1.4 - 0.2) * torch.tensor([tw * ts, th * ts])
+    r2 = torch.randint(0, 60, (C, N, 2), generator=g, dtype=torch.int32)
+    r2[:, ::5] = r2[:, ::5] * 20                      # some cover the whole grid
+    depths = torch.rand(C, N, generator=g) * 50 + 0.1
+    depths[:, ::3] = depths[:, :1].clone()            # ties
+    if C > 2:
+        r2[1] = 0                                     # a sensor that sees nothing
+    ops._depth_sort_mode.clear()
+    if packed:
+        keep = (r2[..., 0] > 0)
+        cam = torch.nonzero(keep)[:, 0]
+        args = (m2[keep], r2[keep], depths[keep])
+        want = isect.isect_tiles(*(n(x) for x in args), ts, tw, th, n_cameras=C, camera_ids=n(cam))
+        got = ops.isect_tiles(*(t(x) for x in args), ts, tw, th, packed=True, n_cameras=C, camera_ids=t(cam),
+                              gaussian_ids=torch.zeros_like(t(cam)))
+    else:
+        want = isect.isect_tiles(n(m2), n(r2), n(depths), ts, tw, th)
+        got = ops.isect_tiles(t(m2), t(r2), t(depths), ts, tw, th)
+    for a, b, what in zip(got, want, ("tiles per Gaussian", "ids", "flatten ids")):
+        assert np.array_equal(n(a), b), what
+    offs = ops.isect_offset_encode(got[1], C, tw, th)
+    assert np.array_equal(n(offs), isect.isect_offset_encode(want[1], C, tw, th))
+
+
+@pytest.mark.parametrize("turns", [0.3, 0.99, 1.0, 1.01, 2.4, 4.5])
+def test_block_split_of_rectangles_around_the_turn(turns):
+    """Lidar rectangles that wrap past the last azimuth tile, end just short of or just past a full
+    turn, and go round more than once (their tiles then list the Gaussian once per turn)."""
+    from oracle import isect
+    from splatad_b200 import ops, scenes
+    C, N = 2, 700
+    g = torch.Generator().manual_seed(int(turns * 100))
+    eb = scenes.elevation_boundaries(scenes.beams_128(), 8)
+    means2d = torch.stack([torch.rand(C, N, generator=g) * 360 - 180, torch.rand(C, N, generator=g) * 44 - 27], -1)
+    radii = torch.rand(C, N, 2, generator=g) * torch.tensor([3.0, 3.0]) + 1e-3
+    radii[:, ::4, 0] = 180.0 * turns * (0.98 + 0.04 * torch.rand(C, radii[:, ::4].shape[1], generator=g))
+    depths = torch.rand(C, N, generator=g) * 50 + 0.1
+    res, n_az = 0.2 * 32, math.ceil(360 / (0.2 * 32))
+    want = list(isect.isect_lidar_tiles(n(means2d), n(radii), n(depths), n(eb), res, -180.0))
+    want.append(isect.isect_offset_encode(want[1], C, n_az, len(eb) - 1))
+    ops._depth_sort_mode.clear()
+    _check(_run_lidar(means2d, radii, depths, eb, res, -180.0), want, f"{turns} turns")
