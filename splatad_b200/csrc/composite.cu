@@ -38,24 +38,6 @@ __device__ __forceinline__ void stage_row(float *__restrict__ dst, const float *
     }
 }
 
-// acc[0 .. 4 * ceil(n / 4)) += row * w for a staged (zero-padded, 16-byte aligned) row: one
-// 16-byte shared-memory load and one uniform test per four channels.
-template <int CDIM>
-__device__ __forceinline__ void axpy_staged(float (&acc)[CDIM], const float *__restrict__ row, uint32_t n,
-                                            float w) {
-    const float4 *r4 = reinterpret_cast<const float4 *>(row);
-#pragma unroll
-    for (int k4 = 0; k4 < CDIM / 4; ++k4) {
-        if ((uint32_t)(4 * k4) < n) {
-            const float4 v = r4[k4];
-            acc[4 * k4 + 0] += v.x * w;
-            acc[4 * k4 + 1] += v.y * w;
-            acc[4 * k4 + 2] += v.z * w;
-            acc[4 * k4 + 3] += v.w * w;
-        }
-    }
-}
-
 // acc += row * w over a staged row of exactly CDIM floats (zero behind the channels in use).
 template <int CDIM>
 __device__ __forceinline__ void axpy_staged_full(float (&acc)[CDIM], const float *__restrict__ row, float w) {
@@ -73,12 +55,120 @@ __device__ __forceinline__ void axpy_staged_full(float (&acc)[CDIM], const float
 }
 
 // ---------------------------------------------------------------------------------------
-// Camera forward. __launch_bounds__(1024): a tile may have up to 1024 pixels, and 64 registers let
-// four 256-thread CTAs share an SM (with 66 the lidar kernel got three: 2.05 rounds of its 912 CTAs
-// instead of 1.54).
+// Camera tiles. A thread draws PX pixels next to each other in a row, so that everything that depends on
+// the Gaussian and the row alone is worked out once per thread, and the per-pixel arithmetic runs on
+// pairs of pixels (packed FP32: two results per issued instruction). A warp covers a compact patch of
+// the tile - 8 x 8 pixels of a 16 x 16 tile with PX = 2, 16 x 8 with PX = 4.
 // ---------------------------------------------------------------------------------------
+constexpr float kLog2E = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+
+template <int PX>
+struct TilePixels {
+    uint32_t x, y;   // of the thread's first pixel, within the tile
+};
+
+// threads of a CTA: whole rows of ceil(tile_size / PX) threads, rounded up to whole warps by the caller
+template <int PX>
+__host__ __device__ inline uint32_t tile_threads(uint32_t tile_size) {
+    return tile_size * ((tile_size + PX - 1) / PX);
+}
+
+template <int PX>
+__device__ __forceinline__ TilePixels<PX> tile_pixels(uint32_t tile_size, uint32_t tr) {
+    TilePixels<PX> p;
+    if (PX == 2 && tile_size == 16u) {   // 8 x 8 patches
+        const uint32_t w = tr >> 5, l = tr & 31u;
+        p.x = (w & 1u) * 8u + (l & 3u) * 2u;
+        p.y = (w >> 1) * 8u + (l >> 2);
+    } else {
+        const uint32_t per_row = (tile_size + PX - 1) / PX;
+        p.y = tr / per_row;
+        p.x = (tr - p.y * per_row) * PX;
+    }
+    return p;
+}
+
+// Pixel centres of a warp's patch.
+struct PatchBox { float x0, x1, y0, y1; };
+
+// Per-warp boxes of the CTA's patches; an empty patch gets an empty box (nothing is visible in it).
+template <int PX>
+__device__ __forceinline__ void patch_boxes(PatchBox *s_box, float px, float py, uint32_t n_inside) {
+    PatchBox b = {3.0e38f, -3.0e38f, 3.0e38f, -3.0e38f};
+    if (n_inside) b = {px, px + (float)(n_inside - 1), py, py};
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        b.x0 = fminf(b.x0, __shfl_xor_sync(0xffffffffu, b.x0, off));
+        b.x1 = fmaxf(b.x1, __shfl_xor_sync(0xffffffffu, b.x1, off));
+        b.y0 = fminf(b.y0, __shfl_xor_sync(0xffffffffu, b.y0, off));
+        b.y1 = fmaxf(b.y1, __shfl_xor_sync(0xffffffffu, b.y1, off));
+    }
+    if ((threadIdx.x & 31u) == 0u) s_box[threadIdx.x >> 5] = b;
+}
+
+// A list entry as its staging thread sees it, and the warps whose patch it can reach.
+struct PixelEntry {
+    float4 A, B;       // mean, its velocity | conic, opacity
+    uint32_t seen;     // bit w: may contribute to a pixel of warp w's patch
+};
+
+__device__ __forceinline__ PixelEntry load_pixel_entry(int32_t g, const float2 *__restrict__ means2d,
+                                                       const float *__restrict__ conics,
+                                                       const float *__restrict__ opacities,
+                                                       const float2 *__restrict__ pix_vels) {
+    PixelEntry e;
+    const float2 xy = __ldg(means2d + g), v = __ldg(pix_vels + g);
+    e.A = make_float4(xy.x, xy.y, v.x, v.y);
+    e.B = make_float4(__ldg(conics + 3 * (size_t)g), __ldg(conics + 3 * (size_t)g + 1),
+                      __ldg(conics + 3 * (size_t)g + 2), __ldg(opacities + g));
+    e.seen = 0u;
+    return e;
+}
+
+// The mean moves with the row's shutter time; roll_lo / roll_hi bound it over the tile.
+__device__ __forceinline__ uint32_t warps_that_see(const PixelEntry &e, const PatchBox *s_box, uint32_t n_warps,
+                                                   float roll_lo, float roll_hi) {
+    const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
+    if (test.never) return 0u;
+    const float mx_a = e.A.x + roll_lo * e.A.z, mx_b = e.A.x + roll_hi * e.A.z;
+    const float my_a = e.A.y + roll_lo * e.A.w, my_b = e.A.y + roll_hi * e.A.w;
+    const float mx_lo = fminf(mx_a, mx_b), mx_hi = fmaxf(mx_a, mx_b);
+    const float my_lo = fminf(my_a, my_b), my_hi = fmaxf(my_a, my_b);
+    uint32_t seen = 0u;
+    for (uint32_t w = 0; w < n_warps; ++w) {
+        const PatchBox b = s_box[w];
+        if (b.x0 <= b.x1 && !test.misses(mx_lo - b.x1, mx_hi - b.x0, my_lo - b.y1, my_hi - b.y0)) seen |= 1u << w;
+    }
+    return seen;
+}
+
+// The staged form: exp(-sigma) = 2^(a dx^2 + b dx dy + c dy^2) with the conic scaled once per entry.
+__device__ __forceinline__ float4 scaled_conic(float4 B) {
+    return make_float4(-0.5f * kLog2E * B.x, -kLog2E * B.y, -0.5f * kLog2E * B.z, B.w);
+}
+
+__device__ __forceinline__ float exp2_approx(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// exponents of a pair of pixels in one row: dx of the two, the row's b * dy and c * dy * dy
+__device__ __forceinline__ float2 pair_power(float a, float2 dx, float bdy, float cdy2) {
+    const float2 t = __ffma2_rn(make_float2(a, a), dx, make_float2(bdy, bdy));
+    return __ffma2_rn(t, dx, make_float2(cdy2, cdy2));
+}
+
+// ---------------------------------------------------------------------------------------
+// Camera forward. Bound by instruction issue: two pixels per thread take 50 instructions per entry where
+// one took 40, and a warp passes over the entries that cannot reach its 8 x 8 patch without looking at
+// them. A pixel that has stopped moves its column out to where every alpha vanishes, which costs the
+// other pixels nothing; a warp leaves when all of its pixels have. Camera benchmark frame: 0.326 -> 0.xxx ms.
+// ---------------------------------------------------------------------------------------
+constexpr float kPixelGone = 1e18f;   // a column no Gaussian reaches: sigma overflows, alpha is 0 (or NaN, never drawn)
+
 template <int CDIM>
-__global__ void __launch_bounds__(1024) rasterize_to_pixels_fwd_kernel(
+__global__ void __launch_bounds__(512) rasterize_to_pixels_fwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
     const float *__restrict__ opacities, const float2 *__restrict__ pix_vels,
@@ -86,125 +176,144 @@ __global__ void __launch_bounds__(1024) rasterize_to_pixels_fwd_kernel(
     uint32_t H, uint32_t tile_size, uint32_t tile_w, uint32_t tile_h,
     const int32_t *__restrict__ offsets, const int32_t *__restrict__ flatten_ids,
     float *__restrict__ render_colors, float *__restrict__ render_alphas,
-    int32_t *__restrict__ last_ids, uint32_t stage_colors) {
+    int32_t *__restrict__ last_ids) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ uint32_t s_warp_kept[16];
+    __shared__ PatchBox s_box[16];
     const uint32_t bs = blockDim.x;
-    float4 *sA = reinterpret_cast<float4 *>(smem_raw);   // x, y, vx, vy
-    float4 *sB = sA + bs;                                // conic a, b, c, opacity
-    int32_t *sId = reinterpret_cast<int32_t *>(sB + bs);
-    uint32_t *sPos = reinterpret_cast<uint32_t *>(sId + bs);   // list position of the staged entry
-    // colour rows of the batch (when they fit): the inner loop then never waits on global memory
-    float *sCol = reinterpret_cast<float *>(sPos + bs);
-    __shared__ uint32_t s_warp_kept[32];
-    const uint32_t cpad = (channels + 3u) & ~3u;
+    float4 *sA = reinterpret_cast<float4 *>(smem_raw);               // x, y, vx, vy
+    float4 *sB = sA + bs;                                            // scaled conic, opacity
+    float *sCol = reinterpret_cast<float *>(sB + bs);                // [bs * CDIM], zeros behind the channels
+    int32_t *sPos = reinterpret_cast<int32_t *>(sCol + bs * CDIM);   // list position of the staged entry
+    uint32_t *sSeen = reinterpret_cast<uint32_t *>(sPos + bs);       // warps that may see it
     const bool vec = (channels % 4u == 0u) && ((reinterpret_cast<uintptr_t>(colors) & 15u) == 0u);
 
     const uint32_t tiles_per_cam = tile_w * tile_h;
     const uint32_t cam = blockIdx.x / tiles_per_cam;
     const uint32_t tile = blockIdx.x - cam * tiles_per_cam;
     const uint32_t ty = tile / tile_w, tx = tile - ty * tile_w;
-    const uint32_t tr = threadIdx.x;
-    const uint32_t i = ty * tile_size + tr / tile_size;
-    const uint32_t j = tx * tile_size + tr % tile_size;
-    const bool inside = (tr < tile_size * tile_size) && (i < H && j < W);
-    const float px = (float)j + 0.5f, py = (float)i + 0.5f;
+    const uint32_t tr = threadIdx.x, lane = tr & 31u, warp = tr >> 5, n_warps = bs >> 5;
+    const TilePixels<2> tp = tile_pixels<2>(tile_size, tr);
+    const uint32_t i = ty * tile_size + tp.y, j = tx * tile_size + tp.x;
+    uint32_t n_inside = 0;   // pixels of this thread inside the tile and the image
+    if (tp.y < tile_size && i < H && j < W) n_inside = min(min(2u, tile_size - tp.x), W - j);
+    const float px0 = (float)j + 0.5f, py = (float)i + 0.5f;
     const float rs = rs_time[cam];
     const float roll = rs * ((py - 0.5f) / (float)(H - 1) - 0.5f);
-
-    // pixel centres of this tile and the rolling-shutter offsets of its first and last row: a
-    // Gaussian that cannot be seen anywhere in that box is not staged at all
-    const float box_x0 = (float)(tx * tile_size) + 0.5f;
-    const float box_x1 = (float)min((tx + 1) * tile_size, W) - 0.5f;
-    const float box_y0 = (float)(ty * tile_size) + 0.5f;
-    const float box_y1 = (float)min((ty + 1) * tile_size, H) - 0.5f;
-    const float roll_a = rs * ((box_y0 - 0.5f) / (float)(H - 1) - 0.5f);
-    const float roll_b = rs * ((box_y1 - 0.5f) / (float)(H - 1) - 0.5f);
+    // shutter times of the tile's first and last row
+    const float roll_a = rs * ((float)(ty * tile_size) / (float)(H - 1) - 0.5f);
+    const float roll_b = rs * ((float)(min((ty + 1) * tile_size, H) - 1) / (float)(H - 1) - 0.5f);
     const float roll_lo = fminf(roll_a, roll_b), roll_hi = fmaxf(roll_a, roll_b);
-    const uint32_t lane = tr & 31u, warp = tr >> 5, n_warps = bs >> 5;
+    patch_boxes<2>(s_box, px0, py, n_inside);
 
     const TileRange range = tile_range(offsets, blockIdx.x, C * tiles_per_cam, n_isects);
     const uint32_t num_batches = (uint32_t)(range.end - range.start + bs - 1) / bs;
 
-    bool done = !inside;
-    float T = 1.f;
-    uint32_t cur_idx = 0;
-    float pix_out[CDIM];
+    float2 px = make_float2(n_inside > 0 ? px0 : kPixelGone, n_inside > 1 ? px0 + 1.f : kPixelGone);
+    float2 T = make_float2(1.f, 1.f);
+    int32_t last0 = 0, last1 = 0;
+    float out[2][CDIM];
 #pragma unroll
-    for (int k = 0; k < CDIM; ++k) pix_out[k] = 0.f;
+    for (int k = 0; k < CDIM; ++k) out[0][k] = out[1][k] = 0.f;
+    bool gone = n_inside == 0;   // both pixels have stopped (or are not there)
+    bool warp_done = __all_sync(0xffffffffu, gone);
 
+    int32_t next_id = 0;
+    if (range.start + (int32_t)tr < range.end) next_id = flatten_ids[range.start + tr];
     for (uint32_t b = 0; b < num_batches; ++b) {
-        if (__syncthreads_count(done) >= (int)bs) break;
-        const uint32_t batch_start = (uint32_t)range.start + bs * b;
-        const uint32_t idx = batch_start + tr;
-        bool keep = false;
-        int32_t g = 0;
-        float4 A, B;
-        if (idx < (uint32_t)range.end) {
-            g = flatten_ids[idx];
-            const float2 xy = means2d[g];
-            const float2 v = pix_vels[g];
-            A = make_float4(xy.x, xy.y, v.x, v.y);
-            B = make_float4(conics[3 * (size_t)g], conics[3 * (size_t)g + 1],
-                            conics[3 * (size_t)g + 2], opacities[g]);
-            // offsets mean - pixel over the tile; the mean moves with the row's shutter time
-            const float mx_a = A.x + roll_lo * A.z, mx_b = A.x + roll_hi * A.z;
-            const float my_a = A.y + roll_lo * A.w, my_b = A.y + roll_hi * A.w;
-            keep = !never_visible_in_box(B.x, B.y, B.z, B.w, fminf(mx_a, mx_b) - box_x1,
-                                         fmaxf(mx_a, mx_b) - box_x0, fminf(my_a, my_b) - box_y1,
-                                         fmaxf(my_a, my_b) - box_y0);
+        if (__syncthreads_and(warp_done)) break;
+        const int32_t idx = range.start + (int32_t)(bs * b + tr);
+        const int32_t g = next_id;
+        PixelEntry e;
+        e.seen = 0u;
+        if (idx < range.end) {
+            e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
+            if (idx + (int32_t)bs < range.end) next_id = flatten_ids[idx + bs];   // on its way meanwhile
+            e.seen = warps_that_see(e, s_box, n_warps, roll_lo, roll_hi);
         }
         // compact the survivors to the front of the staging arrays, list order kept
-        const uint32_t kept_mask = __ballot_sync(0xffffffffu, keep);
+        const uint32_t kept_mask = __ballot_sync(0xffffffffu, e.seen != 0u);
         if (lane == 0) s_warp_kept[warp] = __popc(kept_mask);
         __syncthreads();
-        uint32_t pos = __popc(kept_mask & ((1u << lane) - 1u)), batch_size = 0;
+        uint32_t pos = __popc(kept_mask & ((1u << lane) - 1u)), n_kept = 0;
         for (uint32_t w = 0; w < n_warps; ++w) {
             const uint32_t cnt = s_warp_kept[w];
             if (w < warp) pos += cnt;
-            batch_size += cnt;
+            n_kept += cnt;
         }
-        if (keep) {
-            sA[pos] = A;
-            sB[pos] = B;
-            sId[pos] = g;
+        if (e.seen) {
+            sA[pos] = e.A;
+            sB[pos] = scaled_conic(e.B);
             sPos[pos] = idx;
-            if (stage_colors) stage_row(sCol + pos * cpad, colors, (size_t)g, channels, vec);
+            sSeen[pos] = e.seen;
+            float *row = sCol + pos * CDIM;
+            stage_row(row, colors, (size_t)g, channels, vec);
+            for (uint32_t k = (channels + 3u) & ~3u; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
         }
         __syncthreads();
-        if (__all_sync(0xffffffffu, done)) continue;
-        for (uint32_t t = 0; t < batch_size && !done; ++t) {
-            const float4 A = sA[t];
-            const float4 B = sB[t];
-            const float dx = A.x + roll * A.z - px;
-            const float dy = A.y + roll * A.w - py;
-            const float sigma = 0.5f * (B.x * dx * dx + B.z * dy * dy) + B.y * dx * dy;
-            const float alpha = fminf(kAlphaMax, B.w * __expf(-sigma));
-            if (sigma < 0.f || alpha < kAlphaMin) continue;
-            const float next_T = T * (1.f - alpha);
-            if (next_T <= kTStop) { done = true; break; }
-            const float vis = alpha * T;
-            if (stage_colors) {
-                axpy_staged<CDIM>(pix_out, sCol + t * cpad, channels, vis);
-            } else {
-                const float *c_ptr = colors + (size_t)sId[t] * channels;
+        if (warp_done) continue;
+        for (uint32_t t0 = 0; t0 < n_kept && !warp_done; t0 += 32) {
+            const uint32_t mine = t0 + lane;
+            uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u));
+            while (todo && !(warp_done = __all_sync(0xffffffffu, gone))) {
+                const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
+                todo &= todo - 1u;
+                const float4 A = sA[t], B = sB[t];
+                const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
+                const float2 dx = __fadd2_rn(make_float2(mx, mx), make_float2(-px.x, -px.y));
+                const float2 pw = pair_power(B.x, dx, B.y * dy, B.z * dy * dy);
+                const float2 av = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
+                const bool ok0 = pw.x <= 0.f && av.x >= kAlphaMin, ok1 = pw.y <= 0.f && av.y >= kAlphaMin;
+                if (!(ok0 || ok1)) continue;
+                const float2 alpha = make_float2(ok0 ? fminf(kAlphaMax, av.x) : 0.f, ok1 ? fminf(kAlphaMax, av.y) : 0.f);
+                const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
+                const float2 next_T = __fmul2_rn(T, om);
+                float2 vis = __fmul2_rn(alpha, T);
+                const bool stop0 = ok0 && next_T.x <= kTStop, stop1 = ok1 && next_T.y <= kTStop;
+                if (stop0) { px.x = kPixelGone; vis.x = 0.f; } else T.x = next_T.x;
+                if (stop1) { px.y = kPixelGone; vis.y = 0.f; } else T.y = next_T.y;
+                gone = px.x == kPixelGone && px.y == kPixelGone;
+                const float4 *row = reinterpret_cast<const float4 *>(sCol + t * CDIM);
+                const float2 w0 = make_float2(vis.x, vis.x), w1 = make_float2(vis.y, vis.y);
 #pragma unroll
-                for (int k = 0; k < CDIM; ++k)
-                    if ((uint32_t)k < channels) pix_out[k] += __ldg(c_ptr + k) * vis;
+                for (int k = 0; k < CDIM; k += 4) {
+                    const float4 c4 = row[k / 4];
+#pragma unroll
+                    for (int h = 0; h < 4; h += 2) {
+                        const float2 c2 = h ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
+                        const float2 a = __ffma2_rn(c2, w0, make_float2(out[0][k + h], out[0][k + h + 1]));
+                        const float2 d = __ffma2_rn(c2, w1, make_float2(out[1][k + h], out[1][k + h + 1]));
+                        out[0][k + h] = a.x; out[0][k + h + 1] = a.y;
+                        out[1][k + h] = d.x; out[1][k + h + 1] = d.y;
+                    }
+                }
+                const int32_t entry = sPos[t];
+                if (ok0 && !stop0) last0 = entry;
+                if (ok1 && !stop1) last1 = entry;
             }
-            cur_idx = sPos[t];
-            T = next_T;
+            warp_done = __all_sync(0xffffffffu, gone);
         }
     }
-    if (inside) {
-        const size_t pix = ((size_t)cam * H + i) * W + j;
-        render_alphas[pix] = 1.f - T;
-        const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
+    const bool vec_out = channels == 4u && (reinterpret_cast<uintptr_t>(render_colors) & 15u) == 0u;
+    const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if ((uint32_t)h >= n_inside) break;
+        const size_t pix = ((size_t)cam * H + i) * W + j + h;
+        const float Tk = h ? T.y : T.x;
+        render_alphas[pix] = 1.f - Tk;
+        last_ids[pix] = h ? last1 : last0;
+        float *dst = render_colors + pix * channels;
+        if (CDIM == 4 && vec_out) {   // one 16-byte store per pixel
+            float4 v = make_float4(out[h][0], out[h][1], out[h][2], out[h][3]);
+            if (bg) v = make_float4(v.x + Tk * bg[0], v.y + Tk * bg[1], v.z + Tk * bg[2], v.w + Tk * bg[3]);
+            *reinterpret_cast<float4 *>(dst) = v;
+            continue;
+        }
 #pragma unroll
         for (int k = 0; k < CDIM; ++k)
-            if ((uint32_t)k < channels)
-                render_colors[pix * channels + k] = bg ? (pix_out[k] + T * bg[k]) : pix_out[k];
-        last_ids[pix] = (int32_t)cur_idx;
+            if ((uint32_t)k < channels) dst[k] = bg ? out[h][k] + Tk * bg[k] : out[h][k];
     }
 }
 
@@ -397,11 +506,54 @@ __device__ __forceinline__ int block_max_int(int v, int *red /* [32] */) {
     return m;
 }
 
+// What a lane does with the warp total it ends up holding: which array it belongs to, and the factor
+// common to all pixels (times the entry's opacity where the derivative runs through sigma).
+struct GradSlot {
+    float *base;
+    uint32_t stride;
+    float scale;
+    bool times_opacity;
+    __device__ __forceinline__ void add(size_t g, float total, float opacity, bool writes) const {
+        const float v = total * (times_opacity ? scale * opacity : scale);
+        if (writes && base != nullptr && v != 0.f) atomicAdd(base + g * stride, v);
+    }
+};
+
+template <bool kAbs>
+__device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t channels, float *v_colors,
+                                                    float *v_conics, float *v_means2d, float *v_pix_vels,
+                                                    float *v_opacities, float *v_means2d_abs) {
+    if (slot < cdim) return {(uint32_t)slot < channels ? v_colors + slot : nullptr, channels, 1.f, false};
+    switch (slot - cdim) {
+        case 0: return {v_conics, 3u, -0.5f, true};
+        case 1: return {v_conics + 1, 3u, -1.f, true};
+        case 2: return {v_conics + 2, 3u, -0.5f, true};
+        case 3: return {v_means2d, 2u, kLn2, true};
+        case 4: return {v_means2d + 1, 2u, kLn2, true};
+        case 5: return {v_pix_vels, 2u, kLn2, true};
+        case 6: return {v_pix_vels + 1, 2u, kLn2, true};
+        case 7: return {v_opacities, 1u, 1.f, false};
+        case 8: return {kAbs ? v_means2d_abs : nullptr, 2u, kLn2, true};
+        case 9: return {kAbs ? v_means2d_abs + 1 : nullptr, 2u, kLn2, true};
+        default: return {nullptr, 0u, 0.f, false};
+    }
+}
+
 // ---------------------------------------------------------------------------------------
-// Camera backward
+// Camera backward: back to front from the last entry any pixel of the tile consumed.
+//
+// What bounds it is instruction issue, and the parts that do not depend on the pixel were most of it:
+// with one pixel per thread the 14 warp totals of an entry took as many instructions as the gradients
+// themselves. So a thread takes four pixels of a row (two with more than 8 channels), adds their terms
+// up before anything is exchanged, and as dy and the row's shutter time are common to them it needs only
+// the sums of v, v dx and v dx^2 (v = exp(-sigma) dL/dalpha). The channels behind an entry enter through
+// one number per pixel: dL/dalpha = T (c . g) - (1 / (1 - alpha)) (sum over the entries behind of
+// their weight times their (c . g)), g the pixel's cotangent - a running scalar in place of a running colour.
+// Camera benchmark frame, training step: 1.50 -> 0.5x ms.
 // ---------------------------------------------------------------------------------------
-template <int CDIM>
-__global__ void rasterize_to_pixels_bwd_kernel(
+template <int CDIM, int PX, bool kAbs>
+__global__ void __launch_bounds__(PX == 4 || CDIM > 16 ? 256 : 512)
+rasterize_to_pixels_bwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
     const float *__restrict__ opacities, const float2 *__restrict__ pix_vels,
@@ -413,88 +565,102 @@ __global__ void rasterize_to_pixels_bwd_kernel(
     float *__restrict__ v_means2d_abs, float *__restrict__ v_means2d,
     float *__restrict__ v_conics, float *__restrict__ v_colors, float *__restrict__ v_opacities,
     float *__restrict__ v_pix_vels) {
+    static_assert(PX % 2 == 0, "pixels are handled in pairs");
+    constexpr int P2 = PX / 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int red[32];
+    __shared__ uint32_t s_warp_kept[32];
+    __shared__ PatchBox s_box[16];
     const uint32_t bs = blockDim.x;
     float4 *sA = reinterpret_cast<float4 *>(smem_raw);
     float4 *sB = sA + bs;
-    int32_t *sId = reinterpret_cast<int32_t *>(sB + bs);
-    int32_t *sPos = sId + bs;                            // list position of the staged entry
-    float *sRgb = reinterpret_cast<float *>(sPos + bs);  // [bs * CDIM]
-    __shared__ uint32_t s_warp_kept[32];
+    float *sRgb = reinterpret_cast<float *>(sB + bs);                  // [bs * CDIM], zeros behind the channels
+    int32_t *sId = reinterpret_cast<int32_t *>(sRgb + bs * CDIM);
+    int32_t *sPos = sId + bs;                                          // list position of the staged entry
+    uint32_t *sSeen = reinterpret_cast<uint32_t *>(sPos + bs);         // warps that may see it
 
     const uint32_t tiles_per_cam = tile_w * tile_h;
     const uint32_t cam = blockIdx.x / tiles_per_cam;
     const uint32_t tile = blockIdx.x - cam * tiles_per_cam;
     const uint32_t ty = tile / tile_w, tx = tile - ty * tile_w;
-    const uint32_t tr = threadIdx.x;
-    const uint32_t i = ty * tile_size + tr / tile_size;
-    const uint32_t j = tx * tile_size + tr % tile_size;
-    const bool inside = (tr < tile_size * tile_size) && (i < H && j < W);
-    const float px = (float)j + 0.5f, py = (float)i + 0.5f;
+    const uint32_t tr = threadIdx.x, lane = tr & 31, warp = tr >> 5, n_warps = bs >> 5;
+    const TilePixels<PX> tp = tile_pixels<PX>(tile_size, tr);
+    const uint32_t i = ty * tile_size + tp.y, j = tx * tile_size + tp.x;
+    // pixels of this thread inside the tile and the image
+    uint32_t n_inside = 0;
+    if (tp.y < tile_size && i < H && j < W) n_inside = min(min((uint32_t)PX, tile_size - tp.x), W - j);
+    const float px0 = (float)j + 0.5f, py = (float)i + 0.5f;
     const float rs = rs_time[cam];
     const float roll = rs * ((py - 0.5f) / (float)(H - 1) - 0.5f);
-    const size_t pix = ((size_t)cam * H + min(i, H - 1)) * W + min(j, W - 1);
-    // box of the tile's pixel centres and the shutter offsets of its first and last row, as in the
-    // forward kernel: entries that cannot be seen anywhere in the tile are not staged
-    const float box_x0 = (float)(tx * tile_size) + 0.5f;
-    const float box_x1 = (float)min((tx + 1) * tile_size, W) - 0.5f;
-    const float box_y0 = (float)(ty * tile_size) + 0.5f;
-    const float box_y1 = (float)min((ty + 1) * tile_size, H) - 0.5f;
-    const float roll_a = rs * ((box_y0 - 0.5f) / (float)(H - 1) - 0.5f);
-    const float roll_b = rs * ((box_y1 - 0.5f) / (float)(H - 1) - 0.5f);
+    // shutter times of the tile's first and last row
+    const float roll_a = rs * ((float)(ty * tile_size) / (float)(H - 1) - 0.5f);
+    const float roll_b = rs * ((float)(min((ty + 1) * tile_size, H) - 1) / (float)(H - 1) - 0.5f);
     const float roll_lo = fminf(roll_a, roll_b), roll_hi = fmaxf(roll_a, roll_b);
+    patch_boxes<PX>(s_box, px0, py, n_inside);
 
     const TileRange range = tile_range(offsets, blockIdx.x, C * tiles_per_cam, n_isects);
     const bool vec = (channels % 4u == 0u) && ((reinterpret_cast<uintptr_t>(colors) & 15u) == 0u);
 
-    const float T_final = 1.f - render_alphas[pix];
-    float T = T_final;
-    const int32_t bin_final = inside ? last_ids[pix] : 0;
-    float buffer[CDIM], v_render_c[CDIM];
-    float bg_dot = 0.f;
+    float2 T[P2], behind[P2];        // transmittance in front of the entry; weighted (c . g) behind it
+    float v_out[PX][CDIM];           // cotangents of the pixels' channels
+    int32_t bin_final[PX];
+    int32_t thread_last = -1;
 #pragma unroll
-    for (int k = 0; k < CDIM; ++k) {
-        buffer[k] = 0.f;
-        v_render_c[k] = ((uint32_t)k < channels && inside) ? v_render_colors[pix * channels + k] : 0.f;
-        if (backgrounds != nullptr && (uint32_t)k < channels)
-            bg_dot += backgrounds[(size_t)cam * channels + k] * v_render_c[k];
+    for (int k = 0; k < PX; ++k) {
+        const bool in = (uint32_t)k < n_inside;
+        const size_t pix = ((size_t)cam * H + (in ? i : 0u)) * W + (in ? j + k : 0u);
+        const float T_final = in ? 1.f - render_alphas[pix] : 1.f;
+        bin_final[k] = in ? last_ids[pix] : -1;
+        thread_last = max(thread_last, bin_final[k]);
+        float bg_dot = 0.f;
+#pragma unroll
+        for (int c = 0; c < CDIM; ++c) {
+            v_out[k][c] = (in && (uint32_t)c < channels) ? v_render_colors[pix * channels + c] : 0.f;
+            if (backgrounds != nullptr && (uint32_t)c < channels)
+                bg_dot += backgrounds[(size_t)cam * channels + c] * v_out[k][c];
+        }
+        const float v_a = in ? v_render_alphas[pix] : 0.f;
+        // what the background and the alpha output receive through everything in front of them
+        const float last = -T_final * (v_a - bg_dot);
+        if (k & 1) { T[k / 2].y = T_final; behind[k / 2].y = last; }
+        else { T[k / 2].x = T_final; behind[k / 2].x = last; }
     }
-    const float v_render_a = inside ? v_render_alphas[pix] : 0.f;
 
-    // last list position consumed by any pixel of this tile
-    const int32_t tile_last = block_max_int(bin_final, red);
-    int32_t warp_bin_final = bin_final;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-        warp_bin_final = max(warp_bin_final, __shfl_xor_sync(0xffffffffu, warp_bin_final, off));
+    // last list position consumed by any pixel of this tile / warp
+    const int32_t tile_last = block_max_int(thread_last, red);
+    const int32_t warp_last = __reduce_max_sync(0xffffffffu, thread_last);
     const int32_t eff_end = min(range.end, tile_last + 1);
     if (eff_end <= range.start) return;
     const uint32_t num_batches = (uint32_t)(eff_end - range.start + bs - 1) / bs;
-    const uint32_t lane = tr & 31, warp = tr >> 5, n_warps = bs >> 5;
 
+    // Where the warp total that ends up on this lane goes: colours first, then the geometry.
+    constexpr int kGeo = kAbs ? 10 : 8;
+    constexpr int kSlots = CDIM + kGeo <= 16 ? 16 : 32;
+    constexpr bool kSplit = CDIM + kGeo > 32;   // the geometry in a butterfly of its own
+    const GradSlot slot_a = pixel_grad_slot<kAbs>(kSplit ? (int)lane : (int)(lane * kSlots / 32u), CDIM, channels, v_colors,
+                                                  v_conics, v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
+    const bool writes_a = kSlots == 32 || (lane & 1u) == 0u;
+
+    int32_t next_id = 0;
+    {
+        const int32_t idx = eff_end - 1 - (int32_t)tr;
+        if (idx >= range.start) next_id = flatten_ids[idx];
+    }
     for (uint32_t b = 0; b < num_batches; ++b) {
-        __syncthreads();
         const int32_t batch_end = eff_end - 1 - (int32_t)(bs * b);
         const int32_t idx = batch_end - (int32_t)tr;
-        bool keep = false;
-        int32_t g = 0;
-        float4 A, B0;
+        const int32_t g = next_id;
+        PixelEntry e;
+        e.seen = 0u;
         if (idx >= range.start) {
-            g = flatten_ids[idx];
-            const float2 xy = means2d[g];
-            const float2 v = pix_vels[g];
-            A = make_float4(xy.x, xy.y, v.x, v.y);
-            B0 = make_float4(conics[3 * (size_t)g], conics[3 * (size_t)g + 1],
-                             conics[3 * (size_t)g + 2], opacities[g]);
-            const float mx_a = A.x + roll_lo * A.z, mx_b = A.x + roll_hi * A.z;
-            const float my_a = A.y + roll_lo * A.w, my_b = A.y + roll_hi * A.w;
-            keep = !never_visible_in_box(B0.x, B0.y, B0.z, B0.w, fminf(mx_a, mx_b) - box_x1,
-                                         fmaxf(mx_a, mx_b) - box_x0, fminf(my_a, my_b) - box_y1,
-                                         fmaxf(my_a, my_b) - box_y0);
+            e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
+            e.seen = warps_that_see(e, s_box, n_warps, roll_lo, roll_hi);
+            const int32_t ahead = idx - (int32_t)bs;   // the id of the next batch's entry is on its way meanwhile
+            if (ahead >= range.start) next_id = flatten_ids[ahead];
         }
         // survivors to the front, still back to front in list order
-        const uint32_t kept_mask = __ballot_sync(0xffffffffu, keep);
+        const uint32_t kept_mask = __ballot_sync(0xffffffffu, e.seen != 0u);
+        __syncthreads();   // the batch before has been read
         if (lane == 0) s_warp_kept[warp] = __popc(kept_mask);
         __syncthreads();
         uint32_t pos = __popc(kept_mask & ((1u << lane) - 1u)), n_kept = 0;
@@ -503,118 +669,122 @@ __global__ void rasterize_to_pixels_bwd_kernel(
             if (w < warp) pos += cnt;
             n_kept += cnt;
         }
-        if (keep) {
-            sA[pos] = A;
-            sB[pos] = B0;
+        if (e.seen) {
+            sA[pos] = e.A;
+            sB[pos] = scaled_conic(e.B);
             sId[pos] = g;
             sPos[pos] = idx;
-            // rows of CDIM floats (channels, then zeros): the channel loops run in packed pairs
+            sSeen[pos] = e.seen;
             float *row = sRgb + pos * CDIM;
             stage_row(row, colors, (size_t)g, channels, vec);
             for (uint32_t k = (channels + 3u) & ~3u; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
         }
         __syncthreads();
-        for (uint32_t t = 0; t < n_kept; ++t) {
-            const int32_t entry = sPos[t];
-            if (entry > warp_bin_final) continue;   // behind everything this warp consumed
-            bool valid = inside && (entry <= bin_final);
-            float alpha = 0.f, opac = 0.f, vis = 0.f, dx = 0.f, dy = 0.f;
-            float4 B = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (valid) {
-                const float4 A = sA[t];
-                B = sB[t];
-                opac = B.w;
-                dx = A.x + roll * A.z - px;
-                dy = A.y + roll * A.w - py;
-                const float sigma = 0.5f * (B.x * dx * dx + B.z * dy * dy) + B.y * dx * dy;
-                vis = __expf(-sigma);
-                alpha = fminf(kAlphaMax, opac * vis);
-                if (sigma < 0.f || alpha < kAlphaMin) valid = false;
-            }
-            if (!__any_sync(0xffffffffu, valid)) continue;
-            float v_rgb[CDIM];
+        for (uint32_t t0 = 0; t0 < n_kept; t0 += 32) {
+            const uint32_t mine = t0 + lane;
+            uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u) && sPos[mine] <= warp_last);
+            while (todo) {
+                const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
+                todo &= todo - 1u;
+                const float4 A = sA[t], B = sB[t];
+                const int32_t entry = sPos[t];
+                const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
+                const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
+                float2 dx[P2], vis[P2], av[P2];
+                bool any = false;
 #pragma unroll
-            for (int k = 0; k < CDIM; ++k) v_rgb[k] = 0.f;
-            float v_conic_x = 0.f, v_conic_y = 0.f, v_conic_z = 0.f;
-            float v_x = 0.f, v_y = 0.f, v_ax = 0.f, v_ay = 0.f, v_vx = 0.f, v_vy = 0.f, v_o = 0.f;
-            if (valid) {
-                const float ra = 1.f / (1.f - alpha);
-                T *= ra;
-                const float fac = alpha * T;
-                // two channels per instruction (packed FP32 multiply-adds); channels beyond the
-                // rendered ones have zero rows, zero cotangents and zero buffers
-                const float *rgb = sRgb + (uint32_t)t * CDIM;
-                const float2 fac2 = make_float2(fac, fac), T2 = make_float2(T, T), nra2 = make_float2(-ra, -ra);
-                float2 va2 = make_float2(0.f, 0.f);
+                for (int q = 0; q < P2; ++q) {
+                    dx[q] = make_float2(mx - (px0 + (float)(2 * q)), mx - (px0 + (float)(2 * q + 1)));
+                    const float2 pw = pair_power(B.x, dx[q], bdy, cdy2);
+                    const float2 ex = make_float2(exp2_approx(pw.x), exp2_approx(pw.y));
+                    av[q] = __fmul2_rn(make_float2(B.w, B.w), ex);
+                    const bool ok0 = pw.x <= 0.f && av[q].x >= kAlphaMin && entry <= bin_final[2 * q];
+                    const bool ok1 = pw.y <= 0.f && av[q].y >= kAlphaMin && entry <= bin_final[2 * q + 1];
+                    any = any || ok0 || ok1;
+                    if (!ok0) av[q].x = 0.f;
+                    if (!ok1) av[q].y = 0.f;
+                    // a capped alpha passes no gradient on to the geometry
+                    vis[q] = make_float2(ok0 && av[q].x <= kAlphaMax ? ex.x : 0.f, ok1 && av[q].y <= kAlphaMax ? ex.y : 0.f);
+                }
+                if (!__any_sync(0xffffffffu, any)) continue;
+                float sum[CDIM + kGeo];
+                float2 s0 = make_float2(0.f, 0.f), s1 = s0, s2 = s0, ax = s0, ay = s0;
+                float4 rgb[CDIM / 4];
 #pragma unroll
-                for (int k = 0; k < CDIM; k += 4) {
-                    const float4 c4 = *reinterpret_cast<const float4 *>(rgb + k);
+                for (int k = 0; k < CDIM / 4; ++k) rgb[k] = reinterpret_cast<const float4 *>(sRgb + t * CDIM)[k];
+#pragma unroll
+                for (int q = 0; q < P2; ++q) {
+                    const float2 alpha = make_float2(fminf(kAlphaMax, av[q].x), fminf(kAlphaMax, av[q].y));
+                    const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
+                    const float2 ra = make_float2(1.f / om.x, 1.f / om.y);
+                    T[q] = __fmul2_rn(T[q], ra);
+                    const float2 fac = __fmul2_rn(alpha, T[q]);
+                    float2 dot;   // (c . g) of the two pixels
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const int q = k + 2 * h;
-                        const float2 c2 = h ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
-                        const float2 vr2 = make_float2(v_render_c[q], v_render_c[q + 1]);
-                        const float2 b2 = make_float2(buffer[q], buffer[q + 1]);
-                        const float2 g2 = __fmul2_rn(fac2, vr2);
-                        v_rgb[q] = g2.x; v_rgb[q + 1] = g2.y;
-                        const float2 u2 = __ffma2_rn(c2, T2, __fmul2_rn(b2, nra2));   // rgb T - buffer ra
-                        va2 = __ffma2_rn(u2, vr2, va2);
-                        const float2 nb2 = __ffma2_rn(c2, fac2, b2);
-                        buffer[q] = nb2.x; buffer[q + 1] = nb2.y;
+                        const float *v = v_out[2 * q + h];
+                        const float f = h ? fac.y : fac.x;
+                        const float2 f2 = make_float2(f, f);
+                        float2 d2 = make_float2(0.f, 0.f);
+#pragma unroll
+                        for (int k = 0; k < CDIM; k += 2) {
+                            const float4 c4 = rgb[k / 4];
+                            const float2 c2 = (k & 2) ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
+                            const float2 v2 = make_float2(v[k], v[k + 1]);
+                            d2 = k == 0 ? __fmul2_rn(c2, v2) : __ffma2_rn(c2, v2, d2);
+                            const float2 acc = (q == 0 && h == 0) ? __fmul2_rn(f2, v2)
+                                                                  : __ffma2_rn(f2, v2, make_float2(sum[k], sum[k + 1]));
+                            sum[k] = acc.x; sum[k + 1] = acc.y;
+                        }
+                        if (h) dot.y = d2.x + d2.y; else dot.x = d2.x + d2.y;
+                    }
+                    const float2 nra = make_float2(-ra.x, -ra.y);
+                    const float2 v_alpha = __ffma2_rn(T[q], dot, __fmul2_rn(nra, behind[q]));
+                    behind[q] = __ffma2_rn(fac, dot, behind[q]);
+                    const float2 v = __fmul2_rn(vis[q], v_alpha), vx = __fmul2_rn(v, dx[q]);
+                    s0 = q == 0 ? v : __fadd2_rn(s0, v);
+                    s1 = q == 0 ? vx : __fadd2_rn(s1, vx);
+                    s2 = q == 0 ? __fmul2_rn(vx, dx[q]) : __ffma2_rn(vx, dx[q], s2);
+                    if (kAbs) {
+                        const float2 gx = __ffma2_rn(make_float2(2.f * B.x, 2.f * B.x), dx[q], make_float2(bdy, bdy));
+                        const float2 gy = __ffma2_rn(make_float2(B.y, B.y), dx[q], make_float2(2.f * B.z * dy, 2.f * B.z * dy));
+                        const float2 wx = __fmul2_rn(v, gx), wy = __fmul2_rn(v, gy);
+                        ax = __fadd2_rn(ax, make_float2(fabsf(wx.x), fabsf(wx.y)));
+                        ay = __fadd2_rn(ay, make_float2(fabsf(wy.x), fabsf(wy.y)));
                     }
                 }
-                float v_alpha = va2.x + va2.y;
-                v_alpha += T_final * ra * v_render_a;
-                if (backgrounds != nullptr) v_alpha += -T_final * ra * bg_dot;
-                if (opac * vis <= kAlphaMax) {
-                    const float v_sigma = -opac * vis * v_alpha;
-                    v_conic_x = 0.5f * v_sigma * dx * dx;
-                    v_conic_y = v_sigma * dx * dy;
-                    v_conic_z = 0.5f * v_sigma * dy * dy;
-                    v_x = v_sigma * (B.x * dx + B.y * dy);
-                    v_y = v_sigma * (B.y * dx + B.z * dy);
-                    v_vx = v_x * roll;
-                    v_vy = v_y * roll;
-                    v_ax = fabsf(v_x);
-                    v_ay = fabsf(v_y);
-                    v_o = vis * v_alpha;
+                // sigma's derivatives: v_sigma = -opacity v; the factors that are the same for every
+                // pixel follow when the totals are written
+                const float m0 = s0.x + s0.y, m1 = s1.x + s1.y, my = dy * m0;
+                const float gx = 2.f * B.x * m1 + B.y * my, gy = B.y * m1 + 2.f * B.z * my;
+                sum[CDIM + 0] = s2.x + s2.y;
+                sum[CDIM + 1] = dy * m1;
+                sum[CDIM + 2] = dy * my;
+                sum[CDIM + 3] = gx;
+                sum[CDIM + 4] = gy;
+                sum[CDIM + 5] = gx * roll;
+                sum[CDIM + 6] = gy * roll;
+                sum[CDIM + 7] = m0;
+                if (kAbs) {
+                    sum[CDIM + 8] = ax.x + ax.y;
+                    sum[CDIM + 9] = ay.x + ay.y;
+                }
+                const size_t g = (size_t)sId[t];
+                float slots[kSlots];
+#pragma unroll
+                for (int k = 0; k < kSlots; ++k) slots[k] = k < (kSplit ? CDIM : CDIM + kGeo) ? sum[k] : 0.f;
+                const float total = warp_sum_slots<kSlots>(slots, lane);
+                slot_a.add(g, total, B.w, writes_a);
+                if (kSplit) {
+                    float geo[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) geo[k] = k < kGeo ? sum[CDIM + k] : 0.f;
+                    const float geo_total = warp_sum_slots<16>(geo, lane);
+                    const GradSlot slot_b = pixel_grad_slot<kAbs>(CDIM + (int)(lane >> 1), CDIM, channels, v_colors, v_conics,
+                                                                  v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
+                    slot_b.add(g, geo_total, B.w, (lane & 1u) == 0u);
                 }
             }
-            // warp totals by multi-value butterflies; each total then sits on its own lane, which adds it in
-            const size_t g = (size_t)sId[t];
-            float g_tot;
-            uint32_t gi;   // index of the geometry gradient this lane ends up holding
-            if (CDIM + 10 <= 16) {
-                // up to 6 channels: colours and geometry share one 16-value butterfly
-                float gs[16] = {v_conic_x, v_conic_y, v_conic_z, v_x, v_y, v_vx, v_vy, v_o, v_ax, v_ay,
-                                0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int k = 0; k < CDIM && k < 6; ++k) gs[10 + k] = v_rgb[k];
-                g_tot = warp_sum_slots<16>(gs, lane);
-                gi = lane >> 1;
-                if ((lane & 1u) == 0u && gi >= 10u && gi - 10u < channels)
-                    atomicAdd(v_colors + g * channels + (gi - 10u), g_tot);
-            } else {
-                constexpr int kColorSlots = pow2_at_least(CDIM);
-                float cs[kColorSlots];
-#pragma unroll
-                for (int k = 0; k < kColorSlots; ++k) cs[k] = k < CDIM ? v_rgb[k] : 0.f;
-                float gs[16] = {v_conic_x, v_conic_y, v_conic_z, v_x, v_y, v_vx, v_vy, v_o, v_ax, v_ay,
-                                0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                const float c_tot = warp_sum_slots<kColorSlots>(cs, lane);
-                g_tot = warp_sum_slots<16>(gs, lane);
-                gi = lane >> 1;
-                const uint32_t ci = (lane * (uint32_t)kColorSlots) >> 5;
-                if ((lane & (32u / kColorSlots - 1u)) == 0u && ci < channels)
-                    atomicAdd(v_colors + g * channels + ci, c_tot);
-            }
-            float *dst = nullptr;
-            if (gi < 3u) dst = v_conics + 3 * g + gi;
-            else if (gi < 5u) dst = v_means2d + 2 * g + (gi - 3u);
-            else if (gi < 7u) dst = v_pix_vels + 2 * g + (gi - 5u);
-            else if (gi == 7u) dst = v_opacities + g;
-            else if (gi < 10u && v_means2d_abs != nullptr) dst = v_means2d_abs + 2 * g + (gi - 8u);
-            if ((lane & 1u) == 0u && dst != nullptr) atomicAdd(dst, g_tot);
         }
     }
 }
@@ -904,21 +1074,17 @@ extern "C" int splatad_rasterize_to_pixels_fwd(
                 SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_fwd: null input");
     const uint32_t blocks = C * tile_width * tile_height;
     if (blocks == 0 || image_width == 0 || image_height == 0) return SPLATAD_OK;
-    const uint32_t bs = ((tile_size * tile_size + 31) / 32) * 32;   // whole warps
-    size_t smem = (size_t)bs * (2 * sizeof(float4) + 2 * sizeof(int32_t));
-    // the batch's colour rows ride along in shared memory while a block stays under 64 KB
-    const size_t smem_colors = (size_t)bs * ((channels + 3u) & ~3u) * sizeof(float);
-    const uint32_t stage_colors = (smem + smem_colors <= 64 * 1024) ? 1u : 0u;
-    if (stage_colors) smem += smem_colors;
+    const uint32_t bs = ((tile_threads<2>(tile_size) + 31) / 32) * 32;   // whole warps
 #define CALL(D)                                                                                   \
     {                                                                                             \
+        const size_t smem = (size_t)bs * (2 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float)); \
         int rc = set_smem(rasterize_to_pixels_fwd_kernel<D>, smem, "rasterize_to_pixels_fwd");    \
         if (rc != SPLATAD_OK) return rc;                                                          \
         launch_chained(rasterize_to_pixels_fwd_kernel<D>, blocks, bs, smem, (cudaStream_t)stream, \
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
             image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
-            render_colors, render_alphas, last_ids, stage_colors);                                \
+            render_colors, render_alphas, last_ids);                                              \
     }
     {
         SPL_PROF("rasterize_to_pixels_fwd_kernel", (cudaStream_t)stream);
@@ -949,27 +1115,34 @@ extern "C" int splatad_rasterize_to_pixels_bwd(
                     v_render_alphas && v_means2d && v_conics && v_colors && v_opacities &&
                     v_pix_vels && rolling_shutter_time,
                 SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_bwd: null argument");
-    const uint32_t bs = ((tile_size * tile_size + 31) / 32) * 32;   // whole warps
-    const uint32_t cdim = channels <= 4 ? 4u : channels <= 8 ? 8u : channels <= 16 ? 16u : channels <= 20 ? 20u : 32u;
-    const size_t smem = (size_t)bs * (2 * sizeof(float4) + 2 * sizeof(int32_t) + cdim * sizeof(float));   // rows of CDIM floats
-#define CALL(D)                                                                                   \
+    const uint32_t samples = ((tile_size * tile_size + 31) / 32) * 32;
+    SPL_REQUIRE(samples <= 512 || channels <= 16, SPLATAD_ERR_BAD_ARG,
+                "rasterize_to_pixels_bwd: a tile of %u pixels (%u threads at one per pixel) with %u channels is more "
+                "than the backward pass takes: use a smaller tile or at most 16 channels per call",
+                tile_size * tile_size, samples, channels);
+#define CALL_ABS(D, A)                                                                            \
     {                                                                                             \
-        int rc = check_block_size(rasterize_to_pixels_bwd_kernel<D>, bs, channels, "rasterize_to_pixels_bwd"); \
+        constexpr int kPx = D <= 8 ? 4 : 2;                                                       \
+        auto kernel = rasterize_to_pixels_bwd_kernel<D, kPx, A>;                                  \
+        const uint32_t bs = ((tile_threads<kPx>(tile_size) + 31) / 32) * 32;                      \
+        const size_t smem = (size_t)bs * (2 * sizeof(float4) + 3 * sizeof(int32_t) + D * sizeof(float)); \
+        int rc = set_smem(kernel, smem, "rasterize_to_pixels_bwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
-        rc = set_smem(rasterize_to_pixels_bwd_kernel<D>, smem, "rasterize_to_pixels_bwd");    \
-        if (rc != SPLATAD_OK) return rc;                                                          \
-        rasterize_to_pixels_bwd_kernel<D><<<blocks, bs, smem, (cudaStream_t)stream>>>(            \
+        kernel<<<blocks, bs, smem, (cudaStream_t)stream>>>(                                       \
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
             image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
             render_alphas, last_ids, v_render_colors, v_render_alphas, v_means2d_abs, v_means2d,  \
             v_conics, v_colors, v_opacities, v_pix_vels);                                         \
     }
+#define CALL(D)                                                                                   \
+    if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)
     {
         SPL_PROF("rasterize_to_pixels_bwd_kernel", (cudaStream_t)stream);
         SPL_DISPATCH_CDIM(channels, CALL);
     }
 #undef CALL
+#undef CALL_ABS
     return check_launch("rasterize_to_pixels_bwd");
 }
 
