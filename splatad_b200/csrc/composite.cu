@@ -2,15 +2,12 @@
 // pixels (rasterize_to_pixels) and to lidar points (rasterize_to_points), forward and
 // backward. FP32 on the CUDA cores; there is no dense contraction in this path.
 //
-// One CTA per tile, one thread per pixel / lidar point. A CTA walks its tile's list in
-// batches of blockDim Gaussians staged into shared memory as two float4 (+ extras for lidar),
-// stops as soon as every pixel of the tile is saturated, and a warp whose 32 pixels are all
-// saturated skips the batch body. The backward pass starts at the last list position any
-// pixel of the tile actually consumed instead of the end of the list. The camera forward kernel
-// stages only Gaussians that can reach alpha >= 1/255 somewhere in the tile (an exact, conservative
-// test of the quadratic form over the tile's box of pixel centres, once per tile and Gaussian): the
-// bounding rectangles behind the tile lists are loose, a quarter to a third of their entries never
-// touch a pixel of the tile. The same test did not pay for lidar tiles and is not used there.
+// A CTA walks a tile's list - or, for lidars, its part of a tile's points - in batches staged into shared
+// memory, and stops as soon as every sample is saturated. A warp covers a compact patch of samples, and an
+// entry is staged only if it can reach alpha >= 1/255 somewhere in one of the CTA's patches (an exact,
+// conservative bound of the quadratic form over the patch's box) and looked at only by the warps it
+// can reach: the bounding rectangles behind the tile lists are loose. The backward pass starts at the
+// last list position any of the CTA's samples consumed instead of the end of the list.
 //
 // Semantics follow the reference kernels
 //   pixels fwd  gsplat/cuda/csrc/rasterization.cu:1360-1518     bwd 2833-3089
@@ -163,12 +160,15 @@ __device__ __forceinline__ float2 pair_power(float a, float2 dx, float bdy, floa
 // Camera forward. Bound by instruction issue: two pixels per thread take 50 instructions per entry where
 // one took 40, and a warp passes over the entries that cannot reach its 8 x 8 patch without looking at
 // them. A pixel that has stopped moves its column out to where every alpha vanishes, which costs the
-// other pixels nothing; a warp leaves when all of its pixels have. Camera benchmark frame: 0.326 -> 0.xxx ms.
+// other pixels nothing; a warp leaves when all of its pixels have. Camera benchmark frame: 0.338 -> 0.248 ms.
 // ---------------------------------------------------------------------------------------
 constexpr float kPixelGone = 1e18f;   // a column no Gaussian reaches: sigma overflows, alpha is 0 (or NaN, never drawn)
 
+// registers per thread: as many CTAs of 128 threads per SM as the accumulators leave room for
+constexpr int pixels_fwd_regs(int cdim) { return cdim <= 8 ? 64 : cdim <= 16 ? 80 : cdim <= 20 ? 96 : 128; }
+
 template <int CDIM>
-__global__ void __launch_bounds__(512) rasterize_to_pixels_fwd_kernel(
+__global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
     const float *__restrict__ opacities, const float2 *__restrict__ pix_vels,
@@ -318,40 +318,180 @@ __global__ void __launch_bounds__(512) rasterize_to_pixels_fwd_kernel(
 }
 
 // ---------------------------------------------------------------------------------------
-// Lidar forward
+// Lidar tiles. The points of a tile are cut into patches of one warp each - 8 columns x 4 beams of the
+// usual 32 x 8 tile - and the warps of a tile are spread over several small CTAs: tiles differ widely in
+// how many entries saturate them (41 on average in the lidar benchmark, several hundred at worst), and
+// a scan of 64 tiles does not fill the machine with one CTA per tile.
 // ---------------------------------------------------------------------------------------
+struct PointPatch {
+    uint32_t col, row;     // first point of the thread within the tile
+    bool patched;          // patches are kPatchW columns wide, else points in row-major order
+};
+
+constexpr uint32_t kPatchW = 8;
+
+// Thread `index` of the tile's threads (PX points in one beam or, in row-major order, PX in sequence).
+template <int PX>
+__device__ __forceinline__ PointPatch point_patch(uint32_t tile_width, uint32_t tile_height, uint32_t index) {
+    constexpr uint32_t kPatchH = 32 * PX / kPatchW;
+    PointPatch p;
+    p.patched = tile_width % kPatchW == 0u && tile_height % kPatchH == 0u;
+    if (p.patched) {
+        const uint32_t patch = index >> 5, lane = index & 31u, per_row = tile_width / kPatchW;
+        p.col = (patch % per_row) * kPatchW + (lane * PX) % kPatchW;
+        p.row = (patch / per_row) * kPatchH + (lane * PX) / kPatchW;
+    } else {
+        p.row = index * PX / tile_width;   // the first of PX points in sequence
+        p.col = index * PX - p.row * tile_width;
+    }
+    return p;
+}
+
+// Azimuths, elevations (as centre and half width) and time offsets of a warp's points.
+struct PointBox { float az, az_half, el, el_half, roll_lo, roll_hi; };
+
+struct PointExtent {
+    float az0 = 3.0e38f, az1 = -3.0e38f, el0 = 3.0e38f, el1 = -3.0e38f, r0 = 3.0e38f, r1 = -3.0e38f;
+    __device__ __forceinline__ void add(float az, float el, float roll) {
+        az0 = fminf(az0, az); az1 = fmaxf(az1, az);
+        el0 = fminf(el0, el); el1 = fmaxf(el1, el);
+        r0 = fminf(r0, roll); r1 = fmaxf(r1, roll);
+    }
+    // the box of the whole warp, written by its first lane; no points: a negative half width
+    __device__ __forceinline__ void write_box(PointBox *box) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            az0 = fminf(az0, __shfl_xor_sync(0xffffffffu, az0, off)); az1 = fmaxf(az1, __shfl_xor_sync(0xffffffffu, az1, off));
+            el0 = fminf(el0, __shfl_xor_sync(0xffffffffu, el0, off)); el1 = fmaxf(el1, __shfl_xor_sync(0xffffffffu, el1, off));
+            r0 = fminf(r0, __shfl_xor_sync(0xffffffffu, r0, off)); r1 = fmaxf(r1, __shfl_xor_sync(0xffffffffu, r1, off));
+        }
+        if ((threadIdx.x & 31u) == 0u)
+            *box = {0.5f * (az0 + az1), 0.5f * (az1 - az0), 0.5f * (el0 + el1), 0.5f * (el1 - el0), r0, r1};
+    }
+};
+
+struct PointEntry {
+    float4 A, B;      // azimuth, elevation, their velocities | conic, opacity
+    float4 C;         // range velocity, depth compensation (2), range
+};
+
+__device__ __forceinline__ PointEntry load_point_entry(int32_t g, const float2 *__restrict__ means2d,
+                                                       const float *__restrict__ conics,
+                                                       const float *__restrict__ opacities,
+                                                       const float *__restrict__ pix_vels,
+                                                       const float2 *__restrict__ depth_comps) {
+    PointEntry e;
+    const float2 xy = __ldg(means2d + g), dc = __ldg(depth_comps + g);
+    const float *v = pix_vels + 3 * (size_t)g, *q = conics + 3 * (size_t)g;
+    e.A = make_float4(xy.x, xy.y, __ldg(v), __ldg(v + 1));
+    e.B = make_float4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(opacities + g));
+    e.C = make_float4(__ldg(v + 2), dc.x, dc.y, 0.f);
+    return e;
+}
+
+// Offsets of a moving mean from the points of a box, [lo, hi]: a range that reaches across half a turn
+// is the whole turn. The slack of a millidegree covers the rounding of the wrapped differences.
+__device__ __forceinline__ void angle_range(float mean, float vel, float centre, float half, float roll_lo, float roll_hi,
+                                            float &lo, float &hi) {
+    const float a = roll_lo * vel, b = roll_hi * vel;
+    const float d = angle_difference(mean + 0.5f * (a + b), centre);
+    const float reach = half + 0.5f * fabsf(b - a) + 1e-3f;
+    lo = d - reach;
+    hi = d + reach;
+    if (lo < -180.f || hi > 180.f) { lo = -180.f; hi = 180.f; }
+}
+
+// Bit w: the entry may contribute to a point of box w.
+__device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const PointBox *s_box, uint32_t n_boxes) {
+    const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
+    if (test.never) return 0u;
+    uint32_t seen = 0u;
+    for (uint32_t w = 0; w < n_boxes; ++w) {
+        const PointBox b = s_box[w];
+        if (!(b.az_half >= 0.f)) continue;
+        float x_lo, x_hi, y_lo, y_hi;
+        angle_range(e.A.x, e.A.z, b.az, b.az_half, b.roll_lo, b.roll_hi, x_lo, x_hi);
+        angle_range(e.A.y, e.A.w, b.el, b.el_half, b.roll_lo, b.roll_hi, y_lo, y_hi);
+        if (!test.misses(x_lo, x_hi, y_lo, y_hi)) seen |= 1u << w;
+    }
+    return seen;
+}
+
+// Offset of an entry from a point and its exp(-sigma); sigma decides with alpha whether it is blended.
+struct PointFootprint { float dx, dy, sigma, vis; };
+
+__device__ __forceinline__ PointFootprint point_footprint(const float4 &A, const float4 &B, float roll, float az, float el) {
+    PointFootprint f;
+    f.dx = angle_difference(A.x + roll * A.z, az);
+    f.dy = angle_difference(A.y + roll * A.w, el);
+    f.sigma = 0.5f * (B.x * f.dx * f.dx + B.z * f.dy * f.dy) + B.y * f.dx * f.dy;
+    f.vis = __expf(-f.sigma);
+    return f;
+}
+
+// Copies the feature row of entry g, the range behind it when it comes from its own array, then zeros.
 template <int CDIM>
-__global__ void __launch_bounds__(1024) rasterize_to_points_fwd_kernel(
+__device__ __forceinline__ void stage_features(float *row, const float *__restrict__ colors, size_t g, uint32_t fstride,
+                                               bool vec, bool has_range, float range) {
+    uint32_t filled = 0;
+    if (fstride) {
+        stage_row(row, colors, g, fstride, vec);
+        filled = (fstride + 3u) & ~3u;
+    }
+    if (has_range) {
+        row[fstride] = range;
+        filled = max(filled, fstride + 1u);
+    }
+    for (uint32_t k = filled; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
+}
+
+// ---------------------------------------------------------------------------------------
+// Lidar forward. One point per lane; a warp looks only at the entries that can reach its patch (a ninth
+// of the (point, entry) pairs of a small scan contribute, two thirds of the benchmark's) and evaluates
+// two of them at a time, because what it waits for is the chain from the offsets through the exponential
+// to the transmittance. The rendered rows leave through shared memory: a beam's eight points
+// are consecutive floats.
+// ---------------------------------------------------------------------------------------
+// entries per thread and batch (their loads overlap), while the shared memory of a batch stays small
+constexpr uint32_t points_fwd_stage(int cdim) { return cdim <= 8 ? 2 : 1; }
+constexpr int points_fwd_regs(int cdim) { return cdim <= 20 ? 96 : 112; }
+
+template <int CDIM>
+__global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors,
     const float *__restrict__ ranges /* optional: last channel comes from here */, uint32_t channels,
     const float *__restrict__ opacities, const float *__restrict__ pix_vels /* [.,3] */,
     const float2 *__restrict__ depth_comps, const float *__restrict__ backgrounds,
     const float4 *__restrict__ raster_pts, uint32_t W, uint32_t H, uint32_t tile_width,
-    uint32_t tile_height, uint32_t grid_w, uint32_t grid_h, int compute_alpha_sum,
+    uint32_t tile_height, uint32_t grid_w, uint32_t grid_h, uint32_t ctas_per_tile, int compute_alpha_sum,
     float alpha_sum_threshold, const int32_t *__restrict__ offsets,
     const int32_t *__restrict__ flatten_ids, uint32_t depth_idx,
     float *__restrict__ render_colors, float *__restrict__ render_alphas,
     float *__restrict__ alpha_sum_out, int32_t *__restrict__ last_ids,
-    float *__restrict__ median_depths, uint32_t stage_features) {
-    chain_enter();
+    float *__restrict__ median_depths) {
+    constexpr uint32_t kStage = points_fwd_stage(CDIM);
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const uint32_t bs = blockDim.x;
-    float4 *sA = reinterpret_cast<float4 *>(smem_raw);   // az, el, v_az, v_el
-    float4 *sB = sA + bs;                                // conic a, b, c, opacity
-    float4 *sC = sB + bs;                                // v_range, dc.x, dc.y, range (depth channel)
-    int32_t *sId = reinterpret_cast<int32_t *>(sC + bs);
-    // feature rows of the batch (when they fit): the inner loop then never waits on global memory
-    float *sFeat = reinterpret_cast<float *>(sId + bs);
+    __shared__ PointBox s_box[8];
+    __shared__ uint32_t s_warp_kept[kStage * 8];
+    const uint32_t bs = blockDim.x, cap = kStage * bs;
+    float4 *sA = reinterpret_cast<float4 *>(smem_raw);
+    float4 *sB = sA + cap;
+    float4 *sC = sB + cap;
+    float *sFeat = reinterpret_cast<float *>(sC + cap);                 // [cap * CDIM]
+    int32_t *sPos = reinterpret_cast<int32_t *>(sFeat + cap * CDIM);    // list position
+    uint32_t *sSeen = reinterpret_cast<uint32_t *>(sPos + cap);         // warps that may see it
 
     const uint32_t tiles_per_cam = grid_w * grid_h;
-    const uint32_t cam = blockIdx.x / tiles_per_cam;
-    const uint32_t tile = blockIdx.x - cam * tiles_per_cam;
+    const uint32_t gtile = blockIdx.x / ctas_per_tile, part = blockIdx.x - gtile * ctas_per_tile;
+    const uint32_t cam = gtile / tiles_per_cam;
+    const uint32_t tile = gtile - cam * tiles_per_cam;
     const uint32_t ty = tile / grid_w, tx = tile - ty * grid_w;
-    const uint32_t tr = threadIdx.x;
-    const uint32_t i = ty * tile_height + tr / tile_width;
-    const uint32_t j = tx * tile_width + tr % tile_width;
-    const bool in_image = (tr < tile_width * tile_height) && (i < H && j < W);
+    const uint32_t tr = threadIdx.x, lane = tr & 31u, warp = tr >> 5, n_warps = bs >> 5;
+    const uint32_t index = part * bs + tr;
+    const PointPatch pp = point_patch<1>(tile_width, tile_height, index);
+    const uint32_t i = ty * tile_height + pp.row, j = tx * tile_width + pp.col;
+    const bool in_image = index < tile_width * tile_height && i < H && j < W;
     bool inside = in_image;
     const size_t pix = ((size_t)cam * H + i) * W + j;
     float px = 0.f, py = 0.f, pz = 0.f, roll = 0.f;
@@ -360,102 +500,145 @@ __global__ void __launch_bounds__(1024) rasterize_to_points_fwd_kernel(
         px = rp.x; py = rp.y; pz = rp.z; roll = rp.w;
         if (pz <= 0.f) inside = false;
     }
+    PointExtent extent;
+    if (inside) extent.add(px, py, roll);
+    extent.write_box(s_box + warp);
+    // the points are an input of the frame; everything below comes from the kernels before this one
+    chain_enter();
 
-    const TileRange range = tile_range(offsets, blockIdx.x, C * tiles_per_cam, n_isects);
-    const uint32_t num_batches = (uint32_t)(range.end - range.start + bs - 1) / bs;
+    const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
+    const uint32_t num_batches = (uint32_t)(range.end - range.start + cap - 1) / cap;
 
-    // with a separate range array the feature rows hold channels - 1 columns
+    // with a separate range array the feature rows hold channels - 1 columns; a staged row holds all CDIM
+    // accumulated channels: the features, behind them the range when it comes from its own array, then
+    // zeros, so that one unconditional multiply-add pass covers them
     const uint32_t fstride = ranges ? channels - 1 : channels;
-    // a staged row holds all CDIM accumulated channels: the features, behind them the range when it
-    // comes from its own array, then zeros, so that one unconditional multiply-add pass covers them
-    constexpr uint32_t fpad = (uint32_t)CDIM;
     const bool vec = (fstride % 4u == 0u) && ((reinterpret_cast<uintptr_t>(colors) & 15u) == 0u);
     bool done = !inside;
+    bool warp_done = __all_sync(0xffffffffu, done);
     float T = 1.f;
-    uint32_t cur_idx = 0;
+    int32_t cur_idx = 0;
     float depth_extra = 0.f, alpha_sum = 0.f, median = 0.f;
+    const float alpha_sum_limit = pz - alpha_sum_threshold;
     float pix_out[CDIM];
 #pragma unroll
     for (int k = 0; k < CDIM; ++k) pix_out[k] = 0.f;
 
+    int32_t next_id[kStage];
+#pragma unroll
+    for (uint32_t q = 0; q < kStage; ++q) {
+        const int32_t idx = range.start + (int32_t)(q * bs + tr);
+        next_id[q] = idx < range.end ? flatten_ids[idx] : 0;
+    }
     for (uint32_t b = 0; b < num_batches; ++b) {
-        if (__syncthreads_count(done) >= (int)bs) break;
-        const uint32_t batch_start = (uint32_t)range.start + bs * b;
-        const uint32_t idx = batch_start + tr;
-        if (idx < (uint32_t)range.end) {
-            const int32_t g = flatten_ids[idx];
-            const float2 xy = means2d[g];
-            const float *v = pix_vels + 3 * (size_t)g;
-            const float2 dc = depth_comps[g];
-            sA[tr] = make_float4(xy.x, xy.y, v[0], v[1]);
-            sB[tr] = make_float4(conics[3 * (size_t)g], conics[3 * (size_t)g + 1],
-                                 conics[3 * (size_t)g + 2], opacities[g]);
-            const float range = ranges ? ranges[g] : colors[(size_t)g * channels + depth_idx];
-            sC[tr] = make_float4(v[2], dc.x, dc.y, range);
-            sId[tr] = g;
-            if (stage_features) {
-                float *row = sFeat + tr * fpad;
-                uint32_t filled = 0;
-                if (fstride) {
-                    stage_row(row, colors, (size_t)g, fstride, vec);
-                    filled = (fstride + 3u) & ~3u;
-                }
-                if (ranges) {
-                    row[fstride] = range;
-                    filled = max(filled, fstride + 1u);
-                }
-                for (uint32_t k = filled; k < fpad; ++k) row[k] = 0.f;
-            }
+        if (__syncthreads_and(warp_done)) break;
+        const int32_t batch_start = range.start + (int32_t)(cap * b);
+        PointEntry e[kStage];
+        int32_t g[kStage];
+        uint32_t seen[kStage], kept[kStage];
+#pragma unroll
+        for (uint32_t q = 0; q < kStage; ++q) {
+            g[q] = next_id[q];
+            const int32_t idx = batch_start + (int32_t)(q * bs + tr);
+            if (idx < range.end) e[q] = load_point_entry(g[q], means2d, conics, opacities, pix_vels, depth_comps);
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kStage; ++q) {
+            const int32_t idx = batch_start + (int32_t)(q * bs + tr);
+            if (idx < range.end) e[q].C.w = ranges ? __ldg(ranges + g[q]) : __ldg(colors + (size_t)g[q] * channels + depth_idx);
+            if (idx + (int32_t)cap < range.end) next_id[q] = flatten_ids[idx + cap];   // on its way meanwhile
+        }
+        // compact the survivors to the front of the staging arrays, list order kept
+#pragma unroll
+        for (uint32_t q = 0; q < kStage; ++q) {
+            seen[q] = batch_start + (int32_t)(q * bs + tr) < range.end ? boxes_that_see(e[q], s_box, n_warps) : 0u;
+            kept[q] = __ballot_sync(0xffffffffu, seen[q] != 0u);
+            if (lane == 0) s_warp_kept[q * n_warps + warp] = __popc(kept[q]);
         }
         __syncthreads();
-        if (__all_sync(0xffffffffu, done)) continue;
-        const uint32_t batch_size = min(bs, (uint32_t)range.end - batch_start);
-        for (uint32_t t = 0; t < batch_size && !done; ++t) {
-            const float4 A = sA[t];
-            const float4 B = sB[t];
-            const float dx = angle_difference(A.x + roll * A.z, px);
-            const float dy = angle_difference(A.y + roll * A.w, py);
-            const float sigma = 0.5f * (B.x * dx * dx + B.z * dy * dy) + B.y * dx * dy;
-            const float alpha = fminf(kAlphaMax, B.w * __expf(-sigma));
-            if (sigma < 0.f || alpha < kAlphaMin) continue;
+        uint32_t n_kept = 0, pos[kStage];
+#pragma unroll
+        for (uint32_t q = 0; q < kStage; ++q) {
+            pos[q] = __popc(kept[q] & ((1u << lane) - 1u));
+            for (uint32_t w = 0; w < n_warps; ++w) {
+                if (w == warp) pos[q] += n_kept;
+                n_kept += s_warp_kept[q * n_warps + w];
+            }
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kStage; ++q)
+            if (seen[q]) {
+                sA[pos[q]] = e[q].A;
+                sB[pos[q]] = e[q].B;
+                sC[pos[q]] = e[q].C;
+                sPos[pos[q]] = batch_start + (int32_t)(q * bs + tr);
+                sSeen[pos[q]] = seen[q];
+                stage_features<CDIM>(sFeat + pos[q] * CDIM, colors, (size_t)g[q], fstride, vec, ranges != nullptr, e[q].C.w);
+            }
+        __syncthreads();
+        if (warp_done) continue;
+        const auto blend = [&](uint32_t t, const PointFootprint &f, float alpha) {
             const float next_T = T * (1.f - alpha);
-            if (next_T <= kTStop) { done = true; break; }
+            if (next_T <= kTStop) { done = true; return; }
             const float vis = alpha * T;
             const float4 Cc = sC[t];
-            if (stage_features) {
-                // the zero padding of a staged row adds nothing to the channels behind it
-                axpy_staged_full<CDIM>(pix_out, sFeat + t * fpad, vis);
-            } else {
-                const float *c_ptr = colors + (size_t)sId[t] * fstride;
-#pragma unroll
-                for (int k = 0; k < CDIM; ++k) {
-                    if ((uint32_t)k < fstride) pix_out[k] += __ldg(c_ptr + k) * vis;
-                    else if ((uint32_t)k < channels) pix_out[k] += Cc.w * vis;
-                }
-            }
-            const float dterm = Cc.y * dx + Cc.z * dy + Cc.x * roll;
+            axpy_staged_full<CDIM>(pix_out, sFeat + t * CDIM, vis);   // the zero padding adds nothing
+            const float dterm = Cc.y * f.dx + Cc.z * f.dy + Cc.x * roll;
             depth_extra += dterm * vis;
             if (T > 0.5f && next_T <= 0.5f) median = Cc.w + dterm;
-            if (compute_alpha_sum && Cc.w < (pz - alpha_sum_threshold)) alpha_sum += alpha;
-            cur_idx = batch_start + t;
+            if (compute_alpha_sum && Cc.w < alpha_sum_limit) alpha_sum += alpha;
+            cur_idx = sPos[t];
             T = next_T;
+        };
+        for (uint32_t t0 = 0; t0 < n_kept && !warp_done; t0 += 32) {
+            const uint32_t mine = t0 + lane;
+            uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u));
+            while (todo && !(warp_done = __all_sync(0xffffffffu, done))) {
+                // two entries at a time; an odd one out is evaluated twice and blended once
+                const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
+                todo &= todo - 1u;
+                const bool two = todo != 0u;
+                const uint32_t u = two ? t0 + (uint32_t)__ffs(todo) - 1u : t;
+                todo &= todo - 1u;   // of 0: stays 0
+                const float4 A0 = sA[t], B0 = sB[t], A1 = sA[u], B1 = sB[u];
+                const PointFootprint f0 = point_footprint(A0, B0, roll, px, py), f1 = point_footprint(A1, B1, roll, px, py);
+                const float alpha0 = fminf(kAlphaMax, B0.w * f0.vis), alpha1 = fminf(kAlphaMax, B1.w * f1.vis);
+                const bool ok0 = !(f0.sigma < 0.f || alpha0 < kAlphaMin), ok1 = two && !(f1.sigma < 0.f || alpha1 < kAlphaMin);
+                if (ok0 && !done) blend(t, f0, alpha0);
+                if (ok1 && !done) blend(u, f1, alpha1);
+            }
+            warp_done = __all_sync(0xffffffffu, done);
         }
     }
-    if (in_image) {
-        // points that are not rendered (range <= 0) produce zeros everywhere
-        render_alphas[pix] = inside ? 1.f - T : 0.f;
-        const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
+    // points that are not rendered (range <= 0) produce zeros everywhere
+    const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
+    __syncthreads();   // the rendered rows take the place of the feature rows
+    float *rows = sFeat + warp * 32u * CDIM;
 #pragma unroll
-        for (int k = 0; k < CDIM; ++k)
-            if ((uint32_t)k < channels) {
-                float v = pix_out[k];
-                if ((uint32_t)k == depth_idx) v += depth_extra;
-                if (bg) v += T * bg[k];
-                render_colors[pix * channels + k] = inside ? v : 0.f;
-            }
-        last_ids[pix] = inside ? (int32_t)cur_idx : 0;
+    for (int k = 0; k < CDIM; ++k)
+        if ((uint32_t)k < channels) {
+            float v = pix_out[k];
+            if ((uint32_t)k == depth_idx) v += depth_extra;
+            if (bg) v += T * bg[k];
+            v = inside ? v : 0.f;
+            if (pp.patched) rows[lane * channels + k] = v;
+            else if (in_image) render_colors[pix * channels + k] = v;
+        }
+    if (in_image) {
+        render_alphas[pix] = inside ? 1.f - T : 0.f;
+        last_ids[pix] = inside ? cur_idx : 0;
         median_depths[pix] = inside ? median : 0.f;
         if (alpha_sum_out != nullptr) alpha_sum_out[pix] = inside ? alpha_sum : 0.f;
+    }
+    if (!pp.patched) return;
+    __syncwarp();
+    const uint32_t i0 = __shfl_sync(0xffffffffu, i, 0), j0 = __shfl_sync(0xffffffffu, j, 0);
+    const bool any = __shfl_sync(0xffffffffu, (int)(index < tile_width * tile_height), 0);
+    const uint32_t n = any && j0 < W ? min(kPatchW, W - j0) * channels : 0u;
+    for (uint32_t r = 0; r < 32u / kPatchW && i0 + r < H; ++r) {
+        float *dst = render_colors + (((size_t)cam * H + i0 + r) * W + j0) * channels;
+        const float *src = rows + r * kPatchW * channels;
+        for (uint32_t k = lane; k < n; k += 32u) dst[k] = src[k];
     }
 }
 
@@ -549,7 +732,7 @@ __device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t
 // the sums of v, v dx and v dx^2 (v = exp(-sigma) dL/dalpha). The channels behind an entry enter through
 // one number per pixel: dL/dalpha = T (c . g) - (1 / (1 - alpha)) (sum over the entries behind of
 // their weight times their (c . g)), g the pixel's cotangent - a running scalar in place of a running colour.
-// Camera benchmark frame, training step: 1.50 -> 0.5x ms.
+// Camera benchmark's training step: 1.55 -> 0.50 ms.
 // ---------------------------------------------------------------------------------------
 template <int CDIM, int PX, bool kAbs>
 __global__ void __launch_bounds__(PX == 4 || CDIM > 16 ? 256 : 512)
@@ -790,17 +973,45 @@ rasterize_to_pixels_bwd_kernel(
 }
 
 // ---------------------------------------------------------------------------------------
-// Lidar backward
+// Lidar backward: as the camera's, with two points per thread. Every point has its own elevation and time
+// offset, so each term is formed per point - in pairs - before the sum over the thread's points goes into
+// the warp totals. `behind` also carries the depth compensation of the range channel.
 // ---------------------------------------------------------------------------------------
-template <int CDIM>
-__global__ void rasterize_to_points_bwd_kernel(
+template <bool kAbs>
+__device__ __forceinline__ GradSlot point_grad_slot(int slot, int cdim, uint32_t channels, uint32_t fstride, float *v_colors,
+                                                    float *v_ranges, float *v_conics, float *v_means2d, float *v_pix_vels,
+                                                    float *v_depth_comps, float *v_opacities, float *v_means2d_abs) {
+    if (slot < cdim) {
+        if ((uint32_t)slot < fstride) return {v_colors + slot, fstride, 1.f, false};
+        return {(uint32_t)slot < channels ? v_ranges : nullptr, 1u, 1.f, false};
+    }
+    switch (slot - cdim) {
+        case 0: return {v_conics, 3u, 0.5f, false};
+        case 1: return {v_conics + 1, 3u, 1.f, false};
+        case 2: return {v_conics + 2, 3u, 0.5f, false};
+        case 3: return {v_means2d, 2u, 1.f, false};
+        case 4: return {v_means2d + 1, 2u, 1.f, false};
+        case 5: return {v_pix_vels, 3u, 1.f, false};
+        case 6: return {v_pix_vels + 1, 3u, 1.f, false};
+        case 7: return {v_pix_vels + 2, 3u, 1.f, false};
+        case 8: return {v_depth_comps, 2u, 1.f, false};
+        case 9: return {v_depth_comps + 1, 2u, 1.f, false};
+        case 10: return {v_opacities, 1u, 1.f, false};
+        case 11: return {kAbs ? v_means2d_abs : nullptr, 2u, 1.f, false};
+        case 12: return {kAbs ? v_means2d_abs + 1 : nullptr, 2u, 1.f, false};
+        default: return {nullptr, 0u, 0.f, false};
+    }
+}
+
+template <int CDIM, bool kAbs>
+__global__ void __launch_bounds__(256) rasterize_to_points_bwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors,
     const float *__restrict__ ranges, uint32_t channels,
     const float *__restrict__ opacities, const float *__restrict__ pix_vels,
     const float2 *__restrict__ depth_comps, const float *__restrict__ backgrounds,
     const float4 *__restrict__ raster_pts, uint32_t W, uint32_t H, uint32_t tile_width,
-    uint32_t tile_height, uint32_t grid_w, uint32_t grid_h, int compute_alpha_sum,
+    uint32_t tile_height, uint32_t grid_w, uint32_t grid_h, uint32_t ctas_per_tile, int compute_alpha_sum,
     float alpha_sum_threshold, const int32_t *__restrict__ offsets,
     const int32_t *__restrict__ flatten_ids, uint32_t depth_idx,
     const float *__restrict__ render_alphas, const int32_t *__restrict__ last_ids,
@@ -811,203 +1022,219 @@ __global__ void rasterize_to_points_bwd_kernel(
     float *__restrict__ v_depth_comps, float *__restrict__ v_ranges) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int red[32];
+    __shared__ PointBox s_box[8];
+    __shared__ uint32_t s_warp_kept[8];
     const uint32_t bs = blockDim.x;
     float4 *sA = reinterpret_cast<float4 *>(smem_raw);
     float4 *sB = sA + bs;
-    float4 *sC = sB + bs;   // v_range, dc.x, dc.y, unused
-    int32_t *sId = reinterpret_cast<int32_t *>(sC + bs);
-    float *sRgb = reinterpret_cast<float *>(sId + bs);
+    float4 *sC = sB + bs;   // range velocity, depth compensation (2), range
+    float *sRgb = reinterpret_cast<float *>(sC + bs);                  // [bs * CDIM], zeros behind the channels
+    int32_t *sId = reinterpret_cast<int32_t *>(sRgb + bs * CDIM);
+    int32_t *sPos = sId + bs;
+    uint32_t *sSeen = reinterpret_cast<uint32_t *>(sPos + bs);
 
     const uint32_t tiles_per_cam = grid_w * grid_h;
-    const uint32_t cam = blockIdx.x / tiles_per_cam;
-    const uint32_t tile = blockIdx.x - cam * tiles_per_cam;
+    const uint32_t gtile = blockIdx.x / ctas_per_tile, part = blockIdx.x - gtile * ctas_per_tile;
+    const uint32_t cam = gtile / tiles_per_cam;
+    const uint32_t tile = gtile - cam * tiles_per_cam;
     const uint32_t ty = tile / grid_w, tx = tile - ty * grid_w;
-    const uint32_t tr = threadIdx.x;
-    const uint32_t i = ty * tile_height + tr / tile_width;
-    const uint32_t j = tx * tile_width + tr % tile_width;
-    bool inside = (tr < tile_width * tile_height) && (i < H && j < W);
-    const size_t pix = ((size_t)cam * H + min(i, H - 1)) * W + min(j, W - 1);
-    float px = 0.f, py = 0.f, pz = 0.f, roll = 0.f;
-    if (inside) {
-        const float4 rp = raster_pts[pix];
-        px = rp.x; py = rp.y; pz = rp.z; roll = rp.w;
-        if (pz <= 0.f) inside = false;
-    }
+    const uint32_t tr = threadIdx.x, lane = tr & 31u, warp = tr >> 5, n_warps = bs >> 5;
+    const uint32_t index = part * bs + tr;
+    const PointPatch pp = point_patch<2>(tile_width, tile_height, index);
 
-    const TileRange range = tile_range(offsets, blockIdx.x, C * tiles_per_cam, n_isects);
-
+    const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
     const uint32_t fstride = ranges ? channels - 1 : channels;
     const bool vec = (fstride % 4u == 0u) && ((reinterpret_cast<uintptr_t>(colors) & 15u) == 0u);
-    const float T_final = 1.f - render_alphas[pix];
-    float T = T_final;
-    const int32_t bin_final = inside ? last_ids[pix] : 0;
-    float buffer[CDIM], v_render_c[CDIM];
-    float buffer_extra = 0.f;   // depth-compensation part of the depth channel's buffer
-    float bg_dot = 0.f, v_depth_c = 0.f;
-#pragma unroll
-    for (int k = 0; k < CDIM; ++k) {
-        buffer[k] = 0.f;
-        v_render_c[k] = ((uint32_t)k < channels && inside) ? v_render_colors[pix * channels + k] : 0.f;
-        if ((uint32_t)k == depth_idx) v_depth_c = v_render_c[k];
-        if (backgrounds != nullptr && (uint32_t)k < channels)
-            bg_dot += backgrounds[(size_t)cam * channels + k] * v_render_c[k];
-    }
-    const float v_render_a = inside ? v_render_alphas[pix] : 0.f;
-    const float v_asum = (inside && v_alpha_sum != nullptr) ? v_alpha_sum[pix] : 0.f;
 
-    const int32_t tile_last = block_max_int(bin_final, red);
-    int32_t warp_bin_final = bin_final;
+    float2 az, el, roll, T, behind, v_depth, v_asum, sum_limit;
+    float v_out[2][CDIM];
+    int32_t bin_final[2], thread_last = -1;
+    PointExtent extent;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-        warp_bin_final = max(warp_bin_final, __shfl_xor_sync(0xffffffffu, warp_bin_final, off));
-    const int32_t eff_end = min(range.end, tile_last + 1);
+    for (int h = 0; h < 2; ++h) {
+        // the second point follows the first in its beam, or in the tile's row-major order
+        uint32_t row = pp.row, col = pp.col + h;
+        if (col >= tile_width) { col -= tile_width; ++row; }
+        const uint32_t i = ty * tile_height + row, j = tx * tile_width + col;
+        bool in = row < tile_height && i < H && j < W;
+        const size_t pix = in ? ((size_t)cam * H + i) * W + j : 0u;
+        float4 rp = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (in) {
+            rp = raster_pts[pix];
+            if (rp.z <= 0.f) in = false;
+        }
+        if (in) extent.add(rp.x, rp.y, rp.w);
+        const float T_final = in ? 1.f - render_alphas[pix] : 1.f;
+        bin_final[h] = in ? last_ids[pix] : -1;
+        thread_last = max(thread_last, bin_final[h]);
+        float bg_dot = 0.f, vd = 0.f;
+#pragma unroll
+        for (int c = 0; c < CDIM; ++c) {
+            v_out[h][c] = (in && (uint32_t)c < channels) ? v_render_colors[pix * channels + c] : 0.f;
+            if ((uint32_t)c == depth_idx) vd = v_out[h][c];
+            if (backgrounds != nullptr && (uint32_t)c < channels)
+                bg_dot += backgrounds[(size_t)cam * channels + c] * v_out[h][c];
+        }
+        const float va = in ? v_render_alphas[pix] : 0.f;
+        const float vs = (in && compute_alpha_sum && v_alpha_sum != nullptr) ? v_alpha_sum[pix] : 0.f;
+        // what the background and the alpha output receive through everything in front of them
+        const float last = -T_final * (va - bg_dot);
+        const float limit = rp.z - alpha_sum_threshold;
+        if (h) { az.y = rp.x; el.y = rp.y; roll.y = rp.w; T.y = T_final; behind.y = last; v_depth.y = vd; v_asum.y = vs; sum_limit.y = limit; }
+        else { az.x = rp.x; el.x = rp.y; roll.x = rp.w; T.x = T_final; behind.x = last; v_depth.x = vd; v_asum.x = vs; sum_limit.x = limit; }
+    }
+    extent.write_box(s_box + warp);
+
+    // last list position consumed by any point of this CTA / warp
+    const int32_t cta_last = block_max_int(thread_last, red);
+    const int32_t warp_last = __reduce_max_sync(0xffffffffu, thread_last);
+    const int32_t eff_end = min(range.end, cta_last + 1);
     if (eff_end <= range.start) return;
     const uint32_t num_batches = (uint32_t)(eff_end - range.start + bs - 1) / bs;
-    const uint32_t lane = tr & 31;
 
+    constexpr int kGeo = kAbs ? 13 : 11;
+    constexpr int kSlots = CDIM + kGeo <= 16 ? 16 : 32;
+    constexpr bool kSplit = CDIM + kGeo > 32;   // the geometry in a butterfly of its own
+    const GradSlot slot_a = point_grad_slot<kAbs>(kSplit ? (int)lane : (int)(lane * kSlots / 32u), CDIM, channels, fstride,
+                                                  v_colors, v_ranges, v_conics, v_means2d, v_pix_vels, v_depth_comps,
+                                                  v_opacities, v_means2d_abs);
+    const bool writes_a = kSlots == 32 || (lane & 1u) == 0u;
+
+    int32_t next_id = 0;
+    {
+        const int32_t idx = eff_end - 1 - (int32_t)tr;
+        if (idx >= range.start) next_id = flatten_ids[idx];
+    }
     for (uint32_t b = 0; b < num_batches; ++b) {
-        __syncthreads();
-        const int32_t batch_end = eff_end - 1 - (int32_t)(bs * b);
-        const int32_t batch_size = min((int32_t)bs, batch_end + 1 - range.start);
-        const int32_t idx = batch_end - (int32_t)tr;
+        const int32_t idx = eff_end - 1 - (int32_t)(bs * b) - (int32_t)tr;
+        const int32_t g = next_id;
+        PointEntry e;
+        uint32_t seen = 0u;
         if (idx >= range.start) {
-            const int32_t g = flatten_ids[idx];
-            const float2 xy = means2d[g];
-            const float *v = pix_vels + 3 * (size_t)g;
-            const float2 dc = depth_comps[g];
-            sA[tr] = make_float4(xy.x, xy.y, v[0], v[1]);
-            sB[tr] = make_float4(conics[3 * (size_t)g], conics[3 * (size_t)g + 1],
-                                 conics[3 * (size_t)g + 2], opacities[g]);
-            sC[tr] = make_float4(v[2], dc.x, dc.y, 0.f);
-            sId[tr] = g;
-            // rows of CDIM floats: the channels, then zeros, so that the channel loops below run in
-            // packed pairs without tests
-            float *row = sRgb + tr * CDIM;
-            uint32_t filled = 0;
-            if (fstride) {
-                stage_row(row, colors, (size_t)g, fstride, vec);
-                filled = (fstride + 3u) & ~3u;
-            }
-            if (ranges) {
-                row[fstride] = ranges[g];
-                filled = max(filled, fstride + 1u);
-            }
-            for (uint32_t k = filled; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
+            e = load_point_entry(g, means2d, conics, opacities, pix_vels, depth_comps);
+            e.C.w = ranges ? __ldg(ranges + g) : __ldg(colors + (size_t)g * channels + depth_idx);
+            const int32_t ahead = idx - (int32_t)bs;   // the id of the next batch's entry is on its way meanwhile
+            if (ahead >= range.start) next_id = flatten_ids[ahead];
+            seen = boxes_that_see(e, s_box, n_warps);
+        }
+        // survivors to the front, still back to front in list order
+        const uint32_t kept_mask = __ballot_sync(0xffffffffu, seen != 0u);
+        __syncthreads();   // the batch before has been read
+        if (lane == 0) s_warp_kept[warp] = __popc(kept_mask);
+        __syncthreads();
+        uint32_t pos = __popc(kept_mask & ((1u << lane) - 1u)), n_kept = 0;
+        for (uint32_t w = 0; w < n_warps; ++w) {
+            const uint32_t cnt = s_warp_kept[w];
+            if (w < warp) pos += cnt;
+            n_kept += cnt;
+        }
+        if (seen) {
+            sA[pos] = e.A;
+            sB[pos] = e.B;
+            sC[pos] = e.C;
+            sId[pos] = g;
+            sPos[pos] = idx;
+            sSeen[pos] = seen;
+            stage_features<CDIM>(sRgb + pos * CDIM, colors, (size_t)g, fstride, vec, ranges != nullptr, e.C.w);
         }
         __syncthreads();
-        for (int32_t t = max(0, batch_end - warp_bin_final); t < batch_size; ++t) {
-            bool valid = inside && (batch_end - t <= bin_final);
-            float alpha = 0.f, opac = 0.f, vis = 0.f, dx = 0.f, dy = 0.f;
-            float4 B = make_float4(0.f, 0.f, 0.f, 0.f), Cc = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (valid) {
-                const float4 A = sA[t];
-                B = sB[t];
-                Cc = sC[t];
-                opac = B.w;
-                dx = angle_difference(A.x + roll * A.z, px);
-                dy = angle_difference(A.y + roll * A.w, py);
-                const float sigma = 0.5f * (B.x * dx * dx + B.z * dy * dy) + B.y * dx * dy;
-                vis = __expf(-sigma);
-                alpha = fminf(kAlphaMax, opac * vis);
-                if (sigma < 0.f || alpha < kAlphaMin) valid = false;
-            }
-            if (!__any_sync(0xffffffffu, valid)) continue;
-            float v_rgb[CDIM];
+        for (uint32_t t0 = 0; t0 < n_kept; t0 += 32) {
+            const uint32_t mine = t0 + lane;
+            uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u) && sPos[mine] <= warp_last);
+            while (todo) {
+                const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
+                todo &= todo - 1u;
+                const float4 A = sA[t], B = sB[t];
+                const int32_t entry = sPos[t];
+                const PointFootprint f0 = point_footprint(A, B, roll.x, az.x, el.x), f1 = point_footprint(A, B, roll.y, az.y, el.y);
+                const float a0 = fminf(kAlphaMax, B.w * f0.vis), a1 = fminf(kAlphaMax, B.w * f1.vis);
+                const bool ok0 = entry <= bin_final[0] && !(f0.sigma < 0.f || a0 < kAlphaMin);
+                const bool ok1 = entry <= bin_final[1] && !(f1.sigma < 0.f || a1 < kAlphaMin);
+                if (!__any_sync(0xffffffffu, ok0 || ok1)) continue;
+                const float4 Cc = sC[t];
+                const float2 dx = make_float2(f0.dx, f1.dx), dy = make_float2(f0.dy, f1.dy);
+                const float2 vis = make_float2(ok0 ? f0.vis : 0.f, ok1 ? f1.vis : 0.f);
+                const float2 alpha = make_float2(ok0 ? a0 : 0.f, ok1 ? a1 : 0.f);
+                // a capped alpha passes no gradient on to the geometry
+                const float2 open = make_float2(B.w * f0.vis <= kAlphaMax ? 1.f : 0.f, B.w * f1.vis <= kAlphaMax ? 1.f : 0.f);
+                const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
+                const float2 ra = make_float2(1.f / om.x, 1.f / om.y);
+                T = __fmul2_rn(T, ra);
+                const float2 fac = __fmul2_rn(alpha, T);
+                const float2 dterm = __ffma2_rn(make_float2(Cc.x, Cc.x), roll,
+                                                __ffma2_rn(make_float2(Cc.z, Cc.z), dy, __fmul2_rn(make_float2(Cc.y, Cc.y), dx)));
+                float sum[CDIM + kGeo];
+                float2 dot = __fmul2_rn(dterm, v_depth);   // (c . g) of the two points, the compensated range in it
 #pragma unroll
-            for (int k = 0; k < CDIM; ++k) v_rgb[k] = 0.f;
-            float v_conic_x = 0.f, v_conic_y = 0.f, v_conic_z = 0.f;
-            float v_x = 0.f, v_y = 0.f, v_ax = 0.f, v_ay = 0.f, v_o = 0.f;
-            float v_vx = 0.f, v_vy = 0.f, v_vz = 0.f, v_dcx = 0.f, v_dcy = 0.f;
-            if (valid) {
-                const float ra = 1.f / (1.f - alpha);
-                T *= ra;
-                const float fac = alpha * T;
-                const float dterm = Cc.y * dx + Cc.z * dy + Cc.x * roll;
-                // two channels per instruction (packed FP32 multiply-adds); channels beyond the
-                // rendered ones have zero rows, zero cotangents and zero buffers
-                const float *rgb = sRgb + (uint32_t)t * CDIM;
-                const float2 fac2 = make_float2(fac, fac), T2 = make_float2(T, T), nra2 = make_float2(-ra, -ra);
-                float2 va2 = make_float2(0.f, 0.f);
+                for (int h = 0; h < 2; ++h) {
+                    const float *v = v_out[h];
+                    const float2 f2 = h ? make_float2(fac.y, fac.y) : make_float2(fac.x, fac.x);
+                    float2 d2 = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int k = 0; k < CDIM; k += 4) {
-                    const float4 c4 = *reinterpret_cast<const float4 *>(rgb + k);
+                    for (int k = 0; k < CDIM; k += 4) {
+                        const float4 c4 = *reinterpret_cast<const float4 *>(sRgb + t * CDIM + k);
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int q = k + 2 * h;
-                        const float2 c2 = h ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
-                        const float2 vr2 = make_float2(v_render_c[q], v_render_c[q + 1]);
-                        const float2 b2 = make_float2(buffer[q], buffer[q + 1]);
-                        const float2 g2 = __fmul2_rn(fac2, vr2);
-                        v_rgb[q] = g2.x; v_rgb[q + 1] = g2.y;
-                        const float2 u2 = __ffma2_rn(c2, T2, __fmul2_rn(b2, nra2));   // rgb T - buffer ra
-                        va2 = __ffma2_rn(u2, vr2, va2);
-                        const float2 nb2 = __ffma2_rn(c2, fac2, b2);
-                        buffer[q] = nb2.x; buffer[q + 1] = nb2.y;
+                        for (int m = 0; m < 4; m += 2) {
+                            const float2 c2 = m ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
+                            const float2 v2 = make_float2(v[k + m], v[k + m + 1]);
+                            d2 = k + m == 0 ? __fmul2_rn(c2, v2) : __ffma2_rn(c2, v2, d2);
+                            const float2 acc = h == 0 ? __fmul2_rn(f2, v2) : __ffma2_rn(f2, v2, make_float2(sum[k + m], sum[k + m + 1]));
+                            sum[k + m] = acc.x; sum[k + m + 1] = acc.y;
+                        }
                     }
+                    if (h) dot.y += d2.x + d2.y; else dot.x += d2.x + d2.y;
                 }
-                float v_alpha = va2.x + va2.y;
-                v_alpha -= buffer_extra * ra * v_depth_c;   // the depth channel's buffer also holds the compensation terms
-                const float v_rgb_depth = fac * v_depth_c;
-                v_alpha += dterm * T * v_depth_c;
-                v_alpha += T_final * ra * v_render_a;
-                if (backgrounds != nullptr) v_alpha += -T_final * ra * bg_dot;
-                if (opac * vis <= kAlphaMax) {
-                    v_dcx = v_rgb_depth * dx;
-                    v_dcy = v_rgb_depth * dy;
-                    v_vz = v_rgb_depth * roll;
-                    const float v_sigma = -opac * vis * v_alpha;
-                    v_conic_x = 0.5f * v_sigma * dx * dx;
-                    v_conic_y = v_sigma * dx * dy;
-                    v_conic_z = 0.5f * v_sigma * dy * dy;
-                    v_x = v_sigma * (B.x * dx + B.y * dy) + v_rgb_depth * Cc.y;
-                    v_y = v_sigma * (B.y * dx + B.z * dy) + v_rgb_depth * Cc.z;
-                    v_vx = v_x * roll;
-                    v_vy = v_y * roll;
-                    v_ax = fabsf(v_x);
-                    v_ay = fabsf(v_y);
-                    v_o = vis * v_alpha;
+                const float2 v_alpha = __ffma2_rn(T, dot, __fmul2_rn(make_float2(-ra.x, -ra.y), behind));
+                behind = __ffma2_rn(fac, dot, behind);
+                // v = -dL/dsigma / opacity; the alpha sum reaches the entries in front of the point
+                const float2 v_main = __fmul2_rn(__fmul2_rn(vis, open), v_alpha);
+                float2 v_sum = make_float2(0.f, 0.f);
+                if (compute_alpha_sum) {
+                    const float g_depth = sRgb[t * CDIM + depth_idx];
+                    v_sum = __fmul2_rn(vis, make_float2(g_depth < sum_limit.x ? v_asum.x : 0.f, g_depth < sum_limit.y ? v_asum.y : 0.f));
                 }
-                buffer_extra += dterm * fac;
-
-                const float g_depth = rgb[depth_idx];
-                if (compute_alpha_sum && g_depth < (pz - alpha_sum_threshold)) {
-                    const float vs = v_asum * -opac * vis;
-                    const float ux = vs * (B.x * dx + B.y * dy);
-                    const float uy = vs * (B.y * dx + B.z * dy);
-                    v_x += ux; v_y += uy;
-                    v_vx += ux * roll; v_vy += uy * roll;
-                    v_ax += fabsf(ux); v_ay += fabsf(uy);
-                    v_conic_x += vs * 0.5f * dx * dx;
-                    v_conic_y += vs * dx * dy;
-                    v_conic_z += vs * 0.5f * dy * dy;
-                    v_o += v_asum * vis;
+                const float2 v = __fadd2_rn(v_main, v_sum);
+                const float2 w = __fmul2_rn(make_float2(-B.w, -B.w), v);                   // dL/dsigma
+                const float2 vd = __fmul2_rn(__fmul2_rn(fac, open), v_depth);              // dL/d(range term)
+                const float2 bx = make_float2(B.x, B.x), by = make_float2(B.y, B.y), bz = make_float2(B.z, B.z);
+                const float2 sx = __ffma2_rn(bx, dx, __fmul2_rn(by, dy)), sy = __ffma2_rn(by, dx, __fmul2_rn(bz, dy));
+                const float2 gx = __ffma2_rn(w, sx, __fmul2_rn(vd, make_float2(Cc.y, Cc.y)));
+                const float2 gy = __ffma2_rn(w, sy, __fmul2_rn(vd, make_float2(Cc.z, Cc.z)));
+                const float2 wx = __fmul2_rn(w, dx), wy = __fmul2_rn(w, dy);
+                const auto both = [](float2 p, float2 q) { const float2 r = __fmul2_rn(p, q); return r.x + r.y; };
+                sum[CDIM + 0] = both(wx, dx);
+                sum[CDIM + 1] = both(wx, dy);
+                sum[CDIM + 2] = both(wy, dy);
+                sum[CDIM + 3] = gx.x + gx.y;
+                sum[CDIM + 4] = gy.x + gy.y;
+                sum[CDIM + 5] = both(gx, roll);
+                sum[CDIM + 6] = both(gy, roll);
+                sum[CDIM + 7] = both(vd, roll);
+                sum[CDIM + 8] = both(vd, dx);
+                sum[CDIM + 9] = both(vd, dy);
+                sum[CDIM + 10] = v.x + v.y;
+                if (kAbs) {
+                    const float2 us = __fmul2_rn(make_float2(-B.w, -B.w), v_sum);
+                    const float2 ux = __fmul2_rn(us, sx), uy = __fmul2_rn(us, sy);
+                    sum[CDIM + 11] = fabsf(gx.x - ux.x) + fabsf(ux.x) + fabsf(gx.y - ux.y) + fabsf(ux.y);
+                    sum[CDIM + 12] = fabsf(gy.x - uy.x) + fabsf(uy.x) + fabsf(gy.y - uy.y) + fabsf(uy.y);
                 }
-            }
-            // warp totals: the feature gradients in one multi-value butterfly, the thirteen geometry
-            // gradients in another; each total then sits on its own lane, which adds it in
-            constexpr int kColorSlots = pow2_at_least(CDIM);
-            float cs[kColorSlots];
+                const size_t gid = (size_t)sId[t];
+                float slots[kSlots];
 #pragma unroll
-            for (int k = 0; k < kColorSlots; ++k) cs[k] = k < CDIM ? v_rgb[k] : 0.f;
-            float gs[16] = {v_conic_x, v_conic_y, v_conic_z, v_x, v_y, v_vx, v_vy, v_vz, v_dcx, v_dcy,
-                            v_o, v_ax, v_ay, 0.f, 0.f, 0.f};
-            const float c_tot = warp_sum_slots<kColorSlots>(cs, lane);
-            const float g_tot = warp_sum_slots<16>(gs, lane);
-            const size_t g = (size_t)sId[t];
-            const uint32_t ci = (lane * (uint32_t)kColorSlots) >> 5;
-            if ((lane & (32u / kColorSlots - 1u)) == 0u) {
-                if (ci < fstride) atomicAdd(v_colors + g * fstride + ci, c_tot);
-                else if (ci < channels) atomicAdd(v_ranges + g, c_tot);
+                for (int k = 0; k < kSlots; ++k) slots[k] = k < (kSplit ? CDIM : CDIM + kGeo) ? sum[k] : 0.f;
+                slot_a.add(gid, warp_sum_slots<kSlots>(slots, lane), 1.f, writes_a);
+                if (kSplit) {
+                    float geo[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) geo[k] = k < kGeo ? sum[CDIM + k] : 0.f;
+                    const float geo_total = warp_sum_slots<16>(geo, lane);
+                    const GradSlot slot_b = point_grad_slot<kAbs>(CDIM + (int)(lane >> 1), CDIM, channels, fstride, v_colors,
+                                                                  v_ranges, v_conics, v_means2d, v_pix_vels, v_depth_comps,
+                                                                  v_opacities, v_means2d_abs);
+                    slot_b.add(gid, geo_total, 1.f, (lane & 1u) == 0u);
+                }
             }
-            const uint32_t gi = lane >> 1;
-            float *dst = nullptr;
-            if (gi < 3u) dst = v_conics + 3 * g + gi;
-            else if (gi < 5u) dst = v_means2d + 2 * g + (gi - 3u);
-            else if (gi < 8u) dst = v_pix_vels + 3 * g + (gi - 5u);
-            else if (gi < 10u) dst = v_depth_comps + 2 * g + (gi - 8u);
-            else if (gi == 10u) dst = v_opacities + g;
-            else if (gi < 13u && v_means2d_abs != nullptr) dst = v_means2d_abs + 2 * g + (gi - 11u);
-            if ((lane & 1u) == 0u && dst != nullptr) atomicAdd(dst, g_tot);
         }
     }
 }
@@ -1024,19 +1251,11 @@ __global__ void rasterize_to_points_bwd_kernel(
         else { CALL(32); }                                                                       \
     } while (0)
 
-// A tile may have up to 1024 samples, one thread each; the backward kernels with many channels
-// need more registers per thread than a block of that size can have. Said here, with the numbers,
-// rather than by a failed launch.
-template <typename K>
-static int check_block_size(K kernel, uint32_t threads, uint32_t channels, const char *what) {
-    if (threads <= 256) return SPLATAD_OK;
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) return check_launch(what);
-    SPL_REQUIRE((uint32_t)fa.maxThreadsPerBlock >= threads, SPLATAD_ERR_BAD_ARG,
-                "%s: a tile of %u samples with %u channels needs blocks of %u threads, this kernel runs at "
-                "most %d (%d registers per thread): use a smaller tile or fewer channels per call",
-                what, threads, channels, threads, fa.maxThreadsPerBlock, fa.numRegs);
-    return SPLATAD_OK;
+// Warps per CTA of the lidar kernels. Two when the tiles fill the machine: a CTA ends with its slowest
+// warp. Four when they do not, where the staging of a batch - which more warps share - is a part of the
+// chain every warp waits for (32 x 512 points: forward 146 us with one warp per CTA, 124 with four).
+static uint32_t point_warps_per_cta(uint64_t tiles, uint32_t warps_per_tile) {
+    return min(tiles * warps_per_tile >= (uint64_t)kNumSMs * 16 ? 2u : 4u, warps_per_tile);
 }
 
 template <typename K>
@@ -1177,25 +1396,23 @@ extern "C" int splatad_rasterize_to_points_fwd(
                 SPLATAD_ERR_BAD_ARG, "rasterize_to_points_fwd: null input");
     const uint32_t blocks = C * tile_grid_width * tile_grid_height;
     if (blocks == 0 || image_width == 0 || image_height == 0) return SPLATAD_OK;
-    const uint32_t bs = ((tile_width * tile_height + 31) / 32) * 32;   // whole warps
-    size_t smem = (size_t)bs * (3 * sizeof(float4) + sizeof(int32_t));
-    // the batch's feature rows ride along in shared memory while a block stays under 64 KB
-    const uint32_t cdim = channels <= 4 ? 4u : channels <= 8 ? 8u : channels <= 16 ? 16u : channels <= 20 ? 20u : 32u;
-    const size_t smem_feat = (size_t)bs * cdim * sizeof(float);   // rows of CDIM floats, see SPL_DISPATCH_CDIM
-    const uint32_t stage_features = (smem + smem_feat <= 64 * 1024) ? 1u : 0u;
-    if (stage_features) smem += smem_feat;
+    const uint32_t warps = div_up(tile_width * tile_height, 32);
+    const uint32_t per_cta = point_warps_per_cta(blocks, warps), parts = div_up(warps, per_cta), bs = 32 * per_cta;
+    SPL_REQUIRE((uint64_t)blocks * parts <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_points_fwd: too many tiles");
 #define CALL(D)                                                                                   \
     {                                                                                             \
+        const size_t smem = (size_t)points_fwd_stage(D) * bs *                                    \
+                            (3 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float));       \
         int rc = set_smem(rasterize_to_points_fwd_kernel<D>, smem, "rasterize_to_points_fwd");    \
         if (rc != SPLATAD_OK) return rc;                                                          \
-        launch_chained(rasterize_to_points_fwd_kernel<D>, blocks, bs, smem, (cudaStream_t)stream, \
+        launch_chained(rasterize_to_points_fwd_kernel<D>, blocks * parts, bs, smem, (cudaStream_t)stream, \
             C, n_isects, (const float2 *)means2d, conics, lidar_features, gaussian_ranges,        \
             channels, opacities,                                                                  \
             pix_vels, (const float2 *)depth_compensations, backgrounds,                           \
             (const float4 *)raster_pts, image_width, image_height, tile_width, tile_height,       \
-            tile_grid_width, tile_grid_height, compute_alpha_sum_until_points,                    \
+            tile_grid_width, tile_grid_height, parts, compute_alpha_sum_until_points,             \
             alpha_sum_threshold, tile_offsets, flatten_ids, depth_channel_idx, render_features,   \
-            render_alphas, alpha_sum_until_points, last_ids, median_depths, stage_features);      \
+            render_alphas, alpha_sum_until_points, last_ids, median_depths);                      \
     }
     {
         SPL_PROF("rasterize_to_points_fwd_kernel", (cudaStream_t)stream);
@@ -1236,30 +1453,38 @@ extern "C" int splatad_rasterize_to_points_bwd(
                 "rasterize_to_points_bwd: features / v_features missing");
     SPL_REQUIRE(!gaussian_ranges || (v_gaussian_ranges && depth_channel_idx == channels - 1),
                 SPLATAD_ERR_BAD_ARG, "rasterize_to_points_bwd: range array needs v_gaussian_ranges");
-    const uint32_t bs = ((tile_width * tile_height + 31) / 32) * 32;   // whole warps
-    const uint32_t cdim = channels <= 4 ? 4u : channels <= 8 ? 8u : channels <= 16 ? 16u : channels <= 20 ? 20u : 32u;
-    const size_t smem = (size_t)bs * (3 * sizeof(float4) + sizeof(int32_t) + cdim * sizeof(float));   // rows of CDIM floats
-#define CALL(D)                                                                                   \
+    const uint32_t samples = ((tile_width * tile_height + 31) / 32) * 32;
+    SPL_REQUIRE(samples <= 512 || channels <= 16, SPLATAD_ERR_BAD_ARG,
+                "rasterize_to_points_bwd: a tile of %u points (%u threads at one per point) with %u channels is more "
+                "than the backward pass takes: use a smaller tile or at most 16 channels per call",
+                tile_width * tile_height, samples, channels);
+    const uint32_t warps = div_up(tile_width * tile_height, 64);
+    const uint32_t per_cta = point_warps_per_cta(blocks, warps), parts = div_up(warps, per_cta), bs = 32 * per_cta;
+    SPL_REQUIRE((uint64_t)blocks * parts <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_points_bwd: too many tiles");
+#define CALL_ABS(D, A)                                                                            \
     {                                                                                             \
-        int rc = check_block_size(rasterize_to_points_bwd_kernel<D>, bs, channels, "rasterize_to_points_bwd"); \
+        auto kernel = rasterize_to_points_bwd_kernel<D, A>;                                       \
+        const size_t smem = (size_t)bs * (3 * sizeof(float4) + 3 * sizeof(int32_t) + D * sizeof(float)); \
+        int rc = set_smem(kernel, smem, "rasterize_to_points_bwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
-        rc = set_smem(rasterize_to_points_bwd_kernel<D>, smem, "rasterize_to_points_bwd");    \
-        if (rc != SPLATAD_OK) return rc;                                                          \
-        rasterize_to_points_bwd_kernel<D><<<blocks, bs, smem, (cudaStream_t)stream>>>(            \
+        kernel<<<blocks * parts, bs, smem, (cudaStream_t)stream>>>(                               \
             C, n_isects, (const float2 *)means2d, conics, lidar_features, gaussian_ranges,        \
             channels, opacities,                                                                  \
             pix_vels, (const float2 *)depth_compensations, backgrounds,                           \
             (const float4 *)raster_pts, image_width, image_height, tile_width, tile_height,       \
-            tile_grid_width, tile_grid_height, compute_alpha_sum_until_points,                    \
+            tile_grid_width, tile_grid_height, parts, compute_alpha_sum_until_points,             \
             alpha_sum_threshold, tile_offsets, flatten_ids, depth_channel_idx, render_alphas,     \
             last_ids, v_render_features, v_render_alphas, v_alpha_sum_until_points,               \
             v_means2d_abs, v_means2d, v_conics, v_features, v_opacities, v_pix_vels,              \
             v_depth_compensations, v_gaussian_ranges);                                            \
     }
+#define CALL(D)                                                                                   \
+    if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)
     {
         SPL_PROF("rasterize_to_points_bwd_kernel", (cudaStream_t)stream);
         SPL_DISPATCH_CDIM(channels, CALL);
     }
 #undef CALL
+#undef CALL_ABS
     return check_launch("rasterize_to_points_bwd");
 }

@@ -350,3 +350,72 @@ def test_rasterize_to_points_split_ranges(channels):
     if channels > 1:
         _grad_check("split features", B["f"].grad, n(A["feats"].grad[..., :-1]), rel=1e-5)
     _grad_check("split ranges", B["r"].grad, n(A["feats"].grad[..., -1]), rel=1e-5)
+
+
+@pytest.mark.parametrize("ts,W,H,channels,absgrad", [(1, 9, 5, 3, False), (5, 33, 21, 4, True), (16, 17, 16, 1, False),
+                                                     (16, 15, 2, 8, True), (17, 50, 40, 9, False), (31, 62, 45, 3, True),
+                                                     (16, 40, 33, 20, True), (8, 30, 30, 32, False)])
+def test_pixels_several_per_thread(ts, W, H, channels, absgrad):
+    """Threads draw two or four pixels of a row, warps cover patches of a tile and skip what cannot reach
+    them: tile sizes that are no multiple of either, images that end inside a patch or a thread's
+    pixels, every channel group, forward and backward against the oracle."""
+    from oracle import composite
+    from splatad_b200 import ops
+    c = _camera_case(1, 900, W, H, ts, channels, 1000 * ts + channels)
+    g = torch.Generator().manual_seed(3)
+    v_c, v_a = torch.randn(1, H, W, channels, generator=g), torch.randn(1, H, W, 1, generator=g)
+    keys = ("means2d", "conics", "colors", "opacities", "pix_vels")
+    args = [n(c[k]) for k in keys] + [n(c["rs"]), None, W, H, ts, c["offsets"], c["flatten_ids"]]
+    ref_f = composite.rasterize_to_pixels_fwd(*args, dtype=np.float64)
+    f32 = composite.rasterize_to_pixels_fwd(*args, amb_tol=1e-4)
+    same = (f32["last_ids"] == ref_f["last_ids"]) & ~f32["ambiguous"]
+    assert same.mean() > 0.9
+    mask, mk = t(same[..., None].astype(np.float32)), same[..., None].astype(np.float64)
+    leaves = {k: t(c[k]).requires_grad_(True) for k in keys}
+    out_c, out_a = ops.rasterize_to_pixels(*(leaves[k] for k in keys), W, H, ts, t(c["offsets"], torch.int32),
+                                           t(c["flatten_ids"], torch.int32), t(c["rs"]), absgrad=absgrad)
+    _check_fwd(f"pixels tile {ts} {W}x{H} ch={channels}", n(out_c), n(out_a), f32)
+    torch.autograd.backward([out_c, out_a], [t(v_c) * mask, t(v_a) * mask])
+    ref = composite.rasterize_to_pixels_bwd(*args, ref_f["render_alphas"], ref_f["last_ids"], n(v_c) * mk, n(v_a) * mk,
+                                            absgrad=absgrad)
+    for k in keys:
+        _grad_check(f"tile {ts} ch={channels} v_{k}", leaves[k].grad, ref["v_" + k])
+    if absgrad:
+        _grad_check(f"tile {ts} ch={channels} absgrad", leaves["means2d"].absgrad, ref["v_means2d_abs"])
+
+
+@pytest.mark.parametrize("tw,th,H,W,channels,asum,absgrad", [(32, 8, 20, 130, 3, True, True), (8, 4, 9, 100, 17, False, False),
+                                                             (5, 3, 10, 64, 9, True, False), (64, 16, 40, 96, 16, False, True),
+                                                             (1, 1, 6, 40, 2, True, False), (32, 8, 130, 1024, 5, True, False),
+                                                             (8, 8, 17, 70, 32, False, False)])
+def test_points_in_patches(tw, th, H, W, channels, asum, absgrad):
+    """Patches of 8 x 4 and 8 x 8 points, tiles that cannot be cut into them, scans that end inside a
+    patch, patches without a single return, one and several CTAs per tile, few tiles and many:
+    forward and backward against the oracle."""
+    from oracle import composite
+    from splatad_b200 import ops
+    c = _lidar_case(1, 1500, H, W, tw, th, channels, 100 * tw + channels)
+    c["pts"][0, : min(th, H), : min(tw, W), 2] = 0.0
+    g = torch.Generator().manual_seed(4)
+    v_c, v_a, v_s = (torch.randn(1, H, W, k, generator=g) for k in (channels, 1, 1))
+    keys = ("means2d", "conics", "feats", "opacities", "pix_vels", "dcomp")
+    args = [n(c[k]) for k in keys] + [None, n(c["pts"]), W, H, tw, th, c["offsets"], c["flatten_ids"], asum, 0.5]
+    ref_f = composite.rasterize_to_points_fwd(*args, dtype=np.float64)
+    f32 = composite.rasterize_to_points_fwd(*args, amb_tol=1e-4)
+    same = (f32["last_ids"] == ref_f["last_ids"]) & ~f32["ambiguous"]
+    assert same.mean() > 0.9
+    mask, mk = t(same[..., None].astype(np.float32)), same[..., None].astype(np.float64)
+    leaves = {k: t(c[k]).requires_grad_(True) for k in keys}
+    out_c, out_a, out_s, out_m = ops.rasterize_to_points(
+        *(leaves[k] for k in keys), t(c["pts"]), W, H, tw, th, t(c["offsets"], torch.int32),
+        t(c["flatten_ids"], torch.int32), asum, 0.5, absgrad=absgrad)
+    _check_fwd(f"points tile {tw}x{th} ch={channels}", n(out_c), n(out_a), f32, depth_channel=channels - 1)
+    cot = [t(v_c) * mask, t(v_a) * mask] + ([t(v_s) * mask] if asum else [])
+    torch.autograd.backward([out_c, out_a] + ([out_s] if asum else []), cot)
+    ref = composite.rasterize_to_points_bwd(*args, ref_f["render_alphas"], ref_f["last_ids"], n(v_c) * mk, n(v_a) * mk,
+                                            (n(v_s) * mk) if asum else None, absgrad=absgrad)
+    names = ("v_means2d", "v_conics", "v_colors", "v_opacities", "v_pix_vels", "v_depth_comps")
+    for k, name in zip(keys, names):
+        _grad_check(f"tile {tw}x{th} ch={channels} {name}", leaves[k].grad, ref[name])
+    if absgrad:
+        _grad_check(f"tile {tw}x{th} ch={channels} absgrad", leaves["means2d"].absgrad, ref["v_means2d_abs"])
