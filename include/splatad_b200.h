@@ -434,6 +434,46 @@ int splatad_rasterize_to_pixels_bwd(
     float *v_means2d_abs, float *v_means2d, float *v_conics, float *v_colors, float *v_opacities,
     float *v_pix_vels, void *stream);
 
+/* The same pair for the "expected depth" render modes: with expected_last_channel != 0 the last channel
+ * leaves divided by max(alpha, 1e-10) (the torch ops behind the kernel in gsplat/rendering.py:423-430);
+ * expected_render is that render when the cotangents are those of the divided channel, NULL otherwise. */
+int splatad_rasterize_expected_to_pixels_fwd(
+    uint32_t C, int64_t n_isects, const float *means2d, const float *conics, const float *colors,
+    uint32_t channels, const float *opacities, const float *pix_vels,
+    const float *rolling_shutter_time, const float *backgrounds, uint32_t image_width,
+    uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
+    const int32_t *tile_offsets, const int32_t *flatten_ids, int32_t expected_last_channel,
+    float *render_colors, float *render_alphas, int32_t *last_ids, void *stream);
+int splatad_rasterize_expected_to_pixels_bwd(
+    uint32_t C, int64_t n_isects, const float *means2d, const float *conics, const float *colors,
+    uint32_t channels, const float *opacities, const float *pix_vels,
+    const float *rolling_shutter_time, const float *backgrounds, uint32_t image_width,
+    uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
+    const int32_t *tile_offsets, const int32_t *flatten_ids, const float *expected_render,
+    const float *render_alphas, const int32_t *last_ids, const float *v_render_colors,
+    const float *v_render_alphas, float *v_means2d_abs, float *v_means2d, float *v_conics,
+    float *v_colors, float *v_opacities, float *v_pix_vels, void *stream);
+
+/* What the compositing reads per projected row, from the per-Gaussian parameters (the torch gathers,
+ * products and concatenations of gsplat/rendering.py:325-343, 383-384). Row i belongs to Gaussian
+ * gaussian_ids[i] of sensor camera_ids[i] (packed, int64), or i % N of sensor i / N (NULL).
+ * opacity_rows: rows [n] = opacities[.] * compensations[n] (NULL: 1). color_rows: rows [n, D (+ 1)] from
+ * colors [N,D] ([C,N,D] with colors_per_camera != 0), the depths [n] behind them when given.
+ * VJPs: v_opacities [N] and v_colors are accumulated with atomics (zero-initialise them),
+ * v_compensations [n] and v_depths [n] = v_depths_in (NULL: 0) + the last of `width` channels are
+ * written; each may be NULL. */
+int splatad_opacity_rows_fwd(uint32_t n, uint32_t N, const int64_t *gaussian_ids, const float *opacities,
+                             const float *compensations, float *rows, void *stream);
+int splatad_opacity_rows_bwd(uint32_t n, uint32_t N, const int64_t *gaussian_ids, const float *opacities,
+                             const float *compensations, const float *v_rows, float *v_opacities,
+                             float *v_compensations, void *stream);
+int splatad_color_rows_fwd(uint32_t n, uint32_t N, uint32_t D, const int64_t *camera_ids,
+                           const int64_t *gaussian_ids, uint32_t colors_per_camera, const float *colors,
+                           const float *depths, float *rows, void *stream);
+int splatad_color_rows_bwd(uint32_t n, uint32_t N, uint32_t D, uint32_t width, const int64_t *camera_ids,
+                           const int64_t *gaussian_ids, uint32_t colors_per_camera, const float *v_rows,
+                           float *v_colors, const float *v_depths_in, float *v_depths, void *stream);
+
 /* rasterize_to_points_fwd_tensor - gsplat/cuda/csrc/rasterization.cu:2221-2831, kernel
  * 2021-2219. raster_pts [C,H,W,4] = (azimuth deg, elevation deg, range m, time offset s);
  * points with range <= 0 are not rendered and produce zeros. pix_vels [.,3],

@@ -9,6 +9,8 @@ exception is raised.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import re
 import subprocess
@@ -20,6 +22,7 @@ import torch
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 _REPO_DIR = os.path.dirname(_PKG_DIR)
 LIB_PATH = os.path.join(_PKG_DIR, "libsplatad_b200.so")
+HOST_PATH = os.path.join(_PKG_DIR, "_host.so")
 HEADER_PATH = os.path.join(_REPO_DIR, "include", "splatad_b200.h")
 CSRC_DIR = os.path.join(_PKG_DIR, "csrc")
 
@@ -112,6 +115,25 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native host side of a frame (``csrc/host/frames.cpp``), bound to the CUDA library. Loaded on first use."""
+    global _host
+    if _host is None:
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: run `python -c 'import __graft_entry__ as g; g.build()'` or "
+                               "`make -C splatad_b200/csrc`")
+        load()
+        loader = importlib.machinery.ExtensionFileLoader("_host", HOST_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
+        loader.exec_module(module)
+        module.bind_library(LIB_PATH)
+        _host = module
+    return _host
+
+
 def last_error() -> str:
     return load().splatad_last_error().decode("utf-8", "replace")
 
@@ -191,21 +213,17 @@ def workspace(tag: str, nbytes: int, device: torch.device) -> torch.Tensor:
     """Scratch buffer for (tag, device, current stream of that device). Work enqueued on one stream
     is ordered, so consecutive calls may share a buffer; two streams never do."""
     index = device.index if device.index is not None else torch.cuda.current_device()
+    if not DEBUG:
+        return host().workspace(tag, nbytes, index)   # shared with the frames of the native host side
     key = (tag, index, torch.cuda.current_stream(device).cuda_stream)
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
-        # grow with headroom so slowly growing scenes do not reallocate every frame
-        size = max(int(nbytes * 1.25) + 1024, 1 << 16)
-        if DEBUG:
-            # exactly the bytes asked for, canary bytes right behind them; the library is told the
-            # size without the canaries
-            whole = torch.empty(nbytes + CANARY_BYTES, dtype=torch.uint8, device=device)
-            whole[nbytes:].fill_(CANARY_VALUE)
-            _canaries[key] = whole[nbytes:]
-            buf = whole[:nbytes]
-        else:
-            buf = torch.empty(size, dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
+        # exactly the bytes asked for, canary bytes right behind them; the library is told the size
+        # without the canaries
+        whole = torch.empty(nbytes + CANARY_BYTES, dtype=torch.uint8, device=device)
+        whole[nbytes:].fill_(CANARY_VALUE)
+        _canaries[key] = whole[nbytes:]
+        buf = _workspaces[key] = whole[:nbytes]
     return buf
 
 
@@ -295,3 +313,5 @@ def release_workspaces() -> None:
     _canaries.clear()
     _pinned.clear()
     _free_slots.clear()
+    if _host is not None:
+        _host.release()

@@ -162,6 +162,7 @@ __device__ __forceinline__ float2 pair_power(float a, float2 dx, float bdy, floa
 // them. A pixel that has stopped moves its column out to where every alpha vanishes, which costs the
 // other pixels nothing; a warp leaves when all of its pixels have. Camera benchmark frame: 0.338 -> 0.248 ms.
 // ---------------------------------------------------------------------------------------
+constexpr float kExpectedMin = 1e-10f;   // alphas below it do not divide (gsplat/rendering.py:423-430)
 constexpr float kPixelGone = 1e18f;   // a column no Gaussian reaches: sigma overflows, alpha is 0 (or NaN, never drawn)
 
 // registers per thread: as many CTAs of 128 threads per SM as the accumulators leave room for
@@ -176,7 +177,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
     uint32_t H, uint32_t tile_size, uint32_t tile_w, uint32_t tile_h,
     const int32_t *__restrict__ offsets, const int32_t *__restrict__ flatten_ids,
     float *__restrict__ render_colors, float *__restrict__ render_alphas,
-    int32_t *__restrict__ last_ids) {
+    int32_t *__restrict__ last_ids, uint32_t expected /* divide the last channel by the alpha */) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_warp_kept[16];
@@ -308,12 +309,17 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
         if (CDIM == 4 && vec_out) {   // one 16-byte store per pixel
             float4 v = make_float4(out[h][0], out[h][1], out[h][2], out[h][3]);
             if (bg) v = make_float4(v.x + Tk * bg[0], v.y + Tk * bg[1], v.z + Tk * bg[2], v.w + Tk * bg[3]);
+            if (expected) v.w /= fmaxf(1.f - Tk, kExpectedMin);
             *reinterpret_cast<float4 *>(dst) = v;
             continue;
         }
 #pragma unroll
         for (int k = 0; k < CDIM; ++k)
-            if ((uint32_t)k < channels) dst[k] = bg ? out[h][k] + Tk * bg[k] : out[h][k];
+            if ((uint32_t)k < channels) {
+                float v = bg ? out[h][k] + Tk * bg[k] : out[h][k];
+                if (expected && (uint32_t)k + 1u == channels) v /= fmaxf(1.f - Tk, kExpectedMin);
+                dst[k] = v;
+            }
     }
 }
 
@@ -747,7 +753,7 @@ rasterize_to_pixels_bwd_kernel(
     const float *__restrict__ v_render_colors, const float *__restrict__ v_render_alphas,
     float *__restrict__ v_means2d_abs, float *__restrict__ v_means2d,
     float *__restrict__ v_conics, float *__restrict__ v_colors, float *__restrict__ v_opacities,
-    float *__restrict__ v_pix_vels) {
+    float *__restrict__ v_pix_vels, const float *__restrict__ expected /* render whose last channel was divided by the alpha */) {
     static_assert(PX % 2 == 0, "pixels are handled in pairs");
     constexpr int P2 = PX / 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -792,17 +798,21 @@ rasterize_to_pixels_bwd_kernel(
     for (int k = 0; k < PX; ++k) {
         const bool in = (uint32_t)k < n_inside;
         const size_t pix = ((size_t)cam * H + (in ? i : 0u)) * W + (in ? j + k : 0u);
-        const float T_final = in ? 1.f - render_alphas[pix] : 1.f;
+        const float a_final = in ? render_alphas[pix] : 0.f, T_final = 1.f - a_final;
         bin_final[k] = in ? last_ids[pix] : -1;
         thread_last = max(thread_last, bin_final[k]);
+        float v_a = in ? v_render_alphas[pix] : 0.f;
         float bg_dot = 0.f;
+        const float divisor = fmaxf(a_final, kExpectedMin);
+        if (in && expected != nullptr && a_final >= kExpectedMin)
+            v_a -= v_render_colors[pix * channels + channels - 1] * expected[pix * channels + channels - 1] / divisor;
 #pragma unroll
         for (int c = 0; c < CDIM; ++c) {
             v_out[k][c] = (in && (uint32_t)c < channels) ? v_render_colors[pix * channels + c] : 0.f;
+            if (expected != nullptr && (uint32_t)c + 1u == channels) v_out[k][c] /= divisor;
             if (backgrounds != nullptr && (uint32_t)c < channels)
                 bg_dot += backgrounds[(size_t)cam * channels + c] * v_out[k][c];
         }
-        const float v_a = in ? v_render_alphas[pix] : 0.f;
         // what the background and the alpha output receive through everything in front of them
         const float last = -T_final * (v_a - bg_dot);
         if (k & 1) { T[k / 2].y = T_final; behind[k / 2].y = last; }
@@ -1282,6 +1292,19 @@ extern "C" int splatad_rasterize_to_pixels_fwd(
     uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
     const int32_t *tile_offsets, const int32_t *flatten_ids, float *render_colors,
     float *render_alphas, int32_t *last_ids, void *stream) {
+    return splatad_rasterize_expected_to_pixels_fwd(C, n_isects, means2d, conics, colors, channels, opacities, pix_vels,
+                                                    rolling_shutter_time, backgrounds, image_width, image_height,
+                                                    tile_size, tile_width, tile_height, tile_offsets, flatten_ids, 0,
+                                                    render_colors, render_alphas, last_ids, stream);
+}
+
+extern "C" int splatad_rasterize_expected_to_pixels_fwd(
+    uint32_t C, int64_t n_isects, const float *means2d, const float *conics, const float *colors,
+    uint32_t channels, const float *opacities, const float *pix_vels,
+    const float *rolling_shutter_time, const float *backgrounds, uint32_t image_width,
+    uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
+    const int32_t *tile_offsets, const int32_t *flatten_ids, int32_t expected_last_channel, float *render_colors,
+    float *render_alphas, int32_t *last_ids, void *stream) {
     SPL_REQUIRE(channels >= 1 && channels <= SPLATAD_MAX_CHANNELS, SPLATAD_ERR_CHANNELS,
                 "rasterize_to_pixels_fwd: unsupported channel count %u (1..%d)", channels,
                 SPLATAD_MAX_CHANNELS);
@@ -1303,7 +1326,7 @@ extern "C" int splatad_rasterize_to_pixels_fwd(
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
             image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
-            render_colors, render_alphas, last_ids);                                              \
+            render_colors, render_alphas, last_ids, (uint32_t)(expected_last_channel != 0));      \
     }
     {
         SPL_PROF("rasterize_to_pixels_fwd_kernel", (cudaStream_t)stream);
@@ -1319,6 +1342,22 @@ extern "C" int splatad_rasterize_to_pixels_bwd(
     const float *rolling_shutter_time, const float *backgrounds, uint32_t image_width,
     uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
     const int32_t *tile_offsets, const int32_t *flatten_ids, const float *render_alphas,
+    const int32_t *last_ids, const float *v_render_colors, const float *v_render_alphas,
+    float *v_means2d_abs, float *v_means2d, float *v_conics, float *v_colors, float *v_opacities,
+    float *v_pix_vels, void *stream) {
+    return splatad_rasterize_expected_to_pixels_bwd(
+        C, n_isects, means2d, conics, colors, channels, opacities, pix_vels, rolling_shutter_time, backgrounds,
+        image_width, image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids, nullptr, render_alphas,
+        last_ids, v_render_colors, v_render_alphas, v_means2d_abs, v_means2d, v_conics, v_colors, v_opacities,
+        v_pix_vels, stream);
+}
+
+extern "C" int splatad_rasterize_expected_to_pixels_bwd(
+    uint32_t C, int64_t n_isects, const float *means2d, const float *conics, const float *colors,
+    uint32_t channels, const float *opacities, const float *pix_vels,
+    const float *rolling_shutter_time, const float *backgrounds, uint32_t image_width,
+    uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
+    const int32_t *tile_offsets, const int32_t *flatten_ids, const float *expected_render, const float *render_alphas,
     const int32_t *last_ids, const float *v_render_colors, const float *v_render_alphas,
     float *v_means2d_abs, float *v_means2d, float *v_conics, float *v_colors, float *v_opacities,
     float *v_pix_vels, void *stream) {
@@ -1352,7 +1391,7 @@ extern "C" int splatad_rasterize_to_pixels_bwd(
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
             image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
             render_alphas, last_ids, v_render_colors, v_render_alphas, v_means2d_abs, v_means2d,  \
-            v_conics, v_colors, v_opacities, v_pix_vels);                                         \
+            v_conics, v_colors, v_opacities, v_pix_vels, expected_render);                        \
     }
 #define CALL(D)                                                                                   \
     if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)

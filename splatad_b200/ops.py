@@ -24,7 +24,6 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
-import struct
 from typing import Optional, Tuple
 
 import torch
@@ -54,6 +53,32 @@ def velocity_grads(enabled: bool = True):
         yield
     finally:
         _RETURN_VELOCITY_GRADS = prev
+
+
+def list_room(count: int) -> int:
+    """List entries a frame is given room for, from the count of the last frame of its shape."""
+    return count + count // 8 + 65536
+
+
+def packed_room(count: int, most: int) -> int:
+    """The same for packed rows."""
+    return min((count + count // 8 + 4096 + 0xFFFF) & ~0xFFFF, most)
+
+
+def note_counts(key, n_isects: int, status: int, depth_range: int, ranged: bool) -> None:
+    """Keeps what a natively enqueued frame reported about its lists for the next frame of its shape."""
+    if status & 2 or n_isects > 0x7FFFFFFF:
+        raise RuntimeError(f"isect: {n_isects} intersections do not fit int32 flatten ids / offsets")
+    _isect_count_hint[key] = n_isects
+    if status & 4:
+        if ranged:
+            # an end bucket overflowed under the depth range carried over from the last frame: the frame
+            # is rendered again without one
+            _depth_range_hint.pop(key, None)
+        else:
+            _depth_sort_mode[key] = 2   # crowded depth buckets: this shape takes the radix sort from now on
+    elif depth_range:
+        _depth_range_hint[key] = (depth_range & 0xFFFFFFFF, depth_range >> 32)
 
 
 def _f(t: Optional[Tensor]) -> Optional[Tensor]:
@@ -335,16 +360,11 @@ def fully_fused_lidar_projection(
     packed: bool = False,
     sparse_grad: bool = False,
     calc_compensations: bool = False,
-    frame: Optional["LidarFrame"] = None,
 ):
     """Projects Gaussians to a batch of spherical lidars (azimuth / elevation in degrees, range).
 
     Returns (radii [C,N,2] float degrees, means2d, depths (range), conics, compensations,
     pix_vels [C,N,3], depth_compensations [C,N,2]).
-
-    ``frame`` (not part of the reference's API): a :class:`LidarFrame` that has already projected
-    exactly these inputs; its outputs are returned with this op's backward attached and nothing is
-    launched.
     """
     C = viewmats.size(0)
     N = means.size(0)
@@ -372,7 +392,7 @@ def fully_fused_lidar_projection(
     return _FullyFusedLidarProjection.apply(
         means, covars, quats, scales, velocities, viewmats, min_elevation, max_elevation,
         min_azimuth, max_azimuth, linear_velocity, angular_velocity, rolling_shutter_time, eps2d,
-        near_plane, far_plane, radius_clip, calc_compensations, frame,
+        near_plane, far_plane, radius_clip, calc_compensations,
     )
 
 
@@ -450,35 +470,28 @@ class _FullyFusedLidarProjection(torch.autograd.Function):
     @staticmethod
     def forward(ctx, means, covars, quats, scales, velocities, viewmats, min_elevation,
                 max_elevation, min_azimuth, max_azimuth, linear_velocity, angular_velocity,
-                rolling_shutter_time, eps2d, near_plane, far_plane, radius_clip, calc_compensations,
-                frame=None):
+                rolling_shutter_time, eps2d, near_plane, far_plane, radius_clip, calc_compensations):
         means, covars, quats, scales, velocities, viewmats, lin, ang, rs = _proj_inputs(
             means, covars, quats, scales, velocities, viewmats, linear_velocity, angular_velocity,
             rolling_shutter_time)
         C, N = viewmats.shape[0], means.shape[0]
         dev = means.device
         f32 = dict(dtype=torch.float32, device=dev)
-        if frame is not None:
-            # projected by the single-call frame already: only the graph node is made here
-            assert not calc_compensations and covars is None and frame.radii.shape == (C, N, 2)
-            radii, means2d, depths, conics = frame.radii, frame.means2d, frame.depths, frame.conics
-            pix_vels, depth_comps, compensations = frame.pix_vels, frame.depth_compensations, None
-        else:
-            radii = torch.empty((C, N, 2), **f32)
-            means2d = torch.empty((C, N, 2), **f32)
-            depths = torch.empty((C, N), **f32)
-            conics = torch.empty((C, N, 3), **f32)
-            pix_vels = torch.empty((C, N, 3), **f32)
-            depth_comps = torch.empty((C, N, 2), **f32)
-            compensations = torch.empty((C, N), **f32) if calc_compensations else None
-            _call(
-                "splatad_lidar_projection_fwd", C, N, _lib.ptr(means), _lib.ptr(covars), _lib.ptr(quats),
-                _lib.ptr(scales), _lib.ptr(velocities), _lib.ptr(viewmats), min_elevation, max_elevation,
-                min_azimuth, max_azimuth, _lib.ptr(lin), _lib.ptr(ang), _lib.ptr(rs), eps2d, near_plane,
-                far_plane, radius_clip, _lib.ptr(radii), _lib.ptr(means2d), _lib.ptr(depths),
-                _lib.ptr(conics), _lib.ptr(compensations), _lib.ptr(pix_vels), _lib.ptr(depth_comps),
-                _lib.stream_ptr(dev),
-            )
+        radii = torch.empty((C, N, 2), **f32)
+        means2d = torch.empty((C, N, 2), **f32)
+        depths = torch.empty((C, N), **f32)
+        conics = torch.empty((C, N, 3), **f32)
+        pix_vels = torch.empty((C, N, 3), **f32)
+        depth_comps = torch.empty((C, N, 2), **f32)
+        compensations = torch.empty((C, N), **f32) if calc_compensations else None
+        _call(
+            "splatad_lidar_projection_fwd", C, N, _lib.ptr(means), _lib.ptr(covars), _lib.ptr(quats),
+            _lib.ptr(scales), _lib.ptr(velocities), _lib.ptr(viewmats), min_elevation, max_elevation,
+            min_azimuth, max_azimuth, _lib.ptr(lin), _lib.ptr(ang), _lib.ptr(rs), eps2d, near_plane,
+            far_plane, radius_clip, _lib.ptr(radii), _lib.ptr(means2d), _lib.ptr(depths),
+            _lib.ptr(conics), _lib.ptr(compensations), _lib.ptr(pix_vels), _lib.ptr(depth_comps),
+            _lib.stream_ptr(dev),
+        )
         ctx.save_for_backward(means, covars, quats, scales, velocities, viewmats, lin, ang, rs, radii,
                               conics, compensations)
         ctx.eps2d = eps2d
@@ -518,7 +531,7 @@ class _FullyFusedLidarProjection(torch.autograd.Function):
             v_quats = None
         if not ctx.needs_input_grad[3]:
             v_scales = None
-        return (v_means, v_covars, v_quats, v_scales, v_vel, v_viewmats) + (None,) * 13
+        return (v_means, v_covars, v_quats, v_scales, v_vel, v_viewmats) + (None,) * 12
 
 
 class PendingPackedCount:
@@ -601,7 +614,7 @@ class _FullyFusedProjectionPacked(torch.autograd.Function):
             hint = _packed_nnz_hint.get(key)
             capacity = None
             if hint:
-                capacity = min((hint + hint // 8 + 4096 + 0xFFFF) & ~0xFFFF, C * N)
+                capacity = packed_room(hint, C * N)
                 out = outputs(capacity)
                 fill(capacity, out)
             if pending is not None and capacity is not None:
@@ -1015,7 +1028,7 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
         return DeferredIsect.done(*exact(), C, n_tiles_total)
     # Enqueue plan and fill back to back with room for somewhat more intersections than last time;
     # the count is read when the caller asks for the exact tensors.
-    capacity = hint + hint // 8 + 65536
+    capacity = list_room(hint)
     slot = _lib.acquire_pinned_slot(dev)
     # the rectangle count kernel hands the count to the host itself (slot[4:6]) when the lists are
     # built by the row / column split; the event behind the plan is the fallback
@@ -1154,125 +1167,6 @@ def _n_isects_arg(isect_offsets: Tensor, flatten_ids: Tensor, total_follows: boo
     return -1
 
 
-class LidarFrame:
-    """A lidar frame enqueued by :func:`lidar_frame_fwd`: the outputs are on their way, the
-    intersection count arrives in a pinned slot. ``finish()`` waits for the count and returns the
-    exact-length (isect_ids, flatten_ids), or None when the count outgrew the room the frame was
-    given (the frame then has to be rendered the ordinary way)."""
-
-    def __init__(self, tensors, capacity, counted, slot, key, sequence, ranged=False):
-        self.__dict__.update(tensors)
-        self._capacity, self._counted, self._slot, self._key = capacity, counted, slot, key
-        self._sequence, self._ranged = sequence, ranged
-
-    def finish(self):
-        n_isects, status = _lib.wait_for_count(self._slot, self._sequence, self._counted)
-        depth_range = _lib.early_depth_range(self._slot, self._sequence)
-        _lib.release_pinned_slot(self._slot)
-        if status & 2 or n_isects > 0x7FFFFFFF:
-            raise RuntimeError(f"isect: {n_isects} intersections do not fit int32 flatten ids / offsets")
-        _isect_count_hint[self._key] = n_isects
-        if status & 4:
-            if self._ranged:
-                # an end bucket overflowed under the depth range carried over from the last frame:
-                # the frame is rendered again without one
-                _depth_range_hint.pop(self._key, None)
-            else:
-                _depth_sort_mode[self._key] = 2   # crowded depth buckets: this shape takes the radix sort from now on
-            return None
-        if depth_range is not None:
-            _depth_range_hint[self._key] = depth_range
-        if n_isects > self._capacity:
-            return None
-        isect_ids = self.isect_buf[:n_isects]
-        isect_ids._splatad_tile_offsets = (self.C, self.offsets_buf[:-1])
-        return isect_ids, self.flatten_buf[:n_isects]
-
-
-@torch.no_grad()
-def lidar_frame_fwd(means, quats, scales, velocities, opacities_cn, lidar_features, viewmats, linear_velocity,
-                    angular_velocity, rolling_shutter_time, raster_pts, tile_elevation_boundaries,
-                    azimuth_resolution, tile_width, tile_height, min_azimuth, max_azimuth, min_elevation,
-                    max_elevation, eps2d, near_plane, far_plane, radius_clip, compute_alpha_sum,
-                    alpha_sum_threshold, expected_grid=None) -> Optional["LidarFrame"]:
-    """Forward pass of a whole lidar frame (projection, tile intersection, compositing) through ONE
-    library call (``splatad_lidar_frame_fwd``), for frames that need no gradients: the host work
-    between the 22 launches of a frame, not the GPU, is what limits the frame rate of small frames.
-    Needs the intersection count of an earlier frame of the same shape on this stream to size the
-    lists (returns None when there is none yet: render that frame with the individual ops).
-    Not part of the reference's API; used by ``splatad_b200.lidar_rasterization``."""
-    C, N = viewmats.shape[0], means.shape[0]
-    D = lidar_features.shape[-1]
-    dev = means.device
-    if C * N == 0 or D + 1 > _lib.MAX_CHANNELS:
-        return None
-    lib = _lib.load()
-    eb = _f(tile_elevation_boundaries)
-    n_rows = int(eb.numel()) - 1
-    tile_az = float(azimuth_resolution) * int(tile_width)
-    n_cols = int(lib.splatad_lidar_azimuth_tiles(tile_az))
-    if expected_grid is not None and tuple(expected_grid) != (n_rows, n_cols):
-        return None   # the caller's tile grid is not the one the intersection builds
-    n_tiles_total = C * n_cols * n_rows
-    stream = _lib.stream_ptr(dev)
-    key = ("lidar_tiles", C, N, C * N, n_tiles_total, dev.index, int(stream))
-    hint = _isect_count_hint.get(key)
-    if hint is None or _depth_sort_mode.get(key, 1) != 1:
-        return None
-    capacity = hint + hint // 8 + 65536
-    H, W = raster_pts.shape[1:3]
-    f32 = dict(dtype=torch.float32, device=dev)
-    i32 = dict(dtype=torch.int32, device=dev)
-    t = dict(
-        C=C, grid=(n_rows, n_cols),
-        radii=torch.empty((C, N, 2), **f32), means2d=torch.empty((C, N, 2), **f32),
-        depths=torch.empty((C, N), **f32), conics=torch.empty((C, N, 3), **f32),
-        pix_vels=torch.empty((C, N, 3), **f32), depth_compensations=torch.empty((C, N, 2), **f32),
-        tiles_per_gauss=torch.empty((C, N), **i32),
-        isect_buf=torch.empty(capacity, dtype=torch.int64, device=dev), flatten_buf=torch.empty(capacity, **i32),
-        offsets_buf=torch.empty(n_tiles_total + 1, **i32),
-        render=torch.empty((C, H, W, D + 1), **f32), alphas=torch.empty((C, H, W, 1), **f32),
-        alpha_sum=torch.empty((C, H, W, 1), **f32) if compute_alpha_sum else None,
-        last_ids=torch.empty((C, H, W), **i32), median_depths=torch.empty((C, H, W, 1), **f32),
-    )
-    plan_ws = _lib.workspace("isect_plan", lib.splatad_isect_plan_workspace_bytes(C * N), dev)
-    fill_ws = _lib.workspace("isect_fill", lib.splatad_isect_fill_workspace_bytes(capacity), dev)
-    slot = _lib.acquire_pinned_slot(dev)
-    sequence = _lib.next_sequence()   # the count kernel stores the count + this number into slot[4:6]
-    # the depth range of the last frame of this shape, widened by a tenth on either side, spans this
-    # frame's depth buckets: the rectangle count then fills them and one kernel less is launched
-    ranged = False
-    last_range = _depth_range_hint.get(key)
-    if last_range is not None:
-        lo, hi = (struct.unpack("<f", struct.pack("<I", b))[0] for b in last_range)
-        if 0.0 <= lo <= hi < float("inf"):
-            pad = 0.1 * (hi - lo) + 1e-3
-            lo_bits, hi_bits = (struct.unpack("<I", struct.pack("<f", v))[0] for v in (max(lo - pad, 0.0), hi + pad))
-            lib.splatad_isect_set_depth_range_hint(lo_bits, hi_bits)
-            ranged = True
-    p = _lib.ptr
-    try:
-        _call("splatad_lidar_frame_fwd", C, N, p(_f(means)), p(_f(quats)), p(_f(scales)), p(_f(velocities)),
-              p(_f(opacities_cn)), p(_f(lidar_features)), D, p(_f(viewmats)), p(_f(linear_velocity)),
-              p(_f(angular_velocity)), p(_f(rolling_shutter_time)), p(_f(raster_pts)), W, H, p(eb), n_rows + 1,
-              float(azimuth_resolution), int(tile_width), int(tile_height), float(min_azimuth), float(max_azimuth),
-              float(min_elevation), float(max_elevation), float(eps2d), float(near_plane), float(far_plane),
-              float(radius_clip), int(bool(compute_alpha_sum)), float(alpha_sum_threshold), p(t["radii"]),
-              p(t["means2d"]), p(t["depths"]), p(t["conics"]), p(t["pix_vels"]), p(t["depth_compensations"]),
-              p(t["tiles_per_gauss"]), capacity, p(t["isect_buf"]), p(t["flatten_buf"]), p(t["offsets_buf"]),
-              p(t["render"]), p(t["alphas"]), p(t["alpha_sum"]), p(t["last_ids"]), p(t["median_depths"]),
-              p(plan_ws), plan_ws.numel(), p(fill_ws), fill_ws.numel(), slot.data_ptr(), slot.data_ptr() + 32, sequence,
-              stream)
-    except BaseException:
-        if ranged:
-            lib.splatad_isect_set_depth_range_hint(1, 0)   # disarm: no later plan of this thread inherits the range
-        _lib.release_pinned_slot(slot)
-        raise
-    counted = torch.cuda.Event()      # fallback: the counters the plan copies at its end
-    counted.record(torch.cuda.current_stream(dev))
-    return LidarFrame(t, capacity, counted, slot, key, sequence, ranged)
-
-
 @torch.no_grad()
 def isect_tiles(
     means2d: Tensor,  # [C, N, 2] or [nnz, 2]
@@ -1380,6 +1274,10 @@ def map_points_to_lidar_tiles(
 
     Returns (tile ids int64 [total] = sensor << 32 | tile, flatten ids int32 [total]), ordered by
     tile id (ties in point order) when ``sort``."""
+    if not packed and not _lib.DEBUG:
+        out = _lib.host().map_points(points2d, elev_boundaries, tile_azim_resolution, min_azim, sort)
+        if out is not None:
+            return out
     if packed:
         nnz = points2d.size(0)
         assert points2d.shape == (nnz, 2), points2d.size()
@@ -1409,6 +1307,10 @@ def map_points_to_lidar_tiles(
 def points_mapping_offset_encode(point_ids: Tensor, n_lidars: int, tile_width: int, tile_height: int) -> Tensor:
     """Sorted point tile ids -> start of every tile's list, [C, tile_height, tile_width] int32
     (gsplat/cuda/_wrapper.py:760-776)."""
+    if not _lib.DEBUG:
+        out = _lib.host().encode_points(point_ids, n_lidars, tile_width, tile_height)
+        if out is not None:
+            return out
     point_ids = point_ids.contiguous()
     dev = point_ids.device
     offsets = torch.empty((n_lidars, tile_height, tile_width), dtype=torch.int32, device=dev)
@@ -1432,6 +1334,10 @@ def populate_image_from_points(
     """Raster image [C, image_height, image_width, 5] whose pixels take the values of the points
     listed for their tile, in list order (gsplat/cuda/_wrapper.py:778-809)."""
     assert points.shape[-1] == 5, points.shape
+    if not _lib.DEBUG:
+        out = _lib.host().populate_image(points, image_width, image_height, tile_width, tile_height, tile_offsets, flatten_id)
+        if out is not None:
+            return out
     pts = _f(points)
     dev = pts.device
     C, grid_h, grid_w = tile_offsets.shape
@@ -1668,7 +1574,7 @@ def rasterize_to_points_split(
     pix_vels: Tensor, depth_compensations: Tensor, raster_pts: Tensor, image_width: int, image_height: int,
     tile_width: int, tile_height: int, isect_offsets: Tensor, flatten_ids: Tensor,
     compute_alpha_sum_until_points: bool, compute_alpha_sum_until_points_threshold: float,
-    absgrad: bool = False, total_follows: bool = False, frame: Optional["LidarFrame"] = None,
+    absgrad: bool = False, total_follows: bool = False,
 ) -> Tuple[Tensor, Tensor, Optional[Tensor], Tensor]:
     """:func:`rasterize_to_points` with the Gaussians' ranges given as their own [C,N] tensor instead
     of being concatenated to the features as last channel (what ``lidar_rasterization`` of the
@@ -1681,7 +1587,7 @@ def rasterize_to_points_split(
         opacities.contiguous(), pix_vels.contiguous(), depth_compensations.contiguous(), None,
         raster_pts.contiguous(), image_width, image_height, tile_width, tile_height,
         isect_offsets.contiguous(), flatten_ids.contiguous(), compute_alpha_sum_until_points,
-        compute_alpha_sum_until_points_threshold, absgrad, lidar_features.shape[-1], total_follows, frame)
+        compute_alpha_sum_until_points_threshold, absgrad, lidar_features.shape[-1], total_follows)
 
 
 class _RasterizeToPoints(torch.autograd.Function):
@@ -1689,9 +1595,7 @@ class _RasterizeToPoints(torch.autograd.Function):
     def forward(ctx, means2d, conics, colors, ranges, opacities, pix_vels, depth_compensations, backgrounds,
                 raster_pts, width, height, tile_width, tile_height, isect_offsets, flatten_ids,
                 compute_alpha_sum_until_points, compute_alpha_sum_until_points_threshold, absgrad,
-                depth_channel_idx, total_follows=False, frame=None):
-        # ``frame`` (optional): a LidarFrame that has composited exactly these inputs over exactly
-        # these lists; its images are returned with this op's backward attached, nothing is launched.
+                depth_channel_idx, total_follows=False):
         # ``ranges`` (optional, [C,N] / [nnz]): the Gaussians' ranges as a separate array; the rendered
         # channel count is then colors.shape[-1] + 1 with the range as last channel.
         dev = means2d.device
@@ -1704,26 +1608,21 @@ class _RasterizeToPoints(torch.autograd.Function):
         f32 = dict(dtype=torch.float32, device=dev)
         ctx.n_isects_arg = _n_isects_arg(isect_offsets, flatten_ids, total_follows)
         _debug_check_lists("rasterize_to_points", flatten_ids, means2d.numel() // 2, isect_offsets, total_follows)
-        if frame is not None:
-            render_colors, render_alphas, median_depths = frame.render, frame.alphas, frame.median_depths
-            alpha_sum, last_ids = frame.alpha_sum, frame.last_ids
-            assert render_colors.shape == (C, height, width, channels) and ranges is not None and bg is None
-        else:
-            render_colors = torch.empty((C, height, width, channels), **f32)
-            render_alphas = torch.empty((C, height, width, 1), **f32)
-            median_depths = torch.empty((C, height, width, 1), **f32)
-            alpha_sum = torch.empty((C, height, width, 1), **f32) if compute_alpha_sum_until_points else None
-            last_ids = torch.empty((C, height, width), dtype=torch.int32, device=dev)
-            _call(
-                "splatad_rasterize_to_points_fwd", C, ctx.n_isects_arg, _lib.ptr(means2d),
-                _lib.ptr(conics_f), _lib.ptr(colors_f) if colors_f.numel() else None, _lib.ptr(ranges_f), channels,
-                _lib.ptr(opac_f), _lib.ptr(vels_f),
-                _lib.ptr(dc_f), _lib.ptr(bg), _lib.ptr(pts_f), width, height, tile_width, tile_height,
-                grid_w, grid_h, int(bool(compute_alpha_sum_until_points)),
-                float(compute_alpha_sum_until_points_threshold), _lib.ptr(isect_offsets),
-                _lib.ptr(flatten_ids), depth_channel_idx, _lib.ptr(render_colors), _lib.ptr(render_alphas),
-                _lib.ptr(alpha_sum), _lib.ptr(last_ids), _lib.ptr(median_depths), _lib.stream_ptr(dev),
-            )
+        render_colors = torch.empty((C, height, width, channels), **f32)
+        render_alphas = torch.empty((C, height, width, 1), **f32)
+        median_depths = torch.empty((C, height, width, 1), **f32)
+        alpha_sum = torch.empty((C, height, width, 1), **f32) if compute_alpha_sum_until_points else None
+        last_ids = torch.empty((C, height, width), dtype=torch.int32, device=dev)
+        _call(
+            "splatad_rasterize_to_points_fwd", C, ctx.n_isects_arg, _lib.ptr(means2d),
+            _lib.ptr(conics_f), _lib.ptr(colors_f) if colors_f.numel() else None, _lib.ptr(ranges_f), channels,
+            _lib.ptr(opac_f), _lib.ptr(vels_f),
+            _lib.ptr(dc_f), _lib.ptr(bg), _lib.ptr(pts_f), width, height, tile_width, tile_height,
+            grid_w, grid_h, int(bool(compute_alpha_sum_until_points)),
+            float(compute_alpha_sum_until_points_threshold), _lib.ptr(isect_offsets),
+            _lib.ptr(flatten_ids), depth_channel_idx, _lib.ptr(render_colors), _lib.ptr(render_alphas),
+            _lib.ptr(alpha_sum), _lib.ptr(last_ids), _lib.ptr(median_depths), _lib.stream_ptr(dev),
+        )
         ctx.save_for_backward(means2d, conics_f, colors_f, ranges_f, opac_f, vels_f, dc_f, bg, pts_f,
                               isect_offsets, flatten_ids, render_alphas, last_ids)
         ctx.meta = (width, height, tile_width, tile_height, absgrad,
@@ -1763,7 +1662,7 @@ class _RasterizeToPoints(torch.autograd.Function):
         if ctx.needs_input_grad[7]:
             v_backgrounds = (v_render_colors * (1.0 - render_alphas).float()).sum(dim=(1, 2))
         return (v_means2d, v_conics, v_colors, v_ranges, v_opacities, v_pix_vels, v_depth_comps,
-                v_backgrounds) + (None,) * 13
+                v_backgrounds) + (None,) * 12
 
 
 # =============================================================================================
