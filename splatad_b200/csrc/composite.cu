@@ -649,6 +649,183 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
 }
 
 // ---------------------------------------------------------------------------------------
+// Lidar forward for few patches: all warps of a CTA work on ONE patch, a share of the entries each. What
+// depends on the order - the transmittance, where a point stops, its median - stays one chain per point,
+// with the same operations as above, but it is all that is left in the chain:
+//   1. every warp evaluates its share of the entries, alphas and range terms to shared memory;
+//   2. one warp runs down the alphas: transmittance, weights (left in the alphas' place), median, sums;
+//   3. every warp adds the features of its share, and the partial sums are added at the end.
+// A 32 x 512 scan has 512 patches of up to 300 relevant entries: 124 -> 65 us.
+// ---------------------------------------------------------------------------------------
+constexpr uint32_t kCoopWarps = 8, kCoopChunk = 32;
+
+template <int CDIM>
+__global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_to_points_fwd_coop_kernel(
+    uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
+    const float *__restrict__ conics, const float *__restrict__ colors,
+    const float *__restrict__ ranges, uint32_t channels,
+    const float *__restrict__ opacities, const float *__restrict__ pix_vels /* [.,3] */,
+    const float2 *__restrict__ depth_comps, const float *__restrict__ backgrounds,
+    const float4 *__restrict__ raster_pts, uint32_t W, uint32_t H, uint32_t tile_width,
+    uint32_t tile_height, uint32_t grid_w, uint32_t grid_h, uint32_t patches_per_tile, int compute_alpha_sum,
+    float alpha_sum_threshold, const int32_t *__restrict__ offsets,
+    const int32_t *__restrict__ flatten_ids, uint32_t depth_idx,
+    float *__restrict__ render_colors, float *__restrict__ render_alphas,
+    float *__restrict__ alpha_sum_out, int32_t *__restrict__ last_ids,
+    float *__restrict__ median_depths) {
+    constexpr uint32_t kThreadsC = kCoopWarps * 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ PointBox s_box;
+    __shared__ uint32_t s_warp_kept[kCoopWarps];
+    __shared__ int s_done;
+    float4 *sA = reinterpret_cast<float4 *>(smem_raw);
+    float4 *sB = sA + kThreadsC;
+    float4 *sC = sB + kThreadsC;
+    float *sFeat = reinterpret_cast<float *>(sC + kThreadsC);               // [kThreadsC * CDIM]
+    float *sAlpha = sFeat + kThreadsC * CDIM;                               // [2][kCoopChunk][32] alphas, then weights
+    float *sTerm = sAlpha + 2 * kCoopChunk * 32;                            // [2][kCoopChunk][32] range terms
+    int32_t *sPos = reinterpret_cast<int32_t *>(sTerm + 2 * kCoopChunk * 32);
+
+    const uint32_t tiles_per_cam = grid_w * grid_h;
+    const uint32_t gtile = blockIdx.x / patches_per_tile, part = blockIdx.x - gtile * patches_per_tile;
+    const uint32_t cam = gtile / tiles_per_cam;
+    const uint32_t tile = gtile - cam * tiles_per_cam;
+    const uint32_t ty = tile / grid_w, tx = tile - ty * grid_w;
+    const uint32_t tr = threadIdx.x, lane = tr & 31u, warp = tr >> 5;
+    const uint32_t index = part * 32u + lane;   // every warp holds the same points
+    const PointPatch pp = point_patch<1>(tile_width, tile_height, index);
+    const uint32_t i = ty * tile_height + pp.row, j = tx * tile_width + pp.col;
+    const bool in_image = index < tile_width * tile_height && i < H && j < W;
+    bool inside = in_image;
+    const size_t pix = ((size_t)cam * H + i) * W + j;
+    float px = 0.f, py = 0.f, pz = 0.f, roll = 0.f;
+    if (inside) {
+        const float4 rp = raster_pts[pix];
+        px = rp.x; py = rp.y; pz = rp.z; roll = rp.w;
+        if (pz <= 0.f) inside = false;
+    }
+    PointExtent extent;
+    if (inside) extent.add(px, py, roll);
+    if (warp == 0) extent.write_box(&s_box);
+    if (tr == 0) s_done = 0;
+    // the points are an input of the frame; everything below comes from the kernels before this one
+    chain_enter();
+
+    const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
+    const uint32_t num_batches = (uint32_t)(range.end - range.start + kThreadsC - 1) / kThreadsC;
+    const uint32_t fstride = ranges ? channels - 1 : channels;
+    const bool vec = (fstride % 4u == 0u) && ((reinterpret_cast<uintptr_t>(colors) & 15u) == 0u);
+    // the chain, held by the first warp
+    bool done = !inside;
+    float T = 1.f, depth_extra = 0.f, alpha_sum = 0.f, median = 0.f;
+    int32_t cur_idx = 0;
+    const float alpha_sum_limit = pz - alpha_sum_threshold;
+    float pix_out[CDIM];
+#pragma unroll
+    for (int k = 0; k < CDIM; ++k) pix_out[k] = 0.f;
+
+    int32_t next_id = range.start + (int32_t)tr < range.end ? flatten_ids[range.start + tr] : 0;
+    bool finished = __all_sync(0xffffffffu, !inside);   // the same in every warp
+    uint32_t buffer = 0;
+    for (uint32_t b = 0; b < num_batches && !finished; ++b) {
+        const int32_t idx = range.start + (int32_t)(kThreadsC * b + tr);
+        const int32_t g = next_id;
+        PointEntry e;
+        if (idx < range.end) {
+            e = load_point_entry(g, means2d, conics, opacities, pix_vels, depth_comps);
+            e.C.w = ranges ? __ldg(ranges + g) : __ldg(colors + (size_t)g * channels + depth_idx);
+            if (idx + (int32_t)kThreadsC < range.end) next_id = flatten_ids[idx + kThreadsC];   // on its way meanwhile
+        }
+        __syncthreads();   // the batch before has been read; the box and the flag have been written
+        const bool seen = idx < range.end && boxes_that_see(e, &s_box, 1u) != 0u;
+        const uint32_t kept = __ballot_sync(0xffffffffu, seen);
+        if (lane == 0) s_warp_kept[warp] = __popc(kept);
+        __syncthreads();
+        uint32_t n_kept = 0, pos = __popc(kept & ((1u << lane) - 1u));
+#pragma unroll
+        for (uint32_t w = 0; w < kCoopWarps; ++w) {
+            if (w == warp) pos += n_kept;
+            n_kept += s_warp_kept[w];
+        }
+        if (seen) {
+            sA[pos] = e.A;
+            sB[pos] = e.B;
+            sC[pos] = e.C;
+            sPos[pos] = idx;
+            stage_features<CDIM>(sFeat + pos * CDIM, colors, (size_t)g, fstride, vec, ranges != nullptr, e.C.w);
+        }
+        __syncthreads();
+        for (uint32_t c0 = 0; c0 < n_kept && !finished; c0 += kCoopChunk) {
+            const uint32_t n = min(kCoopChunk, n_kept - c0);
+            float *al = sAlpha + buffer * kCoopChunk * 32, *dt = sTerm + buffer * kCoopChunk * 32;
+            buffer ^= 1u;
+            for (uint32_t q = warp; q < n; q += kCoopWarps) {
+                const uint32_t t = c0 + q;
+                const float4 A = sA[t], B = sB[t], Cc = sC[t];
+                const PointFootprint f = point_footprint(A, B, roll, px, py);
+                const float alpha = fminf(kAlphaMax, B.w * f.vis);
+                al[q * 32 + lane] = f.sigma < 0.f || alpha < kAlphaMin ? 0.f : alpha;
+                dt[q * 32 + lane] = Cc.y * f.dx + Cc.z * f.dy + Cc.x * roll;
+            }
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll 4
+                for (uint32_t q = 0; q < n; ++q) {
+                    const float alpha = al[q * 32 + lane], dterm = dt[q * 32 + lane], range_q = sC[c0 + q].w;
+                    const float next_T = T * (1.f - alpha), vis = alpha * T;
+                    if (alpha > 0.f && next_T <= kTStop) done = true;
+                    const bool take = alpha > 0.f && !done;
+                    if (take) {
+                        depth_extra += dterm * vis;
+                        if (T > 0.5f && next_T <= 0.5f) median = range_q + dterm;
+                        if (compute_alpha_sum && range_q < alpha_sum_limit) alpha_sum += alpha;
+                        cur_idx = sPos[c0 + q];
+                        T = next_T;
+                    }
+                    al[q * 32 + lane] = take ? vis : 0.f;
+                }
+                if (__all_sync(0xffffffffu, done) && lane == 0) s_done = 1;
+            }
+            __syncthreads();
+            finished = s_done != 0;
+            for (uint32_t q = warp; q < n; q += kCoopWarps) {
+                const float vis = al[q * 32 + lane];
+                if (__any_sync(0xffffffffu, vis != 0.f)) axpy_staged_full<CDIM>(pix_out, sFeat + (c0 + q) * CDIM, vis);
+            }
+        }
+    }
+    // partial sums of the warps, added in order
+    __syncthreads();
+    float *parts = reinterpret_cast<float *>(smem_raw);   // [warps][32][CDIM]
+#pragma unroll
+    for (int k = 0; k < CDIM; k += 4)
+        *reinterpret_cast<float4 *>(parts + (warp * 32 + lane) * CDIM + k) =
+            make_float4(pix_out[k], pix_out[k + 1], pix_out[k + 2], pix_out[k + 3]);
+    float *s_T = parts + kCoopWarps * 32 * CDIM, *s_extra = s_T + 32;
+    if (warp == 0) {
+        s_T[lane] = T;
+        s_extra[lane] = depth_extra;
+        if (in_image) {
+            // points that are not rendered (range <= 0) produce zeros everywhere
+            render_alphas[pix] = inside ? 1.f - T : 0.f;
+            last_ids[pix] = inside ? cur_idx : 0;
+            median_depths[pix] = inside ? median : 0.f;
+            if (alpha_sum_out != nullptr) alpha_sum_out[pix] = inside ? alpha_sum : 0.f;
+        }
+    }
+    __syncthreads();
+    const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
+    for (uint32_t k = warp; k < channels; k += kCoopWarps) {
+        float v = 0.f;
+#pragma unroll
+        for (uint32_t w = 0; w < kCoopWarps; ++w) v += parts[(w * 32 + lane) * CDIM + k];
+        if (k == depth_idx) v += s_extra[lane];
+        if (bg) v += s_T[lane] * bg[k];
+        if (in_image) render_colors[pix * channels + k] = inside ? v : 0.f;
+    }
+}
+
+// ---------------------------------------------------------------------------------------
 // Backward helpers
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ float warp_sum(float v) {
@@ -1013,8 +1190,10 @@ __device__ __forceinline__ GradSlot point_grad_slot(int slot, int cdim, uint32_t
     }
 }
 
+constexpr uint32_t kPointsBwdStage = 2;   // entries per thread and batch: their loads overlap
+
 template <int CDIM, bool kAbs>
-__global__ void __launch_bounds__(256) rasterize_to_points_bwd_kernel(
+__global__ void __launch_bounds__(256, CDIM <= 20 ? 2 : 1) rasterize_to_points_bwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors,
     const float *__restrict__ ranges, uint32_t channels,
@@ -1031,17 +1210,17 @@ __global__ void __launch_bounds__(256) rasterize_to_points_bwd_kernel(
     float *__restrict__ v_opacities, float *__restrict__ v_pix_vels,
     float *__restrict__ v_depth_comps, float *__restrict__ v_ranges) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int red[32];
-    __shared__ PointBox s_box[8];
-    __shared__ uint32_t s_warp_kept[8];
-    const uint32_t bs = blockDim.x;
+    __shared__ PointBox s_box;
+    constexpr uint32_t kStage = kPointsBwdStage;
+    __shared__ uint32_t s_warp_kept[kStage * 8];
+    const uint32_t bs = blockDim.x, cap = kStage * bs;
     float4 *sA = reinterpret_cast<float4 *>(smem_raw);
-    float4 *sB = sA + bs;
-    float4 *sC = sB + bs;   // range velocity, depth compensation (2), range
-    float *sRgb = reinterpret_cast<float *>(sC + bs);                  // [bs * CDIM], zeros behind the channels
-    int32_t *sId = reinterpret_cast<int32_t *>(sRgb + bs * CDIM);
-    int32_t *sPos = sId + bs;
-    uint32_t *sSeen = reinterpret_cast<uint32_t *>(sPos + bs);
+    float4 *sB = sA + cap;
+    float4 *sC = sB + cap;   // range velocity, depth compensation (2), range
+    float *sRgb = reinterpret_cast<float *>(sC + cap);                 // [cap * CDIM], zeros behind the channels
+    int32_t *sId = reinterpret_cast<int32_t *>(sRgb + cap * CDIM);
+    int32_t *sPos = sId + cap;
+    float4 *sSeg = reinterpret_cast<float4 *>(sPos + cap);   // [warps][32] what a segment does to its two points
 
     const uint32_t tiles_per_cam = grid_w * grid_h;
     const uint32_t gtile = blockIdx.x / ctas_per_tile, part = blockIdx.x - gtile * ctas_per_tile;
@@ -1049,8 +1228,7 @@ __global__ void __launch_bounds__(256) rasterize_to_points_bwd_kernel(
     const uint32_t tile = gtile - cam * tiles_per_cam;
     const uint32_t ty = tile / grid_w, tx = tile - ty * grid_w;
     const uint32_t tr = threadIdx.x, lane = tr & 31u, warp = tr >> 5, n_warps = bs >> 5;
-    const uint32_t index = part * bs + tr;
-    const PointPatch pp = point_patch<2>(tile_width, tile_height, index);
+    const PointPatch pp = point_patch<2>(tile_width, tile_height, part * 32u + lane);   // every warp holds the same points
 
     const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
     const uint32_t fstride = ranges ? channels - 1 : channels;
@@ -1093,14 +1271,12 @@ __global__ void __launch_bounds__(256) rasterize_to_points_bwd_kernel(
         if (h) { az.y = rp.x; el.y = rp.y; roll.y = rp.w; T.y = T_final; behind.y = last; v_depth.y = vd; v_asum.y = vs; sum_limit.y = limit; }
         else { az.x = rp.x; el.x = rp.y; roll.x = rp.w; T.x = T_final; behind.x = last; v_depth.x = vd; v_asum.x = vs; sum_limit.x = limit; }
     }
-    extent.write_box(s_box + warp);
+    if (warp == 0) extent.write_box(&s_box);
 
-    // last list position consumed by any point of this CTA / warp
-    const int32_t cta_last = block_max_int(thread_last, red);
-    const int32_t warp_last = __reduce_max_sync(0xffffffffu, thread_last);
-    const int32_t eff_end = min(range.end, cta_last + 1);
+    // last list position consumed by any of the patch's points
+    const int32_t eff_end = min(range.end, __reduce_max_sync(0xffffffffu, thread_last) + 1);
     if (eff_end <= range.start) return;
-    const uint32_t num_batches = (uint32_t)(eff_end - range.start + bs - 1) / bs;
+    const uint32_t num_batches = (uint32_t)(eff_end - range.start + cap - 1) / cap;
 
     constexpr int kGeo = kAbs ? 13 : 11;
     constexpr int kSlots = CDIM + kGeo <= 16 ? 16 : 32;
@@ -1110,63 +1286,118 @@ __global__ void __launch_bounds__(256) rasterize_to_points_bwd_kernel(
                                                   v_opacities, v_means2d_abs);
     const bool writes_a = kSlots == 32 || (lane & 1u) == 0u;
 
-    int32_t next_id = 0;
-    {
-        const int32_t idx = eff_end - 1 - (int32_t)tr;
-        if (idx >= range.start) next_id = flatten_ids[idx];
+    int32_t next_id[kStage];
+#pragma unroll
+    for (uint32_t q = 0; q < kStage; ++q) {
+        const int32_t idx = eff_end - 1 - (int32_t)(q * bs + tr);
+        next_id[q] = idx >= range.start ? flatten_ids[idx] : 0;
     }
     for (uint32_t b = 0; b < num_batches; ++b) {
-        const int32_t idx = eff_end - 1 - (int32_t)(bs * b) - (int32_t)tr;
-        const int32_t g = next_id;
-        PointEntry e;
-        uint32_t seen = 0u;
-        if (idx >= range.start) {
-            e = load_point_entry(g, means2d, conics, opacities, pix_vels, depth_comps);
-            e.C.w = ranges ? __ldg(ranges + g) : __ldg(colors + (size_t)g * channels + depth_idx);
-            const int32_t ahead = idx - (int32_t)bs;   // the id of the next batch's entry is on its way meanwhile
-            if (ahead >= range.start) next_id = flatten_ids[ahead];
-            seen = boxes_that_see(e, s_box, n_warps);
+        const int32_t batch_end = eff_end - 1 - (int32_t)(cap * b);
+        PointEntry e[kStage];
+        int32_t g[kStage];
+        uint32_t kept[kStage];
+        bool seen[kStage];
+#pragma unroll
+        for (uint32_t q = 0; q < kStage; ++q) {
+            const int32_t idx = batch_end - (int32_t)(q * bs + tr), ahead = idx - (int32_t)cap;
+            g[q] = next_id[q];
+            if (idx >= range.start) {
+                e[q] = load_point_entry(g[q], means2d, conics, opacities, pix_vels, depth_comps);
+                e[q].C.w = ranges ? __ldg(ranges + g[q]) : __ldg(colors + (size_t)g[q] * channels + depth_idx);
+            }
+            if (ahead >= range.start) next_id[q] = flatten_ids[ahead];   // on its way meanwhile
         }
+        __syncthreads();   // the batch before has been read; the box has been written
         // survivors to the front, still back to front in list order
-        const uint32_t kept_mask = __ballot_sync(0xffffffffu, seen != 0u);
-        __syncthreads();   // the batch before has been read
-        if (lane == 0) s_warp_kept[warp] = __popc(kept_mask);
-        __syncthreads();
-        uint32_t pos = __popc(kept_mask & ((1u << lane) - 1u)), n_kept = 0;
-        for (uint32_t w = 0; w < n_warps; ++w) {
-            const uint32_t cnt = s_warp_kept[w];
-            if (w < warp) pos += cnt;
-            n_kept += cnt;
-        }
-        if (seen) {
-            sA[pos] = e.A;
-            sB[pos] = e.B;
-            sC[pos] = e.C;
-            sId[pos] = g;
-            sPos[pos] = idx;
-            sSeen[pos] = seen;
-            stage_features<CDIM>(sRgb + pos * CDIM, colors, (size_t)g, fstride, vec, ranges != nullptr, e.C.w);
+#pragma unroll
+        for (uint32_t q = 0; q < kStage; ++q) {
+            seen[q] = batch_end - (int32_t)(q * bs + tr) >= range.start && boxes_that_see(e[q], &s_box, 1u) != 0u;
+            kept[q] = __ballot_sync(0xffffffffu, seen[q]);
+            if (lane == 0) s_warp_kept[q * n_warps + warp] = __popc(kept[q]);
         }
         __syncthreads();
-        for (uint32_t t0 = 0; t0 < n_kept; t0 += 32) {
-            const uint32_t mine = t0 + lane;
-            uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u) && sPos[mine] <= warp_last);
-            while (todo) {
-                const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
-                todo &= todo - 1u;
-                const float4 A = sA[t], B = sB[t];
-                const int32_t entry = sPos[t];
-                const PointFootprint f0 = point_footprint(A, B, roll.x, az.x, el.x), f1 = point_footprint(A, B, roll.y, az.y, el.y);
-                const float a0 = fminf(kAlphaMax, B.w * f0.vis), a1 = fminf(kAlphaMax, B.w * f1.vis);
-                const bool ok0 = entry <= bin_final[0] && !(f0.sigma < 0.f || a0 < kAlphaMin);
-                const bool ok1 = entry <= bin_final[1] && !(f1.sigma < 0.f || a1 < kAlphaMin);
-                if (!__any_sync(0xffffffffu, ok0 || ok1)) continue;
+        uint32_t n_kept = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kStage; ++q) {
+            uint32_t pos = __popc(kept[q] & ((1u << lane) - 1u));
+            for (uint32_t w = 0; w < n_warps; ++w) {
+                if (w == warp) pos += n_kept;
+                n_kept += s_warp_kept[q * n_warps + w];
+            }
+            if (seen[q]) {
+                sA[pos] = e[q].A;
+                sB[pos] = e[q].B;
+                sC[pos] = e[q].C;
+                sId[pos] = g[q];
+                sPos[pos] = batch_end - (int32_t)(q * bs + tr);
+                stage_features<CDIM>(sRgb + pos * CDIM, colors, (size_t)g[q], fstride, vec, ranges != nullptr, e[q].C.w);
+            }
+        }
+        __syncthreads();
+        // The entries are cut into one segment per warp. A warp first runs its segment from T = 1 and nothing
+        // behind it; those products and sums of the segments behind its own are what its second run starts
+        // from, in which the gradients are formed. (One warp per patch: the only segment starts where the
+        // batch before ended.)
+        const uint32_t per = (n_kept + n_warps - 1) / n_warps;
+        const uint32_t t_lo = min(n_kept, warp * per), t_hi = min(n_kept, t_lo + per);
+        const auto evaluate = [&](uint32_t t, float4 &B, float2 &dx, float2 &dy, float2 &vis, float2 &alpha, float2 &open) {
+            const float4 A = sA[t];
+            B = sB[t];
+            const int32_t entry = sPos[t];
+            const PointFootprint f0 = point_footprint(A, B, roll.x, az.x, el.x), f1 = point_footprint(A, B, roll.y, az.y, el.y);
+            const float a0 = fminf(kAlphaMax, B.w * f0.vis), a1 = fminf(kAlphaMax, B.w * f1.vis);
+            const bool ok0 = entry <= bin_final[0] && !(f0.sigma < 0.f || a0 < kAlphaMin);
+            const bool ok1 = entry <= bin_final[1] && !(f1.sigma < 0.f || a1 < kAlphaMin);
+            dx = make_float2(f0.dx, f1.dx);
+            dy = make_float2(f0.dy, f1.dy);
+            vis = make_float2(ok0 ? f0.vis : 0.f, ok1 ? f1.vis : 0.f);
+            alpha = make_float2(ok0 ? a0 : 0.f, ok1 ? a1 : 0.f);
+            // a capped alpha passes no gradient on to the geometry
+            open = make_float2(B.w * f0.vis <= kAlphaMax ? 1.f : 0.f, B.w * f1.vis <= kAlphaMax ? 1.f : 0.f);
+            return ok0 || ok1;
+        };
+        float2 T_batch = T, behind_batch = behind;
+        if (n_warps > 1) {
+            float2 P = make_float2(1.f, 1.f), Q = make_float2(0.f, 0.f);
+            for (uint32_t t = t_lo; t < t_hi; ++t) {
+                float4 B;
+                float2 dx, dy, vis, alpha, open;
+                if (!__any_sync(0xffffffffu, evaluate(t, B, dx, dy, vis, alpha, open))) continue;
                 const float4 Cc = sC[t];
-                const float2 dx = make_float2(f0.dx, f1.dx), dy = make_float2(f0.dy, f1.dy);
-                const float2 vis = make_float2(ok0 ? f0.vis : 0.f, ok1 ? f1.vis : 0.f);
-                const float2 alpha = make_float2(ok0 ? a0 : 0.f, ok1 ? a1 : 0.f);
-                // a capped alpha passes no gradient on to the geometry
-                const float2 open = make_float2(B.w * f0.vis <= kAlphaMax ? 1.f : 0.f, B.w * f1.vis <= kAlphaMax ? 1.f : 0.f);
+                const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
+                P = __fmul2_rn(P, make_float2(1.f / om.x, 1.f / om.y));
+                const float2 dterm = __ffma2_rn(make_float2(Cc.x, Cc.x), roll,
+                                                __ffma2_rn(make_float2(Cc.z, Cc.z), dy, __fmul2_rn(make_float2(Cc.y, Cc.y), dx)));
+                float2 dot = __fmul2_rn(dterm, v_depth);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float2 d2 = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int k = 0; k < CDIM; k += 4) {
+                        const float4 c4 = *reinterpret_cast<const float4 *>(sRgb + t * CDIM + k);
+                        d2 = __ffma2_rn(make_float2(c4.x, c4.y), make_float2(v_out[h][k], v_out[h][k + 1]), d2);
+                        d2 = __ffma2_rn(make_float2(c4.z, c4.w), make_float2(v_out[h][k + 2], v_out[h][k + 3]), d2);
+                    }
+                    if (h) dot.y += d2.x + d2.y; else dot.x += d2.x + d2.y;
+                }
+                Q = __ffma2_rn(__fmul2_rn(alpha, P), dot, Q);
+            }
+            sSeg[warp * 32 + lane] = make_float4(P.x, P.y, Q.x, Q.y);
+            __syncthreads();
+            for (uint32_t w = 0; w < n_warps; ++w) {
+                if (w == warp) { T = T_batch; behind = behind_batch; }
+                const float4 s = sSeg[w * 32 + lane];
+                behind_batch = __ffma2_rn(T_batch, make_float2(s.z, s.w), behind_batch);
+                T_batch = __fmul2_rn(T_batch, make_float2(s.x, s.y));
+            }
+        }
+        {
+            for (uint32_t t = t_lo; t < t_hi; ++t) {
+                float4 B;
+                float2 dx, dy, vis, alpha, open;
+                if (!__any_sync(0xffffffffu, evaluate(t, B, dx, dy, vis, alpha, open))) continue;
+                const float4 Cc = sC[t];
                 const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
                 const float2 ra = make_float2(1.f / om.x, 1.f / om.y);
                 T = __fmul2_rn(T, ra);
@@ -1246,6 +1477,7 @@ __global__ void __launch_bounds__(256) rasterize_to_points_bwd_kernel(
                 }
             }
         }
+        if (n_warps > 1) { T = T_batch; behind = behind_batch; }
     }
 }
 
@@ -1261,11 +1493,16 @@ __global__ void __launch_bounds__(256) rasterize_to_points_bwd_kernel(
         else { CALL(32); }                                                                       \
     } while (0)
 
-// Warps per CTA of the lidar kernels. Two when the tiles fill the machine: a CTA ends with its slowest
-// warp. Four when they do not, where the staging of a batch - which more warps share - is a part of the
-// chain every warp waits for (32 x 512 points: forward 146 us with one warp per CTA, 124 with four).
-static uint32_t point_warps_per_cta(uint64_t tiles, uint32_t warps_per_tile) {
-    return min(tiles * warps_per_tile >= (uint64_t)kNumSMs * 16 ? 2u : 4u, warps_per_tile);
+// Patches below which all warps of a CTA share one in the forward pass: the shared work costs more
+// instructions in all, so the patches must be too few to fill the machine (2176 patches: 53 us apart, 102
+// shared; 512: 124 and 65).
+constexpr uint64_t kCoopPatches = kNumSMs * 8;
+
+// Warps - segments of the list - per patch in the backward pass: every segment is run twice, which pays
+// while the patches alone leave the schedulers waiting on one warp's chain (256 patches: 405 us with one
+// segment, 178 with four, 109 with eight; 1088: 124, 100 and 104; 3648: 172, and 231 with four).
+static uint32_t point_segments(uint64_t patches) {
+    return patches < (uint64_t)kNumSMs * 4 ? 8u : patches < (uint64_t)kNumSMs * 16 ? 4u : 1u;
 }
 
 template <typename K>
@@ -1436,15 +1673,19 @@ extern "C" int splatad_rasterize_to_points_fwd(
     const uint32_t blocks = C * tile_grid_width * tile_grid_height;
     if (blocks == 0 || image_width == 0 || image_height == 0) return SPLATAD_OK;
     const uint32_t warps = div_up(tile_width * tile_height, 32);
-    const uint32_t per_cta = point_warps_per_cta(blocks, warps), parts = div_up(warps, per_cta), bs = 32 * per_cta;
+    const bool coop = (uint64_t)blocks * warps < kCoopPatches;
+    // two warps per CTA otherwise: a CTA ends with its slowest warp
+    const uint32_t per_cta = min(2u, warps), parts = coop ? warps : div_up(warps, per_cta), bs = coop ? kCoopWarps * 32 : 32 * per_cta;
     SPL_REQUIRE((uint64_t)blocks * parts <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_points_fwd: too many tiles");
 #define CALL(D)                                                                                   \
     {                                                                                             \
-        const size_t smem = (size_t)points_fwd_stage(D) * bs *                                    \
-                            (3 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float));       \
-        int rc = set_smem(rasterize_to_points_fwd_kernel<D>, smem, "rasterize_to_points_fwd");    \
+        auto kernel = coop ? rasterize_to_points_fwd_coop_kernel<D> : rasterize_to_points_fwd_kernel<D>; \
+        const size_t smem = (size_t)(coop ? 1 : points_fwd_stage(D)) * bs *                       \
+                                (3 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float)) +  \
+                            (coop ? 4 * kCoopChunk * 32 * sizeof(float) : 0);                     \
+        int rc = set_smem(kernel, smem, "rasterize_to_points_fwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
-        launch_chained(rasterize_to_points_fwd_kernel<D>, blocks * parts, bs, smem, (cudaStream_t)stream, \
+        launch_chained(kernel, blocks * parts, bs, smem, (cudaStream_t)stream,                    \
             C, n_isects, (const float2 *)means2d, conics, lidar_features, gaussian_ranges,        \
             channels, opacities,                                                                  \
             pix_vels, (const float2 *)depth_compensations, backgrounds,                           \
@@ -1497,13 +1738,13 @@ extern "C" int splatad_rasterize_to_points_bwd(
                 "rasterize_to_points_bwd: a tile of %u points (%u threads at one per point) with %u channels is more "
                 "than the backward pass takes: use a smaller tile or at most 16 channels per call",
                 tile_width * tile_height, samples, channels);
-    const uint32_t warps = div_up(tile_width * tile_height, 64);
-    const uint32_t per_cta = point_warps_per_cta(blocks, warps), parts = div_up(warps, per_cta), bs = 32 * per_cta;
+    const uint32_t parts = div_up(tile_width * tile_height, 64), bs = 32 * point_segments((uint64_t)blocks * parts);
     SPL_REQUIRE((uint64_t)blocks * parts <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_points_bwd: too many tiles");
 #define CALL_ABS(D, A)                                                                            \
     {                                                                                             \
         auto kernel = rasterize_to_points_bwd_kernel<D, A>;                                       \
-        const size_t smem = (size_t)bs * (3 * sizeof(float4) + 3 * sizeof(int32_t) + D * sizeof(float)); \
+        const size_t smem = (size_t)bs * (sizeof(float4) + kPointsBwdStage *                      \
+                                          (3 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float))); \
         int rc = set_smem(kernel, smem, "rasterize_to_points_bwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
         kernel<<<blocks * parts, bs, smem, (cudaStream_t)stream>>>(                               \
