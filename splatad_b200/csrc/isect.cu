@@ -1026,37 +1026,39 @@ emit_kernel(GridArgs<kLidar> a, EmitArgs e, const uint32_t *__restrict__ eoff,
 // depth-ordered rectangles without ever writing the emission out, in two stable steps.
 //
 //   A. blocks: the tile grid is cut into blocks of 4 x 8 tiles. Every depth-ordered entry appends one
-//              record - the 32-bit mask of the block's tiles it covers, its depth bits and flatten
-//              index - to the list of each block it touches (2.3 records per entry for the lidar
-//              benchmark, 3.1 for the camera's, against 5.9 and 5.2 for whole tile rows). A CTA takes
+//              record - the 32-bit mask of the block's tiles it covers and its place in the depth order
+//              - to the list of each block it touches (2.3 records per entry for the lidar benchmark,
+//              3.1 for the camera's, against 5.9 and 5.2 for whole tile rows). A CTA takes
 //              512 consecutive entries; its warps mark their lanes' blocks in one word per (warp,
 //              block), so that an entry's rank in a block's list is a population count.
-//   B. tiles:  a warp takes 256 records of a block, 32 at a time, one record per lane. A 32 x 32 bit
-//              transpose of the masks gives every lane the records that cover ITS tile: that is the
-//              count. To write, the lanes whose record covers tile t store their entry to consecutive
-//              places of t's list.
+//   B. tiles:  a CTA takes a unit of a block's records, every warp 32 at a time, one record per lane. A
+//              32 x 32 bit transpose of the masks gives every lane the records that cover ITS tile: that
+//              is the count, and, a second time, the order in which the unit's entries are written.
 //
-// Per intersection this costs 2 warp instructions per 32 lanes' worth of output at the lidar
-// benchmark's density (a fifth of a block per record) and 0.5 at the camera rig's (three fifths);
-// walking the row runs of a rectangle output by output, which it replaces, took 6, and the radix
-// passes over (tile, entry) pairs that grids of more than 128 tile rows took before move 44 B per
-// intersection. What bounds it now is the 12 B of every list entry.
+// Walking the row runs of a rectangle output by output, which this replaces, took 6 warp instructions per
+// 32 outputs' lane, and the radix passes over (tile, entry) pairs that grids of more than 128 tile rows took
+// before move 44 B per intersection (14 of the 17 ms of six cameras' frame). What bounds it now is the 12 B
+// of every list entry, written at 4.3 TB/s where the lists are long (a fill: 7.5).
 // Positions are exclusive sums over (earlier tiles, earlier units, earlier CTAs, lower lanes), all of
 // them plain scans: the result is the same for any scheduling, and no block waits for another.
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t kBlkW = 4, kBlkH = 8;                   // tiles per block: one per lane
 static_assert(kBlkW * kBlkH == 32, "one lane per tile of a block");
 constexpr uint32_t kBlkThreads = 512, kBlkWarps = kBlkThreads / 32;   // step A: one entry per thread
-constexpr uint32_t kBlkUnit = 128;                         // step B: records per warp
+// Step B: a CTA takes a unit of 512 consecutive records of a block, or of 1024 where the lists outgrow the
+// L2: a run's ends are sectors that two units write in parts, which costs little while they meet in
+// the cache (six cameras, 5.8 GB of lists: 1540 us with 512, 1340 with 1024; 116 MB: 42 and 45).
+constexpr uint32_t kBlkUnitMin = 512, kBlkUnitMax = 1024;
+constexpr uint64_t kBlkLongLists = (126ull << 20) / 12;    // entries
+constexpr uint32_t kBlkWords = 2;                          // writing: 32-record groups per warp
+constexpr uint32_t kBlkCountThreads = 128;                 // counting
 constexpr uint32_t kBlkMaxPerSensor = 1024;                // blocks per sensor (32768 tiles)
 constexpr uint32_t kBlkMaxPerRow = 256;                    // block columns: shared-memory tables of step A
 constexpr uint32_t kBlkRows = 2;                           // block rows per CTA of step A's scatter
 constexpr uint32_t kBlkMaxBlocks = 16384;                  // blocks over all sensors
 constexpr uint32_t kBlkMaxSensors = 4096;
 constexpr uint32_t kBlkMaxExtent = 8192;                   // tiles per row / rows: the packed rectangle's 16-bit fields
-constexpr uint32_t kBlkGridB = 8 * kNumSMs;                // persistent grid of step B: counting
-constexpr uint32_t kBlkOutThreads = 128;                   // step B, writing: 37 KB of staging per CTA
-constexpr uint32_t kBlkGridOut = 6 * kNumSMs;
+constexpr uint32_t kBlkGridB = 16 * kNumSMs;               // persistent grid of step B: counting
 
 struct BlkArgs {
     // entries in (sensor, depth bits, flatten index) order
@@ -1070,6 +1072,7 @@ struct BlkArgs {
     uint32_t width, height;       // tile grid of a sensor
     uint32_t bx, by, blocks;      // blocks per row, per column, per sensor
     uint32_t tile_n_bits;
+    uint32_t unit;                // records per step-B unit
     // workspace
     uint32_t total, ctas;         // elements (>= entries), step-A CTAs launched
     uint32_t *table;              // [blocks][ctas] records per (block, step-A CTA); scanned in place
@@ -1077,6 +1080,7 @@ struct BlkArgs {
     uint32_t *unit_start;         // [C * blocks + 1] first step-B unit of every block
     uint2 *rec;                   // [capacity] {tiles covered, entry}
     uint32_t *unit_cnt;           // [units][32] list entries per (unit, tile); scanned per block in place
+    uint4 *unit_info;             // [units] {block, first record, end}
     uint32_t *tile_base;          // [C * n_tiles] totals, then first list position of every tile
 };
 
@@ -1245,7 +1249,7 @@ blk_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket) {
         const uint32_t v = i < n_blocks ? __ldcg(a.rec_start + i) : 0u;
         uint32_t tr, tu;
         const uint32_t er = block_excl_scan(v, wt, tr);
-        const uint32_t eu = block_excl_scan((v + kBlkUnit - 1) / kBlkUnit, wt, tu);
+        const uint32_t eu = block_excl_scan((v + a.unit - 1) / a.unit, wt, tu);
         if (i < n_blocks) {
             a.rec_start[i] = recs + er;
             a.unit_start[i] = units + eu;
@@ -1346,8 +1350,8 @@ __device__ __forceinline__ BlkUnit blk_unit(const BlkArgs &a, uint32_t u, uint32
     // blocks without records own no unit: the search ends at the last of equal starts, which has one
     v.block = warp_find(a.unit_start, a.C * a.blocks, u, lane);
     const uint32_t cap = (uint32_t)min(a.capacity, (int64_t)0x7fffffff);
-    v.lo = min(cap, __ldg(a.rec_start + v.block) + (u - __ldg(a.unit_start + v.block)) * kBlkUnit);
-    v.hi = min(min(cap, __ldg(a.rec_start + v.block + 1)), v.lo + kBlkUnit);
+    v.lo = min(cap, __ldg(a.rec_start + v.block) + (u - __ldg(a.unit_start + v.block)) * a.unit);
+    v.hi = min(min(cap, __ldg(a.rec_start + v.block + 1)), v.lo + a.unit);
     return v;
 }
 
@@ -1375,23 +1379,34 @@ __device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x, uint32_t lan
     return x;
 }
 
-__global__ void __launch_bounds__(kThreads)
+template <uint32_t kWords>   // 32-record groups per warp
+__global__ void __launch_bounds__(kBlkCountThreads)
 tile_count_kernel(BlkArgs a) {
     chain_enter();
+    constexpr uint32_t kWarps = kBlkCountThreads / 32;
+    __shared__ uint32_t s_cnt[kWarps][32];
     if (blk_overflow(a)) return;
-    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t n_units = a.unit_start[a.C * a.blocks];
-    for (uint32_t u = (blockIdx.x * kThreads + threadIdx.x) >> 5; u < n_units; u += gridDim.x * (kThreads / 32)) {
+    for (uint32_t u = blockIdx.x; u < n_units; u += gridDim.x) {
         const BlkUnit v = blk_unit(a, u, lane);
-        uint32_t m[kBlkUnit / 32], cnt = 0;
+        uint32_t m[kWords], cnt = 0;
 #pragma unroll
-        for (uint32_t j = 0; j < kBlkUnit / 32; ++j) {
-            const uint32_t p = v.lo + 32 * j + lane;
+        for (uint32_t j = 0; j < kWords; ++j) {
+            const uint32_t p = v.lo + 32 * (warp * kWords + j) + lane;
             m[j] = p < v.hi ? __ldg(&a.rec[p].x) : 0u;
         }
 #pragma unroll
-        for (uint32_t j = 0; j < kBlkUnit / 32; ++j) cnt += __popc(warp_transpose_bits(m[j], lane));
-        a.unit_cnt[(size_t)u * 32 + lane] = cnt;
+        for (uint32_t j = 0; j < kWords; ++j) cnt += __popc(warp_transpose_bits(m[j], lane));
+        s_cnt[warp][lane] = cnt;
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (uint32_t w = 1; w < kWarps; ++w) cnt += s_cnt[w][lane];
+            a.unit_cnt[(size_t)u * 32 + lane] = cnt;
+            if (lane == 0) a.unit_info[u] = make_uint4(v.block, v.lo, v.hi, 0u);
+        }
+        __syncthreads();
     }
 }
 
@@ -1469,18 +1484,22 @@ tile_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket, int32_t *__
     }
 }
 
-// Every warp puts its unit's list entries in tile order in shared memory first - as (record, tile), two
-// bytes each - and then writes them out 32 at a time. (Storing straight from the lanes whose record
-// covers a tile needs no staging, but a store instruction costs the SM about eight cycles of moving
-// addresses and data however few of its lanes are active, and a fifth were: 180 us for the lidar
-// benchmark's 15.3 M entries.)
-__global__ void __launch_bounds__(kBlkOutThreads)
+// A CTA puts its unit's list entries in tile order in shared memory first - as record numbers, two bytes
+// each - and its warps then write a few tiles' runs each, in steps that begin on a multiple of 32
+// entries: whole 32-byte sectors but for the two ends of a run. (Storing straight from the lanes whose record
+// covers a tile needs no staging, but sectors written in parts cost the L2 more than whole ones and a fifth
+// of the lanes were active: 180 us for the lidar benchmark's 15.3 M entries. A unit of 128 records per
+// warp, its runs not aligned: 73 us; this: 67. Six cameras: 1920 -> 1340 us.)
+template <uint32_t kWarps>
+__global__ void __launch_bounds__(kWarps * 32)
 tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restrict__ flatten_ids,
                     int64_t *__restrict__ counters) {
     chain_enter();
-    constexpr uint32_t kWords = kBlkUnit / 32;
-    __shared__ uint16_t s_out[kBlkOutThreads / 32][kBlkUnit * 32];
-    __shared__ uint2 s_pair[kBlkOutThreads / 32][kBlkUnit];
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    uint2 *s_pair = reinterpret_cast<uint2 *>(s_raw);
+    uint16_t *s_out = reinterpret_cast<uint16_t *>(s_pair + kWarps * kBlkWords * 32);
+    __shared__ uint32_t s_n[kWarps][32];       // entries per (warp, tile)
+    __shared__ uint4 s_run[32];                       // per tile: first place in s_out, entries, list position, id
     if (blk_overflow(a)) {
         if (blockIdx.x == 0 && threadIdx.x == 0)
             atomicOr((unsigned long long *)&counters[CNT_STATUS], (unsigned long long)ST_OVERFLOW_CAPACITY);
@@ -1489,70 +1508,75 @@ tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restr
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t n_units = a.unit_start[a.C * a.blocks];
     const uint32_t cap = (uint32_t)min(a.capacity, (int64_t)0x7fffffff);
-    uint16_t *out = s_out[warp];
-    uint2 *pair = s_pair[warp];
-    for (uint32_t u = blockIdx.x * (kBlkOutThreads / 32) + warp; u < n_units; u += gridDim.x * (kBlkOutThreads / 32)) {
-        const BlkUnit v = blk_unit(a, u, lane);
-        const BlkTile t = blk_tile(a, v.block, lane);
-        const bool in_grid = t.x < a.width && t.y < a.height;
+    uint4 info = make_uint4(0u, 0u, 0u, 0u);
+    if (blockIdx.x < n_units) info = __ldg(a.unit_info + blockIdx.x);
+    for (uint32_t u = blockIdx.x; u < n_units; u += gridDim.x) {
+        const uint4 v = info;   // {block, first record, end}
+        uint2 rec[kBlkWords];
+#pragma unroll
+        for (uint32_t j = 0; j < kBlkWords; ++j) {
+            const uint32_t p = v.y + 32 * (warp * kBlkWords + j) + lane;
+            rec[j] = p < v.z ? __ldg(a.rec + p) : make_uint2(0u, 0u);
+        }
+        if (u + gridDim.x < n_units) info = __ldg(a.unit_info + u + gridDim.x);
+        const BlkTile t = blk_tile(a, v.x, lane);
         const uint32_t tile = t.y * a.width + t.x;
         uint32_t at = 0;   // lane l: list position of the unit's first entry of tile l
-        if (in_grid) at = __ldg(a.tile_base + t.sensor * a.n_tiles + tile) + __ldg(a.unit_cnt + (size_t)u * 32 + lane);
-        uint2 rec[kWords];
+        if (t.x < a.width && t.y < a.height)
+            at = __ldg(a.tile_base + t.sensor * a.n_tiles + tile) + __ldg(a.unit_cnt + (size_t)u * 32 + lane);
+        uint32_t word[kBlkWords], n = 0;   // lane l: which records cover tile l, how many
 #pragma unroll
-        for (uint32_t j = 0; j < kWords; ++j) {
-            const uint32_t p = v.lo + 32 * j + lane;
-            rec[j] = p < v.hi ? __ldg(a.rec + p) : make_uint2(0u, 0u);
-        }
-        uint32_t word[kWords], n = 0;   // lane l: which records cover tile l, how many
-#pragma unroll
-        for (uint32_t j = 0; j < kWords; ++j) {
-            if (v.lo + 32 * j + lane < v.hi) pair[32 * j + lane] = __ldg(a.pair + rec[j].y);
+        for (uint32_t j = 0; j < kBlkWords; ++j) {
+            if (rec[j].x) s_pair[32 * (warp * kBlkWords + j) + lane] = __ldg(a.pair + rec[j].y);
             word[j] = warp_transpose_bits(rec[j].x, lane);
             n += __popc(word[j]);
         }
-        uint32_t inc = n;
+        s_n[warp][lane] = n;
+        __syncthreads();
+        uint32_t before = 0, all = 0;   // lane l: entries of tile l in earlier warps, in the unit
+#pragma unroll
+        for (uint32_t w = 0; w < kWarps; ++w) {
+            const uint32_t c = s_n[w][lane];
+            if (w < warp) before += c;
+            all += c;
+        }
+        uint32_t first = all;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xffffffffu, inc, off);
-            if (lane >= (uint32_t)off) inc += o;
+            const uint32_t o = __shfl_up_sync(0xffffffffu, first, off);
+            if (lane >= (uint32_t)off) first += o;
         }
-        const uint32_t n_out = __shfl_sync(0xffffffffu, inc, 31);
-        uint32_t local = inc - n;
-        at -= local;                    // list position of local place 0 as seen by tile l
+        first -= all;
+        if (warp == 0) s_run[lane] = make_uint4(first, all, at, (t.sensor << a.tile_n_bits) | tile);
+        uint32_t local = first + before;
 #pragma unroll
-        for (uint32_t j = 0; j < kWords; ++j) {
+        for (uint32_t j = 0; j < kBlkWords; ++j) {
             uint32_t w = word[j];
             while (w) {
                 const uint32_t r = __ffs(w) - 1;
                 w &= w - 1;
-                out[local++] = (uint16_t)((32 * j + r) | (lane << 8));
+                s_out[local++] = (uint16_t)(32 * (warp * kBlkWords + j) + r);
             }
         }
-        __syncwarp();
-        // four steps of 32 entries in flight per warp: the shared-memory loads and shuffles of one step
-        // follow each other, and 37 KB per CTA leave a scheduler six warps to fill the waits
-        const uint32_t hi0 = (t.sensor << a.tile_n_bits) | (__shfl_sync(0xffffffffu, tile, 0));
-        for (uint32_t i0 = lane; i0 < n_out + lane; i0 += 4 * 32) {
-            uint32_t o[4], pos[4];
-            uint2 e[4];
+        __syncthreads();
+        for (uint32_t l = warp; l < 32; l += kWarps) {
+            const uint4 run = s_run[l];
+            const uint32_t end = min(run.z + run.y, cap);
+            const uint16_t *src = s_out + run.x - run.z;   // indexed by list position
+            for (uint32_t p0 = run.z & ~31u; p0 < end; p0 += 4 * 32) {
 #pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) o[q] = i0 + 32 * q < n_out ? out[i0 + 32 * q] : 0u;
-#pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                pos[q] = i0 + 32 * q + __shfl_sync(0xffffffffu, at, o[q] >> 8);
-                e[q] = pair[o[q] & 0xffu];
-            }
-#pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                const uint32_t l = o[q] >> 8, id = hi0 + (l / kBlkW) * a.width + (l & (kBlkW - 1));
-                if (i0 + 32 * q < n_out && pos[q] < cap) {
-                    isect_ids[pos[q]] = (int64_t)(((uint64_t)id << 32) | e[q].x);
-                    flatten_ids[pos[q]] = (int32_t)e[q].y;
+                for (uint32_t q = 0; q < 4; ++q) {
+                    if (p0 + 32 * q >= end) break;
+                    const uint32_t p = p0 + 32 * q + lane;
+                    if (p >= run.z && p < end) {
+                        const uint2 e = s_pair[src[(int32_t)p]];
+                        isect_ids[p] = (int64_t)(((uint64_t)run.w << 32) | e.x);
+                        flatten_ids[p] = (int32_t)e.y;
+                    }
                 }
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -1660,6 +1684,7 @@ static FillWs carve_fill(void *ws, uint64_t cap) {
 
 struct BlkWs {
     uint32_t *rec_start, *unit_start, *unit_cnt, *tile_base;
+    uint4 *unit_info;
     uint2 *rec;
     size_t bytes;
 };
@@ -1673,7 +1698,8 @@ static BlkWs carve_blocks(void *ws, uint64_t cap) {
     w.unit_start = (uint32_t *)take(sizeof(uint32_t) * (kBlkMaxBlocks + 1));
     w.tile_base = (uint32_t *)take(sizeof(uint32_t) * kBlkMaxBlocks * 32);
     // a record stands for at least one list entry; every block rounds its records up to whole units
-    w.unit_cnt = (uint32_t *)take(sizeof(uint32_t) * 32 * (cap / kBlkUnit + kBlkMaxBlocks));
+    w.unit_cnt = (uint32_t *)take(sizeof(uint32_t) * 32 * (cap / kBlkUnitMin + kBlkMaxBlocks));
+    w.unit_info = (uint4 *)take(sizeof(uint4) * (cap / kBlkUnitMin + kBlkMaxBlocks));
     w.rec = (uint2 *)take(sizeof(uint2) * cap);
     w.bytes = off;
     return w;
@@ -1942,12 +1968,12 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
         a.total = g.total;
         a.rec_start = w.rec_start; a.unit_start = w.unit_start;
         a.rec = w.rec;
-        a.unit_cnt = w.unit_cnt; a.tile_base = w.tile_base;
+        a.unit_cnt = w.unit_cnt; a.unit_info = w.unit_info; a.tile_base = w.tile_base;
         const uint32_t ctas_a = div_up(g.total, kBlkThreads) + (g.C > 1 ? g.C : 0u);
         a.ctas = ctas_a;
         const uint32_t n_blocks = a.C * a.blocks;
-        const uint32_t units_max = div_up((uint64_t)capacity, kBlkUnit) + n_blocks;
-        const uint32_t ctas_b = min(div_up(units_max, kThreads / 32), kBlkGridB);
+        a.unit = (uint64_t)capacity > kBlkLongLists ? kBlkUnitMax : kBlkUnitMin;
+        const uint32_t units_max = div_up((uint64_t)capacity, a.unit) + n_blocks;
         const size_t smem_count = sizeof(uint32_t) * a.blocks;
         const size_t smem_scatter = sizeof(uint32_t) * kBlkWarps * min(kBlkRows, a.by) * a.bx * (g.lidar ? 5 : 2);
         auto count = g.lidar ? blk_count_kernel<true> : blk_count_kernel<false>;
@@ -1969,7 +1995,9 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
         }
         {
             SPL_PROF("tile_count_kernel", st);
-            launch_chained(tile_count_kernel, ctas_b, kThreads, 0, st, a);
+            auto kernel = a.unit == kBlkUnitMax ? tile_count_kernel<kBlkUnitMax / kBlkCountThreads>
+                                                : tile_count_kernel<kBlkUnitMin / kBlkCountThreads>;
+            launch_chained(kernel, min(units_max, kBlkGridB), kBlkCountThreads, 0, st, a);
         }
         {
             SPL_PROF("tile_scan_kernel", st);
@@ -1978,7 +2006,14 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
         }
         {
             SPL_PROF("tile_scatter_kernel", st);
-            launch_chained(tile_scatter_kernel, min(div_up(units_max, kBlkOutThreads / 32), kBlkGridOut), kBlkOutThreads, 0, st, a, isect_ids, flatten_ids, p.counters);
+            constexpr uint32_t kMin = kBlkUnitMin / (32 * kBlkWords), kMax = kBlkUnitMax / (32 * kBlkWords);
+            const bool longer = a.unit == kBlkUnitMax;
+            auto kernel = longer ? tile_scatter_kernel<kMax> : tile_scatter_kernel<kMin>;
+            // records' pairs and 32 places of two bytes per record: 36 or 72 KB, six or three CTAs per SM
+            const size_t smem = (size_t)a.unit * (sizeof(uint2) + 32 * sizeof(uint16_t));
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            launch_chained(kernel, min(units_max, (longer ? 3u : 6u) * kNumSMs), a.unit / kBlkWords, smem, st, a, isect_ids,
+                           flatten_ids, p.counters);
         }
     } else {
         FillWs f = carve_fill(fill_workspace, (uint64_t)capacity);

@@ -1030,8 +1030,8 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
     # the count is read when the caller asks for the exact tensors.
     capacity = list_room(hint)
     slot = _lib.acquire_pinned_slot(dev)
-    # the rectangle count kernel hands the count to the host itself (slot[4:6]) when the lists are
-    # built by the row / column split; the event behind the plan is the fallback
+    # a kernel of the plan hands the count to the host itself (slot[4:6]); the event behind the plan is
+    # the fallback
     sequence = _lib.next_sequence()
     lib.splatad_isect_set_early_count(slot.data_ptr() + 32, sequence)
     try:

@@ -266,7 +266,7 @@ def test_depth_range_hint_never_changes_the_lists(lo, hi):
                                        (5, 300, 64, 40), (2, 1025, 1, 70), (130, 64, 9, 3)])
 @pytest.mark.parametrize("packed", [False, True])
 def test_block_split_at_the_edges_of_its_blocks(C, N, tw, th, packed):
-    """The lists are built over blocks of 4 x 8 tiles, 512 entries per step-A block and 128 records per
+    """The lists are built over blocks of 4 x 8 tiles, 512 entries per step-A block and 512 records per
     unit: grids one tile short of, at and beyond a block's edges, entry counts around the chunk sizes,
     sensors without a single entry, more sensors than a warp has lanes. Bit for bit the oracle's lists."""
     from oracle import isect
