@@ -160,7 +160,7 @@ __device__ __forceinline__ float2 pair_power(float a, float2 dx, float bdy, floa
 // Camera forward. Bound by instruction issue: two pixels per thread take 50 instructions per entry where
 // one took 40, and a warp passes over the entries that cannot reach its 8 x 8 patch without looking at
 // them. A pixel that has stopped moves its column out to where every alpha vanishes, which costs the
-// other pixels nothing; a warp leaves when all of its pixels have. Camera benchmark frame: 0.338 -> 0.248 ms.
+// other pixels nothing; a warp leaves when all of its pixels have. Camera benchmark frame: 0.338 -> 0.209 ms.
 // ---------------------------------------------------------------------------------------
 constexpr float kExpectedMin = 1e-10f;   // alphas below it do not divide (gsplat/rendering.py:423-430)
 constexpr float kPixelGone = 1e18f;   // a column no Gaussian reaches: sigma overflows, alpha is 0 (or NaN, never drawn)
@@ -213,12 +213,12 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
 
     float2 px = make_float2(n_inside > 0 ? px0 : kPixelGone, n_inside > 1 ? px0 + 1.f : kPixelGone);
     float2 T = make_float2(1.f, 1.f);
-    int32_t last0 = 0, last1 = 0;
+    constexpr uint32_t kNoEntry = 0xffffffffu;
+    int32_t pos0 = 0, pos1 = 0;   // list position of the last entry blended
     float out[2][CDIM];
 #pragma unroll
     for (int k = 0; k < CDIM; ++k) out[0][k] = out[1][k] = 0.f;
-    bool gone = n_inside == 0;   // both pixels have stopped (or are not there)
-    bool warp_done = __all_sync(0xffffffffu, gone);
+    bool warp_done = __all_sync(0xffffffffu, n_inside == 0);
 
     int32_t next_id = 0;
     if (range.start + (int32_t)tr < range.end) next_id = flatten_ids[range.start + tr];
@@ -254,10 +254,11 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
         }
         __syncthreads();
         if (warp_done) continue;
+        uint32_t last0 = kNoEntry, last1 = kNoEntry;   // this batch's
         for (uint32_t t0 = 0; t0 < n_kept && !warp_done; t0 += 32) {
             const uint32_t mine = t0 + lane;
             uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u));
-            while (todo && !(warp_done = __all_sync(0xffffffffu, gone))) {
+            while (todo) {
                 const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
                 todo &= todo - 1u;
                 const float4 A = sA[t], B = sB[t];
@@ -265,16 +266,22 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
                 const float2 dx = __fadd2_rn(make_float2(mx, mx), make_float2(-px.x, -px.y));
                 const float2 pw = pair_power(B.x, dx, B.y * dy, B.z * dy * dy);
                 const float2 av = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
-                const bool ok0 = pw.x <= 0.f && av.x >= kAlphaMin, ok1 = pw.y <= 0.f && av.y >= kAlphaMin;
-                if (!(ok0 || ok1)) continue;
+                bool ok0 = pw.x <= 0.f && av.x >= kAlphaMin, ok1 = pw.y <= 0.f && av.y >= kAlphaMin;
+                if (!__any_sync(0xffffffffu, ok0 || ok1)) continue;
                 const float2 alpha = make_float2(ok0 ? fminf(kAlphaMax, av.x) : 0.f, ok1 ? fminf(kAlphaMax, av.y) : 0.f);
                 const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
-                const float2 next_T = __fmul2_rn(T, om);
+                float2 next_T = __fmul2_rn(T, om);
                 float2 vis = __fmul2_rn(alpha, T);
-                const bool stop0 = ok0 && next_T.x <= kTStop, stop1 = ok1 && next_T.y <= kTStop;
-                if (stop0) { px.x = kPixelGone; vis.x = 0.f; } else T.x = next_T.x;
-                if (stop1) { px.y = kPixelGone; vis.y = 0.f; } else T.y = next_T.y;
-                gone = px.x == kPixelGone && px.y == kPixelGone;
+                // T stays above the limit, so only a blended entry can take a pixel below it; few entries do
+                if (__any_sync(0xffffffffu, fminf(next_T.x, next_T.y) <= kTStop)) {
+                    if (next_T.x <= kTStop) { px.x = kPixelGone; vis.x = 0.f; next_T.x = T.x; ok0 = false; }
+                    if (next_T.y <= kTStop) { px.y = kPixelGone; vis.y = 0.f; next_T.y = T.y; ok1 = false; }
+                    warp_done = __all_sync(0xffffffffu, px.x == kPixelGone && px.y == kPixelGone);
+                    if (warp_done) todo = 0u;
+                }
+                if (ok0) last0 = t;
+                if (ok1) last1 = t;
+                T = next_T;
                 const float4 *row = reinterpret_cast<const float4 *>(sCol + t * CDIM);
                 const float2 w0 = make_float2(vis.x, vis.x), w1 = make_float2(vis.y, vis.y);
 #pragma unroll
@@ -289,12 +296,11 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
                         out[1][k + h] = d.x; out[1][k + h + 1] = d.y;
                     }
                 }
-                const int32_t entry = sPos[t];
-                if (ok0 && !stop0) last0 = entry;
-                if (ok1 && !stop1) last1 = entry;
             }
-            warp_done = __all_sync(0xffffffffu, gone);
         }
+        // staged place -> list position
+        if (last0 != kNoEntry) pos0 = sPos[last0];
+        if (last1 != kNoEntry) pos1 = sPos[last1];
     }
     const bool vec_out = channels == 4u && (reinterpret_cast<uintptr_t>(render_colors) & 15u) == 0u;
     const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
@@ -304,7 +310,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
         const size_t pix = ((size_t)cam * H + i) * W + j + h;
         const float Tk = h ? T.y : T.x;
         render_alphas[pix] = 1.f - Tk;
-        last_ids[pix] = h ? last1 : last0;
+        last_ids[pix] = h ? pos1 : pos0;
         float *dst = render_colors + pix * channels;
         if (CDIM == 4 && vec_out) {   // one 16-byte store per pixel
             float4 v = make_float4(out[h][0], out[h][1], out[h][2], out[h][3]);
@@ -834,32 +840,54 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// Sums kSlots (a power of two <= 32) per-lane values over the warp at once: every step halves the
-// number of values a lane carries and swaps the other half with the partner lane, kSlots - 1
-// shuffles in all (plus one per remaining lane bit) where one butterfly per value takes 5 * kSlots.
-// Returns, on lane l, the warp total of value (l * kSlots) / 32; lanes that share an index return
-// the same total. v is destroyed.
-template <int kSlots>
-__device__ __forceinline__ float warp_sum_slots(float (&v)[kSlots], uint32_t lane) {
-    int off = 16;
+// Sums N <= 32 per-lane values over the warp at once: every step pairs the first half of the values a lane
+// carries with the second, keeps one of each pair and swaps the other with the partner lane; an odd value
+// out is summed on both sides. 12 values take 48 instructions where one butterfly per value takes 120 (and
+// padding them to 16 62). sum_slot() says which value's total a lane ends up with, and which of the lanes
+// that hold the same one writes it. Call with kOff = 16.
+template <int N, int kOff>
+__device__ __forceinline__ float warp_sum_values(const float (&v)[N], uint32_t lane) {
+    constexpr int kPairs = N / 2, kNext = kPairs + (N & 1);
+    const bool upper = (lane & (uint32_t)kOff) != 0u;
+    float next[kNext];
+    if (N & 1) next[kPairs] = v[N - 1] + __shfl_xor_sync(0xffffffffu, v[N - 1], kOff);
 #pragma unroll
-    for (int half = kSlots / 2; half >= 1; half >>= 1) {
-        const bool upper = (lane & (uint32_t)off) != 0u;
-#pragma unroll
-        for (int i = 0; i < half; ++i) {
-            const float send = upper ? v[i] : v[i + half];
-            const float keep = upper ? v[i + half] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-        }
-        off >>= 1;
+    for (int i = 0; i < kPairs; ++i) {
+        const float send = upper ? v[i] : v[i + kPairs], keep = upper ? v[i + kPairs] : v[i];
+        next[i] = keep + __shfl_xor_sync(0xffffffffu, send, kOff);
     }
-    float r = v[0];
+    if constexpr (kOff > 1) return warp_sum_values<kNext, kOff / 2>(next, lane);
+    else return next[0];
+}
+
+struct SumSlot { int value; bool writes; };
+
+template <int N>
+__device__ __forceinline__ SumSlot sum_slot(uint32_t lane) {
+    // backwards through the steps: place 0 of the last one is which place of the first?
+    int sizes[6] = {N, 0, 0, 0, 0, 0};
 #pragma unroll
-    for (; off >= 1; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
+    for (int s = 0; s < 5; ++s) sizes[s + 1] = sizes[s] / 2 + (sizes[s] & 1);
+    SumSlot r = {0, true};
+#pragma unroll
+    for (int s = 4; s >= 0; --s) {
+        const int pairs = sizes[s] / 2;
+        const bool upper = (lane & (16u >> s)) != 0u;
+        if (r.value == pairs) { r.value = sizes[s] - 1; r.writes = r.writes && !upper; }   // the odd one out (or the only one)
+        else if (upper) r.value += pairs;
+    }
     return r;
 }
 
-constexpr int pow2_at_least(int n) { return n <= 1 ? 1 : 2 * pow2_at_least((n + 1) / 2); }
+// 1 / x of two values in [0.001, 1]: one Newton-Raphson step on the hardware's approximation (which is off by
+// up to one unit in the last place) gives the correctly rounded quotient for every float in that range - all
+// 85 million of them compared - at half the instructions of a division.
+__device__ __forceinline__ float2 reciprocal_pair(float2 x) {
+    float2 r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
+    return __ffma2_rn(r, __ffma2_rn(make_float2(-x.x, -x.y), r, make_float2(1.f, 1.f)), r);
+}
 
 __device__ __forceinline__ int block_max_int(int v, int *red /* [32] */) {
 #pragma unroll
@@ -915,7 +943,7 @@ __device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t
 // the sums of v, v dx and v dx^2 (v = exp(-sigma) dL/dalpha). The channels behind an entry enter through
 // one number per pixel: dL/dalpha = T (c . g) - (1 / (1 - alpha)) (sum over the entries behind of
 // their weight times their (c . g)), g the pixel's cotangent - a running scalar in place of a running colour.
-// Camera benchmark's training step: 1.55 -> 0.50 ms.
+// Camera benchmark's training step: 1.55 -> 0.42 ms.
 // ---------------------------------------------------------------------------------------
 template <int CDIM, int PX, bool kAbs>
 __global__ void __launch_bounds__(PX == 4 || CDIM > 16 ? 256 : 512)
@@ -1005,11 +1033,11 @@ rasterize_to_pixels_bwd_kernel(
 
     // Where the warp total that ends up on this lane goes: colours first, then the geometry.
     constexpr int kGeo = kAbs ? 10 : 8;
-    constexpr int kSlots = CDIM + kGeo <= 16 ? 16 : 32;
     constexpr bool kSplit = CDIM + kGeo > 32;   // the geometry in a butterfly of its own
-    const GradSlot slot_a = pixel_grad_slot<kAbs>(kSplit ? (int)lane : (int)(lane * kSlots / 32u), CDIM, channels, v_colors,
+    constexpr int kSums = kSplit ? CDIM : CDIM + kGeo;
+    const SumSlot mine_a = sum_slot<kSums>(lane);
+    const GradSlot slot_a = pixel_grad_slot<kAbs>(mine_a.value, CDIM, channels, v_colors,
                                                   v_conics, v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
-    const bool writes_a = kSlots == 32 || (lane & 1u) == 0u;
 
     int32_t next_id = 0;
     {
@@ -1086,7 +1114,7 @@ rasterize_to_pixels_bwd_kernel(
                 for (int q = 0; q < P2; ++q) {
                     const float2 alpha = make_float2(fminf(kAlphaMax, av[q].x), fminf(kAlphaMax, av[q].y));
                     const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
-                    const float2 ra = make_float2(1.f / om.x, 1.f / om.y);
+                    const float2 ra = reciprocal_pair(om);
                     T[q] = __fmul2_rn(T[q], ra);
                     const float2 fac = __fmul2_rn(alpha, T[q]);
                     float2 dot;   // (c . g) of the two pixels
@@ -1140,19 +1168,19 @@ rasterize_to_pixels_bwd_kernel(
                     sum[CDIM + 9] = ay.x + ay.y;
                 }
                 const size_t g = (size_t)sId[t];
-                float slots[kSlots];
+                float sums[kSums];
 #pragma unroll
-                for (int k = 0; k < kSlots; ++k) slots[k] = k < (kSplit ? CDIM : CDIM + kGeo) ? sum[k] : 0.f;
-                const float total = warp_sum_slots<kSlots>(slots, lane);
-                slot_a.add(g, total, B.w, writes_a);
+                for (int k = 0; k < kSums; ++k) sums[k] = sum[k];
+                slot_a.add(g, warp_sum_values<kSums, 16>(sums, lane), B.w, mine_a.writes);
                 if (kSplit) {
-                    float geo[16];
+                    float geo[kGeo];
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) geo[k] = k < kGeo ? sum[CDIM + k] : 0.f;
-                    const float geo_total = warp_sum_slots<16>(geo, lane);
-                    const GradSlot slot_b = pixel_grad_slot<kAbs>(CDIM + (int)(lane >> 1), CDIM, channels, v_colors, v_conics,
+                    for (int k = 0; k < kGeo; ++k) geo[k] = sum[CDIM + k];
+                    const float geo_total = warp_sum_values<kGeo, 16>(geo, lane);
+                    const SumSlot mine_b = sum_slot<kGeo>(lane);
+                    const GradSlot slot_b = pixel_grad_slot<kAbs>(CDIM + mine_b.value, CDIM, channels, v_colors, v_conics,
                                                                   v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
-                    slot_b.add(g, geo_total, B.w, (lane & 1u) == 0u);
+                    slot_b.add(g, geo_total, B.w, mine_b.writes);
                 }
             }
         }
@@ -1279,12 +1307,12 @@ __global__ void __launch_bounds__(256, CDIM <= 20 ? 2 : 1) rasterize_to_points_b
     const uint32_t num_batches = (uint32_t)(eff_end - range.start + cap - 1) / cap;
 
     constexpr int kGeo = kAbs ? 13 : 11;
-    constexpr int kSlots = CDIM + kGeo <= 16 ? 16 : 32;
     constexpr bool kSplit = CDIM + kGeo > 32;   // the geometry in a butterfly of its own
-    const GradSlot slot_a = point_grad_slot<kAbs>(kSplit ? (int)lane : (int)(lane * kSlots / 32u), CDIM, channels, fstride,
+    constexpr int kSums = kSplit ? CDIM : CDIM + kGeo;
+    const SumSlot mine_a = sum_slot<kSums>(lane);
+    const GradSlot slot_a = point_grad_slot<kAbs>(mine_a.value, CDIM, channels, fstride,
                                                   v_colors, v_ranges, v_conics, v_means2d, v_pix_vels, v_depth_comps,
                                                   v_opacities, v_means2d_abs);
-    const bool writes_a = kSlots == 32 || (lane & 1u) == 0u;
 
     int32_t next_id[kStage];
 #pragma unroll
@@ -1366,7 +1394,7 @@ __global__ void __launch_bounds__(256, CDIM <= 20 ? 2 : 1) rasterize_to_points_b
                 if (!__any_sync(0xffffffffu, evaluate(t, B, dx, dy, vis, alpha, open))) continue;
                 const float4 Cc = sC[t];
                 const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
-                P = __fmul2_rn(P, make_float2(1.f / om.x, 1.f / om.y));
+                P = __fmul2_rn(P, reciprocal_pair(om));
                 const float2 dterm = __ffma2_rn(make_float2(Cc.x, Cc.x), roll,
                                                 __ffma2_rn(make_float2(Cc.z, Cc.z), dy, __fmul2_rn(make_float2(Cc.y, Cc.y), dx)));
                 float2 dot = __fmul2_rn(dterm, v_depth);
@@ -1399,7 +1427,7 @@ __global__ void __launch_bounds__(256, CDIM <= 20 ? 2 : 1) rasterize_to_points_b
                 if (!__any_sync(0xffffffffu, evaluate(t, B, dx, dy, vis, alpha, open))) continue;
                 const float4 Cc = sC[t];
                 const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
-                const float2 ra = make_float2(1.f / om.x, 1.f / om.y);
+                const float2 ra = reciprocal_pair(om);
                 T = __fmul2_rn(T, ra);
                 const float2 fac = __fmul2_rn(alpha, T);
                 const float2 dterm = __ffma2_rn(make_float2(Cc.x, Cc.x), roll,
@@ -1461,19 +1489,20 @@ __global__ void __launch_bounds__(256, CDIM <= 20 ? 2 : 1) rasterize_to_points_b
                     sum[CDIM + 12] = fabsf(gy.x - uy.x) + fabsf(uy.x) + fabsf(gy.y - uy.y) + fabsf(uy.y);
                 }
                 const size_t gid = (size_t)sId[t];
-                float slots[kSlots];
+                float sums[kSums];
 #pragma unroll
-                for (int k = 0; k < kSlots; ++k) slots[k] = k < (kSplit ? CDIM : CDIM + kGeo) ? sum[k] : 0.f;
-                slot_a.add(gid, warp_sum_slots<kSlots>(slots, lane), 1.f, writes_a);
+                for (int k = 0; k < kSums; ++k) sums[k] = sum[k];
+                slot_a.add(gid, warp_sum_values<kSums, 16>(sums, lane), 1.f, mine_a.writes);
                 if (kSplit) {
-                    float geo[16];
+                    float geo[kGeo];
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) geo[k] = k < kGeo ? sum[CDIM + k] : 0.f;
-                    const float geo_total = warp_sum_slots<16>(geo, lane);
-                    const GradSlot slot_b = point_grad_slot<kAbs>(CDIM + (int)(lane >> 1), CDIM, channels, fstride, v_colors,
+                    for (int k = 0; k < kGeo; ++k) geo[k] = sum[CDIM + k];
+                    const float geo_total = warp_sum_values<kGeo, 16>(geo, lane);
+                    const SumSlot mine_b = sum_slot<kGeo>(lane);
+                    const GradSlot slot_b = point_grad_slot<kAbs>(CDIM + mine_b.value, CDIM, channels, fstride, v_colors,
                                                                   v_ranges, v_conics, v_means2d, v_pix_vels, v_depth_comps,
                                                                   v_opacities, v_means2d_abs);
-                    slot_b.add(gid, geo_total, 1.f, (lane & 1u) == 0u);
+                    slot_b.add(gid, geo_total, 1.f, mine_b.writes);
                 }
             }
         }
