@@ -466,7 +466,7 @@ __device__ __forceinline__ void stage_features(float *row, const float *__restri
 // ---------------------------------------------------------------------------------------
 // entries per thread and batch (their loads overlap), while the shared memory of a batch stays small
 constexpr uint32_t points_fwd_stage(int cdim) { return cdim <= 8 ? 2 : 1; }
-constexpr int points_fwd_regs(int cdim) { return cdim <= 20 ? 96 : 112; }
+constexpr int points_fwd_regs(int cdim) { return cdim <= 8 ? 96 : cdim <= 20 ? 80 : 112; }
 
 template <int CDIM>
 __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kernel(
@@ -945,8 +945,12 @@ __device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t
 // their weight times their (c . g)), g the pixel's cotangent - a running scalar in place of a running colour.
 // Camera benchmark's training step: 1.55 -> 0.42 ms.
 // ---------------------------------------------------------------------------------------
+// registers per thread, by measurement: more warps pay up to a few spilled words (4 channels: 421 us at 100
+// registers, 370 at 80, 384 at 64)
+constexpr int pixels_bwd_regs(int cdim) { return cdim <= 4 ? 80 : cdim <= 20 ? 96 : 168; }
+
 template <int CDIM, int PX, bool kAbs>
-__global__ void __launch_bounds__(PX == 4 || CDIM > 16 ? 256 : 512)
+__global__ void __maxnreg__(pixels_bwd_regs(CDIM))
 rasterize_to_pixels_bwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
