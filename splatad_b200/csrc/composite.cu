@@ -482,6 +482,7 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
     float *__restrict__ render_colors, float *__restrict__ render_alphas,
     float *__restrict__ alpha_sum_out, int32_t *__restrict__ last_ids,
     float *__restrict__ median_depths) {
+    chain_enter();
     constexpr uint32_t kStage = points_fwd_stage(CDIM);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ PointBox s_box[8];
@@ -515,9 +516,6 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
     PointExtent extent;
     if (inside) extent.add(px, py, roll);
     extent.write_box(s_box + warp);
-    // the points are an input of the frame; everything below comes from the kernels before this one
-    chain_enter();
-
     const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
     const uint32_t num_batches = (uint32_t)(range.end - range.start + cap - 1) / cap;
 
@@ -679,6 +677,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     float *__restrict__ render_colors, float *__restrict__ render_alphas,
     float *__restrict__ alpha_sum_out, int32_t *__restrict__ last_ids,
     float *__restrict__ median_depths) {
+    chain_enter();
     constexpr uint32_t kThreadsC = kCoopWarps * 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ PointBox s_box;
@@ -714,9 +713,6 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     if (inside) extent.add(px, py, roll);
     if (warp == 0) extent.write_box(&s_box);
     if (tr == 0) s_done = 0;
-    // the points are an input of the frame; everything below comes from the kernels before this one
-    chain_enter();
-
     const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
     const uint32_t num_batches = (uint32_t)(range.end - range.start + kThreadsC - 1) / kThreadsC;
     const uint32_t fstride = ranges ? channels - 1 : channels;
@@ -963,6 +959,7 @@ rasterize_to_pixels_bwd_kernel(
     float *__restrict__ v_means2d_abs, float *__restrict__ v_means2d,
     float *__restrict__ v_conics, float *__restrict__ v_colors, float *__restrict__ v_opacities,
     float *__restrict__ v_pix_vels, const float *__restrict__ expected /* render whose last channel was divided by the alpha */) {
+    chain_enter();
     static_assert(PX % 2 == 0, "pixels are handled in pairs");
     constexpr int P2 = PX / 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1241,6 +1238,7 @@ __global__ void __launch_bounds__(256, CDIM <= 20 ? 2 : 1) rasterize_to_points_b
     float *__restrict__ v_means2d, float *__restrict__ v_conics, float *__restrict__ v_colors,
     float *__restrict__ v_opacities, float *__restrict__ v_pix_vels,
     float *__restrict__ v_depth_comps, float *__restrict__ v_ranges) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ PointBox s_box;
     constexpr uint32_t kStage = kPointsBwdStage;
@@ -1656,7 +1654,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
         const size_t smem = (size_t)bs * (2 * sizeof(float4) + 3 * sizeof(int32_t) + D * sizeof(float)); \
         int rc = set_smem(kernel, smem, "rasterize_to_pixels_bwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
-        kernel<<<blocks, bs, smem, (cudaStream_t)stream>>>(                                       \
+        launch_chained(kernel, blocks, bs, smem, (cudaStream_t)stream,                            \
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
             image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
@@ -1780,7 +1778,7 @@ extern "C" int splatad_rasterize_to_points_bwd(
                                           (3 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float))); \
         int rc = set_smem(kernel, smem, "rasterize_to_points_bwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
-        kernel<<<blocks * parts, bs, smem, (cudaStream_t)stream>>>(                               \
+        launch_chained(kernel, blocks * parts, bs, smem, (cudaStream_t)stream,                    \
             C, n_isects, (const float2 *)means2d, conics, lidar_features, gaussian_ranges,        \
             channels, opacities,                                                                  \
             pix_vels, (const float2 *)depth_compensations, backgrounds,                           \

@@ -27,7 +27,7 @@ extern "C" int splatad_lidar_frame_fwd(
     SPL_REQUIRE(n_features + 1 <= SPLATAD_MAX_CHANNELS, SPLATAD_ERR_CHANNELS,
                 "lidar_frame_fwd: %u features + range exceed %d channels; render in chunks with the individual "
                 "entry points", n_features, SPLATAD_MAX_CHANNELS);
-    SPL_REQUIRE(opacities_cn && tile_offsets && capacity > 0 && host_counts, SPLATAD_ERR_BAD_ARG,
+    SPL_REQUIRE(opacities_cn && tile_offsets && capacity > 0 && (host_counts || early_count_pair), SPLATAD_ERR_BAD_ARG,
                 "lidar_frame_fwd: null argument");
     int rc = splatad_lidar_projection_fwd(C, N, means, nullptr, quats, scales, velocities, viewmats, min_elevation,
                                           max_elevation, min_azimuth, max_azimuth, linear_velocity,

@@ -152,9 +152,9 @@ Tensor workspace(const char *tag, size_t bytes, c10::cuda::CUDAStream stream) {
     return t;
 }
 
-// Pinned words that one frame owns until its counts have been read: [0..3] the counters the plan copies
-// at its end, [4..7] {count, sequence, status, depth range} stored by a kernel long before, [8] the packed row
-// count. Recycled per stream: the late copy into [0..3] is ordered before the next frame's.
+// Pinned words that one frame owns until its counts have been read, stored by its kernels: [4..7] {count,
+// sequence, status, depth range}, [8] the packed row count. (The plan's own copy of its counters at its end is
+// not asked for: it breaks the chain of launches, 8 us of a small frame's 120.)
 struct Slot {
     StreamKey key;
     Tensor t;
@@ -216,8 +216,7 @@ Counts read_counts(const Slot &slot, int64_t sequence, c10::cuda::CUDAStream str
         c.status = slot.word[6];
         c.depth_range = slot.word[7];
     } else {
-        c.n_isects = slot.word[0];
-        c.status = slot.word[2];
+        TORCH_CHECK(false, "the frame has ended without reporting its intersection count");
     }
     return c;
 }
@@ -463,7 +462,7 @@ py::object lidar_frame(const Tensor &means, const Tensor &quats, const Tensor &s
                 (float)far_plane, (float)radius_clip, alpha_sum, (float)threshold, M(f->radii), M(f->means2d), M(f->depths), M(f->conics),
                 M(f->pix_vels), M(f->depth_comps), I(f->tiles_per_gauss), capacity, L(f->isect_ids), I(f->flatten_ids), I(f->offsets),
                 M(f->render), M(f->alphas), M(f->alpha_sum), I(f->last_ids), M(f->median), plan_ws.data_ptr(), (size_t)plan_ws.numel(),
-                fill_ws.data_ptr(), (size_t)fill_ws.numel(), words, words + 4, sequence, stream.stream()));
+                fill_ws.data_ptr(), (size_t)fill_ws.numel(), nullptr, words + 4, sequence, stream.stream()));
         } else {
             // the compensated opacities come between projection and compositing
             check(lib.splatad_lidar_projection_fwd(
@@ -476,7 +475,7 @@ py::object lidar_frame(const Tensor &means, const Tensor &quats, const Tensor &s
                 return fn((uint32_t)C, (uint32_t)N, (uint64_t)(C * N), F(f->means2d), F(f->radii), F(f->depths), nullptr, F(boundaries),
                           (uint32_t)(rows + 1), (float)(az_res * (double)tile_w), (float)min_az, 1, I(f->tiles_per_gauss), tail...);
             };
-            check(grid(lib.splatad_isect_lidar_tiles_plan, plan_ws.data_ptr(), (size_t)plan_ws.numel(), words, stream.stream()));
+            check(grid(lib.splatad_isect_lidar_tiles_plan, plan_ws.data_ptr(), (size_t)plan_ws.numel(), (int64_t *)nullptr, stream.stream()));
             check(grid(lib.splatad_isect_lidar_tiles_fill, plan_ws.data_ptr(), fill_ws.data_ptr(), (size_t)fill_ws.numel(), capacity,
                        L(f->isect_ids), I(f->flatten_ids), I(f->offsets), (int64_t *)nullptr, stream.stream()));
             check(lib.splatad_rasterize_to_points_fwd(
@@ -758,8 +757,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
         };
         {
             const PlanRequests requests(slot, sequence, last_range);
-            check(grid(lib.splatad_isect_tiles_plan, plan_ws.data_ptr(), (size_t)plan_ws.numel(), const_cast<int64_t *>(slot.word),
-                       stream.stream()));
+            check(grid(lib.splatad_isect_tiles_plan, plan_ws.data_ptr(), (size_t)plan_ws.numel(), (int64_t *)nullptr, stream.stream()));
         }
         check(grid(lib.splatad_isect_tiles_fill, plan_ws.data_ptr(), fill_ws.data_ptr(), (size_t)fill_ws.numel(), capacity,
                    L(f->isect_ids), I(f->flatten_ids), I(f->offsets), (int64_t *)nullptr, stream.stream()));

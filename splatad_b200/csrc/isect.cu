@@ -254,8 +254,7 @@ __device__ __forceinline__ void tell_host(volatile int64_t *early_host, int64_t 
     early_host[2] = status;
     early_host[3] = depth_range;   // dmin bits | dmax bits << 32 of the listed elements, 0: not known here
     __threadfence_system();
-    early_host[1] = seq;
-    __threadfence_system();
+    early_host[1] = seq;   // on its way at the latest when the kernel ends
 }
 
 // tiles_per_gauss[idx] for every (sensor, Gaussian) / packed row. With `rect` the rectangle is also
@@ -625,12 +624,11 @@ depth_bucket_count_kernel(const uint32_t *__restrict__ depth_bits, const int32_t
 // Blocks of 1024 threads, one bucket per thread: starts within the block's 1024 buckets, counts
 // back to zero (they become the scatter's cursors), the block's total. The block that finishes
 // last turns the block totals into block offsets (a bucket's start = bstart[b] + boff[b >> 10]), sets
-// the status bit for oversized buckets, tells the polling host when asked, and - for a grouped order -
+// the status bit for oversized buckets and - for a grouped order -
 // notes where every group's entries and its chunks of `chunk` entries start.
 __global__ void __launch_bounds__(1024)
 depth_bucket_scan_kernel(uint32_t *__restrict__ bcount, uint32_t *__restrict__ bstart, uint32_t *__restrict__ boff,
-                         int64_t *__restrict__ counters, volatile int64_t *early_host, int64_t early_seq,
-                         uint32_t groups, uint32_t per, uint32_t chunk, uint32_t *__restrict__ group_start,
+                         int64_t *__restrict__ counters, uint32_t groups, uint32_t per, uint32_t chunk, uint32_t *__restrict__ group_start,
                          uint32_t *__restrict__ group_chunk /* both [groups + 1]; nullptr: not asked for */) {
     chain_enter();
     __shared__ uint32_t wt[33];
@@ -679,11 +677,6 @@ depth_bucket_scan_kernel(uint32_t *__restrict__ bcount, uint32_t *__restrict__ b
             boff[n_scan] = inc;
             counters[CNT_TICKET] = 0;
             __threadfence();
-            if (early_host != nullptr)
-                tell_host(early_host, early_seq, counters[CNT_NISECT],
-                          (int64_t)atomicOr((unsigned long long *)&counters[CNT_STATUS], 0ull),
-                          (int64_t)(((unsigned long long)(uint32_t)counters[CNT_DMAX] << 32) |
-                                    (unsigned long long)(uint32_t)counters[CNT_DMIN]));
         }
     }
     if (group_start == nullptr) return;
@@ -716,9 +709,16 @@ depth_bucket_scan_kernel(uint32_t *__restrict__ bcount, uint32_t *__restrict__ b
 __global__ void __launch_bounds__(kThreads)
 depth_bucket_scatter_kernel(const uint32_t *__restrict__ depth_bits, const int32_t *__restrict__ tiles_per_gauss,
                             uint32_t total, BucketLayout layout, const int64_t *__restrict__ counters,
+                            volatile int64_t *early_host /* optional: the polling host's words */, int64_t early_seq,
                             const uint32_t *__restrict__ bstart, const uint32_t *__restrict__ boff,
                             uint32_t *__restrict__ bcursor, uint2 *__restrict__ pairs /* {bits, flatten index} */) {
     chain_enter();
+    // All the host wants to know is there since the bucket scan. Telling it takes a fence over the host link, which
+    // would be the end of that kernel's last block; here the other blocks' work covers it (20,000 Gaussians: 4 us).
+    if (early_host != nullptr && blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1)
+        tell_host(early_host, early_seq, counters[CNT_NISECT], counters[CNT_STATUS],
+                  (int64_t)(((unsigned long long)(uint32_t)counters[CNT_DMAX] << 32) |
+                            (unsigned long long)(uint32_t)counters[CNT_DMIN]));
     const DepthBuckets bucket = depth_buckets(counters, layout.per);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         if (tiles_per_gauss[i] <= 0) continue;
@@ -1776,7 +1776,7 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
     const BucketLayout layout = bucket_layout(g, blocks);
     const uint32_t cgrid = min(div_up(g.total, kCountThreads), (uint32_t)(2 * kNumSMs));
     // the intersection count is known when the rectangle count ends: a host that has asked for it (to
-    // size or cut its lists) gets it from a kernel - the rectangle count itself, or the bucket scan right
+    // size or cut its lists) gets it from a kernel - the rectangle count itself, or the bucket scatter soon
     // behind it, which also knows whether the bucket sort applies - and need not wait for the depth
     // order. Both list constructions report it: a host left to wait for words that never came gave up
     // after 20 ms, which was 87 % of a three-camera training step (22.6 -> 3.2 ms).
@@ -1825,13 +1825,14 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
         {
             SPL_PROF("depth_bucket_scan_kernel", st);
             launch_chained(depth_bucket_scan_kernel, p.n_buckets / 1024, 1024, 0, st, p.bcount, p.bstart, p.boff,
-                           p.counters, (volatile int64_t *)early, seq, layout.groups, layout.per, kBlkThreads,
+                           p.counters, layout.groups, layout.per, kBlkThreads,
                            blocks ? p.group_start : (uint32_t *)nullptr, p.group_chunk);
         }
         {
             SPL_PROF("depth_bucket_scatter_kernel", st);
             launch_chained(depth_bucket_scatter_kernel, bgrid, kThreads, 0, st, g.depth_bits,
                            (const int32_t *)tiles_per_gauss, g.total, layout, (const int64_t *)p.counters,
+                           (volatile int64_t *)early, seq,
                            (const uint32_t *)p.bstart, (const uint32_t *)p.boff, p.bcount, pairs);
         }
         {
@@ -2012,8 +2013,10 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
             // records' pairs and 32 places of two bytes per record: 36 or 72 KB, six or three CTAs per SM
             const size_t smem = (size_t)a.unit * (sizeof(uint2) + 32 * sizeof(uint16_t));
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            launch_chained(kernel, min(units_max, (longer ? 3u : 6u) * kNumSMs), a.unit / kBlkWords, smem, st, a, isect_ids,
-                           flatten_ids, p.counters);
+            const uint32_t grid = min(units_max, (longer ? 3u : 6u) * kNumSMs);
+            // long lists: not placed while the scan still holds its SMs (six cameras: 1340 us, and 80 more chained)
+            if (longer) kernel<<<grid, a.unit / kBlkWords, smem, st>>>(a, isect_ids, flatten_ids, p.counters);
+            else launch_chained(kernel, grid, a.unit / kBlkWords, smem, st, a, isect_ids, flatten_ids, p.counters);
         }
     } else {
         FillWs f = carve_fill(fill_workspace, (uint64_t)capacity);
@@ -2130,6 +2133,7 @@ points_tile_kernel(uint32_t total, uint32_t N, const int64_t *__restrict__ camer
                    float tile_azim_resolution, float min_azim, uint32_t n_tiles_azim, uint32_t n_tiles_elev,
                    uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, int64_t *__restrict__ tile_ids,
                    int32_t *__restrict__ flatten_ids, int64_t *__restrict__ count) {
+    chain_enter();
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx == 0 && count != nullptr) *count = (int64_t)total;
     if (idx >= total) return;
@@ -2159,6 +2163,7 @@ __global__ void __launch_bounds__(kThreads)
 points_ids_kernel(uint32_t total, uint32_t n_tiles, const uint32_t *__restrict__ keys,
                   const uint32_t *__restrict__ vals, int64_t *__restrict__ tile_ids,
                   int32_t *__restrict__ flatten_ids) {
+    chain_enter();
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const uint32_t key = keys[idx];
@@ -2171,6 +2176,7 @@ points_ids_kernel(uint32_t total, uint32_t n_tiles, const uint32_t *__restrict__
 __global__ void __launch_bounds__(kThreads)
 points_offset_encode_kernel(const int64_t *__restrict__ point_ids, int64_t n, uint32_t C, uint32_t n_tiles,
                             int32_t *__restrict__ offsets) {
+    chain_enter();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= C * n_tiles) return;
     int64_t l = 0, h = n;
@@ -2189,6 +2195,7 @@ __global__ void populate_image_kernel(uint32_t C, int64_t n_points, const float 
                                       uint32_t W, uint32_t H, uint32_t tile_width, uint32_t tile_height,
                                       uint32_t grid_w, uint32_t grid_h, const int32_t *__restrict__ offsets,
                                       const int32_t *__restrict__ flatten_ids, float *__restrict__ image) {
+    chain_enter();
     const uint32_t tiles_per_cam = grid_w * grid_h;
     const uint32_t cam = blockIdx.x / tiles_per_cam;
     const uint32_t tile = blockIdx.x - cam * tiles_per_cam;
@@ -2408,7 +2415,7 @@ extern "C" int splatad_map_points_to_lidar_tiles(
     const uint32_t grid = div_up(total, kThreads);
     if (!sort) {
         SPL_PROF("points_tile_kernel", st);
-        points_tile_kernel<<<grid, kThreads, 0, st>>>(total, n_per, camera_ids, (const float2 *)points2d,
+        launch_chained(points_tile_kernel, grid, kThreads, 0, st, total, n_per, camera_ids, (const float2 *)points2d,
                                                      elev_boundaries, tile_azim_resolution, min_azim, n_az,
                                                      n_el, nullptr, nullptr, tile_ids, flatten_ids, nullptr);
         return check_launch("map_points_to_lidar_tiles");
@@ -2418,7 +2425,7 @@ extern "C" int splatad_map_points_to_lidar_tiles(
                 "map_points_to_lidar_tiles: workspace too small (%zu < %zu)", workspace_bytes, p.bytes);
     {
         SPL_PROF("points_tile_kernel", st);
-        points_tile_kernel<<<grid, kThreads, 0, st>>>(total, n_per, camera_ids, (const float2 *)points2d,
+        launch_chained(points_tile_kernel, grid, kThreads, 0, st, total, n_per, camera_ids, (const float2 *)points2d,
                                                      elev_boundaries, tile_azim_resolution, min_azim, n_az,
                                                      n_el, p.keyA, p.valA, nullptr, nullptr, p.count);
     }
@@ -2436,16 +2443,16 @@ extern "C" int splatad_map_points_to_lidar_tiles(
         const uint32_t mask = (1u << bits_per) - 1u;
         {
             SPL_PROF("points_sort_upsweep", st);
-            radix_upsweep_kernel<false><<<kSortGrid, kSortThreads, 0, st>>>(s, shift, mask, p.hist);
+            launch_chained(radix_upsweep_kernel<false>, kSortGrid, kSortThreads, 0, st, s, shift, mask, p.hist);
         }
         {
             SPL_PROF("points_sort_rowscan", st);
-            radix_rowscan_kernel<<<kRadixBins, ((kSortGrid + 31) / 32) * 32, 0, st>>>(p.hist, kSortGrid,
+            launch_chained(radix_rowscan_kernel, kRadixBins, ((kSortGrid + 31) / 32) * 32, 0, st, p.hist, kSortGrid,
                                                                                     p.digit_totals);
         }
         {
             SPL_PROF("points_sort_downsweep", st);
-            radix_downsweep_kernel<false, false><<<kSortGrid, kSortThreads, 0, st>>>(
+            launch_chained(radix_downsweep_kernel<false, false>, kSortGrid, kSortThreads, 0, st,
                 s, shift, (int)bits_per, mask, p.hist, p.digit_totals, kb, vb, nofin, nullptr);
         }
         uint32_t *t;
@@ -2454,7 +2461,7 @@ extern "C" int splatad_map_points_to_lidar_tiles(
     }
     {
         SPL_PROF("points_ids_kernel", st);
-        points_ids_kernel<<<grid, kThreads, 0, st>>>(total, n_az * n_el, ka, va, tile_ids, flatten_ids);
+        launch_chained(points_ids_kernel, grid, kThreads, 0, st, total, n_az * n_el, ka, va, tile_ids, flatten_ids);
     }
     return check_launch("map_points_to_lidar_tiles");
 }
@@ -2470,7 +2477,7 @@ extern "C" int splatad_points_mapping_offset_encode(const int64_t *point_ids, in
     const uint32_t total = (uint32_t)(C * n_tiles);
     {
         SPL_PROF("points_offset_encode_kernel", (cudaStream_t)stream);
-        points_offset_encode_kernel<<<div_up(total, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
+        launch_chained(points_offset_encode_kernel, div_up(total, kThreads), kThreads, 0, (cudaStream_t)stream,
             point_ids, n_points, C, (uint32_t)n_tiles, offsets);
     }
     return check_launch("points_mapping_offset_encode");
@@ -2494,7 +2501,7 @@ extern "C" int splatad_populate_image_from_points(
     const uint32_t bs = ((tile_width * tile_height + 31) / 32) * 32;
     {
         SPL_PROF("populate_image_kernel", st);
-        populate_image_kernel<<<blocks, bs, 0, st>>>(C, n_points, points, image_width, image_height, tile_width,
+        launch_chained(populate_image_kernel, blocks, bs, 0, st, C, n_points, points, image_width, image_height, tile_width,
                                                     tile_height, tile_grid_width, tile_grid_height, tile_offsets,
                                                     flatten_ids, image);
     }

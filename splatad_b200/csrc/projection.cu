@@ -330,6 +330,7 @@ lidar_projection_fwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ me
                             float *__restrict__ depths, float *__restrict__ conics,
                             float *__restrict__ compensations, float *__restrict__ pix_vels,
                             float *__restrict__ depth_comps) {
+    chain_enter();
     __shared__ __align__(16) float smem[kStageFloats];
     const uint32_t g0 = blockIdx.x * kThreads;
     const uint32_t n = min((uint32_t)kThreads, N - g0);
@@ -393,6 +394,7 @@ lidar_projection_fwd_pipelined_kernel(uint32_t C, uint32_t N, uint32_t n_slabs, 
                                       float *__restrict__ means2d, float *__restrict__ depths,
                                       float *__restrict__ conics, float *__restrict__ compensations,
                                       float *__restrict__ pix_vels, float *__restrict__ depth_comps) {
+    chain_enter();
     __shared__ ProjSlab slab[2];
     __shared__ __align__(16) float s_out[kThreads * 6];
     __shared__ __align__(8) unsigned long long bar[2];
@@ -499,6 +501,7 @@ projection_fwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
                       int32_t *__restrict__ radii, float *__restrict__ means2d,
                       float *__restrict__ depths, float *__restrict__ conics,
                       float *__restrict__ compensations, float *__restrict__ pix_vels) {
+    chain_enter();
     __shared__ __align__(16) float smem[kStageFloats];
     const uint32_t g0 = blockIdx.x * kThreads;
     const uint32_t n = min((uint32_t)kThreads, N - g0);
@@ -549,6 +552,7 @@ projection_packed_fwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ m
                              int32_t *__restrict__ radii, float *__restrict__ means2d,
                              float *__restrict__ depths, float *__restrict__ conics,
                              float *__restrict__ compensations, float *__restrict__ pix_vels) {
+    chain_enter();
     __shared__ __align__(16) float smem[kStageFloats];
     __shared__ int32_t warp_counts[kThreads / 32];
     const uint32_t g0 = blockIdx.x * kThreads;
@@ -617,6 +621,7 @@ projection_packed_fwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ m
 __global__ void __launch_bounds__(1024)
 packed_scan_kernel(const int32_t *__restrict__ counts, int32_t *__restrict__ offsets, uint32_t C,
                    uint32_t nblocks, int32_t *__restrict__ indptr, int64_t *__restrict__ nnz_out) {
+    chain_enter();
     // rounds of 4096 counts, four consecutive ones per thread (one strip per thread, read twice, took 44 us
     // for the 47 k counts of six cameras and two million Gaussians, this 25)
     __shared__ int32_t warp_sum[33];
@@ -910,6 +915,7 @@ projection_bwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
                       float *__restrict__ v_covars, float *__restrict__ v_quats,
                       float *__restrict__ v_scales, float *__restrict__ v_viewmats,
                       float *__restrict__ v_velocities) {
+    chain_enter();
     __shared__ __align__(16) float smem[kStageFloats];
     __shared__ float red[(kThreads / 32) * 12];
     const uint32_t g0 = blockIdx.x * kThreads;
@@ -966,6 +972,7 @@ lidar_projection_bwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ me
                             float *__restrict__ v_covars, float *__restrict__ v_quats,
                             float *__restrict__ v_scales, float *__restrict__ v_viewmats,
                             float *__restrict__ v_velocities) {
+    chain_enter();
     __shared__ __align__(16) float smem[kStageFloats];
     __shared__ float red[(kThreads / 32) * 12];
     const uint32_t g0 = blockIdx.x * kThreads;
@@ -1045,6 +1052,7 @@ projection_packed_bwd_kernel(uint32_t C, uint32_t N, uint32_t nnz, const float *
                              float *__restrict__ v_means, float *__restrict__ v_covars,
                              float *__restrict__ v_quats, float *__restrict__ v_scales,
                              float *__restrict__ v_viewmats, float *__restrict__ v_velocities) {
+    chain_enter();
     const uint32_t idx = blockIdx.x * kThreads + threadIdx.x;
     if (idx >= nnz) return;
     // (sparse gradients are written, not added)
@@ -1151,13 +1159,13 @@ extern "C" int splatad_lidar_projection_fwd(
         SPL_PROF("lidar_projection_fwd_kernel", st);
         const uint32_t n_rounds = div_up(N, kThreads);   // the ragged last slab rides along
         const uint32_t grid = n_rounds < (uint32_t)(4 * kNumSMs) ? n_rounds : (uint32_t)(4 * kNumSMs);
-        lidar_projection_fwd_pipelined_kernel<<<grid, kThreads, 0, st>>>(
+        launch_chained(lidar_projection_fwd_pipelined_kernel, grid, kThreads, 0, st,
             C, N, n_slabs, means, quats, scales, velocities, viewmats, min_elevation, max_elevation, min_azimuth,
             max_azimuth, linear_velocity, angular_velocity, rolling_shutter_time, eps2d, near_plane, far_plane,
             radius_clip, radii, means2d, depths, conics, compensations, pix_vels, depth_compensations);
     } else {
         SPL_PROF("lidar_projection_fwd_kernel", st);
-        lidar_projection_fwd_kernel<<<div_up(N, kThreads), kThreads, 0, st>>>(
+        launch_chained(lidar_projection_fwd_kernel, div_up(N, kThreads), kThreads, 0, st,
             C, N, means, covars, quats, scales, velocities, viewmats, min_elevation, max_elevation,
             min_azimuth, max_azimuth, linear_velocity, angular_velocity, rolling_shutter_time, eps2d,
             near_plane, far_plane, radius_clip, radii, means2d, depths, conics, compensations,
@@ -1202,7 +1210,7 @@ extern "C" int splatad_lidar_projection_bwd(
     if (C == 0 || N == 0) return SPLATAD_OK;
     {
         SPL_PROF("lidar_projection_bwd_kernel", (cudaStream_t)stream);
-        lidar_projection_bwd_kernel<<<div_up(N, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
+        launch_chained(lidar_projection_bwd_kernel, div_up(N, kThreads), kThreads, 0, (cudaStream_t)stream,
             C, N, means, covars, quats, scales, velocities, viewmats, linear_velocity,
             angular_velocity, rolling_shutter_time, eps2d, radii, conics, compensations, v_means2d,
             v_depths, v_conics, v_compensations, v_pix_vels, v_depth_compensations, v_means, v_covars,
@@ -1228,7 +1236,7 @@ extern "C" int splatad_projection_fwd(
     if (C == 0 || N == 0) return SPLATAD_OK;
     {
         SPL_PROF("projection_fwd_kernel", (cudaStream_t)stream);
-        projection_fwd_kernel<<<div_up(N, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
+        launch_chained(projection_fwd_kernel, div_up(N, kThreads), kThreads, 0, (cudaStream_t)stream,
             C, N, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
             linear_velocity, angular_velocity, rolling_shutter_time, eps2d, near_plane, far_plane,
             radius_clip, radii, means2d, depths, conics, compensations, pix_vels);
@@ -1256,7 +1264,7 @@ extern "C" int splatad_projection_bwd(
     if (C == 0 || N == 0) return SPLATAD_OK;
     {
         SPL_PROF("projection_bwd_kernel", (cudaStream_t)stream);
-        projection_bwd_kernel<<<div_up(N, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
+        launch_chained(projection_bwd_kernel, div_up(N, kThreads), kThreads, 0, (cudaStream_t)stream,
             C, N, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
             linear_velocity, angular_velocity, rolling_shutter_time, eps2d, radii, conics,
             compensations, v_means2d, v_depths, v_conics, v_compensations, v_pix_vels, v_means,
@@ -1291,7 +1299,7 @@ extern "C" int splatad_projection_packed_count(
     cudaStream_t st = (cudaStream_t)stream;
     {
         SPL_PROF("projection_packed_fwd_kernel", st);
-        projection_packed_fwd_kernel<<<nblocks, kThreads, 0, st>>>(
+        launch_chained(projection_packed_fwd_kernel, nblocks, kThreads, 0, st,
             C, N, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
             linear_velocity, angular_velocity, rolling_shutter_time, eps2d, near_plane, far_plane,
             radius_clip, counts, nullptr, (int64_t)-1, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
@@ -1299,7 +1307,7 @@ extern "C" int splatad_projection_packed_count(
     }
     {
         SPL_PROF("packed_scan_kernel", st);
-        packed_scan_kernel<<<1, 1024, 0, st>>>(counts, offsets, C, nblocks, indptr, nnz_device);
+        launch_chained(packed_scan_kernel, 1, 1024, 0, st, counts, offsets, C, nblocks, indptr, nnz_device);
     }
     return check_launch("projection_packed_count");
 }
@@ -1323,7 +1331,7 @@ extern "C" int splatad_projection_packed_fill(
     const int32_t *offsets = (const int32_t *)workspace + (size_t)C * nblocks;
     {
         SPL_PROF("projection_packed_fwd_kernel", (cudaStream_t)stream);
-        projection_packed_fwd_kernel<<<nblocks, kThreads, 0, (cudaStream_t)stream>>>(
+        launch_chained(projection_packed_fwd_kernel, nblocks, kThreads, 0, (cudaStream_t)stream,
             C, N, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
             linear_velocity, angular_velocity, rolling_shutter_time, eps2d, near_plane, far_plane,
             radius_clip, nullptr, offsets, capacity, (const int32_t *)workspace, camera_ids, gaussian_ids, radii,
@@ -1355,7 +1363,7 @@ extern "C" int splatad_projection_packed_bwd(
                 SPLATAD_ERR_BAD_ARG, "projection_packed_bwd: null input");
     {
         SPL_PROF("projection_packed_bwd_kernel", (cudaStream_t)stream);
-        projection_packed_bwd_kernel<<<div_up(nnz, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
+        launch_chained(projection_packed_bwd_kernel, div_up(nnz, kThreads), kThreads, 0, (cudaStream_t)stream,
             C, N, nnz, means, covars, quats, scales, velocities, viewmats, Ks, image_width,
             image_height, linear_velocity, angular_velocity, rolling_shutter_time, eps2d, camera_ids,
             gaussian_ids, conics, compensations, v_means2d, v_depths, v_conics, v_compensations,
@@ -1432,11 +1440,11 @@ extern "C" int splatad_projection_packed_count_noalloc(
     cudaStream_t st = (cudaStream_t)stream;
     // every slot the scan reads is written by the count pass of this same call: nothing in the
     // scratch needs clearing, and what earlier (larger) calls left behind is never read
-    projection_packed_fwd_kernel<<<(uint32_t)nblocks, kThreads, 0, st>>>(
+    launch_chained(projection_packed_fwd_kernel, (uint32_t)nblocks, kThreads, 0, st,
         C, N, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
         linear_velocity, angular_velocity, rolling_shutter_time, eps2d, near_plane, far_plane,
         radius_clip, counts, nullptr, (int64_t)-1, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
         nullptr, nullptr);
-    packed_scan_kernel<<<1, 1024, 0, st>>>(counts, offsets, C, (uint32_t)nblocks, indptr, nnz_device);
+    launch_chained(packed_scan_kernel, 1, 1024, 0, st, counts, offsets, C, (uint32_t)nblocks, indptr, nnz_device);
     return check_launch("projection_packed_count_noalloc");
 }

@@ -10,6 +10,7 @@ namespace splatad {
 __global__ void __launch_bounds__(kThreads)
 opacity_rows_fwd_kernel(uint32_t n, uint32_t N, const int64_t *__restrict__ ids, const float *__restrict__ opacities,
                         const float *__restrict__ comps, float *__restrict__ out) {
+    chain_enter();
     const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     const uint32_t g = ids ? (uint32_t)ids[i] : i % N;
@@ -21,6 +22,7 @@ __global__ void __launch_bounds__(kThreads)
 opacity_rows_bwd_kernel(uint32_t n, uint32_t N, const int64_t *__restrict__ ids, const float *__restrict__ opacities,
                         const float *__restrict__ comps, const float *__restrict__ v_rows,
                         float *__restrict__ v_opacities, float *__restrict__ v_comps) {
+    chain_enter();
     const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     const uint32_t g = ids ? (uint32_t)ids[i] : i % N;
@@ -40,6 +42,7 @@ __global__ void __launch_bounds__(kThreads)
 color_rows_fwd_kernel(uint64_t n_out, uint32_t N, uint32_t D, uint32_t width, const int64_t *__restrict__ camera_ids,
                       const int64_t *__restrict__ gaussian_ids, uint32_t per_camera, const float *__restrict__ colors,
                       const float *__restrict__ depths, float *__restrict__ out) {
+    chain_enter();
     const uint64_t e = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (e >= n_out) return;
     const uint32_t i = (uint32_t)(e / width), k = (uint32_t)(e - (uint64_t)i * width);
@@ -50,6 +53,7 @@ __global__ void __launch_bounds__(kThreads)
 color_rows_bwd_kernel(uint64_t n_in, uint32_t N, uint32_t D, uint32_t width, const int64_t *__restrict__ camera_ids,
                       const int64_t *__restrict__ gaussian_ids, uint32_t per_camera, const float *__restrict__ v_rows,
                       float *__restrict__ v_colors) {
+    chain_enter();
     const uint64_t e = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (e >= n_in) return;
     const uint32_t i = (uint32_t)(e / D), k = (uint32_t)(e - (uint64_t)i * D);
@@ -60,6 +64,7 @@ color_rows_bwd_kernel(uint64_t n_in, uint32_t N, uint32_t D, uint32_t width, con
 __global__ void __launch_bounds__(kThreads)
 last_channel_kernel(uint32_t n, uint32_t width, const float *__restrict__ v_rows, const float *__restrict__ add,
                     float *__restrict__ out) {
+    chain_enter();
     const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     const float v = v_rows[(size_t)i * width + width - 1];
@@ -75,7 +80,7 @@ extern "C" int splatad_opacity_rows_fwd(uint32_t n, uint32_t N, const int64_t *g
     if (n == 0) return SPLATAD_OK;
     SPL_REQUIRE(N > 0 && opacities && rows, SPLATAD_ERR_BAD_ARG, "opacity_rows_fwd: null argument");
     SPL_PROF("opacity_rows_fwd_kernel", (cudaStream_t)stream);
-    opacity_rows_fwd_kernel<<<div_up(n, kThreads), kThreads, 0, (cudaStream_t)stream>>>(n, N, gaussian_ids, opacities,
+    launch_chained(opacity_rows_fwd_kernel, div_up(n, kThreads), kThreads, 0, (cudaStream_t)stream, n, N, gaussian_ids, opacities,
                                                                                        compensations, rows);
     return check_launch("opacity_rows_fwd");
 }
@@ -86,7 +91,7 @@ extern "C" int splatad_opacity_rows_bwd(uint32_t n, uint32_t N, const int64_t *g
     if (n == 0 || (!v_opacities && !v_compensations)) return SPLATAD_OK;
     SPL_REQUIRE(N > 0 && opacities && v_rows, SPLATAD_ERR_BAD_ARG, "opacity_rows_bwd: null argument");
     SPL_PROF("opacity_rows_bwd_kernel", (cudaStream_t)stream);
-    opacity_rows_bwd_kernel<<<div_up(n, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
+    launch_chained(opacity_rows_bwd_kernel, div_up(n, kThreads), kThreads, 0, (cudaStream_t)stream,
         n, N, gaussian_ids, opacities, compensations, v_rows, v_opacities, v_compensations);
     return check_launch("opacity_rows_bwd");
 }
@@ -100,7 +105,7 @@ extern "C" int splatad_color_rows_fwd(uint32_t n, uint32_t N, uint32_t D, const 
                 SPLATAD_ERR_BAD_ARG, "color_rows_fwd: null argument");
     SPL_PROF("color_rows_fwd_kernel", (cudaStream_t)stream);
     const uint64_t n_out = (uint64_t)n * width;
-    color_rows_fwd_kernel<<<div_up(n_out, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
+    launch_chained(color_rows_fwd_kernel, div_up(n_out, kThreads), kThreads, 0, (cudaStream_t)stream,
         n_out, N, D, width, camera_ids, gaussian_ids, colors_per_camera, colors, depths, rows);
     return check_launch("color_rows_fwd");
 }
@@ -114,10 +119,10 @@ extern "C" int splatad_color_rows_bwd(uint32_t n, uint32_t N, uint32_t D, uint32
     SPL_PROF("color_rows_bwd_kernel", (cudaStream_t)stream);
     if (v_colors != nullptr && D > 0) {
         const uint64_t n_in = (uint64_t)n * D;
-        color_rows_bwd_kernel<<<div_up(n_in, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
+        launch_chained(color_rows_bwd_kernel, div_up(n_in, kThreads), kThreads, 0, (cudaStream_t)stream,
             n_in, N, D, width, camera_ids, gaussian_ids, colors_per_camera, v_rows, v_colors);
     }
     if (v_depths != nullptr)
-        last_channel_kernel<<<div_up(n, kThreads), kThreads, 0, (cudaStream_t)stream>>>(n, width, v_rows, v_depths_in, v_depths);
+        launch_chained(last_channel_kernel, div_up(n, kThreads), kThreads, 0, (cudaStream_t)stream, n, width, v_rows, v_depths_in, v_depths);
     return check_launch("color_rows_bwd");
 }

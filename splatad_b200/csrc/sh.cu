@@ -364,6 +364,7 @@ __device__ __forceinline__ void scatter_rows_add(float *__restrict__ dst, const 
 
 __global__ void __launch_bounds__(kShThreads)
 sh_colors_fwd_kernel(const ShColorArgs a, float *__restrict__ colors) {
+    chain_enter();
     extern __shared__ __align__(16) float sm[];   // [kShThreads][3K+1] floats, then the row indices
     const uint32_t row = 3 * a.K;
     int64_t *rows = reinterpret_cast<int64_t *>(sm + ((kShThreads * (row + 1) + 1) & ~1u));
@@ -416,6 +417,7 @@ sh_colors_fwd_kernel(const ShColorArgs a, float *__restrict__ colors) {
 __global__ void __launch_bounds__(kShThreads)
 sh_colors_bwd_kernel(const ShColorArgs a, const float *__restrict__ v_colors, float *__restrict__ v_coeffs,
                      float *__restrict__ v_means, float *__restrict__ v_campos, float *__restrict__ v_depths) {
+    chain_enter();
     extern __shared__ __align__(16) float sm[];
     const uint32_t row = 3 * a.K;
     int64_t *rows = reinterpret_cast<int64_t *>(sm + ((kShThreads * (row + 1) + 1) & ~1u));
@@ -531,6 +533,7 @@ sh_colors_bwd_kernel(const ShColorArgs a, const float *__restrict__ v_colors, fl
 // Camera centres in world coordinates, the translation column of inverse(viewmat), by cofactors
 // in double precision (the general 4 x 4 inverse: the last row need not be 0 0 0 1).
 __global__ void camera_centers_kernel(uint32_t C, const float *__restrict__ viewmats, float *__restrict__ campos) {
+    chain_enter();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     double m[4][4];
@@ -591,7 +594,7 @@ extern "C" int splatad_sh_colors_fwd(uint32_t n_elems, uint32_t N, uint32_t K, u
         cudaFuncSetAttribute(sh_colors_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     {
         SPL_PROF("sh_colors_fwd_kernel", (cudaStream_t)stream);
-        sh_colors_fwd_kernel<<<div_up(n_elems, kShThreads), kShThreads, smem, (cudaStream_t)stream>>>(a, colors);
+        launch_chained(sh_colors_fwd_kernel, div_up(n_elems, kShThreads), kShThreads, smem, (cudaStream_t)stream, a, colors);
     }
     return check_launch("sh_colors_fwd");
 }
@@ -614,7 +617,7 @@ extern "C" int splatad_sh_colors_bwd(uint32_t n_elems, uint32_t N, uint32_t K, u
         cudaFuncSetAttribute(sh_colors_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     {
         SPL_PROF("sh_colors_bwd_kernel", (cudaStream_t)stream);
-        sh_colors_bwd_kernel<<<div_up(n_elems, kShThreads), kShThreads, smem, (cudaStream_t)stream>>>(
+        launch_chained(sh_colors_bwd_kernel, div_up(n_elems, kShThreads), kShThreads, smem, (cudaStream_t)stream,
             a, v_colors, v_coeffs, v_means, v_campos, v_depths);
     }
     return check_launch("sh_colors_bwd");
@@ -665,6 +668,6 @@ extern "C" int splatad_sh_bwd(uint32_t n_elems, uint32_t K, uint32_t degrees_to_
 extern "C" int splatad_camera_centers(uint32_t C, const float *viewmats, float *campos, void *stream) {
     if (C == 0) return SPLATAD_OK;
     SPL_REQUIRE(viewmats && campos, SPLATAD_ERR_BAD_ARG, "camera_centers: null argument");
-    camera_centers_kernel<<<div_up(C, 64), 64, 0, (cudaStream_t)stream>>>(C, viewmats, campos);
+    launch_chained(camera_centers_kernel, div_up(C, 64), 64, 0, (cudaStream_t)stream, C, viewmats, campos);
     return check_launch("camera_centers");
 }
