@@ -533,62 +533,251 @@ projection_fwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
 
 // ---------------------------------------------------------------------------------------
 // Camera forward, packed (COO) layout: rows ordered camera-major, Gaussian-minor.
-// Pass 1 (block_counts != nullptr) counts the visible Gaussians of each (camera, block);
-// pass 2 (block_offsets != nullptr) recomputes and writes rows at the scanned offsets.
+// The count pass finds out which (camera, Gaussian) pairs are visible, the fill pass projects those
+// and writes their rows at the scanned offsets. Both hold a block's Gaussians in shared memory and
+// project from a queue of pairs: a camera of a surround rig sees about a sixth of the Gaussians, and
+// projecting them in place left most lanes of every warp waiting for the few that passed the culling
+// (374 us for both passes over two million Gaussians and six cameras, bound by instruction issue; 225
+// this way, 126 of them in the count). The count pass queues what a bound on the extent cannot rule out, projects
+// exactly that, and leaves one bit per pair; the fill pass queues the pairs whose bit is set.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads)
-projection_packed_fwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
-                             const float *__restrict__ covars, const float *__restrict__ quats,
-                             const float *__restrict__ scales, const float *__restrict__ velocities,
-                             const float *__restrict__ viewmats, const float *__restrict__ Ks,
-                             int width, int height, const float *__restrict__ lin_vel,
-                             const float *__restrict__ ang_vel, const float *__restrict__ rs_time,
-                             float eps2d, float near_plane, float far_plane, float radius_clip,
-                             int32_t *__restrict__ block_counts,        // [C, nblocks] pass 1
-                             const int32_t *__restrict__ block_offsets, // [C, nblocks] pass 2 (exclusive)
-                             int64_t capacity /* rows the outputs hold; < 0: as many as needed */,
-                             const int32_t *__restrict__ counts_ro /* pass 2, capacity >= 0: pass 1's counts */,
-                             int64_t *__restrict__ camera_ids, int64_t *__restrict__ gaussian_ids,
-                             int32_t *__restrict__ radii, float *__restrict__ means2d,
-                             float *__restrict__ depths, float *__restrict__ conics,
-                             float *__restrict__ compensations, float *__restrict__ pix_vels) {
-    chain_enter();
-    __shared__ __align__(16) float smem[kStageFloats];
-    __shared__ int32_t warp_counts[kThreads / 32];
-    const uint32_t g0 = blockIdx.x * kThreads;
-    const uint32_t n = min((uint32_t)kThreads, N - g0);
-    const uint32_t t = threadIdx.x;
-    const bool live = t < n;
-    const uint32_t lane = t & 31, warp = t >> 5;
-    GaussIn in = load_gaussian<false>(means, covars, quats, scales, velocities, N, g0, smem);
-    const Sym3 covar = to_sym(in.covar);
+constexpr uint32_t kPackedCams = 8;   // cameras a queue covers: kPackedCams * kThreads pairs
+constexpr uint32_t kPackedWords = kThreads / 32;
 
-    for (uint32_t c = 0; c < C; ++c) {
-        SensorCam s = load_cam(viewmats, Ks, lin_vel, ang_vel, rs_time, c);
-        CamProj o = project_cam(s, cam_limits(s.K, width, height), in.mean, covar, velocities != nullptr, in.vel,
-                                width, height, eps2d, near_plane, far_plane, radius_clip);
-        const bool vis = live && o.valid;
-        const uint32_t ballot = __ballot_sync(0xffffffffu, vis);
-        if (lane == 0) warp_counts[warp] = __popc(ballot);
-        __syncthreads();
-        int32_t before = 0, total = 0;
+struct PackedShared {
+    __align__(16) float gauss[kStageFloats];   // means [256*3] | velocities [256*3] | covariances [6][256]
+    SensorCam cam[kPackedCams];
+    CamLimits lim[kPackedCams];
+    float stretch[kPackedCams];                // bound on the squared norm of the world-to-camera rotation
+    uint32_t mask[kPackedCams][kPackedWords];
+    uint32_t before[kPackedCams][kPackedWords];
+    uint32_t start[kPackedCams + 1];
+    uint16_t queue[kPackedCams * kThreads];    // camera << 8 | Gaussian
+};
+static_assert(kThreads == 256, "a queue entry holds the Gaussian in eight bits");
+
+// Largest absolute row sum of R R^T: 1 for a rotation, never below the squared spectral norm.
+__device__ __forceinline__ float stretch_bound(const M3 &R) {
+    float most = 0.f;
 #pragma unroll
-        for (int w = 0; w < kThreads / 32; ++w) {
-            const int32_t cw = warp_counts[w];
-            if (w < (int)warp) before += cw;
-            total += cw;
+    for (int i = 0; i < 3; ++i) {
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            sum += fabsf(R.m[i][0] * R.m[j][0] + R.m[i][1] * R.m[j][1] + R.m[i][2] * R.m[j][2]);
+        most = fmaxf(most, sum);
+    }
+    return most;
+}
+
+// True only where project_cam is certain to cull: outside the depth range, or outside the image by
+// an extent that is never below the one project_cam finds. A row j of the Jacobian gives the
+// variance j^T S j <= |S| |j|^2, with the Frobenius norm for |S|; the margins (0.1 % of the extent,
+// 0.01 pixel, 1e-5 of the terms that cancel in the mean) are orders above the rounding of either
+// side. Comparisons with a NaN are false, which leaves the pair to project_cam.
+__device__ __forceinline__ bool surely_culled(const SensorCam &s, const CamLimits &lim, float stretch, V3 mean,
+                                              float norm, bool has_vel, V3 vel_w, int width, int height,
+                                              float eps2d, float near_plane, float far_plane, float radius_clip) {
+    const V3 p = mul(s.pose.R, mean) + s.pose.t;
+    if (p.z < near_plane || p.z > far_plane) return true;
+    const float rz = __fdividef(1.f, p.z);
+    const float xr = p.x * rz, yr = p.y * rz;
+    const float txr = fminf(lim.x_pos, fmaxf(-lim.x_neg, xr)), tyr = fminf(lim.y_pos, fmaxf(-lim.y_neg, yr));
+    const float j00 = fabsf(s.K.fx * rz), j11 = fabsf(s.K.fy * rz);
+    const float j02 = fabsf(j00 * txr), j12 = fabsf(j11 * tyr);
+    const float top = norm * stretch;
+    const float vx = top * (j00 * j00 + j02 * j02) + eps2d, vy = top * (j11 * j11 + j12 * j12) + eps2d;
+    float ex = 3.003f * vx * rsqrtf(vx), ey = 3.003f * vy * rsqrtf(vy);   // a NaN for a variance of zero
+    if (ex <= radius_clip && ey <= radius_clip) return true;
+    if (s.rs_time > 0.f) {
+        V3 tv = s.lin + cross(s.ang, p);
+        if (has_vel) tv = tv - mul(s.pose.R, vel_w);
+        const float half_time = 0.5005f * s.rs_time;
+        ex += (j00 * fabsf(tv.x) + j02 * fabsf(tv.z)) * half_time;
+        ey += (j11 * fabsf(tv.y) + j12 * fabsf(tv.z)) * half_time;
+    }
+    const float mx = s.K.fx * xr, my = s.K.fy * yr;
+    ex += 0.01f + 1e-5f * (fabsf(mx) + fabsf(s.K.cx));
+    ey += 0.01f + 1e-5f * (fabsf(my) + fabsf(s.K.cy));
+    const float x = mx + s.K.cx, y = my + s.K.cy;
+    return x + ex <= 0.f || x - ex >= (float)width || y + ey <= 0.f || y - ey >= (float)height;
+}
+
+__device__ __forceinline__ void packed_load_cameras(PackedShared &sh, const float *viewmats, const float *Ks,
+                                                    const float *lin_vel, const float *ang_vel,
+                                                    const float *rs_time, uint32_t c0, uint32_t nc, int width,
+                                                    int height) {
+    if (threadIdx.x < nc) {
+        const uint32_t c = threadIdx.x;
+        const SensorCam s = load_cam(viewmats, Ks, lin_vel, ang_vel, rs_time, c0 + c);
+        sh.cam[c] = s;
+        sh.lim[c] = cam_limits(s.K, width, height);
+        sh.stretch[c] = stretch_bound(s.pose.R);
+    }
+}
+
+// This thread's covariance into shared memory; returns its Frobenius norm.
+__device__ __forceinline__ float packed_keep_covariance(PackedShared &sh, const GaussIn &in) {
+    const Sym3 S = to_sym(in.covar);
+    float *covar = sh.gauss + kThreads * 6 + threadIdx.x;
+    covar[0] = S.xx; covar[kThreads] = S.xy; covar[2 * kThreads] = S.xz;
+    covar[3 * kThreads] = S.yy; covar[4 * kThreads] = S.yz; covar[5 * kThreads] = S.zz;
+    return sqrtf(S.xx * S.xx + S.yy * S.yy + S.zz * S.zz + 2.f * (S.xy * S.xy + S.xz * S.xz + S.yz * S.yz));
+}
+
+__device__ __forceinline__ CamProj packed_project(const PackedShared &sh, uint32_t c, uint32_t g, bool has_vel,
+                                                  int width, int height, float eps2d, float near_plane,
+                                                  float far_plane, float radius_clip) {
+    const float *covar = sh.gauss + kThreads * 6 + g;
+    Sym3 S;
+    S.xx = covar[0]; S.xy = covar[kThreads]; S.xz = covar[2 * kThreads];
+    S.yy = covar[3 * kThreads]; S.yz = covar[4 * kThreads]; S.zz = covar[5 * kThreads];
+    const V3 vel = has_vel ? ld3(sh.gauss + kThreads * 3 + 3 * g) : v3(0.f, 0.f, 0.f);
+    return project_cam(sh.cam[c], sh.lim[c], ld3(sh.gauss + 3 * g), S, has_vel, vel, width, height, eps2d,
+                       near_plane, far_plane, radius_clip);
+}
+
+// Blocks per SM by measurement, same scene: the count with 4 of them 146 us, 5 126, 6 129 (spills); the
+// fill 110 with 4, 105 with 5, 99 with 6 (whose 44 bytes of spills cost less than the waiting they fill).
+__global__ void __launch_bounds__(kThreads, 5)
+projection_packed_count_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
+                               const float *__restrict__ covars, const float *__restrict__ quats,
+                               const float *__restrict__ scales, const float *__restrict__ velocities,
+                               const float *__restrict__ viewmats, const float *__restrict__ Ks,
+                               int width, int height, const float *__restrict__ lin_vel,
+                               const float *__restrict__ ang_vel, const float *__restrict__ rs_time,
+                               float eps2d, float near_plane, float far_plane, float radius_clip,
+                               int32_t *__restrict__ block_counts,   // [C, nblocks]
+                               uint32_t *__restrict__ masks /* [C, nblocks, 8] or null */) {
+    chain_enter();
+    __shared__ PackedShared sh;
+    __shared__ uint32_t queued;
+    const uint32_t g0 = blockIdx.x * kThreads;
+    const uint32_t t = threadIdx.x, lane = t & 31;
+    const bool live = t < min((uint32_t)kThreads, N - g0), has_vel = velocities != nullptr;
+    packed_load_cameras(sh, viewmats, Ks, lin_vel, ang_vel, rs_time, 0, min(C, kPackedCams), width, height);
+    const GaussIn in = load_gaussian<false>(means, covars, quats, scales, velocities, N, g0, sh.gauss);
+    const float norm = packed_keep_covariance(sh, in);
+
+    for (uint32_t c0 = 0; c0 < C; c0 += kPackedCams) {
+        const uint32_t nc = min(C - c0, kPackedCams);
+        if (c0 > 0) {
+            __syncthreads();
+            packed_load_cameras(sh, viewmats, Ks, lin_vel, ang_vel, rs_time, c0, nc, width, height);
+        }
+        if (t < kPackedCams * kPackedWords) (&sh.mask[0][0])[t] = 0;
+        if (t == 0) queued = 0;
+        __syncthreads();
+#pragma unroll 1
+        for (uint32_t c = 0; c < nc; ++c) {
+            const bool keep = live && !surely_culled(sh.cam[c], sh.lim[c], sh.stretch[c], in.mean, norm, has_vel,
+                                                     in.vel, width, height, eps2d, near_plane, far_plane,
+                                                     radius_clip);
+            const uint32_t ballot = __ballot_sync(0xffffffffu, keep);
+            uint32_t base = 0;
+            if (lane == 0 && ballot != 0) base = atomicAdd(&queued, (uint32_t)__popc(ballot));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (keep) sh.queue[base + __popc(ballot & ((1u << lane) - 1u))] = (uint16_t)(c << 8 | t);
         }
         __syncthreads();
-        if (block_counts != nullptr) {
-            if (t == 0) block_counts[(size_t)c * gridDim.x + blockIdx.x] = total;
-            continue;
+        const uint32_t pairs = queued;
+#pragma unroll 1
+        for (uint32_t i = t; i < pairs; i += kThreads) {
+            const uint32_t c = sh.queue[i] >> 8, g = sh.queue[i] & 255u;
+            if (packed_project(sh, c, g, has_vel, width, height, eps2d, near_plane, far_plane, radius_clip).valid)
+                atomicOr(&sh.mask[c][g >> 5], 1u << (g & 31));
         }
-        if (vis) {
-            const int64_t row = (int64_t)block_offsets[(size_t)c * gridDim.x + blockIdx.x] + before +
-                                __popc(ballot & ((1u << lane) - 1u));
+        __syncthreads();
+        if (t < kPackedCams * kPackedWords) {
+            const uint32_t c = t / kPackedWords, w = t % kPackedWords, word = sh.mask[c][w];
+            uint32_t count = __popc(word);
+#pragma unroll
+            for (int off = kPackedWords / 2; off > 0; off >>= 1) count += __shfl_xor_sync(0xffffffffu, count, off);
+            if (c < nc) {
+                const size_t at = (size_t)(c0 + c) * gridDim.x + blockIdx.x;
+                if (masks != nullptr) masks[at * kPackedWords + w] = word;
+                if (w == 0) block_counts[at] = (int32_t)count;
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, 6)
+projection_packed_fill_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
+                              const float *__restrict__ covars, const float *__restrict__ quats,
+                              const float *__restrict__ scales, const float *__restrict__ velocities,
+                              const float *__restrict__ viewmats, const float *__restrict__ Ks,
+                              int width, int height, const float *__restrict__ lin_vel,
+                              const float *__restrict__ ang_vel, const float *__restrict__ rs_time,
+                              float eps2d, float near_plane, float far_plane, float radius_clip,
+                              const int32_t *__restrict__ block_counts,   // [C, nblocks]
+                              const int32_t *__restrict__ block_offsets,  // [C, nblocks] (exclusive)
+                              const uint32_t *__restrict__ masks,         // [C, nblocks, 8]
+                              int64_t capacity /* rows the outputs hold; < 0: as many as needed */,
+                              int64_t *__restrict__ camera_ids, int64_t *__restrict__ gaussian_ids,
+                              int32_t *__restrict__ radii, float *__restrict__ means2d,
+                              float *__restrict__ depths, float *__restrict__ conics,
+                              float *__restrict__ compensations, float *__restrict__ pix_vels) {
+    chain_enter();
+    __shared__ PackedShared sh;
+    __shared__ int64_t first_row[kPackedCams];   // row of the camera's first pair, less its place in the queue
+    const uint32_t g0 = blockIdx.x * kThreads;
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const bool has_vel = velocities != nullptr;
+    for (uint32_t c0 = 0; c0 < C; c0 += kPackedCams) {
+        const uint32_t nc = min(C - c0, kPackedCams);
+        if (c0 > 0) __syncthreads();
+        int32_t offset = 0;
+        if (t < kPackedCams * kPackedWords) {
+            const uint32_t c = t / kPackedWords, w = t % kPackedWords;
+            const size_t at = (size_t)(c0 + c) * gridDim.x + blockIdx.x;
+            const uint32_t word = c < nc ? masks[at * kPackedWords + w] : 0u;
+            if (c < nc) offset = block_offsets[at];
+            uint32_t inc = __popc(word);
+#pragma unroll
+            for (int off = 1; off < (int)kPackedWords; off <<= 1) {
+                const uint32_t o = __shfl_up_sync(0xffffffffu, inc, off, kPackedWords);
+                if (w >= (uint32_t)off) inc += o;
+            }
+            sh.mask[c][w] = word;
+            sh.before[c][w] = inc - __popc(word);
+            if (w == kPackedWords - 1) sh.start[c + 1] = inc;
+        }
+        packed_load_cameras(sh, viewmats, Ks, lin_vel, ang_vel, rs_time, c0, nc, width, height);
+        if (c0 == 0) {
+            const GaussIn in = load_gaussian<false>(means, covars, quats, scales, velocities, N, g0, sh.gauss);
+            packed_keep_covariance(sh, in);
+        } else {
+            __syncthreads();
+        }
+        if (t < kPackedCams * kPackedWords && t % kPackedWords == 0) {
+            const uint32_t c = t / kPackedWords;
+            uint32_t start = 0;
+            for (uint32_t k = 0; k < c; ++k) start += sh.start[k + 1];
+            first_row[c] = (int64_t)offset - start;
+            sh.before[c][0] = start;   // the first word's count before it is zero: its place holds the start
+        }
+        __syncthreads();
+        uint32_t pairs = 0;
+#pragma unroll
+        for (uint32_t c = 0; c < kPackedCams; ++c) pairs += sh.start[c + 1];
+#pragma unroll 1
+        for (uint32_t c = 0; c < nc; ++c) {
+            const uint32_t word = sh.mask[c][warp];
+            if (word >> lane & 1u) {
+                const uint32_t before = sh.before[c][0] + (warp > 0 ? sh.before[c][warp] : 0u);
+                sh.queue[before + __popc(word & ((1u << lane) - 1u))] = (uint16_t)(c << 8 | t);
+            }
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (uint32_t i = t; i < pairs; i += kThreads) {
+            const uint32_t c = sh.queue[i] >> 8, g = sh.queue[i] & 255u;
+            const int64_t row = first_row[c] + i;
             if (capacity >= 0 && row >= capacity) continue;   // the caller sees nnz > capacity and refills
-            camera_ids[row] = (int64_t)c;
-            gaussian_ids[row] = (int64_t)(g0 + t);
+            const CamProj o = packed_project(sh, c, g, has_vel, width, height, eps2d, near_plane, far_plane, radius_clip);
+            camera_ids[row] = (int64_t)(c0 + c);
+            gaussian_ids[row] = (int64_t)(g0 + g);
             radii[2 * row] = (int32_t)o.ex;
             radii[2 * row + 1] = (int32_t)o.ey;
             means2d[2 * row] = o.mean2d.x;
@@ -604,9 +793,9 @@ projection_packed_fwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ m
     }
     // Outputs with room to spare (written before the host knows the row count): the rows behind the
     // last packed one get ids 0 and radii 0, which every consumer skips.
-    if (block_counts == nullptr && capacity >= 0 && counts_ro != nullptr) {
+    if (capacity >= 0) {
         const size_t last = (size_t)C * gridDim.x - 1;
-        const int64_t nnz = (int64_t)block_offsets[last] + counts_ro[last];
+        const int64_t nnz = (int64_t)block_offsets[last] + block_counts[last];
         for (int64_t r = nnz + (int64_t)blockIdx.x * kThreads + t; r < capacity; r += (int64_t)gridDim.x * kThreads) {
             camera_ids[r] = 0;
             gaussian_ids[r] = 0;
@@ -1274,8 +1463,8 @@ extern "C" int splatad_projection_bwd(
 }
 
 extern "C" size_t splatad_projection_packed_workspace_bytes(uint32_t C, uint32_t N) {
-    // block counts + block offsets
-    return 2 * sizeof(int32_t) * (size_t)C * div_up(N, kThreads) + 256;
+    // block counts + block offsets + one bit per (camera, Gaussian)
+    return (2 + kPackedWords) * sizeof(int32_t) * (size_t)C * div_up(N, kThreads) + 256;
 }
 
 extern "C" int splatad_projection_packed_count(
@@ -1298,12 +1487,11 @@ extern "C" int splatad_projection_packed_count(
     int32_t *offsets = counts + (size_t)C * nblocks;
     cudaStream_t st = (cudaStream_t)stream;
     {
-        SPL_PROF("projection_packed_fwd_kernel", st);
-        launch_chained(projection_packed_fwd_kernel, nblocks, kThreads, 0, st,
+        SPL_PROF("projection_packed_count_kernel", st);
+        launch_chained(projection_packed_count_kernel, nblocks, kThreads, 0, st,
             C, N, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
             linear_velocity, angular_velocity, rolling_shutter_time, eps2d, near_plane, far_plane,
-            radius_clip, counts, nullptr, (int64_t)-1, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-            nullptr, nullptr, nullptr);
+            radius_clip, counts, reinterpret_cast<uint32_t *>(offsets + (size_t)C * nblocks));
     }
     {
         SPL_PROF("packed_scan_kernel", st);
@@ -1330,11 +1518,12 @@ extern "C" int splatad_projection_packed_fill(
     const uint32_t nblocks = div_up(N, kThreads);
     const int32_t *offsets = (const int32_t *)workspace + (size_t)C * nblocks;
     {
-        SPL_PROF("projection_packed_fwd_kernel", (cudaStream_t)stream);
-        launch_chained(projection_packed_fwd_kernel, nblocks, kThreads, 0, (cudaStream_t)stream,
+        SPL_PROF("projection_packed_fill_kernel", (cudaStream_t)stream);
+        launch_chained(projection_packed_fill_kernel, nblocks, kThreads, 0, (cudaStream_t)stream,
             C, N, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
             linear_velocity, angular_velocity, rolling_shutter_time, eps2d, near_plane, far_plane,
-            radius_clip, nullptr, offsets, capacity, (const int32_t *)workspace, camera_ids, gaussian_ids, radii,
+            radius_clip, (const int32_t *)workspace, offsets,
+            reinterpret_cast<const uint32_t *>(offsets + (size_t)C * nblocks), capacity, camera_ids, gaussian_ids, radii,
             means2d, depths, conics, compensations, pix_vels);
     }
     return check_launch("projection_packed_fill");
@@ -1440,11 +1629,10 @@ extern "C" int splatad_projection_packed_count_noalloc(
     cudaStream_t st = (cudaStream_t)stream;
     // every slot the scan reads is written by the count pass of this same call: nothing in the
     // scratch needs clearing, and what earlier (larger) calls left behind is never read
-    launch_chained(projection_packed_fwd_kernel, (uint32_t)nblocks, kThreads, 0, st,
+    launch_chained(projection_packed_count_kernel, (uint32_t)nblocks, kThreads, 0, st,
         C, N, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
         linear_velocity, angular_velocity, rolling_shutter_time, eps2d, near_plane, far_plane,
-        radius_clip, counts, nullptr, (int64_t)-1, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-        nullptr, nullptr);
+        radius_clip, counts, nullptr);
     launch_chained(packed_scan_kernel, 1, 1024, 0, st, counts, offsets, C, (uint32_t)nblocks, indptr, nnz_device);
     return check_launch("projection_packed_count_noalloc");
 }

@@ -191,6 +191,37 @@ def test_camera_projection_packed_matches_unpacked():
     assert torch.equal(p_pix_vels, pix_vels[c_ref, g_ref])
 
 
+@pytest.mark.parametrize("N,C,use_covars,kw", [
+    (1, 1, False, {}), (255, 9, False, {}), (256, 8, True, {}), (257, 17, False, dict(radius_clip=6.0)),
+    (40000, 6, False, {}), (40000, 9, True, dict(eps2d=0.0)), (40000, 3, False, dict(near_plane=-5.0)),
+])
+def test_camera_projection_packed_selects_what_the_dense_kernel_keeps(N, C, use_covars, kw):
+    """The packed pass rules pairs out by a bound on their extent before it projects them: block and
+    camera-group remainders, a rolling shutter, a world-to-camera matrix that is no rotation, no blur, a
+    minimum radius, and points behind the camera must select exactly the pairs of the dense kernel."""
+    from splatad_b200 import ops
+
+    means, quats, scales, vel, g = _scene(N, 31 + N, "cam")
+    scales = scales * torch.exp(torch.randn(N, 3, generator=g))
+    vm, Ks, lin, ang, rs = (x.repeat_interleave((C + 1) // 2, 0)[:C].clone() for x in _camera_sensors(g))
+    vm[:, :3, 3] += torch.randn(C, 3, generator=g)
+    vm[C // 2, :3, :3] = vm[C // 2, :3, :3] @ torch.tensor([[1.5, 0.4, 0.0], [0.0, 0.7, 0.0], [0.0, 0.2, 1.2]])
+    covars = None
+    if use_covars:
+        from oracle import projection as op
+        i, j = torch.triu_indices(3, 3)
+        covars = t(op.quat_scale_to_covar(quats, scales)[:, i, j])
+    args = (t(means), covars, None if use_covars else t(quats), None if use_covars else t(scales), t(vel), t(vm), t(Ks),
+            320, 240, t(lin), t(ang), t(rs))
+    options = {**CAM_KW, **kw}
+    dense = ops.fully_fused_projection(*args, calc_compensations=True, **options)
+    packed = ops.fully_fused_projection(*args, packed=True, calc_compensations=True, **options)
+    c_ref, g_ref = torch.nonzero(dense[3].abs().sum(-1) > 0, as_tuple=True)
+    assert torch.equal(packed[0], c_ref) and torch.equal(packed[1], g_ref)
+    for p_out, d_out in zip(packed[2:], dense):
+        assert torch.equal(p_out, d_out[c_ref, g_ref])
+
+
 def test_camera_projection_packed_repeated_frames_fill_ahead_of_the_count():
     """From the second frame of a shape on the packed rows are written before the host has the
     count (into room sized from the previous frame) and cut to length afterwards; a frame that
