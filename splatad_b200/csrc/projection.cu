@@ -277,7 +277,6 @@ constexpr int kStageFloats = kThreads * 12;
 
 // Issues every global->shared copy of this block's slab first and synchronises once, so the
 // loads of all arrays are in flight together.
-template <bool kNeedQS>
 __device__ __forceinline__ GaussIn load_gaussian(const float *__restrict__ means,
                                                  const float *__restrict__ covars,
                                                  const float *__restrict__ quats,
@@ -336,7 +335,7 @@ lidar_projection_fwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ me
     const uint32_t n = min((uint32_t)kThreads, N - g0);
     const uint32_t t = threadIdx.x;
     const bool live = t < n;
-    GaussIn in = load_gaussian<false>(means, covars, quats, scales, velocities, N, g0, smem);
+    GaussIn in = load_gaussian(means, covars, quats, scales, velocities, N, g0, smem);
     const Sym3 covar = to_sym(in.covar);
 
     for (uint32_t c = 0; c < C; ++c) {
@@ -507,7 +506,7 @@ projection_fwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
     const uint32_t n = min((uint32_t)kThreads, N - g0);
     const uint32_t t = threadIdx.x;
     const bool live = t < n;
-    GaussIn in = load_gaussian<false>(means, covars, quats, scales, velocities, N, g0, smem);
+    GaussIn in = load_gaussian(means, covars, quats, scales, velocities, N, g0, smem);
     const Sym3 covar = to_sym(in.covar);
 
     for (uint32_t c = 0; c < C; ++c) {
@@ -656,7 +655,7 @@ projection_packed_count_kernel(uint32_t C, uint32_t N, const float *__restrict__
     const uint32_t t = threadIdx.x, lane = t & 31;
     const bool live = t < min((uint32_t)kThreads, N - g0), has_vel = velocities != nullptr;
     packed_load_cameras(sh, viewmats, Ks, lin_vel, ang_vel, rs_time, 0, min(C, kPackedCams), width, height);
-    const GaussIn in = load_gaussian<false>(means, covars, quats, scales, velocities, N, g0, sh.gauss);
+    const GaussIn in = load_gaussian(means, covars, quats, scales, velocities, N, g0, sh.gauss);
     const float norm = packed_keep_covariance(sh, in);
 
     for (uint32_t c0 = 0; c0 < C; c0 += kPackedCams) {
@@ -745,7 +744,7 @@ projection_packed_fill_kernel(uint32_t C, uint32_t N, const float *__restrict__ 
         }
         packed_load_cameras(sh, viewmats, Ks, lin_vel, ang_vel, rs_time, c0, nc, width, height);
         if (c0 == 0) {
-            const GaussIn in = load_gaussian<false>(means, covars, quats, scales, velocities, N, g0, sh.gauss);
+            const GaussIn in = load_gaussian(means, covars, quats, scales, velocities, N, g0, sh.gauss);
             packed_keep_covariance(sh, in);
         } else {
             __syncthreads();
@@ -982,58 +981,58 @@ __device__ __forceinline__ void covar_grad_to_triu(const M3 &g, float *o) {
     o[5] = g.m[2][2];
 }
 
-// Writes the per-Gaussian parameter gradients of this block (means, and covars or
-// quats+scales, optionally velocities) through shared memory.
-__device__ __forceinline__ void store_param_grads(const GaussIn &in, bool use_covars, bool touched, V3 v_mean,
-                                                  const M3 &v_covar, V3 v_vel_w, uint32_t g0,
-                                                  uint32_t n, float *smem, float *v_means,
-                                                  float *v_covars, float *v_quats, float *v_scales,
-                                                  float *v_velocities) {
-    const uint32_t t = threadIdx.x;
-    const bool live = t < n;
-    if (v_means != nullptr) {
-        if (live) { smem[3 * t] = v_mean.x; smem[3 * t + 1] = v_mean.y; smem[3 * t + 2] = v_mean.z; }
-        __syncthreads();
-        stage_out(v_means + (size_t)g0 * 3, smem, n * 3);
-        __syncthreads();
-    }
-    if (v_velocities != nullptr) {
-        if (live) { smem[3 * t] = v_vel_w.x; smem[3 * t + 1] = v_vel_w.y; smem[3 * t + 2] = v_vel_w.z; }
-        __syncthreads();
-        stage_out(v_velocities + (size_t)g0 * 3, smem, n * 3);
-        __syncthreads();
-    }
+// Gradients of Gaussian g. Rows are stored as they come from the queue of the kernels below; the L2
+// merges what consecutive lanes write.
+__device__ __forceinline__ void store3(float *base, size_t g, V3 v) {
+    if (base == nullptr) return;
+    base[3 * g] = v.x; base[3 * g + 1] = v.y; base[3 * g + 2] = v.z;
+}
+
+__device__ __forceinline__ void store_param_grads(const GaussIn &in, bool use_covars, size_t g, V3 v_mean, const M3 &v_covar,
+                                                  V3 v_vel_w, float *v_means, float *v_covars, float *v_quats,
+                                                  float *v_scales, float *v_velocities) {
+    store3(v_means, g, v_mean);
+    store3(v_velocities, g, v_vel_w);
     if (use_covars) {
-        if (v_covars != nullptr) {
-            if (live) covar_grad_to_triu(v_covar, smem + 6 * t);
-            __syncthreads();
-            stage_out(v_covars + (size_t)g0 * 6, smem, n * 6);
-            __syncthreads();
-        }
-    } else {
-        V4 v_quat; v_quat.x = v_quat.y = v_quat.z = v_quat.w = 0.f;
-        V3 v_scale = v3(0.f, 0.f, 0.f);
-        if (touched) {
-            M3 R = quat_to_rotmat(in.quat);
-            quat_scale_to_covar_vjp(in.quat, in.scale, R, v_covar, v_quat, v_scale);
-        }
-        if (v_quats != nullptr && live)
-            reinterpret_cast<float4 *>(v_quats)[g0 + t] = make_float4(v_quat.x, v_quat.y, v_quat.z, v_quat.w);
-        if (v_scales != nullptr) {
-            if (live) { smem[3 * t] = v_scale.x; smem[3 * t + 1] = v_scale.y; smem[3 * t + 2] = v_scale.z; }
-            __syncthreads();
-            stage_out(v_scales + (size_t)g0 * 3, smem, n * 3);
-            __syncthreads();
-        }
+        if (v_covars != nullptr) covar_grad_to_triu(v_covar, v_covars + 6 * g);
+        return;
     }
+    V4 v_quat; v_quat.x = v_quat.y = v_quat.z = v_quat.w = 0.f;
+    V3 v_scale = v3(0.f, 0.f, 0.f);
+    const M3 R = quat_to_rotmat(in.quat);
+    quat_scale_to_covar_vjp(in.quat, in.scale, R, v_covar, v_quat, v_scale);
+    if (v_quats != nullptr)
+        reinterpret_cast<float4 *>(v_quats)[g] = make_float4(v_quat.x, v_quat.y, v_quat.z, v_quat.w);
+    store3(v_scales, g, v_scale);
+}
+
+__device__ __forceinline__ GaussIn gather_gaussian(const float *__restrict__ means, const float *__restrict__ covars,
+                                                   const float *__restrict__ quats, const float *__restrict__ scales,
+                                                   const float *__restrict__ velocities, size_t g) {
+    GaussIn in;
+    in.mean = ld3(means + 3 * g);
+    in.vel = velocities != nullptr ? ld3(velocities + 3 * g) : v3(0.f, 0.f, 0.f);
+    if (covars != nullptr) {
+        in.covar = covar_from_triu(covars + 6 * g);
+    } else {
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(quats) + g);
+        in.quat.x = q.x; in.quat.y = q.y; in.quat.z = q.z; in.quat.w = q.w;
+        in.scale = ld3(scales + 3 * g);
+        in.covar = quat_scale_to_covar(in.quat, in.scale);
+    }
+    return in;
 }
 
 // ---------------------------------------------------------------------------------------
 // Every VJP is linear in the cotangents: a (sensor, Gaussian) pair whose cotangents are all zero adds
-// nothing, and a block without any other leaves zero gradients without reading its Gaussians. In a scene
-// whose sensors are saturated by what is near, that is nearly all of the blocks (lidar benchmark,
-// 1 M Gaussians: 110 -> 55 us). Gaussians that a camera sees are spread over all blocks: there only the
-// pairs are looked at (the block test took 5 of 33 us without finding a block). A NaN counts as nonzero.
+// nothing. In a scene whose sensors are saturated by what is near that is most pairs, and one thread per
+// Gaussian leaves the blocks waiting for the few lanes that have work. The [C, N] kernels therefore give
+// a block a span of up to kBwdSpan * 256 Gaussians: it reads the cotangents in order, 16 bytes at a time,
+// marks the Gaussians that have one, stores zeros over the span (unless all are marked) and works through
+// the queue of the marked ones. A NaN counts as nonzero.
+// Lidar scan, 1 M Gaussians: 55 us with one thread per Gaussian and blocks without a cotangent left out,
+// 39 with spans of 4 * 256, 31 with 8, 37 with 16 (too few blocks to share the work out evenly); camera,
+// 211 k Gaussians: 27 -> 23 us. Reading the cotangents and storing the zeros take 13 us of the 31.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ bool pair_nonzero(const float *v_mean2d, float v_depth, const float *v_conic, const float *v_comp,
                                              const float *v_vel, int n_vel, const float *v_dc) {
@@ -1045,21 +1044,74 @@ __device__ __forceinline__ bool pair_nonzero(const float *v_mean2d, float v_dept
            (v2 != 0.f) | (k != 0.f) | (d0 != 0.f) | (d1 != 0.f);
 }
 
-__device__ __forceinline__ bool slab_nonzero(const float *__restrict__ base, size_t first, uint32_t n) {
-    if (base == nullptr) return false;
-    const float *p = base + first;
-    bool any = false;
+constexpr uint32_t kBwdSpan = 8;
+
+struct BwdQueue {
+    uint32_t count;
+    __align__(4) uint8_t marked[kBwdSpan * kThreads];
+    uint16_t local[kBwdSpan * kThreads];
+};
+
+// Marks the Gaussians [0, n) of a span that have a nonzero among their K values at p.
+template <uint32_t K>
+__device__ __forceinline__ void mark_nonzero(BwdQueue &q, const float *__restrict__ p, uint32_t n) {
+    const uint32_t values = K * n;
     uint32_t i = threadIdx.x;
     if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
-        const uint32_t nvec = n >> 2;
+        const uint32_t nvec = values >> 2;
+#pragma unroll 4
         for (; i < nvec; i += kThreads) {
             const float4 v = __ldg(reinterpret_cast<const float4 *>(p) + i);
-            any = any || v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f;
+            if ((v.x != 0.f) | (v.y != 0.f) | (v.z != 0.f) | (v.w != 0.f)) {
+                if (v.x != 0.f) q.marked[4 * i / K] = 1;
+                if (v.y != 0.f) q.marked[(4 * i + 1) / K] = 1;
+                if (v.z != 0.f) q.marked[(4 * i + 2) / K] = 1;
+                if (v.w != 0.f) q.marked[(4 * i + 3) / K] = 1;
+            }
         }
         i = (nvec << 2) + threadIdx.x;
     }
-    for (; i < n; i += kThreads) any = any || __ldg(p + i) != 0.f;
-    return any;
+    for (; i < values; i += kThreads)
+        if (__ldg(p + i) != 0.f) q.marked[i / K] = 1;
+}
+
+// Gaussians of [first, first + n) with a cotangent, as q.local[0 .. q.count). Callers bring n <= kBwdSpan * 256.
+template <uint32_t kVel>
+__device__ __forceinline__ uint32_t queue_touched(BwdQueue &q, uint32_t C, uint32_t N, uint32_t first, uint32_t n,
+                                                  const float *__restrict__ v_means2d, const float *__restrict__ v_depths,
+                                                  const float *__restrict__ v_conics, const float *__restrict__ v_comps,
+                                                  const float *__restrict__ v_vels, const float *__restrict__ v_dcs) {
+    const uint32_t t = threadIdx.x, lane = t & 31;
+    for (uint32_t i = t; i < (n + 3) / 4; i += kThreads) reinterpret_cast<uint32_t *>(q.marked)[i] = 0;
+    if (t == 0) q.count = 0;
+    __syncthreads();
+    for (uint32_t c = 0; c < C; ++c) {
+        const size_t i = (size_t)c * N + first;
+        mark_nonzero<3>(q, v_conics + 3 * i, n);
+        mark_nonzero<2>(q, v_means2d + 2 * i, n);
+        mark_nonzero<1>(q, v_depths + i, n);
+        mark_nonzero<kVel>(q, v_vels + kVel * i, n);
+        if (v_dcs != nullptr) mark_nonzero<2>(q, v_dcs + 2 * i, n);
+        if (v_comps != nullptr) mark_nonzero<1>(q, v_comps + i, n);
+    }
+    __syncthreads();
+    for (uint32_t i0 = 0; i0 < n; i0 += kThreads) {
+        const uint32_t i = i0 + t;
+        const bool keep = i < n && q.marked[i] != 0;
+        const uint32_t ballot = __ballot_sync(0xffffffffu, keep);
+        uint32_t base = 0;
+        if (lane == 0 && ballot != 0) base = atomicAdd(&q.count, (uint32_t)__popc(ballot));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (keep) q.local[base + __popc(ballot & ((1u << lane) - 1u))] = (uint16_t)i;
+    }
+    __syncthreads();
+    return q.count;
+}
+
+// Gaussians per block: the whole span only where that still fills the two blocks each SM holds.
+static uint32_t bwd_span(uint32_t N) {
+    const uint32_t blocks = div_up(N, kThreads);
+    return kThreads * max(1u, min(kBwdSpan, blocks / (2 * 148)));
 }
 
 __device__ __forceinline__ void store_zeros(float *base, size_t first, uint32_t n) {
@@ -1090,7 +1142,7 @@ __device__ __forceinline__ void store_zero_param_grads(uint32_t g0, uint32_t n, 
 // Camera backward, [C, N] layout
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads)
-projection_bwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
+projection_bwd_kernel(uint32_t C, uint32_t N, uint32_t span, const float *__restrict__ means,
                       const float *__restrict__ covars, const float *__restrict__ quats,
                       const float *__restrict__ scales, const float *__restrict__ velocities,
                       const float *__restrict__ viewmats, const float *__restrict__ Ks, int width,
@@ -1105,47 +1157,54 @@ projection_bwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
                       float *__restrict__ v_scales, float *__restrict__ v_viewmats,
                       float *__restrict__ v_velocities) {
     chain_enter();
-    __shared__ __align__(16) float smem[kStageFloats];
+    __shared__ BwdQueue queue;
     __shared__ float red[(kThreads / 32) * 12];
-    const uint32_t g0 = blockIdx.x * kThreads;
-    const uint32_t n = min((uint32_t)kThreads, N - g0);
-    const uint32_t t = threadIdx.x;
-    const bool live = t < n;
-    GaussIn in = load_gaussian<true>(means, covars, quats, scales, velocities, N, g0, smem);
-
-    bool touched = false;
-    V3 v_mean = v3(0.f, 0.f, 0.f), v_vel_w = v3(0.f, 0.f, 0.f);
-    M3 v_covar = m3_zero();
-    for (uint32_t c = 0; c < C; ++c) {
-        SensorCam s = load_cam(viewmats, Ks, lin_vel, ang_vel, rs_time, c);
-        const size_t i = (size_t)c * N + g0 + t;
-        M3 v_R = m3_zero();
-        V3 v_t = v3(0.f, 0.f, 0.f);
-        if (live && radii[2 * i] > 0 &&
-            pair_nonzero(v_means2d + 2 * i, v_depths[i], v_conics + 3 * i, v_compensations ? v_compensations + i : nullptr,
-                         v_pix_vels + 2 * i, 2, nullptr)) {
-            touched = true;
-            const float cn[3] = {conics[3 * i], conics[3 * i + 1], conics[3 * i + 2]};
-            const float vcn[3] = {v_conics[3 * i], v_conics[3 * i + 1], v_conics[3 * i + 2]};
-            const bool has_comp = v_compensations != nullptr;
-            cam_pair_bwd(s, in, velocities != nullptr, width, height, eps2d, cn,
-                         has_comp ? compensations[i] : 0.f, has_comp,
-                         v2(v_means2d[2 * i], v_means2d[2 * i + 1]), v_depths[i], vcn,
-                         has_comp ? v_compensations[i] : 0.f,
-                         v2(v_pix_vels[2 * i], v_pix_vels[2 * i + 1]), v_mean, v_covar, v_R, v_t,
-                         v_vel_w);
-        }
-        if (v_viewmats != nullptr) block_reduce_viewmat(v_R, v_t, v_viewmats + 16 * c, red);
+    const uint32_t first = blockIdx.x * span, n = min(span, N - first);
+    const uint32_t count = queue_touched<2>(queue, C, N, first, n, v_means2d, v_depths, v_conics, v_compensations,
+                                            v_pix_vels, nullptr);
+    if (count < n) {
+        store_zero_param_grads(first, n, covars != nullptr, v_means, v_covars, v_quats, v_scales, v_velocities);
+        __syncthreads();   // the gradients below go over these zeros
     }
-    store_param_grads(in, covars != nullptr, touched, v_mean, v_covar, v_vel_w, g0, n, smem, v_means,
-                      v_covars, v_quats, v_scales, v_velocities);
+#pragma unroll 1
+    for (uint32_t k0 = 0; k0 < count; k0 += kThreads) {   // every thread: the viewmat reduction is the block's
+        const bool live = k0 + threadIdx.x < count;
+        if (v_viewmats == nullptr && !live) break;
+        const size_t g = first + queue.local[live ? k0 + threadIdx.x : k0];
+        const GaussIn in = gather_gaussian(means, covars, quats, scales, velocities, g);
+        V3 v_mean = v3(0.f, 0.f, 0.f), v_vel_w = v3(0.f, 0.f, 0.f);
+        M3 v_covar = m3_zero();
+        for (uint32_t c = 0; c < C; ++c) {
+            const SensorCam s = load_cam(viewmats, Ks, lin_vel, ang_vel, rs_time, c);
+            const size_t i = (size_t)c * N + g;
+            M3 v_R = m3_zero();
+            V3 v_t = v3(0.f, 0.f, 0.f);
+            if (live && radii[2 * i] > 0 &&
+                pair_nonzero(v_means2d + 2 * i, v_depths[i], v_conics + 3 * i, v_compensations ? v_compensations + i : nullptr,
+                             v_pix_vels + 2 * i, 2, nullptr)) {
+                const float cn[3] = {conics[3 * i], conics[3 * i + 1], conics[3 * i + 2]};
+                const float vcn[3] = {v_conics[3 * i], v_conics[3 * i + 1], v_conics[3 * i + 2]};
+                const bool has_comp = v_compensations != nullptr;
+                cam_pair_bwd(s, in, velocities != nullptr, width, height, eps2d, cn,
+                             has_comp ? compensations[i] : 0.f, has_comp,
+                             v2(v_means2d[2 * i], v_means2d[2 * i + 1]), v_depths[i], vcn,
+                             has_comp ? v_compensations[i] : 0.f,
+                             v2(v_pix_vels[2 * i], v_pix_vels[2 * i + 1]), v_mean, v_covar, v_R, v_t,
+                             v_vel_w);
+            }
+            if (v_viewmats != nullptr) block_reduce_viewmat(v_R, v_t, v_viewmats + 16 * c, red);
+        }
+        if (live)
+            store_param_grads(in, covars != nullptr, g, v_mean, v_covar, v_vel_w, v_means, v_covars, v_quats, v_scales,
+                              v_velocities);
+    }
 }
 
 // ---------------------------------------------------------------------------------------
 // Lidar backward, [C, N] layout
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads)
-lidar_projection_bwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ means,
+lidar_projection_bwd_kernel(uint32_t C, uint32_t N, uint32_t span, const float *__restrict__ means,
                             const float *__restrict__ covars, const float *__restrict__ quats,
                             const float *__restrict__ scales, const float *__restrict__ velocities,
                             const float *__restrict__ viewmats, const float *__restrict__ lin_vel,
@@ -1162,60 +1221,48 @@ lidar_projection_bwd_kernel(uint32_t C, uint32_t N, const float *__restrict__ me
                             float *__restrict__ v_scales, float *__restrict__ v_viewmats,
                             float *__restrict__ v_velocities) {
     chain_enter();
-    __shared__ __align__(16) float smem[kStageFloats];
+    __shared__ BwdQueue queue;
     __shared__ float red[(kThreads / 32) * 12];
-    const uint32_t g0 = blockIdx.x * kThreads;
-    const uint32_t n = min((uint32_t)kThreads, N - g0);
-    const uint32_t t = threadIdx.x;
-    const bool live = t < n;
-    bool any = false;
-    for (uint32_t c = 0; c < C; ++c) {
-        const size_t i0 = (size_t)c * N + g0;
-        any = any || slab_nonzero(v_conics, 3 * i0, 3 * n);
+    const uint32_t first = blockIdx.x * span, n = min(span, N - first);
+    const uint32_t count = queue_touched<3>(queue, C, N, first, n, v_means2d, v_depths, v_conics, v_compensations,
+                                            v_pix_vels, v_depth_comps);
+    if (count < n) {
+        store_zero_param_grads(first, n, covars != nullptr, v_means, v_covars, v_quats, v_scales, v_velocities);
+        __syncthreads();   // the gradients below go over these zeros
     }
-    // (the rest is looked at only where the first array, usually nonzero with the others, decides nothing)
-    any = __syncthreads_or(any);
-    for (uint32_t c = 0; c < C && !any; ++c) {
-        const size_t i0 = (size_t)c * N + g0;
-        any = any || slab_nonzero(v_means2d, 2 * i0, 2 * n);
-        any = any || slab_nonzero(v_depths, i0, n);
-        any = any || slab_nonzero(v_compensations, i0, n);
-        any = any || slab_nonzero(v_pix_vels, 3 * i0, 3 * n);
-        any = any || slab_nonzero(v_depth_comps, 2 * i0, 2 * n);
-    }
-    if (!__syncthreads_or(any)) {
-        store_zero_param_grads(g0, n, covars != nullptr, v_means, v_covars, v_quats, v_scales, v_velocities);
-        return;
-    }
-    GaussIn in = load_gaussian<true>(means, covars, quats, scales, velocities, N, g0, smem);
-
-    bool touched = false;
-    V3 v_mean = v3(0.f, 0.f, 0.f), v_vel_w = v3(0.f, 0.f, 0.f);
-    M3 v_covar = m3_zero();
-    for (uint32_t c = 0; c < C; ++c) {
-        SensorLidar s = load_lidar(viewmats, lin_vel, ang_vel, rs_time, c);
-        const size_t i = (size_t)c * N + g0 + t;
-        M3 v_R = m3_zero();
-        V3 v_t = v3(0.f, 0.f, 0.f);
-        if (live && radii[2 * i] > 0.f &&
-            pair_nonzero(v_means2d + 2 * i, v_depths[i], v_conics + 3 * i, v_compensations ? v_compensations + i : nullptr,
-                         v_pix_vels + 3 * i, 3, v_depth_comps + 2 * i)) {
-            touched = true;
-            const float cn[3] = {conics[3 * i], conics[3 * i + 1], conics[3 * i + 2]};
-            const float vcn[3] = {v_conics[3 * i], v_conics[3 * i + 1], v_conics[3 * i + 2]};
-            const bool has_comp = v_compensations != nullptr;
-            lidar_pair_bwd(s, in, velocities != nullptr, eps2d, cn,
-                           has_comp ? compensations[i] : 0.f, has_comp,
-                           v2(v_means2d[2 * i], v_means2d[2 * i + 1]), v_depths[i], vcn,
-                           has_comp ? v_compensations[i] : 0.f,
-                           v3(v_pix_vels[3 * i], v_pix_vels[3 * i + 1], v_pix_vels[3 * i + 2]),
-                           v2(v_depth_comps[2 * i], v_depth_comps[2 * i + 1]), v_mean, v_covar,
-                           v_R, v_t, v_vel_w);
+#pragma unroll 1
+    for (uint32_t k0 = 0; k0 < count; k0 += kThreads) {   // every thread: the viewmat reduction is the block's
+        const bool live = k0 + threadIdx.x < count;
+        if (v_viewmats == nullptr && !live) break;
+        const size_t g = first + queue.local[live ? k0 + threadIdx.x : k0];
+        const GaussIn in = gather_gaussian(means, covars, quats, scales, velocities, g);
+        V3 v_mean = v3(0.f, 0.f, 0.f), v_vel_w = v3(0.f, 0.f, 0.f);
+        M3 v_covar = m3_zero();
+        for (uint32_t c = 0; c < C; ++c) {
+            const SensorLidar s = load_lidar(viewmats, lin_vel, ang_vel, rs_time, c);
+            const size_t i = (size_t)c * N + g;
+            M3 v_R = m3_zero();
+            V3 v_t = v3(0.f, 0.f, 0.f);
+            if (live && radii[2 * i] > 0.f &&
+                pair_nonzero(v_means2d + 2 * i, v_depths[i], v_conics + 3 * i, v_compensations ? v_compensations + i : nullptr,
+                             v_pix_vels + 3 * i, 3, v_depth_comps + 2 * i)) {
+                const float cn[3] = {conics[3 * i], conics[3 * i + 1], conics[3 * i + 2]};
+                const float vcn[3] = {v_conics[3 * i], v_conics[3 * i + 1], v_conics[3 * i + 2]};
+                const bool has_comp = v_compensations != nullptr;
+                lidar_pair_bwd(s, in, velocities != nullptr, eps2d, cn,
+                               has_comp ? compensations[i] : 0.f, has_comp,
+                               v2(v_means2d[2 * i], v_means2d[2 * i + 1]), v_depths[i], vcn,
+                               has_comp ? v_compensations[i] : 0.f,
+                               v3(v_pix_vels[3 * i], v_pix_vels[3 * i + 1], v_pix_vels[3 * i + 2]),
+                               v2(v_depth_comps[2 * i], v_depth_comps[2 * i + 1]), v_mean, v_covar,
+                               v_R, v_t, v_vel_w);
+            }
+            if (v_viewmats != nullptr) block_reduce_viewmat(v_R, v_t, v_viewmats + 16 * c, red);
         }
-        if (v_viewmats != nullptr) block_reduce_viewmat(v_R, v_t, v_viewmats + 16 * c, red);
+        if (live)
+            store_param_grads(in, covars != nullptr, g, v_mean, v_covar, v_vel_w, v_means, v_covars, v_quats, v_scales,
+                              v_velocities);
     }
-    store_param_grads(in, covars != nullptr, touched, v_mean, v_covar, v_vel_w, g0, n, smem, v_means,
-                      v_covars, v_quats, v_scales, v_velocities);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1250,17 +1297,7 @@ projection_packed_bwd_kernel(uint32_t C, uint32_t N, uint32_t nnz, const float *
         return;
     const uint32_t c = (uint32_t)camera_ids[idx];
     const uint32_t g = (uint32_t)gaussian_ids[idx];
-    GaussIn in;
-    in.mean = ld3(means + 3 * (size_t)g);
-    in.vel = velocities != nullptr ? ld3(velocities + 3 * (size_t)g) : v3(0.f, 0.f, 0.f);
-    if (covars != nullptr) {
-        in.covar = covar_from_triu(covars + 6 * (size_t)g);
-    } else {
-        const float4 q = __ldg(reinterpret_cast<const float4 *>(quats) + g);
-        in.quat.x = q.x; in.quat.y = q.y; in.quat.z = q.z; in.quat.w = q.w;
-        in.scale = ld3(scales + 3 * (size_t)g);
-        in.covar = quat_scale_to_covar(in.quat, in.scale);
-    }
+    const GaussIn in = gather_gaussian(means, covars, quats, scales, velocities, g);
     SensorCam s = load_cam(viewmats, Ks, lin_vel, ang_vel, rs_time, c);
     const size_t i = idx;
     const float cn[3] = {conics[3 * i], conics[3 * i + 1], conics[3 * i + 2]};
@@ -1399,8 +1436,9 @@ extern "C" int splatad_lidar_projection_bwd(
     if (C == 0 || N == 0) return SPLATAD_OK;
     {
         SPL_PROF("lidar_projection_bwd_kernel", (cudaStream_t)stream);
-        launch_chained(lidar_projection_bwd_kernel, div_up(N, kThreads), kThreads, 0, (cudaStream_t)stream,
-            C, N, means, covars, quats, scales, velocities, viewmats, linear_velocity,
+        const uint32_t span = bwd_span(N);
+        launch_chained(lidar_projection_bwd_kernel, div_up(N, span), kThreads, 0, (cudaStream_t)stream,
+            C, N, span, means, covars, quats, scales, velocities, viewmats, linear_velocity,
             angular_velocity, rolling_shutter_time, eps2d, radii, conics, compensations, v_means2d,
             v_depths, v_conics, v_compensations, v_pix_vels, v_depth_compensations, v_means, v_covars,
             v_quats, v_scales, v_viewmats, v_velocities);
@@ -1453,8 +1491,9 @@ extern "C" int splatad_projection_bwd(
     if (C == 0 || N == 0) return SPLATAD_OK;
     {
         SPL_PROF("projection_bwd_kernel", (cudaStream_t)stream);
-        launch_chained(projection_bwd_kernel, div_up(N, kThreads), kThreads, 0, (cudaStream_t)stream,
-            C, N, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
+        const uint32_t span = bwd_span(N);
+        launch_chained(projection_bwd_kernel, div_up(N, span), kThreads, 0, (cudaStream_t)stream,
+            C, N, span, means, covars, quats, scales, velocities, viewmats, Ks, image_width, image_height,
             linear_velocity, angular_velocity, rolling_shutter_time, eps2d, radii, conics,
             compensations, v_means2d, v_depths, v_conics, v_compensations, v_pix_vels, v_means,
             v_covars, v_quats, v_scales, v_viewmats, v_velocities);

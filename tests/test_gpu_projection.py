@@ -367,6 +367,58 @@ def test_camera_projection_bwd(packed, sparse):
         _grad_check(f"camera bwd packed={packed} sparse={sparse} d/d{k}", a, b)
 
 
+@pytest.mark.parametrize("kind", ["camera", "lidar"])
+@pytest.mark.parametrize("N,share", [(257, 0.02), (151_553, 0.0), (160_001, 0.003), (160_001, 1.0), (700_001, 0.2)])
+def test_projection_bwd_of_the_gaussians_with_a_cotangent(kind, N, share):
+    """The dense backward queues the Gaussians that have a cotangent, block by block: the gradients are
+    those of the same Gaussians alone (a block of them per 256), and zero elsewhere."""
+    from splatad_b200 import ops
+
+    means, quats, scales, vel, g = _scene(N, 51, "cam" if kind == "camera" else "lidar")
+    if kind == "camera":
+        vm, Ks, lin, ang, rs = _camera_sensors(g)
+    else:
+        vm, lin, ang, rs = _lidar_sensors(2, g)
+    chosen = torch.rand(N, generator=g) < share
+    if share > 0:
+        chosen[-1] = True
+
+    def gradients(rows, cotangents=None):
+        L = [x.to(DEV).requires_grad_(True) for x in (means[rows], quats[rows], scales[rows], vel[rows], vm)]
+        with ops.velocity_grads(True):
+            if kind == "camera":
+                out = ops.fully_fused_projection(L[0], None, L[1], L[2], L[3], L[4], t(Ks), 320, 240, t(lin), t(ang),
+                                                 t(rs), calc_compensations=True, **CAM_KW)
+            else:
+                out = ops.fully_fused_lidar_projection(L[0], None, L[1], L[2], L[3], L[4], t(lin), t(ang), t(rs),
+                                                       calc_compensations=True, **LIDAR_KW)
+        outs = out[1:]
+        if cotangents is None:
+            # one kind of output at a time carries it: every array has to be looked at
+            which = torch.randint(len(outs), (N,), generator=g)
+            cotangents = []
+            for k, o in enumerate(outs):
+                m = (chosen & (which == k)).to(DEV)
+                cotangents.append(torch.randn(o.shape, device=DEV) * (m[None, :, None] if o.dim() == 3 else m[None]))
+        return cotangents, torch.autograd.grad(outs, L, cotangents)
+
+    cotangents, full = gradients(torch.arange(N))
+    rows = torch.nonzero(chosen).squeeze(1)
+    for a in full[:4]:
+        assert torch.all(a[~chosen.to(DEV)] == 0)
+    if rows.numel() == 0:
+        assert torch.all(full[4] == 0)
+        return
+    for k0 in range(0, rows.numel(), 75_000):   # small enough for a span of one block
+        part = rows[k0:k0 + 75_000]
+        _, alone = gradients(part, [c[:, part.to(DEV)].contiguous() for c in cotangents])
+        for a, b in zip(full[:4], alone[:4]):
+            assert torch.equal(a[part.to(DEV)], b)
+    if rows.numel() <= 75_000:
+        # sums over the Gaussians in another order: rounding of a sum of up to 75 000 float32 terms
+        _grad_check(f"{kind} bwd d/dvm", full[4][:, :3], alone[4][:, :3])
+
+
 def test_velocity_gradient_default_is_none():
     """The reference's fused projections return no gradient for ``velocities``; so does the default here."""
     from splatad_b200 import ops
