@@ -486,7 +486,7 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
     constexpr uint32_t kStage = points_fwd_stage(CDIM);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ PointBox s_box[8];
-    __shared__ uint32_t s_warp_kept[kStage * 8];
+    __shared__ uint32_t s_warp_kept[kStage * 16];
     const uint32_t bs = blockDim.x, cap = kStage * bs;
     float4 *sA = reinterpret_cast<float4 *>(smem_raw);
     float4 *sB = sA + cap;
@@ -656,12 +656,17 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
 // Lidar forward for few patches: all warps of a CTA work on ONE patch, a share of the entries each. What
 // depends on the order - the transmittance, where a point stops, its median - stays one chain per point,
 // with the same operations as above, but it is all that is left in the chain:
-//   1. every warp evaluates its share of the entries, alphas and range terms to shared memory;
-//   2. one warp runs down the alphas: transmittance, weights (left in the alphas' place), median, sums;
-//   3. every warp adds the features of its share, and the partial sums are added at the end.
-// A 32 x 512 scan has 512 patches of up to 300 relevant entries: 124 -> 65 us.
+//   1. every warp evaluates its share of the entries and leaves the alphas in shared memory;
+//   2. one warp multiplies its way down them and leaves the transmittance in front of each entry;
+//   3. every warp goes over its share again: weights, where a point stops, median, sums, features. The
+//      warps' partial results are put together at the end.
+// The chain runs on behind a point's stop: the transmittance never rises, so an entry is blended exactly
+// if what it would leave is above the threshold. What bounds this is the chain of batches, barriers and
+// multiplications of the patch with the longest list, not the machine (15 % of its issue slots).
+// A 32 x 512 scan has 512 patches of up to 1900 entries: 124 us apart, 66 with all of step 3 but the features
+// in step 2's warp, 46 like this (47 with four blocks per SM, 50 with 64 entries between barriers).
 // ---------------------------------------------------------------------------------------
-constexpr uint32_t kCoopWarps = 8, kCoopChunk = 32;
+constexpr uint32_t kCoopWarps = 8, kCoopChunk = 32, kCoopShare = kCoopChunk / kCoopWarps;
 
 template <int CDIM>
 __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_to_points_fwd_coop_kernel(
@@ -687,9 +692,8 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     float4 *sB = sA + kThreadsC;
     float4 *sC = sB + kThreadsC;
     float *sFeat = reinterpret_cast<float *>(sC + kThreadsC);               // [kThreadsC * CDIM]
-    float *sAlpha = sFeat + kThreadsC * CDIM;                               // [2][kCoopChunk][32] alphas, then weights
-    float *sTerm = sAlpha + 2 * kCoopChunk * 32;                            // [2][kCoopChunk][32] range terms
-    int32_t *sPos = reinterpret_cast<int32_t *>(sTerm + 2 * kCoopChunk * 32);
+    float *sAlpha = sFeat + kThreadsC * CDIM;   // [2][kCoopChunk][32] alphas, then transmittances
+    int32_t *sPos = reinterpret_cast<int32_t *>(sAlpha + 2 * kCoopChunk * 32);
 
     const uint32_t tiles_per_cam = grid_w * grid_h;
     const uint32_t gtile = blockIdx.x / patches_per_tile, part = blockIdx.x - gtile * patches_per_tile;
@@ -717,8 +721,8 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     const uint32_t num_batches = (uint32_t)(range.end - range.start + kThreadsC - 1) / kThreadsC;
     const uint32_t fstride = ranges ? channels - 1 : channels;
     const bool vec = (fstride % 4u == 0u) && ((reinterpret_cast<uintptr_t>(colors) & 15u) == 0u);
-    // the chain, held by the first warp
-    bool done = !inside;
+    float T_run = inside ? 1.f : 0.f;   // the chain, held by the first warp
+    // of this warp's share
     float T = 1.f, depth_extra = 0.f, alpha_sum = 0.f, median = 0.f;
     int32_t cur_idx = 0;
     const float alpha_sum_limit = pz - alpha_sum_threshold;
@@ -759,40 +763,47 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
         __syncthreads();
         for (uint32_t c0 = 0; c0 < n_kept && !finished; c0 += kCoopChunk) {
             const uint32_t n = min(kCoopChunk, n_kept - c0);
-            float *al = sAlpha + buffer * kCoopChunk * 32, *dt = sTerm + buffer * kCoopChunk * 32;
+            float *al = sAlpha + buffer * kCoopChunk * 32 + lane;
             buffer ^= 1u;
-            for (uint32_t q = warp; q < n; q += kCoopWarps) {
-                const uint32_t t = c0 + q;
+            float alpha[kCoopShare], dterm[kCoopShare];
+#pragma unroll
+            for (uint32_t r = 0; r < kCoopShare; ++r) {
+                const uint32_t q = warp + r * kCoopWarps, t = c0 + min(q, n - 1u);
                 const float4 A = sA[t], B = sB[t], Cc = sC[t];
                 const PointFootprint f = point_footprint(A, B, roll, px, py);
-                const float alpha = fminf(kAlphaMax, B.w * f.vis);
-                al[q * 32 + lane] = f.sigma < 0.f || alpha < kAlphaMin ? 0.f : alpha;
-                dt[q * 32 + lane] = Cc.y * f.dx + Cc.z * f.dy + Cc.x * roll;
+                const float a = fminf(kAlphaMax, B.w * f.vis);
+                alpha[r] = q >= n || f.sigma < 0.f || a < kAlphaMin ? 0.f : a;
+                dterm[r] = Cc.y * f.dx + Cc.z * f.dy + Cc.x * roll;
+                al[q * 32] = alpha[r];
             }
             __syncthreads();
             if (warp == 0) {
-#pragma unroll 4
-                for (uint32_t q = 0; q < n; ++q) {
-                    const float alpha = al[q * 32 + lane], dterm = dt[q * 32 + lane], range_q = sC[c0 + q].w;
-                    const float next_T = T * (1.f - alpha), vis = alpha * T;
-                    if (alpha > 0.f && next_T <= kTStop) done = true;
-                    const bool take = alpha > 0.f && !done;
-                    if (take) {
-                        depth_extra += dterm * vis;
-                        if (T > 0.5f && next_T <= 0.5f) median = range_q + dterm;
-                        if (compute_alpha_sum && range_q < alpha_sum_limit) alpha_sum += alpha;
-                        cur_idx = sPos[c0 + q];
-                        T = next_T;
-                    }
-                    al[q * 32 + lane] = take ? vis : 0.f;
+#pragma unroll
+                for (uint32_t q = 0; q < kCoopChunk; ++q) {
+                    const float a = al[q * 32];
+                    al[q * 32] = T_run;
+                    T_run *= 1.f - a;
                 }
-                if (__all_sync(0xffffffffu, done) && lane == 0) s_done = 1;
+                if (__all_sync(0xffffffffu, T_run <= kTStop) && lane == 0) s_done = 1;
             }
             __syncthreads();
             finished = s_done != 0;
-            for (uint32_t q = warp; q < n; q += kCoopWarps) {
-                const float vis = al[q * 32 + lane];
-                if (__any_sync(0xffffffffu, vis != 0.f)) axpy_staged_full<CDIM>(pix_out, sFeat + (c0 + q) * CDIM, vis);
+#pragma unroll
+            for (uint32_t r = 0; r < kCoopShare; ++r) {
+                const uint32_t q = warp + r * kCoopWarps;
+                const float before = al[q * 32], next_T = before * (1.f - alpha[r]);
+                const bool take = alpha[r] > 0.f && next_T > kTStop;
+                const float vis = take ? alpha[r] * before : 0.f;
+                if (!__any_sync(0xffffffffu, take)) continue;
+                const float range_q = sC[c0 + q].w;
+                if (take) {
+                    depth_extra += dterm[r] * vis;
+                    if (before > 0.5f && next_T <= 0.5f) median = range_q + dterm[r];
+                    if (compute_alpha_sum && range_q < alpha_sum_limit) alpha_sum += alpha[r];
+                    cur_idx = sPos[c0 + q];
+                    T = next_T;
+                }
+                axpy_staged_full<CDIM>(pix_out, sFeat + (c0 + q) * CDIM, vis);
             }
         }
     }
@@ -803,26 +814,40 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     for (int k = 0; k < CDIM; k += 4)
         *reinterpret_cast<float4 *>(parts + (warp * 32 + lane) * CDIM + k) =
             make_float4(pix_out[k], pix_out[k + 1], pix_out[k + 2], pix_out[k + 3]);
-    float *s_T = parts + kCoopWarps * 32 * CDIM, *s_extra = s_T + 32;
-    if (warp == 0) {
-        s_T[lane] = T;
-        s_extra[lane] = depth_extra;
-        if (in_image) {
-            // points that are not rendered (range <= 0) produce zeros everywhere
-            render_alphas[pix] = inside ? 1.f - T : 0.f;
-            last_ids[pix] = inside ? cur_idx : 0;
-            median_depths[pix] = inside ? median : 0.f;
-            if (alpha_sum_out != nullptr) alpha_sum_out[pix] = inside ? alpha_sum : 0.f;
-        }
-    }
+    float *s_T = parts + kCoopWarps * 32 * CDIM, *s_extra = s_T + kCoopWarps * 32, *s_sum = s_extra + kCoopWarps * 32,
+          *s_median = s_sum + kCoopWarps * 32;   // [warps][32] each
+    int32_t *s_last = reinterpret_cast<int32_t *>(s_median + kCoopWarps * 32);
+    s_T[tr] = T;
+    s_extra[tr] = depth_extra;
+    s_sum[tr] = alpha_sum;
+    s_median[tr] = median;
+    s_last[tr] = cur_idx;
     __syncthreads();
+    // the last transmittance and the last entry are the smallest and the largest of the warps'; the median
+    // was met by one warp alone
+    T = s_T[lane]; depth_extra = s_extra[lane]; alpha_sum = s_sum[lane]; median = s_median[lane]; cur_idx = s_last[lane];
+#pragma unroll
+    for (uint32_t w = 1; w < kCoopWarps; ++w) {
+        T = fminf(T, s_T[w * 32 + lane]);
+        depth_extra += s_extra[w * 32 + lane];
+        alpha_sum += s_sum[w * 32 + lane];
+        median += s_median[w * 32 + lane];
+        cur_idx = max(cur_idx, s_last[w * 32 + lane]);
+    }
+    if (warp == 0 && in_image) {
+        // points that are not rendered (range <= 0) produce zeros everywhere
+        render_alphas[pix] = inside ? 1.f - T : 0.f;
+        last_ids[pix] = inside ? cur_idx : 0;
+        median_depths[pix] = inside ? median : 0.f;
+        if (alpha_sum_out != nullptr) alpha_sum_out[pix] = inside ? alpha_sum : 0.f;
+    }
     const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
     for (uint32_t k = warp; k < channels; k += kCoopWarps) {
         float v = 0.f;
 #pragma unroll
         for (uint32_t w = 0; w < kCoopWarps; ++w) v += parts[(w * 32 + lane) * CDIM + k];
-        if (k == depth_idx) v += s_extra[lane];
-        if (bg) v += s_T[lane] * bg[k];
+        if (k == depth_idx) v += depth_extra;
+        if (bg) v += T * bg[k];
         if (in_image) render_colors[pix * channels + k] = inside ? v : 0.f;
     }
 }
@@ -1222,7 +1247,7 @@ __device__ __forceinline__ GradSlot point_grad_slot(int slot, int cdim, uint32_t
 constexpr uint32_t kPointsBwdStage = 2;   // entries per thread and batch: their loads overlap
 
 template <int CDIM, bool kAbs>
-__global__ void __launch_bounds__(256, CDIM <= 20 ? 2 : 1) rasterize_to_points_bwd_kernel(
+__global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 ? 1 : 2) rasterize_to_points_bwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors,
     const float *__restrict__ ranges, uint32_t channels,
@@ -1242,7 +1267,7 @@ __global__ void __launch_bounds__(256, CDIM <= 20 ? 2 : 1) rasterize_to_points_b
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ PointBox s_box;
     constexpr uint32_t kStage = kPointsBwdStage;
-    __shared__ uint32_t s_warp_kept[kStage * 8];
+    __shared__ uint32_t s_warp_kept[kStage * 16];
     const uint32_t bs = blockDim.x, cap = kStage * bs;
     float4 *sA = reinterpret_cast<float4 *>(smem_raw);
     float4 *sB = sA + cap;
@@ -1531,8 +1556,10 @@ constexpr uint64_t kCoopPatches = kNumSMs * 8;
 
 // Warps - segments of the list - per patch in the backward pass: every segment is run twice, which pays
 // while the patches alone leave the schedulers waiting on one warp's chain (256 patches: 405 us with one
-// segment, 178 with four, 109 with eight; 1088: 124, 100 and 104; 3648: 172, and 231 with four).
-static uint32_t point_segments(uint64_t patches) {
+// segment, 178 with four, 96 with eight, 78 with sixteen; 1088: 124, 100 and 104; 3648: 172, and 231 with
+// four). Sixteen take an SM each, and only up to eight channels stay within their 128 registers.
+static uint32_t point_segments(uint64_t patches, uint32_t channels) {
+    if (channels <= 8 && patches < (uint64_t)kNumSMs * 2) return 16u;
     return patches < (uint64_t)kNumSMs * 4 ? 8u : patches < (uint64_t)kNumSMs * 16 ? 4u : 1u;
 }
 
@@ -1713,7 +1740,7 @@ extern "C" int splatad_rasterize_to_points_fwd(
         auto kernel = coop ? rasterize_to_points_fwd_coop_kernel<D> : rasterize_to_points_fwd_kernel<D>; \
         const size_t smem = (size_t)(coop ? 1 : points_fwd_stage(D)) * bs *                       \
                                 (3 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float)) +  \
-                            (coop ? 4 * kCoopChunk * 32 * sizeof(float) : 0);                     \
+                            (coop ? 2 * kCoopChunk * 32 * sizeof(float) : 0);                     \
         int rc = set_smem(kernel, smem, "rasterize_to_points_fwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
         launch_chained(kernel, blocks * parts, bs, smem, (cudaStream_t)stream,                    \
@@ -1769,7 +1796,7 @@ extern "C" int splatad_rasterize_to_points_bwd(
                 "rasterize_to_points_bwd: a tile of %u points (%u threads at one per point) with %u channels is more "
                 "than the backward pass takes: use a smaller tile or at most 16 channels per call",
                 tile_width * tile_height, samples, channels);
-    const uint32_t parts = div_up(tile_width * tile_height, 64), bs = 32 * point_segments((uint64_t)blocks * parts);
+    const uint32_t parts = div_up(tile_width * tile_height, 64), bs = 32 * point_segments((uint64_t)blocks * parts, channels);
     SPL_REQUIRE((uint64_t)blocks * parts <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_points_bwd: too many tiles");
 #define CALL_ABS(D, A)                                                                            \
     {                                                                                             \
