@@ -395,6 +395,13 @@ int splatad_map_points_to_lidar_tiles(
     const float *elev_boundaries, uint32_t n_boundaries, float tile_azim_resolution, float min_azim,
     int32_t sort, void *workspace, size_t workspace_bytes, int64_t *tile_ids, int32_t *flatten_ids,
     void *stream);
+/* No counterpart in the reference: the same for points that lie point_stride >= 2 floats apart, as in the
+ * rows of a point cloud, without a packed copy of their first two columns. */
+int splatad_map_strided_points_to_lidar_tiles(
+    uint32_t C, uint32_t N, uint64_t total_elems, const float *points2d, uint32_t point_stride,
+    const int64_t *camera_ids, const float *elev_boundaries, uint32_t n_boundaries,
+    float tile_azim_resolution, float min_azim, int32_t sort, void *workspace, size_t workspace_bytes,
+    int64_t *tile_ids, int32_t *flatten_ids, void *stream);
 int splatad_points_mapping_offset_encode(const int64_t *point_ids, int64_t n_points, uint32_t C,
                                          uint32_t tile_width, uint32_t tile_height, int32_t *offsets,
                                          void *stream);

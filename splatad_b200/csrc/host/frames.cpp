@@ -44,7 +44,7 @@ using OptTensor = c10::optional<Tensor>;
     X(splatad_isect_lidar_tiles_fill) X(splatad_isect_set_early_count) X(splatad_isect_set_depth_range_hint)             \
     X(splatad_rasterize_expected_to_pixels_fwd) X(splatad_rasterize_expected_to_pixels_bwd)                              \
     X(splatad_lidar_frame_fwd) X(splatad_rasterize_to_points_fwd) X(splatad_rasterize_to_points_bwd) X(splatad_map_points_workspace_bytes)          \
-    X(splatad_map_points_to_lidar_tiles) X(splatad_points_mapping_offset_encode) X(splatad_populate_image_from_points)
+    X(splatad_map_strided_points_to_lidar_tiles) X(splatad_points_mapping_offset_encode) X(splatad_populate_image_from_points)
 
 struct Lib {
 #define SPL_MEMBER(name) decltype(&::name) name = nullptr;
@@ -829,23 +829,28 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
 // Lidar points -> tiles -> raster image. None: arguments for the Python bindings to check or convert.
 // ---------------------------------------------------------------------------------------------
 py::object map_points(const Tensor &points2d, const Tensor &boundaries, double tile_az, double min_az, bool sort) {
-    if (!points2d.defined() || !points2d.is_cuda() || points2d.dim() != 3 || points2d.size(2) != 2 || points2d.numel() == 0)
+    if (!points2d.defined() || !points2d.is_cuda() || points2d.layout() != at::kStrided || points2d.dim() != 3 ||
+        points2d.size(2) != 2 || points2d.numel() == 0 || points2d.is_conj() || points2d.is_neg())
         return py::none();
     const c10::DeviceIndex dev = points2d.get_device();
     const c10::cuda::CUDAGuard guard(dev);
     const at::NoGradGuard no_grad;
-    const Tensor pts = points2d.scalar_type() == at::kFloat ? points2d.contiguous() : Tensor();
-    if (!plain(pts, dev) || !plain(boundaries, dev) || boundaries.dim() != 1) return py::none();
+    if (points2d.scalar_type() != at::kFloat || !plain(boundaries, dev) || boundaries.dim() != 1) return py::none();
+    const int64_t C = points2d.size(0), N = points2d.size(1), total = C * N;
+    // the first two columns of a point cloud are read where they are
+    int64_t stride = points2d.stride(1);
+    const bool rows = points2d.stride(2) == 1 && stride >= 2 && stride < 0x7fffffff && (C == 1 || points2d.stride(0) == N * stride);
+    const Tensor pts = rows ? points2d : points2d.contiguous();
+    if (!rows) stride = 2;
     const auto stream = c10::cuda::getCurrentCUDAStream();
-    const int64_t C = pts.size(0), N = pts.size(1), total = C * N;
-    const auto options = pts.options();
+    const auto options = points2d.options().requires_grad(false);
     const Tensor ids = at::empty({total}, options.dtype(at::kLong)), flat = at::empty({total}, options.dtype(at::kInt));
     Tensor ws;
     if (sort) ws = workspace("map_points", lib.splatad_map_points_workspace_bytes((uint64_t)total), stream);
-    check(lib.splatad_map_points_to_lidar_tiles((uint32_t)C, (uint32_t)N, (uint64_t)total, F(pts), nullptr, F(boundaries),
-                                                (uint32_t)boundaries.numel(), (float)tile_az, (float)min_az, sort,
-                                                sort ? ws.data_ptr() : nullptr, sort ? (size_t)ws.numel() : 0, L(ids), I(flat),
-                                                stream.stream()));
+    check(lib.splatad_map_strided_points_to_lidar_tiles((uint32_t)C, (uint32_t)N, (uint64_t)total, F(pts), (uint32_t)stride, nullptr,
+                                                        F(boundaries), (uint32_t)boundaries.numel(), (float)tile_az, (float)min_az,
+                                                        sort, sort ? ws.data_ptr() : nullptr, sort ? (size_t)ws.numel() : 0, L(ids),
+                                                        I(flat), stream.stream()));
     return py::make_tuple(ids, flat);
 }
 

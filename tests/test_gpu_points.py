@@ -40,6 +40,25 @@ def test_map_points_and_offsets_vs_oracle(C, N, sort):
         assert np.array_equal(n(offs), isect.points_mapping_offset_encode(want_ids, C, n_az, 16))
 
 
+@pytest.mark.parametrize("C,N,n_az,n_el", [
+    (1, 2047, 1, 1), (1, 2049, 2, 1), (2, 4097, 32, 32), (1, 30_000, 89, 23), (1, 30_000, 2049, 1), (1, 1_300_000, 64, 16),
+])
+def test_map_points_in_one_pass_over_the_tiles(C, N, n_az, n_el):
+    """Up to 2048 tiles are sorted in one pass, in blocks of 2048 points: one tile, 2047, 2048 and 2049 of
+    them, remainders of a block, several blocks' worth per block, crowded tiles; read in place from the
+    rows of a point cloud. Bit for bit the oracle's."""
+    from oracle import isect
+    from splatad_b200 import ops
+    pts = _points(C, N, 20 + n_az)
+    pts[:, ::3, :2] = pts[:, :1, :2]                    # a third of the points in one tile
+    eb, res = torch.linspace(-45.0, 45.0, n_el + 1), 360.0 / n_az
+    want_ids, want_flat = isect.map_points_to_lidar_tiles(n(pts[..., :2]), n(eb), res, -180.0)
+    cloud = t(pts)
+    for points2d in (cloud[..., :2], cloud[..., :2].contiguous(), cloud.transpose(0, 1).contiguous().transpose(0, 1)[..., :2]):
+        ids, flat = ops.map_points_to_lidar_tiles(points2d, t(eb), res, -180.0)
+        assert np.array_equal(n(ids), want_ids) and np.array_equal(n(flat), want_flat)
+
+
 def test_map_points_packed_and_empty():
     from oracle import isect
     from splatad_b200 import ops
