@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <utility>
+
 #include "../../include/splatad_b200.h"
 
 namespace splatad {
@@ -64,8 +66,8 @@ __device__ __forceinline__ void chain_enter() {
 }
 
 template <typename... KP, typename... A>
-inline void launch_chained(void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                           A &&...args) {
+inline void launch_chained_if(bool chained, void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              A &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -75,8 +77,14 @@ inline void launch_chained(void (*kernel)(KP...), dim3 grid, dim3 block, size_t 
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chained ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KP>(args)...);   // errors surface in check_launch()
+}
+
+template <typename... KP, typename... A>
+inline void launch_chained(void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                           A &&...args) {
+    launch_chained_if(true, kernel, grid, block, smem, st, std::forward<A>(args)...);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1549,6 +1549,13 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         else { CALL(32); }                                                                       \
     } while (0)
 
+// The forward kernels of more blocks than the machine holds at once start on empty SMs. Chained, their first
+// blocks are placed beside the last of the colour or list kernels before them, on SMs that keep that kernel's
+// large shared memory and small first-level cache for as long as one block follows another, and the gathers of a
+// long kernel need the cache: 1920 x 1080 with spherical harmonics 437 us a frame chained, 411 apart; six cameras
+// 3490 and 3370; 128 x 1800 lidar 294 and 289. Below, the launch gap weighs more (640 x 360: 101 and 103).
+static bool fits_at_once(uint64_t blocks) { return blocks <= (uint64_t)kNumSMs * 8; }
+
 // Patches below which all warps of a CTA share one in the forward pass: the shared work costs more
 // instructions in all, so the patches must be too few to fill the machine (2176 patches: 53 us apart, 102
 // shared; 512: 124 and 65).
@@ -1617,7 +1624,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
         const size_t smem = (size_t)bs * (2 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float)); \
         int rc = set_smem(rasterize_to_pixels_fwd_kernel<D>, smem, "rasterize_to_pixels_fwd");    \
         if (rc != SPLATAD_OK) return rc;                                                          \
-        launch_chained(rasterize_to_pixels_fwd_kernel<D>, blocks, bs, smem, (cudaStream_t)stream, \
+        launch_chained_if(fits_at_once(blocks), rasterize_to_pixels_fwd_kernel<D>, blocks, bs, smem,  \
+            (cudaStream_t)stream,                                                                 \
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
             image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
@@ -1743,7 +1751,8 @@ extern "C" int splatad_rasterize_to_points_fwd(
                             (coop ? 2 * kCoopChunk * 32 * sizeof(float) : 0);                     \
         int rc = set_smem(kernel, smem, "rasterize_to_points_fwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
-        launch_chained(kernel, blocks * parts, bs, smem, (cudaStream_t)stream,                    \
+        launch_chained_if(fits_at_once((uint64_t)blocks * parts), kernel, blocks * parts, bs, smem, \
+            (cudaStream_t)stream,                                                                 \
             C, n_isects, (const float2 *)means2d, conics, lidar_features, gaussian_ranges,        \
             channels, opacities,                                                                  \
             pix_vels, (const float2 *)depth_compensations, backgrounds,                           \

@@ -2017,8 +2017,7 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             const uint32_t grid = min(units_max, (longer ? 3u : 6u) * kNumSMs);
             // long lists: not placed while the scan still holds its SMs (six cameras: 1340 us, and 80 more chained)
-            if (longer) kernel<<<grid, a.unit / kBlkWords, smem, st>>>(a, isect_ids, flatten_ids, p.counters);
-            else launch_chained(kernel, grid, a.unit / kBlkWords, smem, st, a, isect_ids, flatten_ids, p.counters);
+            launch_chained_if(!longer, kernel, grid, a.unit / kBlkWords, smem, st, a, isect_ids, flatten_ids, p.counters);
         }
     } else {
         FillWs f = carve_fill(fill_workspace, (uint64_t)capacity);
