@@ -253,12 +253,13 @@ def fp32_probe(dev, n_sms):
     return flops / (best * 1e-3) / 1e12
 
 
-def count_row_records(meta, cfg):
-    """Number of (Gaussian, elevation tile row) pairs of a lidar frame: the records step A of the
+def count_block_records(meta, cfg):
+    """Number of (Gaussian, block of 4 x 8 tiles) pairs of a lidar frame: the records step A of the
     tile ordering writes. Same row range as the library's rectangle (first boundary not below the
-    lower edge minus one, up to the first boundary not below the upper edge)."""
+    lower edge minus one, up to the first boundary not below the upper edge); the columns follow from
+    the tile count."""
     radii, means2d = meta["radii"], meta["means2d"]
-    vis = radii[..., 0] > 0
+    vis = meta["tiles_per_gauss"] > 0
     eb = torch.as_tensor(cfg["tile_elevation_boundaries"], dtype=torch.float32, device=radii.device).contiguous()
     ne = eb.numel() - 1
     el = means2d[..., 1][vis].contiguous()
@@ -267,7 +268,14 @@ def count_row_records(meta, cfg):
     i_hi = torch.maximum(i_lo, torch.searchsorted(eb, el + rad, right=False))
     y0 = torch.clamp(i_lo - 1, min=0)
     y1 = torch.clamp(i_hi, max=ne)
-    return int(torch.clamp(y1 - y0, min=0).sum())
+    rows = torch.clamp(y1 - y0, min=1)
+    width = meta["tiles_per_gauss"][vis].long() // rows
+    grid_w = meta["tile_grid_width"]
+    left = means2d[..., 0][vis] - radii[..., 0][vis] - cfg.get("min_azimuth", -180.0)
+    x0 = torch.floor(torch.remainder(left, 360.0) * (grid_w / 360.0)).long()
+    block_rows = (y1 - 1) // 8 - y0 // 8 + 1
+    block_cols = torch.clamp((x0 % 4 + width + 3) // 4, max=(grid_w + 3) // 4)
+    return int((torch.clamp(block_rows, min=0) * block_cols).sum())
 
 
 def count_pairs_lidar(meta, cfg):
@@ -515,8 +523,8 @@ def roofline_stages(prof, cam_prof, n_gauss, n_vis, n_isects, n_rec, pairs, cam_
                     "kernels": sum(prof[k][0] for k in prof if k.startswith(("depthsort", "radix_", "depth_bucket"))),
                     "algorithmic_bytes": int(b), "achieved": round(b / (t * 1e-3) / 1e9, 1), "peak": peak,
                     "unit": "GB/s", "frac": round(b / (t * 1e-3) / 1e9 / peak, 4)})
-    t = ms_of("isect_count", "depthsort", "radix_", "depth_bucket", "rowsplit", "colsplit", "init_counters", "emit",
-              "tilesort")
+    t = ms_of("isect_count", "depthsort", "radix_", "depth_bucket", "blk_", "tile_count", "tile_scan", "tile_scatter",
+              "init_counters", "emit", "tilesort")
     if t > 0:
         b = n_isects * 24
         out.append({"stage": "tile ordering (count .. lists)", "bound": "hbm", "ms": round(t, 4),
@@ -546,10 +554,7 @@ def roofline_stages(prof, cam_prof, n_gauss, n_vis, n_isects, n_rec, pairs, cam_
 # DRAM bytes (read + written) per launch on the headline frame, from the ncu captures summarised
 # under profiles/ (file named after the kernel); kernels without a committed capture give null.
 NCU_TRAFFIC = {
-    "colsplit_scatter_kernel": (229_227_008, "profiles/colsplit_and_rowsplit_scatter_config2.md"),
-    "rowsplit_scatter_kernel": (64_200_000, "profiles/colsplit_and_rowsplit_scatter_config2.md"),
     "lidar_projection_fwd_kernel": (45_829_376, "profiles/lidar_projection_fwd_config2.md"),
-    "rasterize_to_points_fwd_kernel": (5_130_000, "profiles/rasterize_to_points_fwd_config2.md"),
     "depth_bucket_scatter_kernel": (11_567_616, "profiles/depth_bucket_kernels_config2.md"),
     "depth_bucket_count_kernel": (9_038_592, "profiles/depth_bucket_kernels_config2.md"),
     "depth_bucket_rank_kernel": (9_005_056, "profiles/depth_bucket_kernels_config2.md"),
@@ -731,16 +736,16 @@ def run_ours(args):
         peak, peak_src = load_peaks()
         dom = max(prof.items(), key=lambda kv: kv[1][1])
         dom_name, (dom_cnt, dom_ms) = dom
-        # algorithmic bytes per launch. Tile ordering of config 2 is a row / column split: step A
-        # writes one 16-byte record per (Gaussian, tile row), step B reads the records once and
-        # writes 8 + 4 bytes per intersection.
+        # algorithmic bytes per launch. Tile ordering of config 2 is a block split: step A writes one
+        # 8-byte record per (Gaussian, block of 4 x 8 tiles), step B reads the records once and writes
+        # 8 + 4 bytes per intersection.
         n_vis = int((out[3]["radii"][..., 0] > 0).sum())
-        n_rec = count_row_records(out[3], cfg)
+        n_rec = count_block_records(out[3], cfg)
         bytes_per_launch = {
-            "colsplit_scatter_kernel": n_rec * 16 + n_isects * 12,
-            "colsplit_count_kernel": n_rec * 8,
-            "rowsplit_scatter_kernel": n_vis * 16 + n_rec * 16,
-            "rowsplit_count_kernel": n_vis * 12,
+            "tile_scatter_kernel": n_rec * 8 + n_isects * 12,
+            "tile_count_kernel": n_rec * 4,
+            "blk_scatter_kernel": n_vis * 8 + n_rec * 8,
+            "blk_count_kernel": n_vis * 8,
             "tilesort_downsweep": n_isects * (8 + 8 + 2),       # read pair, write pair (last pass 12 B)
             "tilesort_upsweep": n_isects * 4,
             "emit_kernel": n_isects * 8 + n_vis * 20,

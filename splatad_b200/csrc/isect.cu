@@ -2012,10 +2012,10 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
             constexpr uint32_t kMin = kBlkUnitMin / (32 * kBlkWords), kMax = kBlkUnitMax / (32 * kBlkWords);
             const bool longer = a.unit == kBlkUnitMax;
             auto kernel = longer ? tile_scatter_kernel<kMax> : tile_scatter_kernel<kMin>;
-            // records' pairs and 32 places of two bytes per record: 36 or 72 KB, six or three CTAs per SM
+            // records' pairs and 32 places of two bytes per record: 36 or 72 KB, five or three CTAs per SM
             const size_t smem = (size_t)a.unit * (sizeof(uint2) + 32 * sizeof(uint16_t));
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            const uint32_t grid = min(units_max, (longer ? 3u : 6u) * kNumSMs);
+            const uint32_t grid = min(units_max, (longer ? 3u : 5u) * kNumSMs);
             // long lists: not placed while the scan still holds its SMs (six cameras: 1340 us, and 80 more chained)
             launch_chained_if(!longer, kernel, grid, a.unit / kBlkWords, smem, st, a, isect_ids, flatten_ids, p.counters);
         }
