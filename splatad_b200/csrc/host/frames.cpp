@@ -272,7 +272,7 @@ void keep_state(AutogradContext *ctx, const c10::intrusive_ptr<T> &s) {
 // Lidar
 // ---------------------------------------------------------------------------------------------
 struct LidarFrame : torch::CustomClassHolder {
-    int64_t C = 0, N = 0, W = 0, H = 0, rows = 0, cols = 0, D = 0;
+    int64_t C = 0, N = 0, W = 0, H = 0, rows = 0, cols = 0, D = 0, n_isects = 0;
     uint32_t tile_w = 0, tile_h = 0;
     float eps2d = 0.f, threshold = 0.f;
     bool alpha_sum_wanted = false, absgrad = false;
@@ -342,6 +342,7 @@ struct LidarCompositeNode : torch::autograd::Function<LidarCompositeNode> {
                                 f->last_ids, f->offsets, f->flatten_ids});
         auto kept = c10::make_intrusive<LidarFrame>();
         kept->C = f->C; kept->W = f->W; kept->H = f->H; kept->rows = f->rows; kept->cols = f->cols; kept->D = f->D;
+        kept->n_isects = f->n_isects;
         kept->tile_w = f->tile_w; kept->tile_h = f->tile_h; kept->threshold = f->threshold;
         kept->alpha_sum_wanted = f->alpha_sum_wanted; kept->absgrad = f->absgrad;
         keep_state(ctx, kept);
@@ -374,7 +375,7 @@ struct LidarCompositeNode : torch::autograd::Function<LidarCompositeNode> {
         if (f->absgrad) zeros.add(v_abs, means2d.sizes());
         zeros.make(options);
         check(lib.splatad_rasterize_to_points_bwd(
-            (uint32_t)f->C, -1, F(means2d), F(conics), F(features), F(depths), (uint32_t)(f->D + 1), F(opacities), F(pix_vels),
+            (uint32_t)f->C, f->n_isects, F(means2d), F(conics), F(features), F(depths), (uint32_t)(f->D + 1), F(opacities), F(pix_vels),
             F(depth_comps), nullptr, F(saved[7]), (uint32_t)f->W, (uint32_t)f->H, f->tile_w, f->tile_h, (uint32_t)f->cols,
             (uint32_t)f->rows, f->alpha_sum_wanted, f->threshold, I(saved[10]), I(saved[11]), (uint32_t)f->D, F(alphas), I(saved[9]),
             F(v_render), F(v_alphas), F(v_sum), M(v_abs), M(v_means2d), M(v_conics), M(v_features), M(v_opacities), M(v_pix_vels),
@@ -488,6 +489,7 @@ py::object lidar_frame(const Tensor &means, const Tensor &quats, const Tensor &s
         counts = read_counts(slot, sequence, stream);
     }
     if (!usable(counts, capacity)) return py::make_tuple(counts.n_isects, counts.status, counts.depth_range, py::none());
+    f->n_isects = counts.n_isects;   // none: the lists are null pointers, which the backward pass must not ask for
     f->isect_ids = head(f->isect_ids, counts.n_isects);
     f->flatten_ids = head(f->flatten_ids, counts.n_isects);
     Tensor opacities_cn = f->opacities.defined() ? f->opacities : opacities.unsqueeze(0);
@@ -511,7 +513,7 @@ py::object lidar_frame(const Tensor &means, const Tensor &quats, const Tensor &s
 // Cameras
 // ---------------------------------------------------------------------------------------------
 struct CameraFrame : torch::CustomClassHolder {
-    int64_t C = 0, N = 0, n = 0, W = 0, H = 0, tile_size = 0, tile_w = 0, tile_h = 0, channels = 0;
+    int64_t C = 0, N = 0, n = 0, W = 0, H = 0, tile_size = 0, tile_w = 0, tile_h = 0, channels = 0, n_isects = 0;
     int64_t K = 0, D = 0, sh_degree = -1;     // spherical harmonics (K coefficients) or D plain channels
     bool packed = false, per_camera = false, depth = false, expected = false, absgrad = false;
     float eps2d = 0.f;
@@ -522,7 +524,7 @@ struct CameraFrame : torch::CustomClassHolder {
         auto k = c10::make_intrusive<CameraFrame>();
         k->C = C; k->N = N; k->n = n; k->W = W; k->H = H; k->tile_size = tile_size; k->tile_w = tile_w; k->tile_h = tile_h;
         k->channels = channels; k->K = K; k->D = D; k->sh_degree = sh_degree; k->packed = packed; k->per_camera = per_camera;
-        k->depth = depth; k->expected = expected; k->absgrad = absgrad; k->eps2d = eps2d;
+        k->depth = depth; k->expected = expected; k->absgrad = absgrad; k->eps2d = eps2d; k->n_isects = n_isects;
         return k;
     }
 };
@@ -646,7 +648,7 @@ struct CameraCompositeNode : torch::autograd::Function<CameraCompositeNode> {
         if (f->absgrad) zeros.add(v_abs, means2d.sizes());
         zeros.make(options);
         check(lib.splatad_rasterize_expected_to_pixels_bwd(
-            (uint32_t)f->C, -1, F(means2d), F(conics), F(colors), (uint32_t)f->channels, F(opacities), F(pix_vels), F(saved[5]),
+            (uint32_t)f->C, f->n_isects, F(means2d), F(conics), F(colors), (uint32_t)f->channels, F(opacities), F(pix_vels), F(saved[5]),
             F(saved[6]), (uint32_t)f->W, (uint32_t)f->H, (uint32_t)f->tile_size, (uint32_t)f->tile_w, (uint32_t)f->tile_h, I(saved[9]),
             I(saved[10]), F(saved[11]), F(saved[7]), I(saved[8]), F(v_render), F(v_alphas), M(v_abs), M(v_means2d), M(v_conics),
             M(v_colors), M(v_opacities), M(v_pix_vels), c10::cuda::getCurrentCUDAStream().stream()));
@@ -806,6 +808,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
         for (Tensor *t : {&f->camera_ids, &f->gaussian_ids, &f->radii, &f->means2d, &f->depths, &f->conics, &f->comps, &f->pix_vels,
                           &f->tiles_per_gauss, &f->opacities, &f->colors})
             *t = head(*t, nnz);
+    f->n_isects = counts.n_isects;   // none: the lists are null pointers, which the backward pass must not ask for
     f->isect_ids = head(f->isect_ids, counts.n_isects);
     f->flatten_ids = head(f->flatten_ids, counts.n_isects);
     Tensor opacities_r = f->opacities.defined() ? f->opacities : opacities.unsqueeze(0);

@@ -1,0 +1,44 @@
+"""Frames through the native host side (``csrc/host/frames.cpp``): from the second frame of a shape on, one call
+enqueues the frame and puts its own two nodes into the autograd graph. Whatever it takes, its images, lists,
+gradients and refusals are those of the individual ops."""
+
+import pytest
+import torch
+
+from gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+def _to_gpu(cfg):
+    return {k: (v.to(DEV) if isinstance(v, torch.Tensor) else v) for k, v in cfg.items()}
+
+
+def _forget():
+    """No frame has a predecessor: the next one is rendered by the individual ops."""
+    from splatad_b200 import ops
+    for hint in (ops._isect_count_hint, ops._packed_nnz_hint, ops._depth_range_hint, ops._depth_sort_mode):
+        hint.clear()
+
+
+@pytest.mark.parametrize("kind", ["lidar", "camera"])
+def test_a_frame_that_sees_nothing_has_zero_gradients(kind):
+    import splatad_b200
+    from splatad_b200 import scenes
+    if kind == "lidar":
+        g = _to_gpu(scenes.config2(N=20_011))
+        render, away = splatad_b200.lidar_rasterization, torch.tensor([0.0, 0.0, 1e4], device=DEV)
+    else:
+        g = _to_gpu(scenes.config1(N=20_011, packed=False))
+        render, away = splatad_b200.rasterization, torch.tensor([0.0, 0.0, -1e4], device=DEV)
+    names = ("means", "quats", "scales", "opacities", "lidar_features" if kind == "lidar" else "colors")
+    _forget()
+    render(**g)                                        # its counts size the next frame of the shape
+    leaves = {k: g[k].clone().requires_grad_(True) for k in names}
+    *images, meta = render(**{**g, **leaves, "means": leaves["means"] + away}, absgrad=True)
+    assert meta["flatten_ids"].numel() == 0 and float(images[1].detach().abs().max()) == 0.0
+    meta["means2d"].retain_grad()
+    sum(i.sum() for i in images).backward()
+    for k in names:
+        assert leaves[k].grad is not None and float(leaves[k].grad.abs().max()) == 0.0, k
+    assert float(meta["means2d"].grad.abs().max()) == 0.0 and float(meta["means2d"].absgrad.abs().max()) == 0.0
