@@ -419,7 +419,8 @@ int splatad_populate_image_from_points(
 /* rasterize_to_pixels_fwd_tensor - gsplat/cuda/csrc/rasterization.cu:1520-2019, kernel
  * 1360-1518. Inputs are [C,N,..] or packed [nnz,..] (flatten_ids index either);
  * backgrounds [C,channels] or NULL. Outputs: render_colors [C,H,W,channels],
- * render_alphas [C,H,W], last_ids [C,H,W] int32; every pixel is written. */
+ * render_alphas [C,H,W], last_ids [C,H,W] int32 (the sign bit is set where a pixel's colour is not finite: the
+ * backward pass then keeps what is not finite to the pixels that blend it); every pixel is written. */
 int splatad_rasterize_to_pixels_fwd(
     uint32_t C, int64_t n_isects, const float *means2d, const float *conics, const float *colors,
     uint32_t channels, const float *opacities, const float *pix_vels,

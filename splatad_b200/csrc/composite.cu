@@ -57,6 +57,7 @@ __device__ __forceinline__ void axpy_staged_full(float (&acc)[CDIM], const float
 // pairs of pixels (packed FP32: two results per issued instruction). A warp covers a compact patch of
 // the tile - 8 x 8 pixels of a 16 x 16 tile with PX = 2, 16 x 8 with PX = 4.
 // ---------------------------------------------------------------------------------------
+constexpr float kExpectedMin = 1e-10f;   // alphas below it do not divide (gsplat/rendering.py:423-430)
 constexpr float kLog2E = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 
 template <int PX>
@@ -157,12 +158,180 @@ __device__ __forceinline__ float2 pair_power(float a, float2 dx, float bdy, floa
 }
 
 // ---------------------------------------------------------------------------------------
+// Values that are not finite. The kernels below let every pixel of a warp take every entry that one of them
+// blends, with weight zero where it is not blended - and zero times an infinity is a NaN. A pixel that comes out
+// with one is worked out again by itself, and its last id marked: the backward kernel leaves the tiles that hold
+// a mark, or a cotangent that is not finite, to a pass in which a pixel takes nothing from an entry that it does
+// not blend. Both out of line and from nothing but the kernels' own arguments, so that the kernels hold
+// nothing for them. (Looking at the staged colours instead costs the forward kernel of the camera benchmark 220 ->
+// 237 us and the backward one 396 -> 440; two loop bodies, one of them careful, 6 to 9 % of a training step.)
+// ---------------------------------------------------------------------------------------
+constexpr int32_t kOddPixel = INT32_MIN;   // in a last id: the pixel blended something that is not finite
+
+__device__ __forceinline__ int32_t last_position(int32_t last_id) { return last_id & INT32_MAX; }
+
+struct PixelTask {
+    uint32_t C, W, H, tile_size, tile_w, tile_h, channels;
+    int64_t n_isects;
+    const float2 *means2d, *pix_vels;
+    const float *conics, *opacities, *colors, *rs_time, *backgrounds;
+    const int32_t *offsets, *flatten_ids;
+};
+
+// Where a pixel of the calling thread lies; `pix` is its place in the images.
+struct TaskPixel {
+    bool inside;
+    float x, y, roll;
+    size_t pix;
+    const float *bg;
+};
+
+template <int PX>
+__device__ __forceinline__ TaskPixel task_pixel(const PixelTask &a, uint32_t k) {
+    const uint32_t per_cam = a.tile_w * a.tile_h, cam = blockIdx.x / per_cam, tile = blockIdx.x - cam * per_cam;
+    const uint32_t ty = tile / a.tile_w, tx = tile - ty * a.tile_w;
+    const TilePixels<PX> tp = tile_pixels<PX>(a.tile_size, threadIdx.x);
+    const uint32_t i = ty * a.tile_size + tp.y, j = tx * a.tile_size + tp.x + k;
+    TaskPixel p;
+    p.inside = tp.y < a.tile_size && tp.x + k < a.tile_size && i < a.H && j < a.W;
+    p.x = (float)j + 0.5f;
+    p.y = (float)i + 0.5f;
+    p.roll = a.rs_time[cam] * ((p.y - 0.5f) / (float)(a.H - 1) - 0.5f);
+    p.pix = ((size_t)cam * a.H + i) * a.W + j;
+    p.bg = a.backgrounds ? a.backgrounds + (size_t)cam * a.channels : nullptr;
+    return p;
+}
+
+struct PixelAlpha {
+    float4 B;              // scaled conic, opacity
+    float dx, dy, vis, alpha;
+    bool blends;
+};
+
+__device__ __forceinline__ PixelAlpha pixel_alpha(const PixelTask &a, int32_t g, const TaskPixel &p) {
+    const PixelEntry e = load_pixel_entry(g, a.means2d, a.conics, a.opacities, a.pix_vels);
+    PixelAlpha r;
+    r.B = scaled_conic(e.B);
+    r.dx = e.A.x + p.roll * e.A.z - p.x;
+    r.dy = e.A.y + p.roll * e.A.w - p.y;
+    const float power = fmaf(fmaf(r.B.x, r.dx, r.B.y * r.dy), r.dx, r.B.z * r.dy * r.dy);
+    r.vis = exp2_approx(power);
+    r.alpha = r.B.w * r.vis;
+    r.blends = power <= 0.f && r.alpha >= kAlphaMin;
+    return r;
+}
+
+template <int PX>
+__device__ __noinline__ void odd_pixels_fwd(const PixelTask &a, float *colors_out, float *alphas, int32_t *last_ids, bool expected) {
+    const TileRange range = tile_range(a.offsets, blockIdx.x, a.C * a.tile_w * a.tile_h, a.n_isects);
+    for (uint32_t h = 0; h < (uint32_t)PX; ++h) {
+        const TaskPixel p = task_pixel<PX>(a, h);
+        if (!p.inside) continue;
+        float *color = colors_out + p.pix * a.channels, T = 1.f;
+        int32_t pos = 0;
+        for (uint32_t k = 0; k < a.channels; ++k) color[k] = 0.f;
+        for (int32_t idx = range.start; idx < range.end; ++idx) {
+            const int32_t g = a.flatten_ids[idx];
+            const PixelAlpha e = pixel_alpha(a, g, p);
+            if (!e.blends) continue;
+            const float alpha = fminf(kAlphaMax, e.alpha), next_T = T * (1.f - alpha), vis = alpha * T;
+            if (next_T <= kTStop) break;
+            for (uint32_t k = 0; k < a.channels; ++k) color[k] = fmaf(a.colors[(size_t)g * a.channels + k], vis, color[k]);
+            pos = idx;
+            T = next_T;
+        }
+        alphas[p.pix] = 1.f - T;
+        last_ids[p.pix] = pos | kOddPixel;
+        for (uint32_t k = 0; p.bg != nullptr && k < a.channels; ++k) color[k] += T * p.bg[k];
+        if (expected) color[a.channels - 1] /= fmaxf(1.f - T, kExpectedMin);
+    }
+}
+
+struct PixelGrads {
+    const float *alphas, *v_colors_in, *v_alphas, *expected;
+    const int32_t *last_ids;
+    float *means2d, *means2d_abs, *conics, *colors, *opacities, *pix_vels;
+};
+
+__device__ __forceinline__ void add_warp_total(float *to, float v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if ((threadIdx.x & 31u) == 0u && v != 0.f) atomicAdd(to, v);
+}
+
+// By whole warps.
+template <int PX>
+__device__ __noinline__ void odd_pixels_bwd(const PixelTask &a, const PixelGrads &grad) {
+    const TileRange range = tile_range(a.offsets, blockIdx.x, a.C * a.tile_w * a.tile_h, a.n_isects);
+    const uint32_t n = a.channels;
+    for (uint32_t h = 0; h < (uint32_t)PX; ++h) {
+        const TaskPixel p = task_pixel<PX>(a, h);
+        const int32_t last = p.inside ? min(range.end - 1, last_position(grad.last_ids[p.pix])) : -1;
+        const float *v_out = grad.v_colors_in + p.pix * n;
+        float T = 1.f, behind = 0.f, divisor = 1.f;
+        if (last >= 0) {
+            const float alpha = grad.alphas[p.pix];
+            float v_a = grad.v_alphas[p.pix], bg_dot = 0.f;
+            T = 1.f - alpha;
+            if (grad.expected != nullptr) {
+                divisor = fmaxf(alpha, kExpectedMin);
+                if (alpha >= kExpectedMin) v_a -= v_out[n - 1] * grad.expected[p.pix * n + n - 1] / divisor;
+            }
+            for (uint32_t k = 0; p.bg != nullptr && k < n; ++k) bg_dot += p.bg[k] * (k + 1 == n ? v_out[k] / divisor : v_out[k]);
+            behind = -T * (v_a - bg_dot);
+        }
+        for (int32_t idx = __reduce_max_sync(0xffffffffu, last); idx >= range.start; --idx) {
+            const size_t g = (size_t)a.flatten_ids[idx];
+            const PixelAlpha e = pixel_alpha(a, (int32_t)g, p);
+            const bool ok = e.blends && idx <= last;
+            if (!__any_sync(0xffffffffu, ok)) continue;
+            float fac = 0.f, v_alpha = 0.f;
+            if (ok) {
+                const float alpha = fminf(kAlphaMax, e.alpha), ra = 1.f / (1.f - alpha);
+                T *= ra;
+                fac = alpha * T;
+                float dot = 0.f;
+                for (uint32_t k = 0; k < n; ++k) dot = fmaf(a.colors[g * n + k], k + 1 == n ? v_out[k] / divisor : v_out[k], dot);
+                v_alpha = fmaf(T, dot, -ra * behind);
+                behind = fmaf(fac, dot, behind);
+            }
+            for (uint32_t k = 0; k < n; ++k)
+                add_warp_total(grad.colors + g * n + k, ok ? fac * (k + 1 == n ? v_out[k] / divisor : v_out[k]) : 0.f);
+            // a capped alpha passes no gradient on to the geometry
+            float v = 0.f, wx = 0.f, wy = 0.f, q0 = 0.f, q1 = 0.f, q2 = 0.f, vx = 0.f, vy = 0.f;
+            if (ok && e.alpha <= kAlphaMax) {
+                v = e.vis * v_alpha;
+                const float w = -e.B.w * v;   // dL/dsigma
+                q0 = 0.5f * w * e.dx * e.dx;
+                q1 = w * e.dx * e.dy;
+                q2 = 0.5f * w * e.dy * e.dy;
+                wx = kLn2 * e.B.w * v * (2.f * e.B.x * e.dx + e.B.y * e.dy);
+                wy = kLn2 * e.B.w * v * (e.B.y * e.dx + 2.f * e.B.z * e.dy);
+                vx = wx * p.roll;
+                vy = wy * p.roll;
+            }
+            add_warp_total(grad.conics + 3 * g, q0);
+            add_warp_total(grad.conics + 3 * g + 1, q1);
+            add_warp_total(grad.conics + 3 * g + 2, q2);
+            add_warp_total(grad.means2d + 2 * g, wx);
+            add_warp_total(grad.means2d + 2 * g + 1, wy);
+            add_warp_total(grad.pix_vels + 2 * g, vx);
+            add_warp_total(grad.pix_vels + 2 * g + 1, vy);
+            add_warp_total(grad.opacities + g, v);
+            if (grad.means2d_abs != nullptr) {
+                add_warp_total(grad.means2d_abs + 2 * g, fabsf(wx));
+                add_warp_total(grad.means2d_abs + 2 * g + 1, fabsf(wy));
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------
 // Camera forward. Bound by instruction issue: two pixels per thread take 50 instructions per entry where
 // one took 40, and a warp passes over the entries that cannot reach its 8 x 8 patch without looking at
 // them. A pixel that has stopped moves its column out to where every alpha vanishes, which costs the
 // other pixels nothing; a warp leaves when all of its pixels have. Camera benchmark frame: 0.338 -> 0.209 ms.
 // ---------------------------------------------------------------------------------------
-constexpr float kExpectedMin = 1e-10f;   // alphas below it do not divide (gsplat/rendering.py:423-430)
 constexpr float kPixelGone = 1e18f;   // a column no Gaussian reaches: sigma overflows, alpha is 0 (or NaN, never drawn)
 
 // registers per thread: as many CTAs of 128 threads per SM as the accumulators leave room for
@@ -304,6 +473,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
     }
     const bool vec_out = channels == 4u && (reinterpret_cast<uintptr_t>(render_colors) & 15u) == 0u;
     const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
+    float none = 0.f;   // a NaN: see odd_pixels_fwd()
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         if ((uint32_t)h >= n_inside) break;
@@ -312,6 +482,8 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
         render_alphas[pix] = 1.f - Tk;
         last_ids[pix] = h ? pos1 : pos0;
         float *dst = render_colors + pix * channels;
+#pragma unroll
+        for (int k = 0; k < CDIM; ++k) none = fmaf(out[h][k], 0.f, none);
         if (CDIM == 4 && vec_out) {   // one 16-byte store per pixel
             float4 v = make_float4(out[h][0], out[h][1], out[h][2], out[h][3]);
             if (bg) v = make_float4(v.x + Tk * bg[0], v.y + Tk * bg[1], v.z + Tk * bg[2], v.w + Tk * bg[3]);
@@ -326,6 +498,11 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
                 if (expected && (uint32_t)k + 1u == channels) v /= fmaxf(1.f - Tk, kExpectedMin);
                 dst[k] = v;
             }
+    }
+    if (none != 0.f) {
+        const PixelTask task = {C, W, H, tile_size, tile_w, tile_h, channels, n_isects, means2d, pix_vels, conics, opacities,
+                                colors, rs_time, backgrounds, offsets, flatten_ids};
+        odd_pixels_fwd<2>(task, render_colors, render_alphas, last_ids, expected != 0u);
     }
 }
 
@@ -624,11 +801,13 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
     const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
     __syncthreads();   // the rendered rows take the place of the feature rows
     float *rows = sFeat + warp * 32u * CDIM;
+    float none = 0.f;   // a NaN: see odd_points_bwd()
 #pragma unroll
     for (int k = 0; k < CDIM; ++k)
         if ((uint32_t)k < channels) {
             float v = pix_out[k];
             if ((uint32_t)k == depth_idx) v += depth_extra;
+            none = fmaf(v, 0.f, none);
             if (bg) v += T * bg[k];
             v = inside ? v : 0.f;
             if (pp.patched) rows[lane * channels + k] = v;
@@ -636,7 +815,7 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
         }
     if (in_image) {
         render_alphas[pix] = inside ? 1.f - T : 0.f;
-        last_ids[pix] = inside ? cur_idx : 0;
+        last_ids[pix] = inside ? cur_idx | (none != 0.f ? kOddPixel : 0) : 0;
         median_depths[pix] = inside ? median : 0.f;
         if (alpha_sum_out != nullptr) alpha_sum_out[pix] = inside ? alpha_sum : 0.f;
     }
@@ -793,17 +972,15 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
                 const uint32_t q = warp + r * kCoopWarps;
                 const float before = al[q * 32], next_T = before * (1.f - alpha[r]);
                 const bool take = alpha[r] > 0.f && next_T > kTStop;
-                const float vis = take ? alpha[r] * before : 0.f;
-                if (!__any_sync(0xffffffffu, take)) continue;
-                const float range_q = sC[c0 + q].w;
                 if (take) {
+                    const float vis = alpha[r] * before, range_q = sC[c0 + q].w;
                     depth_extra += dterm[r] * vis;
                     if (before > 0.5f && next_T <= 0.5f) median = range_q + dterm[r];
                     if (compute_alpha_sum && range_q < alpha_sum_limit) alpha_sum += alpha[r];
                     cur_idx = sPos[c0 + q];
                     T = next_T;
+                    axpy_staged_full<CDIM>(pix_out, sFeat + (c0 + q) * CDIM, vis);   // here: elsewhere it would be 0 * inf
                 }
-                axpy_staged_full<CDIM>(pix_out, sFeat + (c0 + q) * CDIM, vis);
             }
         }
     }
@@ -821,23 +998,29 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     s_extra[tr] = depth_extra;
     s_sum[tr] = alpha_sum;
     s_median[tr] = median;
-    s_last[tr] = cur_idx;
+    float none = fmaf(depth_extra, 0.f, 0.f);   // a NaN: see odd_points_bwd()
+#pragma unroll
+    for (int k = 0; k < CDIM; ++k) none = fmaf(pix_out[k], 0.f, none);
+    s_last[tr] = none != 0.f ? cur_idx | kOddPixel : cur_idx;
     __syncthreads();
     // the last transmittance and the last entry are the smallest and the largest of the warps'; the median
     // was met by one warp alone
     T = s_T[lane]; depth_extra = s_extra[lane]; alpha_sum = s_sum[lane]; median = s_median[lane]; cur_idx = s_last[lane];
+    int32_t mark = cur_idx & kOddPixel;
+    cur_idx = last_position(cur_idx);
 #pragma unroll
     for (uint32_t w = 1; w < kCoopWarps; ++w) {
         T = fminf(T, s_T[w * 32 + lane]);
         depth_extra += s_extra[w * 32 + lane];
         alpha_sum += s_sum[w * 32 + lane];
         median += s_median[w * 32 + lane];
-        cur_idx = max(cur_idx, s_last[w * 32 + lane]);
+        mark |= s_last[w * 32 + lane] & kOddPixel;
+        cur_idx = max(cur_idx, last_position(s_last[w * 32 + lane]));
     }
     if (warp == 0 && in_image) {
         // points that are not rendered (range <= 0) produce zeros everywhere
         render_alphas[pix] = inside ? 1.f - T : 0.f;
-        last_ids[pix] = inside ? cur_idx : 0;
+        last_ids[pix] = inside ? cur_idx | mark : 0;
         median_depths[pix] = inside ? median : 0.f;
         if (alpha_sum_out != nullptr) alpha_sum_out[pix] = inside ? alpha_sum : 0.f;
     }
@@ -1025,13 +1208,14 @@ rasterize_to_pixels_bwd_kernel(
     float v_out[PX][CDIM];           // cotangents of the pixels' channels
     int32_t bin_final[PX];
     int32_t thread_last = -1;
+    float none = 0.f;                // a NaN: see odd_pixels_bwd()
 #pragma unroll
     for (int k = 0; k < PX; ++k) {
         const bool in = (uint32_t)k < n_inside;
         const size_t pix = ((size_t)cam * H + (in ? i : 0u)) * W + (in ? j + k : 0u);
         const float a_final = in ? render_alphas[pix] : 0.f, T_final = 1.f - a_final;
         bin_final[k] = in ? last_ids[pix] : -1;
-        thread_last = max(thread_last, bin_final[k]);
+        thread_last = (in && bin_final[k] < 0) ? INT32_MAX : max(thread_last, bin_final[k]);
         float v_a = in ? v_render_alphas[pix] : 0.f;
         float bg_dot = 0.f;
         const float divisor = fmaxf(a_final, kExpectedMin);
@@ -1043,15 +1227,25 @@ rasterize_to_pixels_bwd_kernel(
             if (expected != nullptr && (uint32_t)c + 1u == channels) v_out[k][c] /= divisor;
             if (backgrounds != nullptr && (uint32_t)c < channels)
                 bg_dot += backgrounds[(size_t)cam * channels + c] * v_out[k][c];
+            none = fmaf(v_out[k][c], 0.f, none);
         }
         // what the background and the alpha output receive through everything in front of them
         const float last = -T_final * (v_a - bg_dot);
+        none = fmaf(last, 0.f, none);
         if (k & 1) { T[k / 2].y = T_final; behind[k / 2].y = last; }
         else { T[k / 2].x = T_final; behind[k / 2].x = last; }
     }
 
     // last list position consumed by any pixel of this tile / warp
-    const int32_t tile_last = block_max_int(thread_last, red);
+    const int32_t tile_last = block_max_int(none != 0.f ? INT32_MAX : thread_last, red);
+    if (tile_last == INT32_MAX) {
+        const PixelTask task = {C, W, H, tile_size, tile_w, tile_h, channels, n_isects, means2d, pix_vels, conics, opacities,
+                                colors, rs_time, backgrounds, offsets, flatten_ids};
+        const PixelGrads grads = {render_alphas, v_render_colors, v_render_alphas, expected, last_ids, v_means2d,
+                                  kAbs ? v_means2d_abs : nullptr, v_conics, v_colors, v_opacities, v_pix_vels};
+        odd_pixels_bwd<PX>(task, grads);
+        return;
+    }
     const int32_t warp_last = __reduce_max_sync(0xffffffffu, thread_last);
     const int32_t eff_end = min(range.end, tile_last + 1);
     if (eff_end <= range.start) return;
@@ -1244,6 +1438,113 @@ __device__ __forceinline__ GradSlot point_grad_slot(int slot, int cdim, uint32_t
     }
 }
 
+// What odd_pixels_bwd() is to cameras: the patch of the calling warp, two points per lane, one after the other.
+struct PointTask {
+    uint32_t C, W, H, tile_width, tile_height, grid_w, grid_h, ctas_per_tile, channels, depth_idx;
+    int64_t n_isects;
+    bool alpha_sum;
+    float alpha_sum_threshold;
+    const float2 *means2d, *depth_comps;
+    const float *pix_vels, *conics, *opacities, *colors, *ranges, *backgrounds;
+    const float4 *raster_pts;
+    const int32_t *offsets, *flatten_ids;
+};
+
+struct PointGrads {
+    const float *alphas, *v_colors_in, *v_alphas, *v_alpha_sum;
+    const int32_t *last_ids;
+    float *means2d, *means2d_abs, *conics, *colors, *ranges, *opacities, *pix_vels, *depth_comps;
+};
+
+__device__ __noinline__ void odd_points_bwd(const PointTask &a, const PointGrads &grad) {
+    const uint32_t n = a.channels, fstride = a.ranges ? n - 1 : n, per_cam = a.grid_w * a.grid_h;
+    const uint32_t gtile = blockIdx.x / a.ctas_per_tile, part = blockIdx.x - gtile * a.ctas_per_tile, cam = gtile / per_cam;
+    const uint32_t tile = gtile - cam * per_cam, ty = tile / a.grid_w, tx = tile - ty * a.grid_w;
+    const TileRange tiles = tile_range(a.offsets, gtile, a.C * per_cam, a.n_isects);
+    const PointPatch pp = point_patch<2>(a.tile_width, a.tile_height, part * 32u + (threadIdx.x & 31u));
+    for (uint32_t h = 0; h < 2; ++h) {
+        uint32_t row = pp.row, col = pp.col + h;
+        if (col >= a.tile_width) { col -= a.tile_width; ++row; }
+        const uint32_t i = ty * a.tile_height + row, j = tx * a.tile_width + col;
+        const size_t pix = ((size_t)cam * a.H + i) * a.W + j;
+        float4 pt = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < a.tile_height && i < a.H && j < a.W) pt = a.raster_pts[pix];
+        int32_t last = -1;
+        float T = 1.f, behind = 0.f, v_depth = 0.f, v_asum = 0.f;
+        const float *v_out = grad.v_colors_in + pix * n;
+        if (pt.z > 0.f) {
+            last = min(tiles.end - 1, last_position(grad.last_ids[pix]));
+            T = 1.f - grad.alphas[pix];
+            float bg_dot = 0.f;
+            for (uint32_t k = 0; a.backgrounds != nullptr && k < n; ++k) bg_dot += a.backgrounds[(size_t)cam * n + k] * v_out[k];
+            behind = -T * (grad.v_alphas[pix] - bg_dot);
+            v_depth = v_out[a.depth_idx];
+            if (a.alpha_sum && grad.v_alpha_sum != nullptr) v_asum = grad.v_alpha_sum[pix];
+        }
+        for (int32_t idx = __reduce_max_sync(0xffffffffu, last); idx >= tiles.start; --idx) {
+            const size_t g = (size_t)a.flatten_ids[idx];
+            const PointEntry e = load_point_entry((int32_t)g, a.means2d, a.conics, a.opacities, a.pix_vels, a.depth_comps);
+            const float range = a.ranges ? a.ranges[g] : a.colors[g * n + a.depth_idx];
+            const PointFootprint f = point_footprint(e.A, e.B, pt.w, pt.x, pt.y);
+            const float alpha = fminf(kAlphaMax, e.B.w * f.vis);
+            const bool ok = idx <= last && !(f.sigma < 0.f || alpha < kAlphaMin);
+            if (!__any_sync(0xffffffffu, ok)) continue;
+            float fac = 0.f, v_alpha = 0.f;
+            if (ok) {
+                const float ra = 1.f / (1.f - alpha);
+                T *= ra;
+                fac = alpha * T;
+                float dot = (e.C.y * f.dx + e.C.z * f.dy + e.C.x * pt.w) * v_depth;
+                for (uint32_t k = 0; k < fstride; ++k) dot = fmaf(a.colors[g * fstride + k], v_out[k], dot);
+                if (a.ranges) dot = fmaf(range, v_out[fstride], dot);
+                v_alpha = fmaf(T, dot, -ra * behind);
+                behind = fmaf(fac, dot, behind);
+            }
+            for (uint32_t k = 0; k < fstride; ++k) add_warp_total(grad.colors + g * fstride + k, ok ? fac * v_out[k] : 0.f);
+            if (a.ranges) add_warp_total(grad.ranges + g, ok ? fac * v_out[fstride] : 0.f);
+            float q0 = 0.f, q1 = 0.f, q2 = 0.f, mx = 0.f, my = 0.f, ax = 0.f, ay = 0.f, v_o = 0.f;
+            float vd = 0.f, vx = 0.f, vy = 0.f, vz = 0.f, dx = 0.f, dy = 0.f;
+            const auto through_sigma = [&](float v, float gx, float gy) {
+                const float w = -e.B.w * v;   // dL/dsigma
+                const float ux = w * (e.B.x * f.dx + e.B.y * f.dy) + gx, uy = w * (e.B.y * f.dx + e.B.z * f.dy) + gy;
+                q0 += 0.5f * w * f.dx * f.dx;
+                q1 += w * f.dx * f.dy;
+                q2 += 0.5f * w * f.dy * f.dy;
+                mx += ux;
+                my += uy;
+                vx = mx * pt.w;
+                vy = my * pt.w;
+                ax += fabsf(ux);
+                ay += fabsf(uy);
+                v_o += v;
+            };
+            if (ok && e.B.w * f.vis <= kAlphaMax) {   // a capped alpha passes no gradient on to the geometry
+                vd = fac * v_depth;
+                vz = vd * pt.w;
+                dx = vd * f.dx;
+                dy = vd * f.dy;
+                through_sigma(f.vis * v_alpha, vd * e.C.y, vd * e.C.z);
+            }
+            if (ok && a.alpha_sum && range < pt.z - a.alpha_sum_threshold) through_sigma(f.vis * v_asum, 0.f, 0.f);
+            add_warp_total(grad.conics + 3 * g, q0);
+            add_warp_total(grad.conics + 3 * g + 1, q1);
+            add_warp_total(grad.conics + 3 * g + 2, q2);
+            add_warp_total(grad.means2d + 2 * g, mx);
+            add_warp_total(grad.means2d + 2 * g + 1, my);
+            add_warp_total(grad.pix_vels + 3 * g, vx);
+            add_warp_total(grad.pix_vels + 3 * g + 1, vy);
+            add_warp_total(grad.pix_vels + 3 * g + 2, vz);
+            add_warp_total(grad.depth_comps + 2 * g, dx);
+            add_warp_total(grad.depth_comps + 2 * g + 1, dy);
+            add_warp_total(grad.opacities + g, v_o);
+            if (grad.means2d_abs != nullptr) {
+                add_warp_total(grad.means2d_abs + 2 * g, ax);
+                add_warp_total(grad.means2d_abs + 2 * g + 1, ay);
+            }
+        }
+    }
+}
+
 constexpr uint32_t kPointsBwdStage = 2;   // entries per thread and batch: their loads overlap
 
 template <int CDIM, bool kAbs>
@@ -1292,6 +1593,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
     float2 az, el, roll, T, behind, v_depth, v_asum, sum_limit;
     float v_out[2][CDIM];
     int32_t bin_final[2], thread_last = -1;
+    float none = 0.f;   // a NaN: see odd_points_bwd()
     PointExtent extent;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -1309,7 +1611,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         if (in) extent.add(rp.x, rp.y, rp.w);
         const float T_final = in ? 1.f - render_alphas[pix] : 1.f;
         bin_final[h] = in ? last_ids[pix] : -1;
-        thread_last = max(thread_last, bin_final[h]);
+        thread_last = (in && bin_final[h] < 0) ? INT32_MAX : max(thread_last, bin_final[h]);
         float bg_dot = 0.f, vd = 0.f;
 #pragma unroll
         for (int c = 0; c < CDIM; ++c) {
@@ -1317,11 +1619,13 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
             if ((uint32_t)c == depth_idx) vd = v_out[h][c];
             if (backgrounds != nullptr && (uint32_t)c < channels)
                 bg_dot += backgrounds[(size_t)cam * channels + c] * v_out[h][c];
+            none = fmaf(v_out[h][c], 0.f, none);
         }
         const float va = in ? v_render_alphas[pix] : 0.f;
         const float vs = (in && compute_alpha_sum && v_alpha_sum != nullptr) ? v_alpha_sum[pix] : 0.f;
         // what the background and the alpha output receive through everything in front of them
         const float last = -T_final * (va - bg_dot);
+        none = fmaf(last, 0.f, fmaf(vs, 0.f, none));
         const float limit = rp.z - alpha_sum_threshold;
         if (h) { az.y = rp.x; el.y = rp.y; roll.y = rp.w; T.y = T_final; behind.y = last; v_depth.y = vd; v_asum.y = vs; sum_limit.y = limit; }
         else { az.x = rp.x; el.x = rp.y; roll.x = rp.w; T.x = T_final; behind.x = last; v_depth.x = vd; v_asum.x = vs; sum_limit.x = limit; }
@@ -1329,7 +1633,19 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
     if (warp == 0) extent.write_box(&s_box);
 
     // last list position consumed by any of the patch's points
-    const int32_t eff_end = min(range.end, __reduce_max_sync(0xffffffffu, thread_last) + 1);
+    const int32_t patch_last = __reduce_max_sync(0xffffffffu, none != 0.f ? INT32_MAX : thread_last);
+    if (patch_last == INT32_MAX) {
+        if (warp != 0u) return;
+        const PointTask task = {C, W, H, tile_width, tile_height, grid_w, grid_h, ctas_per_tile, channels, depth_idx, n_isects,
+                                compute_alpha_sum != 0, alpha_sum_threshold, means2d, depth_comps, pix_vels, conics, opacities,
+                                colors, ranges, backgrounds, raster_pts, offsets, flatten_ids};
+        const PointGrads grads = {render_alphas, v_render_colors, v_render_alphas, v_alpha_sum, last_ids, v_means2d,
+                                  kAbs ? v_means2d_abs : nullptr, v_conics, v_colors, v_ranges, v_opacities, v_pix_vels,
+                                  v_depth_comps};
+        odd_points_bwd(task, grads);
+        return;
+    }
+    const int32_t eff_end = min(range.end, patch_last + 1);
     if (eff_end <= range.start) return;
     const uint32_t num_batches = (uint32_t)(eff_end - range.start + cap - 1) / cap;
 
