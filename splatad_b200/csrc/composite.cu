@@ -123,7 +123,10 @@ __device__ __forceinline__ PixelEntry load_pixel_entry(int32_t g, const float2 *
     return e;
 }
 
+constexpr uint32_t kOddEntry = 1u << 31;   // beside the warps of a CTA: see odd_pixels_fwd()
+
 // The mean moves with the row's shutter time; roll_lo / roll_hi bound it over the tile.
+template <bool kMarkOdd>
 __device__ __forceinline__ uint32_t warps_that_see(const PixelEntry &e, const PatchBox *s_box, uint32_t n_warps,
                                                    float roll_lo, float roll_hi) {
     const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
@@ -133,6 +136,10 @@ __device__ __forceinline__ uint32_t warps_that_see(const PixelEntry &e, const Pa
     const float mx_lo = fminf(mx_a, mx_b), mx_hi = fmaxf(mx_a, mx_b);
     const float my_lo = fminf(my_a, my_b), my_hi = fmaxf(my_a, my_b);
     uint32_t seen = 0u;
+    if (kMarkOdd) {   // a NaN somewhere, an opacity without bound, a conic too flat or too steep
+        const bool plain = fabsf(e.B.x) > 1e-30f && fabsf(e.B.x) + fabsf(e.B.y) + fabsf(e.B.z) < 1e30f;
+        if (!plain || !(mx_lo <= mx_hi) || !(my_lo <= my_hi) || !(test.s_max < 1e30f)) seen = kOddEntry;
+    }
     for (uint32_t w = 0; w < n_warps; ++w) {
         const PatchBox b = s_box[w];
         if (b.x0 <= b.x1 && !test.misses(mx_lo - b.x1, mx_hi - b.x0, my_lo - b.y1, my_hi - b.y0)) seen |= 1u << w;
@@ -162,8 +169,11 @@ __device__ __forceinline__ float2 pair_power(float a, float2 dx, float bdy, floa
 // blends, with weight zero where it is not blended - and zero times an infinity is a NaN. A pixel that comes out
 // with one is worked out again by itself, and its last id marked: the backward kernel leaves the tiles that hold
 // a mark, or a cotangent that is not finite, to a pass in which a pixel takes nothing from an entry that it does
-// not blend. Both out of line and from nothing but the kernels' own arguments, so that the kernels hold
-// nothing for them. (Looking at the staged colours instead costs the forward kernel of the camera benchmark 220 ->
+// not blend. A NaN in an entry's geometry or opacity makes its alpha the largest there is wherever sigma is not
+// negative; the kernels' comparisons drop it, and theirs is also a conic so flat that it reaches the column a pixel
+// moves to when it stops (see kPixelGone): a warp that meets such an entry works all of its pixels out again.
+// Both out of line and from nothing but the kernels' own arguments, so that the kernels hold nothing for
+// them. (Looking at the staged colours instead costs the forward kernel of the camera benchmark 220 ->
 // 237 us and the backward one 396 -> 440; two loop bodies, one of them careful, 6 to 9 % of a training step.)
 // ---------------------------------------------------------------------------------------
 constexpr int32_t kOddPixel = INT32_MIN;   // in a last id: the pixel blended something that is not finite
@@ -217,7 +227,7 @@ __device__ __forceinline__ PixelAlpha pixel_alpha(const PixelTask &a, int32_t g,
     const float power = fmaf(fmaf(r.B.x, r.dx, r.B.y * r.dy), r.dx, r.B.z * r.dy * r.dy);
     r.vis = exp2_approx(power);
     r.alpha = r.B.w * r.vis;
-    r.blends = power <= 0.f && r.alpha >= kAlphaMin;
+    r.blends = !(power > 0.f) && !(r.alpha < kAlphaMin);   // a NaN is blended, with the capped alpha
     return r;
 }
 
@@ -387,6 +397,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
     float out[2][CDIM];
 #pragma unroll
     for (int k = 0; k < CDIM; ++k) out[0][k] = out[1][k] = 0.f;
+    uint32_t odd = 0u;   // kOddEntry: the warp was to blend one
     bool warp_done = __all_sync(0xffffffffu, n_inside == 0);
 
     int32_t next_id = 0;
@@ -400,7 +411,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
         if (idx < range.end) {
             e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
             if (idx + (int32_t)bs < range.end) next_id = flatten_ids[idx + bs];   // on its way meanwhile
-            e.seen = warps_that_see(e, s_box, n_warps, roll_lo, roll_hi);
+            e.seen = warps_that_see<true>(e, s_box, n_warps, roll_lo, roll_hi);
         }
         // compact the survivors to the front of the staging arrays, list order kept
         const uint32_t kept_mask = __ballot_sync(0xffffffffu, e.seen != 0u);
@@ -426,7 +437,9 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
         uint32_t last0 = kNoEntry, last1 = kNoEntry;   // this batch's
         for (uint32_t t0 = 0; t0 < n_kept && !warp_done; t0 += 32) {
             const uint32_t mine = t0 + lane;
-            uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u));
+            const uint32_t seen = mine < n_kept ? sSeen[mine] : 0u;
+            uint32_t todo = __ballot_sync(0xffffffffu, (seen >> warp) & 1u);
+            odd |= seen;
             while (todo) {
                 const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
                 todo &= todo - 1u;
@@ -499,7 +512,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
                 dst[k] = v;
             }
     }
-    if (none != 0.f) {
+    if (__any_sync(0xffffffffu, odd >= kOddEntry) || none != 0.f) {
         const PixelTask task = {C, W, H, tile_size, tile_w, tile_h, channels, n_isects, means2d, pix_vels, conics, opacities,
                                 colors, rs_time, backgrounds, offsets, flatten_ids};
         odd_pixels_fwd<2>(task, render_colors, render_alphas, last_ids, expected != 0u);
@@ -1272,7 +1285,7 @@ rasterize_to_pixels_bwd_kernel(
         e.seen = 0u;
         if (idx >= range.start) {
             e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
-            e.seen = warps_that_see(e, s_box, n_warps, roll_lo, roll_hi);
+            e.seen = warps_that_see<false>(e, s_box, n_warps, roll_lo, roll_hi);
             const int32_t ahead = idx - (int32_t)bs;   // the id of the next batch's entry is on its way meanwhile
             if (ahead >= range.start) next_id = flatten_ids[ahead];
         }

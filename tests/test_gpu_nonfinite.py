@@ -111,3 +111,43 @@ def test_a_cotangent_that_is_not_finite_reaches_its_own_gaussians_only(kind, a, 
         g, w = _per_row(got[name])[~mine], _per_row(want[name])[~mine]
         assert torch.isfinite(g).all(), name
         _close(g, w, 5e-4)        # sums in another order (atomics): 1e-4 from run to run
+
+
+@pytest.mark.parametrize("channels", [3, 13])
+@pytest.mark.parametrize("what", ["opacities", "means2d", "conics", "pix_vels", "one row", "flat conic"])
+def test_a_nan_in_the_geometry_is_blended_with_the_capped_alpha(what, channels):
+    """As in the reference, whose minimum of the cap and a NaN is the cap, and as in the oracle."""
+    import numpy as np
+    from gpu_util import assert_close, n, t
+    from oracle import composite
+    from splatad_b200 import ops
+    from test_gpu_composite import _camera_case
+    H = 1 if what == "one row" else 60
+    c = _camera_case(1, 300, 100, H, 16, channels, 5)
+    if what == "flat conic":                       # and opaque enough around it that pixels have stopped before
+        c["conics"][:, ::3] = 0.0
+        c["opacities"][:] = 0.6
+    elif what != "one row":
+        c[what][:, ::29] = float("nan")
+    args = [n(c[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels", "rs")]
+    tail = (None, c["W"], c["H"], c["ts"], c["offsets"], c["flatten_ids"])
+    ref = composite.rasterize_to_pixels_fwd(*args, *tail)
+    leaves = {k: t(c[k]).requires_grad_(True) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")}
+    image, alphas = ops.rasterize_to_pixels(
+        leaves["means2d"], leaves["conics"], leaves["colors"], leaves["opacities"], leaves["pix_vels"], c["W"], c["H"], c["ts"],
+        t(c["offsets"], torch.int32), t(c["flatten_ids"], torch.int32), t(c["rs"]))
+    sure = ~ref["ambiguous"]
+    assert sure.mean() > 0.95 and ref["contributing"] > c["W"] * c["H"] // 2
+    assert_close("colors", n(image), ref["render_colors"], 1e-4, 1e-5, mask=sure[..., None])
+    assert_close("alphas", n(alphas), ref["render_alphas"], 1e-4, 1e-5, mask=sure[..., None])
+    mask = sure.astype(np.float32)
+    (image * t(mask)[..., None]).sum().backward()
+    f64 = composite.rasterize_to_pixels_fwd(*args, *tail, dtype=np.float64)
+    want = composite.rasterize_to_pixels_bwd(*args, *tail, f64["render_alphas"], f64["last_ids"],
+                                             np.broadcast_to(mask[..., None], n(image).shape).astype(np.float64),
+                                             np.zeros(n(alphas).shape))
+    for k in ("means2d", "conics", "colors", "opacities", "pix_vels"):
+        got, ref_k = n(leaves[k].grad), want["v_" + k]
+        assert np.array_equal(np.isfinite(got), np.isfinite(ref_k)), k
+        got, ref_k = np.nan_to_num(got).astype(np.float64), np.nan_to_num(ref_k)
+        assert np.linalg.norm(got - ref_k) <= 2e-3 * max(np.linalg.norm(ref_k), 1e-20), k
