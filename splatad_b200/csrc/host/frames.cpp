@@ -86,6 +86,16 @@ bool plain(const Tensor &t, c10::DeviceIndex dev) {
 }
 bool plain(const OptTensor &t, c10::DeviceIndex dev) { return !t || plain(*t, dev); }
 
+// The frame goes into the graph if any of the tensors its nodes take requires a gradient, also one that gets none.
+bool wants_grad(std::initializer_list<const Tensor *> all, std::initializer_list<const OptTensor *> maybe) {
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor *t : all)
+        if (t->requires_grad()) return true;
+    for (const OptTensor *t : maybe)
+        if (*t && (*t)->requires_grad()) return true;
+    return false;
+}
+
 bool shaped(const Tensor &t, at::IntArrayRef s) { return t.sizes() == s; }
 bool shaped(const OptTensor &t, at::IntArrayRef s) { return !t || t->sizes() == s; }
 
@@ -410,8 +420,7 @@ py::object lidar_frame(const Tensor &means, const Tensor &quats, const Tensor &s
         return py::none();
     if ((int64_t)lib.splatad_lidar_azimuth_tiles((float)(az_res * (double)tile_w)) != cols || cols * tile_w < W || rows * tile_h < H)
         return py::none();
-    const bool grad = at::GradMode::is_enabled() && (means.requires_grad() || quats.requires_grad() || scales.requires_grad() ||
-                                                     opacities.requires_grad() || features.requires_grad());
+    const bool grad = wants_grad({&means, &quats, &scales, &opacities, &features, &raster_pts}, {&velocities, &lin, &ang, &rs});
 
     const c10::cuda::CUDAGuard guard(dev);
     const auto stream = c10::cuda::getCurrentCUDAStream();
@@ -693,8 +702,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
     if (channels > max_channels || channels > SPLATAD_MAX_CHANNELS) return py::none();
     if (backgrounds && mode != 2 && !shaped(backgrounds, {C, D})) return py::none();
     if (tile_size * tile_size > 512 && channels > 16) return py::none();   // the backward pass would refuse it
-    const bool grad = at::GradMode::is_enabled() && (means.requires_grad() || quats.requires_grad() || scales.requires_grad() ||
-                                                     opacities.requires_grad() || (mode != 2 && colors.requires_grad()));
+    const bool grad = wants_grad({&means, &quats, &scales, &opacities, &Ks, mode == 2 ? &means : &colors}, {&velocities, &lin, &ang, &rs});
 
     const c10::cuda::CUDAGuard guard(dev);
     const auto stream = c10::cuda::getCurrentCUDAStream();

@@ -42,3 +42,23 @@ def test_a_frame_that_sees_nothing_has_zero_gradients(kind):
     for k in names:
         assert leaves[k].grad is not None and float(leaves[k].grad.abs().max()) == 0.0, k
     assert float(meta["means2d"].grad.abs().max()) == 0.0 and float(meta["means2d"].absgrad.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("kind,name", [("lidar", "velocities"), ("lidar", "linear_velocity"), ("lidar", "raster_pts"),
+                                       ("camera", "velocities"), ("camera", "Ks"), ("camera", "rolling_shutter_time")])
+def test_a_tensor_without_a_gradient_of_its_own_keeps_the_frame_in_the_graph(kind, name):
+    """The ops take it as an input of a node and give it no gradient; so does a frame's second call."""
+    import splatad_b200
+    from splatad_b200 import scenes
+    g = _to_gpu(scenes.config2(N=20_011) if kind == "lidar" else scenes.config1(N=20_011))
+    render = splatad_b200.lidar_rasterization if kind == "lidar" else splatad_b200.rasterization
+    if g.get(name) is None:
+        assert name == "velocities"
+        g[name] = torch.zeros_like(g["means"])
+    g[name] = g[name].clone().requires_grad_(True)
+    _forget()
+    for _ in range(2):
+        images = render(**g)
+        assert images[0].requires_grad
+        images[0].sum().backward()
+        assert g[name].grad is None
