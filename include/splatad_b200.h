@@ -469,7 +469,7 @@ int splatad_rasterize_expected_to_pixels_bwd(
  * colors [N,D] ([C,N,D] with colors_per_camera != 0), the depths [n] behind them when given.
  * VJPs: v_opacities [N] and v_colors are accumulated with atomics (zero-initialise them),
  * v_compensations [n] and v_depths [n] = v_depths_in (NULL: 0) + the last of `width` channels are
- * written; each may be NULL. */
+ * written; each may be NULL, and opacities too where v_compensations is. */
 int splatad_opacity_rows_fwd(uint32_t n, uint32_t N, const int64_t *gaussian_ids, const float *opacities,
                              const float *compensations, float *rows, void *stream);
 int splatad_opacity_rows_bwd(uint32_t n, uint32_t N, const int64_t *gaussian_ids, const float *opacities,

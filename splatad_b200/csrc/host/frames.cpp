@@ -214,6 +214,12 @@ Tensor zero_motion(int64_t C, const at::TensorOptions &options) {
     return t;
 }
 
+// The opacities as a projection node keeps them: not at all unless a compensation's gradient needs their values, and
+// where the ops multiply a copy of them, a copy - what may be edited in place behind the ops may be here.
+Tensor kept_opacities(const Tensor &opacities, const Tensor &comps, bool copied) {
+    return !comps.defined() ? Tensor() : copied ? opacities.detach().clone() : opacities;
+}
+
 // What came of the lists: the caller keeps the counts and decides whether the frame stands.
 struct Counts {
     int64_t n_isects = 0, status = 0, depth_range = 0;
@@ -296,7 +302,8 @@ struct LidarProjectionNode : torch::autograd::Function<LidarProjectionNode> {
     static variable_list forward(AutogradContext *ctx, const Tensor &means, const Tensor &quats, const Tensor &scales,
                                  const Tensor &opacities, const OptTensor &velocities, const Tensor &viewmats, const Tensor &lin,
                                  const Tensor &ang, const Tensor &rs, c10::intrusive_ptr<LidarFrame> f) {
-        ctx->save_for_backward({means, quats, scales, opacities, velocities.value_or(Tensor()), viewmats, lin, ang, rs, f->conics, f->comps, f->radii});
+        ctx->save_for_backward({means, quats, scales, kept_opacities(opacities, f->comps, f->C > 1), velocities.value_or(Tensor()), viewmats, lin,
+                                ang, rs, f->conics, f->comps, f->radii});
         auto kept = c10::make_intrusive<LidarFrame>();   // sizes only: the outputs must not hold themselves
         kept->C = f->C; kept->N = f->N; kept->eps2d = f->eps2d;
         keep_state(ctx, kept);
@@ -523,6 +530,7 @@ py::object lidar_frame(const Tensor &means, const Tensor &quats, const Tensor &s
 // ---------------------------------------------------------------------------------------------
 struct CameraFrame : torch::CustomClassHolder {
     int64_t C = 0, N = 0, n = 0, W = 0, H = 0, tile_size = 0, tile_w = 0, tile_h = 0, channels = 0, n_isects = 0;
+    std::vector<int64_t> color_sizes;
     int64_t K = 0, D = 0, sh_degree = -1;     // spherical harmonics (K coefficients) or D plain channels
     bool packed = false, per_camera = false, depth = false, expected = false, absgrad = false;
     float eps2d = 0.f;
@@ -534,6 +542,7 @@ struct CameraFrame : torch::CustomClassHolder {
         k->C = C; k->N = N; k->n = n; k->W = W; k->H = H; k->tile_size = tile_size; k->tile_w = tile_w; k->tile_h = tile_h;
         k->channels = channels; k->K = K; k->D = D; k->sh_degree = sh_degree; k->packed = packed; k->per_camera = per_camera;
         k->depth = depth; k->expected = expected; k->absgrad = absgrad; k->eps2d = eps2d; k->n_isects = n_isects;
+        k->color_sizes = color_sizes;
         return k;
     }
 };
@@ -543,8 +552,10 @@ struct CameraProjectionNode : torch::autograd::Function<CameraProjectionNode> {
                                  const Tensor &opacities, const OptTensor &colors, const OptTensor &velocities, const Tensor &viewmats,
                                  const Tensor &Ks, const Tensor &lin, const Tensor &ang, const Tensor &rs,
                                  c10::intrusive_ptr<CameraFrame> f) {
-        ctx->save_for_backward({means, quats, scales, opacities, colors.value_or(Tensor()), velocities.value_or(Tensor()), viewmats, Ks, lin, ang, rs, f->conics, f->comps,
-                                f->radii, f->camera_ids, f->gaussian_ids, f->campos});
+        ctx->save_for_backward({means, quats, scales, kept_opacities(opacities, f->comps, f->packed || f->C > 1),
+                                f->sh_degree >= 0 ? colors.value_or(Tensor()) : Tensor(), velocities.value_or(Tensor()), viewmats, Ks, lin,
+                                ang, rs, f->conics, f->comps, f->radii, f->camera_ids, f->gaussian_ids, f->campos});
+        if (colors) f->color_sizes = colors->sizes().vec();
         keep_state(ctx, f->sizes());
         ctx->set_materialize_grads(false);
         variable_list out{f->means2d, f->depths, f->conics, f->pix_vels};
@@ -585,8 +596,8 @@ struct CameraProjectionNode : torch::autograd::Function<CameraProjectionNode> {
             zeros.add(v_quats, quats.sizes());
             zeros.add(v_scales, scales.sizes());
         }
-        if (v_rows_o.defined()) zeros.add(v_opacities, opacities.sizes());
-        if (v_rows_c.defined() && ctx->needs_input_grad(4)) zeros.add(v_colors, colors.sizes());
+        if (v_rows_o.defined()) zeros.add(v_opacities, {f->N});
+        if (v_rows_c.defined() && ctx->needs_input_grad(4)) zeros.add(v_colors, f->color_sizes);
         zeros.make(options);
         if (comps.defined()) v_comps = v_rows_o.defined() ? at::empty_like(comps) : at::zeros_like(comps);
         if (v_rows_o.defined())

@@ -110,7 +110,7 @@ extern "C" int splatad_opacity_rows_bwd(uint32_t n, uint32_t N, const int64_t *g
                                         const float *compensations, const float *v_rows, float *v_opacities,
                                         float *v_compensations, void *stream) {
     if (n == 0 || (!v_opacities && !v_compensations)) return SPLATAD_OK;
-    SPL_REQUIRE(N > 0 && opacities && v_rows, SPLATAD_ERR_BAD_ARG, "opacity_rows_bwd: null argument");
+    SPL_REQUIRE(N > 0 && (opacities || !v_compensations) && v_rows, SPLATAD_ERR_BAD_ARG, "opacity_rows_bwd: null argument");
     SPL_PROF("opacity_rows_bwd_kernel", (cudaStream_t)stream);
     launch_chained(opacity_rows_bwd_kernel, div_up(n, kThreads), kThreads, 0, (cudaStream_t)stream,
         n, N, gaussian_ids, opacities, compensations, v_rows, v_opacities, v_compensations);

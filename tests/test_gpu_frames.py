@@ -62,3 +62,25 @@ def test_a_tensor_without_a_gradient_of_its_own_keeps_the_frame_in_the_graph(kin
         assert images[0].requires_grad
         images[0].sum().backward()
         assert g[name].grad is None
+
+
+@pytest.mark.parametrize("rasterize_mode", ["classic", "antialiased"])
+@pytest.mark.parametrize("name", ["opacities", "colors"])
+def test_what_the_ops_gather_may_be_edited_before_the_backward_pass(name, rasterize_mode):
+    import splatad_b200
+    from splatad_b200 import scenes
+    g = _to_gpu(scenes.config1(N=20_011))
+    g.update(sh_degree=None, colors=torch.rand(20_011, 3, device=DEV), rasterize_mode=rasterize_mode)
+    _forget()
+    grads = []
+    for edit in (False, False, True):        # by the ops, by the native frame, and edited behind its back
+        leaves = {k: g[k].clone().requires_grad_(True) for k in ("means", "scales")}
+        values = g[name].clone()
+        image, alphas, _ = splatad_b200.rasterization(**{**g, **leaves, name: values})
+        if edit:
+            values.mul_(0.5)
+        (image.square().mean() + alphas.mean()).backward()
+        grads.append([v.grad for v in leaves.values()])
+    for a, b, c in zip(*grads):              # sums in another order (atomics): 1e-4 from run to run
+        assert float((b - a).norm()) <= 5e-4 * float(a.norm())
+        assert float((c - a).norm()) <= 5e-4 * float(a.norm())
