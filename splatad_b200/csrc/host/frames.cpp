@@ -79,9 +79,11 @@ float *M(const Tensor &t) { return t.defined() && t.numel() ? t.data_ptr<float>(
 int32_t *I(const Tensor &t) { return t.defined() && t.numel() ? t.data_ptr<int32_t>() : nullptr; }
 int64_t *L(const Tensor &t) { return t.defined() && t.numel() ? t.data_ptr<int64_t>() : nullptr; }
 
-// float32, dense, contiguous, on GPU `dev`: what the kernels read without a conversion
+// float32, dense, contiguous, on GPU `dev`: what the kernels read without a conversion. Not a tensor that stands for
+// another - a dual number of forward-mode differentiation, whose tangent would be lost, or a transform's wrapper:
+// the ops say what they say to those.
 bool plain(const Tensor &t, c10::DeviceIndex dev) {
-    return t.defined() && t.is_cuda() && t.get_device() == dev && t.scalar_type() == at::kFloat && t.layout() == at::kStrided &&
+    return t.defined() && t.has_storage() && !t.unsafeGetTensorImpl()->is_python_dispatch() && !t._fw_grad(0).defined() && t.is_cuda() && t.get_device() == dev && t.scalar_type() == at::kFloat && t.layout() == at::kStrided &&
            t.is_contiguous() && !t.is_conj() && !t.is_neg();
 }
 bool plain(const OptTensor &t, c10::DeviceIndex dev) { return !t || plain(*t, dev); }

@@ -84,3 +84,20 @@ def test_what_the_ops_gather_may_be_edited_before_the_backward_pass(name, raster
     for a, b, c in zip(*grads):              # sums in another order (atomics): 1e-4 from run to run
         assert float((b - a).norm()) <= 5e-4 * float(a.norm())
         assert float((c - a).norm()) <= 5e-4 * float(a.norm())
+
+
+@pytest.mark.parametrize("kind", ["lidar", "camera"])
+def test_forward_mode_and_transforms_are_refused_as_by_the_ops(kind):
+    import splatad_b200
+    import torch.autograd.forward_ad as forward_ad
+    from splatad_b200 import scenes
+    g = _to_gpu(scenes.config2(N=20_011) if kind == "lidar" else scenes.config1(N=20_011))
+    render = splatad_b200.lidar_rasterization if kind == "lidar" else splatad_b200.rasterization
+    _forget()
+    render(**g)                              # from here on frames of this shape are native ones
+    with forward_ad.dual_level():
+        dual = forward_ad.make_dual(g["means"], torch.ones_like(g["means"]))
+        with pytest.raises(NotImplementedError):
+            render(**dict(g, means=dual))
+    with pytest.raises(RuntimeError, match="setup_context"):
+        torch.func.grad(lambda means: render(**dict(g, means=means))[0].sum())(g["means"])
