@@ -152,6 +152,7 @@ Tensor cotangent(const Tensor &g, const Tensor &like) {
 using StreamKey = std::pair<int, cudaStream_t>;
 std::map<std::pair<std::string, StreamKey>, Tensor> workspaces;
 std::map<StreamKey, std::vector<Tensor>> free_slots;
+std::map<StreamKey, Tensor> still;
 
 Tensor workspace(const char *tag, size_t bytes, c10::cuda::CUDAStream stream) {
     Tensor &t = workspaces[{tag, {stream.device_index(), stream.stream()}}];
@@ -203,16 +204,14 @@ bool wait_for(volatile int64_t *word, int64_t value, c10::cuda::CUDAStream strea
 void release() {
     workspaces.clear();
     free_slots.clear();
+    still.clear();
 }
 
-// Motion of a sensor that stands still.
-Tensor zero_motion(int64_t C, const at::TensorOptions &options) {
-    static std::map<int, Tensor> cache;
-    Tensor &t = cache[options.device().index()];
-    if (!t.defined() || t.numel() < 3 * C) {
-        t = at::zeros({std::max<int64_t>(3 * C, 64)}, options);
-        c10::cuda::getCurrentCUDAStream(options.device().index()).synchronize();   // any stream may read it from here on
-    }
+// Motion of a sensor that stands still. Per stream, like the workspaces: what replaces a smaller one, or a release,
+// gives the memory back to the stream whose kernels read it.
+Tensor zero_motion(int64_t C, const at::TensorOptions &options, c10::cuda::CUDAStream stream) {
+    Tensor &t = still[{stream.device_index(), stream.stream()}];
+    if (!t.defined() || t.numel() < 3 * C) t = at::zeros({std::max<int64_t>(3 * C, 64)}, options);
     return t;
 }
 
@@ -437,8 +436,8 @@ py::object lidar_frame(const Tensor &means, const Tensor &quats, const Tensor &s
     const auto ints = options.dtype(at::kInt);
     auto f = c10::make_intrusive<LidarFrame>();
     Counts counts;
-    const Tensor still = zero_motion(C, options);
-    const Tensor lin_t = lin ? *lin : alias(still, {C, 3}), ang_t = ang ? *ang : alias(still, {C, 3}), rs_t = rs ? *rs : alias(still, {C});
+    const Tensor zeros = zero_motion(C, options, stream);
+    const Tensor lin_t = lin ? *lin : alias(zeros, {C, 3}), ang_t = ang ? *ang : alias(zeros, {C, 3}), rs_t = rs ? *rs : alias(zeros, {C});
     {
         const at::NoGradGuard no_grad;
         f->C = C; f->N = N; f->W = W; f->H = H; f->rows = rows; f->cols = cols; f->D = D;
@@ -721,8 +720,8 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
     const auto stream = c10::cuda::getCurrentCUDAStream();
     const auto options = at::TensorOptions().dtype(at::kFloat).device(at::kCUDA, dev);
     const auto ints = options.dtype(at::kInt), longs = options.dtype(at::kLong);
-    const Tensor still = zero_motion(C, options);
-    const Tensor lin_t = lin ? *lin : alias(still, {C, 3}), ang_t = ang ? *ang : alias(still, {C, 3}), rs_t = rs ? *rs : alias(still, {C});
+    const Tensor zeros = zero_motion(C, options, stream);
+    const Tensor lin_t = lin ? *lin : alias(zeros, {C, 3}), ang_t = ang ? *ang : alias(zeros, {C, 3}), rs_t = rs ? *rs : alias(zeros, {C});
     auto f = c10::make_intrusive<CameraFrame>();
     const int64_t tile_w = (W + tile_size - 1) / tile_size, tile_h = (H + tile_size - 1) / tile_size;
     f->C = C; f->N = N; f->n = rows_max; f->W = W; f->H = H; f->tile_size = tile_size; f->tile_w = tile_w; f->tile_h = tile_h;

@@ -101,3 +101,29 @@ def test_forward_mode_and_transforms_are_refused_as_by_the_ops(kind):
             render(**dict(g, means=dual))
     with pytest.raises(RuntimeError, match="setup_context"):
         torch.func.grad(lambda means: render(**dict(g, means=means))[0].sum())(g["means"])
+
+
+def test_sensors_that_stand_still_on_several_streams():
+    """More sensors on a second stream while frames of the first are in flight, a release in between: the zeros
+    a frame reads are its stream's own."""
+    import splatad_b200
+    from splatad_b200 import _lib, scenes
+    g = _to_gpu(scenes.config1(N=20_011))
+    for k in ("linear_velocity", "angular_velocity", "rolling_shutter_time"):
+        g[k] = None
+    many = dict(g, viewmats=g["viewmats"].repeat(30, 1, 1), Ks=g["Ks"].repeat(30, 1, 1), width=160, height=90)
+    _forget()
+    want, want_many = splatad_b200.rasterization(**g)[0], splatad_b200.rasterization(**many)[0]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for i in range(6):
+        frames = []
+        for stream in streams:
+            with torch.cuda.stream(stream):
+                frames.append((splatad_b200.rasterization(**g)[0], splatad_b200.rasterization(**many)[0]))
+                torch.full((4096,), 7.0, device=DEV)     # takes whatever memory has been given back
+        torch.cuda.synchronize()
+        for one, rig in frames:
+            assert torch.equal(one, want) and torch.equal(rig, want_many)
+        if i == 2:
+            _lib.release_workspaces()
