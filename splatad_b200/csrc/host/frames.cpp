@@ -193,11 +193,24 @@ int64_t next_sequence() {
     return ++sequence;
 }
 
+// One turn of a polling loop.
+inline void pause() {
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#elif defined(__aarch64__)
+    asm volatile("yield" ::: "memory");
+#endif
+}
+
+// A word that a kernel stores; what it stored before (with a fence in between) may be read behind this.
+inline int64_t load_word(volatile int64_t *word) { return __atomic_load_n(const_cast<int64_t *>(word), __ATOMIC_ACQUIRE); }
+
 // Waits until *word == value; false when the stream has drained without that.
 bool wait_for(volatile int64_t *word, int64_t value, c10::cuda::CUDAStream stream) {
     for (uint32_t i = 0;; ++i) {
-        if (*word == value) return true;
-        if ((i & 4095u) == 4095u && stream.query()) return *word == value;
+        if (load_word(word) == value) return true;
+        if ((i & 4095u) == 4095u && stream.query()) return load_word(word) == value;
+        pause();
     }
 }
 
@@ -816,9 +829,9 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
         counts = read_counts(slot, sequence, stream);
         if (packed) {
             // behind the lists' count in the stream, so the rows' has arrived (or its store is about to)
-            for (uint32_t i = 0; (nnz = slot.word[8]) < 0; ++i)
+            for (uint32_t i = 0; (nnz = load_word(slot.word + 8)) < 0; ++i, pause())
                 if ((i & 4095u) == 4095u && stream.query()) break;
-            nnz = slot.word[8];
+            nnz = load_word(slot.word + 8);
         }
     }
     if (nnz <= 0 || nnz > rows_max || !usable(counts, capacity))
