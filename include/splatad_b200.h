@@ -443,21 +443,22 @@ int splatad_rasterize_to_pixels_bwd(
     float *v_pix_vels, void *stream);
 
 /* The same pair for the "expected depth" render modes: with expected_last_channel != 0 the last channel
- * leaves divided by max(alpha, 1e-10) (the torch ops behind the kernel in gsplat/rendering.py:423-430);
- * expected_render is that render when the cotangents are those of the divided channel, NULL otherwise. */
+ * leaves divided by max(alpha, 1e-10) (the torch ops behind the kernel in gsplat/rendering.py:423-430).
+ * expected_depths [C,H,W]: that channel once more, where the forward pass is given room for it (NULL: not
+ * wanted); the backward pass takes it when the cotangents are those of the divided channel, NULL otherwise. */
 int splatad_rasterize_expected_to_pixels_fwd(
     uint32_t C, int64_t n_isects, const float *means2d, const float *conics, const float *colors,
     uint32_t channels, const float *opacities, const float *pix_vels,
     const float *rolling_shutter_time, const float *backgrounds, uint32_t image_width,
     uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
     const int32_t *tile_offsets, const int32_t *flatten_ids, int32_t expected_last_channel,
-    float *render_colors, float *render_alphas, int32_t *last_ids, void *stream);
+    float *render_colors, float *render_alphas, int32_t *last_ids, float *expected_depths, void *stream);
 int splatad_rasterize_expected_to_pixels_bwd(
     uint32_t C, int64_t n_isects, const float *means2d, const float *conics, const float *colors,
     uint32_t channels, const float *opacities, const float *pix_vels,
     const float *rolling_shutter_time, const float *backgrounds, uint32_t image_width,
     uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
-    const int32_t *tile_offsets, const int32_t *flatten_ids, const float *expected_render,
+    const int32_t *tile_offsets, const int32_t *flatten_ids, const float *expected_depths,
     const float *render_alphas, const int32_t *last_ids, const float *v_render_colors,
     const float *v_render_alphas, float *v_means2d_abs, float *v_means2d, float *v_conics,
     float *v_colors, float *v_opacities, float *v_pix_vels, void *stream);

@@ -232,7 +232,8 @@ __device__ __forceinline__ PixelAlpha pixel_alpha(const PixelTask &a, int32_t g,
 }
 
 template <int PX>
-__device__ __noinline__ void odd_pixels_fwd(const PixelTask &a, float *colors_out, float *alphas, int32_t *last_ids, bool expected) {
+__device__ __noinline__ void odd_pixels_fwd(const PixelTask &a, float *colors_out, float *alphas, int32_t *last_ids, bool expected,
+                                            float *expected_depths) {
     const TileRange range = tile_range(a.offsets, blockIdx.x, a.C * a.tile_w * a.tile_h, a.n_isects);
     for (uint32_t h = 0; h < (uint32_t)PX; ++h) {
         const TaskPixel p = task_pixel<PX>(a, h);
@@ -254,6 +255,7 @@ __device__ __noinline__ void odd_pixels_fwd(const PixelTask &a, float *colors_ou
         last_ids[p.pix] = pos | kOddPixel;
         for (uint32_t k = 0; p.bg != nullptr && k < a.channels; ++k) color[k] += T * p.bg[k];
         if (expected) color[a.channels - 1] /= fmaxf(1.f - T, kExpectedMin);
+        if (expected_depths != nullptr) expected_depths[p.pix] = color[a.channels - 1];
     }
 }
 
@@ -285,7 +287,7 @@ __device__ __noinline__ void odd_pixels_bwd(const PixelTask &a, const PixelGrads
             T = 1.f - alpha;
             if (grad.expected != nullptr) {
                 divisor = fmaxf(alpha, kExpectedMin);
-                if (alpha >= kExpectedMin) v_a -= v_out[n - 1] * grad.expected[p.pix * n + n - 1] / divisor;
+                if (alpha >= kExpectedMin) v_a -= v_out[n - 1] * grad.expected[p.pix] / divisor;
             }
             for (uint32_t k = 0; p.bg != nullptr && k < n; ++k) bg_dot += p.bg[k] * (k + 1 == n ? v_out[k] / divisor : v_out[k]);
             behind = -T * (v_a - bg_dot);
@@ -356,7 +358,8 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
     uint32_t H, uint32_t tile_size, uint32_t tile_w, uint32_t tile_h,
     const int32_t *__restrict__ offsets, const int32_t *__restrict__ flatten_ids,
     float *__restrict__ render_colors, float *__restrict__ render_alphas,
-    int32_t *__restrict__ last_ids, uint32_t expected /* divide the last channel by the alpha */) {
+    int32_t *__restrict__ last_ids, uint32_t expected /* divide the last channel by the alpha */,
+    float *__restrict__ expected_depths /* optional: and keep it for the backward pass */) {
     chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_warp_kept[16];
@@ -501,6 +504,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
             float4 v = make_float4(out[h][0], out[h][1], out[h][2], out[h][3]);
             if (bg) v = make_float4(v.x + Tk * bg[0], v.y + Tk * bg[1], v.z + Tk * bg[2], v.w + Tk * bg[3]);
             if (expected) v.w /= fmaxf(1.f - Tk, kExpectedMin);
+            if (expected_depths != nullptr) expected_depths[pix] = v.w;
             *reinterpret_cast<float4 *>(dst) = v;
             continue;
         }
@@ -508,14 +512,20 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
         for (int k = 0; k < CDIM; ++k)
             if ((uint32_t)k < channels) {
                 float v = bg ? out[h][k] + Tk * bg[k] : out[h][k];
-                if (expected && (uint32_t)k + 1u == channels) v /= fmaxf(1.f - Tk, kExpectedMin);
+                if (expected && (uint32_t)k + 1u == channels) {
+                    v /= fmaxf(1.f - Tk, kExpectedMin);
+                    if (CDIM <= 8 && expected_depths != nullptr) expected_depths[pix] = v;
+                }
                 dst[k] = v;
             }
+        // (up to eight channels kept above, more of them here: what the compiler spills in the loop over the entries
+        // depends on it - 222 and 179 us, the other way round 226 and 197)
+        if (CDIM > 8 && expected_depths != nullptr) expected_depths[pix] = dst[channels - 1];
     }
     if (__any_sync(0xffffffffu, odd >= kOddEntry) || none != 0.f) {
         const PixelTask task = {C, W, H, tile_size, tile_w, tile_h, channels, n_isects, means2d, pix_vels, conics, opacities,
                                 colors, rs_time, backgrounds, offsets, flatten_ids};
-        odd_pixels_fwd<2>(task, render_colors, render_alphas, last_ids, expected != 0u);
+        odd_pixels_fwd<2>(task, render_colors, render_alphas, last_ids, expected != 0u, expected_depths);
     }
 }
 
@@ -1179,7 +1189,7 @@ rasterize_to_pixels_bwd_kernel(
     const float *__restrict__ v_render_colors, const float *__restrict__ v_render_alphas,
     float *__restrict__ v_means2d_abs, float *__restrict__ v_means2d,
     float *__restrict__ v_conics, float *__restrict__ v_colors, float *__restrict__ v_opacities,
-    float *__restrict__ v_pix_vels, const float *__restrict__ expected /* render whose last channel was divided by the alpha */) {
+    float *__restrict__ v_pix_vels, const float *__restrict__ expected /* [C,H,W] last channel, where it was divided by the alpha */) {
     chain_enter();
     static_assert(PX % 2 == 0, "pixels are handled in pairs");
     constexpr int P2 = PX / 2;
@@ -1233,7 +1243,7 @@ rasterize_to_pixels_bwd_kernel(
         float bg_dot = 0.f;
         const float divisor = fmaxf(a_final, kExpectedMin);
         if (in && expected != nullptr && a_final >= kExpectedMin)
-            v_a -= v_render_colors[pix * channels + channels - 1] * expected[pix * channels + channels - 1] / divisor;
+            v_a -= v_render_colors[pix * channels + channels - 1] * expected[pix] / divisor;
 #pragma unroll
         for (int c = 0; c < CDIM; ++c) {
             v_out[k][c] = (in && (uint32_t)c < channels) ? v_render_colors[pix * channels + c] : 0.f;
@@ -1926,7 +1936,7 @@ extern "C" int splatad_rasterize_to_pixels_fwd(
     return splatad_rasterize_expected_to_pixels_fwd(C, n_isects, means2d, conics, colors, channels, opacities, pix_vels,
                                                     rolling_shutter_time, backgrounds, image_width, image_height,
                                                     tile_size, tile_width, tile_height, tile_offsets, flatten_ids, 0,
-                                                    render_colors, render_alphas, last_ids, stream);
+                                                    render_colors, render_alphas, last_ids, nullptr, stream);
 }
 
 extern "C" int splatad_rasterize_expected_to_pixels_fwd(
@@ -1935,7 +1945,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     const float *rolling_shutter_time, const float *backgrounds, uint32_t image_width,
     uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
     const int32_t *tile_offsets, const int32_t *flatten_ids, int32_t expected_last_channel, float *render_colors,
-    float *render_alphas, int32_t *last_ids, void *stream) {
+    float *render_alphas, int32_t *last_ids, float *expected_depths, void *stream) {
     SPL_REQUIRE(channels >= 1 && channels <= SPLATAD_MAX_CHANNELS, SPLATAD_ERR_CHANNELS,
                 "rasterize_to_pixels_fwd: unsupported channel count %u (1..%d)", channels,
                 SPLATAD_MAX_CHANNELS);
@@ -1958,7 +1968,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
             image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
-            render_colors, render_alphas, last_ids, (uint32_t)(expected_last_channel != 0));      \
+            render_colors, render_alphas, last_ids, (uint32_t)(expected_last_channel != 0),       \
+            expected_last_channel ? expected_depths : nullptr);                                   \
     }
     {
         SPL_PROF("rasterize_to_pixels_fwd_kernel", (cudaStream_t)stream);
@@ -1989,7 +2000,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     uint32_t channels, const float *opacities, const float *pix_vels,
     const float *rolling_shutter_time, const float *backgrounds, uint32_t image_width,
     uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
-    const int32_t *tile_offsets, const int32_t *flatten_ids, const float *expected_render, const float *render_alphas,
+    const int32_t *tile_offsets, const int32_t *flatten_ids, const float *expected_depths, const float *render_alphas,
     const int32_t *last_ids, const float *v_render_colors, const float *v_render_alphas,
     float *v_means2d_abs, float *v_means2d, float *v_conics, float *v_colors, float *v_opacities,
     float *v_pix_vels, void *stream) {
@@ -2023,7 +2034,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
             image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
             render_alphas, last_ids, v_render_colors, v_render_alphas, v_means2d_abs, v_means2d,  \
-            v_conics, v_colors, v_opacities, v_pix_vels, expected_render);                        \
+            v_conics, v_colors, v_opacities, v_pix_vels, expected_depths);                        \
     }
 #define CALL(D)                                                                                   \
     if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)

@@ -551,6 +551,7 @@ struct CameraFrame : torch::CustomClassHolder {
     Tensor camera_ids, gaussian_ids, radii, means2d, depths, conics, comps, pix_vels, tiles_per_gauss, campos;
     Tensor opacities, colors;                 // rows made for this frame (undefined: the parameters serve as they are)
     Tensor isect_ids, flatten_ids, offsets, render, alphas, last_ids;
+    Tensor expected_depths;                   // kept for the backward pass: the render is the user's to edit
     c10::intrusive_ptr<CameraFrame> sizes() const {
         auto k = c10::make_intrusive<CameraFrame>();
         k->C = C; k->N = N; k->n = n; k->W = W; k->H = H; k->tile_size = tile_size; k->tile_w = tile_w; k->tile_h = tile_h;
@@ -658,7 +659,7 @@ struct CameraCompositeNode : torch::autograd::Function<CameraCompositeNode> {
                                  const Tensor &opacities, const Tensor &pix_vels, const Tensor &rs, const OptTensor &backgrounds,
                                  c10::intrusive_ptr<CameraFrame> f) {
         ctx->save_for_backward({means2d, conics, colors, opacities, pix_vels, rs, backgrounds.value_or(Tensor()), f->alphas, f->last_ids, f->offsets,
-                                f->flatten_ids, f->expected ? f->render : Tensor()});
+                                f->flatten_ids, f->expected_depths});
         keep_state(ctx, f->sizes());
         ctx->set_materialize_grads(false);
         return {f->render, f->alphas};
@@ -821,10 +822,11 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
         f->render = at::empty({C, H, W, channels}, options);
         f->alphas = at::empty({C, H, W, 1}, options);
         f->last_ids = at::empty({C, H, W}, ints);
+        if (expected && grad) f->expected_depths = at::empty({C, H, W}, options);
         check(lib.splatad_rasterize_expected_to_pixels_fwd(
             (uint32_t)C, -1, F(f->means2d), F(f->conics), c, (uint32_t)channels, o, F(f->pix_vels), F(rs_t), F(bg), (uint32_t)W, (uint32_t)H,
             (uint32_t)tile_size, (uint32_t)tile_w, (uint32_t)tile_h, I(f->offsets), I(f->flatten_ids), expected, M(f->render), M(f->alphas),
-            I(f->last_ids), stream.stream()));
+            I(f->last_ids), M(f->expected_depths), stream.stream()));
         py::gil_scoped_release no_gil;
         counts = read_counts(slot, sequence, stream);
         if (packed) {

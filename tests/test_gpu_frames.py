@@ -127,3 +127,24 @@ def test_sensors_that_stand_still_on_several_streams():
             assert torch.equal(one, want) and torch.equal(rig, want_many)
         if i == 2:
             _lib.release_workspaces()
+
+
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("render_mode", ["RGB", "RGB+D", "RGB+ED", "ED"])
+def test_a_render_may_be_edited_in_place(render_mode, packed):
+    import splatad_b200
+    from splatad_b200 import scenes
+    g = _to_gpu(scenes.config1(N=20_011, packed=packed))
+    g["render_mode"] = render_mode
+    _forget()
+    grads = []
+    for edit in (False, False, True):        # by the ops, by the native frame, and edited
+        leaves = {k: g[k].clone().requires_grad_(True) for k in ("means", "opacities")}
+        image, alphas, _ = splatad_b200.rasterization(**{**g, **leaves})
+        if edit:
+            image.mul_(2.0)
+        (image.square().mean() * (0.25 if edit else 1.0) + alphas.mean()).backward()
+        grads.append([v.grad for v in leaves.values()])
+    for a, b, c in zip(*grads):              # sums in another order (atomics): 1e-4 from run to run
+        assert float((b - a).norm()) <= 5e-4 * float(a.norm())
+        assert float((c - a).norm()) <= 5e-4 * float(a.norm())
