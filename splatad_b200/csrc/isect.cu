@@ -12,8 +12,8 @@
 // buckets - at most C*N 8-byte pairs, L2 resident - and splitting their rectangles stably by blocks of
 // tiles and then by tile (the block split below). Offsets fall out of the split.
 //
-// Grids beyond the block split's tables and depths too crowded for the buckets take the radix split: the
-// elements ordered by depth alone, (sensor*n_tiles + tile, flatten index) pairs emitted in that order,
+// Depths too crowded for the buckets are ordered by radix passes and then grouped by sensor, for the same split.
+// Grids beyond the block split's tables take the radix split: the elements ordered by depth alone, (sensor*n_tiles + tile, flatten index) pairs emitted in that order,
 // and a stable radix split of those 8-byte pairs by the compact tile key (ceil(bits/8) passes), the last
 // pass writing the 64-bit isect_ids and int32 flatten_ids directly; offsets by a binary search per tile.
 //
@@ -765,6 +765,71 @@ depth_bucket_rank_kernel(BucketLayout layout, uint32_t n_buckets, const int64_t 
         } else {
             order[lo + rank] = val;
         }
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// The block split's input from a depth order of radix passes: the entries of all sensors lie in one sequence by
+// depth, so with several sensors further passes - stable, by the sensor - group them, and the sorted sensors say where
+// each one's begin. Without this, crowded depths had to take the radix split over (tile, entry) pairs: a
+// million Gaussians, fifty of them seven kilometres away, 591 us a lidar frame and 332 with it.
+// ---------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(kThreads)
+entry_sensors_kernel(BucketLayout layout, const int64_t *__restrict__ n_entries, const uint32_t *__restrict__ order,
+                     uint32_t *__restrict__ keys) {
+    chain_enter();
+    const uint32_t n = (uint32_t)*n_entries;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) keys[i] = layout.group(order[i]);
+}
+
+// First entry and first chunk of every group; `keys` ascending (not looked at for one group). One block.
+__global__ void __launch_bounds__(1024)
+group_starts_kernel(const int64_t *__restrict__ n_entries, const uint32_t *__restrict__ keys, uint32_t groups, uint32_t chunk,
+                    uint32_t *__restrict__ group_start, uint32_t *__restrict__ group_chunk /* both [groups + 1] */) {
+    chain_enter();
+    __shared__ uint32_t wt[33];
+    const uint32_t n = (uint32_t)*n_entries;
+    const auto first_of = [&](uint32_t g) {
+        if (g == 0u) return 0u;
+        uint32_t lo = 0, hi = n;
+        while (lo < hi && g < groups) {
+            const uint32_t m = (lo + hi) >> 1;
+            if (keys[m] < g) lo = m + 1; else hi = m;
+        }
+        return g < groups ? lo : n;
+    };
+    uint32_t chunks = 0;
+    for (uint32_t g0 = 0; g0 < groups; g0 += 1024) {
+        const uint32_t g = g0 + threadIdx.x;
+        uint32_t lo = 0, mine = 0;
+        if (g < groups) {
+            lo = first_of(g);
+            mine = (first_of(g + 1) - lo + chunk - 1) / chunk;
+        }
+        uint32_t round;
+        const uint32_t ex = block_excl_scan(mine, wt, round);
+        if (g < groups) {
+            group_start[g] = lo;
+            group_chunk[g] = chunks + ex;
+        }
+        chunks += round;
+    }
+    if (threadIdx.x == 0) {
+        group_start[groups] = n;
+        group_chunk[groups] = chunks;
+    }
+}
+
+__global__ void __launch_bounds__(kThreads)
+gather_entries_kernel(const int64_t *__restrict__ n_entries, const uint32_t *__restrict__ order,
+                      const uint32_t *__restrict__ depth_bits, const uint2 *__restrict__ rect,
+                      uint2 *__restrict__ sorted_pair /* {depth bits, flatten index} */, uint2 *__restrict__ sorted_rect) {
+    chain_enter();
+    const uint32_t n = (uint32_t)*n_entries;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t v = order[i];
+        sorted_pair[i] = make_uint2(__ldg(depth_bits + v), v);
+        sorted_rect[i] = __ldg(rect + v);
     }
 }
 
@@ -1722,11 +1787,10 @@ struct IsectGeom {
     const uint32_t *depth_bits;
 };
 
-// The block split applies to sorted output whose depth order is built by buckets, within the limits
-// of its tables (six 1920 x 1080 cameras have 1620 blocks, a 128-beam lidar 30); larger grids and the
-// radix depth order take the radix split.
+// The block split applies to sorted output within the limits of its tables (six 1920 x 1080 cameras have 1620
+// blocks, a 128-beam lidar 30); larger grids take the radix split.
 static bool use_blocks(const IsectGeom &g, int sort) {
-    if (sort != 1 || g.C > kBlkMaxSensors) return false;
+    if (sort == 0 || g.C > kBlkMaxSensors) return false;
     const uint64_t width = g.lidar ? g.lid.lidar.n_tiles_azim : g.cam.cam.tile_width, height = g.n_tiles / width;
     if (width > kBlkMaxExtent || height > kBlkMaxExtent) return false;
     const uint64_t bx = (width + kBlkW - 1) / kBlkW, blocks = bx * ((height + kBlkH - 1) / kBlkH);
@@ -1737,6 +1801,17 @@ static bool use_blocks(const IsectGeom &g, int sort) {
 static BucketLayout bucket_layout(const IsectGeom &g, bool grouped) {
     const uint32_t groups = grouped ? g.C : 1u;
     return BucketLayout{g.camera_ids, g.N, groups, depth_bucket_count(g.total) / groups};
+}
+
+// Radix passes of eight bits that group the depth order by sensor (sort = 2).
+static uint32_t sensor_passes(uint32_t C) { return C == 1 ? 0u : (bit_length(C - 1) + 7) / 8; }
+
+// Where the plan leaves the block split's {depth bits, flatten index} pairs. keyA and valA lie back to back, as do
+// keyB and valB (each g.total words, 256-byte aligned): either has room for g.total pairs. The radix order is in valB
+// after an even number of passes by sensor, in valA after an odd one; the pairs go to the other two.
+static uint2 *plan_pairs(const PlanWs &p, const IsectGeom &g, int sort) {
+    const bool second = sort == 1 || sensor_passes(g.C) % 2 == 1;
+    return reinterpret_cast<uint2 *>(second ? p.keyB : p.keyA);
 }
 
 // One-shot request of the calling thread's next plan (splatad_isect_set_early_count): where the
@@ -1815,10 +1890,9 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
     if (buckets) {
         // depth order of the visible (count > 0) elements by buckets; result in keyB / valB
         const uint32_t bgrid = div_up(g.total, kThreads);   // one element per thread: the atomics' latency needs the parallelism
-        // {bits, flatten index} pairs in bucket order: keyA and valA lie back to back in the workspace
-        // (each g.total words, 256-byte aligned), together room for g.total 8-byte pairs
+        // {bits, flatten index} pairs in bucket order, and in the end
         uint2 *pairs = reinterpret_cast<uint2 *>(p.keyA);
-        uint2 *sorted_pair = reinterpret_cast<uint2 *>(p.keyB);   // the same with keyB and valB
+        uint2 *sorted_pair = plan_pairs(p, g, sort);
         if (!ranged) {
             SPL_PROF("depth_bucket_count_kernel", st);
             launch_chained(depth_bucket_count_kernel, bgrid, kThreads, 0, st, g.depth_bits,
@@ -1894,6 +1968,48 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
         // pass0: gen->A ; pass1: A->B ; pass2: B->A ; pass3: A->B  => sorted order in valB
         e.order = va;
         e.n_order_ptr = p.counters + CNT_NVIS;
+        if (blocks) {
+            const uint32_t grid = min(div_up(g.total, kThreads), (uint32_t)(8 * kNumSMs));
+            const uint32_t passes = sensor_passes(g.C);
+            // ka / va hold the order (B), kb / vb are free
+            if (passes) {
+                SPL_PROF("entry_sensors_kernel", st);
+                launch_chained(entry_sensors_kernel, grid, kThreads, 0, st, layout, e.n_order_ptr, (const uint32_t *)va, kb);
+            }
+            for (uint32_t pass = 0; pass < passes; ++pass) {
+                // the keys lie apart from their values in the first pass: keys A, values B
+                PassSrc s{};
+                s.keys = pass == 0 ? kb : ka; s.vals = va; s.n_ptr = e.n_order_ptr;
+                uint32_t *out_keys = pass == 0 ? ka : kb, *out_vals = vb;
+                {
+                    SPL_PROF("sensorsort_upsweep", st);
+                    launch_chained(radix_upsweep_kernel<false>, kSortGrid, kSortThreads, 0, st, s, (int)(8 * pass), 0xffu, p.hist);
+                }
+                {
+                    SPL_PROF("sensorsort_rowscan", st);
+                    launch_chained(radix_rowscan_kernel, kRadixBins, ((kSortGrid + 31) / 32) * 32, 0, st,
+                                   p.hist, (uint32_t)kSortGrid, p.digit_totals);
+                }
+                {
+                    SPL_PROF("sensorsort_downsweep", st);
+                    launch_chained(radix_downsweep_kernel<false, false>, kSortGrid, kSortThreads, 0, st,
+                                   s, (int)(8 * pass), 8, 0xffu, p.hist, p.digit_totals, out_keys, out_vals, nofin, nullptr);
+                }
+                std::swap(va, vb);
+            }
+            // after one pass the sorted sensors are in B and the order in A, after two in A and B
+            const uint32_t *sensors = passes == 1 ? ka : kb;
+            {
+                SPL_PROF("group_starts_kernel", st);
+                launch_chained(group_starts_kernel, 1, 1024, 0, st, e.n_order_ptr, sensors, g.C, kBlkThreads, p.group_start,
+                               p.group_chunk);
+            }
+            {
+                SPL_PROF("gather_entries_kernel", st);
+                launch_chained(gather_entries_kernel, grid, kThreads, 0, st, e.n_order_ptr, (const uint32_t *)va, g.depth_bits,
+                               (const uint2 *)p.rect, plan_pairs(p, g, sort), p.sorted_rect);
+            }
+        }
     }
     if (!blocks) {
         {
@@ -1954,7 +2070,7 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
                     fill_workspace_bytes, w.bytes);
         BlkArgs a{};
         a.rect = p.sorted_rect;
-        a.pair = (const uint2 *)p.keyB;
+        a.pair = plan_pairs(p, g, sort);
         a.sensor_start = p.group_start;
         a.sensor_cta = p.group_chunk;
         a.counters = p.counters;

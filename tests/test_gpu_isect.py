@@ -315,3 +315,54 @@ def test_block_split_of_rectangles_around_the_turn(turns):
     want.append(isect.isect_offset_encode(want[1], C, n_az, len(eb) - 1))
     ops._depth_sort_mode.clear()
     _check(_run_lidar(means2d, radii, depths, eb, res, -180.0), want, f"{turns} turns")
+
+
+class _AlwaysRadix(dict):
+    """Every shape is taken for one whose depths are too crowded for the buckets."""
+
+    def get(self, key, default=None):
+        return 2
+
+
+@pytest.mark.parametrize("C,N,tw,th", [(1, 1, 1, 1), (1, 513, 3, 7), (2, 513, 5, 9), (3, 1500, 31, 17), (256, 40, 3, 9),
+                                       (257, 40, 9, 3), (600, 9, 2, 2)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_crowded_depths_take_the_block_split(C, N, tw, th, packed, monkeypatch):
+    """Behind the radix passes the entries are grouped by sensor - by none, one or two further passes - and split
+    as behind the buckets. Bit for bit the oracle's lists, by the same kernels."""
+    import ctypes
+    from oracle import isect
+    from splatad_b200 import _lib, ops
+    g = torch.Generator().manual_seed(C * 1000 + N)
+    ts = 16
+    m2 = (torch.rand(C, N, 2, generator=g) * 1.4 - 0.2) * torch.tensor([tw * ts, th * ts])
+    r2 = torch.randint(0, 60, (C, N, 2), generator=g, dtype=torch.int32)
+    depths = torch.rand(C, N, generator=g) * 50 + 0.1
+    depths[:, ::3] = depths[:, :1].clone()            # ties
+    if C > 2:
+        r2[1] = 0                                     # a sensor that sees nothing
+    monkeypatch.setattr(ops, "_depth_sort_mode", _AlwaysRadix())
+    lib = _lib.load()
+    keep = r2[..., 0] > 0
+    cam = torch.nonzero(keep)[:, 0]
+    lib.splatad_profile_enable(1)
+    try:
+        if packed:
+            want = isect.isect_tiles(n(m2[keep]), n(r2[keep]), n(depths[keep]), ts, tw, th, n_cameras=C, camera_ids=n(cam))
+            got = ops.isect_tiles(t(m2[keep]), t(r2[keep], torch.int32), t(depths[keep]), ts, tw, th, packed=True, n_cameras=C,
+                                  camera_ids=cam.to(DEV), gaussian_ids=torch.zeros_like(cam).to(DEV))
+        else:
+            want = isect.isect_tiles(n(m2), n(r2), n(depths), ts, tw, th)
+            got = ops.isect_tiles(t(m2), t(r2, torch.int32), t(depths), ts, tw, th)
+        torch.cuda.synchronize()
+        report = ctypes.create_string_buffer(1 << 16)
+        lib.splatad_profile_report(report, len(report))
+    finally:
+        lib.splatad_profile_enable(0)
+    for a, b, what in zip(got, want, ("tiles per Gaussian", "ids", "flatten ids")):
+        assert np.array_equal(n(a), b), what
+    offs = ops.isect_offset_encode(got[1], C, tw, th)
+    assert np.array_equal(n(offs), isect.isect_offset_encode(want[1], C, tw, th))
+    names = report.value.decode()
+    assert "depthsort_upsweep" in names and "tilesort_upsweep" not in names
+    assert ("tile_scatter_kernel" in names) == (got[1].numel() > 0)

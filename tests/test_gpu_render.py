@@ -415,8 +415,8 @@ def test_config2_full_size_properties():
     """The headline frame (1 M Gaussians, 15.3 M intersections) through properties that do not depend
     on size (the comparison with the CPU oracle at this size is ``test_gpu_full_size.py``) - and by
     building its tile lists twice,
-    with the two independent implementations the library has (row / column split for small tile
-    grids, radix split otherwise), which must agree bit for bit."""
+    with the two independent implementations the library has (block split, and radix split for more
+    blocks than its tables hold), which must agree bit for bit."""
     import splatad_b200
     from splatad_b200 import ops, scenes
     cfg = scenes.config2()
@@ -435,13 +435,13 @@ def test_config2_full_size_properties():
     assert torch.equal((ids & 0xFFFFFFFF).to(torch.int32), m["depths"].reshape(-1)[flat.long()].view(torch.int32))
     tile_of = torch.bucketize(torch.arange(n_isects, device=DEV), offs.reshape(-1).long(), right=True) - 1
     assert torch.equal(ids >> 32, tile_of)
-    # the same lists from the radix split: the packed layout with 64 (empty but one) sensors is
-    # outside the row / column split's reach, and sensor 0 leaves the ids unchanged
+    # the same lists from the radix split: the packed layout with 600 (empty but one) sensors of 30 blocks is
+    # outside the block split's reach, and sensor 0 leaves the ids unchanged
     N = cfg["means"].shape[0]
     zeros = torch.zeros(N, dtype=torch.int64, device=DEV)
     _, ids2, flat2 = ops.isect_lidar_tiles(
         m["means2d"][0], m["radii"][0], m["depths"][0], g["tile_elevation_boundaries"],
-        cfg["azimuth_resolution"] * cfg["tile_width"], cfg["min_azimuth"], packed=True, n_cameras=64,
+        cfg["azimuth_resolution"] * cfg["tile_width"], cfg["min_azimuth"], packed=True, n_cameras=600,
         camera_ids=zeros, gaussian_ids=torch.arange(N, device=DEV))
     assert torch.equal(ids2, ids) and torch.equal(flat2, flat)
     # render: repeatable, alphas in range
