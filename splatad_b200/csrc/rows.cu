@@ -43,10 +43,12 @@ __device__ __forceinline__ size_t color_row(uint32_t i, uint32_t N, const int64_
 // -> 10 us forward and backward; 500 k packed rows of 20: 24 -> 18 and 20 -> 8).
 constexpr uint32_t kColorRows = 64;
 
+static_assert(kColorRows == 64, "the bound on the width below");
+
 struct ByWidth {
-    uint32_t width, magic;   // ceil(2^32 / width): exact while element * width < 2^32; unused for 1
-    __host__ explicit ByWidth(uint32_t w) : width(w), magic(0xffffffffu / w + 1u) {}
-    __device__ __forceinline__ uint32_t row(uint32_t e) const { return width == 1u ? e : __umulhi(e, magic); }
+    uint32_t width, magic;   // ceil(2^32 / width): exact while element * width < 2^32; 0 for 1 and for wider rows
+    __host__ explicit ByWidth(uint32_t w) : width(w), magic(64ull * w * w < 1ull << 32 ? 0xffffffffu / w + 1u : 0u) {}
+    __device__ __forceinline__ uint32_t row(uint32_t e) const { return magic != 0u ? __umulhi(e, magic) : e / width; }
 };
 
 __global__ void __launch_bounds__(kThreads)

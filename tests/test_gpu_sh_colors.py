@@ -124,3 +124,27 @@ def test_camera_centers():
     want.backward(v)
     got.backward(v.float().to(DEV))
     np.testing.assert_allclose(n(got_in.grad), ref_in.grad.numpy(), rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("width", [1, 2, 14, 8191, 8192, 8193, 20_001])
+def test_color_rows_of_any_width(width):
+    """Rows are told apart by a multiplication while that is exact - 64 rows of up to 8191 channels a block - and
+    by a division beyond."""
+    from splatad_b200 import _lib
+    n, N = 130, 50
+    g = torch.Generator().manual_seed(width)
+    ids = torch.randint(0, N, (n,), generator=g).to(DEV)
+    D = width - 1
+    colors, depths = torch.randn(N, D, generator=g).to(DEV), torch.randn(n, generator=g).to(DEV)
+    rows = torch.empty(n, width, device=DEV)
+    stream = _lib.stream_ptr(rows.device)
+    _lib.call("splatad_color_rows_fwd", n, N, D, None, _lib.ptr(ids), 0, _lib.ptr(colors) if D else None, _lib.ptr(depths),
+              _lib.ptr(rows), stream)
+    assert torch.equal(rows, torch.cat([colors[ids], depths[:, None]], -1))
+    if D == 0:
+        return
+    v_rows, v_colors, v_depths = torch.randint(-4, 5, (n, width), generator=g).float().to(DEV), torch.zeros(N, D, device=DEV), torch.empty(n, device=DEV)
+    _lib.call("splatad_color_rows_bwd", n, N, D, width, None, _lib.ptr(ids), 0, _lib.ptr(v_rows), _lib.ptr(v_colors), None,
+              _lib.ptr(v_depths), stream)
+    # sums of small whole numbers: exact in any order
+    assert torch.equal(v_colors, torch.zeros_like(v_colors).index_add_(0, ids, v_rows[:, :D])) and torch.equal(v_depths, v_rows[:, D])
