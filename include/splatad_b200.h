@@ -632,6 +632,11 @@ int splatad_debug_validate_lists(int64_t n_isects, const int32_t *flatten_ids, u
                                  const int64_t *sensor_ids, const int64_t *gaussian_ids, uint64_t n_packed,
                                  uint32_t n_sensors, uint64_t n_gaussians, uint64_t *report, void *stream);
 
+/* Compares the reciprocals the backward compositing kernels work with (1 / (1 - alpha)) with CUDA's division, for every
+ * float whose bits lie in [first_bits, last_bits]: report[0] += differences, report[1] = max(., bits of one). Device
+ * memory, two uint64, zero-initialised. */
+int splatad_debug_check_reciprocals(uint32_t first_bits, uint32_t last_bits, uint64_t *report, void *stream);
+
 /* ------------------------------------------------------------------------------------------
  * Whole frame in one call
  * ---------------------------------------------------------------------------------------- */

@@ -1106,16 +1106,6 @@ __device__ __forceinline__ SumSlot sum_slot(uint32_t lane) {
     return r;
 }
 
-// 1 / x of two values in [0.001, 1]: one Newton-Raphson step on the hardware's approximation (which is off by
-// up to one unit in the last place) gives the correctly rounded quotient for every float in that range - all
-// 85 million of them compared - at half the instructions of a division.
-__device__ __forceinline__ float2 reciprocal_pair(float2 x) {
-    float2 r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
-    return __ffma2_rn(r, __ffma2_rn(make_float2(-x.x, -x.y), r, make_float2(1.f, 1.f)), r);
-}
-
 __device__ __forceinline__ int block_max_int(int v, int *red /* [32] */) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, off));

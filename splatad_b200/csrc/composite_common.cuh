@@ -51,6 +51,16 @@ struct BoxTest {
     }
 };
 
+// 1 / x of two values in [1 - kAlphaMax, 1]: one Newton-Raphson step on the hardware's approximation (which is off
+// by up to one unit in the last place) gives the correctly rounded quotient for every float in that range
+// (splatad_debug_check_reciprocals compares all 83.7 million of them) at half the instructions of a division.
+__device__ __forceinline__ float2 reciprocal_pair(float2 x) {
+    float2 r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
+    return __ffma2_rn(r, __ffma2_rn(make_float2(-x.x, -x.y), r, make_float2(1.f, 1.f)), r);
+}
+
 struct TileRange { int32_t start, end; };
 
 __device__ __forceinline__ TileRange tile_range(const int32_t *__restrict__ offsets, uint32_t tile,

@@ -4,6 +4,7 @@
 // faulting. The Python layer runs it, together with canary words behind every workspace, when
 // SPLATAD_DEBUG=1. No counterpart in the reference.
 #include "common.cuh"
+#include "composite_common.cuh"
 
 namespace splatad {
 
@@ -50,9 +51,30 @@ validate_lists_kernel(int64_t n_isects, const int32_t *__restrict__ flatten_ids,
     }
 }
 
+// report[0] += floats with bit patterns in [first, last] whose reciprocal_pair() is not CUDA's quotient;
+// report[1] = the largest such pattern.
+__global__ void __launch_bounds__(kThreads)
+check_reciprocals_kernel(uint32_t first, uint32_t last, unsigned long long *__restrict__ report) {
+    for (uint64_t b = first + (uint64_t)blockIdx.x * kThreads + threadIdx.x; b <= last; b += (uint64_t)gridDim.x * kThreads) {
+        const float x = __uint_as_float((uint32_t)b), want = __fdiv_rn(1.f, x);
+        const float2 got = reciprocal_pair(make_float2(x, x));
+        if (got.x != want || got.y != want) {
+            atomicAdd(report, 1ull);
+            atomicMax(report + 1, (unsigned long long)b);
+        }
+    }
+}
+
 } // namespace splatad
 
 using namespace splatad;
+
+extern "C" int splatad_debug_check_reciprocals(uint32_t first_bits, uint32_t last_bits, uint64_t *report, void *stream) {
+    SPL_REQUIRE(report != nullptr, SPLATAD_ERR_BAD_ARG, "debug_check_reciprocals: the report array is required");
+    if (last_bits < first_bits) return SPLATAD_OK;
+    check_reciprocals_kernel<<<kNumSMs * 8, kThreads, 0, (cudaStream_t)stream>>>(first_bits, last_bits, (unsigned long long *)report);
+    return check_launch("debug_check_reciprocals");
+}
 
 extern "C" int splatad_debug_validate_lists(int64_t n_isects, const int32_t *flatten_ids, uint64_t n_rows,
                                             const int32_t *tile_offsets, uint32_t n_tiles, int32_t total_follows,

@@ -9,6 +9,7 @@ import subprocess
 import sys
 
 import pytest
+import numpy as np
 import torch
 
 from gpu_util import DEV
@@ -112,3 +113,14 @@ def test_a_write_past_a_workspace_is_caught_by_its_canary():
     proc = _run(_OVERRUN)
     assert proc.returncode == 0, proc.stderr[-3000:]
     assert "caught:" in proc.stdout and "row_index_probe" in proc.stdout and "past its end" in proc.stdout, proc.stdout
+
+
+def test_reciprocals_of_the_backward_pass_are_correctly_rounded():
+    """Every value 1 - alpha can take, from the cap's 1 - 0.999f to 1."""
+    import struct
+    from splatad_b200 import _lib
+    bits = lambda v: struct.unpack("<I", struct.pack("<f", v))[0]   # noqa: E731
+    first = bits(float(np.float32(1.0) - np.float32(0.999)))
+    report = torch.zeros(2, dtype=torch.int64, device=DEV)
+    _lib.call("splatad_debug_check_reciprocals", first, bits(1.0), _lib.ptr(report), _lib.stream_ptr(report.device))
+    assert bits(1.0) - first + 1 == 83_684_865 and report.tolist() == [0, 0]
