@@ -148,3 +148,122 @@ def test_a_render_may_be_edited_in_place(render_mode, packed):
     for a, b, c in zip(*grads):              # sums in another order (atomics): 1e-4 from run to run
         assert float((b - a).norm()) <= 5e-4 * float(a.norm())
         assert float((c - a).norm()) <= 5e-4 * float(a.norm())
+
+
+def _twice(monkeypatch, name, render, kw, leaves, cotangents):
+    """Images, meta and gradients of one call by the ops and one that the native function took."""
+    from splatad_b200 import rendering
+    native = getattr(rendering, name)
+    taken = []
+    monkeypatch.setattr(rendering, name, lambda *a: taken.append(native(*a)) or taken[-1])
+    _forget()
+    out = []
+    for _ in range(2):
+        params = {k: kw[k].clone().requires_grad_(True) for k in leaves}
+        *images, meta = render(**{**kw, **params})
+        meta["means2d"].retain_grad()
+        given = [(i, w) for i, w in zip(images, cotangents(images)) if i is not None and w is not None]
+        torch.autograd.backward([i for i, _ in given], [w for _, w in given])
+        grads = {k: v.grad for k, v in params.items()}
+        grads["means2d"], grads["absgrad"] = meta["means2d"].grad, getattr(meta["means2d"], "absgrad", None)
+        out.append(([None if i is None else i.detach() for i in images], meta, grads))
+    assert taken[0] is None and taken[1] is not None
+    (images, meta, grads), (images2, meta2, grads2) = out
+    assert set(meta) == set(meta2)
+    for k, a in meta.items():
+        b = meta2[k]
+        if not isinstance(a, torch.Tensor):
+            assert a == b, k
+        elif a.dtype.is_floating_point:
+            assert a.shape == b.shape and torch.allclose(a, b, rtol=1e-6, atol=1e-6), k
+        else:
+            assert torch.equal(a, b), k
+    for a, b in zip(images, images2):
+        assert (a is None) == (b is None)
+        if a is not None:      # a product or a division in one kernel or two: a rounding
+            assert a.shape == b.shape and float((a - b).norm()) <= 1e-6 * float(a.norm())
+    for k, a in grads.items():
+        b = grads2[k]
+        assert (a is None) == (b is None), k
+        if a is not None:      # sums in another order (atomics): 1e-4 from run to run
+            assert a.shape == b.shape and float((a - b).norm()) <= 5e-4 * float(a.norm()), k
+
+
+def _all_of(images):
+    g = torch.Generator(device=DEV).manual_seed(1)
+    return [None if i is None else torch.randn(i.shape, generator=g, device=DEV) / i.numel() for i in images]
+
+
+@pytest.mark.parametrize("C,packed,colors,mode,options", [
+    (1, False, "plain", "RGB", {}),
+    (1, False, "plain", "RGB+D", dict(absgrad=True)),
+    (1, False, "plain", "RGB+ED", dict(rasterize_mode="antialiased")),
+    (1, False, "sh", "RGB+ED", dict(backgrounds=True)),
+    (1, False, "sh", "D", {}),
+    (1, False, "plain", "ED", dict(backgrounds=True)),
+    (1, True, "plain", "RGB", dict(backgrounds=True)),
+    (1, True, "plain", "RGB+ED", dict(absgrad=True)),
+    (1, True, "sh", "RGB+D", dict(rasterize_mode="antialiased", absgrad=True)),
+    (1, True, "sh", "ED", {}),
+    (3, False, "plain", "RGB", dict(absgrad=True)),
+    (3, False, "per camera", "RGB+D", dict(backgrounds=True)),
+    (3, False, "per camera sh", "RGB+ED", dict(rasterize_mode="antialiased")),
+    (3, True, "per camera", "RGB+ED", dict(backgrounds=True, rasterize_mode="antialiased")),
+    (3, True, "per camera sh", "RGB", {}),
+    (3, True, "sh", "RGB+ED", dict(absgrad=True, backgrounds=True)),
+])
+@pytest.mark.parametrize("cotangents", ["all", "image only", "alpha only"])
+def test_native_camera_frames_are_those_of_the_ops(C, packed, colors, mode, options, cotangents, monkeypatch):
+    import splatad_b200
+    from splatad_b200 import scenes
+    N = 8_009
+    kw = _to_gpu(scenes.config1(N=N, packed=packed))
+    g = torch.Generator(device=DEV).manual_seed(C)
+    rand = lambda *s: torch.rand(*s, generator=g, device=DEV)   # noqa: E731
+    kw.update(width=333, height=211, render_mode=mode, scales=kw["scales"] * 2.0, **options)
+    kw["Ks"] = torch.tensor([[[210.0, 0.0, 166.0], [0.0, 210.0, 105.0], [0.0, 0.0, 1.0]]], device=DEV).repeat(C, 1, 1)
+    if C > 1:
+        kw["viewmats"] = kw["viewmats"].repeat(C, 1, 1)
+        kw["viewmats"][:, 0, 3] = torch.arange(C, device=DEV) * 2.0
+        for k in ("linear_velocity", "angular_velocity"):
+            kw[k] = kw[k].repeat(C, 1)
+        kw["rolling_shutter_time"] = kw["rolling_shutter_time"].repeat(C)
+    if "sh" not in colors:
+        kw.update(sh_degree=None, colors=rand(C, N, 5) if "per camera" in colors else rand(N, 5))
+    elif "per camera" in colors:
+        kw["colors"] = (rand(C, N, 16, 3) - 0.5) * 0.6
+    if options.get("backgrounds"):
+        kw["backgrounds"] = rand(C, 3 if "sh" in colors else 5)
+    wanted = {"all": _all_of, "image only": lambda i: [_all_of(i)[0], None], "alpha only": lambda i: [None, _all_of(i)[1]]}[cotangents]
+    leaves = ("means", "quats", "scales", "opacities") + (() if mode in ("D", "ED") else ("colors",))
+    if cotangents == "alpha only":
+        leaves = tuple(k for k in leaves if k != "colors")
+    _twice(monkeypatch, "_native_camera_frame", splatad_b200.rasterization, kw, leaves, wanted)
+
+
+@pytest.mark.parametrize("C,features,options", [
+    (1, 1, {}), (1, 7, dict(absgrad=True)), (1, 16, dict(rasterize_mode="antialiased")), (1, 4, dict(compute_alpha_sum_until_points=False)),
+    (2, 4, dict(absgrad=True)), (2, 16, dict(rasterize_mode="antialiased")),
+])
+@pytest.mark.parametrize("cotangents", ["all", "image only", "alpha only", "alpha sum only"])
+def test_native_lidar_frames_are_those_of_the_ops(C, features, options, cotangents, monkeypatch):
+    import splatad_b200
+    from splatad_b200 import scenes
+    at = ("all", "image only", "alpha only", "alpha sum only").index(cotangents) - 1
+    if at == 2 and options.get("compute_alpha_sum_until_points") is False:
+        pytest.skip("no alpha sum")
+    N = 15_013
+    kw = _to_gpu(scenes.config2(N=N, width=600))
+    g = torch.Generator(device=DEV).manual_seed(C)
+    kw.update(lidar_features=torch.randn(C, N, features, generator=g, device=DEV), **options)
+    if C > 1:
+        for k in ("viewmats", "raster_pts", "linear_velocity", "angular_velocity", "rolling_shutter_time"):
+            kw[k] = kw[k].repeat(C, *([1] * (kw[k].dim() - 1)))
+        kw["viewmats"][:, 0, 3] += torch.arange(C, device=DEV) * 1.0
+
+    def wanted(images):
+        every = _all_of(images)
+        return every if at < 0 else [w if i == at else None for i, w in enumerate(every)]
+
+    leaves = ("means", "quats", "scales", "opacities") + (("lidar_features",) if at in (-1, 0) else ())
+    _twice(monkeypatch, "_native_lidar_frame", splatad_b200.lidar_rasterization, kw, leaves, wanted)
