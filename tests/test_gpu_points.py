@@ -41,11 +41,11 @@ def test_map_points_and_offsets_vs_oracle(C, N, sort):
 
 
 @pytest.mark.parametrize("C,N,n_az,n_el", [
-    (1, 2047, 1, 1), (1, 2049, 2, 1), (2, 4097, 32, 32), (1, 30_000, 89, 23), (1, 30_000, 2049, 1), (1, 1_300_000, 64, 16),
+    (1, 1023, 1, 1), (1, 1024, 2, 3), (1, 1025, 2, 1), (1, 2047, 1, 1), (1, 2049, 2, 1), (2, 4097, 32, 32), (1, 30_000, 89, 23), (1, 30_000, 2049, 1), (1, 1_300_000, 64, 16),
 ])
 def test_map_points_in_one_pass_over_the_tiles(C, N, n_az, n_el):
-    """Up to 2048 tiles are sorted in one pass, in blocks of 2048 points: one tile, 2047, 2048 and 2049 of
-    them, remainders of a block, several blocks' worth per block, crowded tiles; read in place from the
+    """Up to 2048 tiles are sorted in one pass, in steps of 1024 points: one tile, 2047, 2048 and 2049 of
+    them, one point short of a step, a whole one and one more, several blocks' worth per block, crowded tiles; read in place from the
     rows of a point cloud. Bit for bit the oracle's."""
     from oracle import isect
     from splatad_b200 import ops
