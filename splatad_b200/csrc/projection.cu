@@ -573,7 +573,9 @@ __device__ __forceinline__ float stretch_bound(const M3 &R) {
 // an extent that is never below the one project_cam finds. A row j of the Jacobian gives the
 // variance j^T S j <= |S| |j|^2, with the Frobenius norm for |S|; the margins (0.1 % of the extent,
 // 0.01 pixel, 1e-5 of the terms that cancel in the mean) are orders above the rounding of either
-// side. Comparisons with a NaN are false, which leaves the pair to project_cam.
+// side. The depth is the one project_cam computes, in this kernel and the dense one alike (a million Gaussians within
+// three units in the last place of a plane: the same ones kept). Comparisons with a NaN are false, which leaves the
+// pair to project_cam.
 __device__ __forceinline__ bool surely_culled(const SensorCam &s, const CamLimits &lim, float stretch, V3 mean,
                                               float norm, bool has_vel, V3 vel_w, int width, int height,
                                               float eps2d, float near_plane, float far_plane, float radius_clip) {
@@ -1111,7 +1113,7 @@ __device__ __forceinline__ uint32_t queue_touched(BwdQueue &q, uint32_t C, uint3
 // Gaussians per block: the whole span only where that still fills the two blocks each SM holds.
 static uint32_t bwd_span(uint32_t N) {
     const uint32_t blocks = div_up(N, kThreads);
-    return kThreads * max(1u, min(kBwdSpan, blocks / (2 * 148)));
+    return kThreads * max(1u, min(kBwdSpan, blocks / (2 * kNumSMs)));
 }
 
 __device__ __forceinline__ void store_zeros(float *base, size_t first, uint32_t n) {

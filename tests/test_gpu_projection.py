@@ -5,6 +5,8 @@ Tolerances: forward 1e-4 relative + 1e-5 absolute (angles / pixels: + 1e-4 absol
 they are O(100) numbers in float32); gradients 1e-3 relative, judged against a float64 oracle.
 """
 
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -519,3 +521,25 @@ def test_lidar_projection_slab_boundaries(N):
                                             *sens, **kw)
     for a, b in zip(fast, plain):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("plane", ["near", "far"])
+def test_packed_and_dense_projection_agree_at_the_depth_planes(plane):
+    """A million Gaussians within three units in the last place of a plane, behind a turned camera: the packed layout
+    keeps exactly those that the dense one does."""
+    from splatad_b200 import ops
+    n, at = 1_000_000, 1.0
+    g = torch.Generator(device=DEV).manual_seed(3)
+    c, s = math.cos(0.3), math.sin(0.3)
+    vm = torch.tensor([[[c, 0.0, -s, 0.0], [0.0, 1.0, 0.0, 0.0], [s, 0.1, c, 0.37], [0.0, 0.0, 0.0, 1.0]]], device=DEV)
+    p = torch.rand(n, 3, generator=g, device=DEV) * 4 - 2
+    z = at + torch.randint(-3, 4, (n,), generator=g, device=DEV).double() * 6e-8
+    row = vm[0, 2].double()
+    p[:, 2] = ((z - row[3] - row[0] * p[:, 0].double() - row[1] * p[:, 1].double()) / row[2]).float()
+    kw = dict(means=p, covars=None, quats=torch.randn(n, 4, device=DEV, generator=g), scales=torch.full((n, 3), 0.05, device=DEV),
+              velocities=None, viewmats=vm, Ks=torch.tensor([[[500.0, 0, 640], [0, 500, 360], [0, 0, 1]]], device=DEV), width=1280,
+              height=720, linear_velocity=torch.zeros(1, 3, device=DEV), angular_velocity=torch.zeros(1, 3, device=DEV),
+              rolling_shutter_time=torch.zeros(1, device=DEV), **({"near_plane": at} if plane == "near" else {"far_plane": at}))
+    dense = (ops.fully_fused_projection(**kw)[0][0, :, 0] > 0).nonzero()[:, 0]
+    packed = ops.fully_fused_projection(**kw, packed=True)[1]
+    assert 50_000 < dense.numel() < n // 2 and torch.equal(dense, packed)
