@@ -292,16 +292,6 @@ def wait_for_count(slot: torch.Tensor, sequence: int, event: torch.cuda.Event, p
     return int(view[0]), int(view[2])
 
 
-def early_depth_range(slot: torch.Tensor, sequence: int):
-    """(lo bits, hi bits) of the depth range a plan reported with its early count (slot[7], valid
-    once slot[5] holds ``sequence``), or None when it reported none."""
-    view = slot.numpy()
-    if not sequence or view[5] != sequence or view[7] == 0:
-        return None
-    word = int(view[7]) & 0xFFFFFFFFFFFFFFFF
-    return word & 0xFFFFFFFF, word >> 32
-
-
 def release_pinned_slot(slot: torch.Tensor) -> None:
     free = _free_slots.setdefault(slot._splatad_stream_key, [])
     if len(free) < 16:

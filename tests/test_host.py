@@ -139,18 +139,25 @@ def test_wait_for_count_polls_the_early_triple_and_falls_back_to_the_event():
     assert b == a + 1 and a > 0
 
 
-def test_early_depth_range_is_read_only_with_a_matching_sequence():
-    """slot[7] holds dmin bits | dmax bits << 32 of the frame's listed depths, valid once slot[5]
-    carries the frame's sequence number; 0 means the reporting kernel did not know the range."""
-    from splatad_b200 import _lib
-    slot = torch.zeros(8, dtype=torch.int64)
+def test_what_a_native_frame_reports_is_kept_for_the_next(monkeypatch):
+    """The count sizes the next frame's lists; the depth range (dmin bits | dmax bits << 32, 0: not known) spans its
+    buckets. An overflow of the buckets drops a range that was carried over, and means the radix sort only without
+    one; more intersections than the ids can number are an error."""
+    from splatad_b200 import ops
+    for name in ("_isect_count_hint", "_depth_range_hint", "_depth_sort_mode"):
+        monkeypatch.setattr(ops, name, {})
     lo, hi = 0x3E99999A, 0x42E20000                    # 0.3 and 113.0 as float bit patterns
-    slot[5], slot[7] = 9, lo | (hi << 32)
-    assert _lib.early_depth_range(slot, 9) == (lo, hi)
-    assert _lib.early_depth_range(slot, 10) is None    # another frame's words
-    assert _lib.early_depth_range(slot, 0) is None     # nothing was armed
-    slot[7] = 0
-    assert _lib.early_depth_range(slot, 9) is None
+    ops.note_counts("shape", 1000, 0, lo | (hi << 32), ranged=False)
+    assert ops._isect_count_hint == {"shape": 1000} and ops._depth_range_hint == {"shape": (lo, hi)}
+    ops.note_counts("shape", 900, 0, 0, ranged=True)
+    assert ops._isect_count_hint == {"shape": 900} and ops._depth_range_hint == {"shape": (lo, hi)}
+    ops.note_counts("shape", 900, 4, lo | (hi << 32), ranged=True)
+    assert ops._depth_range_hint == {} and ops._depth_sort_mode == {}
+    ops.note_counts("shape", 900, 4, lo | (hi << 32), ranged=False)
+    assert ops._depth_range_hint == {} and ops._depth_sort_mode == {"shape": 2}
+    with pytest.raises(RuntimeError, match="do not fit"):
+        ops.note_counts("shape", 2**31, 2, 0, ranged=False)
+    assert ops.list_room(900) > 900 and ops.packed_room(70_000, 10**6) % 65536 == 0 and ops.packed_room(70_000, 70_001) == 70_001
 
 
 def test_gradient_accumulators_share_one_zeroed_buffer():
