@@ -762,7 +762,9 @@ def run_ours(args):
         roofline = None
         if bytes_per_launch is not None:
             achieved = bytes_per_launch / (dom_ms / dom_cnt * 1e-3) / 1e9
-            roofline = {"kernel": dom_name, "bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
+            # the compositing kernels hardly touch DRAM: what bounds them is instruction issue
+            bound = "issue" if dom_name.startswith("rasterize_") else "hbm"
+            roofline = {"kernel": dom_name, "bound": bound, "achieved": round(achieved, 1), "peak": peak,
                         "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic,
                         "traffic_source": traffic_src,
                         "peak_source": f"of {peak_src}", "launches_per_step": dom_cnt,

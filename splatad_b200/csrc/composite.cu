@@ -1160,7 +1160,7 @@ __device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t
 // the sums of v, v dx and v dx^2 (v = exp(-sigma) dL/dalpha). The channels behind an entry enter through
 // one number per pixel: dL/dalpha = T (c . g) - (1 / (1 - alpha)) (sum over the entries behind of
 // their weight times their (c . g)), g the pixel's cotangent - a running scalar in place of a running colour.
-// Camera benchmark's training step: 1.55 -> 0.42 ms.
+// Camera benchmark's training step: 1.55 -> 0.40 ms.
 // ---------------------------------------------------------------------------------------
 // registers per thread, by measurement: more warps pay up to a few spilled words (4 channels: 421 us at 100
 // registers, 370 at 80, 384 at 64)
@@ -1878,22 +1878,26 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         else { CALL(32); }                                                                       \
     } while (0)
 
-// The forward kernels of more blocks than the machine holds at once start on empty SMs. Chained, their first
+// Forward kernels of many blocks start on empty SMs. The line is one for all of them: eight blocks an SM, what the
+// four-channel camera kernel has room for (32 channels hold four, the lidar's 64 threads up to twelve). Chained, their first
 // blocks are placed beside the last of the colour or list kernels before them, on SMs that keep that kernel's
 // large shared memory and small first-level cache for as long as one block follows another, and the gathers need
 // the cache (with all of it given to shared memory the 1920 x 1080 kernel takes 237 us instead of 209): with
-// spherical harmonics 437 us a frame chained, 411 apart; six cameras 3490 and 3370; 128 x 1800 lidar 294 and 289. Below, the launch gap weighs more (640 x 360: 101 and 103).
+// spherical harmonics 437 us a frame chained, 411 apart; six cameras 3490 and 3370; 128 x 1800 lidar 294 and 289.
+// Below, the launch gap weighs more (640 x 360: 101 and 103).
 static bool fits_at_once(uint64_t blocks) { return blocks <= (uint64_t)kNumSMs * 8; }
 
 // Patches below which all warps of a CTA share one in the forward pass: the shared work costs more
-// instructions in all, so the patches must be too few to fill the machine (2176 patches: 53 us apart, 102
-// shared; 512: 124 and 65).
+// instructions in all, so the patches must be too few to fill the machine. Apart and shared, us, 8 channels: 512
+// patches 82 and 31, 800 73 and 42, 1088 72 and 46, 1408 54 and 44, 1856 57 and 52, 2176 58 and 62, 3200 65 and 87; 17
+// channels cross over a little earlier (1856: 66 both). The line lies below the crossing in every case measured.
 constexpr uint64_t kCoopPatches = kNumSMs * 8;
 
 // Warps - segments of the list - per patch in the backward pass: every segment is run twice, which pays
-// while the patches alone leave the schedulers waiting on one warp's chain (256 patches: 405 us with one
-// segment, 178 with four, 96 with eight, 78 with sixteen; 1088: 124, 100 and 104; 3648: 172, and 231 with
-// four). Sixteen take an SM each, and only up to eight channels stay within their 128 registers.
+// while the patches alone leave the schedulers waiting on one warp's chain. One, four and eight segments, us, 8
+// channels: 256 patches 184, 82, 54 (sixteen: 49), 400 174, 74, 60, 544 166, 75, 73, 704 98, 71, 68, 1088 101, 82, 91,
+// 1600 109, 116, 128, 2240 119, 144, 165 (17 channels: 1600 137, 145, 162); so four lose to one from about 1400 on,
+// short of the line below. Sixteen take an SM each, and only up to eight channels stay within their 128 registers.
 static uint32_t point_segments(uint64_t patches, uint32_t channels) {
     if (channels <= 8 && patches < (uint64_t)kNumSMs * 2) return 16u;
     return patches < (uint64_t)kNumSMs * 4 ? 8u : patches < (uint64_t)kNumSMs * 16 ? 4u : 1u;

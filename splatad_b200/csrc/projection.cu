@@ -813,7 +813,7 @@ packed_scan_kernel(const int32_t *__restrict__ counts, int32_t *__restrict__ off
                    uint32_t nblocks, int32_t *__restrict__ indptr, int64_t *__restrict__ nnz_out) {
     chain_enter();
     // rounds of 4096 counts, four consecutive ones per thread (one strip per thread, read twice, took 44 us
-    // for the 47 k counts of six cameras and two million Gaussians, this 25)
+    // for the 47 k counts of six cameras and two million Gaussians, this 29)
     __shared__ int32_t warp_sum[33];
     const uint32_t total = C * nblocks, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     int32_t carry = 0;
