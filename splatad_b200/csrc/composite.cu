@@ -16,6 +16,8 @@
 // Thresholds kept: alpha cap 0.999, alpha < 1/255 skipped, sigma < 0 skipped, a pixel stops
 // (exclusively) when T*(1-alpha) <= 1e-4, median depth where T crosses 0.5, points with
 // range <= 0 are not rendered.
+#include <type_traits>
+
 #include "common.cuh"
 #include "composite_common.cuh"
 
@@ -89,9 +91,8 @@ __device__ __forceinline__ TilePixels<PX> tile_pixels(uint32_t tile_size, uint32
 // Pixel centres of a warp's patch.
 struct PatchBox { float x0, x1, y0, y1; };
 
-// Per-warp boxes of the CTA's patches; an empty patch gets an empty box (nothing is visible in it).
-template <int PX>
-__device__ __forceinline__ void patch_boxes(PatchBox *s_box, float px, float py, uint32_t n_inside) {
+// The box of the calling warp's patch, in every lane; an empty patch gets an empty box (nothing is visible in it).
+__device__ __forceinline__ PatchBox warp_box(float px, float py, uint32_t n_inside) {
     PatchBox b = {3.0e38f, -3.0e38f, 3.0e38f, -3.0e38f};
     if (n_inside) b = {px, px + (float)(n_inside - 1), py, py};
 #pragma unroll
@@ -101,13 +102,12 @@ __device__ __forceinline__ void patch_boxes(PatchBox *s_box, float px, float py,
         b.y0 = fminf(b.y0, __shfl_xor_sync(0xffffffffu, b.y0, off));
         b.y1 = fmaxf(b.y1, __shfl_xor_sync(0xffffffffu, b.y1, off));
     }
-    if ((threadIdx.x & 31u) == 0u) s_box[threadIdx.x >> 5] = b;
+    return b;
 }
 
-// A list entry as its staging thread sees it, and the warps whose patch it can reach.
+// A list entry as its staging lane sees it.
 struct PixelEntry {
     float4 A, B;       // mean, its velocity | conic, opacity
-    uint32_t seen;     // bit w: may contribute to a pixel of warp w's patch
 };
 
 __device__ __forceinline__ PixelEntry load_pixel_entry(int32_t g, const float2 *__restrict__ means2d,
@@ -119,16 +119,19 @@ __device__ __forceinline__ PixelEntry load_pixel_entry(int32_t g, const float2 *
     e.A = make_float4(xy.x, xy.y, v.x, v.y);
     e.B = make_float4(__ldg(conics + 3 * (size_t)g), __ldg(conics + 3 * (size_t)g + 1),
                       __ldg(conics + 3 * (size_t)g + 2), __ldg(opacities + g));
-    e.seen = 0u;
     return e;
 }
 
-constexpr uint32_t kOddEntry = 1u << 31;   // beside the warps of a CTA: see odd_pixels_fwd()
+constexpr uint32_t kSeenEntry = 1u, kCarefulEntry = 2u, kOddEntry = 4u;
 
-// The mean moves with the row's shutter time; roll_lo / roll_hi bound it over the tile.
+// What a warp has to know about an entry: whether it can reach the warp's patch (kSeenEntry; 0: it need not look at it),
+// whether its alphas need looking at one by one (kCarefulEntry: a sigma that could come out negative, an alpha above the
+// cap), and whether it is one for odd_pixels_fwd() (kOddEntry). The alphas of the others need no test but the one
+// against 1/255: with ac - b^2 >= 1e-5 ac the form a dx^2 + 2 b dx dy + c dy^2 is at least 5e-6 (a dx^2 + c dy^2), ten times
+// what its rounding can take away, and an opacity within the cap keeps every alpha there. The mean moves with the
+// row's shutter time; roll_lo / roll_hi bound it over the tile.
 template <bool kMarkOdd>
-__device__ __forceinline__ uint32_t warps_that_see(const PixelEntry &e, const PatchBox *s_box, uint32_t n_warps,
-                                                   float roll_lo, float roll_hi) {
+__device__ __forceinline__ uint32_t patch_sees(const PixelEntry &e, const PatchBox &box, float roll_lo, float roll_hi) {
     const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
     if (test.never) return 0u;
     const float mx_a = e.A.x + roll_lo * e.A.z, mx_b = e.A.x + roll_hi * e.A.z;
@@ -140,10 +143,11 @@ __device__ __forceinline__ uint32_t warps_that_see(const PixelEntry &e, const Pa
         const bool plain = fabsf(e.B.x) > 1e-30f && fabsf(e.B.x) + fabsf(e.B.y) + fabsf(e.B.z) < 1e30f;
         if (!plain || !(mx_lo <= mx_hi) || !(my_lo <= my_hi) || !(test.s_max < 1e30f)) seen = kOddEntry;
     }
-    for (uint32_t w = 0; w < n_warps; ++w) {
-        const PatchBox b = s_box[w];
-        if (b.x0 <= b.x1 && !test.misses(mx_lo - b.x1, mx_hi - b.x0, my_lo - b.y1, my_hi - b.y0)) seen |= 1u << w;
-    }
+    const float ac = e.B.x * e.B.z;
+    const bool sized = e.B.x > 1e-15f && e.B.z > 1e-15f && e.B.x < 1e15f && e.B.z < 1e15f;   // nothing under- or overflows
+    if (!(sized && ac - e.B.y * e.B.y >= 1e-5f * ac && e.B.w <= kAlphaMax)) seen |= kCarefulEntry;
+    if (box.x0 <= box.x1 && !test.misses(mx_lo - box.x1, mx_hi - box.x0, my_lo - box.y1, my_hi - box.y0)) seen |= kSeenEntry;
+    else seen &= kOddEntry;
     return seen;
 }
 
@@ -197,10 +201,10 @@ struct TaskPixel {
 };
 
 template <int PX>
-__device__ __forceinline__ TaskPixel task_pixel(const PixelTask &a, uint32_t k) {
-    const uint32_t per_cam = a.tile_w * a.tile_h, cam = blockIdx.x / per_cam, tile = blockIdx.x - cam * per_cam;
+__device__ __forceinline__ TaskPixel task_pixel(const PixelTask &a, uint32_t gtile, uint32_t tr, uint32_t k) {
+    const uint32_t per_cam = a.tile_w * a.tile_h, cam = gtile / per_cam, tile = gtile - cam * per_cam;
     const uint32_t ty = tile / a.tile_w, tx = tile - ty * a.tile_w;
-    const TilePixels<PX> tp = tile_pixels<PX>(a.tile_size, threadIdx.x);
+    const TilePixels<PX> tp = tile_pixels<PX>(a.tile_size, tr);
     const uint32_t i = ty * a.tile_size + tp.y, j = tx * a.tile_size + tp.x + k;
     TaskPixel p;
     p.inside = tp.y < a.tile_size && tp.x + k < a.tile_size && i < a.H && j < a.W;
@@ -232,11 +236,11 @@ __device__ __forceinline__ PixelAlpha pixel_alpha(const PixelTask &a, int32_t g,
 }
 
 template <int PX>
-__device__ __noinline__ void odd_pixels_fwd(const PixelTask &a, float *colors_out, float *alphas, int32_t *last_ids, bool expected,
+__device__ __noinline__ void odd_pixels_fwd(const PixelTask &a, uint32_t gtile, uint32_t tr, float *colors_out, float *alphas, int32_t *last_ids, bool expected,
                                             float *expected_depths) {
-    const TileRange range = tile_range(a.offsets, blockIdx.x, a.C * a.tile_w * a.tile_h, a.n_isects);
+    const TileRange range = tile_range(a.offsets, gtile, a.C * a.tile_w * a.tile_h, a.n_isects);
     for (uint32_t h = 0; h < (uint32_t)PX; ++h) {
-        const TaskPixel p = task_pixel<PX>(a, h);
+        const TaskPixel p = task_pixel<PX>(a, gtile, tr, h);
         if (!p.inside) continue;
         float *color = colors_out + p.pix * a.channels, T = 1.f;
         int32_t pos = 0;
@@ -273,11 +277,11 @@ __device__ __forceinline__ void add_warp_total(float *to, float v) {
 
 // By whole warps.
 template <int PX>
-__device__ __noinline__ void odd_pixels_bwd(const PixelTask &a, const PixelGrads &grad) {
-    const TileRange range = tile_range(a.offsets, blockIdx.x, a.C * a.tile_w * a.tile_h, a.n_isects);
+__device__ __noinline__ void odd_pixels_bwd(const PixelTask &a, uint32_t gtile, uint32_t tr, const PixelGrads &grad) {
+    const TileRange range = tile_range(a.offsets, gtile, a.C * a.tile_w * a.tile_h, a.n_isects);
     const uint32_t n = a.channels;
     for (uint32_t h = 0; h < (uint32_t)PX; ++h) {
-        const TaskPixel p = task_pixel<PX>(a, h);
+        const TaskPixel p = task_pixel<PX>(a, gtile, tr, h);
         const int32_t last = p.inside ? min(range.end - 1, last_position(grad.last_ids[p.pix])) : -1;
         const float *v_out = grad.v_colors_in + p.pix * n;
         float T = 1.f, behind = 0.f, divisor = 1.f;
@@ -338,49 +342,188 @@ __device__ __noinline__ void odd_pixels_bwd(const PixelTask &a, const PixelGrads
     }
 }
 
+// A row of n floats to shared memory, zeros behind them: all loads are on their way before the first is waited for.
+template <int CDIM>
+__device__ __forceinline__ void stage_whole_row(float4 *dst, const float *__restrict__ src, uint32_t n, bool vec) {
+#pragma unroll
+    for (int k = 0; k < CDIM; k += 4) {
+        float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (vec) {
+            if ((uint32_t)k < n) w = __ldg(reinterpret_cast<const float4 *>(src + k));
+        } else {
+            if ((uint32_t)k < n) w.x = __ldg(src + k);
+            if ((uint32_t)k + 1u < n) w.y = __ldg(src + k + 1);
+            if ((uint32_t)k + 2u < n) w.z = __ldg(src + k + 2);
+            if ((uint32_t)k + 3u < n) w.w = __ldg(src + k + 3);
+        }
+        dst[k / 4] = w;
+    }
+}
+
+// Rows of n floats, whole 16-byte pieces, between a table and a warp's shared memory, where row r lies at r * CDIM: lane r
+// names the table's row for it, `mask` the rows that are wanted. The lanes go over the rows' pieces in
+// sequence, so that one access touches a few lines; a lane that copies a row by itself touches as many lines
+// with every access as there are lanes. Pays for wide rows in 16-byte pieces: forward kernel, 1920 x 1080, 32 channels 727 -> 583 us,
+// 20 channels 396 -> 389; 13 channels, one float at a time, 323 -> 404.
+template <int CDIM, bool kStore>
+__device__ __forceinline__ void copy_rows(float *rows, std::conditional_t<kStore, float, const float> *table, int32_t row_id,
+                                          uint32_t mask, uint32_t n, uint32_t lane) {
+    const uint32_t pieces = n / 4u, skip = 32u / pieces, rest = 32u - skip * pieces;
+    uint32_t r = lane / pieces, k = lane - r * pieces;
+    for (uint32_t round = 0; round < pieces; ++round) {
+        const size_t id = (size_t)__shfl_sync(0xffffffffu, row_id, r);
+        if ((mask >> r) & 1u) {
+            auto *there = reinterpret_cast<std::conditional_t<kStore, float4, const float4> *>(table + id * n) + k;
+            float4 *here = reinterpret_cast<float4 *>(rows + r * CDIM) + k;
+            if constexpr (kStore) *there = *here; else *here = __ldg(there);
+        }
+        r += skip;
+        k += rest;
+        if (k >= pieces) { k -= pieces; ++r; }
+    }
+}
+
+// The values of a thread's PX pixels, next to each other in memory: in 16-byte pieces where they lie so. One float at a
+// time every lane of a warp touches a line of its own, and 32 such loads are what 8 of these are (backward
+// kernel of the 1920 x 1080 benchmark: 335 -> 312 us).
+template <int M>
+__device__ __forceinline__ bool in_pieces(const void *p) { return M % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
+
+template <int M, typename T>
+__device__ __forceinline__ void load_pieces(T (&v)[M], const T *src) {
+    static_assert(sizeof(T) == 4, "");
+#pragma unroll
+    for (int k = 0; k + 4 <= M; k += 4) {
+        const int4 w = __ldg(reinterpret_cast<const int4 *>(src + k));
+        v[k] = reinterpret_cast<const T &>(w.x); v[k + 1] = reinterpret_cast<const T &>(w.y);
+        v[k + 2] = reinterpret_cast<const T &>(w.z); v[k + 3] = reinterpret_cast<const T &>(w.w);
+    }
+}
+
+template <int M, typename T>
+__device__ __forceinline__ void store_pieces(T *dst, const T (&v)[M]) {
+    static_assert(sizeof(T) == 4, "");
+#pragma unroll
+    for (int k = 0; k + 4 <= M; k += 4)
+        *reinterpret_cast<int4 *>(dst + k) = make_int4(reinterpret_cast<const int &>(v[k]), reinterpret_cast<const int &>(v[k + 1]),
+                                                       reinterpret_cast<const int &>(v[k + 2]), reinterpret_cast<const int &>(v[k + 3]));
+}
+
+// One value of each of a thread's pixels; `outside` beyond the image.
+template <int PX, typename T>
+__device__ __forceinline__ void load_pixels(T (&v)[PX], const T *src, uint32_t n_inside, T outside) {
+    if (n_inside == (uint32_t)PX && in_pieces<PX>(src)) load_pieces<PX>(v, src);
+    else
+#pragma unroll
+        for (int k = 0; k < PX; ++k) v[k] = (uint32_t)k < n_inside ? src[k] : outside;
+}
+
+template <int PX, typename T>
+__device__ __forceinline__ void store_pixels(T *dst, const T (&v)[PX], uint32_t n_inside) {
+    if (n_inside == (uint32_t)PX && in_pieces<PX>(dst)) store_pieces<PX>(dst, v);
+    else
+#pragma unroll
+        for (int k = 0; k < PX; ++k)
+            if ((uint32_t)k < n_inside) dst[k] = v[k];
+}
+
+// The channels of a thread's pixels, zeros behind those there are.
+template <int CDIM, int PX, int N>
+__device__ __forceinline__ bool load_whole_channels(float (&v)[PX][CDIM], const float *src, uint32_t channels) {
+    if (channels != (uint32_t)N || !in_pieces<PX * N>(src)) return false;
+    float flat[PX * N];
+    load_pieces<PX * N>(flat, src);
+#pragma unroll
+    for (int k = 0; k < PX; ++k)
+#pragma unroll
+        for (int c = 0; c < CDIM; ++c) v[k][c] = c < N ? flat[k * N + (c < N ? c : 0)] : 0.f;
+    return true;
+}
+
+template <int CDIM, int PX>
+__device__ __forceinline__ void load_channels(float (&v)[PX][CDIM], const float *src, uint32_t channels, uint32_t n_inside) {
+    if constexpr (CDIM == 4)
+        if (n_inside == (uint32_t)PX &&
+            (load_whole_channels<CDIM, PX, 4>(v, src, channels) || load_whole_channels<CDIM, PX, 3>(v, src, channels))) return;
+#pragma unroll
+    for (int k = 0; k < PX; ++k)
+#pragma unroll
+        for (int c = 0; c < CDIM; ++c) v[k][c] = (uint32_t)k < n_inside && (uint32_t)c < channels ? src[k * channels + c] : 0.f;
+}
+
+template <int CDIM, int PX, int N>
+__device__ __forceinline__ bool store_whole_channels(float *dst, const float (&v)[PX][CDIM], uint32_t channels) {
+    if (channels != (uint32_t)N || !in_pieces<PX * N>(dst)) return false;
+    float flat[PX * N];
+#pragma unroll
+    for (int k = 0; k < PX; ++k)
+#pragma unroll
+        for (int c = 0; c < N; ++c) flat[k * N + c] = v[k][c];
+    store_pieces<PX * N>(dst, flat);
+    return true;
+}
+
+template <int CDIM, int PX>
+__device__ __forceinline__ void store_channels(float *dst, const float (&v)[PX][CDIM], uint32_t channels, uint32_t n_inside) {
+    if constexpr (CDIM == 4)
+        if (n_inside == (uint32_t)PX &&
+            (store_whole_channels<CDIM, PX, 4>(dst, v, channels) || store_whole_channels<CDIM, PX, 3>(dst, v, channels))) return;
+#pragma unroll
+    for (int k = 0; k < PX; ++k)
+#pragma unroll
+        for (int c = 0; c < CDIM; ++c)
+            if ((uint32_t)k < n_inside && (uint32_t)c < channels) dst[k * channels + c] = v[k][c];
+}
+
 // ---------------------------------------------------------------------------------------
-// Camera forward. Bound by instruction issue: two pixels per thread take 50 instructions per entry where
-// one took 40, and a warp passes over the entries that cannot reach its 8 x 8 patch without looking at
-// them. A pixel that has stopped moves its column out to where every alpha vanishes, which costs the
-// other pixels nothing; a warp leaves when all of its pixels have. Camera benchmark frame: 0.338 -> 0.209 ms.
+// Camera forward. A warp draws a patch by itself: PX pixels of a row per lane, 16 x 16 pixels of a tile with eight, 16 x 8
+// with four, 8 x 8 with two; no barrier and no other warp's list position concerns it.
+//
+// What bounds it is instruction issue and, as more pixels share a lane, the FP32 pipe. What an entry costs whatever
+// the number of pixels - loads, bits, the row's terms, the stop test - was a third of the work at two pixels, and
+// where Gaussians are larger than tiles (61 of 64 pixels blend a looked-at entry in the benchmark scenes) there is nothing
+// to gain from small patches. So: eight pixels; alphas tested against 1/255 only, unless the entry was marked
+// (patch_sees()); no instruction spent on a sign; the transmittance updated in place by one multiply-add, which rounds once.
+// A pixel that has stopped moves its column out to where every alpha vanishes; a warp leaves when all of its have.
+// 1920 x 1080, 4 channels: 201 M -> 104 M warp instructions, 222 -> 147 us (two pixels 208, four 156); 16 channels, 1237 x 719:
+// 180 -> 152 (1920 x 1080: 8, 13, 20 and 32 channels 313, 376, 448, 683 -> 218, 308, 426, 570). Staging every value twice for the packed operands: 12 us slower; asynchronous copies of the next batches: 9.
 // ---------------------------------------------------------------------------------------
 constexpr float kPixelGone = 1e18f;   // a column no Gaussian reaches: sigma overflows, alpha is 0 (or NaN, never drawn)
 
-// registers per thread: as many CTAs of 128 threads per SM as the accumulators leave room for
-constexpr int pixels_fwd_regs(int cdim) { return cdim <= 8 ? 64 : cdim <= 16 ? 80 : cdim <= 20 ? 96 : 128; }
+// registers per thread, by measurement (4 channels, eight pixels: 147 us at 128 registers, 163 at 112 and 96; 8 channels, four
+// pixels: 218 at 96, 243 at 112 and 128; 20 channels: 426 at 96, 445 at 112 and 160)
+constexpr int pixels_fwd_regs(int cdim, int px) {
+    return cdim <= 4 ? (px == 8 ? 128 : px == 4 ? 80 : 64) : cdim <= 8 ? (px == 4 ? 96 : 72) : cdim <= 16 ? (px == 4 ? 128 : 96) : cdim <= 20 ? 96 : 128;
+}
 
-template <int CDIM>
-__global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kernel(
+template <int CDIM, int PX>
+__global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX)) rasterize_to_pixels_fwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
     const float *__restrict__ opacities, const float2 *__restrict__ pix_vels,
     const float *__restrict__ rs_time, const float *__restrict__ backgrounds, uint32_t W,
-    uint32_t H, uint32_t tile_size, uint32_t tile_w, uint32_t tile_h,
+    uint32_t H, uint32_t tile_size, uint32_t tile_w, uint32_t tile_h, uint32_t patches /* of a tile */,
     const int32_t *__restrict__ offsets, const int32_t *__restrict__ flatten_ids,
     float *__restrict__ render_colors, float *__restrict__ render_alphas,
     int32_t *__restrict__ last_ids, uint32_t expected /* divide the last channel by the alpha */,
     float *__restrict__ expected_depths /* optional: and keep it for the backward pass */) {
     chain_enter();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ uint32_t s_warp_kept[16];
-    __shared__ PatchBox s_box[16];
-    const uint32_t bs = blockDim.x;
-    float4 *sA = reinterpret_cast<float4 *>(smem_raw);               // x, y, vx, vy
-    float4 *sB = sA + bs;                                            // scaled conic, opacity
-    float *sCol = reinterpret_cast<float *>(sB + bs);                // [bs * CDIM], zeros behind the channels
-    int32_t *sPos = reinterpret_cast<int32_t *>(sCol + bs * CDIM);   // list position of the staged entry
-    uint32_t *sSeen = reinterpret_cast<uint32_t *>(sPos + bs);       // warps that may see it
+    static_assert(PX % 2 == 0, "pixels are handled in pairs");
+    constexpr int P2 = PX / 2;
+    __shared__ float4 sA[32];                // x, y, vx, vy
+    __shared__ float4 sB[32];                // scaled conic, minus the opacity
+    __shared__ float4 sCol[32 * CDIM / 4];   // zeros behind the channels
     const bool vec = (channels % 4u == 0u) && ((reinterpret_cast<uintptr_t>(colors) & 15u) == 0u);
 
     const uint32_t tiles_per_cam = tile_w * tile_h;
-    const uint32_t cam = blockIdx.x / tiles_per_cam;
-    const uint32_t tile = blockIdx.x - cam * tiles_per_cam;
+    const uint32_t gtile = blockIdx.x / patches, cam = gtile / tiles_per_cam;
+    const uint32_t tile = gtile - cam * tiles_per_cam;
     const uint32_t ty = tile / tile_w, tx = tile - ty * tile_w;
-    const uint32_t tr = threadIdx.x, lane = tr & 31u, warp = tr >> 5, n_warps = bs >> 5;
-    const TilePixels<2> tp = tile_pixels<2>(tile_size, tr);
+    const uint32_t lane = threadIdx.x, tr = (blockIdx.x - gtile * patches) * 32u + lane;
+    const TilePixels<PX> tp = tile_pixels<PX>(tile_size, tr);
     const uint32_t i = ty * tile_size + tp.y, j = tx * tile_size + tp.x;
     uint32_t n_inside = 0;   // pixels of this thread inside the tile and the image
-    if (tp.y < tile_size && i < H && j < W) n_inside = min(min(2u, tile_size - tp.x), W - j);
+    if (tp.y < tile_size && i < H && j < W) n_inside = min(min((uint32_t)PX, tile_size - tp.x), W - j);
     const float px0 = (float)j + 0.5f, py = (float)i + 0.5f;
     const float rs = rs_time[cam];
     const float roll = rs * ((py - 0.5f) / (float)(H - 1) - 0.5f);
@@ -388,144 +531,180 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM)) rasterize_to_pixels_fwd_kerne
     const float roll_a = rs * ((float)(ty * tile_size) / (float)(H - 1) - 0.5f);
     const float roll_b = rs * ((float)(min((ty + 1) * tile_size, H) - 1) / (float)(H - 1) - 0.5f);
     const float roll_lo = fminf(roll_a, roll_b), roll_hi = fmaxf(roll_a, roll_b);
-    patch_boxes<2>(s_box, px0, py, n_inside);
+    const PatchBox box = warp_box(px0, py, n_inside);
 
-    const TileRange range = tile_range(offsets, blockIdx.x, C * tiles_per_cam, n_isects);
-    const uint32_t num_batches = (uint32_t)(range.end - range.start + bs - 1) / bs;
+    const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
 
-    float2 px = make_float2(n_inside > 0 ? px0 : kPixelGone, n_inside > 1 ? px0 + 1.f : kPixelGone);
-    float2 T = make_float2(1.f, 1.f);
-    constexpr uint32_t kNoEntry = 0xffffffffu;
-    int32_t pos0 = 0, pos1 = 0;   // list position of the last entry blended
-    float out[2][CDIM];
+    float2 npx[P2], T[P2], out[CDIM][P2];   // minus the columns; transmittances; minus the colours, by channel
+    uint32_t blended[PX];                   // entries of the batch, one bit each
+    int32_t pos[PX];                        // list position of the last entry blended
 #pragma unroll
-    for (int k = 0; k < CDIM; ++k) out[0][k] = out[1][k] = 0.f;
+    for (int q = 0; q < P2; ++q) {
+        npx[q] = make_float2(n_inside > 2u * q ? -(px0 + (float)(2 * q)) : -kPixelGone,
+                             n_inside > 2u * q + 1u ? -(px0 + (float)(2 * q + 1)) : -kPixelGone);
+        T[q] = make_float2(1.f, 1.f);
+#pragma unroll
+        for (int c = 0; c < CDIM; ++c) out[c][q] = make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < PX; ++k) pos[k] = 0;
+    const bool together = CDIM >= 20 && vec;   // see copy_rows()
+    if (together)
+        for (uint32_t k = channels; k < (uint32_t)CDIM; ++k) reinterpret_cast<float *>(sCol)[lane * CDIM + k] = 0.f;
     uint32_t odd = 0u;   // kOddEntry: the warp was to blend one
-    bool warp_done = __all_sync(0xffffffffu, n_inside == 0);
+    bool done = __all_sync(0xffffffffu, n_inside == 0);
 
     int32_t next_id = 0;
-    if (range.start + (int32_t)tr < range.end) next_id = flatten_ids[range.start + tr];
-    for (uint32_t b = 0; b < num_batches; ++b) {
-        if (__syncthreads_and(warp_done)) break;
-        const int32_t idx = range.start + (int32_t)(bs * b + tr);
+    if (range.start + (int32_t)lane < range.end) next_id = flatten_ids[range.start + lane];
+    for (int32_t start = range.start; start < range.end && !done; start += 32) {
+        const int32_t idx = start + (int32_t)lane;
         const int32_t g = next_id;
+        uint32_t seen = 0u;
         PixelEntry e;
-        e.seen = 0u;
         if (idx < range.end) {
             e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
-            if (idx + (int32_t)bs < range.end) next_id = flatten_ids[idx + bs];   // on its way meanwhile
-            e.seen = warps_that_see<true>(e, s_box, n_warps, roll_lo, roll_hi);
+            if (idx + 32 < range.end) next_id = flatten_ids[idx + 32];   // on its way meanwhile
+            seen = patch_sees<true>(e, box, roll_lo, roll_hi);
         }
-        // compact the survivors to the front of the staging arrays, list order kept
-        const uint32_t kept_mask = __ballot_sync(0xffffffffu, e.seen != 0u);
-        if (lane == 0) s_warp_kept[warp] = __popc(kept_mask);
-        __syncthreads();
-        uint32_t pos = __popc(kept_mask & ((1u << lane) - 1u)), n_kept = 0;
-        for (uint32_t w = 0; w < n_warps; ++w) {
-            const uint32_t cnt = s_warp_kept[w];
-            if (w < warp) pos += cnt;
-            n_kept += cnt;
+        uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
+        const uint32_t careful = __ballot_sync(0xffffffffu, seen > kSeenEntry);
+        odd |= seen;
+        __syncwarp();   // the batch before has been read
+        if (seen) {
+            sA[lane] = e.A;
+            sB[lane] = scaled_conic(make_float4(e.B.x, e.B.y, e.B.z, -e.B.w));
+            if (!together) stage_whole_row<CDIM>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, vec);
         }
-        if (e.seen) {
-            sA[pos] = e.A;
-            sB[pos] = scaled_conic(e.B);
-            sPos[pos] = idx;
-            sSeen[pos] = e.seen;
-            float *row = sCol + pos * CDIM;
-            stage_row(row, colors, (size_t)g, channels, vec);
-            for (uint32_t k = (channels + 3u) & ~3u; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
-        }
-        __syncthreads();
-        if (warp_done) continue;
-        uint32_t last0 = kNoEntry, last1 = kNoEntry;   // this batch's
-        for (uint32_t t0 = 0; t0 < n_kept && !warp_done; t0 += 32) {
-            const uint32_t mine = t0 + lane;
-            const uint32_t seen = mine < n_kept ? sSeen[mine] : 0u;
-            uint32_t todo = __ballot_sync(0xffffffffu, (seen >> warp) & 1u);
-            odd |= seen;
-            while (todo) {
-                const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
-                todo &= todo - 1u;
-                const float4 A = sA[t], B = sB[t];
-                const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
-                const float2 dx = __fadd2_rn(make_float2(mx, mx), make_float2(-px.x, -px.y));
-                const float2 pw = pair_power(B.x, dx, B.y * dy, B.z * dy * dy);
-                const float2 av = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
-                bool ok0 = pw.x <= 0.f && av.x >= kAlphaMin, ok1 = pw.y <= 0.f && av.y >= kAlphaMin;
-                if (!__any_sync(0xffffffffu, ok0 || ok1)) continue;
-                const float2 alpha = make_float2(ok0 ? fminf(kAlphaMax, av.x) : 0.f, ok1 ? fminf(kAlphaMax, av.y) : 0.f);
-                const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
-                float2 next_T = __fmul2_rn(T, om);
-                float2 vis = __fmul2_rn(alpha, T);
-                // T stays above the limit, so only a blended entry can take a pixel below it; few entries do
-                if (__any_sync(0xffffffffu, fminf(next_T.x, next_T.y) <= kTStop)) {
-                    if (next_T.x <= kTStop) { px.x = kPixelGone; vis.x = 0.f; next_T.x = T.x; ok0 = false; }
-                    if (next_T.y <= kTStop) { px.y = kPixelGone; vis.y = 0.f; next_T.y = T.y; ok1 = false; }
-                    warp_done = __all_sync(0xffffffffu, px.x == kPixelGone && px.y == kPixelGone);
-                    if (warp_done) todo = 0u;
+        if (together) copy_rows<CDIM, false>(reinterpret_cast<float *>(sCol), colors, g, todo, channels, lane);
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < PX; ++k) blended[k] = 0u;
+        while (todo) {
+            const uint32_t t = (uint32_t)__ffs(todo) - 1u, bit = 1u << t;
+            todo ^= bit;
+            const float4 A = sA[t], B = sB[t];
+            const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
+            const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
+            float2 w[P2];   // minus the alphas, then minus the weights
+#pragma unroll
+            for (int q = 0; q < P2; ++q) {
+                const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
+                w[q] = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
+            }
+            if (careful & bit) {
+#pragma unroll
+                for (int q = 0; q < P2; ++q) {
+                    const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
+                    w[q].x = pw.x <= 0.f ? fmaxf(-kAlphaMax, w[q].x) : 0.f;
+                    w[q].y = pw.y <= 0.f ? fmaxf(-kAlphaMax, w[q].y) : 0.f;
                 }
-                if (ok0) last0 = t;
-                if (ok1) last1 = t;
-                T = next_T;
-                const float4 *row = reinterpret_cast<const float4 *>(sCol + t * CDIM);
-                const float2 w0 = make_float2(vis.x, vis.x), w1 = make_float2(vis.y, vis.y);
+            }
+            float low = 1.f;
 #pragma unroll
-                for (int k = 0; k < CDIM; k += 4) {
-                    const float4 c4 = row[k / 4];
+            for (int q = 0; q < P2; ++q) {
+                const bool ok0 = w[q].x <= -kAlphaMin, ok1 = w[q].y <= -kAlphaMin;
+                if (ok0) blended[2 * q] |= bit;
+                if (ok1) blended[2 * q + 1] |= bit;
+                const float2 alpha = make_float2(ok0 ? w[q].x : 0.f, ok1 ? w[q].y : 0.f);
+                w[q] = __fmul2_rn(alpha, T[q]);
+                T[q] = __ffma2_rn(alpha, T[q], T[q]);
+                low = fminf(low, fminf(T[q].x, T[q].y));
+            }
+            // T stays above the limit, so only a blended entry can take a pixel below it; few entries do
+            if (__any_sync(0xffffffffu, low <= kTStop)) {
+                bool gone = true;
 #pragma unroll
-                    for (int h = 0; h < 4; h += 2) {
-                        const float2 c2 = h ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
-                        const float2 a = __ffma2_rn(c2, w0, make_float2(out[0][k + h], out[0][k + h + 1]));
-                        const float2 d = __ffma2_rn(c2, w1, make_float2(out[1][k + h], out[1][k + h + 1]));
-                        out[0][k + h] = a.x; out[0][k + h + 1] = a.y;
-                        out[1][k + h] = d.x; out[1][k + h + 1] = d.y;
+                for (int q = 0; q < P2; ++q) {
+                    if (T[q].x <= kTStop) { npx[q].x = -kPixelGone; T[q].x -= w[q].x; w[q].x = 0.f; blended[2 * q] &= ~bit; }
+                    if (T[q].y <= kTStop) { npx[q].y = -kPixelGone; T[q].y -= w[q].y; w[q].y = 0.f; blended[2 * q + 1] &= ~bit; }
+                    gone = gone && npx[q].x == -kPixelGone && npx[q].y == -kPixelGone;
+                }
+                done = __all_sync(0xffffffffu, gone);
+                if (done) todo = 0u;
+            }
+#pragma unroll
+            for (int c = 0; c < CDIM; c += 4) {
+                const float4 c4 = sCol[t * (CDIM / 4) + c / 4];
+#pragma unroll
+                for (int q = 0; q < P2; ++q) {
+                    out[c][q] = __ffma2_rn(make_float2(c4.x, c4.x), w[q], out[c][q]);
+                    out[c + 1][q] = __ffma2_rn(make_float2(c4.y, c4.y), w[q], out[c + 1][q]);
+                    out[c + 2][q] = __ffma2_rn(make_float2(c4.z, c4.z), w[q], out[c + 2][q]);
+                    out[c + 3][q] = __ffma2_rn(make_float2(c4.w, c4.w), w[q], out[c + 3][q]);
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < PX; ++k)
+            if (blended[k]) pos[k] = start + 31 - __clz(blended[k]);
+    }
+    const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
+    const size_t pix = ((size_t)cam * H + i) * W + j;
+    float none = 0.f;   // a NaN: see odd_pixels_fwd()
+    if constexpr (CDIM == 4) {
+        float alphas[PX], depths[PX], v[PX][CDIM];
+#pragma unroll
+        for (int h = 0; h < PX; ++h) {
+            const float Tk = h & 1 ? T[h / 2].y : T[h / 2].x;
+            alphas[h] = 1.f - Tk;
+            depths[h] = 0.f;
+#pragma unroll
+            for (int k = 0; k < CDIM; ++k) {
+                v[h][k] = -(h & 1 ? out[k][h / 2].y : out[k][h / 2].x);
+                none = fmaf(v[h][k], 0.f, none);
+                if (bg && (uint32_t)k < channels) v[h][k] += Tk * bg[k];
+                if (expected && (uint32_t)k + 1u == channels) depths[h] = v[h][k] /= fmaxf(1.f - Tk, kExpectedMin);
+            }
+        }
+        if (n_inside) {
+            store_pixels<PX>(render_alphas + pix, alphas, n_inside);
+            store_pixels<PX>(last_ids + pix, pos, n_inside);
+            store_channels<CDIM, PX>(render_colors + pix * channels, v, channels, n_inside);
+            if (expected && expected_depths != nullptr) store_pixels<PX>(expected_depths + pix, depths, n_inside);
+        }
+    } else {   // one pixel after the other: all at once costs the 16-channel kernel 13 us in registers
+        const bool drawn_together = together && (reinterpret_cast<uintptr_t>(render_colors) & 15u) == 0u;
+        float4 *row = sCol + lane * (CDIM / 4);
+#pragma unroll
+        for (int h = 0; h < PX; ++h) {
+            const float Tk = h & 1 ? T[h / 2].y : T[h / 2].x;
+            const bool in = (uint32_t)h < n_inside;
+            if (in) {
+                render_alphas[pix + h] = 1.f - Tk;
+                last_ids[pix + h] = pos[h];
+            }
+            if (drawn_together) __syncwarp();
+#pragma unroll
+            for (int k = 0; k < CDIM; k += 4) {
+                float v[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    v[c] = -(h & 1 ? out[k + c][h / 2].y : out[k + c][h / 2].x);
+                    none = fmaf(v[c], 0.f, none);
+                    if (in && (uint32_t)(k + c) < channels) {
+                        if (bg) v[c] += Tk * bg[k + c];
+                        if (expected && (uint32_t)(k + c) + 1u == channels) {
+                            v[c] /= fmaxf(1.f - Tk, kExpectedMin);
+                            if (expected_depths != nullptr) expected_depths[pix + h] = v[c];
+                        }
+                        if (!drawn_together) render_colors[(pix + h) * channels + k + c] = v[c];
                     }
                 }
+                if (drawn_together) row[k / 4] = make_float4(v[0], v[1], v[2], v[3]);
+            }
+            if (drawn_together) {
+                const uint32_t drawn = __ballot_sync(0xffffffffu, in);
+                __syncwarp();
+                copy_rows<CDIM, true>(reinterpret_cast<float *>(sCol), render_colors + (size_t)cam * H * W * channels, (int32_t)(i * W + j) + h,
+                                      drawn, channels, lane);
             }
         }
-        // staged place -> list position
-        if (last0 != kNoEntry) pos0 = sPos[last0];
-        if (last1 != kNoEntry) pos1 = sPos[last1];
-    }
-    const bool vec_out = channels == 4u && (reinterpret_cast<uintptr_t>(render_colors) & 15u) == 0u;
-    const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
-    float none = 0.f;   // a NaN: see odd_pixels_fwd()
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        if ((uint32_t)h >= n_inside) break;
-        const size_t pix = ((size_t)cam * H + i) * W + j + h;
-        const float Tk = h ? T.y : T.x;
-        render_alphas[pix] = 1.f - Tk;
-        last_ids[pix] = h ? pos1 : pos0;
-        float *dst = render_colors + pix * channels;
-#pragma unroll
-        for (int k = 0; k < CDIM; ++k) none = fmaf(out[h][k], 0.f, none);
-        if (CDIM == 4 && vec_out) {   // one 16-byte store per pixel
-            float4 v = make_float4(out[h][0], out[h][1], out[h][2], out[h][3]);
-            if (bg) v = make_float4(v.x + Tk * bg[0], v.y + Tk * bg[1], v.z + Tk * bg[2], v.w + Tk * bg[3]);
-            if (expected) v.w /= fmaxf(1.f - Tk, kExpectedMin);
-            if (expected_depths != nullptr) expected_depths[pix] = v.w;
-            *reinterpret_cast<float4 *>(dst) = v;
-            continue;
-        }
-#pragma unroll
-        for (int k = 0; k < CDIM; ++k)
-            if ((uint32_t)k < channels) {
-                float v = bg ? out[h][k] + Tk * bg[k] : out[h][k];
-                if (expected && (uint32_t)k + 1u == channels) {
-                    v /= fmaxf(1.f - Tk, kExpectedMin);
-                    if (CDIM <= 8 && expected_depths != nullptr) expected_depths[pix] = v;
-                }
-                dst[k] = v;
-            }
-        // (up to eight channels kept above, more of them here: what the compiler spills in the loop over the entries
-        // depends on it - 222 and 179 us, the other way round 226 and 197)
-        if (CDIM > 8 && expected_depths != nullptr) expected_depths[pix] = dst[channels - 1];
+        __syncwarp();   // odd_pixels_fwd() may write again what other lanes wrote
     }
     if (__any_sync(0xffffffffu, odd >= kOddEntry) || none != 0.f) {
         const PixelTask task = {C, W, H, tile_size, tile_w, tile_h, channels, n_isects, means2d, pix_vels, conics, opacities,
                                 colors, rs_time, backgrounds, offsets, flatten_ids};
-        odd_pixels_fwd<2>(task, render_colors, render_alphas, last_ids, expected != 0u, expected_depths);
+        odd_pixels_fwd<PX>(task, gtile, tr, render_colors, render_alphas, last_ids, expected != 0u, expected_depths);
     }
 }
 
@@ -1106,26 +1285,15 @@ __device__ __forceinline__ SumSlot sum_slot(uint32_t lane) {
     return r;
 }
 
-__device__ __forceinline__ int block_max_int(int v, int *red /* [32] */) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, off));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    int m = red[0];
-    for (uint32_t w = 1; w < (blockDim.x + 31) / 32; ++w) m = max(m, red[w]);
-    __syncthreads();
-    return m;
-}
-
 // What a lane does with the warp total it ends up holding: which array it belongs to, and the factor
-// common to all pixels (times the entry's opacity where the derivative runs through sigma).
+// common to all samples (times one of the entry's own, see the kernels).
 struct GradSlot {
     float *base;
     uint32_t stride;
     float scale;
-    bool times_opacity;
-    __device__ __forceinline__ void add(size_t g, float total, float opacity, bool writes) const {
-        const float v = total * (times_opacity ? scale * opacity : scale);
+    bool times_factor;
+    __device__ __forceinline__ void add(size_t g, float total, float factor, bool writes) const {
+        const float v = total * (times_factor ? scale * factor : scale);
         if (writes && base != nullptr && v != 0.f) atomicAdd(base + g * stride, v);
     }
 };
@@ -1136,44 +1304,52 @@ __device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t
                                                     float *v_opacities, float *v_means2d_abs) {
     if (slot < cdim) return {(uint32_t)slot < channels ? v_colors + slot : nullptr, channels, 1.f, false};
     switch (slot - cdim) {
-        case 0: return {v_conics, 3u, -0.5f, true};
-        case 1: return {v_conics + 1, 3u, -1.f, true};
-        case 2: return {v_conics + 2, 3u, -0.5f, true};
-        case 3: return {v_means2d, 2u, kLn2, true};
-        case 4: return {v_means2d + 1, 2u, kLn2, true};
-        case 5: return {v_pix_vels, 2u, kLn2, true};
-        case 6: return {v_pix_vels + 1, 2u, kLn2, true};
-        case 7: return {v_opacities, 1u, 1.f, false};
-        case 8: return {kAbs ? v_means2d_abs : nullptr, 2u, kLn2, true};
-        case 9: return {kAbs ? v_means2d_abs + 1 : nullptr, 2u, kLn2, true};
+        case 0: return {v_conics, 3u, -0.5f, false};
+        case 1: return {v_conics + 1, 3u, -1.f, false};
+        case 2: return {v_conics + 2, 3u, -0.5f, false};
+        case 3: return {v_means2d, 2u, kLn2, false};
+        case 4: return {v_means2d + 1, 2u, kLn2, false};
+        case 5: return {v_pix_vels, 2u, kLn2, false};
+        case 6: return {v_pix_vels + 1, 2u, kLn2, false};
+        case 7: return {v_opacities, 1u, 1.f, true};   // by the opacity
+        case 8: return {kAbs ? v_means2d_abs : nullptr, 2u, kLn2, false};
+        case 9: return {kAbs ? v_means2d_abs + 1 : nullptr, 2u, kLn2, false};
         default: return {nullptr, 0u, 0.f, false};
     }
 }
 
 // ---------------------------------------------------------------------------------------
-// Camera backward: back to front from the last entry any pixel of the tile consumed.
+// Camera backward: back to front from the last entry any pixel of the patch consumed; patches as in the forward kernel.
 //
-// What bounds it is instruction issue, and the parts that do not depend on the pixel were most of it:
-// with one pixel per thread the 14 warp totals of an entry took as many instructions as the gradients
-// themselves. So a thread takes four pixels of a row (two with more than 8 channels), adds their terms
-// up before anything is exchanged, and as dy and the row's shutter time are common to them it needs only
-// the sums of v, v dx and v dx^2 (v = exp(-sigma) dL/dalpha). The channels behind an entry enter through
-// one number per pixel: dL/dalpha = T (c . g) - (1 / (1 - alpha)) (sum over the entries behind of
-// their weight times their (c . g)), g the pixel's cotangent - a running scalar in place of a running colour.
-// Camera benchmark's training step: 1.55 -> 0.40 ms.
+// What bounds it is instruction issue, the FP32 pipe at half its rate, and sixteen warps an SM to hide the way from the
+// exponentials through the reciprocals to the sums. The parts that do not depend on the pixel - the butterflies above all -
+// were most of it with one pixel per thread; eight pixels of a row (four above four channels, two above sixteen) add their
+// terms up before anything is exchanged, and as dy and the row's shutter time are common to them the geometry needs only
+// the sums of v, v dx and v dx^2 (v = alpha dL/dalpha; the opacity's own derivative is the first of them by the opacity). The
+// channels behind an entry enter through one number per pixel: dL/dalpha = T (c . g) - (1 / (1 - alpha)) (sum over
+// the entries behind of their weight times their (c . g)), g the pixel's cotangent - a running scalar in place of a running
+// colour. A pixel lies far out until its last entry comes, which takes a look at few entries of a list instead of a
+// comparison per pixel and entry. The pairs are worked through in one straight line: a branch for the entries that need
+// care between them costs 7 us.
+// 1920 x 1080, 4 channels: 323 M -> 200 M warp instructions, 398 -> 312 us (four pixels 367); 16 channels and absolute
+// gradients, 1237 x 719: 445 -> 374 (1920 x 1080 without: 4, 8, 13, 20 and 32 channels 401, 496, 861, 948, 2000 -> 312, 483, 703, 847, 1940;
+// 640 x 360, two pixels: 159, 174, 136, 148, 282 -> 106, 115, 137, 140, 312). Sums through shared memory instead of butterflies: 361; asynchronous copies
+// of the next batches: 9 us more. The atomics cost 14 us, the butterflies 40.
 // ---------------------------------------------------------------------------------------
-// registers per thread, by measurement: more warps pay up to a few spilled words (4 channels: 421 us at 100
-// registers, 370 at 80, 384 at 64)
-constexpr int pixels_bwd_regs(int cdim) { return cdim <= 4 ? 80 : cdim <= 20 ? 96 : 168; }
+// registers per thread, by measurement (4 channels, eight pixels: 335 us at 128, 348 at 112, 361 at 144; 16 channels:
+// 386 at 168, 394 at 128; 8: 483 at 96, 520 at 128; 20, four pixels: 847 at 168, 980 at 200; 32: 1950 at 128, 2075 at 160)
+constexpr int pixels_bwd_regs(int cdim, int px) {
+    return cdim <= 4 ? (px == 8 ? 128 : px == 4 ? 80 : 72) : cdim <= 8 ? (px == 4 ? 96 : 88) : cdim <= 16 ? (px == 4 ? 168 : 104) : cdim <= 20 ? 168 : 128;
+}
 
 template <int CDIM, int PX, bool kAbs>
-__global__ void __maxnreg__(pixels_bwd_regs(CDIM))
+__global__ void __maxnreg__(pixels_bwd_regs(CDIM, PX))
 rasterize_to_pixels_bwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
     const float *__restrict__ opacities, const float2 *__restrict__ pix_vels,
     const float *__restrict__ rs_time, const float *__restrict__ backgrounds, uint32_t W,
-    uint32_t H, uint32_t tile_size, uint32_t tile_w, uint32_t tile_h,
+    uint32_t H, uint32_t tile_size, uint32_t tile_w, uint32_t tile_h, uint32_t patches /* of a tile */,
     const int32_t *__restrict__ offsets, const int32_t *__restrict__ flatten_ids,
     const float *__restrict__ render_alphas, const int32_t *__restrict__ last_ids,
     const float *__restrict__ v_render_colors, const float *__restrict__ v_render_alphas,
@@ -1183,27 +1359,20 @@ rasterize_to_pixels_bwd_kernel(
     chain_enter();
     static_assert(PX % 2 == 0, "pixels are handled in pairs");
     constexpr int P2 = PX / 2;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int red[32];
-    __shared__ uint32_t s_warp_kept[32];
-    __shared__ PatchBox s_box[16];
-    const uint32_t bs = blockDim.x;
-    float4 *sA = reinterpret_cast<float4 *>(smem_raw);
-    float4 *sB = sA + bs;
-    float *sRgb = reinterpret_cast<float *>(sB + bs);                  // [bs * CDIM], zeros behind the channels
-    int32_t *sId = reinterpret_cast<int32_t *>(sRgb + bs * CDIM);
-    int32_t *sPos = sId + bs;                                          // list position of the staged entry
-    uint32_t *sSeen = reinterpret_cast<uint32_t *>(sPos + bs);         // warps that may see it
+    __shared__ float4 sA[32];                // x, y, vx, vy
+    __shared__ float4 sB[32];                // scaled conic, opacity
+    __shared__ float4 sCol[32 * CDIM / 4];   // zeros behind the channels
+    __shared__ float2 sId[32];               // Gaussian, 1 / opacity
+    __shared__ int32_t sLast[PX][32];        // last list positions of the lanes' pixels
 
     const uint32_t tiles_per_cam = tile_w * tile_h;
-    const uint32_t cam = blockIdx.x / tiles_per_cam;
-    const uint32_t tile = blockIdx.x - cam * tiles_per_cam;
+    const uint32_t gtile = blockIdx.x / patches, cam = gtile / tiles_per_cam;
+    const uint32_t tile = gtile - cam * tiles_per_cam;
     const uint32_t ty = tile / tile_w, tx = tile - ty * tile_w;
-    const uint32_t tr = threadIdx.x, lane = tr & 31, warp = tr >> 5, n_warps = bs >> 5;
+    const uint32_t lane = threadIdx.x, tr = (blockIdx.x - gtile * patches) * 32u + lane;
     const TilePixels<PX> tp = tile_pixels<PX>(tile_size, tr);
     const uint32_t i = ty * tile_size + tp.y, j = tx * tile_size + tp.x;
-    // pixels of this thread inside the tile and the image
-    uint32_t n_inside = 0;
+    uint32_t n_inside = 0;   // pixels of this thread inside the tile and the image
     if (tp.y < tile_size && i < H && j < W) n_inside = min(min((uint32_t)PX, tile_size - tp.x), W - j);
     const float px0 = (float)j + 0.5f, py = (float)i + 0.5f;
     const float rs = rs_time[cam];
@@ -1212,57 +1381,61 @@ rasterize_to_pixels_bwd_kernel(
     const float roll_a = rs * ((float)(ty * tile_size) / (float)(H - 1) - 0.5f);
     const float roll_b = rs * ((float)(min((ty + 1) * tile_size, H) - 1) / (float)(H - 1) - 0.5f);
     const float roll_lo = fminf(roll_a, roll_b), roll_hi = fmaxf(roll_a, roll_b);
-    patch_boxes<PX>(s_box, px0, py, n_inside);
+    const PatchBox box = warp_box(px0, py, n_inside);
 
-    const TileRange range = tile_range(offsets, blockIdx.x, C * tiles_per_cam, n_isects);
+    const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
     const bool vec = (channels % 4u == 0u) && ((reinterpret_cast<uintptr_t>(colors) & 15u) == 0u);
 
+    float2 npx[P2];                  // minus the columns; far out before a pixel's last entry has come
     float2 T[P2], behind[P2];        // transmittance in front of the entry; weighted (c . g) behind it
-    float v_out[PX][CDIM];           // cotangents of the pixels' channels
-    int32_t bin_final[PX];
+    float2 v_out[CDIM][P2];          // cotangents of the pixels' channels
     int32_t thread_last = -1;
     float none = 0.f;                // a NaN: see odd_pixels_bwd()
+    {
+        const size_t pix = ((size_t)cam * H + (n_inside ? i : 0u)) * W + (n_inside ? j : 0u);
+        float a_final[PX], v_a[PX], depths[PX], v[PX][CDIM];
+        int32_t last[PX];
+        load_pixels<PX>(a_final, render_alphas + pix, n_inside, 0.f);
+        load_pixels<PX>(v_a, v_render_alphas + pix, n_inside, 0.f);
+        load_pixels<PX>(last, last_ids + pix, n_inside, -1);
+        load_channels<CDIM, PX>(v, v_render_colors + pix * channels, channels, n_inside);
+        if (expected != nullptr) load_pixels<PX>(depths, expected + pix, n_inside, 0.f);
 #pragma unroll
-    for (int k = 0; k < PX; ++k) {
-        const bool in = (uint32_t)k < n_inside;
-        const size_t pix = ((size_t)cam * H + (in ? i : 0u)) * W + (in ? j + k : 0u);
-        const float a_final = in ? render_alphas[pix] : 0.f, T_final = 1.f - a_final;
-        bin_final[k] = in ? last_ids[pix] : -1;
-        thread_last = (in && bin_final[k] < 0) ? INT32_MAX : max(thread_last, bin_final[k]);
-        float v_a = in ? v_render_alphas[pix] : 0.f;
-        float bg_dot = 0.f;
-        const float divisor = fmaxf(a_final, kExpectedMin);
-        if (in && expected != nullptr && a_final >= kExpectedMin)
-            v_a -= v_render_colors[pix * channels + channels - 1] * expected[pix] / divisor;
+        for (int k = 0; k < PX; ++k) {
+            const bool in = (uint32_t)k < n_inside;
+            const float T_final = 1.f - a_final[k], divisor = fmaxf(a_final[k], kExpectedMin);
+            thread_last = (in && last[k] < 0) ? INT32_MAX : max(thread_last, last[k]);
+            sLast[k][lane] = last[k];
+            float bg_dot = 0.f;
 #pragma unroll
-        for (int c = 0; c < CDIM; ++c) {
-            v_out[k][c] = (in && (uint32_t)c < channels) ? v_render_colors[pix * channels + c] : 0.f;
-            if (expected != nullptr && (uint32_t)c + 1u == channels) v_out[k][c] /= divisor;
-            if (backgrounds != nullptr && (uint32_t)c < channels)
-                bg_dot += backgrounds[(size_t)cam * channels + c] * v_out[k][c];
-            none = fmaf(v_out[k][c], 0.f, none);
+            for (int c = 0; c < CDIM; ++c) {
+                if (expected != nullptr && (uint32_t)c + 1u == channels) {
+                    if (in && a_final[k] >= kExpectedMin) v_a[k] -= v[k][c] * depths[k] / divisor;
+                    v[k][c] /= divisor;
+                }
+                if (backgrounds != nullptr && (uint32_t)c < channels) bg_dot += backgrounds[(size_t)cam * channels + c] * v[k][c];
+                none = fmaf(v[k][c], 0.f, none);
+                if (k & 1) v_out[c][k / 2].y = v[k][c]; else v_out[c][k / 2].x = v[k][c];
+            }
+            // what the background and the alpha output receive through everything in front of them
+            const float to_last = -T_final * (v_a[k] - bg_dot);
+            none = fmaf(to_last, 0.f, none);
+            if (k & 1) { T[k / 2].y = T_final; behind[k / 2].y = to_last; npx[k / 2].y = -kPixelGone; }
+            else { T[k / 2].x = T_final; behind[k / 2].x = to_last; npx[k / 2].x = -kPixelGone; }
         }
-        // what the background and the alpha output receive through everything in front of them
-        const float last = -T_final * (v_a - bg_dot);
-        none = fmaf(last, 0.f, none);
-        if (k & 1) { T[k / 2].y = T_final; behind[k / 2].y = last; }
-        else { T[k / 2].x = T_final; behind[k / 2].x = last; }
     }
 
-    // last list position consumed by any pixel of this tile / warp
-    const int32_t tile_last = block_max_int(none != 0.f ? INT32_MAX : thread_last, red);
-    if (tile_last == INT32_MAX) {
+    // last list position consumed by any pixel of the patch
+    const int32_t warp_last = __reduce_max_sync(0xffffffffu, none != 0.f ? INT32_MAX : thread_last);
+    if (warp_last == INT32_MAX) {
         const PixelTask task = {C, W, H, tile_size, tile_w, tile_h, channels, n_isects, means2d, pix_vels, conics, opacities,
                                 colors, rs_time, backgrounds, offsets, flatten_ids};
         const PixelGrads grads = {render_alphas, v_render_colors, v_render_alphas, expected, last_ids, v_means2d,
                                   kAbs ? v_means2d_abs : nullptr, v_conics, v_colors, v_opacities, v_pix_vels};
-        odd_pixels_bwd<PX>(task, grads);
+        odd_pixels_bwd<PX>(task, gtile, tr, grads);
         return;
     }
-    const int32_t warp_last = __reduce_max_sync(0xffffffffu, thread_last);
-    const int32_t eff_end = min(range.end, tile_last + 1);
-    if (eff_end <= range.start) return;
-    const uint32_t num_batches = (uint32_t)(eff_end - range.start + bs - 1) / bs;
+    const int32_t eff_end = min(range.end, warp_last + 1);
 
     // Where the warp total that ends up on this lane goes: colours first, then the geometry.
     constexpr int kGeo = kAbs ? 10 : 8;
@@ -1272,149 +1445,148 @@ rasterize_to_pixels_bwd_kernel(
     const GradSlot slot_a = pixel_grad_slot<kAbs>(mine_a.value, CDIM, channels, v_colors,
                                                   v_conics, v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
 
+    int32_t waiting = thread_last;   // position of the next entry that is a pixel's of this lane last one; -1: none
+    bool pending = true;             // a lane of the warp waits for one
     int32_t next_id = 0;
-    {
-        const int32_t idx = eff_end - 1 - (int32_t)tr;
-        if (idx >= range.start) next_id = flatten_ids[idx];
-    }
-    for (uint32_t b = 0; b < num_batches; ++b) {
-        const int32_t batch_end = eff_end - 1 - (int32_t)(bs * b);
-        const int32_t idx = batch_end - (int32_t)tr;
+    if (eff_end - 1 - (int32_t)lane >= range.start) next_id = flatten_ids[eff_end - 1 - (int32_t)lane];
+    for (int32_t batch_end = eff_end - 1; batch_end >= range.start; batch_end -= 32) {
+        const int32_t idx = batch_end - (int32_t)lane;
         const int32_t g = next_id;
+        uint32_t seen = 0u;
         PixelEntry e;
-        e.seen = 0u;
         if (idx >= range.start) {
             e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
-            e.seen = warps_that_see<false>(e, s_box, n_warps, roll_lo, roll_hi);
-            const int32_t ahead = idx - (int32_t)bs;   // the id of the next batch's entry is on its way meanwhile
-            if (ahead >= range.start) next_id = flatten_ids[ahead];
+            if (idx - 32 >= range.start) next_id = flatten_ids[idx - 32];   // on its way meanwhile
+            seen = patch_sees<false>(e, box, roll_lo, roll_hi);
         }
-        // survivors to the front, still back to front in list order
-        const uint32_t kept_mask = __ballot_sync(0xffffffffu, e.seen != 0u);
-        __syncthreads();   // the batch before has been read
-        if (lane == 0) s_warp_kept[warp] = __popc(kept_mask);
-        __syncthreads();
-        uint32_t pos = __popc(kept_mask & ((1u << lane) - 1u)), n_kept = 0;
-        for (uint32_t w = 0; w < n_warps; ++w) {
-            const uint32_t cnt = s_warp_kept[w];
-            if (w < warp) pos += cnt;
-            n_kept += cnt;
+        uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
+        const uint32_t careful = __ballot_sync(0xffffffffu, seen > kSeenEntry);
+        __syncwarp();   // the batch before has been read
+        if (seen) {
+            sA[lane] = e.A;
+            sB[lane] = scaled_conic(e.B);
+            sId[lane] = make_float2(__int_as_float(g), 1.f / e.B.w);
+            if (CDIM <= 16) stage_whole_row<CDIM>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, vec);
+            else {   // (20 channels: all loads of a row at once take registers, 990 -> 1130 us)
+                float *row = reinterpret_cast<float *>(sCol) + lane * CDIM;
+                stage_row(row, colors, (size_t)g, channels, vec);
+                for (uint32_t k = (channels + 3u) & ~3u; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
+            }
         }
-        if (e.seen) {
-            sA[pos] = e.A;
-            sB[pos] = scaled_conic(e.B);
-            sId[pos] = g;
-            sPos[pos] = idx;
-            sSeen[pos] = e.seen;
-            float *row = sRgb + pos * CDIM;
-            stage_row(row, colors, (size_t)g, channels, vec);
-            for (uint32_t k = (channels + 3u) & ~3u; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
-        }
-        __syncthreads();
-        for (uint32_t t0 = 0; t0 < n_kept; t0 += 32) {
-            const uint32_t mine = t0 + lane;
-            uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u) && sPos[mine] <= warp_last);
-            while (todo) {
-                const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
-                todo &= todo - 1u;
-                const float4 A = sA[t], B = sB[t];
-                const int32_t entry = sPos[t];
-                const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
-                const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
-                float2 dx[P2], vis[P2], av[P2];
-                bool any = false;
+        __syncwarp();
+        while (todo) {
+            const uint32_t t = (uint32_t)__ffs(todo) - 1u, bit = 1u << t;
+            todo ^= bit;
+            const int32_t entry = batch_end - (int32_t)t;
+            if (pending && __any_sync(0xffffffffu, entry <= waiting)) {
+                // pixels whose last entry this is, or lay behind it: they take part from here on
+                int32_t next = -1;
+#pragma unroll
+                for (int k = 0; k < PX; ++k) {
+                    const int32_t last = sLast[k][lane];
+                    if (entry <= last) {
+                        if (k & 1) npx[k / 2].y = -(px0 + (float)k); else npx[k / 2].x = -(px0 + (float)k);
+                    } else next = max(next, last);
+                }
+                waiting = next;
+                pending = __any_sync(0xffffffffu, waiting >= 0);
+            }
+            const float4 A = sA[t], B = sB[t];
+            const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
+            const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
+            float4 col[CDIM / 4];
+#pragma unroll
+            for (int k = 0; k < CDIM / 4; ++k) col[k] = sCol[t * (CDIM / 4) + k];
+            float2 alpha[P2], v[P2], csum[CDIM];
+#pragma unroll
+            for (int q = 0; q < P2; ++q) {
+                const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
+                const float2 av = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
+                alpha[q] = make_float2(av.x >= kAlphaMin ? av.x : 0.f, av.y >= kAlphaMin ? av.y : 0.f);
+            }
+            uint32_t capped = 0u;   // pixels with a capped alpha, which passes no gradient on to the geometry
+            if (careful & bit) {
 #pragma unroll
                 for (int q = 0; q < P2; ++q) {
-                    dx[q] = make_float2(mx - (px0 + (float)(2 * q)), mx - (px0 + (float)(2 * q + 1)));
-                    const float2 pw = pair_power(B.x, dx[q], bdy, cdy2);
-                    const float2 ex = make_float2(exp2_approx(pw.x), exp2_approx(pw.y));
-                    av[q] = __fmul2_rn(make_float2(B.w, B.w), ex);
-                    const bool ok0 = pw.x <= 0.f && av[q].x >= kAlphaMin && entry <= bin_final[2 * q];
-                    const bool ok1 = pw.y <= 0.f && av[q].y >= kAlphaMin && entry <= bin_final[2 * q + 1];
-                    any = any || ok0 || ok1;
-                    if (!ok0) av[q].x = 0.f;
-                    if (!ok1) av[q].y = 0.f;
-                    // a capped alpha passes no gradient on to the geometry
-                    vis[q] = make_float2(ok0 && av[q].x <= kAlphaMax ? ex.x : 0.f, ok1 && av[q].y <= kAlphaMax ? ex.y : 0.f);
+                    const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
+                    if (alpha[q].x > kAlphaMax) capped |= 1u << (2 * q);
+                    if (alpha[q].y > kAlphaMax) capped |= 2u << (2 * q);
+                    alpha[q].x = pw.x <= 0.f ? fminf(kAlphaMax, alpha[q].x) : 0.f;
+                    alpha[q].y = pw.y <= 0.f ? fminf(kAlphaMax, alpha[q].y) : 0.f;
                 }
-                if (!__any_sync(0xffffffffu, any)) continue;
-                float sum[CDIM + kGeo];
-                float2 s0 = make_float2(0.f, 0.f), s1 = s0, s2 = s0, ax = s0, ay = s0;
-                float4 rgb[CDIM / 4];
+            }
 #pragma unroll
-                for (int k = 0; k < CDIM / 4; ++k) rgb[k] = reinterpret_cast<const float4 *>(sRgb + t * CDIM)[k];
+            for (int q = 0; q < P2; ++q) {
+                const float2 ra = reciprocal_pair(__fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha[q].x, -alpha[q].y)));
+                T[q] = __fmul2_rn(T[q], ra);
+                const float2 fac = __fmul2_rn(alpha[q], T[q]);
+                float2 dot = make_float2(0.f, 0.f);   // (c . g) of the two pixels
+#pragma unroll
+                for (int k = 0; k < CDIM; ++k) {
+                    const float4 c4 = col[k / 4];
+                    const float c = (k & 3) == 0 ? c4.x : (k & 3) == 1 ? c4.y : (k & 3) == 2 ? c4.z : c4.w;
+                    dot = k == 0 ? __fmul2_rn(make_float2(c, c), v_out[k][q]) : __ffma2_rn(make_float2(c, c), v_out[k][q], dot);
+                    csum[k] = q == 0 ? __fmul2_rn(fac, v_out[k][q]) : __ffma2_rn(fac, v_out[k][q], csum[k]);
+                }
+                const float2 v_alpha = __ffma2_rn(T[q], dot, __fmul2_rn(make_float2(-ra.x, -ra.y), behind[q]));
+                behind[q] = __ffma2_rn(fac, dot, behind[q]);
+                v[q] = __fmul2_rn(alpha[q], v_alpha);
+            }
+            if (capped) {
 #pragma unroll
                 for (int q = 0; q < P2; ++q) {
-                    const float2 alpha = make_float2(fminf(kAlphaMax, av[q].x), fminf(kAlphaMax, av[q].y));
-                    const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
-                    const float2 ra = reciprocal_pair(om);
-                    T[q] = __fmul2_rn(T[q], ra);
-                    const float2 fac = __fmul2_rn(alpha, T[q]);
-                    float2 dot;   // (c . g) of the two pixels
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const float *v = v_out[2 * q + h];
-                        const float f = h ? fac.y : fac.x;
-                        const float2 f2 = make_float2(f, f);
-                        float2 d2 = make_float2(0.f, 0.f);
-#pragma unroll
-                        for (int k = 0; k < CDIM; k += 2) {
-                            const float4 c4 = rgb[k / 4];
-                            const float2 c2 = (k & 2) ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
-                            const float2 v2 = make_float2(v[k], v[k + 1]);
-                            d2 = k == 0 ? __fmul2_rn(c2, v2) : __ffma2_rn(c2, v2, d2);
-                            const float2 acc = (q == 0 && h == 0) ? __fmul2_rn(f2, v2)
-                                                                  : __ffma2_rn(f2, v2, make_float2(sum[k], sum[k + 1]));
-                            sum[k] = acc.x; sum[k + 1] = acc.y;
-                        }
-                        if (h) dot.y = d2.x + d2.y; else dot.x = d2.x + d2.y;
-                    }
-                    const float2 nra = make_float2(-ra.x, -ra.y);
-                    const float2 v_alpha = __ffma2_rn(T[q], dot, __fmul2_rn(nra, behind[q]));
-                    behind[q] = __ffma2_rn(fac, dot, behind[q]);
-                    const float2 v = __fmul2_rn(vis[q], v_alpha), vx = __fmul2_rn(v, dx[q]);
-                    s0 = q == 0 ? v : __fadd2_rn(s0, v);
-                    s1 = q == 0 ? vx : __fadd2_rn(s1, vx);
-                    s2 = q == 0 ? __fmul2_rn(vx, dx[q]) : __ffma2_rn(vx, dx[q], s2);
-                    if (kAbs) {
-                        const float2 gx = __ffma2_rn(make_float2(2.f * B.x, 2.f * B.x), dx[q], make_float2(bdy, bdy));
-                        const float2 gy = __ffma2_rn(make_float2(B.y, B.y), dx[q], make_float2(2.f * B.z * dy, 2.f * B.z * dy));
-                        const float2 wx = __fmul2_rn(v, gx), wy = __fmul2_rn(v, gy);
-                        ax = __fadd2_rn(ax, make_float2(fabsf(wx.x), fabsf(wx.y)));
-                        ay = __fadd2_rn(ay, make_float2(fabsf(wy.x), fabsf(wy.y)));
-                    }
+                    if (capped & (1u << (2 * q))) v[q].x = 0.f;
+                    if (capped & (2u << (2 * q))) v[q].y = 0.f;
                 }
-                // sigma's derivatives: v_sigma = -opacity v; the factors that are the same for every
-                // pixel follow when the totals are written
-                const float m0 = s0.x + s0.y, m1 = s1.x + s1.y, my = dy * m0;
-                const float gx = 2.f * B.x * m1 + B.y * my, gy = B.y * m1 + 2.f * B.z * my;
-                sum[CDIM + 0] = s2.x + s2.y;
-                sum[CDIM + 1] = dy * m1;
-                sum[CDIM + 2] = dy * my;
-                sum[CDIM + 3] = gx;
-                sum[CDIM + 4] = gy;
-                sum[CDIM + 5] = gx * roll;
-                sum[CDIM + 6] = gy * roll;
-                sum[CDIM + 7] = m0;
-                if (kAbs) {
-                    sum[CDIM + 8] = ax.x + ax.y;
-                    sum[CDIM + 9] = ay.x + ay.y;
-                }
-                const size_t g = (size_t)sId[t];
-                float sums[kSums];
+            }
+            float2 s0 = make_float2(0.f, 0.f), s1 = s0, s2 = s0, ax = s0, ay = s0;
 #pragma unroll
-                for (int k = 0; k < kSums; ++k) sums[k] = sum[k];
-                slot_a.add(g, warp_sum_values<kSums, 16>(sums, lane), B.w, mine_a.writes);
-                if (kSplit) {
-                    float geo[kGeo];
-#pragma unroll
-                    for (int k = 0; k < kGeo; ++k) geo[k] = sum[CDIM + k];
-                    const float geo_total = warp_sum_values<kGeo, 16>(geo, lane);
-                    const SumSlot mine_b = sum_slot<kGeo>(lane);
-                    const GradSlot slot_b = pixel_grad_slot<kAbs>(CDIM + mine_b.value, CDIM, channels, v_colors, v_conics,
-                                                                  v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
-                    slot_b.add(g, geo_total, B.w, mine_b.writes);
+            for (int q = 0; q < P2; ++q) {
+                const float2 dx = __fadd2_rn(make_float2(mx, mx), npx[q]), vx = __fmul2_rn(v[q], dx);
+                s0 = q == 0 ? v[q] : __fadd2_rn(s0, v[q]);
+                s1 = q == 0 ? vx : __fadd2_rn(s1, vx);
+                s2 = q == 0 ? __fmul2_rn(vx, dx) : __ffma2_rn(vx, dx, s2);
+                if (kAbs) {   // (v first: a pixel that is far out must not meet a conic of any size)
+                    const float2 gx = __ffma2_rn(make_float2(2.f * B.x, 2.f * B.x), vx, __fmul2_rn(make_float2(bdy, bdy), v[q]));
+                    const float2 gy = __ffma2_rn(make_float2(B.y, B.y), vx, __fmul2_rn(make_float2(2.f * B.z * dy, 2.f * B.z * dy), v[q]));
+                    ax = __fadd2_rn(ax, make_float2(fabsf(gx.x), fabsf(gx.y)));
+                    ay = __fadd2_rn(ay, make_float2(fabsf(gy.x), fabsf(gy.y)));
                 }
+            }
+            // sigma's derivatives: v_sigma = -v; the factors that are the same for every
+            // pixel follow when the totals are written
+            float sum[CDIM + kGeo];
+#pragma unroll
+            for (int k = 0; k < CDIM; ++k) sum[k] = csum[k].x + csum[k].y;
+            const float m0 = s0.x + s0.y, m1 = s1.x + s1.y, my = dy * m0;
+            const float gx = 2.f * B.x * m1 + B.y * my, gy = B.y * m1 + 2.f * B.z * my;
+            sum[CDIM + 0] = s2.x + s2.y;
+            sum[CDIM + 1] = dy * m1;
+            sum[CDIM + 2] = dy * my;
+            sum[CDIM + 3] = gx;
+            sum[CDIM + 4] = gy;
+            sum[CDIM + 5] = gx * roll;
+            sum[CDIM + 6] = gy * roll;
+            sum[CDIM + 7] = m0;
+            if (kAbs) {
+                sum[CDIM + 8] = ax.x + ax.y;
+                sum[CDIM + 9] = ay.x + ay.y;
+            }
+            const float2 id = sId[t];
+            const size_t gg = (size_t)__float_as_int(id.x);
+            float sums[kSums];
+#pragma unroll
+            for (int k = 0; k < kSums; ++k) sums[k] = sum[k];
+            slot_a.add(gg, warp_sum_values<kSums, 16>(sums, lane), id.y, mine_a.writes);
+            if (kSplit) {
+                float geo[kGeo];
+#pragma unroll
+                for (int k = 0; k < kGeo; ++k) geo[k] = sum[CDIM + k];
+                const float geo_total = warp_sum_values<kGeo, 16>(geo, lane);
+                const SumSlot mine_b = sum_slot<kGeo>(lane);
+                const GradSlot slot_b = pixel_grad_slot<kAbs>(CDIM + mine_b.value, CDIM, channels, v_colors, v_conics,
+                                                              v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
+                slot_b.add(gg, geo_total, id.y, mine_b.writes);
             }
         }
     }
@@ -1886,6 +2058,27 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
 // spherical harmonics 437 us a frame chained, 411 apart; six cameras 3490 and 3370; 128 x 1800 lidar 294 and 289.
 // Below, the launch gap weighs more (640 x 360: 101 and 103).
 static bool fits_at_once(uint64_t blocks) { return blocks <= (uint64_t)kNumSMs * 8; }
+static bool warps_fit_at_once(uint64_t warps) { return fits_at_once(warps / 4); }
+
+// Pixels per lane of the camera kernels: more of them save instructions, fewer fill the machine. Measured over images
+// of 920 to 10800 tiles of 16 x 16 pixels, us with two / four / eight pixels. Forward, 4 channels: 920 tiles 49 / 70 / 119, 2040 57 /
+// 55 / 70, 2408 57 / 63 / 89, 3311 102 / 83 / 86, 4704 101 / 89 / 103, 7920 177 / 143 / 137, 10800 277 / 203 / 187; 8 channels: 2040
+// 68 / 76, 3510 127 / 114; 13 channels: 920 72 / 104, 2040 97 / 93, 3510 180 / 151. Backward, 4 channels: 920 106 / 154 / 255, 2040 138 /
+// 122 / 153, 3510 250 / 188 / 178, 8160 520 / 360 / 312; 8 and 13 channels: 920 115 / 165 and 137 / 188, 2040 166 / 152 and 226 / 200.
+// A tile whose rows leave lanes over takes fewer (8 x 8 tiles: 99 / 136 / 227; 24 x 24: 106 / 90 / 111).
+static uint32_t tiles_of_256(uint64_t blocks, uint32_t tile_size) {
+    return (uint32_t)(blocks * tile_size * tile_size / 256u < 0xffffffffull ? blocks * tile_size * tile_size / 256u : 0xffffffffull);
+}
+static uint32_t pixels_per_lane(uint32_t tiles, uint32_t four_from, uint32_t eight_from, uint32_t tile_size) {
+    if (tiles >= eight_from && tile_threads<8>(tile_size) % 32u == 0u) return 8u;
+    return tiles >= four_from && tile_threads<4>(tile_size) >= 32u ? 4u : 2u;
+}
+static uint32_t pixels_per_lane_fwd(uint64_t blocks, uint32_t tile_size, uint32_t channels) {
+    return pixels_per_lane(tiles_of_256(blocks, tile_size), channels <= 8 ? 2700u : 1500u, channels <= 4 ? 6000u : ~0u, tile_size);
+}
+static uint32_t pixels_per_lane_bwd(uint64_t blocks, uint32_t tile_size, uint32_t channels) {
+    return pixels_per_lane(tiles_of_256(blocks, tile_size), 1500u, channels <= 4 ? 3000u : ~0u, tile_size);
+}
 
 // Patches below which all warps of a CTA share one in the forward pass: the shared work costs more
 // instructions in all, so the patches must be too few to fill the machine. Apart and shared, us, 8 channels: 512
@@ -1951,25 +2144,27 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
                 SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_fwd: null input");
     const uint32_t blocks = C * tile_width * tile_height;
     if (blocks == 0 || image_width == 0 || image_height == 0) return SPLATAD_OK;
-    const uint32_t bs = ((tile_threads<2>(tile_size) + 31) / 32) * 32;   // whole warps
-#define CALL(D)                                                                                   \
+#define CALL_PX(D, P)                                                                             \
     {                                                                                             \
-        const size_t smem = (size_t)bs * (2 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float)); \
-        int rc = set_smem(rasterize_to_pixels_fwd_kernel<D>, smem, "rasterize_to_pixels_fwd");    \
-        if (rc != SPLATAD_OK) return rc;                                                          \
-        launch_chained_if(fits_at_once(blocks), rasterize_to_pixels_fwd_kernel<D>, blocks, bs, smem,  \
+        const uint32_t patches = div_up(tile_threads<P>(tile_size), 32);                          \
+        SPL_REQUIRE((uint64_t)blocks * patches <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_fwd: too many tiles"); \
+        launch_chained_if(warps_fit_at_once((uint64_t)blocks * patches), rasterize_to_pixels_fwd_kernel<D, P>, blocks * patches, 32, 0, \
             (cudaStream_t)stream,                                                                 \
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
-            image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
+            image_height, tile_size, tile_width, tile_height, patches, tile_offsets, flatten_ids, \
             render_colors, render_alphas, last_ids, (uint32_t)(expected_last_channel != 0),       \
             expected_last_channel ? expected_depths : nullptr);                                   \
     }
+#define CALL(D)                                                                                   \
+    if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2)) else if (D <= 16 && px == 4) CALL_PX(D, (D <= 16 ? 4 : 2)) else CALL_PX(D, 2)
+    const uint32_t px = pixels_per_lane_fwd(blocks, tile_size, channels);
     {
         SPL_PROF("rasterize_to_pixels_fwd_kernel", (cudaStream_t)stream);
         SPL_DISPATCH_CDIM(channels, CALL);
     }
 #undef CALL
+#undef CALL_PX
     return check_launch("rasterize_to_pixels_fwd");
 }
 
@@ -2015,29 +2210,29 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
                 "rasterize_to_pixels_bwd: a tile of %u pixels (%u threads at one per pixel) with %u channels is more "
                 "than the backward pass takes: use a smaller tile or at most 16 channels per call",
                 tile_size * tile_size, samples, channels);
-#define CALL_ABS(D, A)                                                                            \
+#define CALL_PX(D, P, A)                                                                          \
     {                                                                                             \
-        constexpr int kPx = D <= 8 ? 4 : 2;                                                       \
-        auto kernel = rasterize_to_pixels_bwd_kernel<D, kPx, A>;                                  \
-        const uint32_t bs = ((tile_threads<kPx>(tile_size) + 31) / 32) * 32;                      \
-        const size_t smem = (size_t)bs * (2 * sizeof(float4) + 3 * sizeof(int32_t) + D * sizeof(float)); \
-        int rc = set_smem(kernel, smem, "rasterize_to_pixels_bwd");                               \
-        if (rc != SPLATAD_OK) return rc;                                                          \
-        launch_chained(kernel, blocks, bs, smem, (cudaStream_t)stream,                            \
+        const uint32_t patches = div_up(tile_threads<P>(tile_size), 32);                          \
+        SPL_REQUIRE((uint64_t)blocks * patches <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_bwd: too many tiles"); \
+        launch_chained(rasterize_to_pixels_bwd_kernel<D, P, A>, blocks * patches, 32, 0, (cudaStream_t)stream, \
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
-            image_height, tile_size, tile_width, tile_height, tile_offsets, flatten_ids,          \
+            image_height, tile_size, tile_width, tile_height, patches, tile_offsets, flatten_ids, \
             render_alphas, last_ids, v_render_colors, v_render_alphas, v_means2d_abs, v_means2d,  \
             v_conics, v_colors, v_opacities, v_pix_vels, expected_depths);                        \
     }
+#define CALL_ABS(D, A)                                                                            \
+    if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2), A) else if (D <= 20 && px == 4) CALL_PX(D, (D <= 20 ? 4 : 2), A) else CALL_PX(D, 2, A)
 #define CALL(D)                                                                                   \
     if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)
+    const uint32_t px = pixels_per_lane_bwd(blocks, tile_size, channels);
     {
         SPL_PROF("rasterize_to_pixels_bwd_kernel", (cudaStream_t)stream);
         SPL_DISPATCH_CDIM(channels, CALL);
     }
 #undef CALL
 #undef CALL_ABS
+#undef CALL_PX
     return check_launch("rasterize_to_pixels_bwd");
 }
 

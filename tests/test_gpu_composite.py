@@ -384,6 +384,58 @@ def test_pixels_several_per_thread(ts, W, H, channels, absgrad):
         _grad_check(f"tile {ts} ch={channels} absgrad", leaves["means2d"].absgrad, ref["v_means2d_abs"])
 
 
+@pytest.mark.parametrize("C,ts,channels,absgrad", [(24, 16, 3, True), (43, 16, 4, False), (84, 16, 3, False), (86, 16, 4, True),
+                                                   (24, 16, 8, True), (43, 16, 7, False), (24, 16, 13, True), (24, 16, 20, False),
+                                                   (96, 24, 4, False), (96, 32, 2, True)])
+def test_pixels_of_many_tiles(C, ts, channels, absgrad):
+    """Frames of many tiles take four and eight pixels of a row per lane: images that end inside a tile, a row of 16-byte
+    pieces or a lane's pixels, opacities above the cap, and conics on either side of those whose alphas need care
+    (needles, and one that is not positive definite), forward and backward against the oracle."""
+    from oracle import composite
+    from splatad_b200 import ops
+    W, H = (127, 133) if C % 2 else (132, 131)
+    c = _camera_case(C, 120, W, H, ts, channels, 1000 * ts + channels)
+    for k, rho in enumerate((0.999, 0.99999, 0.9999999, 1.5)):   # 1 - rho^2 against 1e-5
+        a, b = c["conics"][:, 2 + k, 0], c["conics"][:, 2 + k, 2]
+        c["conics"][:, 2 + k, 1] = rho * torch.sqrt(a * b)
+    g = torch.Generator().manual_seed(3)
+    v_c, v_a = torch.randn(C, H, W, channels, generator=g), torch.randn(C, H, W, 1, generator=g)
+    keys = ("means2d", "conics", "colors", "opacities", "pix_vels")
+    args = [n(c[k]) for k in keys] + [n(c["rs"]), None, W, H, ts, c["offsets"], c["flatten_ids"]]
+    ref_f = composite.rasterize_to_pixels_fwd(*args, dtype=np.float64)
+    f32 = composite.rasterize_to_pixels_fwd(*args, amb_tol=1e-4)
+    same = (f32["last_ids"] == ref_f["last_ids"]) & ~f32["ambiguous"]
+    assert same.mean() > 0.9
+    # of a form that nearly vanishes or is negative somewhere, the sign and the size hang on the last bits: the pixels
+    # within reach of its rounding are left out (relative to its terms, as the kernel and the oracle sum them)
+    j, i = np.meshgrid(np.arange(W) + 0.5, np.arange(H) + 0.5)
+    roll = n(c["rs"])[:, None, None] * ((i - 0.5) / (H - 1) - 0.5)
+    for k in range(2, 6):
+        m, v, q = (n(c[key])[:, k].astype(np.float64) for key in ("means2d", "pix_vels", "conics"))
+        dx = m[:, 0, None, None] + roll * v[:, 0, None, None] - j
+        dy = m[:, 1, None, None] + roll * v[:, 1, None, None] - i
+        size = 0.5 * (q[:, 0, None, None] * dx * dx + q[:, 2, None, None] * dy * dy)
+        sigma = size + q[:, 1, None, None] * dx * dy
+        same &= ~((np.abs(sigma) < 1e-4 + 1e-5 * size) | ((size > 200.0) & (sigma < 10.0)))
+    assert same.mean() > 0.8
+    mask, mk = t(same[..., None].astype(np.float32)), same[..., None].astype(np.float64)
+    leaves = {k: t(c[k]).requires_grad_(True) for k in keys}
+    out_c, out_a = ops.rasterize_to_pixels(*(leaves[k] for k in keys), W, H, ts, t(c["offsets"], torch.int32),
+                                           t(c["flatten_ids"], torch.int32), t(c["rs"]), absgrad=absgrad)
+    f32["ambiguous"] = ~same
+    for got, want in ((out_c, f32["render_colors"]), (out_a, f32["render_alphas"])):
+        assert_close(f"pixels tile {ts} ch={channels}", n(got), want, 1e-4, 1e-5, mask=same[..., None])
+    torch.autograd.backward([out_c, out_a], [t(v_c) * mask, t(v_a) * mask])
+    ref = composite.rasterize_to_pixels_bwd(*args, ref_f["render_alphas"], ref_f["last_ids"], n(v_c) * mk, n(v_a) * mk,
+                                            absgrad=absgrad)
+    plain = np.r_[0:2, 6:120]   # the needles' own gradients are sums of large terms that cancel
+    for k in keys:
+        _grad_check(f"tile {ts} ch={channels} v_{k}", leaves[k].grad[:, plain], ref["v_" + k].reshape(leaves[k].shape)[:, plain])
+    if absgrad:
+        _grad_check(f"tile {ts} ch={channels} absgrad", leaves["means2d"].absgrad[:, plain],
+                    ref["v_means2d_abs"].reshape(C, 120, 2)[:, plain])
+
+
 @pytest.mark.parametrize("tw,th,H,W,channels,asum,absgrad", [(32, 8, 20, 130, 3, True, True), (8, 4, 9, 100, 17, False, False),
                                                              (5, 3, 10, 64, 9, True, False), (64, 16, 40, 96, 16, False, True),
                                                              (1, 1, 6, 40, 2, True, False), (32, 8, 130, 1024, 5, True, False),
