@@ -748,16 +748,19 @@ struct PointExtent {
         el0 = fminf(el0, el); el1 = fmaxf(el1, el);
         r0 = fminf(r0, roll); r1 = fmaxf(r1, roll);
     }
-    // the box of the whole warp, written by its first lane; no points: a negative half width
-    __device__ __forceinline__ void write_box(PointBox *box) {
+    // the box of the whole warp, in every lane; no points: a negative half width
+    __device__ __forceinline__ PointBox warp_box() {
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
             az0 = fminf(az0, __shfl_xor_sync(0xffffffffu, az0, off)); az1 = fmaxf(az1, __shfl_xor_sync(0xffffffffu, az1, off));
             el0 = fminf(el0, __shfl_xor_sync(0xffffffffu, el0, off)); el1 = fmaxf(el1, __shfl_xor_sync(0xffffffffu, el1, off));
             r0 = fminf(r0, __shfl_xor_sync(0xffffffffu, r0, off)); r1 = fmaxf(r1, __shfl_xor_sync(0xffffffffu, r1, off));
         }
-        if ((threadIdx.x & 31u) == 0u)
-            *box = {0.5f * (az0 + az1), 0.5f * (az1 - az0), 0.5f * (el0 + el1), 0.5f * (el1 - el0), r0, r1};
+        return {0.5f * (az0 + az1), 0.5f * (az1 - az0), 0.5f * (el0 + el1), 0.5f * (el1 - el0), r0, r1};
+    }
+    __device__ __forceinline__ void write_box(PointBox *box) {   // by the warp's first lane
+        const PointBox b = warp_box();
+        if ((threadIdx.x & 31u) == 0u) *box = b;
     }
 };
 
@@ -792,10 +795,16 @@ __device__ __forceinline__ void angle_range(float mean, float vel, float centre,
     if (lo < -180.f || hi > 180.f) { lo = -180.f; hi = 180.f; }
 }
 
-// Bit w: the entry may contribute to a point of box w.
+// Bit w: the entry may contribute to a point of box w; bit 16 + w: its angles may wrap between mean and point there, or its
+// alphas need looking at one by one (as kCarefulEntry for the cameras).
+constexpr uint32_t kCarefulShift = 16;
+
 __device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const PointBox *s_box, uint32_t n_boxes) {
     const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
     if (test.never) return 0u;
+    const float ac = e.B.x * e.B.z;
+    const bool plain = e.B.x > 1e-15f && e.B.z > 1e-15f && e.B.x < 1e15f && e.B.z < 1e15f && ac - e.B.y * e.B.y >= 1e-5f * ac &&
+                       e.B.w <= kAlphaMax;
     uint32_t seen = 0u;
     for (uint32_t w = 0; w < n_boxes; ++w) {
         const PointBox b = s_box[w];
@@ -803,20 +812,28 @@ __device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const Po
         float x_lo, x_hi, y_lo, y_hi;
         angle_range(e.A.x, e.A.z, b.az, b.az_half, b.roll_lo, b.roll_hi, x_lo, x_hi);
         angle_range(e.A.y, e.A.w, b.el, b.el_half, b.roll_lo, b.roll_hi, y_lo, y_hi);
-        if (!test.misses(x_lo, x_hi, y_lo, y_hi)) seen |= 1u << w;
+        if (test.misses(x_lo, x_hi, y_lo, y_hi)) continue;
+        seen |= 1u << w;
+        const float x_a = b.roll_lo * e.A.z, x_b = b.roll_hi * e.A.z, y_a = b.roll_lo * e.A.w, y_b = b.roll_hi * e.A.w;
+        const float x = fabsf(e.A.x + 0.5f * (x_a + x_b) - b.az) + b.az_half + 0.5f * fabsf(x_b - x_a);
+        const float y = fabsf(e.A.y + 0.5f * (y_a + y_b) - b.el) + b.el_half + 0.5f * fabsf(y_b - y_a);
+        if (!(plain && x < 179.9f && y < 179.9f)) seen |= 1u << (w + kCarefulShift);
     }
     return seen;
 }
 
-// Offset of an entry from a point and its exp(-sigma); sigma decides with alpha whether it is blended.
-struct PointFootprint { float dx, dy, sigma, vis; };
+// Offset of an entry from a point and its exp(-sigma) = 2^power; power decides with alpha whether it is blended. The conic
+// is scaled (scaled_conic()). Where nothing wraps the differences are rounded as angle_difference() rounds them.
+struct PointFootprint { float dx, dy, power, vis; };
 
+template <bool kWraps>
 __device__ __forceinline__ PointFootprint point_footprint(const float4 &A, const float4 &B, float roll, float az, float el) {
     PointFootprint f;
-    f.dx = angle_difference(A.x + roll * A.z, az);
-    f.dy = angle_difference(A.y + roll * A.w, el);
-    f.sigma = 0.5f * (B.x * f.dx * f.dx + B.z * f.dy * f.dy) + B.y * f.dx * f.dy;
-    f.vis = __expf(-f.sigma);
+    const float mx = fmaf(roll, A.z, A.x), my = fmaf(roll, A.w, A.y);
+    f.dx = kWraps ? angle_difference(mx, az) : (mx - az + 180.f) - 180.f;
+    f.dy = kWraps ? angle_difference(my, el) : (my - el + 180.f) - 180.f;
+    f.power = fmaf(fmaf(B.x, f.dx, B.y * f.dy), f.dx, B.z * f.dy * f.dy);
+    f.vis = exp2_approx(f.power);
     return f;
 }
 
@@ -840,12 +857,13 @@ __device__ __forceinline__ void stage_features(float *row, const float *__restri
 // Lidar forward. One point per lane; a warp looks only at the entries that can reach its patch (a ninth
 // of the (point, entry) pairs of a small scan contribute, two thirds of the benchmark's) and evaluates
 // two of them at a time, because what it waits for is the chain from the offsets through the exponential
-// to the transmittance. The rendered rows leave through shared memory: a beam's eight points
+// to the transmittance. The wrap of the angles, the sign of sigma and the cap of the alphas are looked at only where the
+// staging thread cannot rule them out (64 x 1083: 58 -> 53 us). The rendered rows leave through shared memory: a beam's eight points
 // are consecutive floats.
 // ---------------------------------------------------------------------------------------
 // entries per thread and batch (their loads overlap), while the shared memory of a batch stays small
 constexpr uint32_t points_fwd_stage(int cdim) { return cdim <= 8 ? 2 : 1; }
-constexpr int points_fwd_regs(int cdim) { return cdim <= 8 ? 96 : cdim <= 20 ? 80 : 112; }
+constexpr int points_fwd_regs(int cdim) { return cdim <= 20 ? 96 : 112; }
 
 template <int CDIM>
 __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kernel(
@@ -958,7 +976,7 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
         for (uint32_t q = 0; q < kStage; ++q)
             if (seen[q]) {
                 sA[pos[q]] = e[q].A;
-                sB[pos[q]] = e[q].B;
+                sB[pos[q]] = scaled_conic(e[q].B);
                 sC[pos[q]] = e[q].C;
                 sPos[pos[q]] = batch_start + (int32_t)(q * bs + tr);
                 sSeen[pos[q]] = seen[q];
@@ -980,19 +998,30 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
             T = next_T;
         };
         for (uint32_t t0 = 0; t0 < n_kept && !warp_done; t0 += 32) {
-            const uint32_t mine = t0 + lane;
-            uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u));
+            const uint32_t mine = t0 + lane, seen_by = mine < n_kept ? sSeen[mine] >> warp : 0u;
+            uint32_t todo = __ballot_sync(0xffffffffu, seen_by & 1u);
+            const uint32_t careful = __ballot_sync(0xffffffffu, (seen_by >> kCarefulShift) & 1u);
             while (todo && !(warp_done = __all_sync(0xffffffffu, done))) {
                 // two entries at a time; an odd one out is evaluated twice and blended once
+                uint32_t bits = todo & (0u - todo);
                 const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
                 todo &= todo - 1u;
                 const bool two = todo != 0u;
                 const uint32_t u = two ? t0 + (uint32_t)__ffs(todo) - 1u : t;
+                bits |= todo & (0u - todo);
                 todo &= todo - 1u;   // of 0: stays 0
                 const float4 A0 = sA[t], B0 = sB[t], A1 = sA[u], B1 = sB[u];
-                const PointFootprint f0 = point_footprint(A0, B0, roll, px, py), f1 = point_footprint(A1, B1, roll, px, py);
-                const float alpha0 = fminf(kAlphaMax, B0.w * f0.vis), alpha1 = fminf(kAlphaMax, B1.w * f1.vis);
-                const bool ok0 = !(f0.sigma < 0.f || alpha0 < kAlphaMin), ok1 = two && !(f1.sigma < 0.f || alpha1 < kAlphaMin);
+                PointFootprint f0 = point_footprint<false>(A0, B0, roll, px, py), f1 = point_footprint<false>(A1, B1, roll, px, py);
+                float alpha0 = B0.w * f0.vis, alpha1 = B1.w * f1.vis;
+                bool ok0 = alpha0 >= kAlphaMin, ok1 = two && alpha1 >= kAlphaMin;
+                if (careful & bits) {
+                    f0 = point_footprint<true>(A0, B0, roll, px, py);
+                    f1 = point_footprint<true>(A1, B1, roll, px, py);
+                    alpha0 = fminf(kAlphaMax, B0.w * f0.vis);
+                    alpha1 = fminf(kAlphaMax, B1.w * f1.vis);
+                    ok0 = !(f0.power > 0.f || alpha0 < kAlphaMin);
+                    ok1 = two && !(f1.power > 0.f || alpha1 < kAlphaMin);
+                }
                 if (ok0 && !done) blend(t, f0, alpha0);
                 if (ok1 && !done) blend(u, f1, alpha1);
             }
@@ -1034,23 +1063,39 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
 }
 
 // ---------------------------------------------------------------------------------------
-// Lidar forward for few patches: all warps of a CTA work on ONE patch, a share of the entries each. What
-// depends on the order - the transmittance, where a point stops, its median - stays one chain per point,
-// with the same operations as above, but it is all that is left in the chain:
-//   1. every warp evaluates its share of the entries and leaves the alphas in shared memory;
-//   2. one warp multiplies its way down them and leaves the transmittance in front of each entry;
-//   3. every warp goes over its share again: weights, where a point stops, median, sums, features. The
-//      warps' partial results are put together at the end.
+// Lidar forward for few patches: all warps of a CTA work on ONE patch, four consecutive entries each of the 32 between two
+// barriers. What depends on the order - the transmittance, where a point stops, its median - stays one chain per point, but
+// only the products of the warps' shares are in it:
+//   1. every warp evaluates its four entries, two per instruction, and leaves the product of their (1 - alpha);
+//   2. behind the barrier every warp multiplies its way through the eight products - its own entries' transmittances begin
+//      at the product of the shares before -, and goes over its share again for weights, where a point stops, median, sums
+//      and features. The warps' partial results are put together at the end.
 // The chain runs on behind a point's stop: the transmittance never rises, so an entry is blended exactly
-// if what it would leave is above the threshold. What bounds this is the chain of batches, barriers and
-// multiplications of the patch with the longest list, not the machine (15 % of its issue slots).
-// A 32 x 512 scan has 512 patches of up to 1900 entries: 124 us apart, 66 with all of step 3 but the features
-// in step 2's warp, 46 like this (47 with four blocks per SM, 50 with 64 entries between barriers).
+// if what it would leave is above the threshold. The next batch's entries are on their way while the chunks of
+// one are worked through, the range terms and features of those that stay while the first chunk is evaluated: a gather
+// of 32 lines holds the load unit for 32 cycles, and 256 entries with all they have took it for 2500.
+// What bounds it is the issue slots of the SM that holds the patch with the longest list (75 instructions per entry kept, 350 of
+// 1900 there) and, eight times, the way from a batch's gathers to its first chunk. A 32 x 512 scan, 8 channels: 43 -> 32 us, 17
+// channels 52 -> 34 (one warp multiplying down all 32 alphas, two barriers, every product by itself: 43).
 // ---------------------------------------------------------------------------------------
-constexpr uint32_t kCoopWarps = 8, kCoopChunk = 32, kCoopShare = kCoopChunk / kCoopWarps;
+constexpr uint32_t kCoopWarps = 8, kCoopShare = 4, kCoopChunk = kCoopWarps * kCoopShare;
+
+__device__ __forceinline__ void async_copy(float *dst_smem, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst_smem)), "l"(__cvta_generic_to_global(src)) : "memory");
+}
+__device__ __forceinline__ void async_copy_row(float *dst_smem, const float *__restrict__ src, uint32_t n, bool vec) {
+    if (vec)
+        for (uint32_t k = 0; k < n; k += 4)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst_smem + k)), "l"(__cvta_generic_to_global(src + k)) : "memory");
+    else
+        for (uint32_t k = 0; k < n; ++k) async_copy(dst_smem + k, src + k);
+}
+__device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+__device__ __forceinline__ float2 half_of(const float4 &v, int h) { return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y); }
 
 template <int CDIM>
-__global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_to_points_fwd_coop_kernel(
+__global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_coop_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors,
     const float *__restrict__ ranges, uint32_t channels,
@@ -1066,15 +1111,13 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     chain_enter();
     constexpr uint32_t kThreadsC = kCoopWarps * 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ PointBox s_box;
-    __shared__ uint32_t s_warp_kept[kCoopWarps];
-    __shared__ int s_done;
-    float4 *sA = reinterpret_cast<float4 *>(smem_raw);
-    float4 *sB = sA + kThreadsC;
-    float4 *sC = sB + kThreadsC;
-    float *sFeat = reinterpret_cast<float *>(sC + kThreadsC);               // [kThreadsC * CDIM]
-    float *sAlpha = sFeat + kThreadsC * CDIM;   // [2][kCoopChunk][32] alphas, then transmittances
-    int32_t *sPos = reinterpret_cast<int32_t *>(sAlpha + 2 * kCoopChunk * 32);
+    __shared__ uint32_t s_warp_kept[2][kCoopWarps];
+    __shared__ float sP[2][kCoopWarps][32];   // products of the warps' shares
+    // by value, so that four entries in sequence are one 16-byte access: azimuth, elevation, their velocities; scaled conic, opacity;
+    // range velocity, depth compensation (2), range
+    float *sE = reinterpret_cast<float *>(smem_raw);                        // [12][kThreadsC]
+    float *sFeat = sE + 12 * kThreadsC;                                     // [kThreadsC * CDIM]
+    int32_t *sPos = reinterpret_cast<int32_t *>(sFeat + kThreadsC * CDIM);  // list position; the sign bit: needs care
 
     const uint32_t tiles_per_cam = grid_w * grid_h;
     const uint32_t gtile = blockIdx.x / patches_per_tile, part = blockIdx.x - gtile * patches_per_tile;
@@ -1088,6 +1131,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     const bool in_image = index < tile_width * tile_height && i < H && j < W;
     bool inside = in_image;
     const size_t pix = ((size_t)cam * H + i) * W + j;
+    const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
     float px = 0.f, py = 0.f, pz = 0.f, roll = 0.f;
     if (inside) {
         const float4 rp = raster_pts[pix];
@@ -1096,13 +1140,12 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     }
     PointExtent extent;
     if (inside) extent.add(px, py, roll);
-    if (warp == 0) extent.write_box(&s_box);
-    if (tr == 0) s_done = 0;
-    const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
+    const PointBox box = extent.warp_box();
     const uint32_t num_batches = (uint32_t)(range.end - range.start + kThreadsC - 1) / kThreadsC;
     const uint32_t fstride = ranges ? channels - 1 : channels;
     const bool vec = (fstride % 4u == 0u) && ((reinterpret_cast<uintptr_t>(colors) & 15u) == 0u);
-    float T_run = inside ? 1.f : 0.f;   // the chain, held by the first warp
+    for (uint32_t k = channels; k < (uint32_t)CDIM; ++k) sFeat[tr * CDIM + k] = 0.f;   // no row is written there
+    float T_run = inside ? 1.f : 0.f;   // the chain, the same in every warp
     // of this warp's share
     float T = 1.f, depth_extra = 0.f, alpha_sum = 0.f, median = 0.f;
     int32_t cur_idx = 0;
@@ -1110,82 +1153,134 @@ __global__ void __launch_bounds__(kCoopWarps * 32, CDIM <= 8 ? 3 : 2) rasterize_
     float pix_out[CDIM];
 #pragma unroll
     for (int k = 0; k < CDIM; ++k) pix_out[k] = 0.f;
+    const float2 roll2 = make_float2(roll, roll), npx2 = make_float2(-px, -px), npy2 = make_float2(-py, -py);
 
-    int32_t next_id = range.start + (int32_t)tr < range.end ? flatten_ids[range.start + tr] : 0;
     bool finished = __all_sync(0xffffffffu, !inside);   // the same in every warp
+    int32_t g = 0, next_id = 0;
+    PointEntry e;
+    // the thread's entry of batch b, as far as the test needs it; the id of the one behind it
+    const auto load_entry = [&](uint32_t b) {
+        const int32_t idx = range.start + (int32_t)(kThreadsC * b + tr);
+        g = next_id;
+        if (idx < range.end) {
+            const float2 xy = __ldg(means2d + g);
+            const float *v = pix_vels + 3 * (size_t)g, *q = conics + 3 * (size_t)g;
+            e.A = make_float4(xy.x, xy.y, __ldg(v), __ldg(v + 1));
+            e.B = make_float4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(opacities + g));
+            if (idx + (int32_t)kThreadsC < range.end) next_id = flatten_ids[idx + kThreadsC];
+        }
+    };
+    if (!finished && range.start + (int32_t)tr < range.end) next_id = flatten_ids[range.start + tr];
+    if (!finished) load_entry(0);
     uint32_t buffer = 0;
     for (uint32_t b = 0; b < num_batches && !finished; ++b) {
         const int32_t idx = range.start + (int32_t)(kThreadsC * b + tr);
-        const int32_t g = next_id;
-        PointEntry e;
-        if (idx < range.end) {
-            e = load_point_entry(g, means2d, conics, opacities, pix_vels, depth_comps);
-            e.C.w = ranges ? __ldg(ranges + g) : __ldg(colors + (size_t)g * channels + depth_idx);
-            if (idx + (int32_t)kThreadsC < range.end) next_id = flatten_ids[idx + kThreadsC];   // on its way meanwhile
-        }
-        __syncthreads();   // the batch before has been read; the box and the flag have been written
-        const bool seen = idx < range.end && boxes_that_see(e, &s_box, 1u) != 0u;
-        const uint32_t kept = __ballot_sync(0xffffffffu, seen);
-        if (lane == 0) s_warp_kept[warp] = __popc(kept);
-        __syncthreads();
+        const uint32_t seen = idx < range.end ? boxes_that_see(e, &box, 1u) : 0u;
+        const uint32_t kept = __ballot_sync(0xffffffffu, seen != 0u);
+        if (lane == 0) s_warp_kept[b & 1u][warp] = __popc(kept);
+        __syncthreads();   // the batch before has been read
         uint32_t n_kept = 0, pos = __popc(kept & ((1u << lane) - 1u));
 #pragma unroll
         for (uint32_t w = 0; w < kCoopWarps; ++w) {
             if (w == warp) pos += n_kept;
-            n_kept += s_warp_kept[w];
+            n_kept += s_warp_kept[b & 1u][w];
         }
         if (seen) {
-            sA[pos] = e.A;
-            sB[pos] = e.B;
-            sC[pos] = e.C;
-            sPos[pos] = idx;
-            stage_features<CDIM>(sFeat + pos * CDIM, colors, (size_t)g, fstride, vec, ranges != nullptr, e.C.w);
+            const float4 B = scaled_conic(e.B);
+            const float v[8] = {e.A.x, e.A.y, e.A.z, e.A.w, B.x, B.y, B.z, B.w};
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) sE[k * kThreadsC + pos] = v[k];
+            sPos[pos] = seen >> kCarefulShift ? idx | INT32_MIN : idx;
+            float *late = sE + 8 * kThreadsC + pos, *row = sFeat + pos * CDIM;
+            const float *dc = reinterpret_cast<const float *>(depth_comps + g);
+            const float *distance = ranges ? ranges + g : colors + (size_t)g * channels + depth_idx;
+            async_copy(late, pix_vels + 3 * (size_t)g + 2);
+            async_copy(late + kThreadsC, dc);
+            async_copy(late + 2 * kThreadsC, dc + 1);
+            async_copy(late + 3 * kThreadsC, distance);
+            async_copy_row(row, colors + (size_t)g * fstride, fstride, vec);
+            if (ranges) async_copy(row + fstride, distance);
         }
+        if (b + 1 < num_batches) load_entry(b + 1);
         __syncthreads();
         for (uint32_t c0 = 0; c0 < n_kept && !finished; c0 += kCoopChunk) {
-            const uint32_t n = min(kCoopChunk, n_kept - c0);
-            float *al = sAlpha + buffer * kCoopChunk * 32 + lane;
+            const uint32_t t0 = c0 + warp * kCoopShare;
+            const bool mine = t0 < n_kept;
+            float alpha[kCoopShare];
+            float2 dx[2], dy[2];
+            int4 at = make_int4(0, 0, 0, 0);
+            float product = 1.f;
+            if (mine) {
+                const auto four = [&](uint32_t k) { return *reinterpret_cast<const float4 *>(sE + k * kThreadsC + t0); };
+                const float4 X = four(0), Y = four(1), VX = four(2), VY = four(3), Ba = four(4), Bb = four(5), Bc = four(6), Op = four(7);
+                at = *reinterpret_cast<const int4 *>(sPos + t0);
+                const float2 turn = make_float2(180.f, 180.f), back = make_float2(-180.f, -180.f);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    // a difference that does not wrap, rounded as angle_difference() rounds it
+                    dx[h] = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(roll2, half_of(VX, h), half_of(X, h)), npx2), turn), back);
+                    dy[h] = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(roll2, half_of(VY, h), half_of(Y, h)), npy2), turn), back);
+                    const float2 slope = __ffma2_rn(half_of(Ba, h), dx[h], __fmul2_rn(half_of(Bb, h), dy[h]));
+                    const float2 pw = __ffma2_rn(slope, dx[h], __fmul2_rn(__fmul2_rn(half_of(Bc, h), dy[h]), dy[h]));
+                    const float2 a = __fmul2_rn(half_of(Op, h), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
+                    alpha[2 * h] = a.x >= kAlphaMin ? a.x : 0.f;
+                    alpha[2 * h + 1] = a.y >= kAlphaMin ? a.y : 0.f;
+                }
+                if (t0 + kCoopShare > n_kept || (at.x | at.y | at.z | at.w) < 0) {
+#pragma unroll
+                    for (uint32_t k = 0; k < kCoopShare; ++k) {
+                        const uint32_t t = t0 + k;
+                        if (t >= n_kept) { alpha[k] = 0.f; continue; }
+                        if (sPos[t] >= 0) continue;
+                        const float *q = sE + t;
+                        const float4 A = make_float4(q[0], q[kThreadsC], q[2 * kThreadsC], q[3 * kThreadsC]);
+                        const float4 B = make_float4(q[4 * kThreadsC], q[5 * kThreadsC], q[6 * kThreadsC], q[7 * kThreadsC]);
+                        const PointFootprint f = point_footprint<true>(A, B, roll, px, py);
+                        const float a = fminf(kAlphaMax, B.w * f.vis), x = f.dx, y = f.dy;
+                        alpha[k] = f.power > 0.f || a < kAlphaMin ? 0.f : a;
+                        if (k & 1) { dx[k / 2].y = x; dy[k / 2].y = y; } else { dx[k / 2].x = x; dy[k / 2].x = y; }
+                    }
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < kCoopShare; ++k) product = fmaf(-alpha[k], product, product);
+            }
+            sP[buffer][warp][lane] = product;
+            if (c0 == 0) async_wait_all();   // the features
+            __syncthreads();
+            float before = T_run;
+#pragma unroll
+            for (uint32_t w = 0; w < kCoopWarps; ++w) {
+                if (w == warp) before = T_run;
+                T_run *= sP[buffer][w][lane];
+            }
             buffer ^= 1u;
-            float alpha[kCoopShare], dterm[kCoopShare];
+            finished = __all_sync(0xffffffffu, T_run <= kTStop);
+            if (!mine) continue;
+            // weights; what is not blended has none, and leaves nothing else behind
+            const auto four = [&](uint32_t k) { return *reinterpret_cast<const float4 *>(sE + k * kThreadsC + t0); };
+            const float4 RV = four(8), DX = four(9), DY = four(10), R = four(11);
+            float vis[kCoopShare];
 #pragma unroll
-            for (uint32_t r = 0; r < kCoopShare; ++r) {
-                const uint32_t q = warp + r * kCoopWarps, t = c0 + min(q, n - 1u);
-                const float4 A = sA[t], B = sB[t], Cc = sC[t];
-                const PointFootprint f = point_footprint(A, B, roll, px, py);
-                const float a = fminf(kAlphaMax, B.w * f.vis);
-                alpha[r] = q >= n || f.sigma < 0.f || a < kAlphaMin ? 0.f : a;
-                dterm[r] = Cc.y * f.dx + Cc.z * f.dy + Cc.x * roll;
-                al[q * 32] = alpha[r];
+            for (uint32_t k = 0; k < kCoopShare; ++k) {
+                const auto of = [&](const float4 &v) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; };
+                const float next_T = fmaf(-alpha[k], before, before);
+                const bool take = alpha[k] > 0.f && next_T > kTStop;
+                const float x = k & 1 ? dx[k / 2].y : dx[k / 2].x, y = k & 1 ? dy[k / 2].y : dy[k / 2].x;
+                const float d = fmaf(of(DX), x, fmaf(of(DY), y, of(RV) * roll));
+                vis[k] = take ? alpha[k] * before : 0.f;
+                depth_extra = fmaf(take ? d : 0.f, vis[k], depth_extra);
+                if (take && before > 0.5f && next_T <= 0.5f) median = of(R) + d;
+                if (compute_alpha_sum && take && of(R) < alpha_sum_limit) alpha_sum += alpha[k];
+                if (take) cur_idx = k == 0 ? at.x : k == 1 ? at.y : k == 2 ? at.z : at.w;
+                if (take) T = next_T;
+                before = next_T;
             }
-            __syncthreads();
-            if (warp == 0) {
 #pragma unroll
-                for (uint32_t q = 0; q < kCoopChunk; ++q) {
-                    const float a = al[q * 32];
-                    al[q * 32] = T_run;
-                    T_run *= 1.f - a;
-                }
-                if (__all_sync(0xffffffffu, T_run <= kTStop) && lane == 0) s_done = 1;
-            }
-            __syncthreads();
-            finished = s_done != 0;
-#pragma unroll
-            for (uint32_t r = 0; r < kCoopShare; ++r) {
-                const uint32_t q = warp + r * kCoopWarps;
-                const float before = al[q * 32], next_T = before * (1.f - alpha[r]);
-                const bool take = alpha[r] > 0.f && next_T > kTStop;
-                if (take) {
-                    const float vis = alpha[r] * before, range_q = sC[c0 + q].w;
-                    depth_extra += dterm[r] * vis;
-                    if (before > 0.5f && next_T <= 0.5f) median = range_q + dterm[r];
-                    if (compute_alpha_sum && range_q < alpha_sum_limit) alpha_sum += alpha[r];
-                    cur_idx = sPos[c0 + q];
-                    T = next_T;
-                    axpy_staged_full<CDIM>(pix_out, sFeat + (c0 + q) * CDIM, vis);   // here: elsewhere it would be 0 * inf
-                }
-            }
+            for (uint32_t k = 0; k < kCoopShare; ++k)                   if (vis[k] > 0.f) axpy_staged_full<CDIM>(pix_out, sFeat + (t0 + k) * CDIM, vis[k]);   // a branch: elsewhere it would be 0 * inf
         }
     }
+    cur_idx &= INT32_MAX;
+    async_wait_all();
     // partial sums of the warps, added in order
     __syncthreads();
     float *parts = reinterpret_cast<float *>(smem_raw);   // [warps][32][CDIM]
@@ -1670,9 +1765,9 @@ __device__ __noinline__ void odd_points_bwd(const PointTask &a, const PointGrads
             const size_t g = (size_t)a.flatten_ids[idx];
             const PointEntry e = load_point_entry((int32_t)g, a.means2d, a.conics, a.opacities, a.pix_vels, a.depth_comps);
             const float range = a.ranges ? a.ranges[g] : a.colors[g * n + a.depth_idx];
-            const PointFootprint f = point_footprint(e.A, e.B, pt.w, pt.x, pt.y);
+            const PointFootprint f = point_footprint<true>(e.A, scaled_conic(e.B), pt.w, pt.x, pt.y);
             const float alpha = fminf(kAlphaMax, e.B.w * f.vis);
-            const bool ok = idx <= last && !(f.sigma < 0.f || alpha < kAlphaMin);
+            const bool ok = idx <= last && !(f.power > 0.f || alpha < kAlphaMin);
             if (!__any_sync(0xffffffffu, ok)) continue;
             float fac = 0.f, v_alpha = 0.f;
             if (ok) {
@@ -1853,7 +1948,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         PointEntry e[kStage];
         int32_t g[kStage];
         uint32_t kept[kStage];
-        bool seen[kStage];
+        uint32_t seen[kStage];
 #pragma unroll
         for (uint32_t q = 0; q < kStage; ++q) {
             const int32_t idx = batch_end - (int32_t)(q * bs + tr), ahead = idx - (int32_t)cap;
@@ -1868,8 +1963,8 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         // survivors to the front, still back to front in list order
 #pragma unroll
         for (uint32_t q = 0; q < kStage; ++q) {
-            seen[q] = batch_end - (int32_t)(q * bs + tr) >= range.start && boxes_that_see(e[q], &s_box, 1u) != 0u;
-            kept[q] = __ballot_sync(0xffffffffu, seen[q]);
+            seen[q] = batch_end - (int32_t)(q * bs + tr) >= range.start ? boxes_that_see(e[q], &s_box, 1u) : 0u;
+            kept[q] = __ballot_sync(0xffffffffu, seen[q] != 0u);
             if (lane == 0) s_warp_kept[q * n_warps + warp] = __popc(kept[q]);
         }
         __syncthreads();
@@ -1885,7 +1980,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
                 sA[pos] = e[q].A;
                 sB[pos] = e[q].B;
                 sC[pos] = e[q].C;
-                sId[pos] = g[q];
+                sId[pos] = seen[q] >> kCarefulShift ? g[q] | INT32_MIN : g[q];
                 sPos[pos] = batch_end - (int32_t)(q * bs + tr);
                 stage_features<CDIM>(sRgb + pos * CDIM, colors, (size_t)g[q], fstride, vec, ranges != nullptr, e[q].C.w);
             }
@@ -1897,20 +1992,36 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         // batch before ended.)
         const uint32_t per = (n_kept + n_warps - 1) / n_warps;
         const uint32_t t_lo = min(n_kept, warp * per), t_hi = min(n_kept, t_lo + per);
-        const auto evaluate = [&](uint32_t t, float4 &B, float2 &dx, float2 &dy, float2 &vis, float2 &alpha, float2 &open) {
+        // alpha and exp(-sigma) of the entry, zeros where a point does not blend it; `open`, of an entry that needs care: zero where
+        // the alpha is capped and passes no gradient on to the geometry
+        const auto evaluate = [&](uint32_t t, int32_t id, float4 &B, float2 &dx, float2 &dy, float2 &vis, float2 &alpha, float2 &open) {
             const float4 A = sA[t];
             B = sB[t];
+            const float4 S = scaled_conic(B);
             const int32_t entry = sPos[t];
-            const PointFootprint f0 = point_footprint(A, B, roll.x, az.x, el.x), f1 = point_footprint(A, B, roll.y, az.y, el.y);
-            const float a0 = fminf(kAlphaMax, B.w * f0.vis), a1 = fminf(kAlphaMax, B.w * f1.vis);
-            const bool ok0 = entry <= bin_final[0] && !(f0.sigma < 0.f || a0 < kAlphaMin);
-            const bool ok1 = entry <= bin_final[1] && !(f1.sigma < 0.f || a1 < kAlphaMin);
-            dx = make_float2(f0.dx, f1.dx);
-            dy = make_float2(f0.dy, f1.dy);
-            vis = make_float2(ok0 ? f0.vis : 0.f, ok1 ? f1.vis : 0.f);
-            alpha = make_float2(ok0 ? a0 : 0.f, ok1 ? a1 : 0.f);
-            // a capped alpha passes no gradient on to the geometry
-            open = make_float2(B.w * f0.vis <= kAlphaMax ? 1.f : 0.f, B.w * f1.vis <= kAlphaMax ? 1.f : 0.f);
+            const float2 mx = __ffma2_rn(roll, make_float2(A.z, A.z), make_float2(A.x, A.x)), my = __ffma2_rn(roll, make_float2(A.w, A.w), make_float2(A.y, A.y));
+            const float2 turn = make_float2(180.f, 180.f), back = make_float2(-180.f, -180.f);
+            dx = __fadd2_rn(__fadd2_rn(__fadd2_rn(mx, make_float2(-az.x, -az.y)), turn), back);
+            dy = __fadd2_rn(__fadd2_rn(__fadd2_rn(my, make_float2(-el.x, -el.y)), turn), back);
+            const float2 slope = __ffma2_rn(make_float2(S.x, S.x), dx, __fmul2_rn(make_float2(S.y, S.y), dy));
+            const float2 pw = __ffma2_rn(slope, dx, __fmul2_rn(__fmul2_rn(make_float2(S.z, S.z), dy), dy));
+            vis = make_float2(exp2_approx(pw.x), exp2_approx(pw.y));
+            alpha = __fmul2_rn(make_float2(B.w, B.w), vis);
+            bool ok0 = alpha.x >= kAlphaMin, ok1 = alpha.y >= kAlphaMin;
+            if (id < 0) {
+                const PointFootprint f0 = point_footprint<true>(A, S, roll.x, az.x, el.x), f1 = point_footprint<true>(A, S, roll.y, az.y, el.y);
+                dx = make_float2(f0.dx, f1.dx);
+                dy = make_float2(f0.dy, f1.dy);
+                vis = make_float2(f0.vis, f1.vis);
+                open = make_float2(B.w * f0.vis <= kAlphaMax ? 1.f : 0.f, B.w * f1.vis <= kAlphaMax ? 1.f : 0.f);
+                alpha = make_float2(fminf(kAlphaMax, B.w * f0.vis), fminf(kAlphaMax, B.w * f1.vis));
+                ok0 = !(f0.power > 0.f || alpha.x < kAlphaMin);
+                ok1 = !(f1.power > 0.f || alpha.y < kAlphaMin);
+            }
+            ok0 = ok0 && entry <= bin_final[0];
+            ok1 = ok1 && entry <= bin_final[1];
+            vis = make_float2(ok0 ? vis.x : 0.f, ok1 ? vis.y : 0.f);
+            alpha = make_float2(ok0 ? alpha.x : 0.f, ok1 ? alpha.y : 0.f);
             return ok0 || ok1;
         };
         float2 T_batch = T, behind_batch = behind;
@@ -1919,7 +2030,8 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
             for (uint32_t t = t_lo; t < t_hi; ++t) {
                 float4 B;
                 float2 dx, dy, vis, alpha, open;
-                if (!__any_sync(0xffffffffu, evaluate(t, B, dx, dy, vis, alpha, open))) continue;
+                const int32_t id = sId[t];
+                if (!__any_sync(0xffffffffu, evaluate(t, id, B, dx, dy, vis, alpha, open))) continue;
                 const float4 Cc = sC[t];
                 const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
                 P = __fmul2_rn(P, reciprocal_pair(om));
@@ -1952,7 +2064,8 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
             for (uint32_t t = t_lo; t < t_hi; ++t) {
                 float4 B;
                 float2 dx, dy, vis, alpha, open;
-                if (!__any_sync(0xffffffffu, evaluate(t, B, dx, dy, vis, alpha, open))) continue;
+                const int32_t id = sId[t];
+                if (!__any_sync(0xffffffffu, evaluate(t, id, B, dx, dy, vis, alpha, open))) continue;
                 const float4 Cc = sC[t];
                 const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
                 const float2 ra = reciprocal_pair(om);
@@ -1984,7 +2097,12 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
                 const float2 v_alpha = __ffma2_rn(T, dot, __fmul2_rn(make_float2(-ra.x, -ra.y), behind));
                 behind = __ffma2_rn(fac, dot, behind);
                 // v = -dL/dsigma / opacity; the alpha sum reaches the entries in front of the point
-                const float2 v_main = __fmul2_rn(__fmul2_rn(vis, open), v_alpha);
+                float2 vis_open = vis, fac_open = fac;
+                if (id < 0) {
+                    vis_open = __fmul2_rn(vis, open);
+                    fac_open = __fmul2_rn(fac, open);
+                }
+                const float2 v_main = __fmul2_rn(vis_open, v_alpha);
                 float2 v_sum = make_float2(0.f, 0.f);
                 if (compute_alpha_sum) {
                     const float g_depth = sRgb[t * CDIM + depth_idx];
@@ -1992,7 +2110,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
                 }
                 const float2 v = __fadd2_rn(v_main, v_sum);
                 const float2 w = __fmul2_rn(make_float2(-B.w, -B.w), v);                   // dL/dsigma
-                const float2 vd = __fmul2_rn(__fmul2_rn(fac, open), v_depth);              // dL/d(range term)
+                const float2 vd = __fmul2_rn(fac_open, v_depth);                           // dL/d(range term)
                 const float2 bx = make_float2(B.x, B.x), by = make_float2(B.y, B.y), bz = make_float2(B.z, B.z);
                 const float2 sx = __ffma2_rn(bx, dx, __fmul2_rn(by, dy)), sy = __ffma2_rn(by, dx, __fmul2_rn(bz, dy));
                 const float2 gx = __ffma2_rn(w, sx, __fmul2_rn(vd, make_float2(Cc.y, Cc.y)));
@@ -2016,7 +2134,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
                     sum[CDIM + 11] = fabsf(gx.x - ux.x) + fabsf(ux.x) + fabsf(gx.y - ux.y) + fabsf(ux.y);
                     sum[CDIM + 12] = fabsf(gy.x - uy.x) + fabsf(uy.x) + fabsf(gy.y - uy.y) + fabsf(uy.y);
                 }
-                const size_t gid = (size_t)sId[t];
+                const size_t gid = (size_t)(id & INT32_MAX);
                 float sums[kSums];
 #pragma unroll
                 for (int k = 0; k < kSums; ++k) sums[k] = sum[k];
@@ -2081,10 +2199,10 @@ static uint32_t pixels_per_lane_bwd(uint64_t blocks, uint32_t tile_size, uint32_
 }
 
 // Patches below which all warps of a CTA share one in the forward pass: the shared work costs more
-// instructions in all, so the patches must be too few to fill the machine. Apart and shared, us, 8 channels: 512
-// patches 82 and 31, 800 73 and 42, 1088 72 and 46, 1408 54 and 44, 1856 57 and 52, 2176 58 and 62, 3200 65 and 87; 17
-// channels cross over a little earlier (1856: 66 both). The line lies below the crossing in every case measured.
-constexpr uint64_t kCoopPatches = kNumSMs * 8;
+// instructions in all, so the patches must be too few to fill the machine. Apart and shared, us, 8 channels: 256
+// patches 157 and 42, 512 109 and 32, 800 64 and 38, 1216 54 and 41, 1600 51 and 51, 2176 49 and 67, 3712 62 and 109; 17
+// channels: 512 126 and 34, 1216 65 and 47, 1600 54 and 58, 2176 56 and 77.
+constexpr uint64_t kCoopPatches = kNumSMs * 10;
 
 // Warps - segments of the list - per patch in the backward pass: every segment is run twice, which pays
 // while the patches alone leave the schedulers waiting on one warp's chain. One, four and eight segments, us, 8
@@ -2277,7 +2395,7 @@ extern "C" int splatad_rasterize_to_points_fwd(
         auto kernel = coop ? rasterize_to_points_fwd_coop_kernel<D> : rasterize_to_points_fwd_kernel<D>; \
         const size_t smem = (size_t)(coop ? 1 : points_fwd_stage(D)) * bs *                       \
                                 (3 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float)) +  \
-                            (coop ? 2 * kCoopChunk * 32 * sizeof(float) : 0);                     \
+                            0;                                                                    \
         int rc = set_smem(kernel, smem, "rasterize_to_points_fwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
         launch_chained_if(fits_at_once((uint64_t)blocks * parts), kernel, blocks * parts, bs, smem, \

@@ -471,3 +471,47 @@ def test_points_in_patches(tw, th, H, W, channels, asum, absgrad):
         _grad_check(f"tile {tw}x{th} ch={channels} {name}", leaves[k].grad, ref[name])
     if absgrad:
         _grad_check(f"tile {tw}x{th} ch={channels} absgrad", leaves["means2d"].absgrad, ref["v_means2d_abs"])
+
+
+@pytest.mark.parametrize("C,H,W,channels", [(1, 16, 256, 3), (1, 32, 300, 9), (6, 64, 512, 5), (6, 64, 512, 18)])
+def test_points_with_needles_and_the_seam(C, H, W, channels):
+    """Entries whose alphas or angles need care beside those that do not - needles on either side of the line, a conic that
+    is not positive definite, opacities above the cap, means on both sides of the half turn - where the warps of a CTA
+    share a patch and where they do not, forward and backward against the oracle."""
+    from oracle import composite
+    from splatad_b200 import ops
+    N, tw, th = 400, 32, 8
+    c = _lidar_case(C, N, H, W, tw, th, channels, 77 * H + channels)
+    c["opacities"][:, ::11] = 0.9995
+    for k, rho in enumerate((0.999, 0.99999, 0.9999999, 1.5)):   # 1 - rho^2 against 1e-5
+        a, b = c["conics"][:, 2 + k, 0], c["conics"][:, 2 + k, 2]
+        c["conics"][:, 2 + k, 1] = rho * torch.sqrt(a * b)
+    g = torch.Generator().manual_seed(4)
+    v_c, v_a, v_s = (torch.randn(C, H, W, k, generator=g) for k in (channels, 1, 1))
+    keys = ("means2d", "conics", "feats", "opacities", "pix_vels", "dcomp")
+    args = [n(c[k]) for k in keys] + [None, n(c["pts"]), W, H, tw, th, c["offsets"], c["flatten_ids"], True, 0.5]
+    ref_f = composite.rasterize_to_points_fwd(*args, dtype=np.float64)
+    f32 = composite.rasterize_to_points_fwd(*args, amb_tol=1e-4)
+    same = (f32["last_ids"] == ref_f["last_ids"]) & ~f32["ambiguous"]
+    # the sign and the size of a form that nearly vanishes or is negative somewhere hang on the last bits
+    pts = n(c["pts"]).astype(np.float64)
+    turn = lambda d: (d + 180.0) % 360.0 - 180.0   # noqa: E731
+    for k in range(2, 6):
+        m, v, q = (n(c[key])[:, k].astype(np.float64)[:, None, None] for key in ("means2d", "pix_vels", "conics"))
+        dx, dy = turn(m[..., 0] + pts[..., 3] * v[..., 0] - pts[..., 0]), m[..., 1] + pts[..., 3] * v[..., 1] - pts[..., 1]
+        size = 0.5 * (q[..., 0] * dx * dx + q[..., 2] * dy * dy)
+        sigma = size + q[..., 1] * dx * dy
+        same &= ~((sigma < 12.0) & ((size > 20.0) | (np.abs(sigma) < 1e-3)))
+    assert same.mean() > 0.6   # four needles and the one with two signs reach a third of the smallest scan
+    mask, mk = t(same[..., None].astype(np.float32)), same[..., None].astype(np.float64)
+    leaves = {k: t(c[k]).requires_grad_(True) for k in keys}
+    out_c, out_a, out_s, _ = ops.rasterize_to_points(*(leaves[k] for k in keys), t(c["pts"]), W, H, tw, th, t(c["offsets"], torch.int32),
+                                                     t(c["flatten_ids"], torch.int32), True, 0.5)
+    for got, want in ((out_c, f32["render_colors"]), (out_a, f32["render_alphas"])):
+        assert_close(f"points {H}x{W} ch={channels}", n(got), want, 2e-4, 2e-5, mask=same[..., None])
+    torch.autograd.backward([out_c, out_a, out_s], [t(v_c) * mask, t(v_a) * mask, t(v_s) * mask])
+    ref = composite.rasterize_to_points_bwd(*args, ref_f["render_alphas"], ref_f["last_ids"], n(v_c) * mk, n(v_a) * mk, n(v_s) * mk)
+    plain = np.r_[0:2, 6:N]   # the needles' own gradients are sums of large terms that cancel
+    names = ("v_means2d", "v_conics", "v_colors", "v_opacities", "v_pix_vels", "v_depth_comps")
+    for k, name in zip(keys, names):
+        _grad_check(f"points {H}x{W} ch={channels} {name}", leaves[k].grad[:, plain], ref[name].reshape(leaves[k].shape)[:, plain])
