@@ -822,9 +822,19 @@ __device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const Po
     return seen;
 }
 
-// Offset of an entry from a point and its exp(-sigma) = 2^power; power decides with alpha whether it is blended. The conic
-// is scaled (scaled_conic()). Where nothing wraps the differences are rounded as angle_difference() rounds them.
-struct PointFootprint { float dx, dy, power, vis; };
+// Offset of an entry from a point and its exp(-sigma); sigma decides with alpha whether it is blended. Every kernel rounds
+// the steps alike - one or two values at a time, and the transmittances' factors as T * (1 - alpha) -, because the median
+// range of a point is that of the entry at which its transmittance crosses a half: the last bit decides between two
+// ranges that may lie far apart. Where nothing wraps the differences are rounded as angle_difference() rounds them.
+struct PointFootprint { float dx, dy, sigma, vis; };
+
+__device__ __forceinline__ float point_sigma(const float4 &B, float dx, float dy) {
+    return fmaf(__fmul_rn(B.y, dx), dy, __fmul_rn(0.5f, fmaf(__fmul_rn(B.x, dx), dx, __fmul_rn(__fmul_rn(B.z, dy), dy))));
+}
+__device__ __forceinline__ float2 point_sigma(float2 a, float2 b, float2 c, float2 dx, float2 dy) {
+    const float2 square = __ffma2_rn(__fmul2_rn(a, dx), dx, __fmul2_rn(__fmul2_rn(c, dy), dy));
+    return __ffma2_rn(__fmul2_rn(b, dx), dy, __fmul2_rn(make_float2(0.5f, 0.5f), square));
+}
 
 template <bool kWraps>
 __device__ __forceinline__ PointFootprint point_footprint(const float4 &A, const float4 &B, float roll, float az, float el) {
@@ -832,8 +842,8 @@ __device__ __forceinline__ PointFootprint point_footprint(const float4 &A, const
     const float mx = fmaf(roll, A.z, A.x), my = fmaf(roll, A.w, A.y);
     f.dx = kWraps ? angle_difference(mx, az) : (mx - az + 180.f) - 180.f;
     f.dy = kWraps ? angle_difference(my, el) : (my - el + 180.f) - 180.f;
-    f.power = fmaf(fmaf(B.x, f.dx, B.y * f.dy), f.dx, B.z * f.dy * f.dy);
-    f.vis = exp2_approx(f.power);
+    f.sigma = point_sigma(B, f.dx, f.dy);
+    f.vis = __expf(-f.sigma);
     return f;
 }
 
@@ -863,7 +873,8 @@ __device__ __forceinline__ void stage_features(float *row, const float *__restri
 // ---------------------------------------------------------------------------------------
 // entries per thread and batch (their loads overlap), while the shared memory of a batch stays small
 constexpr uint32_t points_fwd_stage(int cdim) { return cdim <= 8 ? 2 : 1; }
-constexpr int points_fwd_regs(int cdim) { return cdim <= 20 ? 96 : 112; }
+// (17 channels: 128 x 1800 40 us at 80 registers, 42 at 96; 64 x 1083 64 and 56)
+constexpr int points_fwd_regs(int cdim) { return cdim <= 8 ? 96 : cdim <= 20 ? 80 : 112; }
 
 template <int CDIM>
 __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kernel(
@@ -976,7 +987,7 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
         for (uint32_t q = 0; q < kStage; ++q)
             if (seen[q]) {
                 sA[pos[q]] = e[q].A;
-                sB[pos[q]] = scaled_conic(e[q].B);
+                sB[pos[q]] = e[q].B;
                 sC[pos[q]] = e[q].C;
                 sPos[pos[q]] = batch_start + (int32_t)(q * bs + tr);
                 sSeen[pos[q]] = seen[q];
@@ -1019,8 +1030,8 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
                     f1 = point_footprint<true>(A1, B1, roll, px, py);
                     alpha0 = fminf(kAlphaMax, B0.w * f0.vis);
                     alpha1 = fminf(kAlphaMax, B1.w * f1.vis);
-                    ok0 = !(f0.power > 0.f || alpha0 < kAlphaMin);
-                    ok1 = two && !(f1.power > 0.f || alpha1 < kAlphaMin);
+                    ok0 = !(f0.sigma < 0.f || alpha0 < kAlphaMin);
+                    ok1 = two && !(f1.sigma < 0.f || alpha1 < kAlphaMin);
                 }
                 if (ok0 && !done) blend(t, f0, alpha0);
                 if (ok1 && !done) blend(u, f1, alpha1);
@@ -1064,19 +1075,20 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
 
 // ---------------------------------------------------------------------------------------
 // Lidar forward for few patches: all warps of a CTA work on ONE patch, four consecutive entries each of the 32 between two
-// barriers. What depends on the order - the transmittance, where a point stops, its median - stays one chain per point, but
-// only the products of the warps' shares are in it:
-//   1. every warp evaluates its four entries, two per instruction, and leaves the product of their (1 - alpha);
-//   2. behind the barrier every warp multiplies its way through the eight products - its own entries' transmittances begin
-//      at the product of the shares before -, and goes over its share again for weights, where a point stops, median, sums
-//      and features. The warps' partial results are put together at the end.
+// barriers. What depends on the order - the transmittance, where a point stops, its median - stays one chain per point, with
+// the same operations as above, but it is all that is left in the chain:
+//   1. every warp evaluates its four entries, two per instruction, and leaves their 1 - alpha;
+//   2. behind the barrier every warp multiplies its way down all 32 of them by itself - no second barrier, nothing handed
+//      back -, and goes over its share again for weights, where a point stops, median, sums and features. The warps' partial
+//      results are put together at the end.
 // The chain runs on behind a point's stop: the transmittance never rises, so an entry is blended exactly
 // if what it would leave is above the threshold. The next batch's entries are on their way while the chunks of
 // one are worked through, the range terms and features of those that stay while the first chunk is evaluated: a gather
 // of 32 lines holds the load unit for 32 cycles, and 256 entries with all they have took it for 2500.
 // What bounds it is the issue slots of the SM that holds the patch with the longest list (75 instructions per entry kept, 350 of
-// 1900 there) and, eight times, the way from a batch's gathers to its first chunk. A 32 x 512 scan, 8 channels: 43 -> 32 us, 17
-// channels 52 -> 34 (one warp multiplying down all 32 alphas, two barriers, every product by itself: 43).
+// 1900 there) and, eight times, the way from a batch's gathers to its first chunk. A 32 x 512 scan, 8 channels: 43 -> 35 us (one
+// warp multiplying down all 32, two barriers, everything gathered for every entry: 43; every warp leaving one product of its
+// four, which rounds differently: 32).
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t kCoopWarps = 8, kCoopShare = 4, kCoopChunk = kCoopWarps * kCoopShare;
 
@@ -1112,8 +1124,8 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_co
     constexpr uint32_t kThreadsC = kCoopWarps * 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_warp_kept[2][kCoopWarps];
-    __shared__ float sP[2][kCoopWarps][32];   // products of the warps' shares
-    // by value, so that four entries in sequence are one 16-byte access: azimuth, elevation, their velocities; scaled conic, opacity;
+    __shared__ float4 sLeft[2][kCoopWarps][32];   // 1 - alpha of the warps' shares
+    // by value, so that four entries in sequence are one 16-byte access: azimuth, elevation, their velocities; conic, opacity;
     // range velocity, depth compensation (2), range
     float *sE = reinterpret_cast<float *>(smem_raw);                        // [12][kThreadsC]
     float *sFeat = sE + 12 * kThreadsC;                                     // [kThreadsC * CDIM]
@@ -1186,8 +1198,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_co
             n_kept += s_warp_kept[b & 1u][w];
         }
         if (seen) {
-            const float4 B = scaled_conic(e.B);
-            const float v[8] = {e.A.x, e.A.y, e.A.z, e.A.w, B.x, B.y, B.z, B.w};
+            const float v[8] = {e.A.x, e.A.y, e.A.z, e.A.w, e.B.x, e.B.y, e.B.z, e.B.w};
 #pragma unroll
             for (uint32_t k = 0; k < 8; ++k) sE[k * kThreadsC + pos] = v[k];
             sPos[pos] = seen >> kCarefulShift ? idx | INT32_MIN : idx;
@@ -1209,7 +1220,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_co
             float alpha[kCoopShare];
             float2 dx[2], dy[2];
             int4 at = make_int4(0, 0, 0, 0);
-            float product = 1.f;
+            float4 left = make_float4(1.f, 1.f, 1.f, 1.f);   // 1 - alpha
             if (mine) {
                 const auto four = [&](uint32_t k) { return *reinterpret_cast<const float4 *>(sE + k * kThreadsC + t0); };
                 const float4 X = four(0), Y = four(1), VX = four(2), VY = four(3), Ba = four(4), Bb = four(5), Bc = four(6), Op = four(7);
@@ -1220,9 +1231,8 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_co
                     // a difference that does not wrap, rounded as angle_difference() rounds it
                     dx[h] = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(roll2, half_of(VX, h), half_of(X, h)), npx2), turn), back);
                     dy[h] = __fadd2_rn(__fadd2_rn(__fadd2_rn(__ffma2_rn(roll2, half_of(VY, h), half_of(Y, h)), npy2), turn), back);
-                    const float2 slope = __ffma2_rn(half_of(Ba, h), dx[h], __fmul2_rn(half_of(Bb, h), dy[h]));
-                    const float2 pw = __ffma2_rn(slope, dx[h], __fmul2_rn(__fmul2_rn(half_of(Bc, h), dy[h]), dy[h]));
-                    const float2 a = __fmul2_rn(half_of(Op, h), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
+                    const float2 sigma = point_sigma(half_of(Ba, h), half_of(Bb, h), half_of(Bc, h), dx[h], dy[h]);
+                    const float2 a = __fmul2_rn(half_of(Op, h), make_float2(__expf(-sigma.x), __expf(-sigma.y)));
                     alpha[2 * h] = a.x >= kAlphaMin ? a.x : 0.f;
                     alpha[2 * h + 1] = a.y >= kAlphaMin ? a.y : 0.f;
                 }
@@ -1237,21 +1247,21 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_co
                         const float4 B = make_float4(q[4 * kThreadsC], q[5 * kThreadsC], q[6 * kThreadsC], q[7 * kThreadsC]);
                         const PointFootprint f = point_footprint<true>(A, B, roll, px, py);
                         const float a = fminf(kAlphaMax, B.w * f.vis), x = f.dx, y = f.dy;
-                        alpha[k] = f.power > 0.f || a < kAlphaMin ? 0.f : a;
+                        alpha[k] = f.sigma < 0.f || a < kAlphaMin ? 0.f : a;
                         if (k & 1) { dx[k / 2].y = x; dy[k / 2].y = y; } else { dx[k / 2].x = x; dy[k / 2].x = y; }
                     }
                 }
-#pragma unroll
-                for (uint32_t k = 0; k < kCoopShare; ++k) product = fmaf(-alpha[k], product, product);
+                left = make_float4(1.f - alpha[0], 1.f - alpha[1], 1.f - alpha[2], 1.f - alpha[3]);
             }
-            sP[buffer][warp][lane] = product;
+            sLeft[buffer][warp][lane] = left;
             if (c0 == 0) async_wait_all();   // the features
             __syncthreads();
             float before = T_run;
 #pragma unroll
             for (uint32_t w = 0; w < kCoopWarps; ++w) {
+                const float4 l = sLeft[buffer][w][lane];
                 if (w == warp) before = T_run;
-                T_run *= sP[buffer][w][lane];
+                T_run = T_run * l.x * l.y * l.z * l.w;
             }
             buffer ^= 1u;
             finished = __all_sync(0xffffffffu, T_run <= kTStop);
@@ -1263,7 +1273,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_co
 #pragma unroll
             for (uint32_t k = 0; k < kCoopShare; ++k) {
                 const auto of = [&](const float4 &v) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; };
-                const float next_T = fmaf(-alpha[k], before, before);
+                const float next_T = before * of(left);
                 const bool take = alpha[k] > 0.f && next_T > kTStop;
                 const float x = k & 1 ? dx[k / 2].y : dx[k / 2].x, y = k & 1 ? dy[k / 2].y : dy[k / 2].x;
                 const float d = fmaf(of(DX), x, fmaf(of(DY), y, of(RV) * roll));
@@ -1765,9 +1775,9 @@ __device__ __noinline__ void odd_points_bwd(const PointTask &a, const PointGrads
             const size_t g = (size_t)a.flatten_ids[idx];
             const PointEntry e = load_point_entry((int32_t)g, a.means2d, a.conics, a.opacities, a.pix_vels, a.depth_comps);
             const float range = a.ranges ? a.ranges[g] : a.colors[g * n + a.depth_idx];
-            const PointFootprint f = point_footprint<true>(e.A, scaled_conic(e.B), pt.w, pt.x, pt.y);
+            const PointFootprint f = point_footprint<true>(e.A, e.B, pt.w, pt.x, pt.y);
             const float alpha = fminf(kAlphaMax, e.B.w * f.vis);
-            const bool ok = idx <= last && !(f.power > 0.f || alpha < kAlphaMin);
+            const bool ok = idx <= last && !(f.sigma < 0.f || alpha < kAlphaMin);
             if (!__any_sync(0xffffffffu, ok)) continue;
             float fac = 0.f, v_alpha = 0.f;
             if (ok) {
@@ -1997,26 +2007,24 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         const auto evaluate = [&](uint32_t t, int32_t id, float4 &B, float2 &dx, float2 &dy, float2 &vis, float2 &alpha, float2 &open) {
             const float4 A = sA[t];
             B = sB[t];
-            const float4 S = scaled_conic(B);
             const int32_t entry = sPos[t];
             const float2 mx = __ffma2_rn(roll, make_float2(A.z, A.z), make_float2(A.x, A.x)), my = __ffma2_rn(roll, make_float2(A.w, A.w), make_float2(A.y, A.y));
             const float2 turn = make_float2(180.f, 180.f), back = make_float2(-180.f, -180.f);
             dx = __fadd2_rn(__fadd2_rn(__fadd2_rn(mx, make_float2(-az.x, -az.y)), turn), back);
             dy = __fadd2_rn(__fadd2_rn(__fadd2_rn(my, make_float2(-el.x, -el.y)), turn), back);
-            const float2 slope = __ffma2_rn(make_float2(S.x, S.x), dx, __fmul2_rn(make_float2(S.y, S.y), dy));
-            const float2 pw = __ffma2_rn(slope, dx, __fmul2_rn(__fmul2_rn(make_float2(S.z, S.z), dy), dy));
-            vis = make_float2(exp2_approx(pw.x), exp2_approx(pw.y));
+            const float2 sigma = point_sigma(make_float2(B.x, B.x), make_float2(B.y, B.y), make_float2(B.z, B.z), dx, dy);
+            vis = make_float2(__expf(-sigma.x), __expf(-sigma.y));
             alpha = __fmul2_rn(make_float2(B.w, B.w), vis);
             bool ok0 = alpha.x >= kAlphaMin, ok1 = alpha.y >= kAlphaMin;
             if (id < 0) {
-                const PointFootprint f0 = point_footprint<true>(A, S, roll.x, az.x, el.x), f1 = point_footprint<true>(A, S, roll.y, az.y, el.y);
+                const PointFootprint f0 = point_footprint<true>(A, B, roll.x, az.x, el.x), f1 = point_footprint<true>(A, B, roll.y, az.y, el.y);
                 dx = make_float2(f0.dx, f1.dx);
                 dy = make_float2(f0.dy, f1.dy);
                 vis = make_float2(f0.vis, f1.vis);
                 open = make_float2(B.w * f0.vis <= kAlphaMax ? 1.f : 0.f, B.w * f1.vis <= kAlphaMax ? 1.f : 0.f);
                 alpha = make_float2(fminf(kAlphaMax, B.w * f0.vis), fminf(kAlphaMax, B.w * f1.vis));
-                ok0 = !(f0.power > 0.f || alpha.x < kAlphaMin);
-                ok1 = !(f1.power > 0.f || alpha.y < kAlphaMin);
+                ok0 = !(f0.sigma < 0.f || alpha.x < kAlphaMin);
+                ok1 = !(f1.sigma < 0.f || alpha.y < kAlphaMin);
             }
             ok0 = ok0 && entry <= bin_final[0];
             ok1 = ok1 && entry <= bin_final[1];
