@@ -1334,6 +1334,9 @@ blk_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket) {
 // blockIdx.x: 512 entries of a sensor, blockIdx.y: two block rows. Few rows per CTA, because the entries
 // come in depth order and the nearest ones cover the whole image: the CTA that holds them walks 60 blocks
 // per lane of a 1920 x 1080 grid instead of 270 (70 -> 39 us for the camera benchmark's frame).
+// Bound by instruction issue and by the waits between its phases. A warp clears its own words, a column's sixteen counts are
+// read before the first sum is written, and the columns of a rectangle that does not wrap are whole nibbles but for
+// its two ends: camera benchmark 36 -> 27 us, six cameras 340 -> 233; lidar benchmark 41.
 // kWrap: rectangles may cover the turn more than once and then leave several records in a block (a
 // rectangle spans less than five turns): three more mask words per (warp, block) hold the bits of their
 // lanes' surplus.
@@ -1355,14 +1358,15 @@ blk_scatter_kernel(BlkArgs a) {
     if (tid < n_cols)
         first = __ldg(a.rec_start + c.sensor * a.blocks + r0 * a.bx + tid) +
                 __ldg(a.table + (size_t)(r0 * a.bx + tid) * a.ctas + blockIdx.x);
-    for (uint32_t k = tid; k < plane; k += kBlkThreads) s_mask[k] = 0u;
+    uint32_t *mask = s_mask + warp * n_cols;   // only this warp writes there
+    for (uint32_t k = lane; k < n_cols; k += 32) mask[k] = 0u;
     if (overflow || !c.live) return;
     const BlkRect b = blk_rect(a, rect, tid < c.n);
     const bool layered = kWrap && __syncthreads_or(b.layers > 1);
     if (kWrap && layered)
-        for (uint32_t k = plane + tid; k < 4 * plane; k += kBlkThreads) s_mask[k] = 0u;
-    __syncthreads();
-    uint32_t *mask = s_mask + warp * n_cols;
+        for (uint32_t q = 1; q < 4; ++q)
+            for (uint32_t k = lane; k < n_cols; k += 32) mask[q * plane + k] = 0u;
+    __syncwarp();
     for (uint32_t j = 0; j < kBlkRows; ++j) {
         const uint32_t n = blk_row_cols(b, r0 + j);
         uint32_t *row = mask + j * a.bx;
@@ -1373,22 +1377,32 @@ blk_scatter_kernel(BlkArgs a) {
                 for (uint32_t q = 0; q < 3; ++q)
                     if ((more >> q) & 1u) atomicOr(&row[(q + 1) * plane + s], 1u << lane);
             }
-            if (++s == a.bx) s = 0;
+            if (++s == a.bx && kWrap) s = 0;
         }
     }
     __syncthreads();
     if (tid < n_cols) {
+        uint32_t count[kBlkWarps];   // all of them read before the first base is written: one wait instead of sixteen
+#pragma unroll
+        for (uint32_t w = 0; w < kBlkWarps; ++w) count[w] = __popc(s_mask[w * n_cols + tid]);
+        if (kWrap && layered) {
+#pragma unroll
+            for (uint32_t w = 0; w < kBlkWarps; ++w)
+                for (uint32_t q = 0; q < 3; ++q) count[w] += __popc(s_mask[(q + 1) * plane + w * n_cols + tid]) << q;
+        }
         uint32_t run = first;
 #pragma unroll
         for (uint32_t w = 0; w < kBlkWarps; ++w) {
             s_base[w * n_cols + tid] = run;
-            run += __popc(s_mask[w * n_cols + tid]);
-            if (kWrap && layered)
-                for (uint32_t q = 0; q < 3; ++q) run += __popc(s_mask[(q + 1) * plane + w * n_cols + tid]) << q;
+            run += count[w];
         }
     }
     __syncthreads();
     const uint32_t cap = (uint32_t)min(a.capacity, (int64_t)0x7fffffff);
+    // columns of a rectangle that does not wrap: whole nibbles but for its two ends
+    const uint32_t end = b.x0 + b.w, left = (0xfu << (b.x0 & 3u)) & 0xfu, right = 0xfu >> (3u - ((end - 1u) & 3u));
+    const bool straight = !kWrap || end <= a.width;
+    static_assert(kBlkW == 4, "a nibble per row of a block");
     for (uint32_t j = 0; j < kBlkRows; ++j) {
         const uint32_t n = blk_row_cols(b, r0 + j);
         if (n == 0u) continue;
@@ -1398,13 +1412,14 @@ blk_scatter_kernel(BlkArgs a) {
             uint32_t pos = base[s] + __popc(row[s] & lt);
             if (kWrap && layered)
                 for (uint32_t q = 0; q < 3; ++q) pos += __popc(row[(q + 1) * plane + s] & lt) << q;
-            if (pos < cap) a.rec[pos] = make_uint2(rows * blk_col_bits(a, b, s, 0u), entry);
+            const uint32_t cols = straight ? (i == 0u ? left : 0xfu) & (i + 1u == n ? right : 0xfu) : blk_col_bits(a, b, s, 0u);
+            if (pos < cap) a.rec[pos] = make_uint2(rows * cols, entry);
             if (kWrap)
                 for (uint32_t l = 1; l < b.layers; ++l) {
                     const uint32_t m = blk_col_bits(a, b, s, l);
                     if (m != 0u && ++pos < cap) a.rec[pos] = make_uint2(rows * m, entry);
                 }
-            if (++s == a.bx) s = 0;
+            if (++s == a.bx && kWrap) s = 0;
         }
     }
 }
