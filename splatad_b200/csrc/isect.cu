@@ -1571,7 +1571,9 @@ tile_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket, int32_t *__
 // entries: whole 32-byte sectors but for the two ends of a run. (Storing straight from the lanes whose record
 // covers a tile needs no staging, but sectors written in parts cost the L2 more than whole ones and a fifth
 // of the lanes were active: 180 us for the lidar benchmark's 15.3 M entries. A unit of 128 records per
-// warp, its runs not aligned: 73 us; this: 67. Six cameras: 1920 -> 1340 us.)
+// warp, its runs not aligned: 73 us; this: 67. Six cameras: 1920 -> 1340 us, 1310 with two record numbers to a store: the
+// lanes' places lie in any bank, three or four of them in the same. Four entries of a run read before the first is
+// written: 1340 to 1470, the registers cost a CTA.)
 template <uint32_t kWarps>
 __global__ void __launch_bounds__(kWarps * 32)
 tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restrict__ flatten_ids,
@@ -1634,11 +1636,19 @@ tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restr
 #pragma unroll
         for (uint32_t j = 0; j < kBlkWords; ++j) {
             uint32_t w = word[j];
-            while (w) {
-                const uint32_t r = __ffs(w) - 1;
+            const uint32_t first_rec = 32 * (warp * kBlkWords + j);
+            const auto next = [&] {
+                const uint32_t r = first_rec + __ffs(w) - 1;
                 w &= w - 1;
-                s_out[local++] = (uint16_t)(32 * (warp * kBlkWords + j) + r);
+                return r;
+            };
+            if (w != 0u && (local & 1u)) s_out[local++] = (uint16_t)next();
+            while (w & (w - 1)) {   // two at a time: the lanes' places lie in any bank
+                const uint32_t r = next();
+                *reinterpret_cast<uint32_t *>(s_out + local) = r | next() << 16;
+                local += 2;
             }
+            if (w) s_out[local++] = (uint16_t)next();
         }
         __syncthreads();
         for (uint32_t l = warp; l < 32; l += kWarps) {
