@@ -1703,7 +1703,8 @@ rasterize_to_pixels_bwd_kernel(
 }
 
 // ---------------------------------------------------------------------------------------
-// Lidar backward: as the camera's, with two points per thread. Every point has its own elevation and time
+// Lidar backward: as the camera's, with two points per thread. Wraps, signs and caps only where an entry needs care, as in the
+// forward kernels: 64 x 1083, 8 channels 83 -> 72 us, 17 channels 106 -> 95, 32 x 512 68 -> 58. Every point has its own elevation and time
 // offset, so each term is formed per point - in pairs - before the sum over the thread's points goes into
 // the warp totals. `behind` also carries the depth compensation of the range channel.
 // ---------------------------------------------------------------------------------------
@@ -2219,12 +2220,13 @@ constexpr uint64_t kCoopPatches = kNumSMs * 10;
 
 // Warps - segments of the list - per patch in the backward pass: every segment is run twice, which pays
 // while the patches alone leave the schedulers waiting on one warp's chain. One, four and eight segments, us, 8
-// channels: 256 patches 184, 82, 54 (sixteen: 49), 400 174, 74, 60, 544 166, 75, 73, 704 98, 71, 68, 1088 101, 82, 91,
-// 1600 109, 116, 128, 2240 119, 144, 165 (17 channels: 1600 137, 145, 162); so four lose to one from about 1400 on,
-// short of the line below. Sixteen take an SM each, and only up to eight channels stay within their 128 registers.
+// channels: 400 patches 163, 71, 56, 608 121, 61, 57, 800 100, 66, 64, 1088 85, 72, 80, 1600 93, 96, 108, 2240 97, 118, 138, 2816
+// 126, 136, 164 (256: eight 54, sixteen 49); 17 channels: 400 203, 91, 76, 608 152, 78, 74, 800 124, 87, 87, 1088 107, 95,
+// 105, 1600 121, 128, 147, 2240 126, 152, 182. Sixteen take an SM each, and only up to eight channels stay within their 128
+// registers.
 static uint32_t point_segments(uint64_t patches, uint32_t channels) {
     if (channels <= 8 && patches < (uint64_t)kNumSMs * 2) return 16u;
-    return patches < (uint64_t)kNumSMs * 4 ? 8u : patches < (uint64_t)kNumSMs * 16 ? 4u : 1u;
+    return patches < (uint64_t)kNumSMs * 6 ? 8u : patches < (uint64_t)kNumSMs * 9 ? 4u : 1u;
 }
 
 template <typename K>
