@@ -784,15 +784,17 @@ __device__ __forceinline__ PointEntry load_point_entry(int32_t g, const float2 *
 }
 
 // Offsets of a moving mean from the points of a box, [lo, hi]: a range that reaches across half a turn
-// is the whole turn. The slack of a millidegree covers the rounding of the wrapped differences.
-__device__ __forceinline__ void angle_range(float mean, float vel, float centre, float half, float roll_lo, float roll_hi,
+// is the whole turn. The slack of a millidegree covers the rounding of the wrapped differences. Returns how far the offsets
+// reach before any wrap: below half a turn none of them wraps.
+__device__ __forceinline__ float angle_range(float mean, float vel, float centre, float half, float roll_lo, float roll_hi,
                                             float &lo, float &hi) {
     const float a = roll_lo * vel, b = roll_hi * vel;
-    const float d = angle_difference(mean + 0.5f * (a + b), centre);
+    const float m = mean + 0.5f * (a + b), d = angle_difference(m, centre);
     const float reach = half + 0.5f * fabsf(b - a) + 1e-3f;
     lo = d - reach;
     hi = d + reach;
     if (lo < -180.f || hi > 180.f) { lo = -180.f; hi = 180.f; }
+    return fabsf(m - centre) + reach;
 }
 
 // Bit w: the entry may contribute to a point of box w; bit 16 + w: its angles may wrap between mean and point there, or its
@@ -810,13 +812,10 @@ __device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const Po
         const PointBox b = s_box[w];
         if (!(b.az_half >= 0.f)) continue;
         float x_lo, x_hi, y_lo, y_hi;
-        angle_range(e.A.x, e.A.z, b.az, b.az_half, b.roll_lo, b.roll_hi, x_lo, x_hi);
-        angle_range(e.A.y, e.A.w, b.el, b.el_half, b.roll_lo, b.roll_hi, y_lo, y_hi);
+        const float x = angle_range(e.A.x, e.A.z, b.az, b.az_half, b.roll_lo, b.roll_hi, x_lo, x_hi);
+        const float y = angle_range(e.A.y, e.A.w, b.el, b.el_half, b.roll_lo, b.roll_hi, y_lo, y_hi);
         if (test.misses(x_lo, x_hi, y_lo, y_hi)) continue;
         seen |= 1u << w;
-        const float x_a = b.roll_lo * e.A.z, x_b = b.roll_hi * e.A.z, y_a = b.roll_lo * e.A.w, y_b = b.roll_hi * e.A.w;
-        const float x = fabsf(e.A.x + 0.5f * (x_a + x_b) - b.az) + b.az_half + 0.5f * fabsf(x_b - x_a);
-        const float y = fabsf(e.A.y + 0.5f * (y_a + y_b) - b.el) + b.el_half + 0.5f * fabsf(y_b - y_a);
         if (!(plain && x < 179.9f && y < 179.9f)) seen |= 1u << (w + kCarefulShift);
     }
     return seen;
@@ -825,7 +824,7 @@ __device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const Po
 // Offset of an entry from a point and its exp(-sigma); sigma decides with alpha whether it is blended. Every kernel rounds
 // the steps alike - one or two values at a time, and the transmittances' factors as T * (1 - alpha) -, because the median
 // range of a point is that of the entry at which its transmittance crosses a half: the last bit decides between two
-// ranges that may lie far apart. Where nothing wraps the differences are rounded as angle_difference() rounds them.
+// ranges that may lie far apart.
 struct PointFootprint { float dx, dy, sigma, vis; };
 
 __device__ __forceinline__ float point_sigma(const float4 &B, float dx, float dy) {
@@ -836,12 +835,11 @@ __device__ __forceinline__ float2 point_sigma(float2 a, float2 b, float2 c, floa
     return __ffma2_rn(__fmul2_rn(b, dx), dy, __fmul2_rn(make_float2(0.5f, 0.5f), square));
 }
 
-template <bool kWraps>
 __device__ __forceinline__ PointFootprint point_footprint(const float4 &A, const float4 &B, float roll, float az, float el) {
     PointFootprint f;
     const float mx = fmaf(roll, A.z, A.x), my = fmaf(roll, A.w, A.y);
-    f.dx = kWraps ? angle_difference(mx, az) : (mx - az + 180.f) - 180.f;
-    f.dy = kWraps ? angle_difference(my, el) : (my - el + 180.f) - 180.f;
+    f.dx = angle_difference(mx, az);
+    f.dy = angle_difference(my, el);
     f.sigma = point_sigma(B, f.dx, f.dy);
     f.vis = __expf(-f.sigma);
     return f;
@@ -867,8 +865,8 @@ __device__ __forceinline__ void stage_features(float *row, const float *__restri
 // Lidar forward. One point per lane; a warp looks only at the entries that can reach its patch (a ninth
 // of the (point, entry) pairs of a small scan contribute, two thirds of the benchmark's) and evaluates
 // two of them at a time, because what it waits for is the chain from the offsets through the exponential
-// to the transmittance. The wrap of the angles, the sign of sigma and the cap of the alphas are looked at only where the
-// staging thread cannot rule them out (64 x 1083: 58 -> 53 us). The rendered rows leave through shared memory: a beam's eight points
+// to the transmittance. (Leaving the wrap, the sign of sigma and the cap to the entries that need them, as the other
+// lidar kernels do, gains nothing here: 128 x 1800 43.3 -> 44.4 us.) The rendered rows leave through shared memory: a beam's eight points
 // are consecutive floats.
 // ---------------------------------------------------------------------------------------
 // entries per thread and batch (their loads overlap), while the shared memory of a batch stays small
@@ -892,9 +890,6 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
     float *__restrict__ median_depths) {
     chain_enter();
     constexpr uint32_t kStage = points_fwd_stage(CDIM);
-    // whether an entry needs care is looked up first; with many channels the registers it takes cost more than it saves
-    // (17 channels, 128 x 1800: 40.0 and 41.6 us)
-    constexpr bool kLookFirst = CDIM <= 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ PointBox s_box[8];
     __shared__ uint32_t s_warp_kept[kStage * 16];
@@ -1012,32 +1007,19 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
             T = next_T;
         };
         for (uint32_t t0 = 0; t0 < n_kept && !warp_done; t0 += 32) {
-            const uint32_t mine = t0 + lane, seen_by = mine < n_kept ? sSeen[mine] >> warp : 0u;
-            uint32_t todo = __ballot_sync(0xffffffffu, seen_by & 1u);
-            const uint32_t careful = __ballot_sync(0xffffffffu, (seen_by >> kCarefulShift) & 1u);
+            const uint32_t mine = t0 + lane;
+            uint32_t todo = __ballot_sync(0xffffffffu, mine < n_kept && ((sSeen[mine] >> warp) & 1u));
             while (todo && !(warp_done = __all_sync(0xffffffffu, done))) {
                 // two entries at a time; an odd one out is evaluated twice and blended once
-                uint32_t bits = todo & (0u - todo);
                 const uint32_t t = t0 + (uint32_t)__ffs(todo) - 1u;
                 todo &= todo - 1u;
                 const bool two = todo != 0u;
                 const uint32_t u = two ? t0 + (uint32_t)__ffs(todo) - 1u : t;
-                bits |= todo & (0u - todo);
                 todo &= todo - 1u;   // of 0: stays 0
                 const float4 A0 = sA[t], B0 = sB[t], A1 = sA[u], B1 = sB[u];
-                PointFootprint f0 = point_footprint<!kLookFirst>(A0, B0, roll, px, py), f1 = point_footprint<!kLookFirst>(A1, B1, roll, px, py);
-                float alpha0 = B0.w * f0.vis, alpha1 = B1.w * f1.vis;
-                bool ok0 = alpha0 >= kAlphaMin, ok1 = two && alpha1 >= kAlphaMin;
-                if (!kLookFirst || (careful & bits)) {
-                    if (kLookFirst) {
-                        f0 = point_footprint<true>(A0, B0, roll, px, py);
-                        f1 = point_footprint<true>(A1, B1, roll, px, py);
-                    }
-                    alpha0 = fminf(kAlphaMax, B0.w * f0.vis);
-                    alpha1 = fminf(kAlphaMax, B1.w * f1.vis);
-                    ok0 = !(f0.sigma < 0.f || alpha0 < kAlphaMin);
-                    ok1 = two && !(f1.sigma < 0.f || alpha1 < kAlphaMin);
-                }
+                const PointFootprint f0 = point_footprint(A0, B0, roll, px, py), f1 = point_footprint(A1, B1, roll, px, py);
+                const float alpha0 = fminf(kAlphaMax, B0.w * f0.vis), alpha1 = fminf(kAlphaMax, B1.w * f1.vis);
+                const bool ok0 = !(f0.sigma < 0.f || alpha0 < kAlphaMin), ok1 = two && !(f1.sigma < 0.f || alpha1 < kAlphaMin);
                 if (ok0 && !done) blend(t, f0, alpha0);
                 if (ok1 && !done) blend(u, f1, alpha1);
             }
@@ -1250,7 +1232,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_co
                         const float *q = sE + t;
                         const float4 A = make_float4(q[0], q[kThreadsC], q[2 * kThreadsC], q[3 * kThreadsC]);
                         const float4 B = make_float4(q[4 * kThreadsC], q[5 * kThreadsC], q[6 * kThreadsC], q[7 * kThreadsC]);
-                        const PointFootprint f = point_footprint<true>(A, B, roll, px, py);
+                        const PointFootprint f = point_footprint(A, B, roll, px, py);
                         const float a = fminf(kAlphaMax, B.w * f.vis), x = f.dx, y = f.dy;
                         alpha[k] = f.sigma < 0.f || a < kAlphaMin ? 0.f : a;
                         if (k & 1) { dx[k / 2].y = x; dy[k / 2].y = y; } else { dx[k / 2].x = x; dy[k / 2].x = y; }
@@ -1781,7 +1763,7 @@ __device__ __noinline__ void odd_points_bwd(const PointTask &a, const PointGrads
             const size_t g = (size_t)a.flatten_ids[idx];
             const PointEntry e = load_point_entry((int32_t)g, a.means2d, a.conics, a.opacities, a.pix_vels, a.depth_comps);
             const float range = a.ranges ? a.ranges[g] : a.colors[g * n + a.depth_idx];
-            const PointFootprint f = point_footprint<true>(e.A, e.B, pt.w, pt.x, pt.y);
+            const PointFootprint f = point_footprint(e.A, e.B, pt.w, pt.x, pt.y);
             const float alpha = fminf(kAlphaMax, e.B.w * f.vis);
             const bool ok = idx <= last && !(f.sigma < 0.f || alpha < kAlphaMin);
             if (!__any_sync(0xffffffffu, ok)) continue;
@@ -2023,7 +2005,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
             alpha = __fmul2_rn(make_float2(B.w, B.w), vis);
             bool ok0 = alpha.x >= kAlphaMin, ok1 = alpha.y >= kAlphaMin;
             if (id < 0) {
-                const PointFootprint f0 = point_footprint<true>(A, B, roll.x, az.x, el.x), f1 = point_footprint<true>(A, B, roll.y, az.y, el.y);
+                const PointFootprint f0 = point_footprint(A, B, roll.x, az.x, el.x), f1 = point_footprint(A, B, roll.y, az.y, el.y);
                 dx = make_float2(f0.dx, f1.dx);
                 dy = make_float2(f0.dy, f1.dy);
                 vis = make_float2(f0.vis, f1.vis);
