@@ -151,3 +151,47 @@ def test_a_nan_in_the_geometry_is_blended_with_the_capped_alpha(what, channels):
         assert np.array_equal(np.isfinite(got), np.isfinite(ref_k)), k
         got, ref_k = np.nan_to_num(got).astype(np.float64), np.nan_to_num(ref_k)
         assert np.linalg.norm(got - ref_k) <= 2e-3 * max(np.linalg.norm(ref_k), 1e-20), k
+
+
+@pytest.mark.parametrize("C,channels,mode", [(1600, 3, "x"), (1600, 7, "x"), (1600, 18, "x"), (3200, 4, "y"), (6400, 3, "y")])
+@pytest.mark.parametrize("value", [INF, NAN])
+def test_a_colour_that_is_not_finite_and_hidden_reaches_nothing(C, channels, mode, value):
+    """One half of every tile stops early; a Gaussian behind that has a colour that is not finite and does not reach the other half,
+    which blends one further behind. Nobody blends it: image and gradients are those of a finite colour and its own
+    gradients are zero, also where the backward pass works on both halves at once and the forward pass on each by itself."""
+    from gpu_util import t
+    from splatad_b200 import ops
+    layers, bad, last = 150, 150, 151
+    along, across = (0, 1) if mode == "x" else (1, 0)
+    means = torch.full((layers + 2, 2), 8.0)
+    means[:bad, along], means[bad, along], means[last, along] = 4.0, 3.0, 13.0
+    tight, wide = torch.full((layers + 2,), 0.3), torch.full((layers + 2,), 1e-4)   # (1/px^2) along the split and across it
+    tight[bad], tight[last] = 4.0, 1.0
+    conics = torch.zeros(layers + 2, 3)
+    conics[:, 0], conics[:, 2] = (tight, wide) if mode == "x" else (wide, tight)
+    g = torch.Generator().manual_seed(channels)
+    colors = torch.rand(layers + 2, channels, generator=g)
+    opacities = torch.full((layers + 2,), 0.95)
+    n = layers + 2
+    fixed = dict(means2d=means, conics=conics, opacities=opacities, pix_vels=torch.zeros(n, 2))
+    offsets = t(torch.arange(C)[:, None, None] * n, torch.int32)
+    ids = t(torch.arange(C * n), torch.int32)
+    weights = [t(torch.randn(1, 16, 16, k, generator=g)).expand(C, -1, -1, -1).contiguous() for k in (channels, 1)]
+
+    def run(bad_colour):
+        c = colors.clone()
+        c[bad] = bad_colour
+        p = {k: t(v)[None].expand(C, *v.shape).contiguous().requires_grad_(True) for k, v in dict(colors=c, **fixed).items()}
+        out = ops.rasterize_to_pixels(p["means2d"], p["conics"], p["colors"], p["opacities"], p["pix_vels"], 16, 16, 16,
+                                      offsets, ids, torch.zeros(C, device=DEV), absgrad=True)
+        torch.autograd.backward(out, weights)
+        return [o.detach() for o in out], {**{k: v.grad for k, v in p.items()}, "absolute": p["means2d"].absgrad}
+
+    out, want = run(0.5)
+    assert float(want["colors"][:, bad].abs().max()) == 0.0 and float(want["colors"][:, last].abs().min()) > 0.0
+    spoilt, got = run(value)
+    for a, b in zip(out, spoilt):
+        _close(b, a, 1e-6)                 # as above: in whichever way the tile is worked out
+    for k in want:
+        assert torch.isfinite(got[k]).all() and float(got[k][:, bad].abs().max()) == 0.0, k
+        _close(got[k], want[k], 1e-5)      # sums over a tile in another order
