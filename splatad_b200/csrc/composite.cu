@@ -748,12 +748,18 @@ struct PointBox { float az, az_half, el, el_half, roll_lo, roll_hi; };
 
 struct PointExtent {
     float az0 = 3.0e38f, az1 = -3.0e38f, el0 = 3.0e38f, el1 = -3.0e38f, r0 = 3.0e38f, r1 = -3.0e38f;
+    float none = 0.f;   // a NaN: a coordinate that is not finite
+    template <bool kOdd = true>
     __device__ __forceinline__ void add(float az, float el, float roll) {
         az0 = fminf(az0, az); az1 = fmaxf(az1, az);
         el0 = fminf(el0, el); el1 = fmaxf(el1, el);
         r0 = fminf(r0, roll); r1 = fmaxf(r1, roll);
+        if (kOdd) none = fmaf(az, 0.f, fmaf(el, 0.f, fmaf(roll, 0.f, none)));
     }
-    // the box of the whole warp, in every lane; no points: a negative half width
+    // The box of the whole warp, in every lane; no points: a negative half width. A point with a coordinate that is not
+    // finite takes every entry with the capped alpha: no offset is ruled out where the centre is not a number. (The
+    // backward pass has such patches marked and works on them elsewhere.)
+    template <bool kOdd = true>
     __device__ __forceinline__ PointBox warp_box() {
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -761,10 +767,12 @@ struct PointExtent {
             el0 = fminf(el0, __shfl_xor_sync(0xffffffffu, el0, off)); el1 = fmaxf(el1, __shfl_xor_sync(0xffffffffu, el1, off));
             r0 = fminf(r0, __shfl_xor_sync(0xffffffffu, r0, off)); r1 = fmaxf(r1, __shfl_xor_sync(0xffffffffu, r1, off));
         }
+        if (kOdd && __any_sync(0xffffffffu, none != 0.f)) return {NAN, 0.f, 0.f, 0.f, 0.f, 0.f};
         return {0.5f * (az0 + az1), 0.5f * (az1 - az0), 0.5f * (el0 + el1), 0.5f * (el1 - el0), r0, r1};
     }
+    template <bool kOdd = true>
     __device__ __forceinline__ void write_box(PointBox *box) {   // by the warp's first lane
-        const PointBox b = warp_box();
+        const PointBox b = warp_box<kOdd>();
         if ((threadIdx.x & 31u) == 0u) *box = b;
     }
 };
@@ -806,9 +814,10 @@ __device__ __forceinline__ float angle_range(float mean, float vel, float centre
 // alphas need looking at one by one (as kCarefulEntry for the cameras).
 constexpr uint32_t kCarefulShift = 16;
 
+template <bool kOdd = true>   // kOdd: a box without a centre sees every entry
 __device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const PointBox *s_box, uint32_t n_boxes) {
     const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
-    if (test.never) return 0u;
+    if (!kOdd && test.never) return 0u;
     const float ac = e.B.x * e.B.z;
     const bool plain = e.B.x > 1e-15f && e.B.z > 1e-15f && e.B.x < 1e15f && e.B.z < 1e15f && ac - e.B.y * e.B.y >= 1e-5f * ac &&
                        e.B.w <= kAlphaMax;
@@ -819,7 +828,7 @@ __device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const Po
         float x_lo, x_hi, y_lo, y_hi;
         const float x = angle_range(e.A.x, e.A.z, b.az, b.az_half, b.roll_lo, b.roll_hi, x_lo, x_hi);
         const float y = angle_range(e.A.y, e.A.w, b.el, b.el_half, b.roll_lo, b.roll_hi, y_lo, y_hi);
-        if (test.misses(x_lo, x_hi, y_lo, y_hi)) continue;
+        if (!(kOdd && b.az != b.az) && test.misses(x_lo, x_hi, y_lo, y_hi)) continue;
         seen |= 1u << w;
         if (!(plain && x < 179.9f && y < 179.9f)) seen |= 1u << (w + kCarefulShift);
     }
@@ -1902,7 +1911,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
             rp = raster_pts[pix];
             if (rp.z <= 0.f) in = false;
         }
-        if (in) extent.add(rp.x, rp.y, rp.w);
+        if (in) extent.add<false>(rp.x, rp.y, rp.w);
         const float T_final = in ? 1.f - render_alphas[pix] : 1.f;
         bin_final[h] = in ? last_ids[pix] : -1;
         thread_last = (in && bin_final[h] < 0) ? INT32_MAX : max(thread_last, bin_final[h]);
@@ -1924,7 +1933,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         if (h) { az.y = rp.x; el.y = rp.y; roll.y = rp.w; T.y = T_final; behind.y = last; v_depth.y = vd; v_asum.y = vs; sum_limit.y = limit; }
         else { az.x = rp.x; el.x = rp.y; roll.x = rp.w; T.x = T_final; behind.x = last; v_depth.x = vd; v_asum.x = vs; sum_limit.x = limit; }
     }
-    if (warp == 0) extent.write_box(&s_box);
+    if (warp == 0) extent.write_box<false>(&s_box);
 
     // last list position consumed by any of the patch's points
     const int32_t patch_last = __reduce_max_sync(0xffffffffu, none != 0.f ? INT32_MAX : thread_last);
@@ -1977,7 +1986,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         // survivors to the front, still back to front in list order
 #pragma unroll
         for (uint32_t q = 0; q < kStage; ++q) {
-            seen[q] = batch_end - (int32_t)(q * bs + tr) >= range.start ? boxes_that_see(e[q], &s_box, 1u) : 0u;
+            seen[q] = batch_end - (int32_t)(q * bs + tr) >= range.start ? boxes_that_see<false>(e[q], &s_box, 1u) : 0u;
             kept[q] = __ballot_sync(0xffffffffu, seen[q] != 0u);
             if (lane == 0) s_warp_kept[q * n_warps + warp] = __popc(kept[q]);
         }

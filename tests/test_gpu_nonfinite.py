@@ -195,3 +195,45 @@ def test_a_colour_that_is_not_finite_and_hidden_reaches_nothing(C, channels, mod
     for k in want:
         assert torch.isfinite(got[k]).all() and float(got[k][:, bad].abs().max()) == 0.0, k
         _close(got[k], want[k], 1e-5)      # sums over a tile in another order
+
+
+@pytest.mark.parametrize("C,channels", [(1, 5), (9, 5), (1, 18), (9, 18)])
+@pytest.mark.parametrize("coordinate", [0, 1, 3])
+@pytest.mark.parametrize("value", [NAN, INF])
+def test_a_lidar_point_that_is_not_finite_blends_the_first_entry(C, channels, coordinate, value):
+    """A point without an azimuth, an elevation or a time, among points that have them and in a patch of nothing else: as in the
+    oracle it takes the first entry of its list with the capped alpha and a range that is not a number, in scans whose
+    warps share a patch and in those whose do not. The Gaussians that it does not blend get the gradients of the others."""
+    import numpy as np
+    from gpu_util import assert_close, n, t
+    from oracle import composite
+    from splatad_b200 import ops
+    from test_gpu_composite import _lidar_case
+    H, W, tw, th = 64, 320, 32, 8          # 640 patches a sensor
+    c = _lidar_case(C, 600, H, W, tw, th, channels, 11 * C + channels)
+    c["pts"][:, 5, 7, 2] = 20.0            # alone in its patch
+    c["pts"][:, 5, 7, coordinate] = value
+    c["pts"][:, 32:36, 200:208, 2] = 20.0  # a whole patch
+    c["pts"][:, 32:36, 200:208, coordinate] = value
+    spoilt = ~torch.isfinite(c["pts"]).all(-1).numpy()
+    keys = ("means2d", "conics", "feats", "opacities", "pix_vels", "dcomp")
+    args = [n(c[k]) for k in keys] + [None, n(c["pts"]), W, H, tw, th, c["offsets"], c["flatten_ids"], True, 0.5]
+    ref = composite.rasterize_to_points_fwd(*args, amb_tol=1e-4)
+    assert np.isnan(ref["render_colors"][spoilt][:, -1]).all() and (ref["render_alphas"][spoilt] > 0.9).all()
+    leaves = {k: t(c[k]).requires_grad_(True) for k in keys}
+    image, alphas, sums, medians = ops.rasterize_to_points(
+        *(leaves[k] for k in keys), t(c["pts"]), W, H, tw, th, t(c["offsets"], torch.int32), t(c["flatten_ids"], torch.int32), True, 0.5)
+    sure = ~ref["ambiguous"] | spoilt
+    for got, want in ((image, ref["render_colors"]), (alphas, ref["render_alphas"]), (sums, ref["alpha_sum"])):
+        got, want = n(got), want.reshape(n(got).shape)
+        assert np.array_equal(np.isnan(got[sure]), np.isnan(want[sure]))
+        assert_close("points", np.nan_to_num(got), np.nan_to_num(want), 2e-4, 2e-5, mask=sure[..., None])
+    torch.autograd.backward([image, alphas], [torch.ones_like(image), torch.ones_like(alphas)])
+    f64 = composite.rasterize_to_points_fwd(*args, dtype=np.float64)
+    want = composite.rasterize_to_points_bwd(*args, f64["render_alphas"], f64["last_ids"], np.ones(n(image).shape),
+                                             np.ones(n(alphas).shape), np.zeros(n(alphas).shape))
+    same = (f64["last_ids"] == ref["last_ids"]).mean()
+    assert same > 0.99
+    for k, name in zip(keys, ("v_means2d", "v_conics", "v_colors", "v_opacities", "v_pix_vels", "v_depth_comps")):
+        got, ref_k = n(leaves[k].grad), want[name].reshape(leaves[k].shape)
+        assert np.array_equal(np.isfinite(got), np.isfinite(ref_k)), k
