@@ -23,14 +23,27 @@
 
 namespace splatad {
 
+// Infinities and NaNs become zeros.
+__device__ __forceinline__ float finite_or_zero(float v) { return fabsf(v) < INFINITY ? v : 0.f; }
+__device__ __forceinline__ float4 finite_or_zero(float4 v) {
+    return make_float4(finite_or_zero(v.x), finite_or_zero(v.y), finite_or_zero(v.z), finite_or_zero(v.w));
+}
+
 // Copies row g of a [*, n] float table to dst (one thread per row), zero-padded to a multiple of
 // four floats: 16-byte loads when the rows are 16-byte aligned.
+template <bool kFinite = false>
 __device__ __forceinline__ void stage_row(float *__restrict__ dst, const float *__restrict__ table,
                                           size_t g, uint32_t n, bool vec) {
     const float *src = table + g * n;
     if (vec) {
+        for (uint32_t k = 0; k < n; k += 4) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(src + k));
+            *reinterpret_cast<float4 *>(dst + k) = kFinite ? finite_or_zero(v) : v;
+        }
+    } else if (kFinite) {
         for (uint32_t k = 0; k < n; k += 4)
-            *reinterpret_cast<float4 *>(dst + k) = __ldg(reinterpret_cast<const float4 *>(src + k));
+            *reinterpret_cast<float4 *>(dst + k) = finite_or_zero(make_float4(
+                __ldg(src + k), k + 1 < n ? __ldg(src + k + 1) : 0.f, k + 2 < n ? __ldg(src + k + 2) : 0.f, k + 3 < n ? __ldg(src + k + 3) : 0.f));
     } else {
         const uint32_t npad = (n + 3u) & ~3u;
         for (uint32_t k = 0; k < npad; ++k) dst[k] = k < n ? __ldg(src + k) : 0.f;
@@ -342,11 +355,9 @@ __device__ __noinline__ void odd_pixels_bwd(const PixelTask &a, uint32_t gtile, 
     }
 }
 
-// A row of n floats to shared memory, zeros behind them: all loads are on their way before the first is waited for. Returns
-// whether all of them are finite.
-template <int CDIM>
-__device__ __forceinline__ bool stage_whole_row(float4 *dst, const float *__restrict__ src, uint32_t n, bool vec) {
-    float2 none = make_float2(0.f, 0.f);
+// A row of n floats to shared memory, zeros behind them: all loads are on their way before the first is waited for.
+template <int CDIM, bool kFinite = false>
+__device__ __forceinline__ void stage_whole_row(float4 *dst, const float *__restrict__ src, uint32_t n, bool vec) {
 #pragma unroll
     for (int k = 0; k < CDIM; k += 4) {
         float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -358,11 +369,8 @@ __device__ __forceinline__ bool stage_whole_row(float4 *dst, const float *__rest
             if ((uint32_t)k + 2u < n) w.z = __ldg(src + k + 2);
             if ((uint32_t)k + 3u < n) w.w = __ldg(src + k + 3);
         }
-        dst[k / 4] = w;
-        none = __ffma2_rn(make_float2(w.x, w.y), make_float2(0.f, 0.f), none);
-        none = __ffma2_rn(make_float2(w.z, w.w), make_float2(0.f, 0.f), none);
+        dst[k / 4] = kFinite ? finite_or_zero(w) : w;
     }
-    return none.x + none.y == 0.f;
 }
 
 // Rows of n floats, whole 16-byte pieces, between a table and a warp's shared memory, where row r lies at r * CDIM: lane r
@@ -1566,24 +1574,21 @@ rasterize_to_pixels_bwd_kernel(
             seen = patch_sees<false>(e, box, roll_lo, roll_hi);
         }
         uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
+        const uint32_t careful = __ballot_sync(0xffffffffu, seen > kSeenEntry);
         __syncwarp();   // the batch before has been read
         if (seen) {
             sA[lane] = e.A;
             sB[lane] = scaled_conic(e.B);
             sId[lane] = make_float2(__int_as_float(g), 1.f / e.B.w);
-            bool finite = true;
-            if (CDIM <= 16) finite = stage_whole_row<CDIM>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, vec);
+            // A colour that is not finite is blended by no pixel of the patch - it would have left its mark there. It may lie
+            // behind the last entry of some pixels and out of reach of the others, and must not meet their weights of zero.
+            if (CDIM <= 16) stage_whole_row<CDIM, true>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, vec);
             else {   // (20 channels: all loads of a row at once take registers, 990 -> 1130 us)
                 float *row = reinterpret_cast<float *>(sCol) + lane * CDIM;
-                stage_row(row, colors, (size_t)g, channels, vec);
+                stage_row<true>(row, colors, (size_t)g, channels, vec);
                 for (uint32_t k = (channels + 3u) & ~3u; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
-                float none = 0.f;
-                for (uint32_t k = 0; k < (uint32_t)CDIM; ++k) none = fmaf(row[k], 0.f, none);
-                finite = none == 0.f;
             }
-            if (!finite) seen |= kCarefulEntry;
         }
-        const uint32_t careful = __ballot_sync(0xffffffffu, seen > kSeenEntry);
         __syncwarp();
         while (todo) {
             const uint32_t t = (uint32_t)__ffs(todo) - 1u, bit = 1u << t;
@@ -1625,12 +1630,6 @@ rasterize_to_pixels_bwd_kernel(
                     alpha[q].x = pw.x <= 0.f ? fminf(kAlphaMax, alpha[q].x) : 0.f;
                     alpha[q].y = pw.y <= 0.f ? fminf(kAlphaMax, alpha[q].y) : 0.f;
                 }
-                // A colour that is not finite, blended by a pixel of the patch, has left its mark there. Blended by none - behind
-                // the last entry of some pixels and out of reach of the others - it must not meet a weight of zero.
-                float most = 0.f;
-#pragma unroll
-                for (int q = 0; q < P2; ++q) most = fmaxf(most, fmaxf(alpha[q].x, alpha[q].y));
-                if (!__any_sync(0xffffffffu, most > 0.f)) continue;
             }
 #pragma unroll
             for (int q = 0; q < P2; ++q) {
