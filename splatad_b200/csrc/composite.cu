@@ -373,11 +373,27 @@ __device__ __forceinline__ void stage_whole_row(float4 *dst, const float *__rest
     }
 }
 
+__device__ __forceinline__ void async_copy(float *dst_smem, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst_smem)), "l"(__cvta_generic_to_global(src)) : "memory");
+}
+__device__ __forceinline__ void async_copy_16(float *dst_smem, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst_smem)), "l"(__cvta_generic_to_global(src)) : "memory");
+}
+__device__ __forceinline__ void async_copy_row(float *dst_smem, const float *__restrict__ src, uint32_t n, bool vec) {
+    if (vec)
+        for (uint32_t k = 0; k < n; k += 4) async_copy_16(dst_smem + k, src + k);
+    else
+        for (uint32_t k = 0; k < n; ++k) async_copy(dst_smem + k, src + k);
+}
+__device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Rows of n floats, whole 16-byte pieces, between a table and a warp's shared memory, where row r lies at r * CDIM: lane r
 // names the table's row for it, `mask` the rows that are wanted. The lanes go over the rows' pieces in
 // sequence, so that one access touches a few lines; a lane that copies a row by itself touches as many lines
-// with every access as there are lanes. Pays for wide rows in 16-byte pieces: forward kernel, 1920 x 1080, 32 channels 727 -> 583 us,
-// 20 channels 396 -> 389; 13 channels, one float at a time, 323 -> 404.
+// with every access as there are lanes. Copies to shared memory are asynchronous: none waits for the one before. Forward kernel, a lane
+// per row, rows together, rows together and asynchronous: 1920 x 1080, 32 channels 727, 543, 506 us, 20 channels 396, 408, 377; 640 x 360 and 20
+// channels 111 and 91 (together, asynchronous). One float at a time, of rows that are no multiple of 16 bytes, 13 channels: 297 -> 334, 25: 617 -> 643; the
+// backward kernel has no registers for it (20 channels, two pixels: 950 -> 1128).
 template <int CDIM, bool kStore>
 __device__ __forceinline__ void copy_rows(float *rows, std::conditional_t<kStore, float, const float> *table, int32_t row_id,
                                           uint32_t mask, uint32_t n, uint32_t lane) {
@@ -386,14 +402,21 @@ __device__ __forceinline__ void copy_rows(float *rows, std::conditional_t<kStore
     for (uint32_t round = 0; round < pieces; ++round) {
         const size_t id = (size_t)__shfl_sync(0xffffffffu, row_id, r);
         if ((mask >> r) & 1u) {
-            auto *there = reinterpret_cast<std::conditional_t<kStore, float4, const float4> *>(table + id * n) + k;
-            float4 *here = reinterpret_cast<float4 *>(rows + r * CDIM) + k;
-            if constexpr (kStore) *there = *here; else *here = __ldg(there);
+            auto *there = table + id * n + 4u * k;
+            float *here = rows + r * CDIM + 4u * k;
+            if constexpr (kStore) *reinterpret_cast<float4 *>(there) = *reinterpret_cast<const float4 *>(here);
+            else async_copy_16(here, there);
         }
         r += skip;
         k += rest;
         if (k >= pieces) { k -= pieces; ++r; }
     }
+}
+
+template <int CDIM>
+__device__ __forceinline__ void stage_rows(float *rows, const float *table, int32_t row_id, uint32_t mask, uint32_t n, uint32_t lane) {
+    copy_rows<CDIM, false>(rows, table, row_id, mask, n, lane);
+    async_wait_all();
 }
 
 // The values of a thread's PX pixels, next to each other in memory: in 16-byte pieces where they lie so. One float at a
@@ -509,7 +532,9 @@ constexpr int pixels_fwd_regs(int cdim, int px) {
     return cdim <= 4 ? (px == 8 ? 128 : px == 4 ? 80 : 64) : cdim <= 8 ? (px == 4 ? 96 : 72) : cdim <= 16 ? (px == 4 ? 128 : 96) : cdim <= 20 ? 96 : 128;
 }
 
-template <int CDIM, int PX>
+// kTogether: rows in 16-byte pieces, staged by copy_rows(). A kernel of its own: with both ways in one, 1920 x 1080 and 32 channels
+// take 648 us instead of 506.
+template <int CDIM, int PX, bool kTogether>
 __global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX)) rasterize_to_pixels_fwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
@@ -561,8 +586,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX)) rasterize_to_pixels_fwd_k
     }
 #pragma unroll
     for (int k = 0; k < PX; ++k) pos[k] = 0;
-    const bool together = CDIM >= 20 && vec;   // see copy_rows()
-    if (together)
+    if (kTogether)
         for (uint32_t k = channels; k < (uint32_t)CDIM; ++k) reinterpret_cast<float *>(sCol)[lane * CDIM + k] = 0.f;
     uint32_t odd = 0u;   // kOddEntry: the warp was to blend one
     bool done = __all_sync(0xffffffffu, n_inside == 0);
@@ -586,9 +610,9 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX)) rasterize_to_pixels_fwd_k
         if (seen) {
             sA[lane] = e.A;
             sB[lane] = scaled_conic(make_float4(e.B.x, e.B.y, e.B.z, -e.B.w));
-            if (!together) stage_whole_row<CDIM>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, vec);
+            if (!kTogether) stage_whole_row<CDIM>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, CDIM < 20 && vec);
         }
-        if (together) copy_rows<CDIM, false>(reinterpret_cast<float *>(sCol), colors, g, todo, channels, lane);
+        if (kTogether) stage_rows<CDIM>(reinterpret_cast<float *>(sCol), colors, g, todo, channels, lane);
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < PX; ++k) blended[k] = 0u;
@@ -676,7 +700,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX)) rasterize_to_pixels_fwd_k
             if (expected && expected_depths != nullptr) store_pixels<PX>(expected_depths + pix, depths, n_inside);
         }
     } else {   // one pixel after the other: all at once costs the 16-channel kernel 13 us in registers
-        const bool drawn_together = together && (reinterpret_cast<uintptr_t>(render_colors) & 15u) == 0u;
+        const bool drawn_together = kTogether && (reinterpret_cast<uintptr_t>(render_colors) & 15u) == 0u;
         float4 *row = sCol + lane * (CDIM / 4);
 #pragma unroll
         for (int h = 0; h < PX; ++h) {
@@ -1100,18 +1124,6 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
 // four, which rounds differently: 32).
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t kCoopWarps = 8, kCoopShare = 4, kCoopChunk = kCoopWarps * kCoopShare;
-
-__device__ __forceinline__ void async_copy(float *dst_smem, const float *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst_smem)), "l"(__cvta_generic_to_global(src)) : "memory");
-}
-__device__ __forceinline__ void async_copy_row(float *dst_smem, const float *__restrict__ src, uint32_t n, bool vec) {
-    if (vec)
-        for (uint32_t k = 0; k < n; k += 4)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst_smem + k)), "l"(__cvta_generic_to_global(src + k)) : "memory");
-    else
-        for (uint32_t k = 0; k < n; ++k) async_copy(dst_smem + k, src + k);
-}
-__device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __device__ __forceinline__ float2 half_of(const float4 &v, int h) { return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y); }
 
@@ -2286,8 +2298,9 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
 #define CALL_PX(D, P)                                                                             \
     {                                                                                             \
         const uint32_t patches = div_up(tile_threads<P>(tile_size), 32);                          \
+        const auto kernel = D >= 20 && vec ? rasterize_to_pixels_fwd_kernel<D, P, (D >= 20)> : rasterize_to_pixels_fwd_kernel<D, P, false>; \
         SPL_REQUIRE((uint64_t)blocks * patches <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_fwd: too many tiles"); \
-        launch_chained_if(warps_fit_at_once((uint64_t)blocks * patches), rasterize_to_pixels_fwd_kernel<D, P>, blocks * patches, 32, 0, \
+        launch_chained_if(warps_fit_at_once((uint64_t)blocks * patches), kernel, blocks * patches, 32, 0, \
             (cudaStream_t)stream,                                                                 \
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
@@ -2298,6 +2311,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
 #define CALL(D)                                                                                   \
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2)) else if (D <= 16 && px == 4) CALL_PX(D, (D <= 16 ? 4 : 2)) else CALL_PX(D, 2)
     const uint32_t px = pixels_per_lane_fwd(blocks, tile_size, channels);
+    const bool vec = channels % 4u == 0u && (reinterpret_cast<uintptr_t>(colors) & 15u) == 0u;
     {
         SPL_PROF("rasterize_to_pixels_fwd_kernel", (cudaStream_t)stream);
         SPL_DISPATCH_CDIM(channels, CALL);
