@@ -355,6 +355,12 @@ int splatad_isect_lidar_tiles_fill(
  * device nothing is written and the host waits for host_counts as usual. NULL disarms. */
 int splatad_isect_set_early_count(int64_t *host_pair, int64_t sequence);
 
+/* No counterpart in the reference. Arms a one-shot request for the NEXT _plan call of the calling
+ * thread with sort = 1 and an early count armed: *host_word, pinned (mapped) host memory, receives the
+ * number of elements that the lists hold at least once, before the sequence number of the early
+ * count. NULL disarms. */
+int splatad_isect_set_listed_count(int64_t *host_word);
+
 /* No counterpart in the reference. Arms a one-shot hint for the NEXT _plan call of the calling
  * thread with sort = 1: the depths of the elements it will list are expected within
  * [depth_lo, depth_hi], given as the bit patterns of two non-negative finite floats (the range the
@@ -415,6 +421,12 @@ int splatad_populate_image_from_points(
  * Compositing. `channels` is the true channel count (1..SPLATAD_MAX_CHANNELS): no padding to
  * a supported size is needed, unlike gsplat/cuda/_wrapper.py:876-921.
  * ---------------------------------------------------------------------------------------- */
+
+/* No counterpart in the reference. Arms a one-shot hint for the NEXT camera compositing call of the calling
+ * thread, forward or backward: list entries per Gaussian that the lists hold, as far as the caller knows
+ * it (0: not known, the number of tiles decides alone). It chooses how many pixels a lane draws and cannot change an image;
+ * gradients are the same sums in another order. */
+int splatad_rasterize_set_spread_hint(float tiles_per_gaussian);
 
 /* rasterize_to_pixels_fwd_tensor - gsplat/cuda/csrc/rasterization.cu:1520-2019, kernel
  * 1360-1518. Inputs are [C,N,..] or packed [nnz,..] (flatten_ids index either);

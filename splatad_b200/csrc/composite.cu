@@ -1462,14 +1462,26 @@ __device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t
 // 640 x 360, two pixels: 159, 174, 136, 148, 282 -> 106, 115, 137, 140, 312). Sums through shared memory instead of butterflies: 361; asynchronous copies
 // of the next batches: 9 us more. The atomics cost 14 us, the butterflies 40.
 // ---------------------------------------------------------------------------------------
+// The other variant of a kernel, for the cases that other registers or a skip suit better; pixels_bwd_other() chooses.
+//   Four pixels per lane, up to 8 channels, splats of a few tiles: entries that no pixel blends - behind the last of
+//   those they reach - are left before the sums. 1920 x 1080, 4 / 8 channels, 5.4 tiles per Gaussian 442 / 563 -> 415 / 532 us; 12.7
+//   tiles 362 / 506 -> 371 / 512.
+//   Two pixels, 9 to 16 channels, many tiles: 96 registers. 1920 x 1080, 2.5 and 27.5 tiles per Gaussian 442, 875 -> 404, 834; 640 x 360,
+//   5.1 tiles 153 -> 158.
+//   Above 20 channels, few tiles: the chain of the longest list counts, so no spills, whole rows at once and the skip. 640 x 360, 32
+//   channels, scales of 1, 0.6, 0.3 and 0.1: 326, 346, 244, 205 -> 303, 332, 236, 199; 1920 x 1080: 1862 -> 1999.
+constexpr bool has_other_bwd(int cdim, int px) { return (px == 4 && cdim <= 8) || (px == 2 && cdim == 16) || cdim == 32; }
+constexpr bool pixels_bwd_skips(int cdim, int px, bool other) { return other && cdim != 16; }
+
 // registers per thread, by measurement (4 channels, eight pixels: 335 us at 128, 348 at 112, 361 at 144; 16 channels:
 // 386 at 168, 394 at 128; 8: 483 at 96, 520 at 128; 20, four pixels: 847 at 168, 980 at 200; 32: 1950 at 128, 2075 at 160)
-constexpr int pixels_bwd_regs(int cdim, int px) {
-    return cdim <= 4 ? (px == 8 ? 128 : px == 4 ? 80 : 72) : cdim <= 8 ? (px == 4 ? 96 : 88) : cdim <= 16 ? (px == 4 ? 168 : 104) : cdim <= 20 ? 168 : 128;
+constexpr int pixels_bwd_regs(int cdim, int px, bool other) {
+    return cdim <= 4 ? (px == 8 ? 128 : px == 4 ? 80 : 72) : cdim <= 8 ? (px == 4 ? 96 : 88) : cdim <= 16 ? (px == 4 ? 168 : other ? 96 : 104)
+                     : cdim <= 20 ? 168 : other ? 168 : 128;
 }
 
-template <int CDIM, int PX, bool kAbs>
-__global__ void __maxnreg__(pixels_bwd_regs(CDIM, PX))
+template <int CDIM, int PX, bool kAbs, bool kOther>
+__global__ void __maxnreg__(pixels_bwd_regs(CDIM, PX, kOther))
 rasterize_to_pixels_bwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
@@ -1571,6 +1583,7 @@ rasterize_to_pixels_bwd_kernel(
     const GradSlot slot_a = pixel_grad_slot<kAbs>(mine_a.value, CDIM, channels, v_colors,
                                                   v_conics, v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
 
+    constexpr bool kSkip = pixels_bwd_skips(CDIM, PX, kOther);
     int32_t waiting = thread_last;   // position of the next entry that is a pixel's of this lane last one; -1: none
     bool pending = true;             // a lane of the warp waits for one
     int32_t next_id = 0;
@@ -1594,7 +1607,7 @@ rasterize_to_pixels_bwd_kernel(
             sId[lane] = make_float2(__int_as_float(g), 1.f / e.B.w);
             // A colour that is not finite is blended by no pixel of the patch - it would have left its mark there. It may lie
             // behind the last entry of some pixels and out of reach of the others, and must not meet their weights of zero.
-            if (CDIM <= 16) stage_whole_row<CDIM, true>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, vec);
+            if (CDIM <= 16 || (CDIM == 32 && kOther)) stage_whole_row<CDIM, true>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, vec);
             else {   // (20 channels: all loads of a row at once take registers, 990 -> 1130 us)
                 float *row = reinterpret_cast<float *>(sCol) + lane * CDIM;
                 stage_row<true>(row, colors, (size_t)g, channels, vec);
@@ -1642,6 +1655,12 @@ rasterize_to_pixels_bwd_kernel(
                     alpha[q].x = pw.x <= 0.f ? fminf(kAlphaMax, alpha[q].x) : 0.f;
                     alpha[q].y = pw.y <= 0.f ? fminf(kAlphaMax, alpha[q].y) : 0.f;
                 }
+            }
+            if (kSkip) {
+                bool any = false;
+#pragma unroll
+                for (int q = 0; q < P2; ++q) any = any || alpha[q].x > 0.f || alpha[q].y > 0.f;
+                if (!__any_sync(0xffffffffu, any)) continue;
             }
 #pragma unroll
             for (int q = 0; q < P2; ++q) {
@@ -2210,24 +2229,57 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
 static bool fits_at_once(uint64_t blocks) { return blocks <= (uint64_t)kNumSMs * 8; }
 static bool warps_fit_at_once(uint64_t warps) { return fits_at_once(warps / 4); }
 
-// Pixels per lane of the camera kernels: more of them save instructions, fewer fill the machine. Measured over images
-// of 920 to 10800 tiles of 16 x 16 pixels, us with two / four / eight pixels. Forward, 4 channels: 920 tiles 49 / 70 / 119, 2040 57 /
-// 55 / 70, 2408 57 / 63 / 89, 3311 102 / 83 / 86, 4704 101 / 89 / 103, 7920 177 / 143 / 137, 10800 277 / 203 / 187; 8 channels: 2040
-// 68 / 76, 3510 127 / 114; 13 channels: 920 72 / 104, 2040 97 / 93, 3510 180 / 151. Backward, 4 channels: 920 106 / 154 / 255, 2040 138 /
-// 122 / 153, 3510 250 / 188 / 178, 8160 520 / 360 / 312; 8 and 13 channels: 920 115 / 165 and 137 / 188, 2040 166 / 152 and 226 / 200.
+// Pixels per lane of the camera kernels: more of them save instructions, fewer fill the machine and leave out more of a
+// tile that a small Gaussian does not reach. So the line depends on the number of tiles and on how many of them a Gaussian
+// covers - list entries per listed Gaussian, where the caller knows it (splatad_rasterize_set_spread_hint()), else the
+// number of tiles alone. Measured, us with two / four / eight pixels, scenes of the camera benchmark with scales shrunk (the kernels of four
+// and eight pixels in the one kernel there was before, 16 x 16 pixels with four warps: in brackets).
+// Forward, 4 channels: 8160 tiles, 27.5 per Gaussian 197 / 150 / 144 (214), 12.7: 205 / 162 / 158 (220), 7.5: 187 / 156 / 175 (195), 5.4: 187 / 195 / 268
+// (193), 3.8: 160 / 164 / 245 (161), 2.5: 109 / 116 / 180 (109), Gaussians all of one size, 3.5: 39 / 31 / 37 (41); 5700, 9.6: 148 / 119 / 125, 5.8: 136 / 148 / 195;
+// 3510, 13: 98 / 79 / 84 (105), 6.6: 87 / 96 / 129 (92), 4.3: 105 / 132 / 191 (109); 2040, 8.9: 62 / 66 / 80 (67); 920, 5.1: 62 / 84. 8 channels: 8160, 7.5: 234 / 225
+// (267), 5.4: 238 / 262 (262); 3510, 13: 112 / 104 (142), 6.6: 103 / 120 (122). 16 channels: 8160, 7.5: 343 / 312 (334), 5.4: 349 / 352 (340); 3510, 13: 162 / 146 (171), 6.6: 150 /
+// 157 (152).
+// Backward, 4 channels: 8160 tiles, 27.5: 493 / 347 / 305 (383), 12.7: 506 / 373 / 337 (404), 7.5: 473 / 362 / 376 (383), 5.4: 442 / 415 / 584 (422), 3.8: 365 / 385 / 569
+// (414), 2.5: 229 / 268 / 410 (297); 5700, 9.6: 375 / 276 / 264; 3510, 13: 240 / 180 / 175 (194), 6.6: 208 / 207 / 274 (209), 4.3: 247 / 283 / 418 (288); 2040, 8.9: 156 /
+// 143 / 167 (147), 4.8: 203 / 231 / 397 (233). 8 channels: 8160, 7.5: 582 / 490 (478), 5.4: 567 / 532 (510), 3.8: 469 / 496 (495); 3510, 6.6: 255 / 250 (241), 4.3: 269 / 328 (322).
+// 16 channels: 8160, 7.5: 800 / 735 (763), 5.4: 762 / 778 (735); 3510, 6.6: 362 / 330 (334), 4.3: 363 / 449 (335). 20 channels: 8160, 7.5: 907 / 890 (834), 5.4: 884 / 942 (799).
 // A tile whose rows leave lanes over takes fewer (8 x 8 tiles: 99 / 136 / 227; 24 x 24: 106 / 90 / 111).
 static uint32_t tiles_of_256(uint64_t blocks, uint32_t tile_size) {
     return (uint32_t)(blocks * tile_size * tile_size / 256u < 0xffffffffull ? blocks * tile_size * tile_size / 256u : 0xffffffffull);
 }
-static uint32_t pixels_per_lane(uint32_t tiles, uint32_t four_from, uint32_t eight_from, uint32_t tile_size) {
-    if (tiles >= eight_from && tile_threads<8>(tile_size) % 32u == 0u) return 8u;
-    return tiles >= four_from && tile_threads<4>(tile_size) >= 32u ? 4u : 2u;
+static bool covers(float spread, float line) { return !(spread > 0.f) || spread >= line; }   // 0: not known
+// Tiles of 16 x 16 pixels that a square over `spread` tiles covers.
+static float spread_of_16(float spread, uint32_t tile_size) {
+    if (!(spread > 0.f) || tile_size == 16u) return spread;
+    const float side = 1.f + (sqrtf(spread < 1.f ? 1.f : spread) - 1.f) * (float)tile_size / 16.f;
+    return side * side;
 }
-static uint32_t pixels_per_lane_fwd(uint64_t blocks, uint32_t tile_size, uint32_t channels) {
-    return pixels_per_lane(tiles_of_256(blocks, tile_size), channels <= 8 ? 2700u : 1500u, channels <= 4 ? 6000u : ~0u, tile_size);
+static uint32_t pixels_that_fit(bool four, bool eight, uint32_t tile_size) {
+    if (eight && tile_threads<8>(tile_size) % 32u == 0u) return 8u;
+    return (four || eight) && tile_threads<4>(tile_size) >= 32u ? 4u : 2u;
 }
-static uint32_t pixels_per_lane_bwd(uint64_t blocks, uint32_t tile_size, uint32_t channels) {
-    return pixels_per_lane(tiles_of_256(blocks, tile_size), 1500u, channels <= 4 ? 3000u : ~0u, tile_size);
+static uint32_t pixels_per_lane_fwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread) {
+    const uint32_t tiles = tiles_of_256(blocks, tile_size);
+    const bool many = channels <= 4 && tiles >= 6000u;
+    return pixels_that_fit(tiles >= (channels <= 8 ? 2700u : 1500u) && covers(spread, many ? 3.3f : 7.f), many && covers(spread, 10.f), tile_size);
+}
+static uint32_t pixels_per_lane_bwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread) {
+    const uint32_t tiles = tiles_of_256(blocks, tile_size);
+    const float line = channels <= 4 && tiles >= 6000u ? 4.f : channels <= 8 ? 5.f : channels <= 16 ? 6.f : 7.f;
+    return pixels_that_fit(tiles >= 1500u && covers(spread, line), channels <= 4 && tiles >= 3000u && covers(spread, 9.f), tile_size);
+}
+static bool pixels_bwd_other(uint64_t blocks, uint32_t tile_size, uint32_t channels, uint32_t px, float spread) {
+    const uint32_t tiles = tiles_of_256(blocks, tile_size);
+    if (channels > 20) return tiles < 1500u || (tiles < 3000u && !covers(spread, 7.f));
+    return px == 4 ? !covers(spread, 9.f) : tiles >= 3000u;
+}
+
+// One-shot hint of the calling thread's next camera compositing call.
+static thread_local float t_spread_hint = 0.f;
+static float take_spread_hint(uint32_t tile_size) {
+    const float spread = spread_of_16(t_spread_hint, tile_size);
+    t_spread_hint = 0.f;
+    return spread;
 }
 
 // Patches below which all warps of a CTA share one in the forward pass: the shared work costs more
@@ -2264,6 +2316,11 @@ static int set_smem(K kernel, size_t bytes, const char *what) {
 
 using namespace splatad;
 
+extern "C" int splatad_rasterize_set_spread_hint(float tiles_per_gaussian) {
+    t_spread_hint = tiles_per_gaussian;
+    return SPLATAD_OK;
+}
+
 extern "C" int splatad_rasterize_to_pixels_fwd(
     uint32_t C, int64_t n_isects, const float *means2d, const float *conics, const float *colors,
     uint32_t channels, const float *opacities, const float *pix_vels,
@@ -2284,6 +2341,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
     const int32_t *tile_offsets, const int32_t *flatten_ids, int32_t expected_last_channel, float *render_colors,
     float *render_alphas, int32_t *last_ids, float *expected_depths, void *stream) {
+    const float spread = take_spread_hint(tile_size);
     SPL_REQUIRE(channels >= 1 && channels <= SPLATAD_MAX_CHANNELS, SPLATAD_ERR_CHANNELS,
                 "rasterize_to_pixels_fwd: unsupported channel count %u (1..%d)", channels,
                 SPLATAD_MAX_CHANNELS);
@@ -2310,7 +2368,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     }
 #define CALL(D)                                                                                   \
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2)) else if (D <= 16 && px == 4) CALL_PX(D, (D <= 16 ? 4 : 2)) else CALL_PX(D, 2)
-    const uint32_t px = pixels_per_lane_fwd(blocks, tile_size, channels);
+    const uint32_t px = pixels_per_lane_fwd(blocks, tile_size, channels, spread);
     const bool vec = channels % 4u == 0u && (reinterpret_cast<uintptr_t>(colors) & 15u) == 0u;
     {
         SPL_PROF("rasterize_to_pixels_fwd_kernel", (cudaStream_t)stream);
@@ -2346,6 +2404,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     const int32_t *last_ids, const float *v_render_colors, const float *v_render_alphas,
     float *v_means2d_abs, float *v_means2d, float *v_conics, float *v_colors, float *v_opacities,
     float *v_pix_vels, void *stream) {
+    const float spread = take_spread_hint(tile_size);
     SPL_REQUIRE(channels >= 1 && channels <= SPLATAD_MAX_CHANNELS, SPLATAD_ERR_CHANNELS,
                 "rasterize_to_pixels_bwd: unsupported channel count %u (1..%d)", channels,
                 SPLATAD_MAX_CHANNELS);
@@ -2365,9 +2424,11 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
                 tile_size * tile_size, samples, channels);
 #define CALL_PX(D, P, A)                                                                          \
     {                                                                                             \
+        const auto kernel = has_other_bwd(D, P) && other ? rasterize_to_pixels_bwd_kernel<D, P, A, has_other_bwd(D, P)> \
+                                                         : rasterize_to_pixels_bwd_kernel<D, P, A, false>; \
         const uint32_t patches = div_up(tile_threads<P>(tile_size), 32);                          \
         SPL_REQUIRE((uint64_t)blocks * patches <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_bwd: too many tiles"); \
-        launch_chained(rasterize_to_pixels_bwd_kernel<D, P, A>, blocks * patches, 32, 0, (cudaStream_t)stream, \
+        launch_chained(kernel, blocks * patches, 32, 0, (cudaStream_t)stream,                     \
             C, n_isects, (const float2 *)means2d, conics, colors, channels, opacities,            \
             (const float2 *)pix_vels, rolling_shutter_time, backgrounds, image_width,             \
             image_height, tile_size, tile_width, tile_height, patches, tile_offsets, flatten_ids, \
@@ -2378,7 +2439,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2), A) else if (D <= 20 && px == 4) CALL_PX(D, (D <= 20 ? 4 : 2), A) else CALL_PX(D, 2, A)
 #define CALL(D)                                                                                   \
     if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)
-    const uint32_t px = pixels_per_lane_bwd(blocks, tile_size, channels);
+    const uint32_t px = pixels_per_lane_bwd(blocks, tile_size, channels, spread);
+    const bool other = pixels_bwd_other(blocks, tile_size, channels, px, spread);
     {
         SPL_PROF("rasterize_to_pixels_bwd_kernel", (cudaStream_t)stream);
         SPL_DISPATCH_CDIM(channels, CALL);

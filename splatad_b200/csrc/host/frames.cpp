@@ -42,6 +42,7 @@ using OptTensor = c10::optional<Tensor>;
     X(splatad_isect_plan_workspace_bytes) X(splatad_isect_fill_workspace_bytes) X(splatad_lidar_azimuth_tiles)           \
     X(splatad_isect_tiles_plan) X(splatad_isect_tiles_fill) X(splatad_isect_lidar_tiles_plan)                            \
     X(splatad_isect_lidar_tiles_fill) X(splatad_isect_set_early_count) X(splatad_isect_set_depth_range_hint)             \
+    X(splatad_isect_set_listed_count) X(splatad_rasterize_set_spread_hint)                                               \
     X(splatad_rasterize_expected_to_pixels_fwd) X(splatad_rasterize_expected_to_pixels_bwd)                              \
     X(splatad_lidar_frame_fwd) X(splatad_rasterize_to_points_fwd) X(splatad_rasterize_to_points_bwd) X(splatad_map_points_workspace_bytes)          \
     X(splatad_map_strided_points_to_lidar_tiles) X(splatad_points_mapping_offset_encode) X(splatad_populate_image_from_points)
@@ -166,7 +167,7 @@ Tensor workspace(const char *tag, size_t bytes, c10::cuda::CUDAStream stream) {
 }
 
 // Pinned words that one frame owns until its counts have been read, stored by its kernels: [4..7] {count,
-// sequence, status, depth range}, [8] the packed row count. (The plan's own copy of its counters at its end is
+// sequence, status, depth range}, [8] the packed row count, [9] the elements listed. (The plan's own copy of its counters at its end is
 // not asked for: it breaks the chain of launches, 8 us of a small frame's 120.)
 struct Slot {
     StreamKey key;
@@ -236,7 +237,9 @@ Tensor kept_opacities(const Tensor &opacities, const Tensor &comps, bool copied)
 
 // What came of the lists: the caller keeps the counts and decides whether the frame stands.
 struct Counts {
-    int64_t n_isects = 0, status = 0, depth_range = 0;
+    int64_t n_isects = 0, status = 0, depth_range = 0, listed = 0;
+    // list entries per listed element, 0: not known
+    float spread() const { return listed > 0 ? (float)n_isects / (float)listed : 0.f; }
 };
 
 Counts read_counts(const Slot &slot, int64_t sequence, c10::cuda::CUDAStream stream) {
@@ -245,6 +248,7 @@ Counts read_counts(const Slot &slot, int64_t sequence, c10::cuda::CUDAStream str
         c.n_isects = slot.word[4];
         c.status = slot.word[6];
         c.depth_range = slot.word[7];
+        c.listed = slot.word[9];
     } else {
         TORCH_CHECK(false, "the frame has ended without reporting its intersection count");
     }
@@ -275,10 +279,13 @@ struct PlanRequests {
                 lib.splatad_isect_set_depth_range_hint(wide[0], wide[1]);
             }
         }
+        slot.word[9] = 0;
         lib.splatad_isect_set_early_count(const_cast<int64_t *>(slot.word) + 4, sequence);
+        lib.splatad_isect_set_listed_count(const_cast<int64_t *>(slot.word) + 9);
     }
     ~PlanRequests() {
         lib.splatad_isect_set_early_count(nullptr, 0);
+        lib.splatad_isect_set_listed_count(nullptr);
         lib.splatad_isect_set_depth_range_hint(1, 0);
     }
 };
@@ -547,7 +554,7 @@ struct CameraFrame : torch::CustomClassHolder {
     std::vector<int64_t> color_sizes;
     int64_t K = 0, D = 0, sh_degree = -1;     // spherical harmonics (K coefficients) or D plain channels
     bool packed = false, per_camera = false, depth = false, expected = false, absgrad = false;
-    float eps2d = 0.f;
+    float eps2d = 0.f, spread = 0.f;          // spread: tiles that a listed Gaussian covers on the average, 0: not known
     Tensor camera_ids, gaussian_ids, radii, means2d, depths, conics, comps, pix_vels, tiles_per_gauss, campos;
     Tensor opacities, colors;                 // rows made for this frame (undefined: the parameters serve as they are)
     Tensor isect_ids, flatten_ids, offsets, render, alphas, last_ids;
@@ -557,6 +564,7 @@ struct CameraFrame : torch::CustomClassHolder {
         k->C = C; k->N = N; k->n = n; k->W = W; k->H = H; k->tile_size = tile_size; k->tile_w = tile_w; k->tile_h = tile_h;
         k->channels = channels; k->K = K; k->D = D; k->sh_degree = sh_degree; k->packed = packed; k->per_camera = per_camera;
         k->depth = depth; k->expected = expected; k->absgrad = absgrad; k->eps2d = eps2d; k->n_isects = n_isects;
+        k->spread = spread;
         k->color_sizes = color_sizes;
         return k;
     }
@@ -682,6 +690,7 @@ struct CameraCompositeNode : torch::autograd::Function<CameraCompositeNode> {
         zeros.add(v_pix_vels, pix_vels.sizes());
         if (f->absgrad) zeros.add(v_abs, means2d.sizes());
         zeros.make(options);
+        lib.splatad_rasterize_set_spread_hint(f->spread);
         check(lib.splatad_rasterize_expected_to_pixels_bwd(
             (uint32_t)f->C, f->n_isects, F(means2d), F(conics), F(colors), (uint32_t)f->channels, F(opacities), F(pix_vels), F(saved[5]),
             F(saved[6]), (uint32_t)f->W, (uint32_t)f->H, (uint32_t)f->tile_size, (uint32_t)f->tile_w, (uint32_t)f->tile_h, I(saved[9]),
@@ -702,7 +711,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
                         const OptTensor &lin, const OptTensor &ang, const OptTensor &rs, double near_plane, double far_plane,
                         double radius_clip, double eps2d, int64_t sh_degree, bool packed, int64_t tile_size, const OptTensor &backgrounds,
                         int64_t mode, bool expected, bool absgrad, bool antialiased, int64_t max_channels, int64_t row_capacity,
-                        int64_t capacity, uint64_t last_range) {
+                        int64_t capacity, uint64_t last_range, double last_spread) {
     if (!means.defined() || !means.is_cuda()) return py::none();
     const c10::DeviceIndex dev = means.get_device();
     for (const Tensor *t : {&means, &quats, &scales, &opacities, &colors, &viewmats, &Ks})
@@ -823,6 +832,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
         f->alphas = at::empty({C, H, W, 1}, options);
         f->last_ids = at::empty({C, H, W}, ints);
         if (expected && grad) f->expected_depths = at::empty({C, H, W}, options);
+        lib.splatad_rasterize_set_spread_hint((float)last_spread);
         check(lib.splatad_rasterize_expected_to_pixels_fwd(
             (uint32_t)C, -1, F(f->means2d), F(f->conics), c, (uint32_t)channels, o, F(f->pix_vels), F(rs_t), F(bg), (uint32_t)W, (uint32_t)H,
             (uint32_t)tile_size, (uint32_t)tile_w, (uint32_t)tile_h, I(f->offsets), I(f->flatten_ids), expected, M(f->render), M(f->alphas),
@@ -837,8 +847,9 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
         }
     }
     if (nnz <= 0 || nnz > rows_max || !usable(counts, capacity))
-        return py::make_tuple(nnz, counts.n_isects, counts.status, counts.depth_range, py::none());
+        return py::make_tuple(nnz, counts.n_isects, counts.status, counts.depth_range, counts.listed, py::none());
     f->n = nnz;
+    f->spread = counts.spread();
     if (packed && nnz < rows_max)
         for (Tensor *t : {&f->camera_ids, &f->gaussian_ids, &f->radii, &f->means2d, &f->depths, &f->conics, &f->comps, &f->pix_vels,
                           &f->tiles_per_gauss, &f->opacities, &f->colors})
@@ -857,7 +868,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
         f->render = out[0]; f->alphas = out[1];
     }
     const auto opt = [](const Tensor &t) { return t.defined() ? py::cast(t) : py::object(py::none()); };
-    return py::make_tuple(nnz, counts.n_isects, counts.status, counts.depth_range,
+    return py::make_tuple(nnz, counts.n_isects, counts.status, counts.depth_range, counts.listed,
                           py::make_tuple(f->render, f->alphas, opt(f->camera_ids), opt(f->gaussian_ids), f->radii, f->means2d, f->depths,
                                          f->conics, opacities_r, f->pix_vels, f->tiles_per_gauss, f->isect_ids, f->flatten_ids,
                                          alias(f->offsets, {C, tile_h, tile_w})));

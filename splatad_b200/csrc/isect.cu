@@ -712,15 +712,18 @@ __global__ void __launch_bounds__(kThreads)
 depth_bucket_scatter_kernel(const uint32_t *__restrict__ depth_bits, const int32_t *__restrict__ tiles_per_gauss,
                             uint32_t total, BucketLayout layout, const int64_t *__restrict__ counters,
                             volatile int64_t *early_host /* optional: the polling host's words */, int64_t early_seq,
+                            volatile int64_t *listed_host /* optional, with early_host: elements listed */,
                             const uint32_t *__restrict__ bstart, const uint32_t *__restrict__ boff,
                             uint32_t *__restrict__ bcursor, uint2 *__restrict__ pairs /* {bits, flatten index} */) {
     chain_enter();
     // All the host wants to know is there since the bucket scan. Telling it takes a fence over the host link, which
     // would be the end of that kernel's last block; here the other blocks' work covers it (20,000 Gaussians: 4 us).
-    if (early_host != nullptr && blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1)
+    if (early_host != nullptr && blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) {
+        if (listed_host != nullptr) *listed_host = counters[CNT_NVIS];
         tell_host(early_host, early_seq, counters[CNT_NISECT], counters[CNT_STATUS],
                   (int64_t)(((unsigned long long)(uint32_t)counters[CNT_DMAX] << 32) |
                             (unsigned long long)(uint32_t)counters[CNT_DMIN]));
+    }
     const DepthBuckets bucket = depth_buckets(counters, layout.per);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         if (tiles_per_gauss[i] <= 0) continue;
@@ -1843,6 +1846,7 @@ static uint2 *plan_pairs(const PlanWs &p, const IsectGeom &g, int sort) {
 // rectangle count kernel writes the intersection count for the host, and the number it tags it with.
 static thread_local int64_t *t_early_host = nullptr;
 static thread_local int64_t t_early_seq = 0;
+static thread_local int64_t *t_listed_host = nullptr;
 static thread_local bool t_range_given = false;
 static thread_local uint32_t t_range_lo = 0, t_range_hi = 0;
 
@@ -1882,14 +1886,17 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
     // behind it, which also knows whether the bucket sort applies - and need not wait for the depth
     // order. Both list constructions report it: a host left to wait for words that never came gave up
     // after 20 ms, which was 87 % of a three-camera training step (22.6 -> 3.2 ms).
-    int64_t *early = nullptr;
-    if (t_early_host != nullptr) {
+    const auto on_device = [](int64_t *host) {
         void *dptr = nullptr;
-        if (cudaHostGetDevicePointer(&dptr, t_early_host, 0) == cudaSuccess) early = (int64_t *)dptr;
-        else (void)cudaGetLastError();   // not mapped for this device: the host falls back to the event
-    }
+        if (host != nullptr && cudaHostGetDevicePointer(&dptr, host, 0) != cudaSuccess) {
+            (void)cudaGetLastError();   // not mapped for this device: the host falls back to the event
+            dptr = nullptr;
+        }
+        return (int64_t *)dptr;
+    };
+    int64_t *early = on_device(t_early_host), *listed = on_device(t_listed_host);
     const int64_t seq = t_early_seq;
-    t_early_host = nullptr;
+    t_early_host = t_listed_host = nullptr;
     {
         SPL_PROF("isect_count_kernel", st);
         uint2 *rect = blocks ? p.rect : nullptr;
@@ -1933,7 +1940,7 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
             SPL_PROF("depth_bucket_scatter_kernel", st);
             launch_chained(depth_bucket_scatter_kernel, bgrid, kThreads, 0, st, g.depth_bits,
                            (const int32_t *)tiles_per_gauss, g.total, layout, (const int64_t *)p.counters,
-                           (volatile int64_t *)early, seq,
+                           (volatile int64_t *)early, seq, (volatile int64_t *)listed,
                            (const uint32_t *)p.bstart, (const uint32_t *)p.boff, p.bcount, pairs);
         }
         {
@@ -2673,6 +2680,11 @@ extern "C" int splatad_isect_lidar_tiles_fill(
 extern "C" int splatad_isect_set_early_count(int64_t *host_pair, int64_t sequence) {
     t_early_host = host_pair;
     t_early_seq = sequence;
+    return SPLATAD_OK;
+}
+
+extern "C" int splatad_isect_set_listed_count(int64_t *host_word) {
+    t_listed_host = host_word;
     return SPLATAD_OK;
 }
 

@@ -65,11 +65,13 @@ def packed_room(count: int, most: int) -> int:
     return min((count + count // 8 + 4096 + 0xFFFF) & ~0xFFFF, most)
 
 
-def note_counts(key, n_isects: int, status: int, depth_range: int, ranged: bool) -> None:
+def note_counts(key, n_isects: int, status: int, depth_range: int, ranged: bool, listed: int = 0) -> None:
     """Keeps what a natively enqueued frame reported about its lists for the next frame of its shape."""
     if status & 2 or n_isects > 0x7FFFFFFF:
         raise RuntimeError(f"isect: {n_isects} intersections do not fit int32 flatten ids / offsets")
     _isect_count_hint[key] = n_isects
+    if listed > 0:
+        _spread_hint[key] = n_isects / listed
     if status & 4:
         if ranged:
             # an end bucket overflowed under the depth range carried over from the last frame: the frame
@@ -1017,9 +1019,12 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
             plan()
             torch.cuda.current_stream(dev).synchronize()
             n_isects = read_count()
+        listed = int(host[1]) if sort else 0
         isect_ids, flatten_ids, offsets = fill(n_isects)
         if offsets is not None:
             isect_ids._splatad_tile_offsets = (C, offsets[:n_tiles_total])
+        if listed > 0:
+            _spread_hint[key] = flatten_ids._splatad_spread = n_isects / listed
         return tiles_per_gauss, isect_ids, flatten_ids
 
     if not deferred:
@@ -1041,6 +1046,7 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
     counted = torch.cuda.Event()
     counted.record(torch.cuda.current_stream(dev))
     isect_buf, flat_buf, offsets = fill(capacity)
+    flat_buf._splatad_spread = _spread_hint.get(key, 0.0)
     return DeferredIsect(tiles_per_gauss, isect_buf, flat_buf, offsets, C, n_tiles_total, capacity,
                          counted, lambda: read_count(slot, sequence, counted), exact)
 
@@ -1049,6 +1055,7 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
 # that stream (see _packed_nnz_hint for why the stream is part of the key)
 _isect_count_hint: dict = {}
 _depth_range_hint: dict = {}    # per frame shape and stream: (lo bits, hi bits) of the last frame's listed depths
+_spread_hint: dict = {}         # same keys -> list entries per listed Gaussian of the last frame
 _depth_sort_mode: dict = {}   # same keys -> 2 once a frame of the shape needed the radix depth sort
 
 
@@ -1411,8 +1418,10 @@ def rasterize_to_pixels(
     means2d_c = means2d.contiguous()
     args = (conics.contiguous(), opacities.contiguous(), pix_vels.contiguous(),
             rolling_shutter_time.contiguous())
+    # how many tiles a listed Gaussian covers, where the lists' maker has left it; chooses the split of the work
+    spread = getattr(flatten_ids, "_splatad_spread", 0.0)
     tail = (image_width, image_height, tile_size, isect_offsets.contiguous(), flatten_ids.contiguous(),
-            absgrad, total_follows)
+            absgrad, total_follows, spread)
     if channels <= _lib.MAX_CHANNELS:
         return _RasterizeToPixels.apply(means2d_c, args[0], colors.contiguous(), args[1], args[2],
                                         args[3], backgrounds, *tail)
@@ -1431,7 +1440,7 @@ def rasterize_to_pixels(
 class _RasterizeToPixels(torch.autograd.Function):
     @staticmethod
     def forward(ctx, means2d, conics, colors, opacities, pix_vels, rolling_shutter_time, backgrounds,
-                width, height, tile_size, isect_offsets, flatten_ids, absgrad, total_follows=False):
+                width, height, tile_size, isect_offsets, flatten_ids, absgrad, total_follows=False, spread=0.0):
         dev = means2d.device
         assert means2d.dtype == torch.float32, means2d.dtype
         C, tile_h, tile_w = isect_offsets.shape
@@ -1444,7 +1453,8 @@ class _RasterizeToPixels(torch.autograd.Function):
         last_ids = torch.empty((C, height, width), dtype=torch.int32, device=dev)
         n_isects = _n_isects_arg(isect_offsets, flatten_ids, total_follows)
         _debug_check_lists("rasterize_to_pixels", flatten_ids, means2d.numel() // 2, isect_offsets, total_follows)
-        ctx.n_isects_arg = n_isects
+        ctx.n_isects_arg, ctx.spread = n_isects, spread
+        _lib.load().splatad_rasterize_set_spread_hint(spread)
         _call(
             "splatad_rasterize_to_pixels_fwd", C, n_isects, _lib.ptr(means2d), _lib.ptr(conics_f),
             _lib.ptr(colors_f), channels, _lib.ptr(opac_f), _lib.ptr(vels_f), _lib.ptr(rs), _lib.ptr(bg),
@@ -1467,6 +1477,7 @@ class _RasterizeToPixels(torch.autograd.Function):
         v_render_alphas = _f(v_render_alphas)
         v_means2d, v_conics, v_colors, v_opacities, v_pix_vels, v_abs = _zeros_like_many(
             means2d, conics, colors, opacities, pix_vels, means2d if ctx.absgrad else None)
+        _lib.load().splatad_rasterize_set_spread_hint(ctx.spread)
         _call(
             "splatad_rasterize_to_pixels_bwd", C, ctx.n_isects_arg, _lib.ptr(means2d),
             _lib.ptr(conics), _lib.ptr(colors), channels, _lib.ptr(opacities), _lib.ptr(pix_vels),
@@ -1482,7 +1493,7 @@ class _RasterizeToPixels(torch.autograd.Function):
         if ctx.needs_input_grad[6]:
             v_backgrounds = (v_render_colors * (1.0 - render_alphas).float()).sum(dim=(1, 2))
         return (v_means2d, v_conics, v_colors, v_opacities, v_pix_vels, None, v_backgrounds, None,
-                None, None, None, None, None, None)
+                None, None, None, None, None, None, None)
 
 
 def rasterize_to_points(

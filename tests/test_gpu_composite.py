@@ -422,7 +422,6 @@ def test_pixels_of_many_tiles(C, ts, channels, absgrad):
     leaves = {k: t(c[k]).requires_grad_(True) for k in keys}
     out_c, out_a = ops.rasterize_to_pixels(*(leaves[k] for k in keys), W, H, ts, t(c["offsets"], torch.int32),
                                            t(c["flatten_ids"], torch.int32), t(c["rs"]), absgrad=absgrad)
-    f32["ambiguous"] = ~same
     for got, want in ((out_c, f32["render_colors"]), (out_a, f32["render_alphas"])):
         assert_close(f"pixels tile {ts} ch={channels}", n(got), want, 1e-4, 1e-5, mask=same[..., None])
     torch.autograd.backward([out_c, out_a], [t(v_c) * mask, t(v_a) * mask])
@@ -434,6 +433,84 @@ def test_pixels_of_many_tiles(C, ts, channels, absgrad):
     if absgrad:
         _grad_check(f"tile {ts} ch={channels} absgrad", leaves["means2d"].absgrad[:, plain],
                     ref["v_means2d_abs"].reshape(C, 120, 2)[:, plain])
+
+
+@pytest.mark.parametrize("C,ts,channels,absgrad", [(12, 16, 30, True), (24, 16, 3, False), (24, 16, 7, True), (24, 16, 13, False), (24, 16, 20, True),
+                                                   (43, 16, 4, False), (84, 16, 3, True), (60, 16, 13, True), (60, 20, 8, False), (300, 8, 4, False)])
+def test_pixels_by_how_many_tiles_a_gaussian_covers(C, ts, channels, absgrad):
+    """The hint that chooses how many pixels a lane draws changes no bit of an image, a background and a divided depth among
+    them; every choice matches the oracle, forward and backward."""
+    from oracle import composite
+    from splatad_b200 import ops
+    W, H = (127, 133) if C % 2 else (132, 131)
+    c = _camera_case(C, 60, W, H, ts, channels, 100 * ts + channels, sigma_px=(1.0, 9.0))
+    g = torch.Generator().manual_seed(7)
+    bg = torch.rand(C, channels, generator=g)
+    v_c, v_a = torch.randn(C, H, W, channels, generator=g), torch.randn(C, H, W, 1, generator=g)
+    keys = ("means2d", "conics", "colors", "opacities", "pix_vels")
+    args = [n(c[k]) for k in keys] + [n(c["rs"]), n(bg), W, H, ts, c["offsets"], c["flatten_ids"]]
+    ref_f = composite.rasterize_to_pixels_fwd(*args, dtype=np.float64)
+    f32 = composite.rasterize_to_pixels_fwd(*args, amb_tol=1e-4)
+    same = (f32["last_ids"] == ref_f["last_ids"]) & ~f32["ambiguous"]
+    assert same.mean() > 0.9
+    mask, mk = t(same[..., None].astype(np.float32)), same[..., None].astype(np.float64)
+    ref = composite.rasterize_to_pixels_bwd(*args, ref_f["render_alphas"], ref_f["last_ids"], n(v_c) * mk, n(v_a) * mk,
+                                            absgrad=absgrad)
+    offsets, ids = t(c["offsets"], torch.int32), t(c["flatten_ids"], torch.int32)
+    first = None
+    for spread in (0.0, 2.0, 4.5, 6.5, 8.0, 20.0):
+        ids._splatad_spread = spread
+        leaves = {k: t(c[k]).requires_grad_(True) for k in keys}
+        out_c, out_a = ops.rasterize_to_pixels(*(leaves[k] for k in keys), W, H, ts, offsets, ids, t(c["rs"]), backgrounds=t(bg),
+                                               absgrad=absgrad)
+        if first is None:
+            first = out_c, out_a
+            for got, want in ((out_c, f32["render_colors"]), (out_a, f32["render_alphas"])):
+                assert_close(f"pixels tile {ts} ch={channels}", n(got), want, 1e-4, 1e-5, mask=same[..., None])
+        assert torch.equal(out_c, first[0]) and torch.equal(out_a, first[1])
+        torch.autograd.backward([out_c, out_a], [t(v_c) * mask, t(v_a) * mask])
+        for k in keys:
+            _grad_check(f"tile {ts} ch={channels} spread {spread} v_{k}", leaves[k].grad, ref["v_" + k].reshape(leaves[k].shape))
+        if absgrad:
+            _grad_check(f"tile {ts} ch={channels} spread {spread} absgrad", leaves["means2d"].absgrad,
+                        ref["v_means2d_abs"].reshape(C, 60, 2))
+
+
+@pytest.mark.parametrize("C,channels", [(24, 3), (43, 4), (84, 2), (24, 13), (12, 30)])
+def test_divided_depth_of_many_tiles(C, channels):
+    """The last channel divided by the alpha inside the kernels, forward and backward, against the same division behind them,
+    for every choice of pixels per lane."""
+    from splatad_b200 import _lib, ops
+    W, H, ts = 132, 131, 16
+    c = _camera_case(C, 60, W, H, ts, channels, 9 * channels, sigma_px=(1.0, 9.0))
+    keys = ("means2d", "conics", "colors", "opacities", "pix_vels")
+    dev = {k: t(c[k]) for k in keys}
+    bg, rs = torch.zeros(C, channels, device=DEV), t(c["rs"])
+    bg[:, :-1] = 0.3
+    offsets, ids = t(c["offsets"], torch.int32), t(c["flatten_ids"], torch.int32)
+    g = torch.Generator(device=DEV).manual_seed(8)
+    v_c, v_a = torch.randn(C, H, W, channels, generator=g, device=DEV), torch.randn(C, H, W, 1, generator=g, device=DEV)
+    leaves = {k: v.clone().requires_grad_(True) for k, v in dev.items()}
+    out_c, out_a = ops.rasterize_to_pixels(*(leaves[k] for k in keys), W, H, ts, offsets, ids, rs, backgrounds=bg)
+    want = torch.cat([out_c[..., :-1], out_c[..., -1:] / out_a.clamp(min=1e-10)], -1)
+    torch.autograd.backward([want, out_a], [v_c, v_a])
+    lib, p = _lib.load(), _lib.ptr
+    th, tw = c["offsets"].shape[1:]
+    for spread in (0.0, 2.0, 6.5, 20.0):
+        image, alphas = torch.empty(C, H, W, channels, device=DEV), torch.empty(C, H, W, 1, device=DEV)
+        last, depths = torch.empty(C, H, W, dtype=torch.int32, device=DEV), torch.empty(C, H, W, device=DEV)
+        head = (C, ids.numel(), p(dev["means2d"]), p(dev["conics"]), p(dev["colors"]), channels, p(dev["opacities"]), p(dev["pix_vels"]),
+                p(rs), p(bg), W, H, ts, tw, th, p(offsets), p(ids))
+        lib.splatad_rasterize_set_spread_hint(spread)
+        _lib.call("splatad_rasterize_expected_to_pixels_fwd", *head, 1, p(image), p(alphas), p(last), p(depths), _lib.stream_ptr(ids.device))
+        assert_close(f"depth ch={channels} spread {spread}", n(image), n(want), 1e-6, 1e-7)
+        assert torch.equal(alphas, out_a) and torch.equal(depths, image[..., -1])
+        v = [torch.zeros_like(dev[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")]
+        lib.splatad_rasterize_set_spread_hint(spread)
+        _lib.call("splatad_rasterize_expected_to_pixels_bwd", *head, p(depths), p(alphas), p(last), p(v_c), p(v_a), None, *(p(x) for x in v),
+                  _lib.stream_ptr(ids.device))
+        for k, got in zip(keys, v):
+            _grad_check(f"depth ch={channels} spread {spread} v_{k}", got, n(leaves[k].grad))
 
 
 @pytest.mark.parametrize("tw,th,H,W,channels,asum,absgrad", [(32, 8, 20, 130, 3, True, True), (8, 4, 9, 100, 17, False, False),

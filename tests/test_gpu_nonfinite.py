@@ -11,19 +11,23 @@ pytestmark = pytest.mark.gpu
 INF, NAN = float("inf"), float("nan")
 
 
-def _camera(channels, packed, mode="RGB"):
+def _camera(channels, packed, cameras=1, mode="RGB"):
     import splatad_b200
     from splatad_b200 import scenes
     s = {k: (v.to(DEV) if isinstance(v, torch.Tensor) else v) for k, v in scenes.config1(N=2_003, packed=packed).items()}
     g = torch.Generator(device=DEV).manual_seed(channels)
-    s.update(sh_degree=None, render_mode=mode, width=321, height=203, scales=s["scales"] * 3.0,
+    s.update(sh_degree=None, render_mode=mode, width=321, height=203, scales=s["scales"] * (3.0 if cameras == 1 else 4.5),
              colors=torch.rand(2_003, channels, generator=g, device=DEV))
     s["Ks"] = torch.tensor([[[200.0, 0.0, 160.5], [0.0, 200.0, 101.5], [0.0, 0.0, 1.0]]], device=DEV)
+    for k in ("viewmats", "Ks", "linear_velocity", "angular_velocity", "rolling_shutter_time"):
+        s[k] = s[k].repeat(cameras, *[1] * (s[k].dim() - 1))
 
     def run(colors, weights=None, **kw):
         p = {k: s[k].clone().requires_grad_(True) for k in ("means", "quats", "scales", "opacities")}
         p["colors"] = colors.clone().requires_grad_(True)
-        image, alpha, _ = splatad_b200.rasterization(**{**s, **p, **kw})
+        image, alpha, meta = splatad_b200.rasterization(**{**s, **p, **kw})
+        # Gaussians of many tiles: their number, 273 a camera, decides how many pixels a lane draws
+        assert cameras == 1 or meta["flatten_ids"].numel() > 10 * int((meta["tiles_per_gauss"] > 0).sum())
         torch.autograd.backward([image, alpha], [torch.ones_like(image) if weights is None else weights, torch.ones_like(alpha)])
         return image.detach(), {k: v.grad for k, v in p.items()}
 
@@ -52,11 +56,12 @@ def _lidar(features, columns):
 
 
 _CASES = [("camera", 3, False), ("camera", 3, True), ("camera", 13, False), ("camera", 30, True),
+          ("camera", 7, True, 6), ("camera", 13, False, 6), ("camera", 20, False, 6), ("camera", 3, False, 12), ("camera", 3, True, 24),
           ("lidar", 4, 512), ("lidar", 16, 512), ("lidar", 4, 1800), ("lidar", 16, 1800), ("lidar", 30, 1800)]
 
 
-def _setup(kind, a, b):
-    return _camera(a, b) if kind == "camera" else _lidar(a, b)
+def _setup(kind, *args):
+    return _camera(*args) if kind == "camera" else _lidar(*args)
 
 
 def _per_row(t):
@@ -67,10 +72,11 @@ def _close(got, want, tol):
     assert float((got - want).norm()) <= tol * max(float(want.norm()), 1e-30)
 
 
-@pytest.mark.parametrize("kind,a,b", _CASES)
+@pytest.mark.parametrize("case", _CASES, ids=str)
 @pytest.mark.parametrize("value", [INF, NAN])
-def test_a_colour_that_is_not_finite_reaches_its_own_samples_only(kind, a, b, value):
-    run, colors = _setup(kind, a, b)
+def test_a_colour_that_is_not_finite_reaches_its_own_samples_only(case, value):
+    run, colors = _setup(*case)
+    a = case[1]
     rows = colors.view(-1, a)
     clean, grads = run(colors)
     seen = (grads["colors"].reshape(-1, a).abs().sum(-1) > 0).nonzero()[:, 0]
@@ -90,10 +96,10 @@ def test_a_colour_that_is_not_finite_reaches_its_own_samples_only(kind, a, b, va
     _close(image[~reached], clean[~reached], 1e-6)
 
 
-@pytest.mark.parametrize("kind,a,b", _CASES)
+@pytest.mark.parametrize("case", _CASES, ids=str)
 @pytest.mark.parametrize("value", [INF, NAN])
-def test_a_cotangent_that_is_not_finite_reaches_its_own_gaussians_only(kind, a, b, value):
-    run, colors = _setup(kind, a, b)
+def test_a_cotangent_that_is_not_finite_reaches_its_own_gaussians_only(case, value):
+    run, colors = _setup(*case)
     image, _ = run(colors)
     at = (0, image.shape[1] // 2, image.shape[2] // 2)
     alone = torch.zeros_like(image)
@@ -153,9 +159,10 @@ def test_a_nan_in_the_geometry_is_blended_with_the_capped_alpha(what, channels):
         assert np.linalg.norm(got - ref_k) <= 2e-3 * max(np.linalg.norm(ref_k), 1e-20), k
 
 
-@pytest.mark.parametrize("C,channels,mode", [(1600, 3, "x"), (1600, 7, "x"), (1600, 18, "x"), (3200, 4, "y"), (6400, 3, "y")])
+@pytest.mark.parametrize("C,channels,mode,spread", [(1600, 3, "x", 0), (1600, 3, "x", 8), (1600, 7, "x", 0), (1600, 13, "x", 0), (1600, 18, "x", 0),
+                                                    (3200, 4, "y", 0), (6400, 3, "y", 0), (6400, 3, "x", 5), (1000, 30, "x", 0)])
 @pytest.mark.parametrize("value", [INF, NAN])
-def test_a_colour_that_is_not_finite_and_hidden_reaches_nothing(C, channels, mode, value):
+def test_a_colour_that_is_not_finite_and_hidden_reaches_nothing(C, channels, mode, spread, value):
     """One half of every tile stops early; a Gaussian behind that has a colour that is not finite and does not reach the other half,
     which blends one further behind. Nobody blends it: image and gradients are those of a finite colour and its own
     gradients are zero, also where the backward pass works on both halves at once and the forward pass on each by itself."""
@@ -176,6 +183,7 @@ def test_a_colour_that_is_not_finite_and_hidden_reaches_nothing(C, channels, mod
     fixed = dict(means2d=means, conics=conics, opacities=opacities, pix_vels=torch.zeros(n, 2))
     offsets = t(torch.arange(C)[:, None, None] * n, torch.int32)
     ids = t(torch.arange(C * n), torch.int32)
+    ids._splatad_spread = float(spread)   # as if the Gaussians covered as many tiles
     weights = [t(torch.randn(1, 16, 16, k, generator=g)).expand(C, -1, -1, -1).contiguous() for k in (channels, 1)]
 
     def run(bad_colour):
