@@ -846,7 +846,8 @@ __device__ __forceinline__ float angle_range(float mean, float vel, float centre
 // alphas need looking at one by one (as kCarefulEntry for the cameras).
 constexpr uint32_t kCarefulShift = 16;
 
-template <bool kOdd = true>   // kOdd: a box without a centre sees every entry
+// kMark: with the upper bits; kOdd: a box without a centre sees every entry
+template <bool kMark, bool kOdd>
 __device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const PointBox *s_box, uint32_t n_boxes) {
     const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
     if (!kOdd && test.never) return 0u;
@@ -862,7 +863,7 @@ __device__ __forceinline__ uint32_t boxes_that_see(const PointEntry &e, const Po
         const float y = angle_range(e.A.y, e.A.w, b.el, b.el_half, b.roll_lo, b.roll_hi, y_lo, y_hi);
         if (!(kOdd && b.az != b.az) && test.misses(x_lo, x_hi, y_lo, y_hi)) continue;
         seen |= 1u << w;
-        if (!(plain && x < 179.9f && y < 179.9f)) seen |= 1u << (w + kCarefulShift);
+        if (kMark && !(plain && x < 179.9f && y < 179.9f)) seen |= 1u << (w + kCarefulShift);
     }
     return seen;
 }
@@ -1013,7 +1014,7 @@ __global__ void __maxnreg__(points_fwd_regs(CDIM)) rasterize_to_points_fwd_kerne
         // compact the survivors to the front of the staging arrays, list order kept
 #pragma unroll
         for (uint32_t q = 0; q < kStage; ++q) {
-            seen[q] = batch_start + (int32_t)(q * bs + tr) < range.end ? boxes_that_see(e[q], s_box, n_warps) : 0u;
+            seen[q] = batch_start + (int32_t)(q * bs + tr) < range.end ? boxes_that_see<false, true>(e[q], s_box, n_warps) : 0u;
             kept[q] = __ballot_sync(0xffffffffu, seen[q] != 0u);
             if (lane == 0) s_warp_kept[q * n_warps + warp] = __popc(kept[q]);
         }
@@ -1208,7 +1209,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_co
     uint32_t buffer = 0;
     for (uint32_t b = 0; b < num_batches && !finished; ++b) {
         const int32_t idx = range.start + (int32_t)(kThreadsC * b + tr);
-        const uint32_t seen = idx < range.end ? boxes_that_see(e, &box, 1u) : 0u;
+        const uint32_t seen = idx < range.end ? boxes_that_see<true, true>(e, &box, 1u) : 0u;
         const uint32_t kept = __ballot_sync(0xffffffffu, seen != 0u);
         if (lane == 0) s_warp_kept[b & 1u][warp] = __popc(kept);
         __syncthreads();   // the batch before has been read
@@ -2016,7 +2017,7 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         // survivors to the front, still back to front in list order
 #pragma unroll
         for (uint32_t q = 0; q < kStage; ++q) {
-            seen[q] = batch_end - (int32_t)(q * bs + tr) >= range.start ? boxes_that_see<false>(e[q], &s_box, 1u) : 0u;
+            seen[q] = batch_end - (int32_t)(q * bs + tr) >= range.start ? boxes_that_see<true, false>(e[q], &s_box, 1u) : 0u;
             kept[q] = __ballot_sync(0xffffffffu, seen[q] != 0u);
             if (lane == 0) s_warp_kept[q * n_warps + warp] = __popc(kept[q]);
         }
