@@ -2,12 +2,12 @@
 // pixels (rasterize_to_pixels) and to lidar points (rasterize_to_points), forward and
 // backward. FP32 on the CUDA cores; there is no dense contraction in this path.
 //
-// A CTA walks a tile's list - or, for lidars, its part of a tile's points - in batches staged into shared
-// memory, and stops as soon as every sample is saturated. A warp covers a compact patch of samples, and an
-// entry is staged only if it can reach alpha >= 1/255 somewhere in one of the CTA's patches (an exact,
+// A camera warp draws a patch of a tile by itself; a lidar CTA works on one patch with all its warps, or on one for each of
+// them. Either walks the tile's list in batches staged into shared memory, and stops as soon as every sample is
+// saturated. An entry is staged only if it can reach alpha >= 1/255 somewhere in one of the patches (an exact,
 // conservative bound of the quadratic form over the patch's box) and looked at only by the warps it
 // can reach: the bounding rectangles behind the tile lists are loose. The backward pass starts at the
-// last list position any of the CTA's samples consumed instead of the end of the list.
+// last list position any of the patch's samples consumed instead of the end of the list.
 //
 // Semantics follow the reference kernels
 //   pixels fwd  gsplat/cuda/csrc/rasterization.cu:1360-1518     bwd 2833-3089
@@ -67,10 +67,10 @@ __device__ __forceinline__ void axpy_staged_full(float (&acc)[CDIM], const float
 }
 
 // ---------------------------------------------------------------------------------------
-// Camera tiles. A thread draws PX pixels next to each other in a row, so that everything that depends on
-// the Gaussian and the row alone is worked out once per thread, and the per-pixel arithmetic runs on
+// Camera tiles. A lane draws PX pixels next to each other in a row, so that everything that depends on
+// the Gaussian and the row alone is worked out once per lane, and the per-pixel arithmetic runs on
 // pairs of pixels (packed FP32: two results per issued instruction). A warp covers a compact patch of
-// the tile - 8 x 8 pixels of a 16 x 16 tile with PX = 2, 16 x 8 with PX = 4.
+// the tile - 8 x 8 pixels of a 16 x 16 tile with PX = 2, 16 x 8 with PX = 4, all of it with PX = 8.
 // ---------------------------------------------------------------------------------------
 constexpr float kExpectedMin = 1e-10f;   // alphas below it do not divide (gsplat/rendering.py:423-430)
 constexpr float kLog2E = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
@@ -190,8 +190,9 @@ __device__ __forceinline__ float2 pair_power(float a, float2 dx, float bdy, floa
 // negative; the kernels' comparisons drop it, and theirs is also a conic so flat that it reaches the column a pixel
 // moves to when it stops (see kPixelGone): a warp that meets such an entry works all of its pixels out again.
 // Both out of line and from nothing but the kernels' own arguments, so that the kernels hold nothing for
-// them. (Looking at the staged colours instead costs the forward kernel of the camera benchmark 220 ->
-// 237 us and the backward one 396 -> 440; two loop bodies, one of them careful, 6 to 9 % of a training step.)
+// them. What no pixel of a backward patch blends must not reach it either: there a value that is not finite becomes zero when
+// its row is staged (13 channels 673 -> 676 us, 32 channels 1862 -> 1869; a vote for every entry costs 1 to 4 %, careful entries
+// that leave the loop 3 %).
 // ---------------------------------------------------------------------------------------
 constexpr int32_t kOddPixel = INT32_MIN;   // in a last id: the pixel blended something that is not finite
 
@@ -517,12 +518,12 @@ __device__ __forceinline__ void store_channels(float *dst, const float (&v)[PX][
 //
 // What bounds it is instruction issue and, as more pixels share a lane, the FP32 pipe. What an entry costs whatever
 // the number of pixels - loads, bits, the row's terms, the stop test - was a third of the work at two pixels, and
-// where Gaussians are larger than tiles (61 of 64 pixels blend a looked-at entry in the benchmark scenes) there is nothing
+// where Gaussians are larger than tiles (62 of 64 pixels of an 8 x 8 patch blend an entry that is looked at in the benchmark scenes) there is nothing
 // to gain from small patches. So: eight pixels; alphas tested against 1/255 only, unless the entry was marked
 // (patch_sees()); no instruction spent on a sign; the transmittance updated in place by one multiply-add, which rounds once.
 // A pixel that has stopped moves its column out to where every alpha vanishes; a warp leaves when all of its have.
 // 1920 x 1080, 4 channels: 201 M -> 104 M warp instructions, 222 -> 147 us (two pixels 208, four 156); 16 channels, 1237 x 719:
-// 180 -> 152 (1920 x 1080: 8, 13, 20 and 32 channels 313, 376, 448, 683 -> 218, 308, 426, 570). Staging every value twice for the packed operands: 12 us slower; asynchronous copies of the next batches: 9.
+// 180 -> 152 (1920 x 1080: 8, 13, 20 and 32 channels 303, 360, 432, 662 -> 214, 297, 377, 506; 640 x 360, two pixels: 4, 13, 20 and 32 channels 64, 84, 87, 105 -> 62, 88, 91, 101). Staging every value twice for the packed operands: 12 us slower; asynchronous copies of the next batches: 9.
 // ---------------------------------------------------------------------------------------
 constexpr float kPixelGone = 1e18f;   // a column no Gaussian reaches: sigma overflows, alpha is 0 (or NaN, never drawn)
 
@@ -1308,7 +1309,8 @@ __global__ void __launch_bounds__(kCoopWarps * 32, 2) rasterize_to_points_fwd_co
                 before = next_T;
             }
 #pragma unroll
-            for (uint32_t k = 0; k < kCoopShare; ++k)                   if (vis[k] > 0.f) axpy_staged_full<CDIM>(pix_out, sFeat + (t0 + k) * CDIM, vis[k]);   // a branch: elsewhere it would be 0 * inf
+            for (uint32_t k = 0; k < kCoopShare; ++k)
+                if (vis[k] > 0.f) axpy_staged_full<CDIM>(pix_out, sFeat + (t0 + k) * CDIM, vis[k]);   // a branch: elsewhere it would be 0 * inf
         }
     }
     cur_idx &= INT32_MAX;
@@ -1458,9 +1460,9 @@ __device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t
 // colour. A pixel lies far out until its last entry comes, which takes a look at few entries of a list instead of a
 // comparison per pixel and entry. The pairs are worked through in one straight line: a branch for the entries that need
 // care between them costs 7 us.
-// 1920 x 1080, 4 channels: 323 M -> 200 M warp instructions, 398 -> 312 us (four pixels 367); 16 channels and absolute
-// gradients, 1237 x 719: 445 -> 374 (1920 x 1080 without: 4, 8, 13, 20 and 32 channels 401, 496, 861, 948, 2000 -> 312, 483, 703, 847, 1940;
-// 640 x 360, two pixels: 159, 174, 136, 148, 282 -> 106, 115, 137, 140, 312). Sums through shared memory instead of butterflies: 361; asynchronous copies
+// 1920 x 1080, 4 channels: 323 M -> 200 M warp instructions, 385 -> 305 us (four pixels 347); 16 channels and absolute
+// gradients, 1237 x 719: 445 -> 374 (1920 x 1080 without: 4, 8, 13, 20 and 32 channels 385, 477, 827, 911, 1914 -> 305, 474, 676, 815, 1869;
+// 640 x 360, two pixels: 150, 164, 155, 168, 297 -> 113, 124, 153, 160, 305). Sums through shared memory instead of butterflies: 361; asynchronous copies
 // of the next batches: 9 us more. The atomics cost 14 us, the butterflies 40.
 // ---------------------------------------------------------------------------------------
 // The other variant of a kernel, for the cases that other registers or a skip suit better; pixels_bwd_other() chooses.
@@ -2112,96 +2114,94 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
                 T_batch = __fmul2_rn(T_batch, make_float2(s.x, s.y));
             }
         }
-        {
-            for (uint32_t t = t_lo; t < t_hi; ++t) {
-                float4 B;
-                float2 dx, dy, vis, alpha, open;
-                const int32_t id = sId[t];
-                if (!__any_sync(0xffffffffu, evaluate(t, id, B, dx, dy, vis, alpha, open))) continue;
-                const float4 Cc = sC[t];
-                const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
-                const float2 ra = reciprocal_pair(om);
-                T = __fmul2_rn(T, ra);
-                const float2 fac = __fmul2_rn(alpha, T);
-                const float2 dterm = __ffma2_rn(make_float2(Cc.x, Cc.x), roll,
-                                                __ffma2_rn(make_float2(Cc.z, Cc.z), dy, __fmul2_rn(make_float2(Cc.y, Cc.y), dx)));
-                float sum[CDIM + kGeo];
-                float2 dot = __fmul2_rn(dterm, v_depth);   // (c . g) of the two points, the compensated range in it
+        for (uint32_t t = t_lo; t < t_hi; ++t) {
+            float4 B;
+            float2 dx, dy, vis, alpha, open;
+            const int32_t id = sId[t];
+            if (!__any_sync(0xffffffffu, evaluate(t, id, B, dx, dy, vis, alpha, open))) continue;
+            const float4 Cc = sC[t];
+            const float2 om = __fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha.x, -alpha.y));
+            const float2 ra = reciprocal_pair(om);
+            T = __fmul2_rn(T, ra);
+            const float2 fac = __fmul2_rn(alpha, T);
+            const float2 dterm = __ffma2_rn(make_float2(Cc.x, Cc.x), roll,
+                                            __ffma2_rn(make_float2(Cc.z, Cc.z), dy, __fmul2_rn(make_float2(Cc.y, Cc.y), dx)));
+            float sum[CDIM + kGeo];
+            float2 dot = __fmul2_rn(dterm, v_depth);   // (c . g) of the two points, the compensated range in it
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float *v = v_out[h];
-                    const float2 f2 = h ? make_float2(fac.y, fac.y) : make_float2(fac.x, fac.x);
-                    float2 d2 = make_float2(0.f, 0.f);
+            for (int h = 0; h < 2; ++h) {
+                const float *v = v_out[h];
+                const float2 f2 = h ? make_float2(fac.y, fac.y) : make_float2(fac.x, fac.x);
+                float2 d2 = make_float2(0.f, 0.f);
 #pragma unroll
-                    for (int k = 0; k < CDIM; k += 4) {
-                        const float4 c4 = *reinterpret_cast<const float4 *>(sRgb + t * CDIM + k);
+                for (int k = 0; k < CDIM; k += 4) {
+                    const float4 c4 = *reinterpret_cast<const float4 *>(sRgb + t * CDIM + k);
 #pragma unroll
-                        for (int m = 0; m < 4; m += 2) {
-                            const float2 c2 = m ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
-                            const float2 v2 = make_float2(v[k + m], v[k + m + 1]);
-                            d2 = k + m == 0 ? __fmul2_rn(c2, v2) : __ffma2_rn(c2, v2, d2);
-                            const float2 acc = h == 0 ? __fmul2_rn(f2, v2) : __ffma2_rn(f2, v2, make_float2(sum[k + m], sum[k + m + 1]));
-                            sum[k + m] = acc.x; sum[k + m + 1] = acc.y;
-                        }
+                    for (int m = 0; m < 4; m += 2) {
+                        const float2 c2 = m ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
+                        const float2 v2 = make_float2(v[k + m], v[k + m + 1]);
+                        d2 = k + m == 0 ? __fmul2_rn(c2, v2) : __ffma2_rn(c2, v2, d2);
+                        const float2 acc = h == 0 ? __fmul2_rn(f2, v2) : __ffma2_rn(f2, v2, make_float2(sum[k + m], sum[k + m + 1]));
+                        sum[k + m] = acc.x; sum[k + m + 1] = acc.y;
                     }
-                    if (h) dot.y += d2.x + d2.y; else dot.x += d2.x + d2.y;
                 }
-                const float2 v_alpha = __ffma2_rn(T, dot, __fmul2_rn(make_float2(-ra.x, -ra.y), behind));
-                behind = __ffma2_rn(fac, dot, behind);
-                // v = -dL/dsigma / opacity; the alpha sum reaches the entries in front of the point
-                float2 vis_open = vis, fac_open = fac;
-                if (id < 0) {
-                    vis_open = __fmul2_rn(vis, open);
-                    fac_open = __fmul2_rn(fac, open);
-                }
-                const float2 v_main = __fmul2_rn(vis_open, v_alpha);
-                float2 v_sum = make_float2(0.f, 0.f);
-                if (compute_alpha_sum) {
-                    const float g_depth = sRgb[t * CDIM + depth_idx];
-                    v_sum = __fmul2_rn(vis, make_float2(g_depth < sum_limit.x ? v_asum.x : 0.f, g_depth < sum_limit.y ? v_asum.y : 0.f));
-                }
-                const float2 v = __fadd2_rn(v_main, v_sum);
-                const float2 w = __fmul2_rn(make_float2(-B.w, -B.w), v);                   // dL/dsigma
-                const float2 vd = __fmul2_rn(fac_open, v_depth);                           // dL/d(range term)
-                const float2 bx = make_float2(B.x, B.x), by = make_float2(B.y, B.y), bz = make_float2(B.z, B.z);
-                const float2 sx = __ffma2_rn(bx, dx, __fmul2_rn(by, dy)), sy = __ffma2_rn(by, dx, __fmul2_rn(bz, dy));
-                const float2 gx = __ffma2_rn(w, sx, __fmul2_rn(vd, make_float2(Cc.y, Cc.y)));
-                const float2 gy = __ffma2_rn(w, sy, __fmul2_rn(vd, make_float2(Cc.z, Cc.z)));
-                const float2 wx = __fmul2_rn(w, dx), wy = __fmul2_rn(w, dy);
-                const auto both = [](float2 p, float2 q) { const float2 r = __fmul2_rn(p, q); return r.x + r.y; };
-                sum[CDIM + 0] = both(wx, dx);
-                sum[CDIM + 1] = both(wx, dy);
-                sum[CDIM + 2] = both(wy, dy);
-                sum[CDIM + 3] = gx.x + gx.y;
-                sum[CDIM + 4] = gy.x + gy.y;
-                sum[CDIM + 5] = both(gx, roll);
-                sum[CDIM + 6] = both(gy, roll);
-                sum[CDIM + 7] = both(vd, roll);
-                sum[CDIM + 8] = both(vd, dx);
-                sum[CDIM + 9] = both(vd, dy);
-                sum[CDIM + 10] = v.x + v.y;
-                if (kAbs) {
-                    const float2 us = __fmul2_rn(make_float2(-B.w, -B.w), v_sum);
-                    const float2 ux = __fmul2_rn(us, sx), uy = __fmul2_rn(us, sy);
-                    sum[CDIM + 11] = fabsf(gx.x - ux.x) + fabsf(ux.x) + fabsf(gx.y - ux.y) + fabsf(ux.y);
-                    sum[CDIM + 12] = fabsf(gy.x - uy.x) + fabsf(uy.x) + fabsf(gy.y - uy.y) + fabsf(uy.y);
-                }
-                const size_t gid = (size_t)(id & INT32_MAX);
-                float sums[kSums];
+                if (h) dot.y += d2.x + d2.y; else dot.x += d2.x + d2.y;
+            }
+            const float2 v_alpha = __ffma2_rn(T, dot, __fmul2_rn(make_float2(-ra.x, -ra.y), behind));
+            behind = __ffma2_rn(fac, dot, behind);
+            // v = -dL/dsigma / opacity; the alpha sum reaches the entries in front of the point
+            float2 vis_open = vis, fac_open = fac;
+            if (id < 0) {
+                vis_open = __fmul2_rn(vis, open);
+                fac_open = __fmul2_rn(fac, open);
+            }
+            const float2 v_main = __fmul2_rn(vis_open, v_alpha);
+            float2 v_sum = make_float2(0.f, 0.f);
+            if (compute_alpha_sum) {
+                const float g_depth = sRgb[t * CDIM + depth_idx];
+                v_sum = __fmul2_rn(vis, make_float2(g_depth < sum_limit.x ? v_asum.x : 0.f, g_depth < sum_limit.y ? v_asum.y : 0.f));
+            }
+            const float2 v = __fadd2_rn(v_main, v_sum);
+            const float2 w = __fmul2_rn(make_float2(-B.w, -B.w), v);                   // dL/dsigma
+            const float2 vd = __fmul2_rn(fac_open, v_depth);                           // dL/d(range term)
+            const float2 bx = make_float2(B.x, B.x), by = make_float2(B.y, B.y), bz = make_float2(B.z, B.z);
+            const float2 sx = __ffma2_rn(bx, dx, __fmul2_rn(by, dy)), sy = __ffma2_rn(by, dx, __fmul2_rn(bz, dy));
+            const float2 gx = __ffma2_rn(w, sx, __fmul2_rn(vd, make_float2(Cc.y, Cc.y)));
+            const float2 gy = __ffma2_rn(w, sy, __fmul2_rn(vd, make_float2(Cc.z, Cc.z)));
+            const float2 wx = __fmul2_rn(w, dx), wy = __fmul2_rn(w, dy);
+            const auto both = [](float2 p, float2 q) { const float2 r = __fmul2_rn(p, q); return r.x + r.y; };
+            sum[CDIM + 0] = both(wx, dx);
+            sum[CDIM + 1] = both(wx, dy);
+            sum[CDIM + 2] = both(wy, dy);
+            sum[CDIM + 3] = gx.x + gx.y;
+            sum[CDIM + 4] = gy.x + gy.y;
+            sum[CDIM + 5] = both(gx, roll);
+            sum[CDIM + 6] = both(gy, roll);
+            sum[CDIM + 7] = both(vd, roll);
+            sum[CDIM + 8] = both(vd, dx);
+            sum[CDIM + 9] = both(vd, dy);
+            sum[CDIM + 10] = v.x + v.y;
+            if (kAbs) {
+                const float2 us = __fmul2_rn(make_float2(-B.w, -B.w), v_sum);
+                const float2 ux = __fmul2_rn(us, sx), uy = __fmul2_rn(us, sy);
+                sum[CDIM + 11] = fabsf(gx.x - ux.x) + fabsf(ux.x) + fabsf(gx.y - ux.y) + fabsf(ux.y);
+                sum[CDIM + 12] = fabsf(gy.x - uy.x) + fabsf(uy.x) + fabsf(gy.y - uy.y) + fabsf(uy.y);
+            }
+            const size_t gid = (size_t)(id & INT32_MAX);
+            float sums[kSums];
 #pragma unroll
-                for (int k = 0; k < kSums; ++k) sums[k] = sum[k];
-                slot_a.add(gid, warp_sum_values<kSums, 16>(sums, lane), 1.f, mine_a.writes);
-                if (kSplit) {
-                    float geo[kGeo];
+            for (int k = 0; k < kSums; ++k) sums[k] = sum[k];
+            slot_a.add(gid, warp_sum_values<kSums, 16>(sums, lane), 1.f, mine_a.writes);
+            if (kSplit) {
+                float geo[kGeo];
 #pragma unroll
-                    for (int k = 0; k < kGeo; ++k) geo[k] = sum[CDIM + k];
-                    const float geo_total = warp_sum_values<kGeo, 16>(geo, lane);
-                    const SumSlot mine_b = sum_slot<kGeo>(lane);
-                    const GradSlot slot_b = point_grad_slot<kAbs>(CDIM + mine_b.value, CDIM, channels, fstride, v_colors,
-                                                                  v_ranges, v_conics, v_means2d, v_pix_vels, v_depth_comps,
-                                                                  v_opacities, v_means2d_abs);
-                    slot_b.add(gid, geo_total, 1.f, mine_b.writes);
-                }
+                for (int k = 0; k < kGeo; ++k) geo[k] = sum[CDIM + k];
+                const float geo_total = warp_sum_values<kGeo, 16>(geo, lane);
+                const SumSlot mine_b = sum_slot<kGeo>(lane);
+                const GradSlot slot_b = point_grad_slot<kAbs>(CDIM + mine_b.value, CDIM, channels, fstride, v_colors,
+                                                              v_ranges, v_conics, v_means2d, v_pix_vels, v_depth_comps,
+                                                              v_opacities, v_means2d_abs);
+                slot_b.add(gid, geo_total, 1.f, mine_b.writes);
             }
         }
         if (n_warps > 1) { T = T_batch; behind = behind_batch; }
@@ -2220,13 +2220,13 @@ __global__ void __launch_bounds__(CDIM <= 8 ? 512 : 256, CDIM <= 8 || CDIM > 20 
         else { CALL(32); }                                                                       \
     } while (0)
 
-// Forward kernels of many blocks start on empty SMs. The line is one for all of them: eight blocks an SM, what the
-// four-channel camera kernel has room for (32 channels hold four, the lidar's 64 threads up to twelve). Chained, their first
+// Forward kernels of many blocks start on empty SMs: 1184 blocks of a lidar, four times as many one-warp blocks of a
+// camera. The line is where a frame is faster, not what the kernels have room for. Chained, their first
 // blocks are placed beside the last of the colour or list kernels before them, on SMs that keep that kernel's
 // large shared memory and small first-level cache for as long as one block follows another, and the gathers need
-// the cache (with all of it given to shared memory the 1920 x 1080 kernel takes 237 us instead of 209): with
-// spherical harmonics 437 us a frame chained, 411 apart; six cameras 3490 and 3370; 128 x 1800 lidar 294 and 289.
-// Below, the launch gap weighs more (640 x 360: 101 and 103).
+// the cache. Whole frames, us, chained and apart: with spherical harmonics 640 x 360 (3680 warps) 131.7 and 130.9, 800 x 450 (5800) 133.0
+// and 124.4, 960 x 540 151 and 142, 1280 x 720 198 and 194, 1600 x 900 279 and 274, 1920 x 1080 346 and 345; plain colours 106.5 and 108.3 at 480 x 270, 1 to 3 us the
+// other way from there on, the launch gap; 128 x 1800 lidar with 4 and 16 features 307 and 297, 308 and 302, 128 x 1200 within 1.
 static bool fits_at_once(uint64_t blocks) { return blocks <= (uint64_t)kNumSMs * 8; }
 static bool warps_fit_at_once(uint64_t warps) { return fits_at_once(warps / 4); }
 
@@ -2418,6 +2418,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
                     v_render_alphas && v_means2d && v_conics && v_colors && v_opacities &&
                     v_pix_vels && rolling_shutter_time,
                 SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_bwd: null argument");
+    // (a limit from one thread per pixel, which these kernels do not have; callers count on the error, and frames.cpp asks the same
+    // before it renders)
     const uint32_t samples = ((tile_size * tile_size + 31) / 32) * 32;
     SPL_REQUIRE(samples <= 512 || channels <= 16, SPLATAD_ERR_BAD_ARG,
                 "rasterize_to_pixels_bwd: a tile of %u pixels (%u threads at one per pixel) with %u channels is more "
@@ -2492,8 +2494,7 @@ extern "C" int splatad_rasterize_to_points_fwd(
     {                                                                                             \
         auto kernel = coop ? rasterize_to_points_fwd_coop_kernel<D> : rasterize_to_points_fwd_kernel<D>; \
         const size_t smem = (size_t)(coop ? 1 : points_fwd_stage(D)) * bs *                       \
-                                (3 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float)) +  \
-                            0;                                                                    \
+                                (3 * sizeof(float4) + 2 * sizeof(int32_t) + D * sizeof(float));   \
         int rc = set_smem(kernel, smem, "rasterize_to_points_fwd");                               \
         if (rc != SPLATAD_OK) return rc;                                                          \
         launch_chained_if(fits_at_once((uint64_t)blocks * parts), kernel, blocks * parts, bs, smem, \
