@@ -2238,7 +2238,7 @@ static bool warps_fit_at_once(uint64_t warps) { return fits_at_once(warps / 4); 
 // Forward, 4 channels: 8160 tiles, 27.5 per Gaussian 197 / 150 / 144 (214), 12.7: 205 / 162 / 158 (220), 7.5: 187 / 156 / 175 (195), 5.4: 187 / 195 / 268
 // (193), 3.8: 160 / 164 / 245 (161), 2.5: 109 / 116 / 180 (109), Gaussians all of one size, 3.5: 39 / 31 / 37 (41); 5700, 9.6: 148 / 119 / 125, 5.8: 136 / 148 / 195;
 // 3510, 13: 98 / 79 / 84 (105), 6.6: 87 / 96 / 129 (92), 4.3: 105 / 132 / 191 (109); 2040, 8.9: 62 / 66 / 80 (67); 920, 5.1: 62 / 84. 8 channels: 8160, 7.5: 234 / 225
-// (267), 5.4: 238 / 262 (262); 3510, 13: 112 / 104 (142), 6.6: 103 / 120 (122). 16 channels: 8160, 7.5: 343 / 312 (334), 5.4: 349 / 352 (340); 3510, 13: 162 / 146 (171), 6.6: 150 /
+// (267), 5.4: 238 / 262 (262); 3510, 13: 112 / 104 (142), 6.6: 103 / 120 (122). 16 channels: 8160, 7.5: 343 / 312 (334), 5.4: 402 / 377 (369) and with 13 of them 350 / 352 (340), 2.5: 287 / 284 (271); 3510, 13: 162 / 146 (171), 6.6: 150 /
 // 157 (152).
 // Backward, 4 channels: 8160 tiles, 27.5: 493 / 347 / 305 (383), 12.7: 506 / 373 / 337 (404), 7.5: 473 / 362 / 376 (383), 5.4: 442 / 415 / 584 (422), 3.8: 365 / 385 / 569
 // (414), 2.5: 229 / 268 / 410 (297); 5700, 9.6: 375 / 276 / 264; 3510, 13: 240 / 180 / 175 (194), 6.6: 208 / 207 / 274 (209), 4.3: 247 / 283 / 418 (288); 2040, 8.9: 156 /
@@ -2261,8 +2261,8 @@ static uint32_t pixels_that_fit(bool four, bool eight, uint32_t tile_size) {
 }
 static uint32_t pixels_per_lane_fwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
-    const bool many = channels <= 4 && tiles >= 6000u;
-    return pixels_that_fit(tiles >= (channels <= 8 ? 2700u : 1500u) && covers(spread, many ? 3.3f : 7.f), many && covers(spread, 10.f), tile_size);
+    const float line = tiles < 6000u ? 7.f : channels <= 4 ? 3.3f : channels <= 8 ? 7.f : 5.f;
+    return pixels_that_fit(tiles >= (channels <= 8 ? 2700u : 1500u) && covers(spread, line), channels <= 4 && tiles >= 6000u && covers(spread, 10.f), tile_size);
 }
 static uint32_t pixels_per_lane_bwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);

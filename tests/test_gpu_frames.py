@@ -21,6 +21,28 @@ def _forget():
         hint.clear()
 
 
+@pytest.mark.parametrize("packed", [False, True])
+def test_a_frame_reports_how_many_tiles_its_gaussians_cover(packed):
+    """List entries per Gaussian that the lists hold: from the ops in a first frame, from the plan's own words in the next
+    ones. It goes with the lists and chooses how the next frame is split, which changes no bit of its image."""
+    import splatad_b200
+    from splatad_b200 import ops, scenes
+    g = _to_gpu(scenes.config1(N=20_011, packed=packed))
+    _forget()
+    first = None
+    for hint in (None, None, 1.0, 6.0, 50.0):
+        if hint is None and first is None:
+            ops._spread_hint.clear()
+        elif hint is not None:
+            ops._spread_hint[next(iter(ops._spread_hint))] = hint
+        image, alpha, meta = splatad_b200.rasterization(**g)
+        want = meta["flatten_ids"].numel() / int((meta["tiles_per_gauss"] > 0).sum())
+        assert list(ops._spread_hint.values()) == [pytest.approx(want)] and want > 1.0
+        assert meta["flatten_ids"]._splatad_spread == pytest.approx(want)
+        first = first or (image, alpha)
+        assert torch.equal(image, first[0]) and torch.equal(alpha, first[1])
+
+
 @pytest.mark.parametrize("kind", ["lidar", "camera"])
 def test_a_frame_that_sees_nothing_has_zero_gradients(kind):
     import splatad_b200

@@ -144,7 +144,7 @@ def test_what_a_native_frame_reports_is_kept_for_the_next(monkeypatch):
     buckets. An overflow of the buckets drops a range that was carried over, and means the radix sort only without
     one; more intersections than the ids can number are an error."""
     from splatad_b200 import ops
-    for name in ("_isect_count_hint", "_depth_range_hint", "_depth_sort_mode"):
+    for name in ("_isect_count_hint", "_depth_range_hint", "_depth_sort_mode", "_spread_hint"):
         monkeypatch.setattr(ops, name, {})
     lo, hi = 0x3E99999A, 0x42E20000                    # 0.3 and 113.0 as float bit patterns
     ops.note_counts("shape", 1000, 0, lo | (hi << 32), ranged=False)
@@ -155,6 +155,9 @@ def test_what_a_native_frame_reports_is_kept_for_the_next(monkeypatch):
     assert ops._depth_range_hint == {} and ops._depth_sort_mode == {}
     ops.note_counts("shape", 900, 4, lo | (hi << 32), ranged=False)
     assert ops._depth_range_hint == {} and ops._depth_sort_mode == {"shape": 2}
+    assert ops._spread_hint == {}                      # nobody said how many Gaussians are listed
+    ops.note_counts("shape", 900, 0, 0, True, 300)
+    assert ops._spread_hint == {"shape": 3.0}
     with pytest.raises(RuntimeError, match="do not fit"):
         ops.note_counts("shape", 2**31, 2, 0, ranged=False)
     assert ops.list_room(900) > 900 and ops.packed_room(70_000, 10**6) % 65536 == 0 and ops.packed_room(70_000, 70_001) == 70_001
