@@ -1343,8 +1343,13 @@ blk_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket) {
 // kWrap: rectangles may cover the turn more than once and then leave several records in a block (a
 // rectangle spans less than five turns): three more mask words per (warp, block) hold the bits of their
 // lanes' surplus.
-template <bool kWrap>
-__global__ void __launch_bounds__(kBlkThreads)
+// kCtas an SM, by what the registers leave: the sixteen counts of a column take 64 with wraps, which pays where a CTA has many columns (30
+// of them, 128 x 1800: 37.4 with three CTAs, 35.7 with two; 20, 96 x 1200: 29.2 and 27.1) and not where it has few (10, two sensors of
+// 70 x 556: 35.3 and 41.4; 9, 64 x 1083 and 800,000 Gaussians: 18.9 and 21.0).
+constexpr uint32_t kBlkManyCols = 16;
+
+template <bool kWrap, int kCtas>
+__global__ void __launch_bounds__(kBlkThreads, kCtas)
 blk_scatter_kernel(BlkArgs a) {
     chain_enter();
     extern __shared__ uint32_t s_dyn[];
@@ -2128,7 +2133,8 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
         const size_t smem_count = sizeof(uint32_t) * a.blocks;
         const size_t smem_scatter = sizeof(uint32_t) * kBlkWarps * min(kBlkRows, a.by) * a.bx * (g.lidar ? 5 : 2);
         auto count = g.lidar ? blk_count_kernel<true> : blk_count_kernel<false>;
-        auto scatter = g.lidar ? blk_scatter_kernel<true> : blk_scatter_kernel<false>;
+        auto scatter = !g.lidar ? blk_scatter_kernel<false, 4>
+                       : min(kBlkRows, a.by) * a.bx >= kBlkManyCols ? blk_scatter_kernel<true, 2> : blk_scatter_kernel<true, 3>;
         if (smem_scatter > 48 * 1024)
             cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_scatter);
         unsigned long long *ticket = (unsigned long long *)(p.counters + CNT_TICKET);
