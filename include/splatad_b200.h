@@ -495,6 +495,11 @@ int splatad_color_rows_bwd(uint32_t n, uint32_t N, uint32_t D, uint32_t width, c
                            const int64_t *gaussian_ids, uint32_t colors_per_camera, const float *v_rows,
                            float *v_colors, const float *v_depths_in, float *v_depths, void *stream);
 
+/* No counterpart in the reference. Arms a one-shot hint for the NEXT splatad_rasterize_to_points_fwd call of the
+ * calling thread: rows of its Gaussian arrays (C * N; 0: not known). With the number of patches it chooses whether the warps of a
+ * block share one patch of points; feature sums are then added in another order. */
+int splatad_rasterize_set_rows_hint(uint64_t rows);
+
 /* rasterize_to_points_fwd_tensor - gsplat/cuda/csrc/rasterization.cu:2221-2831, kernel
  * 2021-2219. raster_pts [C,H,W,4] = (azimuth deg, elevation deg, range m, time offset s);
  * points with range <= 0 are not rendered and produce zeros. pix_vels [.,3],

@@ -914,7 +914,8 @@ __device__ __forceinline__ void stage_features(float *row, const float *__restri
 // of the (point, entry) pairs of a small scan contribute, two thirds of the benchmark's) and evaluates
 // two of them at a time, because what it waits for is the chain from the offsets through the exponential
 // to the transmittance. (Leaving the wrap, the sign of sigma and the cap to the entries that need them, as the other
-// lidar kernels do, gains nothing here: 128 x 1800 43.3 -> 44.4 us.) The rendered rows leave through shared memory: a beam's eight points
+// lidar kernels do, gains nothing here: 128 x 1800 43.3 -> 44.4 us. What a scan takes hangs on what lies next to the sensor: 128 x 1800, 17
+// channels 45 to 93 us over eight turns of it, backward 84 to 186; figures of that size here and below are of a turn of 37 degrees.) The rendered rows leave through shared memory: a beam's eight points
 // are consecutive floats.
 // ---------------------------------------------------------------------------------------
 // entries per thread and batch (their loads overlap), while the shared memory of a batch stays small
@@ -2283,21 +2284,29 @@ static float take_spread_hint(uint32_t tile_size) {
     return spread;
 }
 
-// Patches below which all warps of a CTA share one in the forward pass: the shared work costs more
-// instructions in all, so the patches must be too few to fill the machine. Apart and shared, us, 8 channels: 256
-// patches 157 and 42, 512 109 and 32, 800 64 and 38, 1216 54 and 41, 1600 51 and 51, 2176 49 and 67, 3712 62 and 109; 17
-// channels: 512 126 and 34, 1216 65 and 47, 1600 54 and 58, 2176 56 and 77.
-constexpr uint64_t kCoopPatches = kNumSMs * 10;
+// Whether all warps of a CTA share one patch in the forward pass: the shared work costs more instructions in all, so the
+// patches must be too few to fill the machine. Apart and shared, us, 4 / 12 channels beside the range, by rows of Gaussians per patch: 256
+// patches, 40 rows 130 / 146 and 31 / 36, 600 rows 60 / 64 and 19 / 23; 512, 40: 132 / 148 and 39 / 44, 600: 41 / 46 and 27 / 33; 1024, 40: 80 / 89 and 44 / 53, 600: 39 / 42 and
+// 41 / 50. From 1184 patches on it takes sparse scenes, whose lists saturate late and are walked by few warps at their end: 1280 patches, 40
+// rows 78 / 90 and 50 / 60, 100: 54 / 60 and 46 / 58, 250: 46 / 46 and 48 / 58, 600: 35 / 39 and 46 / 56; 1440, 40: 70 / 74 and 52 / 64, 100: 50 / 52 and 52 / 63. 21 channels never: 1280, 40:
+// 95 and 99, 100: 64 and 96. Rows not known (0): as dense.
+static bool shares_patches(uint64_t patches, uint32_t channels, uint64_t rows) {
+    if (patches < kNumSMs * 8u) return true;
+    return patches < kNumSMs * 10u && channels <= 20 && rows > 0 && rows < patches * (channels <= 8 ? 100u : 60u);
+}
+
+// One-shot hint of the calling thread's next lidar compositing call.
+static thread_local uint64_t t_rows_hint = 0;
 
 // Warps - segments of the list - per patch in the backward pass: every segment is run twice, which pays
 // while the patches alone leave the schedulers waiting on one warp's chain. One, four and eight segments, us, 8
 // channels: 400 patches 163, 71, 56, 608 121, 61, 57, 800 100, 66, 64, 1088 85, 72, 80, 1600 93, 96, 108, 2240 97, 118, 138, 2816
 // 126, 136, 164 (256: eight 54, sixteen 49); 17 channels: 400 203, 91, 76, 608 152, 78, 74, 800 124, 87, 87, 1088 107, 95,
-// 105, 1600 121, 128, 147, 2240 126, 152, 182. Sixteen take an SM each, and only up to eight channels stay within their 128
-// registers.
+// 105, 1600 121, 128, 147, 2240 126, 152, 182 (19 channels, 792: four 74, eight 76); 21 channels: 1400 one 311, four 282, 1824 303 and 317. Sixteen take
+// an SM each, and only up to eight channels stay within their 128 registers.
 static uint32_t point_segments(uint64_t patches, uint32_t channels) {
     if (channels <= 8 && patches < (uint64_t)kNumSMs * 2) return 16u;
-    return patches < (uint64_t)kNumSMs * 6 ? 8u : patches < (uint64_t)kNumSMs * 9 ? 4u : 1u;
+    return patches < (uint64_t)kNumSMs * (channels <= 8 ? 6 : 5) ? 8u : patches < (uint64_t)kNumSMs * (channels <= 20 ? 9 : 11) ? 4u : 1u;
 }
 
 template <typename K>
@@ -2316,6 +2325,11 @@ static int set_smem(K kernel, size_t bytes, const char *what) {
 } // namespace splatad
 
 using namespace splatad;
+
+extern "C" int splatad_rasterize_set_rows_hint(uint64_t rows) {
+    t_rows_hint = rows;
+    return SPLATAD_OK;
+}
 
 extern "C" int splatad_rasterize_set_spread_hint(float tiles_per_gaussian) {
     t_spread_hint = tiles_per_gaussian;
@@ -2465,6 +2479,8 @@ extern "C" int splatad_rasterize_to_points_fwd(
     const int32_t *tile_offsets, const int32_t *flatten_ids, uint32_t depth_channel_idx,
     float *render_features, float *render_alphas, float *alpha_sum_until_points,
     int32_t *last_ids, float *median_depths, void *stream) {
+    const uint64_t rows = t_rows_hint;
+    t_rows_hint = 0;
     SPL_REQUIRE(channels >= 1 && channels <= SPLATAD_MAX_CHANNELS, SPLATAD_ERR_CHANNELS,
                 "rasterize_to_points_fwd: unsupported channel count %u (1..%d)", channels,
                 SPLATAD_MAX_CHANNELS);
@@ -2486,7 +2502,7 @@ extern "C" int splatad_rasterize_to_points_fwd(
     const uint32_t blocks = C * tile_grid_width * tile_grid_height;
     if (blocks == 0 || image_width == 0 || image_height == 0) return SPLATAD_OK;
     const uint32_t warps = div_up(tile_width * tile_height, 32);
-    const bool coop = (uint64_t)blocks * warps < kCoopPatches;
+    const bool coop = shares_patches((uint64_t)blocks * warps, channels, rows);
     // two warps per CTA otherwise: a CTA ends with its slowest warp
     const uint32_t per_cta = min(2u, warps), parts = coop ? warps : div_up(warps, per_cta), bs = coop ? kCoopWarps * 32 : 32 * per_cta;
     SPL_REQUIRE((uint64_t)blocks * parts <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_points_fwd: too many tiles");

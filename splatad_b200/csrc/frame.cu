@@ -50,6 +50,7 @@ extern "C" int splatad_lidar_frame_fwd(
     if (rc != SPLATAD_OK) return rc;
     const uint32_t grid_w = splatad_lidar_azimuth_tiles(tile_azim_res);
     const uint32_t grid_h = n_boundaries - 1;
+    splatad_rasterize_set_rows_hint(total);
     // n_isects = -1: the end of the last tile is read from tile_offsets[C * tiles], written by the fill
     return splatad_rasterize_to_points_fwd(C, -1, means2d, conics, lidar_features, depths, n_features + 1,
                                            opacities_cn, pix_vels, depth_compensations, nullptr, raster_pts,

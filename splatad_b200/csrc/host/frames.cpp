@@ -42,7 +42,7 @@ using OptTensor = c10::optional<Tensor>;
     X(splatad_isect_plan_workspace_bytes) X(splatad_isect_fill_workspace_bytes) X(splatad_lidar_azimuth_tiles)           \
     X(splatad_isect_tiles_plan) X(splatad_isect_tiles_fill) X(splatad_isect_lidar_tiles_plan)                            \
     X(splatad_isect_lidar_tiles_fill) X(splatad_isect_set_early_count) X(splatad_isect_set_depth_range_hint)             \
-    X(splatad_isect_set_listed_count) X(splatad_rasterize_set_spread_hint)                                               \
+    X(splatad_isect_set_listed_count) X(splatad_rasterize_set_spread_hint) X(splatad_rasterize_set_rows_hint)            \
     X(splatad_rasterize_expected_to_pixels_fwd) X(splatad_rasterize_expected_to_pixels_bwd)                              \
     X(splatad_lidar_frame_fwd) X(splatad_rasterize_to_points_fwd) X(splatad_rasterize_to_points_bwd) X(splatad_map_points_workspace_bytes)          \
     X(splatad_map_strided_points_to_lidar_tiles) X(splatad_points_mapping_offset_encode) X(splatad_populate_image_from_points)
@@ -516,6 +516,7 @@ py::object lidar_frame(const Tensor &means, const Tensor &quats, const Tensor &s
             check(grid(lib.splatad_isect_lidar_tiles_plan, plan_ws.data_ptr(), (size_t)plan_ws.numel(), (int64_t *)nullptr, stream.stream()));
             check(grid(lib.splatad_isect_lidar_tiles_fill, plan_ws.data_ptr(), fill_ws.data_ptr(), (size_t)fill_ws.numel(), capacity,
                        L(f->isect_ids), I(f->flatten_ids), I(f->offsets), (int64_t *)nullptr, stream.stream()));
+            lib.splatad_rasterize_set_rows_hint((uint64_t)(C * N));
             check(lib.splatad_rasterize_to_points_fwd(
                 (uint32_t)C, -1, F(f->means2d), F(f->conics), F(features), F(f->depths), (uint32_t)(D + 1), opacity, F(f->pix_vels),
                 F(f->depth_comps), nullptr, F(raster_pts), (uint32_t)W, (uint32_t)H, f->tile_w, f->tile_h, (uint32_t)cols, (uint32_t)rows,

@@ -1624,6 +1624,7 @@ class _RasterizeToPoints(torch.autograd.Function):
         median_depths = torch.empty((C, height, width, 1), **f32)
         alpha_sum = torch.empty((C, height, width, 1), **f32) if compute_alpha_sum_until_points else None
         last_ids = torch.empty((C, height, width), dtype=torch.int32, device=dev)
+        _lib.load().splatad_rasterize_set_rows_hint(means2d.numel() // 2)
         _call(
             "splatad_rasterize_to_points_fwd", C, ctx.n_isects_arg, _lib.ptr(means2d),
             _lib.ptr(conics_f), _lib.ptr(colors_f) if colors_f.numel() else None, _lib.ptr(ranges_f), channels,

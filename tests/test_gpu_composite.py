@@ -550,6 +550,38 @@ def test_points_in_patches(tw, th, H, W, channels, asum, absgrad):
         _grad_check(f"tile {tw}x{th} ch={channels} absgrad", leaves["means2d"].absgrad, ref["v_means2d_abs"])
 
 
+@pytest.mark.parametrize("C,N,channels,shared", [(2, 400, 5, True), (2, 65_000, 5, False), (2, 500, 13, True), (2, 39_000, 13, False),
+                                                 (2, 400, 24, False)])
+def test_points_of_sparse_and_dense_scenes(C, N, channels, shared):
+    """Scans of 1184 to 1479 patches share a patch between the warps of a block where the scene is sparse. Either way gives the
+    oracle's features, and the same transmittances bit for bit as without the hint."""
+    from oracle import composite
+    from splatad_b200 import _lib, ops
+    H, W, tw, th = 64, 320, 32, 8                      # 1280 patches
+    c = _lidar_case(C, N, H, W, tw, th, channels, 3 * N + channels)
+    assert (C * N < 1280 * (100 if channels <= 8 else 60) and channels <= 20) == shared
+    keys = ("means2d", "conics", "feats", "opacities", "pix_vels", "dcomp")
+    ref = composite.rasterize_to_points_fwd(*(n(c[k]) for k in keys), None, n(c["pts"]), W, H, tw, th, c["offsets"], c["flatten_ids"],
+                                            True, 0.5)
+    dev = [t(c[k]) for k in keys]
+    offsets, ids, pts = t(c["offsets"], torch.int32), t(c["flatten_ids"], torch.int32), t(c["pts"])
+    out_c, out_a, out_s, out_m = ops.rasterize_to_points(*dev, pts, W, H, tw, th, offsets, ids, True, 0.5)
+    sure = ~ref["ambiguous"][..., None]
+    assert_close("features", n(out_c), ref["render_colors"], 2e-4, 2e-5, mask=sure)
+    assert_close("alphas", n(out_a), ref["render_alphas"], 2e-4, 2e-5, mask=sure)
+    # without the hint: one warp to a patch
+    p, f = _lib.ptr, torch.float32
+    image, alphas, sums, medians = (torch.empty(C, H, W, k, device=DEV, dtype=f) for k in (channels, 1, 1, 1))
+    last = torch.empty(C, H, W, dtype=torch.int32, device=DEV)
+    _lib.call("splatad_rasterize_to_points_fwd", C, ids.numel(), p(dev[0]), p(dev[1]), p(dev[2]), None, channels, p(dev[3]), p(dev[4]), p(dev[5]),
+              None, p(pts), W, H, tw, th, offsets.shape[2], offsets.shape[1], 1, 0.5, p(offsets), p(ids), channels - 1, p(image), p(alphas), p(sums),
+              p(last), p(medians), _lib.stream_ptr(ids.device))
+    assert torch.equal(alphas, out_a)
+    assert_close("medians", n(medians), n(out_m), 1e-5, 1e-6)  # of the same entry, its range term rounded in another order
+    assert_close("features", n(image), n(out_c), 1e-5, 1e-6)   # sums of eight warps added in order, 32-bit
+    assert torch.equal(image, out_c) or shared
+
+
 @pytest.mark.parametrize("C,H,W,channels", [(1, 16, 256, 3), (1, 32, 300, 9), (6, 64, 512, 5), (6, 64, 512, 18)])
 def test_points_with_needles_and_the_seam(C, H, W, channels):
     """Entries whose alphas or angles need care beside those that do not - needles on either side of the line, a conic that
