@@ -2302,11 +2302,13 @@ static thread_local uint64_t t_rows_hint = 0;
 // while the patches alone leave the schedulers waiting on one warp's chain. One, four and eight segments, us, 8
 // channels: 400 patches 163, 71, 56, 608 121, 61, 57, 800 100, 66, 64, 1088 85, 72, 80, 1600 93, 96, 108, 2240 97, 118, 138, 2816
 // 126, 136, 164 (256: eight 54, sixteen 49); 17 channels: 400 203, 91, 76, 608 152, 78, 74, 800 124, 87, 87, 1088 107, 95,
-// 105, 1600 121, 128, 147, 2240 126, 152, 182 (19 channels, 792: four 74, eight 76); 21 channels: 1400 one 311, four 282, 1824 303 and 317. Sixteen take
+// 105, 1600 121, 128, 147, 2240 126, 152, 182 (19 channels, 792: four 74, eight 76); 21 channels: 1400 one 311, four 282, 1824 303 and 317.
+// Sparse scenes gain most: 5 channels, entries per tile 430, 1430, 4300 and 8600: 1344 patches one segment 180, 102, 86, 92, four 105, 92, 86, 83; 1560: 176, 105, 90, 95
+// and 107, 97, 93, 89; 1824: 168, 109, 94, 96 and 117, 107, 102, 98; 2240, 630: 171 and 167. Sixteen take
 // an SM each, and only up to eight channels stay within their 128 registers.
-static uint32_t point_segments(uint64_t patches, uint32_t channels) {
+static uint32_t point_segments(uint64_t patches, uint32_t channels, bool sparse) {
     if (channels <= 8 && patches < (uint64_t)kNumSMs * 2) return 16u;
-    return patches < (uint64_t)kNumSMs * (channels <= 8 ? 6 : 5) ? 8u : patches < (uint64_t)kNumSMs * (channels <= 20 ? 9 : 11) ? 4u : 1u;
+    return patches < (uint64_t)kNumSMs * (channels <= 8 ? 6 : 5) ? 8u : patches < (uint64_t)kNumSMs * (sparse ? 14 : 11) ? 4u : 1u;
 }
 
 template <typename K>
@@ -2567,7 +2569,7 @@ extern "C" int splatad_rasterize_to_points_bwd(
                 "rasterize_to_points_bwd: a tile of %u points (%u threads at one per point) with %u channels is more "
                 "than the backward pass takes: use a smaller tile or at most 16 channels per call",
                 tile_width * tile_height, samples, channels);
-    const uint32_t parts = div_up(tile_width * tile_height, 64), bs = 32 * point_segments((uint64_t)blocks * parts, channels);
+    const uint32_t parts = div_up(tile_width * tile_height, 64), bs = 32 * point_segments((uint64_t)blocks * parts, channels, n_isects > 0 && n_isects < (int64_t)blocks * 1000);
     SPL_REQUIRE((uint64_t)blocks * parts <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_points_bwd: too many tiles");
 #define CALL_ABS(D, A)                                                                            \
     {                                                                                             \
