@@ -2260,15 +2260,25 @@ static uint32_t pixels_that_fit(bool four, bool eight, uint32_t tile_size) {
     if (eight && tile_threads<8>(tile_size) % 32u == 0u) return 8u;
     return (four || eight) && tile_threads<4>(tile_size) >= 32u ? 4u : 2u;
 }
-static uint32_t pixels_per_lane_fwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread) {
+// Sparse scenes: few list entries in all, and the longest list's chain counts; fewer pixels per lane make it shorter. Used where both numbers
+// are known. 4 channels, entries in thousands, two / four / eight pixels, us, forward: 3200 tiles, 8 per Gaussian, 186: 56 / 66 / 99, 698: 62 / 64 / 76,
+// 1490: 84 / 68 / 70; 3536, 12, 255: 56 / 64 / 80, 990: 80 / 70 / 78; 4753, 19, 404: 74 / 68 / 82; 8160, 28, 604: 107 / 87 / 93, 1170: 142 / 113 / 113, 2300: 177 / 138 / 131. Backward: 3200, 186: 136 / 141 /
+// 211, 698: 147 / 141 / 158, 1490: 209 / 162 / 152; 3536, 255: 130 / 140 / 173, 495: 159 / 166 / 199, 990: 197 / 158 / 166, 2090: 245 / 184 / 172; 4753, 404: 174 / 154 / 176, 784: 232 / 184 / 203, 1550: 286 / 213 / 199;
+// 8160, 604: 258 / 193 / 196, 1170: 348 / 256 / 238.
+static bool many_entries(float spread, int64_t entries, int64_t line, float or_spread) {
+    return !(spread > 0.f) || entries <= 0 || entries >= line || spread >= or_spread;
+}
+static uint32_t pixels_per_lane_fwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread, int64_t entries) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
     const float line = tiles < 6000u ? 7.f : channels <= 4 ? 3.3f : channels <= 8 ? 7.f : 5.f;
-    return pixels_that_fit(tiles >= (channels <= 8 ? 2700u : 1500u) && covers(spread, line), channels <= 4 && tiles >= 6000u && covers(spread, 10.f), tile_size);
+    return pixels_that_fit(tiles >= (channels <= 8 ? 2700u : 1500u) && covers(spread, line) && many_entries(spread, entries, 800000, 15.f),
+                           channels <= 4 && tiles >= 6000u && covers(spread, 10.f) && many_entries(spread, entries, 1200000, INFINITY), tile_size);
 }
-static uint32_t pixels_per_lane_bwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread) {
+static uint32_t pixels_per_lane_bwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread, int64_t entries) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
     const float line = channels <= 4 && tiles >= 6000u ? 4.f : channels <= 8 ? 5.f : channels <= 16 ? 6.f : 7.f;
-    return pixels_that_fit(tiles >= 1500u && covers(spread, line), channels <= 4 && tiles >= 3000u && covers(spread, 9.f), tile_size);
+    return pixels_that_fit(tiles >= 1500u && covers(spread, line) && many_entries(spread, entries, 550000, 15.f),
+                           channels <= 4 && tiles >= 3000u && covers(spread, 9.f) && many_entries(spread, entries, 1100000, INFINITY), tile_size);
 }
 static bool pixels_bwd_other(uint64_t blocks, uint32_t tile_size, uint32_t channels, uint32_t px, float spread) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
@@ -2278,10 +2288,13 @@ static bool pixels_bwd_other(uint64_t blocks, uint32_t tile_size, uint32_t chann
 
 // One-shot hint of the calling thread's next camera compositing call.
 static thread_local float t_spread_hint = 0.f;
-static float take_spread_hint(uint32_t tile_size) {
-    const float spread = spread_of_16(t_spread_hint, tile_size);
+static thread_local int64_t t_entries_hint = 0;
+struct SplatHint { float spread; int64_t entries; };   // 0: not known
+static SplatHint take_spread_hint(uint32_t tile_size) {
+    const SplatHint hint = {spread_of_16(t_spread_hint, tile_size), t_entries_hint};
     t_spread_hint = 0.f;
-    return spread;
+    t_entries_hint = 0;
+    return hint;
 }
 
 // Whether all warps of a CTA share one patch in the forward pass: the shared work costs more instructions in all, so the
@@ -2333,8 +2346,9 @@ extern "C" int splatad_rasterize_set_rows_hint(uint64_t rows) {
     return SPLATAD_OK;
 }
 
-extern "C" int splatad_rasterize_set_spread_hint(float tiles_per_gaussian) {
+extern "C" int splatad_rasterize_set_spread_hint(float tiles_per_gaussian, int64_t n_isects) {
     t_spread_hint = tiles_per_gaussian;
+    t_entries_hint = n_isects;
     return SPLATAD_OK;
 }
 
@@ -2358,7 +2372,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     uint32_t image_height, uint32_t tile_size, uint32_t tile_width, uint32_t tile_height,
     const int32_t *tile_offsets, const int32_t *flatten_ids, int32_t expected_last_channel, float *render_colors,
     float *render_alphas, int32_t *last_ids, float *expected_depths, void *stream) {
-    const float spread = take_spread_hint(tile_size);
+    const SplatHint hint = take_spread_hint(tile_size);
     SPL_REQUIRE(channels >= 1 && channels <= SPLATAD_MAX_CHANNELS, SPLATAD_ERR_CHANNELS,
                 "rasterize_to_pixels_fwd: unsupported channel count %u (1..%d)", channels,
                 SPLATAD_MAX_CHANNELS);
@@ -2385,7 +2399,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     }
 #define CALL(D)                                                                                   \
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2)) else if (D <= 16 && px == 4) CALL_PX(D, (D <= 16 ? 4 : 2)) else CALL_PX(D, 2)
-    const uint32_t px = pixels_per_lane_fwd(blocks, tile_size, channels, spread);
+    const uint32_t px = pixels_per_lane_fwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool vec = channels % 4u == 0u && (reinterpret_cast<uintptr_t>(colors) & 15u) == 0u;
     {
         SPL_PROF("rasterize_to_pixels_fwd_kernel", (cudaStream_t)stream);
@@ -2421,7 +2435,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     const int32_t *last_ids, const float *v_render_colors, const float *v_render_alphas,
     float *v_means2d_abs, float *v_means2d, float *v_conics, float *v_colors, float *v_opacities,
     float *v_pix_vels, void *stream) {
-    const float spread = take_spread_hint(tile_size);
+    const SplatHint hint = take_spread_hint(tile_size);
     SPL_REQUIRE(channels >= 1 && channels <= SPLATAD_MAX_CHANNELS, SPLATAD_ERR_CHANNELS,
                 "rasterize_to_pixels_bwd: unsupported channel count %u (1..%d)", channels,
                 SPLATAD_MAX_CHANNELS);
@@ -2458,8 +2472,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2), A) else if (D <= 20 && px == 4) CALL_PX(D, (D <= 20 ? 4 : 2), A) else CALL_PX(D, 2, A)
 #define CALL(D)                                                                                   \
     if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)
-    const uint32_t px = pixels_per_lane_bwd(blocks, tile_size, channels, spread);
-    const bool other = pixels_bwd_other(blocks, tile_size, channels, px, spread);
+    const uint32_t px = pixels_per_lane_bwd(blocks, tile_size, channels, hint.spread, hint.entries);
+    const bool other = pixels_bwd_other(blocks, tile_size, channels, px, hint.spread);
     {
         SPL_PROF("rasterize_to_pixels_bwd_kernel", (cudaStream_t)stream);
         SPL_DISPATCH_CDIM(channels, CALL);

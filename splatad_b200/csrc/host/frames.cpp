@@ -691,7 +691,7 @@ struct CameraCompositeNode : torch::autograd::Function<CameraCompositeNode> {
         zeros.add(v_pix_vels, pix_vels.sizes());
         if (f->absgrad) zeros.add(v_abs, means2d.sizes());
         zeros.make(options);
-        lib.splatad_rasterize_set_spread_hint(f->spread);
+        lib.splatad_rasterize_set_spread_hint(f->spread, f->n_isects);
         check(lib.splatad_rasterize_expected_to_pixels_bwd(
             (uint32_t)f->C, f->n_isects, F(means2d), F(conics), F(colors), (uint32_t)f->channels, F(opacities), F(pix_vels), F(saved[5]),
             F(saved[6]), (uint32_t)f->W, (uint32_t)f->H, (uint32_t)f->tile_size, (uint32_t)f->tile_w, (uint32_t)f->tile_h, I(saved[9]),
@@ -712,7 +712,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
                         const OptTensor &lin, const OptTensor &ang, const OptTensor &rs, double near_plane, double far_plane,
                         double radius_clip, double eps2d, int64_t sh_degree, bool packed, int64_t tile_size, const OptTensor &backgrounds,
                         int64_t mode, bool expected, bool absgrad, bool antialiased, int64_t max_channels, int64_t row_capacity,
-                        int64_t capacity, uint64_t last_range, double last_spread) {
+                        int64_t capacity, uint64_t last_range, double last_spread, int64_t last_count) {
     if (!means.defined() || !means.is_cuda()) return py::none();
     const c10::DeviceIndex dev = means.get_device();
     for (const Tensor *t : {&means, &quats, &scales, &opacities, &colors, &viewmats, &Ks})
@@ -833,7 +833,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
         f->alphas = at::empty({C, H, W, 1}, options);
         f->last_ids = at::empty({C, H, W}, ints);
         if (expected && grad) f->expected_depths = at::empty({C, H, W}, options);
-        lib.splatad_rasterize_set_spread_hint((float)last_spread);
+        lib.splatad_rasterize_set_spread_hint((float)last_spread, last_count);
         check(lib.splatad_rasterize_expected_to_pixels_fwd(
             (uint32_t)C, -1, F(f->means2d), F(f->conics), c, (uint32_t)channels, o, F(f->pix_vels), F(rs_t), F(bg), (uint32_t)W, (uint32_t)H,
             (uint32_t)tile_size, (uint32_t)tile_w, (uint32_t)tile_h, I(f->offsets), I(f->flatten_ids), expected, M(f->render), M(f->alphas),

@@ -1046,7 +1046,7 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
     counted = torch.cuda.Event()
     counted.record(torch.cuda.current_stream(dev))
     isect_buf, flat_buf, offsets = fill(capacity)
-    flat_buf._splatad_spread = _spread_hint.get(key, 0.0)
+    flat_buf._splatad_spread, flat_buf._splatad_count = _spread_hint.get(key, 0.0), hint
     return DeferredIsect(tiles_per_gauss, isect_buf, flat_buf, offsets, C, n_tiles_total, capacity,
                          counted, lambda: read_count(slot, sequence, counted), exact)
 
@@ -1419,7 +1419,8 @@ def rasterize_to_pixels(
     args = (conics.contiguous(), opacities.contiguous(), pix_vels.contiguous(),
             rolling_shutter_time.contiguous())
     # how many tiles a listed Gaussian covers, where the lists' maker has left it; chooses the split of the work
-    spread = getattr(flatten_ids, "_splatad_spread", 0.0)
+    spread = (getattr(flatten_ids, "_splatad_spread", 0.0),
+              getattr(flatten_ids, "_splatad_count", 0 if total_follows else flatten_ids.numel()))
     tail = (image_width, image_height, tile_size, isect_offsets.contiguous(), flatten_ids.contiguous(),
             absgrad, total_follows, spread)
     if channels <= _lib.MAX_CHANNELS:
@@ -1440,7 +1441,7 @@ def rasterize_to_pixels(
 class _RasterizeToPixels(torch.autograd.Function):
     @staticmethod
     def forward(ctx, means2d, conics, colors, opacities, pix_vels, rolling_shutter_time, backgrounds,
-                width, height, tile_size, isect_offsets, flatten_ids, absgrad, total_follows=False, spread=0.0):
+                width, height, tile_size, isect_offsets, flatten_ids, absgrad, total_follows=False, spread=(0.0, 0)):
         dev = means2d.device
         assert means2d.dtype == torch.float32, means2d.dtype
         C, tile_h, tile_w = isect_offsets.shape
@@ -1454,7 +1455,7 @@ class _RasterizeToPixels(torch.autograd.Function):
         n_isects = _n_isects_arg(isect_offsets, flatten_ids, total_follows)
         _debug_check_lists("rasterize_to_pixels", flatten_ids, means2d.numel() // 2, isect_offsets, total_follows)
         ctx.n_isects_arg, ctx.spread = n_isects, spread
-        _lib.load().splatad_rasterize_set_spread_hint(spread)
+        _lib.load().splatad_rasterize_set_spread_hint(*spread)
         _call(
             "splatad_rasterize_to_pixels_fwd", C, n_isects, _lib.ptr(means2d), _lib.ptr(conics_f),
             _lib.ptr(colors_f), channels, _lib.ptr(opac_f), _lib.ptr(vels_f), _lib.ptr(rs), _lib.ptr(bg),
@@ -1477,7 +1478,7 @@ class _RasterizeToPixels(torch.autograd.Function):
         v_render_alphas = _f(v_render_alphas)
         v_means2d, v_conics, v_colors, v_opacities, v_pix_vels, v_abs = _zeros_like_many(
             means2d, conics, colors, opacities, pix_vels, means2d if ctx.absgrad else None)
-        _lib.load().splatad_rasterize_set_spread_hint(ctx.spread)
+        _lib.load().splatad_rasterize_set_spread_hint(*ctx.spread)
         _call(
             "splatad_rasterize_to_pixels_bwd", C, ctx.n_isects_arg, _lib.ptr(means2d),
             _lib.ptr(conics), _lib.ptr(colors), channels, _lib.ptr(opacities), _lib.ptr(pix_vels),

@@ -458,8 +458,8 @@ def test_pixels_by_how_many_tiles_a_gaussian_covers(C, ts, channels, absgrad):
                                             absgrad=absgrad)
     offsets, ids = t(c["offsets"], torch.int32), t(c["flatten_ids"], torch.int32)
     first = None
-    for spread in (0.0, 2.0, 4.5, 6.5, 8.0, 20.0):
-        ids._splatad_spread = spread
+    for spread, count in ((0.0, 0), (2.0, 10**7), (4.5, 10**7), (6.5, 10**7), (8.0, 10**7), (12.0, 700_000), (12.0, 10**5), (20.0, 10**7)):
+        ids._splatad_spread, ids._splatad_count = spread, count
         leaves = {k: t(c[k]).requires_grad_(True) for k in keys}
         out_c, out_a = ops.rasterize_to_pixels(*(leaves[k] for k in keys), W, H, ts, offsets, ids, t(c["rs"]), backgrounds=t(bg),
                                                absgrad=absgrad)
@@ -501,12 +501,12 @@ def test_divided_depth_of_many_tiles(C, channels):
         last, depths = torch.empty(C, H, W, dtype=torch.int32, device=DEV), torch.empty(C, H, W, device=DEV)
         head = (C, ids.numel(), p(dev["means2d"]), p(dev["conics"]), p(dev["colors"]), channels, p(dev["opacities"]), p(dev["pix_vels"]),
                 p(rs), p(bg), W, H, ts, tw, th, p(offsets), p(ids))
-        lib.splatad_rasterize_set_spread_hint(spread)
+        lib.splatad_rasterize_set_spread_hint(spread, 10**7)
         _lib.call("splatad_rasterize_expected_to_pixels_fwd", *head, 1, p(image), p(alphas), p(last), p(depths), _lib.stream_ptr(ids.device))
         assert_close(f"depth ch={channels} spread {spread}", n(image), n(want), 1e-6, 1e-7)
         assert torch.equal(alphas, out_a) and torch.equal(depths, image[..., -1])
         v = [torch.zeros_like(dev[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")]
-        lib.splatad_rasterize_set_spread_hint(spread)
+        lib.splatad_rasterize_set_spread_hint(spread, 10**7)
         _lib.call("splatad_rasterize_expected_to_pixels_bwd", *head, p(depths), p(alphas), p(last), p(v_c), p(v_a), None, *(p(x) for x in v),
                   _lib.stream_ptr(ids.device))
         for k, got in zip(keys, v):
