@@ -263,7 +263,7 @@ bool usable(const Counts &c, int64_t capacity) {
 // the depth range of an earlier frame (word of the early count; 0: none), buckets that span it widened by a
 // tenth on either side - the rectangle count then fills them and one kernel less is launched.
 struct PlanRequests {
-    PlanRequests(const Slot &slot, int64_t sequence, uint64_t last_range) {
+    PlanRequests(const Slot &slot, int64_t sequence, uint64_t last_range, bool listed) {
         if (last_range != 0) {
             const uint32_t bits[2] = {(uint32_t)last_range, (uint32_t)(last_range >> 32)};
             float lo, hi;
@@ -281,7 +281,7 @@ struct PlanRequests {
         }
         slot.word[9] = 0;
         lib.splatad_isect_set_early_count(const_cast<int64_t *>(slot.word) + 4, sequence);
-        lib.splatad_isect_set_listed_count(const_cast<int64_t *>(slot.word) + 9);
+        if (listed) lib.splatad_isect_set_listed_count(const_cast<int64_t *>(slot.word) + 9);
     }
     ~PlanRequests() {
         lib.splatad_isect_set_early_count(nullptr, 0);
@@ -484,7 +484,7 @@ py::object lidar_frame(const Tensor &means, const Tensor &quats, const Tensor &s
         const Tensor fill_ws = workspace("isect_fill", lib.splatad_isect_fill_workspace_bytes((uint64_t)capacity), stream);
         Slot slot(stream);
         const int64_t sequence = next_sequence();
-        const PlanRequests requests(slot, sequence, last_range);
+        const PlanRequests requests(slot, sequence, last_range, false);   // (asking costs the host a call)
         const auto opacity_rows = [&]() -> const float * {
             if (!f->opacities.defined()) return F(opacities);
             check(lib.splatad_opacity_rows_fwd((uint32_t)(C * N), (uint32_t)N, nullptr, F(opacities), F(f->comps), M(f->opacities),
@@ -802,7 +802,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
                       (uint32_t)tile_size, (uint32_t)tile_w, (uint32_t)tile_h, 1, I(f->tiles_per_gauss), tail...);
         };
         {
-            const PlanRequests requests(slot, sequence, last_range);
+            const PlanRequests requests(slot, sequence, last_range, true);
             check(grid(lib.splatad_isect_tiles_plan, plan_ws.data_ptr(), (size_t)plan_ws.numel(), (int64_t *)nullptr, stream.stream()));
         }
         check(grid(lib.splatad_isect_tiles_fill, plan_ws.data_ptr(), fill_ws.data_ptr(), (size_t)fill_ws.numel(), capacity,
