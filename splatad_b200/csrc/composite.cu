@@ -135,16 +135,18 @@ __device__ __forceinline__ PixelEntry load_pixel_entry(int32_t g, const float2 *
     return e;
 }
 
-constexpr uint32_t kSeenEntry = 1u, kCarefulEntry = 2u, kOddEntry = 4u;
+constexpr uint32_t kSeenEntry = 1u, kCarefulEntry = 2u, kOddEntry = 4u, kFullEntry = 8u;
 
 // What a warp has to know about an entry: whether it can reach the warp's patch (kSeenEntry; 0: it need not look at it),
 // whether its alphas need looking at one by one (kCarefulEntry: a sigma that could come out negative, an alpha above the
 // cap), and whether it is one for odd_pixels_fwd() (kOddEntry). The alphas of the others need no test but the one
 // against 1/255: with ac - b^2 >= 1e-5 ac the form a dx^2 + 2 b dx dy + c dy^2 is at least 5e-6 (a dx^2 + c dy^2), ten times
-// what its rounding can take away, and an opacity within the cap keeps every alpha there. The mean moves with the
-// row's shutter time; roll_lo / roll_hi bound it over the tile.
-template <bool kMarkOdd>
-__device__ __forceinline__ uint32_t patch_sees(const PixelEntry &e, const PatchBox &box, float roll_lo, float roll_hi) {
+// what its rounding can take away, and an opacity within the cap keeps every alpha there. Not even that one where every pixel
+// of the patch blends the entry (kFullEntry): sigma is convex, so that the corners of the box bound it from above, and with
+// ac - b^2 >= 0.05 ac its terms are at most forty times itself, which leaves their rounding a tenth of the margin. `most` bounds the
+// alphas in the patch, by the least sigma where that holds, else by the opacity. (kBounds: the last two.) The mean moves with the row's shutter time; roll_lo / roll_hi bound it over the tile.
+template <bool kMarkOdd, bool kBounds>
+__device__ __forceinline__ uint32_t patch_sees(const PixelEntry &e, const PatchBox &box, float roll_lo, float roll_hi, float &most) {
     const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
     if (test.never) return 0u;
     const float mx_a = e.A.x + roll_lo * e.A.z, mx_b = e.A.x + roll_hi * e.A.z;
@@ -156,12 +158,22 @@ __device__ __forceinline__ uint32_t patch_sees(const PixelEntry &e, const PatchB
         const bool plain = fabsf(e.B.x) > 1e-30f && fabsf(e.B.x) + fabsf(e.B.y) + fabsf(e.B.z) < 1e30f;
         if (!plain || !(mx_lo <= mx_hi) || !(my_lo <= my_hi) || !(test.s_max < 1e30f)) seen = kOddEntry;
     }
-    const float ac = e.B.x * e.B.z;
+    const float ac = e.B.x * e.B.z, det = ac - e.B.y * e.B.y;
     const bool sized = e.B.x > 1e-15f && e.B.z > 1e-15f && e.B.x < 1e15f && e.B.z < 1e15f;   // nothing under- or overflows
-    if (!(sized && ac - e.B.y * e.B.y >= 1e-5f * ac && e.B.w <= kAlphaMax)) seen |= kCarefulEntry;
-    if (box.x0 <= box.x1 && !test.misses(mx_lo - box.x1, mx_hi - box.x0, my_lo - box.y1, my_hi - box.y0)) seen |= kSeenEntry;
-    else seen &= kOddEntry;
-    return seen;
+    if (!(sized && det >= 1e-5f * ac && e.B.w <= kAlphaMax)) seen |= kCarefulEntry;
+    const float x0 = mx_lo - box.x1, x1 = mx_hi - box.x0, y0 = my_lo - box.y1, y1 = my_hi - box.y0;
+    if (!kBounds) {
+        if (box.x0 <= box.x1 && !test.misses(x0, x1, y0, y1)) seen |= kSeenEntry;
+        else seen &= kOddEntry;
+        return seen;
+    }
+    const float lowest = BoxTest::with_margin(test.lowest(x0, x1, y0, y1));
+    if (!(box.x0 <= box.x1) || lowest > test.s_max) return seen & kOddEntry;
+    most = fminf(kAlphaMax, det >= 0.05f * ac ? e.B.w * __expf(-lowest) : e.B.w);
+    const float xx = 0.5f * e.B.x * fmaxf(x0 * x0, x1 * x1), yy = 0.5f * e.B.z * fmaxf(y0 * y0, y1 * y1);
+    const float xy = fmaxf(fmaxf(e.B.y * x0 * y0, e.B.y * x0 * y1), fmaxf(e.B.y * x1 * y0, e.B.y * x1 * y1));
+    if (seen == 0u && det >= 0.05f * ac && xx + yy + xy <= __logf(255.f * e.B.w) * 0.999f - 4e-3f) seen = kFullEntry;
+    return seen | kSeenEntry;
 }
 
 // The staged form: exp(-sigma) = 2^(a dx^2 + b dx dy + c dy^2) with the conic scaled once per entry.
@@ -173,6 +185,19 @@ __device__ __forceinline__ float exp2_approx(float x) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
+}
+
+__device__ __forceinline__ float lg2_approx(float x) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The lane of a one-warp block, in a register that stays: read from its special register inside a loop it takes twenty cycles.
+__device__ __forceinline__ uint32_t lane_index() {
+    uint32_t lane;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(lane));
+    return lane;
 }
 
 // exponents of a pair of pixels in one row: dx of the two, the row's b * dy and c * dy * dy
@@ -527,16 +552,28 @@ __device__ __forceinline__ void store_channels(float *dst, const float (&v)[PX][
 // ---------------------------------------------------------------------------------------
 constexpr float kPixelGone = 1e18f;   // a column no Gaussian reaches: sigma overflows, alpha is 0 (or NaN, never drawn)
 
-// registers per thread, by measurement (4 channels, eight pixels: 147 us at 128 registers, 163 at 112 and 96; 8 channels, four
+// log2 of 1.01 kTStop: where the bound of the transmittances comes that low they are looked at (the sums are off by 1e-4 at most)
+constexpr float kLowBound = -13.2733571f;
+
+// registers per thread, by measurement (4 channels, eight pixels: 147 us at 128 registers, 163 at 112 and 96, with runs 130 at 96 (20 warps an SM), 145
+// at 104 to 128 (16), 135 at 80 (24, spills); 8 channels, four
 // pixels: 218 at 96, 243 at 112 and 128; 20 channels: 426 at 96, 445 at 112 and 160)
-constexpr int pixels_fwd_regs(int cdim, int px) {
-    return cdim <= 4 ? (px == 8 ? 128 : px == 4 ? 80 : 64) : cdim <= 8 ? (px == 4 ? 96 : 72) : cdim <= 16 ? (px == 4 ? 128 : 96) : cdim <= 20 ? 96 : 128;
+constexpr int pixels_fwd_regs(int cdim, int px, bool runs) {
+    return runs ? 96 : cdim <= 4 ? (px == 8 ? 128 : px == 4 ? 80 : 64) : cdim <= 8 ? (px == 4 ? 96 : 72) : cdim <= 16 ? (px == 4 ? 128 : 96) : cdim <= 20 ? 96 : 128;
 }
 
+// kRuns: for scenes of large Gaussians, where most entries that are looked at cover their patch (84 % in the camera benchmark, 98 % in
+// its rigs). Those go through in runs that test nothing: every pixel blends them, the last of a run is noted once a batch, and no
+// transmittance can come below the limit before a bound of them all does - the sum of the entries' least logarithms, one scan a
+// batch -, which it reaches with one entry in 15 to 45. Such an entry, one that does not cover the patch and one that needs care are
+// looked at one by one. What bounds it then is the FP32 pipe, at 75 % of its rate within a run, and the batches. 1920 x 1080, 27 tiles per
+// Gaussian 104 M -> 82 M warp instructions, 145 -> 130 us, 54 tiles 119 -> 95, six cameras 584 -> 445. Where few entries cover their patch it
+// is slower by up to half: see covers_patches(). (Entries two by two: 144 us, for the registers; the next batch's entries loaded ahead: no change.)
+//
 // kTogether: rows in 16-byte pieces, staged by copy_rows(). A kernel of its own: with both ways in one, 1920 x 1080 and 32 channels
 // take 648 us instead of 506.
-template <int CDIM, int PX, bool kTogether>
-__global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX)) rasterize_to_pixels_fwd_kernel(
+template <int CDIM, int PX, bool kTogether, bool kRuns>
+__global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX, kRuns)) rasterize_to_pixels_fwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
     const float *__restrict__ opacities, const float2 *__restrict__ pix_vels,
@@ -558,7 +595,9 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX)) rasterize_to_pixels_fwd_k
     const uint32_t gtile = blockIdx.x / patches, cam = gtile / tiles_per_cam;
     const uint32_t tile = gtile - cam * tiles_per_cam;
     const uint32_t ty = tile / tile_w, tx = tile - ty * tile_w;
-    const uint32_t lane = threadIdx.x, tr = (blockIdx.x - gtile * patches) * 32u + lane;
+    uint32_t lane = threadIdx.x;
+    if constexpr (kRuns) lane = lane_index();
+    const uint32_t tr = (blockIdx.x - gtile * patches) * 32u + lane;
     const TilePixels<PX> tp = tile_pixels<PX>(tile_size, tr);
     const uint32_t i = ty * tile_size + tp.y, j = tx * tile_size + tp.x;
     uint32_t n_inside = 0;   // pixels of this thread inside the tile and the image
@@ -575,7 +614,6 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX)) rasterize_to_pixels_fwd_k
     const TileRange range = tile_range(offsets, gtile, C * tiles_per_cam, n_isects);
 
     float2 npx[P2], T[P2], out[CDIM][P2];   // minus the columns; transmittances; minus the colours, by channel
-    uint32_t blended[PX];                   // entries of the batch, one bit each
     int32_t pos[PX];                        // list position of the last entry blended
 #pragma unroll
     for (int q = 0; q < P2; ++q) {
@@ -594,87 +632,259 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX)) rasterize_to_pixels_fwd_k
 
     int32_t next_id = 0;
     if (range.start + (int32_t)lane < range.end) next_id = flatten_ids[range.start + lane];
-    for (int32_t start = range.start; start < range.end && !done; start += 32) {
-        const int32_t idx = start + (int32_t)lane;
-        const int32_t g = next_id;
-        uint32_t seen = 0u;
-        PixelEntry e;
-        if (idx < range.end) {
-            e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
-            if (idx + 32 < range.end) next_id = flatten_ids[idx + 32];   // on its way meanwhile
-            seen = patch_sees<true>(e, box, roll_lo, roll_hi);
-        }
-        uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
-        const uint32_t careful = __ballot_sync(0xffffffffu, seen > kSeenEntry);
-        odd |= seen;
-        __syncwarp();   // the batch before has been read
-        if (seen) {
-            sA[lane] = e.A;
-            sB[lane] = scaled_conic(make_float4(e.B.x, e.B.y, e.B.z, -e.B.w));
-            if (!kTogether) stage_whole_row<CDIM>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, CDIM < 20 && vec);
-        }
-        if (kTogether) stage_rows<CDIM>(reinterpret_cast<float *>(sCol), colors, g, todo, channels, lane);
-        __syncwarp();
+    if constexpr (kRuns) {
+        float bound = 0.f;   // log2 of a transmittance that no pixel that still blends is below, the same in every lane
+        constexpr int kEntry = 2 + CDIM / 4;
+        __shared__ float4 sEntry[32 * kEntry];   // x, y, vx, vy | scaled conic, minus the opacity | channels, zeros behind them
+        __shared__ float sT[PX][32];        // transmittances of the pixels that have stopped
+        __shared__ int32_t sLast[PX][32];   // list positions of the last entries blended
+        __shared__ int32_t sIdx[32];        // list positions
+        int32_t *sl = &sLast[0][lane];      // 32 apart for the lane's pixels
 #pragma unroll
-        for (int k = 0; k < PX; ++k) blended[k] = 0u;
-        while (todo) {
-            const uint32_t t = (uint32_t)__ffs(todo) - 1u, bit = 1u << t;
-            todo ^= bit;
-            const float4 A = sA[t], B = sB[t];
-            const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
-            const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
-            float2 w[P2];   // minus the alphas, then minus the weights
-#pragma unroll
-            for (int q = 0; q < P2; ++q) {
-                const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
-                w[q] = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
+        for (int k = 0; k < PX; ++k) sl[32 * k] = 0;
+        for (int32_t start = range.start; start < range.end && !done; start += 32) {
+            const int32_t idx = start + (int32_t)lane;
+            const int32_t g = next_id;
+            uint32_t seen = 0u;
+            float most = 0.f;
+            PixelEntry e;
+            if (idx < range.end) {
+                e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
+                if (idx + 32 < range.end) next_id = flatten_ids[idx + 32];   // on its way meanwhile
+                seen = patch_sees<true, true>(e, box, roll_lo, roll_hi, most);
             }
-            if (careful & bit) {
+            // The entries to be looked at move up to the front; n of them, bit t of the masks for the one in place t
+            const uint32_t kept = __ballot_sync(0xffffffffu, seen != 0u), n = __popc(kept);
+            const uint32_t place = __popc(kept & ((1u << lane) - 1u));
+            const uint32_t full = __reduce_or_sync(0xffffffffu, (seen & kFullEntry) ? 1u << place : 0u);
+            const uint32_t careful = __reduce_or_sync(0xffffffffu, (seen & (kCarefulEntry | kOddEntry)) ? 1u << place : 0u);
+            odd |= seen & kOddEntry;
+            // what the entries up to this lane's leave of a transmittance, at least
+            float left = seen ? lg2_approx(1.f - most) : 0.f;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const float o = __shfl_up_sync(0xffffffffu, left, off);
+                if ((int)lane >= off) left += o;
+            }
+            __syncwarp();   // the batch before has been read
+            if (seen) {
+                float4 *entry = sEntry + place * kEntry;
+                entry[0] = e.A;
+                entry[1] = scaled_conic(make_float4(e.B.x, e.B.y, e.B.z, -e.B.w));
+                sIdx[place] = idx;
+                stage_whole_row<CDIM>(entry + 2, colors + (size_t)g * channels, channels, CDIM < 20 && vec);
+            }
+            __syncwarp();
+            // minus the alphas of entry t
+            const auto evaluate = [&](uint32_t t, float2 (&w)[P2]) {
+                const float4 A = sEntry[t * kEntry], B = sEntry[t * kEntry + 1];
+                const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
+                const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
 #pragma unroll
                 for (int q = 0; q < P2; ++q) {
                     const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
-                    w[q].x = pw.x <= 0.f ? fmaxf(-kAlphaMax, w[q].x) : 0.f;
-                    w[q].y = pw.y <= 0.f ? fmaxf(-kAlphaMax, w[q].y) : 0.f;
+                    w[q] = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
                 }
-            }
-            float low = 1.f;
+            };
+            const auto drop_small = [&](float2 (&w)[P2]) {
 #pragma unroll
-            for (int q = 0; q < P2; ++q) {
-                const bool ok0 = w[q].x <= -kAlphaMin, ok1 = w[q].y <= -kAlphaMin;
-                if (ok0) blended[2 * q] |= bit;
-                if (ok1) blended[2 * q + 1] |= bit;
-                const float2 alpha = make_float2(ok0 ? w[q].x : 0.f, ok1 ? w[q].y : 0.f);
-                w[q] = __fmul2_rn(alpha, T[q]);
-                T[q] = __ffma2_rn(alpha, T[q], T[q]);
-                low = fminf(low, fminf(T[q].x, T[q].y));
-            }
-            // T stays above the limit, so only a blended entry can take a pixel below it; few entries do
-            if (__any_sync(0xffffffffu, low <= kTStop)) {
-                bool gone = true;
+                for (int q = 0; q < P2; ++q) w[q] = make_float2(w[q].x <= -kAlphaMin ? w[q].x : 0.f, w[q].y <= -kAlphaMin ? w[q].y : 0.f);
+            };
+            const auto pass = [&](float2 (&w)[P2]) {   // to minus the weights
 #pragma unroll
                 for (int q = 0; q < P2; ++q) {
-                    if (T[q].x <= kTStop) { npx[q].x = -kPixelGone; T[q].x -= w[q].x; w[q].x = 0.f; blended[2 * q] &= ~bit; }
-                    if (T[q].y <= kTStop) { npx[q].y = -kPixelGone; T[q].y -= w[q].y; w[q].y = 0.f; blended[2 * q + 1] &= ~bit; }
-                    gone = gone && npx[q].x == -kPixelGone && npx[q].y == -kPixelGone;
+                    const float2 alpha = w[q];
+                    w[q] = __fmul2_rn(alpha, T[q]);
+                    T[q] = __ffma2_rn(alpha, T[q], T[q]);
                 }
-                done = __all_sync(0xffffffffu, gone);
-                if (done) todo = 0u;
-            }
+            };
+            const auto blend = [&](uint32_t t, const float2 (&w)[P2]) {
 #pragma unroll
-            for (int c = 0; c < CDIM; c += 4) {
-                const float4 c4 = sCol[t * (CDIM / 4) + c / 4];
+                for (int c = 0; c < CDIM; c += 4) {
+                    const float4 c4 = sEntry[t * kEntry + 2 + c / 4];
 #pragma unroll
-                for (int q = 0; q < P2; ++q) {
-                    out[c][q] = __ffma2_rn(make_float2(c4.x, c4.x), w[q], out[c][q]);
-                    out[c + 1][q] = __ffma2_rn(make_float2(c4.y, c4.y), w[q], out[c + 1][q]);
-                    out[c + 2][q] = __ffma2_rn(make_float2(c4.z, c4.z), w[q], out[c + 2][q]);
-                    out[c + 3][q] = __ffma2_rn(make_float2(c4.w, c4.w), w[q], out[c + 3][q]);
+                    for (int q = 0; q < P2; ++q) {
+                        out[c][q] = __ffma2_rn(make_float2(c4.x, c4.x), w[q], out[c][q]);
+                        out[c + 1][q] = __ffma2_rn(make_float2(c4.y, c4.y), w[q], out[c + 1][q]);
+                        out[c + 2][q] = __ffma2_rn(make_float2(c4.z, c4.z), w[q], out[c + 2][q]);
+                        out[c + 3][q] = __ffma2_rn(make_float2(c4.w, c4.w), w[q], out[c + 3][q]);
+                    }
                 }
+            };
+            const auto note = [&](uint32_t t, const float2 (&w)[P2]) {
+                const int32_t at = sIdx[t];
+#pragma unroll
+                for (int k = 0; k < PX; ++k)
+                    if ((k & 1 ? w[k / 2].y : w[k / 2].x) != 0.f) sl[32 * k] = at;
+            };
+            // the last of some full entries, as the last one blended of pixel k
+            const auto note_full = [&](int k, uint32_t entries) {
+                if (entries) sl[32 * k] = max(sl[32 * k], sIdx[31 - __clz(entries)]);
+            };
+            float passed = 0.f;   // log2 of what the entries before t leave
+            for (uint32_t t = 0; t < n;) {
+                // T stays above the limit, so only a blended entry can take a pixel below it: the first that might, by the bound
+                const uint32_t below = __ballot_sync(0xffffffffu, seen && place >= t && bound + (left - passed) <= kLowBound);
+                const uint32_t cross = below ? __popc(kept & ((below & (0u - below)) - 1u)) : n;
+                const uint32_t stop = min(cross, (careful >> t) ? t + (uint32_t)__ffs(careful >> t) - 1u : n);
+                while (t < stop) {
+                    const uint32_t rest = ~full >> t, end = min(stop, rest ? t + (uint32_t)__ffs(rest) - 1u : n);
+#pragma unroll 2
+                    for (; t < end; ++t) {
+                        float2 w[P2];
+                        evaluate(t, w);
+                        pass(w);
+                        blend(t, w);
+                    }
+                    if (t >= stop) break;
+                    float2 w[P2];
+                    evaluate(t, w);
+                    drop_small(w);
+                    pass(w);
+                    note(t, w);
+                    blend(t, w);
+                    ++t;
+                }
+                if (t >= n) break;
+                float2 w[P2];
+                evaluate(t, w);
+                if ((careful >> t) & 1u) {
+                    const float4 A = sEntry[t * kEntry], B = sEntry[t * kEntry + 1];
+                    const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
+                    const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
+#pragma unroll
+                    for (int q = 0; q < P2; ++q) {
+                        const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
+                        w[q].x = pw.x <= 0.f ? fmaxf(-kAlphaMax, w[q].x) : 0.f;
+                        w[q].y = pw.y <= 0.f ? fmaxf(-kAlphaMax, w[q].y) : 0.f;
+                    }
+                }
+                drop_small(w);
+                pass(w);
+                float low = 1.f;
+#pragma unroll
+                for (int q = 0; q < P2; ++q) low = fminf(low, fminf(T[q].x, T[q].y));
+                low = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(low)));
+                if (low <= kTStop) {
+                    bool gone = true;
+#pragma unroll
+                    for (int k = 0; k < PX; ++k) {
+                        float &Tk = k & 1 ? T[k / 2].y : T[k / 2].x, &wk = k & 1 ? w[k / 2].y : w[k / 2].x, &column = k & 1 ? npx[k / 2].y : npx[k / 2].x;
+                        if (Tk <= kTStop) {
+                            sT[k][lane] = Tk - wk;
+                            Tk = 1.f;
+                            wk = 0.f;
+                            column = -kPixelGone;
+                            note_full(k, full & ((1u << t) - 1u));
+                        }
+                        gone = gone && column == -kPixelGone;
+                    }
+                    done = __all_sync(0xffffffffu, gone);
+                }
+                note(t, w);
+                blend(t, w);
+                if (done) break;
+                bound = lg2_approx(low);
+                passed = __shfl_sync(0xffffffffu, left, __ffs(__ballot_sync(0xffffffffu, seen && place == t)) - 1);
+                ++t;
             }
+            bound += __shfl_sync(0xffffffffu, left, 31) - passed;
+            if (full && !done)
+#pragma unroll
+                for (int k = 0; k < PX; ++k)
+                    if ((k & 1 ? npx[k / 2].y : npx[k / 2].x) != -kPixelGone) note_full(k, full);
         }
 #pragma unroll
-        for (int k = 0; k < PX; ++k)
-            if (blended[k]) pos[k] = start + 31 - __clz(blended[k]);
+        for (int k = 0; k < PX; ++k) {   // pixels outside the image are gone without having drawn anything
+            pos[k] = sl[32 * k];
+            float &Tk = k & 1 ? T[k / 2].y : T[k / 2].x;
+            if ((k & 1 ? npx[k / 2].y : npx[k / 2].x) == -kPixelGone && n_inside > (uint32_t)k) Tk = sT[k][lane];
+        }
+    } else {
+        for (int32_t start = range.start; start < range.end && !done; start += 32) {
+            const int32_t idx = start + (int32_t)lane;
+            const int32_t g = next_id;
+            uint32_t seen = 0u;
+            PixelEntry e;
+            if (idx < range.end) {
+                e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
+                if (idx + 32 < range.end) next_id = flatten_ids[idx + 32];   // on its way meanwhile
+                float most;
+                seen = patch_sees<true, false>(e, box, roll_lo, roll_hi, most);
+            }
+            uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
+            const uint32_t careful = __ballot_sync(0xffffffffu, seen > kSeenEntry);
+            odd |= seen;
+            __syncwarp();   // the batch before has been read
+            if (seen) {
+                sA[lane] = e.A;
+                sB[lane] = scaled_conic(make_float4(e.B.x, e.B.y, e.B.z, -e.B.w));
+                if (!kTogether) stage_whole_row<CDIM>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, CDIM < 20 && vec);
+            }
+            if (kTogether) stage_rows<CDIM>(reinterpret_cast<float *>(sCol), colors, g, todo, channels, lane);
+            __syncwarp();
+            uint32_t blended[PX];   // entries of the batch, one bit each
+#pragma unroll
+            for (int k = 0; k < PX; ++k) blended[k] = 0u;
+            while (todo) {
+                const uint32_t t = (uint32_t)__ffs(todo) - 1u, bit = 1u << t;
+                todo ^= bit;
+                const float4 A = sA[t], B = sB[t];
+                const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
+                const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
+                float2 w[P2];   // minus the alphas, then minus the weights
+#pragma unroll
+                for (int q = 0; q < P2; ++q) {
+                    const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
+                    w[q] = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
+                }
+                if (careful & bit) {
+#pragma unroll
+                    for (int q = 0; q < P2; ++q) {
+                        const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
+                        w[q].x = pw.x <= 0.f ? fmaxf(-kAlphaMax, w[q].x) : 0.f;
+                        w[q].y = pw.y <= 0.f ? fmaxf(-kAlphaMax, w[q].y) : 0.f;
+                    }
+                }
+                float low = 1.f;
+#pragma unroll
+                for (int q = 0; q < P2; ++q) {
+                    const bool ok0 = w[q].x <= -kAlphaMin, ok1 = w[q].y <= -kAlphaMin;
+                    if (ok0) blended[2 * q] |= bit;
+                    if (ok1) blended[2 * q + 1] |= bit;
+                    const float2 alpha = make_float2(ok0 ? w[q].x : 0.f, ok1 ? w[q].y : 0.f);
+                    w[q] = __fmul2_rn(alpha, T[q]);
+                    T[q] = __ffma2_rn(alpha, T[q], T[q]);
+                    low = fminf(low, fminf(T[q].x, T[q].y));
+                }
+                // T stays above the limit, so only a blended entry can take a pixel below it; few entries do
+                if (__any_sync(0xffffffffu, low <= kTStop)) {
+                    bool gone = true;
+#pragma unroll
+                    for (int q = 0; q < P2; ++q) {
+                        if (T[q].x <= kTStop) { npx[q].x = -kPixelGone; T[q].x -= w[q].x; w[q].x = 0.f; blended[2 * q] &= ~bit; }
+                        if (T[q].y <= kTStop) { npx[q].y = -kPixelGone; T[q].y -= w[q].y; w[q].y = 0.f; blended[2 * q + 1] &= ~bit; }
+                        gone = gone && npx[q].x == -kPixelGone && npx[q].y == -kPixelGone;
+                    }
+                    done = __all_sync(0xffffffffu, gone);
+                    if (done) todo = 0u;
+                }
+#pragma unroll
+                for (int c = 0; c < CDIM; c += 4) {
+                    const float4 c4 = sCol[t * (CDIM / 4) + c / 4];
+#pragma unroll
+                    for (int q = 0; q < P2; ++q) {
+                        out[c][q] = __ffma2_rn(make_float2(c4.x, c4.x), w[q], out[c][q]);
+                        out[c + 1][q] = __ffma2_rn(make_float2(c4.y, c4.y), w[q], out[c + 1][q]);
+                        out[c + 2][q] = __ffma2_rn(make_float2(c4.z, c4.z), w[q], out[c + 2][q]);
+                        out[c + 3][q] = __ffma2_rn(make_float2(c4.w, c4.w), w[q], out[c + 3][q]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < PX; ++k)
+                if (blended[k]) pos[k] = start + 31 - __clz(blended[k]);
+        }
     }
     const float *bg = backgrounds ? backgrounds + (size_t)cam * channels : nullptr;
     const size_t pix = ((size_t)cam * H + i) * W + j;
@@ -1596,14 +1806,15 @@ rasterize_to_pixels_bwd_kernel(
         const int32_t idx = batch_end - (int32_t)lane;
         const int32_t g = next_id;
         uint32_t seen = 0u;
+        float most;
         PixelEntry e;
         if (idx >= range.start) {
             e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
             if (idx - 32 >= range.start) next_id = flatten_ids[idx - 32];   // on its way meanwhile
-            seen = patch_sees<false>(e, box, roll_lo, roll_hi);
+            seen = patch_sees<false, false>(e, box, roll_lo, roll_hi, most);
         }
         uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
-        const uint32_t careful = __ballot_sync(0xffffffffu, seen > kSeenEntry);
+        const uint32_t careful = __ballot_sync(0xffffffffu, (seen & kCarefulEntry) != 0u);
         __syncwarp();   // the batch before has been read
         if (seen) {
             sA[lane] = e.A;
@@ -2268,6 +2479,18 @@ static uint32_t pixels_that_fit(bool four, bool eight, uint32_t tile_size) {
 static bool many_entries(float spread, int64_t entries, int64_t line, float or_spread) {
     return !(spread > 0.f) || entries <= 0 || entries >= line || spread >= or_spread;
 }
+// Whether most entries that the forward kernel looks at cover their patches, so that eight pixels per lane with runs pay (up to four channels): the
+// nearest Gaussians are the ones that count, and they are larger the more tiles the mean one covers and the more of them
+// a tile's list holds. By the product of the two; us, with runs against the better of four and eight pixels without: 8160 tiles, 28 tiles per Gaussian and 74
+// entries per tile (2 k) 117 and 87, 27 and 143 (4 k) 136 and 113, 16 and 682 (11 k) 158 and 162, 88 and 234 (20 k) 103 and 113, 28 and 1190 (33 k) 130 and 149, 130 and 5800 78
+// and 99; 16320, 26 and 198 (5 k) 271 and 246, 41 and 312 (13 k) 236 and 256; 10800, 19 and 357 (7 k) 211 and 195, 36 and 671 (24 k) 152 and 177; 5700, 12 and 507 (6 k) 138 and
+// 125, 20 and 868 (17 k) 119 and 127. Fewer tiles: 3510, 13 and 564 (7 k) 91 and 78, 24 and 1066 (26 k) 80 and 78, 57 and 2540 60 and 68; 2040, 16 and 704 (11 k)
+// 62 and 56, 36 and 1614 (58 k) 43 and 50; 1840, 25 and 1807 (45 k) 40 and 41; 1450, 79 and 3643 (288 k) 23 and 21.
+static bool covers_patches(uint64_t blocks, uint32_t tile_size, float spread, int64_t entries) {
+    const uint32_t tiles = tiles_of_256(blocks, tile_size);
+    return tiles >= 1800u && entries > 0 && tile_threads<8>(tile_size) % 32u == 0u &&
+           (double)spread * (double)entries >= (tiles >= 5000u ? 12500.0 : 30000.0) * tiles;
+}
 static uint32_t pixels_per_lane_fwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread, int64_t entries) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
     const float line = tiles < 6000u ? 7.f : channels <= 4 ? 3.3f : channels <= 8 ? 7.f : 5.f;
@@ -2387,7 +2610,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
 #define CALL_PX(D, P)                                                                             \
     {                                                                                             \
         const uint32_t patches = div_up(tile_threads<P>(tile_size), 32);                          \
-        const auto kernel = D >= 20 && vec ? rasterize_to_pixels_fwd_kernel<D, P, (D >= 20)> : rasterize_to_pixels_fwd_kernel<D, P, false>; \
+        const auto kernel = D >= 20 && vec ? rasterize_to_pixels_fwd_kernel<D, P, (D >= 20), false>  \
+                          : runs ? rasterize_to_pixels_fwd_kernel<D, P, false, (P == 8)> : rasterize_to_pixels_fwd_kernel<D, P, false, false>; \
         SPL_REQUIRE((uint64_t)blocks * patches <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_fwd: too many tiles"); \
         launch_chained_if(warps_fit_at_once((uint64_t)blocks * patches), kernel, blocks * patches, 32, 0, \
             (cudaStream_t)stream,                                                                 \
@@ -2399,7 +2623,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     }
 #define CALL(D)                                                                                   \
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2)) else if (D <= 16 && px == 4) CALL_PX(D, (D <= 16 ? 4 : 2)) else CALL_PX(D, 2)
-    const uint32_t px = pixels_per_lane_fwd(blocks, tile_size, channels, hint.spread, hint.entries);
+    const bool runs = channels <= 4 && covers_patches(blocks, tile_size, hint.spread, hint.entries);
+    const uint32_t px = runs ? 8u : pixels_per_lane_fwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool vec = channels % 4u == 0u && (reinterpret_cast<uintptr_t>(colors) & 15u) == 0u;
     {
         SPL_PROF("rasterize_to_pixels_fwd_kernel", (cudaStream_t)stream);
