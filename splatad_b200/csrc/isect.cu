@@ -1108,18 +1108,17 @@ emit_kernel(GridArgs<kLidar> a, EmitArgs e, const uint32_t *__restrict__ eoff,
 // Walking the row runs of a rectangle output by output, which this replaces, took 6 warp instructions per
 // 32 outputs' lane, and the radix passes over (tile, entry) pairs that grids of more than 128 tile rows took
 // before move 44 B per intersection (14 of the 17 ms of six cameras' frame). What bounds it now is the 12 B
-// of every list entry, written at 4.3 TB/s where the lists are long (a fill: 7.5).
+// of every list entry, written at 4.9 TB/s where the lists are long (a fill: 7.5).
 // Positions are exclusive sums over (earlier tiles, earlier units, earlier CTAs, lower lanes), all of
 // them plain scans: the result is the same for any scheduling, and no block waits for another.
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t kBlkW = 4, kBlkH = 8;                   // tiles per block: one per lane
 static_assert(kBlkW * kBlkH == 32, "one lane per tile of a block");
 constexpr uint32_t kBlkThreads = 512, kBlkWarps = kBlkThreads / 32;   // step A: one entry per thread
-// Step B: a CTA takes a unit of 512 consecutive records of a block, or of 1024 where the lists outgrow the
-// L2: a run's ends are sectors that two units write in parts, which costs little while they meet in
-// the cache (six cameras, 5.8 GB of lists: 1540 us with 512, 1340 with 1024; 116 MB: 42 and 45).
+// Step B: a CTA takes a unit of 512 consecutive records of a block, or of 1024 where the lists are so long that they leave the cache as they
+// are written: figures at tile_scatter_kernel, whose CTAs go with it, six or two an SM.
 constexpr uint32_t kBlkUnitMin = 512, kBlkUnitMax = 1024;
-constexpr uint64_t kBlkLongLists = (126ull << 20) / 12;    // entries
+constexpr uint64_t kBlkLongLists = (800ull << 20) / 12;    // entries
 constexpr uint32_t kBlkWords = 2;                          // writing: 32-record groups per warp
 constexpr uint32_t kBlkCountThreads = 128;                 // counting
 constexpr uint32_t kBlkMaxPerSensor = 1024;                // blocks per sensor (32768 tiles)
@@ -1574,30 +1573,51 @@ tile_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket, int32_t *__
     }
 }
 
-// A CTA puts its unit's list entries in tile order in shared memory first - as record numbers, two bytes
-// each - and its warps then write a few tiles' runs each, in steps that begin on a multiple of 32
-// entries: whole 32-byte sectors but for the two ends of a run. (Storing straight from the lanes whose record
-// covers a tile needs no staging, but sectors written in parts cost the L2 more than whole ones and a fifth
-// of the lanes were active: 180 us for the lidar benchmark's 15.3 M entries. A unit of 128 records per
-// warp, its runs not aligned: 73 us; this: 67. Six cameras: 1920 -> 1340 us, 1310 with two record numbers to a store: the
-// lanes' places lie in any bank, three or four of them in the same. Four entries of a run read before the first is
-// written: 1340 to 1470, the registers cost a CTA.)
+// A CTA leaves its unit's pairs and, by tile, the bits of its records in shared memory; behind that barrier a warp puts a tile's
+// entries in order by itself - a lane takes the bits of 32 records, one scan says where its record numbers go, two bytes
+// each - and writes the run: whole sectors two entries per lane, what is left at the ends by sixteen lanes. (Before, each lane had a
+// tile, the places were summed over the warps and the runs written after another barrier: 64 KB of places for three CTAs an
+// SM. Storing straight from the lanes whose record covers a tile: 180 us for the lidar benchmark's 15.3 M entries.)
+//
+// What bounds it where the lists are long is how they reach the HBM, not the writing itself: with 592 CTAs of 1024 records 100 MB are
+// under way, and the sectors that two units write in parts are evicted between the two, and every such half costs a read
+// and about five whole sectors' time. So whole sectors leave the cache first, halves last, and two CTAs an SM are enough.
+// Six cameras, 5.8 GB of lists: 1310 us before, 1390 with four CTAs an SM, 1250 with two, 1200 with two and that order of leaving (dram
+// reads 401 -> 265 MB); units of 512: 1400. Shorter lists want smaller units and more CTAs, us before and with six of 512 records, by MB of lists: 116 (camera
+// benchmark) 43.5 and 39.5, 184 (lidar benchmark) 66 and 56, 206 (three cameras) 74.5 and 60, 580 (200 k Gaussians, six cameras) 138 and 133; with two of 1024
+// 43.6, 66, 76 and 138, but 302 instead of 338 at 1450 MB. Four entries per lane (32-byte stores): 68 instead of 58 and
+// 1430 instead of 1360, their record numbers lie in the same banks.
+__device__ __forceinline__ uint64_t keep_in_cache() {
+    uint64_t policy;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
+    return policy;
+}
+__device__ __forceinline__ void store_kept(int64_t *to, uint64_t v, uint64_t policy) {
+    asm volatile("st.global.L2::cache_hint.b64 [%0], %1, %2;" ::"l"(__cvta_generic_to_global(to)), "l"(v), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void store_kept(int32_t *to, uint32_t v, uint64_t policy) {
+    asm volatile("st.global.L2::cache_hint.b32 [%0], %1, %2;" ::"l"(__cvta_generic_to_global(to)), "r"(v), "l"(policy) : "memory");
+}
+
 template <uint32_t kWarps>
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void __launch_bounds__(kWarps * 32, kWarps > 8 ? 2 : 6)
 tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restrict__ flatten_ids,
                     int64_t *__restrict__ counters) {
     chain_enter();
-    extern __shared__ __align__(16) unsigned char s_raw[];
-    uint2 *s_pair = reinterpret_cast<uint2 *>(s_raw);
-    uint16_t *s_out = reinterpret_cast<uint16_t *>(s_pair + kWarps * kBlkWords * 32);
-    __shared__ uint32_t s_n[kWarps][32];       // entries per (warp, tile)
-    __shared__ uint4 s_run[32];                       // per tile: first place in s_out, entries, list position, id
+    constexpr uint32_t kUnit = kWarps * kBlkWords * 32, kWords = kUnit / 32;   // words of a tile: its bits over the unit's records
+    constexpr uint32_t kTiles = 32 / kWords, kRoom = kUnit + 8;   // tiles a warp puts in order at a time; places of one, from a multiple of eight on
+    static_assert(kWords == 16 || kWords == 32, "a tile's words lie in a warp or in half of one");
+    __shared__ uint2 s_pair[kUnit];
+    __shared__ uint32_t s_word[32][kWords + 1];
+    __shared__ __align__(16) uint16_t s_out[kWarps][kTiles * kRoom];   // record numbers in list order
     if (blk_overflow(a)) {
         if (blockIdx.x == 0 && threadIdx.x == 0)
             atomicOr((unsigned long long *)&counters[CNT_STATUS], (unsigned long long)ST_OVERFLOW_CAPACITY);
         return;
     }
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t kept = keep_in_cache();
+    const bool wide = ((reinterpret_cast<uintptr_t>(isect_ids) & 15u) | (reinterpret_cast<uintptr_t>(flatten_ids) & 7u)) == 0u;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = lane % kWords, half = lane / kWords;
     const uint32_t n_units = a.unit_start[a.C * a.blocks];
     const uint32_t cap = (uint32_t)min(a.capacity, (int64_t)0x7fffffff);
     uint4 info = make_uint4(0u, 0u, 0u, 0u);
@@ -1616,67 +1636,71 @@ tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restr
         uint32_t at = 0;   // lane l: list position of the unit's first entry of tile l
         if (t.x < a.width && t.y < a.height)
             at = __ldg(a.tile_base + t.sensor * a.n_tiles + tile) + __ldg(a.unit_cnt + (size_t)u * 32 + lane);
-        uint32_t word[kBlkWords], n = 0;   // lane l: which records cover tile l, how many
+        const uint32_t high = (t.sensor << a.tile_n_bits) | tile;
+        __syncthreads();   // the unit before has been written
 #pragma unroll
         for (uint32_t j = 0; j < kBlkWords; ++j) {
-            if (rec[j].x) s_pair[32 * (warp * kBlkWords + j) + lane] = __ldg(a.pair + rec[j].y);
-            word[j] = warp_transpose_bits(rec[j].x, lane);
-            n += __popc(word[j]);
+            const uint32_t w = warp * kBlkWords + j;
+            if (rec[j].x) s_pair[32 * w + lane] = __ldg(a.pair + rec[j].y);
+            s_word[lane][w] = warp_transpose_bits(rec[j].x, lane);
         }
-        s_n[warp][lane] = n;
         __syncthreads();
-        uint32_t before = 0, all = 0;   // lane l: entries of tile l in earlier warps, in the unit
+        for (uint32_t l0 = warp * kTiles; l0 < 32; l0 += kWarps * kTiles) {
+            // the lanes write down the record numbers of their words of a tile, behind those of the words before
+            uint32_t m = s_word[l0 + half][col], place = __popc(m);
+            const uint32_t mine = place;
 #pragma unroll
-        for (uint32_t w = 0; w < kWarps; ++w) {
-            const uint32_t c = s_n[w][lane];
-            if (w < warp) before += c;
-            all += c;
-        }
-        uint32_t first = all;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xffffffffu, first, off);
-            if (lane >= (uint32_t)off) first += o;
-        }
-        first -= all;
-        if (warp == 0) s_run[lane] = make_uint4(first, all, at, (t.sensor << a.tile_n_bits) | tile);
-        uint32_t local = first + before;
-#pragma unroll
-        for (uint32_t j = 0; j < kBlkWords; ++j) {
-            uint32_t w = word[j];
-            const uint32_t first_rec = 32 * (warp * kBlkWords + j);
+            for (uint32_t off = 1; off < kWords; off <<= 1) {
+                const uint32_t o = __shfl_up_sync(0xffffffffu, place, off, kWords);
+                if (col >= off) place += o;
+            }
+            const uint32_t total = place;   // of the last lane: the tile's entries
+            place += half * kRoom - mine + (__shfl_sync(0xffffffffu, at, l0 + half) & 7u);
+            uint16_t *out = s_out[warp];
             const auto next = [&] {
-                const uint32_t r = first_rec + __ffs(w) - 1;
-                w &= w - 1;
+                const uint32_t r = 32 * col + __ffs(m) - 1;
+                m &= m - 1;
                 return r;
             };
-            if (w != 0u && (local & 1u)) s_out[local++] = (uint16_t)next();
-            while (w & (w - 1)) {   // two at a time: the lanes' places lie in any bank
+            if (m != 0u && (place & 1u)) out[place++] = (uint16_t)next();
+            while (m & (m - 1)) {   // two at a time
                 const uint32_t r = next();
-                *reinterpret_cast<uint32_t *>(s_out + local) = r | next() << 16;
-                local += 2;
+                *reinterpret_cast<uint32_t *>(out + place) = r | next() << 16;
+                place += 2;
             }
-            if (w) s_out[local++] = (uint16_t)next();
-        }
-        __syncthreads();
-        for (uint32_t l = warp; l < 32; l += kWarps) {
-            const uint4 run = s_run[l];
-            const uint32_t end = min(run.z + run.y, cap);
-            const uint16_t *src = s_out + run.x - run.z;   // indexed by list position
-            for (uint32_t p0 = run.z & ~31u; p0 < end; p0 += 4 * 32) {
+            if (m) out[place] = (uint16_t)next();
+            __syncwarp();
 #pragma unroll
-                for (uint32_t q = 0; q < 4; ++q) {
-                    if (p0 + 32 * q >= end) break;
-                    const uint32_t p = p0 + 32 * q + lane;
-                    if (p >= run.z && p < end) {
+            for (uint32_t h = 0; h < kTiles; ++h) {
+                const uint32_t begin = __shfl_sync(0xffffffffu, at, l0 + h), id = __shfl_sync(0xffffffffu, high, l0 + h);
+                const uint32_t end = min(begin + __shfl_sync(0xffffffffu, total, h * kWords + kWords - 1), cap);
+                const uint16_t *src = out + h * kRoom - (begin & ~7u);   // indexed by list position
+                if (!wide) {
+                    for (uint32_t p = begin + lane; p < end; p += 32u) {
                         const uint2 e = s_pair[src[(int32_t)p]];
-                        isect_ids[p] = (int64_t)(((uint64_t)run.w << 32) | e.x);
+                        isect_ids[p] = (int64_t)(((uint64_t)id << 32) | e.x);
                         flatten_ids[p] = (int32_t)e.y;
                     }
+                    continue;
+                }
+                // whole sectors first, then what is left at both ends
+                const uint32_t inner = (begin + 7u) & ~7u, outer = end & ~7u;
+#pragma unroll 2
+                for (uint32_t p = inner + 2u * lane; p < outer; p += 64u) {
+                    const uint32_t r = *reinterpret_cast<const uint32_t *>(src + (int32_t)p);
+                    const uint2 e = s_pair[r & 0xffffu], f = s_pair[r >> 16];
+                    __stcs(reinterpret_cast<uint4 *>(isect_ids + p), make_uint4(e.x, id, f.x, id));
+                    __stcs(reinterpret_cast<uint2 *>(flatten_ids + p), make_uint2(e.y, f.y));
+                }
+                const uint32_t p = lane < 8u ? begin + lane : max(inner, outer) + lane - 8u;
+                if (lane < 16u && p < (lane < 8u ? min(inner, end) : end)) {
+                    const uint2 e = s_pair[src[(int32_t)p]];
+                    store_kept(isect_ids + p, ((uint64_t)id << 32) | e.x, kept);
+                    store_kept(flatten_ids + p, e.y, kept);
                 }
             }
+            __syncwarp();
         }
-        __syncthreads();
     }
 }
 
@@ -2166,12 +2190,9 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
             constexpr uint32_t kMin = kBlkUnitMin / (32 * kBlkWords), kMax = kBlkUnitMax / (32 * kBlkWords);
             const bool longer = a.unit == kBlkUnitMax;
             auto kernel = longer ? tile_scatter_kernel<kMax> : tile_scatter_kernel<kMin>;
-            // records' pairs and 32 places of two bytes per record: 36 or 72 KB, five or three CTAs per SM
-            const size_t smem = (size_t)a.unit * (sizeof(uint2) + 32 * sizeof(uint16_t));
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            const uint32_t grid = min(units_max, (longer ? 3u : 5u) * kNumSMs);
+            const uint32_t grid = min(units_max, (longer ? 2u : 6u) * kNumSMs);
             // long lists: not placed while the scan still holds its SMs (six cameras: 1340 us, and 80 more chained)
-            launch_chained_if(!longer, kernel, grid, a.unit / kBlkWords, smem, st, a, isect_ids, flatten_ids, p.counters);
+            launch_chained_if(!longer, kernel, grid, a.unit / kBlkWords, 0, st, a, isect_ids, flatten_ids, p.counters);
         }
     } else {
         FillWs f = carve_fill(fill_workspace, (uint64_t)capacity);
