@@ -200,6 +200,23 @@ __device__ __forceinline__ uint32_t lane_index() {
     return lane;
 }
 
+// Shared memory by an address in a register of its own.
+__device__ __forceinline__ uint32_t smem_register(const void *p) {
+    uint32_t a;
+    asm volatile("mov.u32 %0, %1;" : "=r"(a) : "r"(smem_addr(p)));
+    return a;
+}
+__device__ __forceinline__ float4 lds4(uint32_t a, int offset) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a + offset));
+    return v;
+}
+__device__ __forceinline__ float2 lds2(uint32_t a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+}
+
 // exponents of a pair of pixels in one row: dx of the two, the row's b * dy and c * dy * dy
 __device__ __forceinline__ float2 pair_power(float a, float2 dx, float bdy, float cdy2) {
     const float2 t = __ffma2_rn(make_float2(a, a), dx, make_float2(bdy, bdy));
@@ -1682,6 +1699,12 @@ __device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t
 //   tiles 362 / 506 -> 371 / 512.
 //   Two pixels, 9 to 16 channels, many tiles: 96 registers. 1920 x 1080, 2.5 and 27.5 tiles per Gaussian 442, 875 -> 404, 834; 640 x 360,
 //   5.1 tiles 153 -> 158.
+//   Up to four channels, scenes of large Gaussians (kRunsBwd, chosen as in the forward kernel): what is staged moves up to the front, so that
+// entries that cover the patch follow one another without a look at a mask, a threshold or a pixel's first entry - the place of the next one is known -,
+// two at a time with one butterfly for their 24 sums, whose five steps are the longest chain there is. 200 M -> 180 M warp instructions, 1920 x
+// 1080 305 -> 287 us, three cameras 366 -> 335. Neither more warps (96 registers, the cotangents in shared memory: 20 an SM, 344) nor fewer (one entry at a time
+// with 128 registers, 16: 337) nor the order of the additions helps: at 12 warps an SM the FP32 pipe is busy 55 % of the time, the
+// exponentials and reciprocals (8 cycles each) 30 %, shuffles (4 cycles an SM) 25 %.
 //   Above 20 channels, few tiles: the chain of the longest list counts, so no spills, whole rows at once and the skip. 640 x 360, 32
 //   channels, scales of 1, 0.6, 0.3 and 0.1: 326, 346, 244, 205 -> 303, 332, 236, 199; 1920 x 1080: 1862 -> 1999.
 constexpr bool has_other_bwd(int cdim, int px) { return (px == 4 && cdim <= 8) || (px == 2 && cdim == 16) || cdim == 32; }
@@ -1689,13 +1712,16 @@ constexpr bool pixels_bwd_skips(int cdim, int px, bool other) { return other && 
 
 // registers per thread, by measurement (4 channels, eight pixels: 335 us at 128, 348 at 112, 361 at 144; 16 channels:
 // 386 at 168, 394 at 128; 8: 483 at 96, 520 at 128; 20, four pixels: 847 at 168, 980 at 200; 32: 1950 at 128, 2075 at 160)
-constexpr int pixels_bwd_regs(int cdim, int px, bool other) {
+constexpr int kPlainBwd = 0, kOtherBwd = 1, kRunsBwd = 2;
+constexpr int pixels_bwd_regs(int cdim, int px, int kind) {
+    const bool other = kind == kOtherBwd;
+    if (kind == kRunsBwd) return 168;
     return cdim <= 4 ? (px == 8 ? 128 : px == 4 ? 80 : 72) : cdim <= 8 ? (px == 4 ? 96 : 88) : cdim <= 16 ? (px == 4 ? 168 : other ? 96 : 104)
                      : cdim <= 20 ? 168 : other ? 168 : 128;
 }
 
-template <int CDIM, int PX, bool kAbs, bool kOther>
-__global__ void __maxnreg__(pixels_bwd_regs(CDIM, PX, kOther))
+template <int CDIM, int PX, bool kAbs, int kKind>
+__global__ void __maxnreg__(pixels_bwd_regs(CDIM, PX, kKind))
 rasterize_to_pixels_bwd_kernel(
     uint32_t C, int64_t n_isects, const float2 *__restrict__ means2d,
     const float *__restrict__ conics, const float *__restrict__ colors, uint32_t channels,
@@ -1711,6 +1737,7 @@ rasterize_to_pixels_bwd_kernel(
     chain_enter();
     static_assert(PX % 2 == 0, "pixels are handled in pairs");
     constexpr int P2 = PX / 2;
+    constexpr bool kOther = kKind == kOtherBwd, kRuns = kKind == kRunsBwd;
     __shared__ float4 sA[32];                // x, y, vx, vy
     __shared__ float4 sB[32];                // scaled conic, opacity
     __shared__ float4 sCol[32 * CDIM / 4];   // zeros behind the channels
@@ -1721,7 +1748,9 @@ rasterize_to_pixels_bwd_kernel(
     const uint32_t gtile = blockIdx.x / patches, cam = gtile / tiles_per_cam;
     const uint32_t tile = gtile - cam * tiles_per_cam;
     const uint32_t ty = tile / tile_w, tx = tile - ty * tile_w;
-    const uint32_t lane = threadIdx.x, tr = (blockIdx.x - gtile * patches) * 32u + lane;
+    uint32_t lane = threadIdx.x;
+    if constexpr (kRuns) lane = lane_index();
+    const uint32_t tr = (blockIdx.x - gtile * patches) * 32u + lane;
     const TilePixels<PX> tp = tile_pixels<PX>(tile_size, tr);
     const uint32_t i = ty * tile_size + tp.y, j = tx * tile_size + tp.x;
     uint32_t n_inside = 0;   // pixels of this thread inside the tile and the image
@@ -1797,158 +1826,320 @@ rasterize_to_pixels_bwd_kernel(
     const GradSlot slot_a = pixel_grad_slot<kAbs>(mine_a.value, CDIM, channels, v_colors,
                                                   v_conics, v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
 
-    constexpr bool kSkip = pixels_bwd_skips(CDIM, PX, kOther);
-    int32_t waiting = thread_last;   // position of the next entry that is a pixel's of this lane last one; -1: none
-    bool pending = true;             // a lane of the warp waits for one
-    int32_t next_id = 0;
-    if (eff_end - 1 - (int32_t)lane >= range.start) next_id = flatten_ids[eff_end - 1 - (int32_t)lane];
-    for (int32_t batch_end = eff_end - 1; batch_end >= range.start; batch_end -= 32) {
-        const int32_t idx = batch_end - (int32_t)lane;
-        const int32_t g = next_id;
-        uint32_t seen = 0u;
-        float most;
-        PixelEntry e;
-        if (idx >= range.start) {
-            e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
-            if (idx - 32 >= range.start) next_id = flatten_ids[idx - 32];   // on its way meanwhile
-            seen = patch_sees<false, false>(e, box, roll_lo, roll_hi, most);
-        }
-        uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
-        const uint32_t careful = __ballot_sync(0xffffffffu, (seen & kCarefulEntry) != 0u);
-        __syncwarp();   // the batch before has been read
-        if (seen) {
-            sA[lane] = e.A;
-            sB[lane] = scaled_conic(e.B);
-            sId[lane] = make_float2(__int_as_float(g), 1.f / e.B.w);
-            // A colour that is not finite is blended by no pixel of the patch - it would have left its mark there. It may lie
-            // behind the last entry of some pixels and out of reach of the others, and must not meet their weights of zero.
-            if (CDIM <= 16 || (CDIM == 32 && kOther)) stage_whole_row<CDIM, true>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, vec);
-            else {   // (20 channels: all loads of a row at once take registers, 990 -> 1130 us)
-                float *row = reinterpret_cast<float *>(sCol) + lane * CDIM;
-                stage_row<true>(row, colors, (size_t)g, channels, vec);
-                for (uint32_t k = (channels + 3u) & ~3u; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
+    if constexpr (kRuns) {
+        int32_t next_id = 0;
+        if (eff_end - 1 - (int32_t)lane >= range.start) next_id = flatten_ids[eff_end - 1 - (int32_t)lane];
+        constexpr uint32_t kEntry = 32 + 4 * CDIM;   // bytes
+        __shared__ float4 sEntry[32 * kEntry / 16];   // x, y, vx, vy | scaled conic, opacity | channels, zeros behind them
+        const uint32_t entries = smem_register(sEntry), ids = smem_register(sId);
+        // two entries' sums: colours and geometry of the first, then of the second
+        static_assert(2 * kSums <= 32, "a lane for every sum of two entries");
+        const SumSlot mine_two = sum_slot<2 * kSums>(lane);
+        const uint32_t two_entry = mine_two.value >= kSums ? 1u : 0u;
+        const GradSlot slot_two = pixel_grad_slot<kAbs>(mine_two.value - (two_entry ? kSums : 0), CDIM, channels, v_colors, v_conics, v_means2d,
+                                                        v_pix_vels, v_opacities, v_means2d_abs);
+        int32_t event = warp_last;   // the next entry that is any pixel's last one
+        for (int32_t batch_end = eff_end - 1; batch_end >= range.start; batch_end -= 32) {
+            const int32_t idx = batch_end - (int32_t)lane;
+            const int32_t g = next_id;
+            uint32_t seen = 0u;
+            float most;
+            PixelEntry e;
+            if (idx >= range.start) {
+                e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
+                if (idx - 32 >= range.start) next_id = flatten_ids[idx - 32];   // on its way meanwhile
+                seen = patch_sees<false, true>(e, box, roll_lo, roll_hi, most);
             }
-        }
-        __syncwarp();
-        while (todo) {
-            const uint32_t t = (uint32_t)__ffs(todo) - 1u, bit = 1u << t;
-            todo ^= bit;
-            const int32_t entry = batch_end - (int32_t)t;
-            if (pending && __any_sync(0xffffffffu, entry <= waiting)) {
-                // pixels whose last entry this is, or lay behind it: they take part from here on
-                int32_t next = -1;
+            const uint32_t kept = __ballot_sync(0xffffffffu, seen != 0u), n = __popc(kept);
+            const uint32_t place = __popc(kept & ((1u << lane) - 1u));
+            const uint32_t full = __reduce_or_sync(0xffffffffu, (seen & kFullEntry) ? 1u << place : 0u);
+            const uint32_t careful = __reduce_or_sync(0xffffffffu, (seen & kCarefulEntry) ? 1u << place : 0u);
+            __syncwarp();   // the batch before has been read
+            if (seen) {
+                float4 *entry = sEntry + place * (kEntry / 16);
+                entry[0] = e.A;
+                entry[1] = scaled_conic(e.B);
+                sId[place] = make_float2(__int_as_float(g), 1.f / e.B.w);
+                stage_whole_row<CDIM, true>(entry + 2, colors + (size_t)g * channels, channels, vec);
+            }
+            __syncwarp();
+            // kCount entries in sequence, whose sums share a butterfly; kFull: they cover the patch
+            const auto process = [&](uint32_t t, auto count, auto covers) {
+                constexpr int kCount = decltype(count)::value;
+                constexpr bool kFull = decltype(covers)::value;
+                float4 A[kCount], B[kCount], col[kCount][CDIM / 4];
+                float mx[kCount], dy[kCount];
+                float2 alpha[kCount][P2];
+                uint32_t capped = 0u;   // pixels with a capped alpha, which passes no gradient on to the geometry
 #pragma unroll
-                for (int k = 0; k < PX; ++k) {
-                    const int32_t last = sLast[k][lane];
-                    if (entry <= last) {
-                        if (k & 1) npx[k / 2].y = -(px0 + (float)k); else npx[k / 2].x = -(px0 + (float)k);
-                    } else next = max(next, last);
+                for (int h = 0; h < kCount; ++h) {
+                    const uint32_t entry = entries + (t + h) * kEntry;
+                    A[h] = lds4(entry, 0);
+                    B[h] = lds4(entry, 16);
+                    mx[h] = A[h].x + roll * A[h].z;
+                    dy[h] = A[h].y + roll * A[h].w - py;
+                    const float bdy = B[h].y * dy[h], cdy2 = B[h].z * dy[h] * dy[h];
+#pragma unroll
+                    for (int q = 0; q < P2; ++q) {
+                        const float2 pw = pair_power(B[h].x, __fadd2_rn(make_float2(mx[h], mx[h]), npx[q]), bdy, cdy2);
+                        alpha[h][q] = __fmul2_rn(make_float2(B[h].w, B[h].w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
+                        if (!kFull) alpha[h][q] = make_float2(alpha[h][q].x >= kAlphaMin ? alpha[h][q].x : 0.f, alpha[h][q].y >= kAlphaMin ? alpha[h][q].y : 0.f);
+                    }
+                    if (!kFull && ((careful >> t) & 1u)) {
+#pragma unroll
+                        for (int q = 0; q < P2; ++q) {
+                            const float2 pw = pair_power(B[h].x, __fadd2_rn(make_float2(mx[h], mx[h]), npx[q]), bdy, cdy2);
+                            if (alpha[h][q].x > kAlphaMax) capped |= 1u << (2 * q);
+                            if (alpha[h][q].y > kAlphaMax) capped |= 2u << (2 * q);
+                            alpha[h][q].x = pw.x <= 0.f ? fminf(kAlphaMax, alpha[h][q].x) : 0.f;
+                            alpha[h][q].y = pw.y <= 0.f ? fminf(kAlphaMax, alpha[h][q].y) : 0.f;
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < CDIM / 4; ++c) col[h][c] = lds4(entry, 32 + 16 * c);
                 }
-                waiting = next;
-                pending = __any_sync(0xffffffffu, waiting >= 0);
-            }
-            const float4 A = sA[t], B = sB[t];
-            const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
-            const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
-            float4 col[CDIM / 4];
+                float2 csum[kCount][CDIM], s0[kCount], s1[kCount], s2[kCount], ax[kCount], ay[kCount];
 #pragma unroll
-            for (int k = 0; k < CDIM / 4; ++k) col[k] = sCol[t * (CDIM / 4) + k];
-            float2 alpha[P2], v[P2], csum[CDIM];
+                for (int q = 0; q < P2; ++q)
 #pragma unroll
-            for (int q = 0; q < P2; ++q) {
-                const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
-                const float2 av = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
-                alpha[q] = make_float2(av.x >= kAlphaMin ? av.x : 0.f, av.y >= kAlphaMin ? av.y : 0.f);
+                    for (int h = 0; h < kCount; ++h) {
+                        const float2 ra = reciprocal_pair(__fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha[h][q].x, -alpha[h][q].y)));
+                        T[q] = __fmul2_rn(T[q], ra);
+                        const float2 fac = __fmul2_rn(alpha[h][q], T[q]);
+                        float2 dot = make_float2(0.f, 0.f);   // (c . g) of the two pixels
+#pragma unroll
+                        for (int k = 0; k < CDIM; ++k) {
+                            const float4 c4 = col[h][k / 4];
+                            const float c = (k & 3) == 0 ? c4.x : (k & 3) == 1 ? c4.y : (k & 3) == 2 ? c4.z : c4.w;
+                            dot = k == 0 ? __fmul2_rn(make_float2(c, c), v_out[k][q]) : __ffma2_rn(make_float2(c, c), v_out[k][q], dot);
+                            csum[h][k] = q == 0 ? __fmul2_rn(fac, v_out[k][q]) : __ffma2_rn(fac, v_out[k][q], csum[h][k]);
+                        }
+                        const float2 v_alpha = __ffma2_rn(T[q], dot, __fmul2_rn(make_float2(-ra.x, -ra.y), behind[q]));
+                        behind[q] = __ffma2_rn(fac, dot, behind[q]);
+                        float2 v = __fmul2_rn(alpha[h][q], v_alpha);
+                        if (!kFull) {
+                            if (capped & (1u << (2 * q))) v.x = 0.f;
+                            if (capped & (2u << (2 * q))) v.y = 0.f;
+                        }
+                        const float2 dx = __fadd2_rn(make_float2(mx[h], mx[h]), npx[q]), vx = __fmul2_rn(v, dx);
+                        s0[h] = q == 0 ? v : __fadd2_rn(s0[h], v);
+                        s1[h] = q == 0 ? vx : __fadd2_rn(s1[h], vx);
+                        s2[h] = q == 0 ? __fmul2_rn(vx, dx) : __ffma2_rn(vx, dx, s2[h]);
+                        if (kAbs) {   // (v first: a pixel that is far out must not meet a conic of any size)
+                            const float bdy = B[h].y * dy[h], cdy = 2.f * B[h].z * dy[h];
+                            const float2 gx = __ffma2_rn(make_float2(2.f * B[h].x, 2.f * B[h].x), vx, __fmul2_rn(make_float2(bdy, bdy), v));
+                            const float2 gy = __ffma2_rn(make_float2(B[h].y, B[h].y), vx, __fmul2_rn(make_float2(cdy, cdy), v));
+                            const float2 bx = make_float2(fabsf(gx.x), fabsf(gx.y)), by = make_float2(fabsf(gy.x), fabsf(gy.y));
+                            ax[h] = q == 0 ? bx : __fadd2_rn(ax[h], bx);
+                            ay[h] = q == 0 ? by : __fadd2_rn(ay[h], by);
+                        }
+                    }
+                float sums[kCount * kSums];
+#pragma unroll
+                for (int h = 0; h < kCount; ++h) {
+                    float *sum = sums + h * kSums;
+#pragma unroll
+                    for (int k = 0; k < CDIM; ++k) sum[k] = csum[h][k].x + csum[h][k].y;
+                    const float m0 = s0[h].x + s0[h].y, m1 = s1[h].x + s1[h].y, my = dy[h] * m0;
+                    const float gx = 2.f * B[h].x * m1 + B[h].y * my, gy = B[h].y * m1 + 2.f * B[h].z * my;
+                    sum[CDIM + 0] = s2[h].x + s2[h].y;
+                    sum[CDIM + 1] = dy[h] * m1;
+                    sum[CDIM + 2] = dy[h] * my;
+                    sum[CDIM + 3] = gx;
+                    sum[CDIM + 4] = gy;
+                    sum[CDIM + 5] = gx * roll;
+                    sum[CDIM + 6] = gy * roll;
+                    sum[CDIM + 7] = m0;
+                    if (kAbs) {
+                        sum[CDIM + 8] = ax[h].x + ax[h].y;
+                        sum[CDIM + 9] = ay[h].x + ay[h].y;
+                    }
+                }
+                const float2 id = lds2(ids + 8u * (kCount == 1 ? t : t + two_entry));
+                const float total = warp_sum_values<kCount * kSums, 16>(sums, lane);
+                if (kCount == 1) slot_a.add((size_t)__float_as_int(id.x), total, id.y, mine_a.writes);
+                else slot_two.add((size_t)__float_as_int(id.x), total, id.y, mine_two.writes);
+            };
+            // the first place at which a pixel of the warp takes part
+            const auto next_event = [&](uint32_t t) {
+                const uint32_t due = __ballot_sync(0xffffffffu, seen && place >= t && idx <= event);
+                return due ? (uint32_t)__popc(kept & ((due & (0u - due)) - 1u)) : n;
+            };
+            uint32_t t = 0, t_event = next_event(0);
+            while (t < n) {
+                if (t == t_event) {
+                    const int32_t entry = __shfl_sync(0xffffffffu, idx, __ffs(__ballot_sync(0xffffffffu, seen && place == t)) - 1);
+                    int32_t next = -1;
+#pragma unroll
+                    for (int k = 0; k < PX; ++k) {
+                        const int32_t last = sLast[k][lane];
+                        if (entry <= last) {
+                            if (k & 1) npx[k / 2].y = -(px0 + (float)k); else npx[k / 2].x = -(px0 + (float)k);
+                        } else next = max(next, last);
+                    }
+                    event = __reduce_max_sync(0xffffffffu, next);
+                    t_event = next_event(t + 1u);
+                }
+                const uint32_t rest = ~full >> t, end = min(t_event, rest ? t + (uint32_t)__ffs(rest) - 1u : n);
+                for (; t + 1u < end; t += 2u) process(t, std::integral_constant<int, 2>(), std::true_type());
+                if (t < end) process(t++, std::integral_constant<int, 1>(), std::true_type());
+                if (t < t_event && t < n) process(t++, std::integral_constant<int, 1>(), std::false_type());
             }
-            uint32_t capped = 0u;   // pixels with a capped alpha, which passes no gradient on to the geometry
-            if (careful & bit) {
+        }
+    } else {
+        constexpr bool kSkip = pixels_bwd_skips(CDIM, PX, kOther);
+        int32_t waiting = thread_last;   // position of the next entry that is a pixel's of this lane last one; -1: none
+        bool pending = true;             // a lane of the warp waits for one
+        int32_t next_id = 0;
+        if (eff_end - 1 - (int32_t)lane >= range.start) next_id = flatten_ids[eff_end - 1 - (int32_t)lane];
+        for (int32_t batch_end = eff_end - 1; batch_end >= range.start; batch_end -= 32) {
+            const int32_t idx = batch_end - (int32_t)lane;
+            const int32_t g = next_id;
+            uint32_t seen = 0u;
+            float most;
+            PixelEntry e;
+            if (idx >= range.start) {
+                e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
+                if (idx - 32 >= range.start) next_id = flatten_ids[idx - 32];   // on its way meanwhile
+                seen = patch_sees<false, false>(e, box, roll_lo, roll_hi, most);
+            }
+            uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
+            const uint32_t careful = __ballot_sync(0xffffffffu, (seen & kCarefulEntry) != 0u);
+            __syncwarp();   // the batch before has been read
+            if (seen) {
+                sA[lane] = e.A;
+                sB[lane] = scaled_conic(e.B);
+                sId[lane] = make_float2(__int_as_float(g), 1.f / e.B.w);
+                // A colour that is not finite is blended by no pixel of the patch - it would have left its mark there. It may lie
+                // behind the last entry of some pixels and out of reach of the others, and must not meet their weights of zero.
+                if (CDIM <= 16 || (CDIM == 32 && kOther)) stage_whole_row<CDIM, true>(sCol + lane * (CDIM / 4), colors + (size_t)g * channels, channels, vec);
+                else {   // (20 channels: all loads of a row at once take registers, 990 -> 1130 us)
+                    float *row = reinterpret_cast<float *>(sCol) + lane * CDIM;
+                    stage_row<true>(row, colors, (size_t)g, channels, vec);
+                    for (uint32_t k = (channels + 3u) & ~3u; k < (uint32_t)CDIM; ++k) row[k] = 0.f;
+                }
+            }
+            __syncwarp();
+            while (todo) {
+                const uint32_t t = (uint32_t)__ffs(todo) - 1u, bit = 1u << t;
+                todo ^= bit;
+                const int32_t entry = batch_end - (int32_t)t;
+                if (pending && __any_sync(0xffffffffu, entry <= waiting)) {
+                    // pixels whose last entry this is, or lay behind it: they take part from here on
+                    int32_t next = -1;
+#pragma unroll
+                    for (int k = 0; k < PX; ++k) {
+                        const int32_t last = sLast[k][lane];
+                        if (entry <= last) {
+                            if (k & 1) npx[k / 2].y = -(px0 + (float)k); else npx[k / 2].x = -(px0 + (float)k);
+                        } else next = max(next, last);
+                    }
+                    waiting = next;
+                    pending = __any_sync(0xffffffffu, waiting >= 0);
+                }
+                const float4 A = sA[t], B = sB[t];
+                const float mx = A.x + roll * A.z, dy = A.y + roll * A.w - py;
+                const float bdy = B.y * dy, cdy2 = B.z * dy * dy;
+                float4 col[CDIM / 4];
+#pragma unroll
+                for (int k = 0; k < CDIM / 4; ++k) col[k] = sCol[t * (CDIM / 4) + k];
+                float2 alpha[P2], v[P2], csum[CDIM];
 #pragma unroll
                 for (int q = 0; q < P2; ++q) {
                     const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
-                    if (alpha[q].x > kAlphaMax) capped |= 1u << (2 * q);
-                    if (alpha[q].y > kAlphaMax) capped |= 2u << (2 * q);
-                    alpha[q].x = pw.x <= 0.f ? fminf(kAlphaMax, alpha[q].x) : 0.f;
-                    alpha[q].y = pw.y <= 0.f ? fminf(kAlphaMax, alpha[q].y) : 0.f;
+                    const float2 av = __fmul2_rn(make_float2(B.w, B.w), make_float2(exp2_approx(pw.x), exp2_approx(pw.y)));
+                    alpha[q] = make_float2(av.x >= kAlphaMin ? av.x : 0.f, av.y >= kAlphaMin ? av.y : 0.f);
                 }
-            }
-            if (kSkip) {
-                bool any = false;
+                uint32_t capped = 0u;   // pixels with a capped alpha, which passes no gradient on to the geometry
+                if (careful & bit) {
 #pragma unroll
-                for (int q = 0; q < P2; ++q) any = any || alpha[q].x > 0.f || alpha[q].y > 0.f;
-                if (!__any_sync(0xffffffffu, any)) continue;
-            }
-#pragma unroll
-            for (int q = 0; q < P2; ++q) {
-                const float2 ra = reciprocal_pair(__fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha[q].x, -alpha[q].y)));
-                T[q] = __fmul2_rn(T[q], ra);
-                const float2 fac = __fmul2_rn(alpha[q], T[q]);
-                float2 dot = make_float2(0.f, 0.f);   // (c . g) of the two pixels
-#pragma unroll
-                for (int k = 0; k < CDIM; ++k) {
-                    const float4 c4 = col[k / 4];
-                    const float c = (k & 3) == 0 ? c4.x : (k & 3) == 1 ? c4.y : (k & 3) == 2 ? c4.z : c4.w;
-                    dot = k == 0 ? __fmul2_rn(make_float2(c, c), v_out[k][q]) : __ffma2_rn(make_float2(c, c), v_out[k][q], dot);
-                    csum[k] = q == 0 ? __fmul2_rn(fac, v_out[k][q]) : __ffma2_rn(fac, v_out[k][q], csum[k]);
+                    for (int q = 0; q < P2; ++q) {
+                        const float2 pw = pair_power(B.x, __fadd2_rn(make_float2(mx, mx), npx[q]), bdy, cdy2);
+                        if (alpha[q].x > kAlphaMax) capped |= 1u << (2 * q);
+                        if (alpha[q].y > kAlphaMax) capped |= 2u << (2 * q);
+                        alpha[q].x = pw.x <= 0.f ? fminf(kAlphaMax, alpha[q].x) : 0.f;
+                        alpha[q].y = pw.y <= 0.f ? fminf(kAlphaMax, alpha[q].y) : 0.f;
+                    }
                 }
-                const float2 v_alpha = __ffma2_rn(T[q], dot, __fmul2_rn(make_float2(-ra.x, -ra.y), behind[q]));
-                behind[q] = __ffma2_rn(fac, dot, behind[q]);
-                v[q] = __fmul2_rn(alpha[q], v_alpha);
-            }
-            if (capped) {
+                if (kSkip) {
+                    bool any = false;
+#pragma unroll
+                    for (int q = 0; q < P2; ++q) any = any || alpha[q].x > 0.f || alpha[q].y > 0.f;
+                    if (!__any_sync(0xffffffffu, any)) continue;
+                }
 #pragma unroll
                 for (int q = 0; q < P2; ++q) {
-                    if (capped & (1u << (2 * q))) v[q].x = 0.f;
-                    if (capped & (2u << (2 * q))) v[q].y = 0.f;
+                    const float2 ra = reciprocal_pair(__fadd2_rn(make_float2(1.f, 1.f), make_float2(-alpha[q].x, -alpha[q].y)));
+                    T[q] = __fmul2_rn(T[q], ra);
+                    const float2 fac = __fmul2_rn(alpha[q], T[q]);
+                    float2 dot = make_float2(0.f, 0.f);   // (c . g) of the two pixels
+#pragma unroll
+                    for (int k = 0; k < CDIM; ++k) {
+                        const float4 c4 = col[k / 4];
+                        const float c = (k & 3) == 0 ? c4.x : (k & 3) == 1 ? c4.y : (k & 3) == 2 ? c4.z : c4.w;
+                        dot = k == 0 ? __fmul2_rn(make_float2(c, c), v_out[k][q]) : __ffma2_rn(make_float2(c, c), v_out[k][q], dot);
+                        csum[k] = q == 0 ? __fmul2_rn(fac, v_out[k][q]) : __ffma2_rn(fac, v_out[k][q], csum[k]);
+                    }
+                    const float2 v_alpha = __ffma2_rn(T[q], dot, __fmul2_rn(make_float2(-ra.x, -ra.y), behind[q]));
+                    behind[q] = __ffma2_rn(fac, dot, behind[q]);
+                    v[q] = __fmul2_rn(alpha[q], v_alpha);
                 }
-            }
-            float2 s0 = make_float2(0.f, 0.f), s1 = s0, s2 = s0, ax = s0, ay = s0;
+                if (capped) {
 #pragma unroll
-            for (int q = 0; q < P2; ++q) {
-                const float2 dx = __fadd2_rn(make_float2(mx, mx), npx[q]), vx = __fmul2_rn(v[q], dx);
-                s0 = q == 0 ? v[q] : __fadd2_rn(s0, v[q]);
-                s1 = q == 0 ? vx : __fadd2_rn(s1, vx);
-                s2 = q == 0 ? __fmul2_rn(vx, dx) : __ffma2_rn(vx, dx, s2);
-                if (kAbs) {   // (v first: a pixel that is far out must not meet a conic of any size)
-                    const float2 gx = __ffma2_rn(make_float2(2.f * B.x, 2.f * B.x), vx, __fmul2_rn(make_float2(bdy, bdy), v[q]));
-                    const float2 gy = __ffma2_rn(make_float2(B.y, B.y), vx, __fmul2_rn(make_float2(2.f * B.z * dy, 2.f * B.z * dy), v[q]));
-                    ax = __fadd2_rn(ax, make_float2(fabsf(gx.x), fabsf(gx.y)));
-                    ay = __fadd2_rn(ay, make_float2(fabsf(gy.x), fabsf(gy.y)));
+                    for (int q = 0; q < P2; ++q) {
+                        if (capped & (1u << (2 * q))) v[q].x = 0.f;
+                        if (capped & (2u << (2 * q))) v[q].y = 0.f;
+                    }
                 }
-            }
-            // sigma's derivatives: v_sigma = -v; the factors that are the same for every
-            // pixel follow when the totals are written
-            float sum[CDIM + kGeo];
+                float2 s0 = make_float2(0.f, 0.f), s1 = s0, s2 = s0, ax = s0, ay = s0;
 #pragma unroll
-            for (int k = 0; k < CDIM; ++k) sum[k] = csum[k].x + csum[k].y;
-            const float m0 = s0.x + s0.y, m1 = s1.x + s1.y, my = dy * m0;
-            const float gx = 2.f * B.x * m1 + B.y * my, gy = B.y * m1 + 2.f * B.z * my;
-            sum[CDIM + 0] = s2.x + s2.y;
-            sum[CDIM + 1] = dy * m1;
-            sum[CDIM + 2] = dy * my;
-            sum[CDIM + 3] = gx;
-            sum[CDIM + 4] = gy;
-            sum[CDIM + 5] = gx * roll;
-            sum[CDIM + 6] = gy * roll;
-            sum[CDIM + 7] = m0;
-            if (kAbs) {
-                sum[CDIM + 8] = ax.x + ax.y;
-                sum[CDIM + 9] = ay.x + ay.y;
-            }
-            const float2 id = sId[t];
-            const size_t gg = (size_t)__float_as_int(id.x);
-            float sums[kSums];
+                for (int q = 0; q < P2; ++q) {
+                    const float2 dx = __fadd2_rn(make_float2(mx, mx), npx[q]), vx = __fmul2_rn(v[q], dx);
+                    s0 = q == 0 ? v[q] : __fadd2_rn(s0, v[q]);
+                    s1 = q == 0 ? vx : __fadd2_rn(s1, vx);
+                    s2 = q == 0 ? __fmul2_rn(vx, dx) : __ffma2_rn(vx, dx, s2);
+                    if (kAbs) {   // (v first: a pixel that is far out must not meet a conic of any size)
+                        const float2 gx = __ffma2_rn(make_float2(2.f * B.x, 2.f * B.x), vx, __fmul2_rn(make_float2(bdy, bdy), v[q]));
+                        const float2 gy = __ffma2_rn(make_float2(B.y, B.y), vx, __fmul2_rn(make_float2(2.f * B.z * dy, 2.f * B.z * dy), v[q]));
+                        ax = __fadd2_rn(ax, make_float2(fabsf(gx.x), fabsf(gx.y)));
+                        ay = __fadd2_rn(ay, make_float2(fabsf(gy.x), fabsf(gy.y)));
+                    }
+                }
+                // sigma's derivatives: v_sigma = -v; the factors that are the same for every
+                // pixel follow when the totals are written
+                float sum[CDIM + kGeo];
 #pragma unroll
-            for (int k = 0; k < kSums; ++k) sums[k] = sum[k];
-            slot_a.add(gg, warp_sum_values<kSums, 16>(sums, lane), id.y, mine_a.writes);
-            if (kSplit) {
-                float geo[kGeo];
+                for (int k = 0; k < CDIM; ++k) sum[k] = csum[k].x + csum[k].y;
+                const float m0 = s0.x + s0.y, m1 = s1.x + s1.y, my = dy * m0;
+                const float gx = 2.f * B.x * m1 + B.y * my, gy = B.y * m1 + 2.f * B.z * my;
+                sum[CDIM + 0] = s2.x + s2.y;
+                sum[CDIM + 1] = dy * m1;
+                sum[CDIM + 2] = dy * my;
+                sum[CDIM + 3] = gx;
+                sum[CDIM + 4] = gy;
+                sum[CDIM + 5] = gx * roll;
+                sum[CDIM + 6] = gy * roll;
+                sum[CDIM + 7] = m0;
+                if (kAbs) {
+                    sum[CDIM + 8] = ax.x + ax.y;
+                    sum[CDIM + 9] = ay.x + ay.y;
+                }
+                const float2 id = sId[t];
+                const size_t gg = (size_t)__float_as_int(id.x);
+                float sums[kSums];
 #pragma unroll
-                for (int k = 0; k < kGeo; ++k) geo[k] = sum[CDIM + k];
-                const float geo_total = warp_sum_values<kGeo, 16>(geo, lane);
-                const SumSlot mine_b = sum_slot<kGeo>(lane);
-                const GradSlot slot_b = pixel_grad_slot<kAbs>(CDIM + mine_b.value, CDIM, channels, v_colors, v_conics,
-                                                              v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
-                slot_b.add(gg, geo_total, id.y, mine_b.writes);
+                for (int k = 0; k < kSums; ++k) sums[k] = sum[k];
+                slot_a.add(gg, warp_sum_values<kSums, 16>(sums, lane), id.y, mine_a.writes);
+                if (kSplit) {
+                    float geo[kGeo];
+#pragma unroll
+                    for (int k = 0; k < kGeo; ++k) geo[k] = sum[CDIM + k];
+                    const float geo_total = warp_sum_values<kGeo, 16>(geo, lane);
+                    const SumSlot mine_b = sum_slot<kGeo>(lane);
+                    const GradSlot slot_b = pixel_grad_slot<kAbs>(CDIM + mine_b.value, CDIM, channels, v_colors, v_conics,
+                                                                  v_means2d, v_pix_vels, v_opacities, v_means2d_abs);
+                    slot_b.add(gg, geo_total, id.y, mine_b.writes);
+                }
             }
         }
     }
@@ -2486,10 +2677,13 @@ static bool many_entries(float spread, int64_t entries, int64_t line, float or_s
 // and 99; 16320, 26 and 198 (5 k) 271 and 246, 41 and 312 (13 k) 236 and 256; 10800, 19 and 357 (7 k) 211 and 195, 36 and 671 (24 k) 152 and 177; 5700, 12 and 507 (6 k) 138 and
 // 125, 20 and 868 (17 k) 119 and 127. Fewer tiles: 3510, 13 and 564 (7 k) 91 and 78, 24 and 1066 (26 k) 80 and 78, 57 and 2540 60 and 68; 2040, 16 and 704 (11 k)
 // 62 and 56, 36 and 1614 (58 k) 43 and 50; 1840, 25 and 1807 (45 k) 40 and 41; 1450, 79 and 3643 (288 k) 23 and 21.
-static bool covers_patches(uint64_t blocks, uint32_t tile_size, float spread, int64_t entries) {
+// Backward, without and with runs: 8160, 16 and 682 (11 k) 338 and 334, 28 and 1190 305 and 287, 130 and 5800 195 and 180; 16320, 26 and 198 (5 k) 532 and 553, 41
+// and 312 (13 k) 532 and 526; 10800, 36 and 671 373 and 350; 3510, 13 and 564 (7 k) 174 and 167, 24 and 1066 (26 k) 170 and 150; 2040, 16 and 704 (11 k) 115
+// and 117, 36 and 1614 (58 k) 103 and 106; 1840, 12 and 829 (10 k) 105 and 111; 1450, 27 and 1171 (31 k) 70 and 64; 920, 18 and 794 (14 k) 60 and 55.
+static bool covers_patches(uint64_t blocks, uint32_t tile_size, float spread, int64_t entries, bool backward) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
-    return tiles >= 1800u && entries > 0 && tile_threads<8>(tile_size) % 32u == 0u &&
-           (double)spread * (double)entries >= (tiles >= 5000u ? 12500.0 : 30000.0) * tiles;
+    return tiles >= (backward ? 900u : 1800u) && entries > 0 && tile_threads<8>(tile_size) % 32u == 0u &&
+           (double)spread * (double)entries >= (backward || tiles >= 5000u ? 12500.0 : 30000.0) * tiles;
 }
 static uint32_t pixels_per_lane_fwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread, int64_t entries) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
@@ -2623,7 +2817,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     }
 #define CALL(D)                                                                                   \
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2)) else if (D <= 16 && px == 4) CALL_PX(D, (D <= 16 ? 4 : 2)) else CALL_PX(D, 2)
-    const bool runs = channels <= 4 && covers_patches(blocks, tile_size, hint.spread, hint.entries);
+    const bool runs = channels <= 4 && covers_patches(blocks, tile_size, hint.spread, hint.entries, false);
     const uint32_t px = runs ? 8u : pixels_per_lane_fwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool vec = channels % 4u == 0u && (reinterpret_cast<uintptr_t>(colors) & 15u) == 0u;
     {
@@ -2682,8 +2876,9 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
                 tile_size * tile_size, samples, channels);
 #define CALL_PX(D, P, A)                                                                          \
     {                                                                                             \
-        const auto kernel = has_other_bwd(D, P) && other ? rasterize_to_pixels_bwd_kernel<D, P, A, has_other_bwd(D, P)> \
-                                                         : rasterize_to_pixels_bwd_kernel<D, P, A, false>; \
+        const auto kernel = P == 8 && runs ? rasterize_to_pixels_bwd_kernel<D, P, A, (P == 8 ? kRunsBwd : kPlainBwd)> \
+                          : has_other_bwd(D, P) && other ? rasterize_to_pixels_bwd_kernel<D, P, A, (has_other_bwd(D, P) ? kOtherBwd : kPlainBwd)> \
+                                                         : rasterize_to_pixels_bwd_kernel<D, P, A, kPlainBwd>; \
         const uint32_t patches = div_up(tile_threads<P>(tile_size), 32);                          \
         SPL_REQUIRE((uint64_t)blocks * patches <= 0x7fffffffull, SPLATAD_ERR_BAD_ARG, "rasterize_to_pixels_bwd: too many tiles"); \
         launch_chained(kernel, blocks * patches, 32, 0, (cudaStream_t)stream,                     \
@@ -2697,7 +2892,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2), A) else if (D <= 20 && px == 4) CALL_PX(D, (D <= 20 ? 4 : 2), A) else CALL_PX(D, 2, A)
 #define CALL(D)                                                                                   \
     if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)
-    const uint32_t px = pixels_per_lane_bwd(blocks, tile_size, channels, hint.spread, hint.entries);
+    const bool runs = channels <= 4 && covers_patches(blocks, tile_size, hint.spread, hint.entries, true);
+    const uint32_t px = runs ? 8u : pixels_per_lane_bwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool other = pixels_bwd_other(blocks, tile_size, channels, px, hint.spread);
     {
         SPL_PROF("rasterize_to_pixels_bwd_kernel", (cudaStream_t)stream);

@@ -476,12 +476,12 @@ def test_pixels_by_how_many_tiles_a_gaussian_covers(C, ts, channels, absgrad):
                         ref["v_means2d_abs"].reshape(C, 60, 2))
 
 
-@pytest.mark.parametrize("C,W,H,ts,channels,sigma_px,N", [
-    (30, 127, 133, 16, 3, (20.0, 90.0), 150), (84, 132, 131, 16, 4, (20.0, 90.0), 90), (30, 128, 128, 16, 1, (3.0, 60.0), 200),
-    (84, 121, 120, 16, 2, (60.0, 400.0), 64), (24, 131, 129, 32, 4, (10.0, 90.0), 150), (110, 130, 130, 24, 3, (20.0, 90.0), 90)])
-def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N):
+@pytest.mark.parametrize("C,W,H,ts,channels,sigma_px,N,absgrad", [
+    (30, 127, 133, 16, 3, (20.0, 90.0), 150, False), (84, 132, 131, 16, 4, (20.0, 90.0), 90, True), (30, 128, 128, 16, 1, (3.0, 60.0), 200, True),
+    (84, 121, 120, 16, 2, (60.0, 400.0), 64, False), (24, 131, 129, 32, 4, (10.0, 90.0), 150, False), (110, 130, 130, 24, 3, (20.0, 90.0), 90, False)])
+def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, absgrad):
     """Scenes of large Gaussians: entries that cover a patch go through without a test in the kernel for them, which the hint
-    chooses; images, alphas and last positions are those of the kernel without runs, bit for bit, and match the oracle. Opaque
+    chooses; images, alphas and last positions are those of the kernel without runs, bit for bit, and match the oracle, as the gradients do. Opaque
     and capped entries, needles, a flat conic and ones that cover part of a patch among them."""
     from oracle import composite
     from splatad_b200 import _lib
@@ -492,28 +492,41 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N):
     q[:, 2] = torch.tensor([1e-4, 0.99e-4, 1e-4])     # as narrow, but large
     c["opacities"][:, 3] = 0.9985
     c["opacities"][:, 4:9] = 0.02
-    args = [n(c[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")] + [n(c["rs"]), None, W, H, ts, c["offsets"], c["flatten_ids"]]
-    want = composite.rasterize_to_pixels_fwd(*args, amb_tol=1e-4)
-    ok = ~want["ambiguous"]
+    keys = ("means2d", "conics", "colors", "opacities", "pix_vels")
+    args = [n(c[k]) for k in keys] + [n(c["rs"]), None, W, H, ts, c["offsets"], c["flatten_ids"]]
+    want, exact = composite.rasterize_to_pixels_fwd(*args, amb_tol=1e-4), composite.rasterize_to_pixels_fwd(*args, dtype=np.float64)
+    ok = ~want["ambiguous"] & (want["last_ids"] == exact["last_ids"])
     assert ok.mean() > 0.9
+    g = torch.Generator().manual_seed(5)
+    v_c, v_a = (torch.randn(C, H, W, k, generator=g) * torch.from_numpy(ok[..., None]) for k in (channels, 1))
+    ref = composite.rasterize_to_pixels_bwd(*args, exact["render_alphas"], exact["last_ids"], n(v_c), n(v_a), absgrad=absgrad)
     lib, p = _lib.load(), _lib.ptr
-    dev = {k: t(c[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels", "rs")}
+    dev = {k: t(c[k]) for k in keys + ("rs",)}
     offsets, ids = t(c["offsets"], torch.int32), t(c["flatten_ids"], torch.int32)
     th, tw = c["offsets"].shape[1:]
-    first = None
+    head = (C, ids.numel(), *(p(dev[k]) for k in keys[:3]), channels, p(dev["opacities"]), p(dev["pix_vels"]), p(dev["rs"]), None, W, H, ts,
+            tw, th, p(offsets), p(ids))
+    cotangents, first = (v_c.to(DEV), v_a.to(DEV)), None
     for spread, count in ((0.0, 0), (100.0, 10**8)):
         image, alphas = torch.empty(C, H, W, channels, device=DEV), torch.empty(C, H, W, 1, device=DEV)
         last = torch.empty(C, H, W, dtype=torch.int32, device=DEV)
         lib.splatad_rasterize_set_spread_hint(spread, count)
-        _lib.call("splatad_rasterize_to_pixels_fwd", C, ids.numel(), p(dev["means2d"]), p(dev["conics"]), p(dev["colors"]), channels,
-                  p(dev["opacities"]), p(dev["pix_vels"]), p(dev["rs"]), None, W, H, ts, tw, th, p(offsets), p(ids), p(image), p(alphas),
-                  p(last), _lib.stream_ptr(ids.device))
+        _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last), _lib.stream_ptr(ids.device))
         if first is None:
             first = image, alphas, last
             assert_close("image", n(image), want["render_colors"], 1e-4, 1e-5, mask=ok[..., None])
             assert (n(last) == want["last_ids"])[ok].all()
-        for got, ref in zip((image, alphas, last), first):
-            assert torch.equal(got, ref)
+        for got, expect in zip((image, alphas, last), first):
+            assert torch.equal(got, expect)
+        v = {k: torch.zeros_like(dev[k]) for k in keys}
+        v_abs = torch.zeros_like(dev["means2d"]) if absgrad else None
+        lib.splatad_rasterize_set_spread_hint(spread, count)
+        _lib.call("splatad_rasterize_to_pixels_bwd", *head, p(alphas), p(last), p(cotangents[0]), p(cotangents[1]), p(v_abs),
+                  *(p(v[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")), _lib.stream_ptr(ids.device))
+        for k in keys:
+            _grad_check(f"spread {spread} v_{k}", v[k], ref["v_" + k].reshape(v[k].shape))
+        if absgrad:
+            _grad_check(f"spread {spread} absgrad", v_abs, ref["v_means2d_abs"].reshape(v_abs.shape))
 
 
 @pytest.mark.parametrize("C,channels", [(24, 3), (43, 4), (84, 2), (24, 13), (12, 30)])
