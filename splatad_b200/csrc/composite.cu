@@ -1699,10 +1699,10 @@ __device__ __forceinline__ GradSlot pixel_grad_slot(int slot, int cdim, uint32_t
 //   tiles 362 / 506 -> 371 / 512.
 //   Two pixels, 9 to 16 channels, many tiles: 96 registers. 1920 x 1080, 2.5 and 27.5 tiles per Gaussian 442, 875 -> 404, 834; 640 x 360,
 //   5.1 tiles 153 -> 158.
-//   Up to four channels, scenes of large Gaussians (kRunsBwd, chosen as in the forward kernel): what is staged moves up to the front, so that
+//   Up to sixteen channels, scenes of large Gaussians (kRunsBwd, chosen as in the forward kernel): what is staged moves up to the front, so that
 // entries that cover the patch follow one another without a look at a mask, a threshold or a pixel's first entry - the place of the next one is known -,
-// two at a time with one butterfly for their 24 sums, whose five steps are the longest chain there is. 200 M -> 180 M warp instructions, 1920 x
-// 1080 305 -> 287 us, three cameras 366 -> 335. Neither more warps (96 registers, the cotangents in shared memory: 20 an SM, 344) nor fewer (one entry at a time
+// two at a time up to eight channels with one butterfly for their 24 or 32 sums, whose five steps are the longest chain there is. 4 channels: 200 M -> 180 M warp
+// instructions, 1920 x 1080 305 -> 287 us, three cameras 366 -> 335; 8 channels 475 -> 448 and 475 -> 438; 14 channels, one at a time, 682 -> 661 and 683 -> 650. Neither more warps (96 registers, the cotangents in shared memory: 20 an SM, 344) nor fewer (one entry at a time
 // with 128 registers, 16: 337) nor the order of the additions helps: at 12 warps an SM the FP32 pipe is busy 55 % of the time, the
 // exponentials and reciprocals (8 cycles each) 30 %, shuffles (4 cycles an SM) 25 %.
 //   Above 20 channels, few tiles: the chain of the longest list counts, so no spills, whole rows at once and the skip. 640 x 360, 32
@@ -1713,9 +1713,10 @@ constexpr bool pixels_bwd_skips(int cdim, int px, bool other) { return other && 
 // registers per thread, by measurement (4 channels, eight pixels: 335 us at 128, 348 at 112, 361 at 144; 16 channels:
 // 386 at 168, 394 at 128; 8: 483 at 96, 520 at 128; 20, four pixels: 847 at 168, 980 at 200; 32: 1950 at 128, 2075 at 160)
 constexpr int kPlainBwd = 0, kOtherBwd = 1, kRunsBwd = 2;
+constexpr bool has_runs_bwd(int cdim, int px) { return px == 8 || (px == 4 && cdim > 4 && cdim <= 16); }
 constexpr int pixels_bwd_regs(int cdim, int px, int kind) {
     const bool other = kind == kOtherBwd;
-    if (kind == kRunsBwd) return 168;
+    if (kind == kRunsBwd) return px == 4 && cdim <= 8 ? 128 : 168;
     return cdim <= 4 ? (px == 8 ? 128 : px == 4 ? 80 : 72) : cdim <= 8 ? (px == 4 ? 96 : 88) : cdim <= 16 ? (px == 4 ? 168 : other ? 96 : 104)
                      : cdim <= 20 ? 168 : other ? 168 : 128;
 }
@@ -1833,8 +1834,8 @@ rasterize_to_pixels_bwd_kernel(
         __shared__ float4 sEntry[32 * kEntry / 16];   // x, y, vx, vy | scaled conic, opacity | channels, zeros behind them
         const uint32_t entries = smem_register(sEntry), ids = smem_register(sId);
         // two entries' sums: colours and geometry of the first, then of the second
-        static_assert(2 * kSums <= 32, "a lane for every sum of two entries");
-        const SumSlot mine_two = sum_slot<2 * kSums>(lane);
+        constexpr bool kTwo = 2 * kSums <= 32;
+        const SumSlot mine_two = sum_slot<kTwo ? 2 * kSums : kSums>(lane);
         const uint32_t two_entry = mine_two.value >= kSums ? 1u : 0u;
         const GradSlot slot_two = pixel_grad_slot<kAbs>(mine_two.value - (two_entry ? kSums : 0), CDIM, channels, v_colors, v_conics, v_means2d,
                                                         v_pix_vels, v_opacities, v_means2d_abs);
@@ -1981,8 +1982,9 @@ rasterize_to_pixels_bwd_kernel(
                     t_event = next_event(t + 1u);
                 }
                 const uint32_t rest = ~full >> t, end = min(t_event, rest ? t + (uint32_t)__ffs(rest) - 1u : n);
-                for (; t + 1u < end; t += 2u) process(t, std::integral_constant<int, 2>(), std::true_type());
-                if (t < end) process(t++, std::integral_constant<int, 1>(), std::true_type());
+                if constexpr (kTwo)
+                    for (; t + 1u < end; t += 2u) process(t, std::integral_constant<int, 2>(), std::true_type());
+                for (; t < end;) process(t++, std::integral_constant<int, 1>(), std::true_type());
                 if (t < t_event && t < n) process(t++, std::integral_constant<int, 1>(), std::false_type());
             }
         }
@@ -2876,7 +2878,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
                 tile_size * tile_size, samples, channels);
 #define CALL_PX(D, P, A)                                                                          \
     {                                                                                             \
-        const auto kernel = P == 8 && runs ? rasterize_to_pixels_bwd_kernel<D, P, A, (P == 8 ? kRunsBwd : kPlainBwd)> \
+        const auto kernel = has_runs_bwd(D, P) && runs ? rasterize_to_pixels_bwd_kernel<D, P, A, (has_runs_bwd(D, P) ? kRunsBwd : kPlainBwd)> \
                           : has_other_bwd(D, P) && other ? rasterize_to_pixels_bwd_kernel<D, P, A, (has_other_bwd(D, P) ? kOtherBwd : kPlainBwd)> \
                                                          : rasterize_to_pixels_bwd_kernel<D, P, A, kPlainBwd>; \
         const uint32_t patches = div_up(tile_threads<P>(tile_size), 32);                          \
@@ -2892,8 +2894,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2), A) else if (D <= 20 && px == 4) CALL_PX(D, (D <= 20 ? 4 : 2), A) else CALL_PX(D, 2, A)
 #define CALL(D)                                                                                   \
     if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)
-    const bool runs = channels <= 4 && covers_patches(blocks, tile_size, hint.spread, hint.entries, true);
-    const uint32_t px = runs ? 8u : pixels_per_lane_bwd(blocks, tile_size, channels, hint.spread, hint.entries);
+    const bool runs = covers_patches(blocks, tile_size, hint.spread, hint.entries, true);
+    const uint32_t px = runs && channels <= 4 ? 8u : pixels_per_lane_bwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool other = pixels_bwd_other(blocks, tile_size, channels, px, hint.spread);
     {
         SPL_PROF("rasterize_to_pixels_bwd_kernel", (cudaStream_t)stream);

@@ -478,7 +478,8 @@ def test_pixels_by_how_many_tiles_a_gaussian_covers(C, ts, channels, absgrad):
 
 @pytest.mark.parametrize("C,W,H,ts,channels,sigma_px,N,absgrad", [
     (30, 127, 133, 16, 3, (20.0, 90.0), 150, False), (84, 132, 131, 16, 4, (20.0, 90.0), 90, True), (30, 128, 128, 16, 1, (3.0, 60.0), 200, True),
-    (84, 121, 120, 16, 2, (60.0, 400.0), 64, False), (24, 131, 129, 32, 4, (10.0, 90.0), 150, False), (110, 130, 130, 24, 3, (20.0, 90.0), 90, False)])
+    (84, 121, 120, 16, 2, (60.0, 400.0), 64, False), (24, 131, 129, 32, 4, (10.0, 90.0), 150, False), (110, 130, 130, 24, 3, (20.0, 90.0), 90, False),
+    (30, 127, 133, 16, 7, (20.0, 90.0), 90, True), (30, 132, 131, 16, 14, (10.0, 90.0), 90, False)])
 def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, absgrad):
     """Scenes of large Gaussians: entries that cover a patch go through without a test in the kernel for them, which the hint
     chooses; images, alphas and last positions are those of the kernel without runs, bit for bit, and match the oracle, as the gradients do. Opaque
