@@ -141,12 +141,35 @@ constexpr uint32_t kSeenEntry = 1u, kCarefulEntry = 2u, kOddEntry = 4u, kFullEnt
 // whether its alphas need looking at one by one (kCarefulEntry: a sigma that could come out negative, an alpha above the
 // cap), and whether it is one for odd_pixels_fwd() (kOddEntry). The alphas of the others need no test but the one
 // against 1/255: with ac - b^2 >= 1e-5 ac the form a dx^2 + 2 b dx dy + c dy^2 is at least 5e-6 (a dx^2 + c dy^2), ten times
-// what its rounding can take away, and an opacity within the cap keeps every alpha there. Not even that one where every pixel
-// of the patch blends the entry (kFullEntry): sigma is convex, so that the corners of the box bound it from above, and with
-// ac - b^2 >= 0.05 ac its terms are at most forty times itself, which leaves their rounding a tenth of the margin. `most` bounds the
-// alphas in the patch, by the least sigma where that holds, else by the opacity. (kBounds: the last two.) The mean moves with the row's shutter time; roll_lo / roll_hi bound it over the tile.
-template <bool kMarkOdd, bool kBounds>
-__device__ __forceinline__ uint32_t patch_sees(const PixelEntry &e, const PatchBox &box, float roll_lo, float roll_hi, float &most) {
+// what its rounding can take away, and an opacity within the cap keeps every alpha there. The mean moves with the
+// row's shutter time; roll_lo / roll_hi bound it over the tile.
+template <bool kMarkOdd>
+__device__ __forceinline__ uint32_t patch_sees(const PixelEntry &e, const PatchBox &box, float roll_lo, float roll_hi) {
+    const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
+    if (test.never) return 0u;
+    const float mx_a = e.A.x + roll_lo * e.A.z, mx_b = e.A.x + roll_hi * e.A.z;
+    const float my_a = e.A.y + roll_lo * e.A.w, my_b = e.A.y + roll_hi * e.A.w;
+    const float mx_lo = fminf(mx_a, mx_b), mx_hi = fmaxf(mx_a, mx_b);
+    const float my_lo = fminf(my_a, my_b), my_hi = fmaxf(my_a, my_b);
+    uint32_t seen = 0u;
+    if (kMarkOdd) {   // a NaN somewhere, an opacity without bound, a conic too flat or too steep
+        const bool plain = fabsf(e.B.x) > 1e-30f && fabsf(e.B.x) + fabsf(e.B.y) + fabsf(e.B.z) < 1e30f;
+        if (!plain || !(mx_lo <= mx_hi) || !(my_lo <= my_hi) || !(test.s_max < 1e30f)) seen = kOddEntry;
+    }
+    const float ac = e.B.x * e.B.z;
+    const bool sized = e.B.x > 1e-15f && e.B.z > 1e-15f && e.B.x < 1e15f && e.B.z < 1e15f;   // nothing under- or overflows
+    if (!(sized && ac - e.B.y * e.B.y >= 1e-5f * ac && e.B.w <= kAlphaMax)) seen |= kCarefulEntry;
+    if (box.x0 <= box.x1 && !test.misses(mx_lo - box.x1, mx_hi - box.x0, my_lo - box.y1, my_hi - box.y0)) seen |= kSeenEntry;
+    else seen &= kOddEntry;
+    return seen;
+}
+
+// The same, and whether every pixel of the patch blends the entry and needs no other care (kFullEntry): sigma is convex, so that the
+// corners of the box bound it from above, and with ac - b^2 >= 0.05 ac its terms are at most forty times itself, which leaves their
+// rounding a tenth of the margin. `most` bounds the alphas in the patch, by the least sigma where that holds, else by the opacity. (One
+// function for both, the other kernels are 1 % slower; the bounds in one of their own, these are 3 %.)
+template <bool kMarkOdd>
+__device__ __forceinline__ uint32_t patch_covered(const PixelEntry &e, const PatchBox &box, float roll_lo, float roll_hi, float &most) {
     const BoxTest test(e.B.x, e.B.y, e.B.z, e.B.w);
     if (test.never) return 0u;
     const float mx_a = e.A.x + roll_lo * e.A.z, mx_b = e.A.x + roll_hi * e.A.z;
@@ -162,12 +185,7 @@ __device__ __forceinline__ uint32_t patch_sees(const PixelEntry &e, const PatchB
     const bool sized = e.B.x > 1e-15f && e.B.z > 1e-15f && e.B.x < 1e15f && e.B.z < 1e15f;   // nothing under- or overflows
     if (!(sized && det >= 1e-5f * ac && e.B.w <= kAlphaMax)) seen |= kCarefulEntry;
     const float x0 = mx_lo - box.x1, x1 = mx_hi - box.x0, y0 = my_lo - box.y1, y1 = my_hi - box.y0;
-    if (!kBounds) {
-        if (box.x0 <= box.x1 && !test.misses(x0, x1, y0, y1)) seen |= kSeenEntry;
-        else seen &= kOddEntry;
-        return seen;
-    }
-    const float lowest = BoxTest::with_margin(test.lowest(x0, x1, y0, y1));
+    const float lowest = test.lowest(x0, x1, y0, y1);
     if (!(box.x0 <= box.x1) || lowest > test.s_max) return seen & kOddEntry;
     most = fminf(kAlphaMax, det >= 0.05f * ac ? e.B.w * __expf(-lowest) : e.B.w);
     const float xx = 0.5f * e.B.x * fmaxf(x0 * x0, x1 * x1), yy = 0.5f * e.B.z * fmaxf(y0 * y0, y1 * y1);
@@ -668,7 +686,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX, kRuns)) rasterize_to_pixel
             if (idx < range.end) {
                 e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
                 if (idx + 32 < range.end) next_id = flatten_ids[idx + 32];   // on its way meanwhile
-                seen = patch_sees<true, true>(e, box, roll_lo, roll_hi, most);
+                seen = patch_covered<true>(e, box, roll_lo, roll_hi, most);
             }
             // The entries to be looked at move up to the front; n of them, bit t of the masks for the one in place t
             const uint32_t kept = __ballot_sync(0xffffffffu, seen != 0u), n = __popc(kept);
@@ -826,8 +844,7 @@ __global__ void __maxnreg__(pixels_fwd_regs(CDIM, PX, kRuns)) rasterize_to_pixel
             if (idx < range.end) {
                 e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
                 if (idx + 32 < range.end) next_id = flatten_ids[idx + 32];   // on its way meanwhile
-                float most;
-                seen = patch_sees<true, false>(e, box, roll_lo, roll_hi, most);
+                seen = patch_sees<true>(e, box, roll_lo, roll_hi);
             }
             uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
             const uint32_t careful = __ballot_sync(0xffffffffu, seen > kSeenEntry);
@@ -1849,7 +1866,7 @@ rasterize_to_pixels_bwd_kernel(
             if (idx >= range.start) {
                 e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
                 if (idx - 32 >= range.start) next_id = flatten_ids[idx - 32];   // on its way meanwhile
-                seen = patch_sees<false, true>(e, box, roll_lo, roll_hi, most);
+                seen = patch_covered<false>(e, box, roll_lo, roll_hi, most);
             }
             const uint32_t kept = __ballot_sync(0xffffffffu, seen != 0u), n = __popc(kept);
             const uint32_t place = __popc(kept & ((1u << lane) - 1u));
@@ -1998,12 +2015,11 @@ rasterize_to_pixels_bwd_kernel(
             const int32_t idx = batch_end - (int32_t)lane;
             const int32_t g = next_id;
             uint32_t seen = 0u;
-            float most;
             PixelEntry e;
             if (idx >= range.start) {
                 e = load_pixel_entry(g, means2d, conics, opacities, pix_vels);
                 if (idx - 32 >= range.start) next_id = flatten_ids[idx - 32];   // on its way meanwhile
-                seen = patch_sees<false, false>(e, box, roll_lo, roll_hi, most);
+                seen = patch_sees<false>(e, box, roll_lo, roll_hi);
             }
             uint32_t todo = __ballot_sync(0xffffffffu, seen != 0u);
             const uint32_t careful = __ballot_sync(0xffffffffu, (seen & kCarefulEntry) != 0u);

@@ -39,9 +39,8 @@ struct BoxTest {
         slope_x = __fdividef(-b, c);                       // minimiser over dy on an edge dx = X: slope_x * X
         slope_y = __fdividef(-b, a);
     }
-    // Sigma is nowhere less in the box, but for rounding; -INF where there is no telling.
-    __device__ __forceinline__ float lowest(float dx_lo, float dx_hi, float dy_lo, float dy_hi) const {
-        if (always || !(dx_lo <= dx_hi && dy_lo <= dy_hi)) return -INFINITY;   // NaN offsets
+    // The least sigma in a box of numbers, of a positive definite conic, but for rounding.
+    __device__ __forceinline__ float nearest(float dx_lo, float dx_hi, float dy_lo, float dy_hi) const {
         const float X = fminf(fmaxf(0.f, dx_lo), dx_hi), Y = fminf(fmaxf(0.f, dy_lo), dy_hi);
         const float y = fminf(fmaxf(slope_x * X, dy_lo), dy_hi);
         const float x = fminf(fmaxf(slope_y * Y, dx_lo), dx_hi);
@@ -49,9 +48,15 @@ struct BoxTest {
         const float s_y = 0.5f * (a * x * x + c * Y * Y) + b * x * Y;
         return fminf(s_x, s_y);
     }
-    static __device__ __forceinline__ float with_margin(float lowest) { return lowest * 0.999f - 1e-3f; }
+    // It less a margin; -INF where there is no telling.
+    __device__ __forceinline__ float lowest(float dx_lo, float dx_hi, float dy_lo, float dy_hi) const {
+        if (always || !(dx_lo <= dx_hi && dy_lo <= dy_hi)) return -INFINITY;   // NaN offsets
+        return nearest(dx_lo, dx_hi, dy_lo, dy_hi) * 0.999f - 1e-3f;
+    }
     __device__ __forceinline__ bool misses(float dx_lo, float dx_hi, float dy_lo, float dy_hi) const {
-        return never || with_margin(lowest(dx_lo, dx_hi, dy_lo, dy_hi)) > s_max;
+        if (never) return true;
+        if (always || !(dx_lo <= dx_hi && dy_lo <= dy_hi)) return false;   // NaN offsets
+        return nearest(dx_lo, dx_hi, dy_lo, dy_hi) * 0.999f - 1e-3f > s_max;
     }
 };
 

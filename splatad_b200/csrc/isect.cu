@@ -1118,7 +1118,7 @@ constexpr uint32_t kBlkThreads = 512, kBlkWarps = kBlkThreads / 32;   // step A:
 // Step B: a CTA takes a unit of 512 consecutive records of a block, or of 1024 where the lists are so long that they leave the cache as they
 // are written: figures at tile_scatter_kernel, whose CTAs go with it, six or two an SM.
 constexpr uint32_t kBlkUnitMin = 512, kBlkUnitMax = 1024;
-constexpr uint64_t kBlkLongLists = (800ull << 20) / 12;    // entries
+constexpr uint64_t kBlkLongLists = (800ull << 20) / 12, kBlkCachedLists = (126ull << 20) / 12;   // entries
 constexpr uint32_t kBlkWords = 2;                          // writing: 32-record groups per warp
 constexpr uint32_t kBlkCountThreads = 128;                 // counting
 constexpr uint32_t kBlkMaxPerSensor = 1024;                // blocks per sensor (32768 tiles)
@@ -1575,16 +1575,18 @@ tile_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket, int32_t *__
 
 // A CTA leaves its unit's pairs and, by tile, the bits of its records in shared memory; behind that barrier a warp puts a tile's
 // entries in order by itself - a lane takes the bits of 32 records, one scan says where its record numbers go, two bytes
-// each - and writes the run: whole sectors two entries per lane, what is left at the ends by sixteen lanes. (Before, each lane had a
+// each - and writes the run: whole sectors two entries per lane, then what is left at the ends; with units of 512 half a
+// warp each for two tiles at a time (one after the other: 56 us instead of 52 for the lidar benchmark, 18.8 instead of 16.8 where lists are short). (Before, each lane had a
 // tile, the places were summed over the warps and the runs written after another barrier: 64 KB of places for three CTAs an
 // SM. Storing straight from the lanes whose record covers a tile: 180 us for the lidar benchmark's 15.3 M entries.)
 //
 // What bounds it where the lists are long is how they reach the HBM, not the writing itself: with 592 CTAs of 1024 records 100 MB are
 // under way, and the sectors that two units write in parts are evicted between the two, and every such half costs a read
-// and about five whole sectors' time. So whole sectors leave the cache first, halves last, and two CTAs an SM are enough.
+// and about five whole sectors' time. So whole sectors leave the cache first, halves last (kStream: where the lists
+// do not stay in the cache anyway), and two CTAs an SM are enough.
 // Six cameras, 5.8 GB of lists: 1310 us before, 1390 with four CTAs an SM, 1250 with two, 1200 with two and that order of leaving (dram
 // reads 401 -> 265 MB); units of 512: 1400. Shorter lists want smaller units and more CTAs, us before and with six of 512 records, by MB of lists: 116 (camera
-// benchmark) 43.5 and 39.5, 184 (lidar benchmark) 66 and 56, 206 (three cameras) 74.5 and 60, 580 (200 k Gaussians, six cameras) 138 and 133; with two of 1024
+// benchmark) 43.5 and 38, 184 (lidar benchmark) 66 and 52, 206 (three cameras) 74.5 and 60, 580 (200 k Gaussians, six cameras) 139 and 135; with two of 1024
 // 43.6, 66, 76 and 138, but 302 instead of 338 at 1450 MB. Four entries per lane (32-byte stores): 68 instead of 58 and
 // 1430 instead of 1360, their record numbers lie in the same banks.
 __device__ __forceinline__ uint64_t keep_in_cache() {
@@ -1599,7 +1601,7 @@ __device__ __forceinline__ void store_kept(int32_t *to, uint32_t v, uint64_t pol
     asm volatile("st.global.L2::cache_hint.b32 [%0], %1, %2;" ::"l"(__cvta_generic_to_global(to)), "r"(v), "l"(policy) : "memory");
 }
 
-template <uint32_t kWarps>
+template <uint32_t kWarps, bool kStream>
 __global__ void __launch_bounds__(kWarps * 32, kWarps > 8 ? 2 : 6)
 tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restrict__ flatten_ids,
                     int64_t *__restrict__ counters) {
@@ -1654,8 +1656,9 @@ tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restr
                 const uint32_t o = __shfl_up_sync(0xffffffffu, place, off, kWords);
                 if (col >= off) place += o;
             }
-            const uint32_t total = place;   // of the last lane: the tile's entries
-            place += half * kRoom - mine + (__shfl_sync(0xffffffffu, at, l0 + half) & 7u);
+            const uint32_t begin = __shfl_sync(0xffffffffu, at, l0 + half), id = __shfl_sync(0xffffffffu, high, l0 + half);
+            const uint32_t end = min(begin + __shfl_sync(0xffffffffu, place, kWords - 1, kWords), cap);   // the last word's lane has the sum
+            place += half * kRoom - mine + (begin & 7u);
             uint16_t *out = s_out[warp];
             const auto next = [&] {
                 const uint32_t r = 32 * col + __ffs(m) - 1;
@@ -1670,34 +1673,37 @@ tile_scatter_kernel(BlkArgs a, int64_t *__restrict__ isect_ids, int32_t *__restr
             }
             if (m) out[place] = (uint16_t)next();
             __syncwarp();
-#pragma unroll
-            for (uint32_t h = 0; h < kTiles; ++h) {
-                const uint32_t begin = __shfl_sync(0xffffffffu, at, l0 + h), id = __shfl_sync(0xffffffffu, high, l0 + h);
-                const uint32_t end = min(begin + __shfl_sync(0xffffffffu, total, h * kWords + kWords - 1), cap);
-                const uint16_t *src = out + h * kRoom - (begin & ~7u);   // indexed by list position
-                if (!wide) {
-                    for (uint32_t p = begin + lane; p < end; p += 32u) {
-                        const uint2 e = s_pair[src[(int32_t)p]];
-                        isect_ids[p] = (int64_t)(((uint64_t)id << 32) | e.x);
-                        flatten_ids[p] = (int32_t)e.y;
-                    }
-                    continue;
-                }
-                // whole sectors first, then what is left at both ends
-                const uint32_t inner = (begin + 7u) & ~7u, outer = end & ~7u;
-#pragma unroll 2
-                for (uint32_t p = inner + 2u * lane; p < outer; p += 64u) {
-                    const uint32_t r = *reinterpret_cast<const uint32_t *>(src + (int32_t)p);
-                    const uint2 e = s_pair[r & 0xffffu], f = s_pair[r >> 16];
-                    __stcs(reinterpret_cast<uint4 *>(isect_ids + p), make_uint4(e.x, id, f.x, id));
-                    __stcs(reinterpret_cast<uint2 *>(flatten_ids + p), make_uint2(e.y, f.y));
-                }
-                const uint32_t p = lane < 8u ? begin + lane : max(inner, outer) + lane - 8u;
-                if (lane < 16u && p < (lane < 8u ? min(inner, end) : end)) {
-                    const uint2 e = s_pair[src[(int32_t)p]];
+            const uint16_t *src = out + half * kRoom - (begin & ~7u);   // indexed by list position
+            const auto store_one = [&](uint32_t p, bool keep) {
+                const uint2 e = s_pair[src[(int32_t)p]];
+                if (keep) {
                     store_kept(isect_ids + p, ((uint64_t)id << 32) | e.x, kept);
                     store_kept(flatten_ids + p, e.y, kept);
+                } else {
+                    isect_ids[p] = (int64_t)(((uint64_t)id << 32) | e.x);
+                    flatten_ids[p] = (int32_t)e.y;
                 }
+            };
+            if (wide) {   // whole sectors first, then what is left at both ends
+                const uint32_t inner = (begin + 7u) & ~7u, outer = end & ~7u;
+#pragma unroll 2
+                for (uint32_t p = inner + 2u * col; p < outer; p += 2u * kWords) {
+                    const uint32_t r = *reinterpret_cast<const uint32_t *>(src + (int32_t)p);
+                    const uint2 e = s_pair[r & 0xffffu], f = s_pair[r >> 16];
+                    const uint4 ids = make_uint4(e.x, id, f.x, id);
+                    const uint2 flat = make_uint2(e.y, f.y);
+                    if (kStream) {
+                        __stcs(reinterpret_cast<uint4 *>(isect_ids + p), ids);
+                        __stcs(reinterpret_cast<uint2 *>(flatten_ids + p), flat);
+                    } else {
+                        *reinterpret_cast<uint4 *>(isect_ids + p) = ids;
+                        *reinterpret_cast<uint2 *>(flatten_ids + p) = flat;
+                    }
+                }
+                const uint32_t p = col < 8u ? begin + col : max(inner, outer) + col - 8u;
+                if (col < 16u && p < (col < 8u ? min(inner, end) : end)) store_one(p, kStream);
+            } else {
+                for (uint32_t p = begin + col; p < end; p += kWords) store_one(p, false);
             }
             __syncwarp();
         }
@@ -2189,7 +2195,8 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
             SPL_PROF("tile_scatter_kernel", st);
             constexpr uint32_t kMin = kBlkUnitMin / (32 * kBlkWords), kMax = kBlkUnitMax / (32 * kBlkWords);
             const bool longer = a.unit == kBlkUnitMax;
-            auto kernel = longer ? tile_scatter_kernel<kMax> : tile_scatter_kernel<kMin>;
+            auto kernel = longer ? tile_scatter_kernel<kMax, true>
+                                 : (uint64_t)capacity > kBlkCachedLists ? tile_scatter_kernel<kMin, true> : tile_scatter_kernel<kMin, false>;
             const uint32_t grid = min(units_max, (longer ? 2u : 6u) * kNumSMs);
             // long lists: not placed while the scan still holds its SMs (six cameras: 1340 us, and 80 more chained)
             launch_chained_if(!longer, kernel, grid, a.unit / kBlkWords, 0, st, a, isect_ids, flatten_ids, p.counters);
