@@ -299,7 +299,7 @@ def test_block_split_at_the_edges_of_its_blocks(C, N, tw, th, packed):
 
 @pytest.mark.parametrize("long_lists", [False, True])
 @pytest.mark.parametrize("ids_off,flat_off", [(0, 0), (1, 0), (0, 1), (3, 2), (2, 4)])
-@pytest.mark.parametrize("C,N,tw,th", [(1, 1, 1, 1), (1, 700, 4, 8), (2, 1400, 9, 9), (1, 3000, 13, 21)])
+@pytest.mark.parametrize("C,N,tw,th", [(1, 1, 1, 1), (1, 700, 4, 8), (2, 1400, 9, 9), (1, 3000, 13, 21), (2, 900, 70, 61)])
 def test_lists_anywhere_in_memory(C, N, tw, th, ids_off, flat_off, long_lists, monkeypatch):
     """The list kernels write two entries at a time where both arrays are aligned for it, one otherwise; short and long runs of
     a tile, and room for so many entries that units of the longer kind are taken. Nothing outside the lists is written."""
@@ -313,13 +313,14 @@ def test_lists_anywhere_in_memory(C, N, tw, th, ids_off, flat_off, long_lists, m
     lists = dict(capacity=72_000_000 if long_lists else 1 << 18)
     ids = torch.full((lists["capacity"] + 16,), -7, dtype=torch.int64, device=DEV)
     flat = torch.full((lists["capacity"] + 16,), -7, dtype=torch.int32, device=DEV)
+    starts = torch.full((C * tw * th + 16,), -7, dtype=torch.int32, device=DEV)
     fill_ws = torch.empty(_lib.load().splatad_isect_fill_workspace_bytes(lists["capacity"]), dtype=torch.uint8, device=DEV)
 
     def elsewhere(name, *args):
         if name == "splatad_isect_tiles_fill":
-            *head, _, _, seen["n"], _, _, offsets, host, stream = args
+            *head, _, _, seen["n"], _, _, _, host, stream = args
             args = (*head, _lib.ptr(fill_ws), fill_ws.numel(), lists["capacity"], ids.data_ptr() + 8 * ids_off,
-                    flat.data_ptr() + 4 * flat_off, offsets, host, stream)
+                    flat.data_ptr() + 4 * flat_off, starts.data_ptr() + 4 * flat_off, host, stream)
         return call(name, *args)
 
     want = _run_cam(means2d, radii, depths, ts, tw, th)
@@ -328,8 +329,10 @@ def test_lists_anywhere_in_memory(C, N, tw, th, ids_off, flat_off, long_lists, m
     n_isects = seen["n"]
     assert n_isects == want[1].numel() > 0
     assert torch.equal(ids[ids_off: ids_off + n_isects], want[1]) and torch.equal(flat[flat_off: flat_off + n_isects], want[2])
-    for buffer, off in ((ids, ids_off), (flat, flat_off)):
-        assert (buffer[:off] == -7).all() and (buffer[off + n_isects: off + n_isects + 64] == -7).all()
+    n_tiles = C * tw * th
+    assert torch.equal(starts[flat_off: flat_off + n_tiles], want[3].flatten()) and starts[flat_off + n_tiles] == n_isects
+    for buffer, off, size in ((ids, ids_off, n_isects), (flat, flat_off, n_isects), (starts, flat_off, n_tiles + 1)):
+        assert (buffer[:off] == -7).all() and (buffer[off + size: off + size + 8] == -7).all()
 
 
 @pytest.mark.parametrize("turns", [0.3, 0.99, 1.0, 1.01, 2.4, 4.5])
