@@ -530,6 +530,55 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, 
             _grad_check(f"spread {spread} absgrad", v_abs, ref["v_means2d_abs"].reshape(v_abs.shape))
 
 
+@pytest.mark.parametrize("what", ["colors", "means2d", "conics", "opacities", "flat", "cotangent"])
+def test_runs_with_values_that_are_not_finite(what):
+    """The kernels with runs and those without them agree on the pixels that a value which is not finite reaches, on the Gaussians that
+    get such a gradient, and on all others."""
+    from splatad_b200 import _lib
+    C, W, H, ts, channels, N = 30, 128, 127, 16, 3, 90
+    c = _camera_case(C, N, W, H, ts, channels, 77, sigma_px=(15.0, 80.0))
+    if what == "flat": c["conics"][:, 5] = torch.tensor([1e-37, 0.0, 1e-37])
+    elif what != "cotangent":
+        c[what][:, 5], c[what][::2, 11] = float("nan"), float("inf")
+    g = torch.Generator().manual_seed(2)
+    v_c, v_a = torch.randn(C, H, W, channels, generator=g), torch.randn(C, H, W, 1, generator=g)
+    if what == "cotangent": v_c[::3, 40, 50, 1], v_a[1, 3, 3] = float("nan"), float("inf")
+    lib, p = _lib.load(), _lib.ptr
+    keys = ("means2d", "conics", "colors", "opacities", "pix_vels")
+    dev = {k: t(c[k]) for k in keys + ("rs",)}
+    offsets, ids, v_c, v_a = t(c["offsets"], torch.int32), t(c["flatten_ids"], torch.int32), t(v_c), t(v_a)
+    th, tw = c["offsets"].shape[1:]
+    head = (C, ids.numel(), *(p(dev[k]) for k in keys[:3]), channels, p(dev["opacities"]), p(dev["pix_vels"]), p(dev["rs"]), None, W, H, ts,
+            tw, th, p(offsets), p(ids))
+    results, hints = [], ((0.0, 0), (100.0, 10**8))
+    for hint in hints:
+        image, alphas = torch.empty(C, H, W, channels, device=DEV), torch.empty(C, H, W, 1, device=DEV)
+        last = torch.empty(C, H, W, dtype=torch.int32, device=DEV)
+        lib.splatad_rasterize_set_spread_hint(*hint)
+        _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last), _lib.stream_ptr(ids.device))
+        results.append((image, alphas, last))
+    (image, alphas, last), (image_r, alphas_r, last_r) = results
+    same = ((last & 0x7FFFFFFF) == (last_r & 0x7FFFFFFF))[..., None]
+    v_c, v_a, gradients = torch.where(same, v_c, 0.0), torch.where(same, v_a, 0.0), []
+    for hint, (_, alphas_h, last_h) in zip(hints, results):
+        grads = {k: torch.zeros_like(dev[k]) for k in keys}
+        lib.splatad_rasterize_set_spread_hint(*hint)
+        _lib.call("splatad_rasterize_to_pixels_bwd", *head, p(alphas_h), p(last_h), p(v_c), p(v_a), None,
+                  *(p(grads[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")), _lib.stream_ptr(ids.device))
+        gradients.append(grads)
+    v, v_r = gradients
+    # pixels are worked out again patch by patch, and patches differ in size: a rounding, and a decision in a few thousand, may differ
+    assert_close("alphas", n(alphas_r), n(alphas), 1e-4, 1e-5, max_bad_frac=1e-3)
+    assert same.float().mean() > 0.999
+    assert (image.isfinite() == image_r.isfinite()).float().mean() > 0.9999
+    both = image.isfinite() & image_r.isfinite()
+    assert_close("image", n(image_r), n(image), 1e-4, 1e-5, mask=n(both).astype(bool), max_bad_frac=1e-3)
+    for k in keys:
+        assert (v[k].isfinite() == v_r[k].isfinite()).float().mean() > 0.999, k
+        both = v[k].isfinite() & v_r[k].isfinite()
+        _grad_check(k, torch.where(both, v_r[k], 0.0), n(torch.where(both, v[k], 0.0)), rel=5e-3)
+
+
 @pytest.mark.parametrize("C,channels", [(24, 3), (43, 4), (84, 2), (24, 13), (12, 30)])
 def test_divided_depth_of_many_tiles(C, channels):
     """The last channel divided by the alpha inside the kernels, forward and backward, against the same division behind them,
