@@ -255,12 +255,12 @@ def _stream_key(device: torch.device) -> Tuple[int, int]:
 
 
 def acquire_pinned_slot(device: torch.device) -> torch.Tensor:
-    """A pinned 4 x int64 host slot owned by one outstanding call (its counts arrive there
+    """A pinned 10 x int64 host slot owned by one outstanding call (its counts arrive there
     asynchronously); give it back with :func:`release_pinned_slot` once it has been read. Slots are
     recycled per (device, stream): a plan copies its counters twice (the count early, everything at
     its end), and only work enqueued later on the same stream is ordered behind the second copy."""
     free = _free_slots.get(_stream_key(device))
-    slot = free.pop() if free else torch.zeros(8, dtype=torch.int64).pin_memory()
+    slot = free.pop() if free else torch.zeros(10, dtype=torch.int64).pin_memory()
     slot._splatad_stream_key = _stream_key(device)
     return slot
 
@@ -276,7 +276,7 @@ def next_sequence() -> int:
 
 
 def wait_for_count(slot: torch.Tensor, sequence: int, event: torch.cuda.Event, patience_s: float = 0.02):
-    """(n_isects, status) of a plan that was given ``slot`` (8 x int64 pinned: [0..3] the counters the
+    """(n_isects, status) of a plan that was given ``slot`` (int64 pinned: [0..3] the counters the
     plan copies at its end, [4..7] the early words {count, sequence, status, depth range}). Polls the triple for
     ``sequence`` - a kernel stores it there itself, long before the plan's own copy - and falls back to waiting for
     ``event`` (recorded behind the plan) when it does not show up within ``patience_s``."""

@@ -2703,6 +2703,9 @@ static bool covers_patches(uint64_t blocks, uint32_t tile_size, float spread, in
     return tiles >= (backward ? 900u : 1800u) && entries > 0 && tile_threads<8>(tile_size) % 32u == 0u &&
            (double)spread * (double)entries >= (backward || tiles >= 5000u ? 12500.0 : 30000.0) * tiles;
 }
+// Name of a camera kernel in the profile, with what was chosen.
+#define PIXELS_KERNEL_NAME(way, px, runs) \
+    ((runs) ? ((px) == 8u ? way "/8,runs" : way "/4,runs") : (px) == 8u ? way "/8" : (px) == 4u ? way "/4" : way "/2")
 static uint32_t pixels_per_lane_fwd(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread, int64_t entries) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
     const float line = tiles < 6000u ? 7.f : channels <= 4 ? 3.3f : channels <= 8 ? 7.f : 5.f;
@@ -2839,7 +2842,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     const uint32_t px = runs ? 8u : pixels_per_lane_fwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool vec = channels % 4u == 0u && (reinterpret_cast<uintptr_t>(colors) & 15u) == 0u;
     {
-        SPL_PROF("rasterize_to_pixels_fwd_kernel", (cudaStream_t)stream);
+        SPL_PROF(PIXELS_KERNEL_NAME("rasterize_to_pixels_fwd_kernel", channels <= 16u ? px : 2u, runs), (cudaStream_t)stream);
         SPL_DISPATCH_CDIM(channels, CALL);
     }
 #undef CALL
@@ -2914,7 +2917,8 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     const uint32_t px = runs && channels <= 4 ? 8u : pixels_per_lane_bwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool other = pixels_bwd_other(blocks, tile_size, channels, px, hint.spread);
     {
-        SPL_PROF("rasterize_to_pixels_bwd_kernel", (cudaStream_t)stream);
+        SPL_PROF(PIXELS_KERNEL_NAME("rasterize_to_pixels_bwd_kernel", channels <= 20u ? px : 2u,
+                                    runs && (px == 8u || (px == 4u && channels > 4u && channels <= 16u))), (cudaStream_t)stream);
         SPL_DISPATCH_CDIM(channels, CALL);
     }
 #undef CALL

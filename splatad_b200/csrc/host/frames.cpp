@@ -712,7 +712,7 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
                         const OptTensor &lin, const OptTensor &ang, const OptTensor &rs, double near_plane, double far_plane,
                         double radius_clip, double eps2d, int64_t sh_degree, bool packed, int64_t tile_size, const OptTensor &backgrounds,
                         int64_t mode, bool expected, bool absgrad, bool antialiased, int64_t max_channels, int64_t row_capacity,
-                        int64_t capacity, uint64_t last_range, double last_spread, int64_t last_count) {
+                        int64_t capacity, uint64_t last_range) {
     if (!means.defined() || !means.is_cuda()) return py::none();
     const c10::DeviceIndex dev = means.get_device();
     for (const Tensor *t : {&means, &quats, &scales, &opacities, &colors, &viewmats, &Ks})
@@ -833,22 +833,25 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
         f->alphas = at::empty({C, H, W, 1}, options);
         f->last_ids = at::empty({C, H, W}, ints);
         if (expected && grad) f->expected_depths = at::empty({C, H, W}, options);
-        lib.splatad_rasterize_set_spread_hint((float)last_spread, last_count);
+        // The counts first: they choose the compositing kernel, and the lists are still being written when they arrive
+        {
+            py::gil_scoped_release no_gil;
+            counts = read_counts(slot, sequence, stream);
+            if (packed) {
+                // behind the lists' count in the stream, so the rows' has arrived (or its store is about to)
+                for (uint32_t i = 0; (nnz = load_word(slot.word + 8)) < 0; ++i, pause())
+                    if ((i & 4095u) == 4095u && stream.query()) break;
+                nnz = load_word(slot.word + 8);
+            }
+        }
+        if (nnz <= 0 || nnz > rows_max || !usable(counts, capacity))
+            return py::make_tuple(nnz, counts.n_isects, counts.status, counts.depth_range, counts.listed, py::none());
+        lib.splatad_rasterize_set_spread_hint(counts.spread(), counts.n_isects);
         check(lib.splatad_rasterize_expected_to_pixels_fwd(
             (uint32_t)C, -1, F(f->means2d), F(f->conics), c, (uint32_t)channels, o, F(f->pix_vels), F(rs_t), F(bg), (uint32_t)W, (uint32_t)H,
             (uint32_t)tile_size, (uint32_t)tile_w, (uint32_t)tile_h, I(f->offsets), I(f->flatten_ids), expected, M(f->render), M(f->alphas),
             I(f->last_ids), M(f->expected_depths), stream.stream()));
-        py::gil_scoped_release no_gil;
-        counts = read_counts(slot, sequence, stream);
-        if (packed) {
-            // behind the lists' count in the stream, so the rows' has arrived (or its store is about to)
-            for (uint32_t i = 0; (nnz = load_word(slot.word + 8)) < 0; ++i, pause())
-                if ((i & 4095u) == 4095u && stream.query()) break;
-            nnz = load_word(slot.word + 8);
-        }
     }
-    if (nnz <= 0 || nnz > rows_max || !usable(counts, capacity))
-        return py::make_tuple(nnz, counts.n_isects, counts.status, counts.depth_range, counts.listed, py::none());
     f->n = nnz;
     f->spread = counts.spread();
     if (packed && nnz < rows_max)

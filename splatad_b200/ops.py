@@ -996,30 +996,33 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
                   _lib.ptr(flatten_ids), _lib.ptr(offsets), None, stream)
         return isect_ids, flatten_ids, offsets
 
-    def read_count(slot=None, sequence=0, event=None):
+    def read_count(slot=None, words=None, sequence=0, event=None):
         if slot is None:
-            n_isects, status = int(host[0]), int(host[2])
+            n_isects, status, listed = int(host[0]), int(host[2]), int(host[1])
         else:
             n_isects, status = _lib.wait_for_count(slot, sequence, event)
+            listed = int(words[9])
+            if not listed and kind == "tiles":   # not early (radix depth sort, memory that is not mapped): with the plan's own copy
+                event.synchronize()
+                listed = int(words[1])
             _lib.release_pinned_slot(slot)
         if status & 2 or n_isects > 0x7FFFFFFF:
             raise RuntimeError(f"isect: {n_isects} intersections do not fit int32 flatten ids / offsets")
         _isect_count_hint[key] = n_isects
         if status & 4 and mode[0] == 1:
             _depth_sort_mode[key] = 2
-            return -1          # the depth buckets were too crowded: the order is not final
-        return n_isects
+            return -1, 0       # the depth buckets were too crowded: the order is not final
+        return n_isects, listed if sort else 0
 
     def exact():
         plan()
         torch.cuda.current_stream(dev).synchronize()
-        n_isects = read_count()
+        n_isects, listed = read_count()
         if n_isects < 0:       # once more, with the radix depth sort
             mode[0] = 2
             plan()
             torch.cuda.current_stream(dev).synchronize()
-            n_isects = read_count()
-        listed = int(host[1]) if sort else 0
+            n_isects, listed = read_count()
         isect_ids, flatten_ids, offsets = fill(n_isects)
         if offsets is not None:
             isect_ids._splatad_tile_offsets = (C, offsets[:n_tiles_total])
@@ -1035,28 +1038,44 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
     # the count is read when the caller asks for the exact tensors.
     capacity = list_room(hint)
     slot = _lib.acquire_pinned_slot(dev)
-    # a kernel of the plan hands the count to the host itself (slot[4:6]); the event behind the plan is
-    # the fallback
+    # a kernel of the plan hands the count to the host itself (slot[4:6], the elements listed in slot[9]); the event
+    # behind the plan is the fallback
     sequence = _lib.next_sequence()
     lib.splatad_isect_set_early_count(slot.data_ptr() + 32, sequence)
+    words = slot.numpy()
+    words[9] = 0
+    lib.splatad_isect_set_listed_count(slot.data_ptr() + 72)
     try:
-        plan(slot)
-    finally:
+        plan(slot)   # takes both requests
+    except BaseException:
         lib.splatad_isect_set_early_count(None, 0)
+        lib.splatad_isect_set_listed_count(None)
+        raise
     counted = torch.cuda.Event()
     counted.record(torch.cuda.current_stream(dev))
     isect_buf, flat_buf, offsets = fill(capacity)
-    flat_buf._splatad_spread, flat_buf._splatad_count = _spread_hint.get(key, 0.0), hint
-    return DeferredIsect(tiles_per_gauss, isect_buf, flat_buf, offsets, C, n_tiles_total, capacity,
-                         counted, lambda: read_count(slot, sequence, counted), exact)
+    count = flat_buf._splatad_counts = _ReadOnce(lambda: read_count(slot, words, sequence, counted))
+    return DeferredIsect(tiles_per_gauss, isect_buf, flat_buf, offsets, C, n_tiles_total, capacity, count, exact)
 
 
 # (kind, shape, tile grid, device, stream) -> intersection count of the last frame of that shape on
 # that stream (see _packed_nnz_hint for why the stream is part of the key)
 _isect_count_hint: dict = {}
 _depth_range_hint: dict = {}    # per frame shape and stream: (lo bits, hi bits) of the last frame's listed depths
-_spread_hint: dict = {}         # same keys -> list entries per listed Gaussian of the last frame
+_spread_hint: dict = {}         # same keys -> list entries per listed Gaussian of the last frame, for whoever wants to know: no frame goes by it
 _depth_sort_mode: dict = {}   # same keys -> 2 once a frame of the shape needed the radix depth sort
+
+
+class _ReadOnce:
+    """(list entries, elements listed) of a plan, read when first asked for: whoever asks waits until they are there."""
+
+    def __init__(self, read):
+        self._read, self._value = read, None
+
+    def __call__(self):
+        if self._value is None:
+            self._value = self._read()
+        return self._value
 
 
 class DeferredIsect:
@@ -1069,20 +1088,18 @@ class DeferredIsect:
     from this object has to be repeated.
     """
 
-    def __init__(self, tiles_per_gauss, isect_buf, flat_buf, offsets, C, n_tiles_total, capacity, counted,
-                 read_count, exact):
+    def __init__(self, tiles_per_gauss, isect_buf, flat_buf, offsets, C, n_tiles_total, capacity, count, exact):
         self.tiles_per_gauss = tiles_per_gauss
         self.flatten_ids = flat_buf
         self._isect_buf = isect_buf
         self._offsets = offsets
         self._C, self._n_tiles_total = C, n_tiles_total
-        self._capacity, self._counted, self._read_count, self._exact = capacity, counted, read_count, exact
+        self._capacity, self._count, self._exact = capacity, count, exact
         self._resolved = None
 
     @classmethod
     def done(cls, tiles_per_gauss, isect_ids, flatten_ids, C, n_tiles_total):
-        d = cls(tiles_per_gauss, isect_ids, flatten_ids, None, C, n_tiles_total, isect_ids.numel(), None,
-                None, None)
+        d = cls(tiles_per_gauss, isect_ids, flatten_ids, None, C, n_tiles_total, isect_ids.numel(), None, None)
         d._resolved = (isect_ids, flatten_ids)
         return d
 
@@ -1103,7 +1120,7 @@ class DeferredIsect:
 
     def resolve(self):
         if self._resolved is None:
-            n_isects = self._read_count()
+            n_isects = self._count()[0]
             if n_isects < 0 or n_isects > self._capacity:
                 return None
             isect_ids = self._isect_buf[:n_isects]
@@ -1418,9 +1435,11 @@ def rasterize_to_pixels(
     means2d_c = means2d.contiguous()
     args = (conics.contiguous(), opacities.contiguous(), pix_vels.contiguous(),
             rolling_shutter_time.contiguous())
-    # how many tiles a listed Gaussian covers, where the lists' maker has left it; chooses the split of the work
-    spread = (getattr(flatten_ids, "_splatad_spread", 0.0),
-              getattr(flatten_ids, "_splatad_count", 0 if total_follows else flatten_ids.numel()))
+    # how many tiles a listed Gaussian covers, where the lists' maker has left it or what to ask for it (at the launch,
+    # when everything before it is enqueued); chooses the split of the work
+    spread = getattr(flatten_ids, "_splatad_counts", None) or (
+        getattr(flatten_ids, "_splatad_spread", 0.0),
+        getattr(flatten_ids, "_splatad_count", 0 if total_follows else flatten_ids.numel()))
     tail = (image_width, image_height, tile_size, isect_offsets.contiguous(), flatten_ids.contiguous(),
             absgrad, total_follows, spread)
     if channels <= _lib.MAX_CHANNELS:
@@ -1454,6 +1473,9 @@ class _RasterizeToPixels(torch.autograd.Function):
         last_ids = torch.empty((C, height, width), dtype=torch.int32, device=dev)
         n_isects = _n_isects_arg(isect_offsets, flatten_ids, total_follows)
         _debug_check_lists("rasterize_to_pixels", flatten_ids, means2d.numel() // 2, isect_offsets, total_follows)
+        if isinstance(spread, _ReadOnce):
+            count, listed = spread()
+            spread = (count / listed, count) if listed > 0 else (0.0, 0)
         ctx.n_isects_arg, ctx.spread = n_isects, spread
         _lib.load().splatad_rasterize_set_spread_hint(*spread)
         _call(

@@ -1,5 +1,7 @@
 """Helpers shared by the GPU parity tests."""
 
+import ctypes
+
 import numpy as np
 import torch
 
@@ -42,3 +44,19 @@ def rel_l2(got, want):
     got = np.asarray(got, dtype=np.float64)
     want = np.asarray(want, dtype=np.float64)
     return float(np.linalg.norm(got - want) / max(np.linalg.norm(want), 1e-30))
+
+
+def launched(fn):
+    """(what fn() returns, the names of the kernels it launched, in order of their first launch)."""
+    from splatad_b200 import _lib
+    lib = _lib.load()
+    torch.cuda.synchronize()
+    lib.splatad_profile_enable(1)
+    try:
+        out = fn()
+        torch.cuda.synchronize()
+        report = ctypes.create_string_buffer(1 << 16)
+        lib.splatad_profile_report(report, len(report))
+    finally:
+        lib.splatad_profile_enable(0)
+    return out, [line.split()[0] for line in report.value.decode().splitlines()]

@@ -5,7 +5,7 @@ gradients and refusals are those of the individual ops."""
 import pytest
 import torch
 
-from gpu_util import DEV
+from gpu_util import DEV, launched
 
 pytestmark = pytest.mark.gpu
 
@@ -41,6 +41,36 @@ def test_a_frame_reports_how_many_tiles_its_gaussians_cover(packed):
         assert meta["flatten_ids"]._splatad_spread == pytest.approx(want)
         first = first or (image, alpha)
         assert torch.equal(image, first[0]) and torch.equal(alpha, first[1])
+
+
+@pytest.mark.parametrize("packed,pose", [(False, False), (True, False), (False, True)])
+def test_a_frame_is_split_by_its_own_counts(packed, pose):
+    """Two scenes of one shape in turn, one of large Gaussians and one of small ones: each takes the compositing kernels it
+    takes by itself, forward and backward, in native frames and (with a pose that is optimised) by the ops."""
+    import splatad_b200
+    from splatad_b200 import scenes
+    g = _to_gpu(scenes.config1(N=150_011, packed=packed))
+    if pose:
+        g["viewmats"] = g["viewmats"].clone().requires_grad_(True)
+    scales = {"large": g["scales"] * 1.5, "small": g["scales"] * 0.25}
+
+    def step(which):
+        leaf = scales[which].clone().requires_grad_(True)
+        image, _, _ = splatad_b200.rasterization(**{**g, "scales": leaf})
+        image.sum().backward()
+
+    def kernels(which):
+        names = [k for k in launched(lambda: step(which))[1] if k.startswith("rasterize_to_pixels")]
+        return names[-2:]   # a count that outgrows its room renders the frame twice
+
+    alone = {}
+    for which in scales:
+        _forget()
+        for _ in range(3):
+            alone[which] = kernels(which)
+    assert all(k.endswith(",runs") for k in alone["large"]) and not any(k.endswith(",runs") for k in alone["small"])
+    for which in ("large", "small", "large", "small", "small", "large"):
+        assert kernels(which) == alone[which], which
 
 
 @pytest.mark.parametrize("kind", ["lidar", "camera"])
