@@ -2688,20 +2688,28 @@ static uint32_t pixels_that_fit(bool four, bool eight, uint32_t tile_size) {
 static bool many_entries(float spread, int64_t entries, int64_t line, float or_spread) {
     return !(spread > 0.f) || entries <= 0 || entries >= line || spread >= or_spread;
 }
-// Whether most entries that the forward kernel looks at cover their patches, so that eight pixels per lane with runs pay (up to four channels): the
+// Whether most entries that a camera kernel looks at cover their patches, so that runs pay (forward: eight pixels per lane, up to four channels): the
 // nearest Gaussians are the ones that count, and they are larger the more tiles the mean one covers and the more of them
-// a tile's list holds. By the product of the two; us, with runs against the better of four and eight pixels without: 8160 tiles, 28 tiles per Gaussian and 74
-// entries per tile (2 k) 117 and 87, 27 and 143 (4 k) 136 and 113, 16 and 682 (11 k) 158 and 162, 88 and 234 (20 k) 103 and 113, 28 and 1190 (33 k) 130 and 149, 130 and 5800 78
-// and 99; 16320, 26 and 198 (5 k) 271 and 246, 41 and 312 (13 k) 236 and 256; 10800, 19 and 357 (7 k) 211 and 195, 36 and 671 (24 k) 152 and 177; 5700, 12 and 507 (6 k) 138 and
-// 125, 20 and 868 (17 k) 119 and 127. Fewer tiles: 3510, 13 and 564 (7 k) 91 and 78, 24 and 1066 (26 k) 80 and 78, 57 and 2540 60 and 68; 2040, 16 and 704 (11 k)
-// 62 and 56, 36 and 1614 (58 k) 43 and 50; 1840, 25 and 1807 (45 k) 40 and 41; 1450, 79 and 3643 (288 k) 23 and 21.
-// Backward, without and with runs: 8160, 16 and 682 (11 k) 338 and 334, 28 and 1190 305 and 287, 130 and 5800 195 and 180; 16320, 26 and 198 (5 k) 532 and 553, 41
-// and 312 (13 k) 532 and 526; 10800, 36 and 671 373 and 350; 3510, 13 and 564 (7 k) 174 and 167, 24 and 1066 (26 k) 170 and 150; 2040, 16 and 704 (11 k) 115
-// and 117, 36 and 1614 (58 k) 103 and 106; 1840, 12 and 829 (10 k) 105 and 111; 1450, 27 and 1171 (31 k) 70 and 64; 920, 18 and 794 (14 k) 60 and 55.
+// a tile's list holds. By the product of the two; us without runs (the better of four and eight pixels) and with. Forward: 8160 tiles, 28 tiles per Gaussian and 74
+// entries per tile (2 k) 87 and 117, 27 and 143 (4 k) 113 and 136, 16 and 682 (11 k) 162 and 158, 27 and 593 (16 k) 156 and 150, 27 and 1171 (32 k) 147 and 133, 129 and 5750 142
+// and 113; 16320, 26 and 198 (5 k) 246 and 271, 92 and 1307 (120 k) 225 and 180; 10800, 19 and 357 (7 k) 195 and 211, 45 and 1414 (64 k) 170 and 142; 5700, 12 and 507 (6 k) 125 and
+// 138, 20 and 1234 (25 k) 117 and 104. Fewer tiles: 3510, 13 and 564 (7 k) 78 and 91, 24 and 1066 (26 k) 78 and 80; 3600, 23 and 2296 (53 k) 85 and 78; 2040, 16 and 704 (11 k)
+// 56 and 62, 18 and 3107 (55 k) 66 and 50; 1450, 79 and 3643 (288 k) 21 and 23.
+// Forward, sparse scenes of large Gaussians: the chain of the longest list counts, and eight pixels make it longer. Entries in millions, 1840 tiles, 68 and 573, 1.1: 53 and 58, 67 and 1124, 2.1:
+// 44 and 33; 3600, 80 and 496, 1.8: 76 and 79, 59 and 596, 2.1: 78 and 81, 42 and 1008, 3.6: 72 and 67; 7200, 81 and 162, 1.2: 111 and 119, 79 and 316, 2.3: 120 and 115; 5600, 55 and
+// 269, 1.5: 114 and 122; rigs of many tiles and few entries in each gain less still: 7290, 43 and 372 (16 k), 2.7: 138 and 142, 8840, 41 and 331 (14 k), 2.9: 162 and 165,
+// but 8000, 31 and 439 (13 k), 3.5: 140 and 123, 10800, 44 and 420 (19 k), 4.5: 184 and 169.
+// Backward: 16320, 26 and 198 (5 k) 532 and 553; 8160, 28 and 360 (10 k) 306 without, 57 and 251 (14 k) 265 and 263, 27 and 593 (16 k) 336 and 326, 27 and 1171 314 and 298, 60
+// and 791 (48 k) 271 and 250; 3600, 14 and 1354 (19 k) 174 and 162; 2040, 9 and 1546 (14 k) 132 and 118, 35 and 629 (22 k) 124 and 109, 25 and 2252 (57 k) 104 and 86; 1840, 39 and 319 (13
+// k) 98 and 91; 1450, 13 and 995 (13 k) 108 and 72; 920, 9 and 3660 (34 k) 90 and 66. With 8 / 14 channels: 8160, 57 and 251 420 / 610 and 410 / 606, 60 and 791 425 / 608 and 397 / 591; 3600, 14 and 1354 250 /
+// 348 and 235 / 342; 2040, 9 and 1546 173 / 227 and 158 / 220, with absolute gradients 191 / 244 and 172 / 232 (fewer tiles take two pixels per lane and no runs).
 static bool covers_patches(uint64_t blocks, uint32_t tile_size, float spread, int64_t entries, bool backward) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
-    return tiles >= (backward ? 900u : 1800u) && entries > 0 && tile_threads<8>(tile_size) % 32u == 0u &&
-           (double)spread * (double)entries >= (backward || tiles >= 5000u ? 12500.0 : 30000.0) * tiles;
+    const double product = (double)spread * (double)entries;   // times the tiles
+    if (entries <= 0 || tile_threads<8>(tile_size) % 32u != 0u) return false;
+    if (backward) return tiles >= 900u && product >= 12500.0 * tiles;
+    if (tiles < 1800u || entries < 2200000) return false;
+    return product >= (tiles < 5000u ? 30000.0 : entries < 400 * (int64_t)tiles ? 17000.0 : 12500.0) * tiles;
 }
 // Name of a camera kernel in the profile, with what was chosen.
 #define PIXELS_KERNEL_NAME(way, px, runs) \

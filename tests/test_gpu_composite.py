@@ -14,7 +14,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import DEV, assert_close, n, rel_l2, t
+from gpu_util import DEV, assert_close, launched, n, rel_l2, t
 
 pytestmark = pytest.mark.gpu
 
@@ -528,6 +528,35 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, 
             _grad_check(f"spread {spread} v_{k}", v[k], ref["v_" + k].reshape(v[k].shape))
         if absgrad:
             _grad_check(f"spread {spread} absgrad", v_abs, ref["v_means2d_abs"].reshape(v_abs.shape))
+
+
+@pytest.mark.parametrize("C,W,H,ts,spread,per_tile,forward,backward", [
+    (2, 640, 360, 16, 68.0, 573, False, True), (2, 640, 360, 16, 38.0, 1400, True, True), (1, 1280, 720, 16, 59.0, 596, False, True),
+    (1, 1280, 720, 16, 23.0, 2296, True, True), (2, 1280, 720, 16, 81.0, 162, False, True), (2, 1280, 720, 16, 79.0, 316, True, True),
+    (3, 1440, 430, 16, 43.0, 372, False, True), (4, 640, 800, 16, 31.0, 439, True, True), (1, 1920, 1080, 16, 27.0, 1171, True, True),
+    (1, 1920, 1080, 16, 16.0, 682, False, False), (1, 640, 360, 16, 79.0, 3643, False, True), (1, 480, 270, 16, 79.0, 9000, False, False),
+    (1, 1280, 720, 24, 59.0, 5000, False, False), (1, 1280, 720, 32, 20.0, 5000, True, True)])
+def test_runs_are_for_dense_lists_of_large_gaussians(C, W, H, ts, spread, per_tile, forward, backward):
+    """Which camera kernels a hint chooses, on both sides of each line: sparse lists, few tiles, rows that leave lanes over."""
+    from splatad_b200 import _lib
+    lib, p = _lib.load(), _lib.ptr
+    tw, th = -(-W // ts), -(-H // ts)
+    offsets, ids = torch.ones(C, th, tw, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)   # empty lists
+    image, alphas, one = torch.empty(C, H, W, 3, device=DEV), torch.zeros(C, H, W, 1, device=DEV), torch.zeros(8, device=DEV)
+    last, rs = torch.full((C, H, W), -1, dtype=torch.int32, device=DEV), torch.zeros(C, device=DEV)
+    head = (C, 1, p(one), p(one), p(one), 3, p(one), p(one), p(rs), None, W, H, ts, tw, th, p(offsets), p(ids))
+    grads = [torch.zeros(8, device=DEV) for _ in range(5)]
+    entries = per_tile * C * tw * th
+
+    def both():
+        lib.splatad_rasterize_set_spread_hint(spread, entries)
+        _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last), _lib.stream_ptr(ids.device))
+        lib.splatad_rasterize_set_spread_hint(spread, entries)
+        _lib.call("splatad_rasterize_to_pixels_bwd", *head, p(alphas), p(last), p(image), p(alphas), None, *(p(g) for g in grads),
+                  _lib.stream_ptr(ids.device))
+
+    names = launched(both)[1]
+    assert [k.endswith("_kernel/8,runs") for k in names] == [forward, backward], names
 
 
 @pytest.mark.parametrize("what", ["colors", "means2d", "conics", "opacities", "flat", "cotangent"])
