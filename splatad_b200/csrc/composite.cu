@@ -218,23 +218,6 @@ __device__ __forceinline__ uint32_t lane_index() {
     return lane;
 }
 
-// Shared memory by an address in a register of its own.
-__device__ __forceinline__ uint32_t smem_register(const void *p) {
-    uint32_t a;
-    asm volatile("mov.u32 %0, %1;" : "=r"(a) : "r"(smem_addr(p)));
-    return a;
-}
-__device__ __forceinline__ float4 lds4(uint32_t a, int offset) {
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a + offset));
-    return v;
-}
-__device__ __forceinline__ float2 lds2(uint32_t a) {
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-    return v;
-}
-
 // exponents of a pair of pixels in one row: dx of the two, the row's b * dy and c * dy * dy
 __device__ __forceinline__ float2 pair_power(float a, float2 dx, float bdy, float cdy2) {
     const float2 t = __ffma2_rn(make_float2(a, a), dx, make_float2(bdy, bdy));
@@ -1847,9 +1830,8 @@ rasterize_to_pixels_bwd_kernel(
     if constexpr (kRuns) {
         int32_t next_id = 0;
         if (eff_end - 1 - (int32_t)lane >= range.start) next_id = flatten_ids[eff_end - 1 - (int32_t)lane];
-        constexpr uint32_t kEntry = 32 + 4 * CDIM;   // bytes
-        __shared__ float4 sEntry[32 * kEntry / 16];   // x, y, vx, vy | scaled conic, opacity | channels, zeros behind them
-        const uint32_t entries = smem_register(sEntry), ids = smem_register(sId);
+        constexpr uint32_t kEntry = 2 + CDIM / 4;
+        __shared__ float4 sEntry[32 * kEntry];   // x, y, vx, vy | scaled conic, opacity | channels, zeros behind them
         // two entries' sums: colours and geometry of the first, then of the second
         constexpr bool kTwo = 2 * kSums <= 32;
         const SumSlot mine_two = sum_slot<kTwo ? 2 * kSums : kSums>(lane);
@@ -1874,7 +1856,7 @@ rasterize_to_pixels_bwd_kernel(
             const uint32_t careful = __reduce_or_sync(0xffffffffu, (seen & kCarefulEntry) ? 1u << place : 0u);
             __syncwarp();   // the batch before has been read
             if (seen) {
-                float4 *entry = sEntry + place * (kEntry / 16);
+                float4 *entry = sEntry + place * kEntry;
                 entry[0] = e.A;
                 entry[1] = scaled_conic(e.B);
                 sId[place] = make_float2(__int_as_float(g), 1.f / e.B.w);
@@ -1891,9 +1873,9 @@ rasterize_to_pixels_bwd_kernel(
                 uint32_t capped = 0u;   // pixels with a capped alpha, which passes no gradient on to the geometry
 #pragma unroll
                 for (int h = 0; h < kCount; ++h) {
-                    const uint32_t entry = entries + (t + h) * kEntry;
-                    A[h] = lds4(entry, 0);
-                    B[h] = lds4(entry, 16);
+                    const float4 *entry = sEntry + (t + h) * kEntry;
+                    A[h] = entry[0];
+                    B[h] = entry[1];
                     mx[h] = A[h].x + roll * A[h].z;
                     dy[h] = A[h].y + roll * A[h].w - py;
                     const float bdy = B[h].y * dy[h], cdy2 = B[h].z * dy[h] * dy[h];
@@ -1914,7 +1896,7 @@ rasterize_to_pixels_bwd_kernel(
                         }
                     }
 #pragma unroll
-                    for (int c = 0; c < CDIM / 4; ++c) col[h][c] = lds4(entry, 32 + 16 * c);
+                    for (int c = 0; c < CDIM / 4; ++c) col[h][c] = entry[2 + c];
                 }
                 float2 csum[kCount][CDIM], s0[kCount], s1[kCount], s2[kCount], ax[kCount], ay[kCount];
 #pragma unroll
@@ -1973,7 +1955,7 @@ rasterize_to_pixels_bwd_kernel(
                         sum[CDIM + 9] = ay[h].x + ay[h].y;
                     }
                 }
-                const float2 id = lds2(ids + 8u * (kCount == 1 ? t : t + two_entry));
+                const float2 id = sId[kCount == 1 ? t : t + two_entry];
                 const float total = warp_sum_values<kCount * kSums, 16>(sums, lane);
                 if (kCount == 1) slot_a.add((size_t)__float_as_int(id.x), total, id.y, mine_a.writes);
                 else slot_two.add((size_t)__float_as_int(id.x), total, id.y, mine_two.writes);
