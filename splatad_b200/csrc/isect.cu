@@ -1118,7 +1118,7 @@ constexpr uint32_t kBlkThreads = 512, kBlkWarps = kBlkThreads / 32;   // step A:
 // Step B: a CTA takes a unit of 512 consecutive records of a block, or of 1024 where the lists are so long that they leave the cache as they
 // are written: figures at tile_scatter_kernel, whose CTAs go with it, six or two an SM.
 constexpr uint32_t kBlkUnitMin = 512, kBlkUnitMax = 1024;
-constexpr uint64_t kBlkLongLists = (800ull << 20) / 12, kBlkCachedLists = (126ull << 20) / 12;   // entries
+constexpr uint64_t kBlkLongLists = (480ull << 20) / 12, kBlkCachedLists = (126ull << 20) / 12;   // entries
 constexpr uint32_t kBlkWords = 2;                          // writing: 32-record groups per warp
 constexpr uint32_t kBlkCountThreads = 128;                 // counting
 constexpr uint32_t kBlkMaxPerSensor = 1024;                // blocks per sensor (32768 tiles)
@@ -1623,11 +1623,13 @@ tile_scan_kernel(BlkArgs a, unsigned long long *__restrict__ ticket, int32_t *__
 // under way, and the sectors that two units write in parts are evicted between the two, and every such half costs a read
 // and about five whole sectors' time. So whole sectors leave the cache first, halves last (kStream: where the lists
 // do not stay in the cache anyway), and two CTAs an SM are enough.
-// Six cameras, 5.8 GB of lists: 1310 us before, 1390 with four CTAs an SM, 1250 with two, 1200 with two and that order of leaving (dram
-// reads 401 -> 265 MB); units of 512: 1400. Shorter lists want smaller units and more CTAs, us before and with six of 512 records, by MB of lists: 116 (camera
-// benchmark) 43.5 and 38, 184 (lidar benchmark) 66 and 52, 206 (three cameras) 74.5 and 60, 580 (200 k Gaussians, six cameras) 139 and 135; with two of 1024
-// 43.6, 66, 76 and 138, but 302 instead of 338 at 1450 MB. Four entries per lane (32-byte stores): 68 instead of 58 and
-// 1430 instead of 1360, their record numbers lie in the same banks.
+// Six cameras, 5.8 GB of lists: 1315 us before, 1390 with four CTAs an SM, 1250 with two, 1215 with two and that order of leaving (dram
+// reads 401 -> 265 MB). Shorter lists want smaller units and more CTAs, us before, with six of 512 records and with two of 1024, by MB of lists: 109 (camera
+// benchmark) 43, 37 and 49, 175 (lidar benchmark) 65, 50 and 60, 258 (three cameras) 75, 61 and 74, 350 (two lidars) 124, 92 and 107, 412 (150 k
+// Gaussians, six cameras) 104, 102 and 106, 555: 140, 144 and 140, 687: 167, 180 and 158, 774: 199, 204 and 182, 1102: 271, 290 and 248, 1378: 329, 348 and 304; whole frames are
+// 1 % faster with the smaller ones at 278 MB, the same at 412, 1 % slower at 555 and 5 % at 774. Four entries per lane (32-byte stores): 68 instead of 58 and
+// 1430 instead of 1360, their record numbers lie in the same banks. (Whole sectors where the arrays begin on 32 bytes, as torch's do; others of
+// 16 and 8 bytes' alignment are written two entries at a time all the same, anything else one by one.)
 __device__ __forceinline__ uint64_t keep_in_cache() {
     uint64_t policy;
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
@@ -2233,13 +2235,13 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
             tile_offsets = nullptr;   // done
         }
         {
-            SPL_PROF("tile_scatter_kernel", st);
+            SPL_PROF(a.unit == kBlkUnitMax ? "tile_scatter_kernel/1024" : "tile_scatter_kernel", st);
             constexpr uint32_t kMin = kBlkUnitMin / (32 * kBlkWords), kMax = kBlkUnitMax / (32 * kBlkWords);
             const bool longer = a.unit == kBlkUnitMax;
             auto kernel = longer ? tile_scatter_kernel<kMax, true>
                                  : (uint64_t)capacity > kBlkCachedLists ? tile_scatter_kernel<kMin, true> : tile_scatter_kernel<kMin, false>;
             const uint32_t grid = min(units_max, (longer ? 2u : 6u) * kNumSMs);
-            // long lists: not placed while the scan still holds its SMs (six cameras: 1340 us, and 80 more chained)
+            // long lists: not placed while the scan still holds its SMs (six cameras: frame 2585 us, 2627 chained)
             launch_chained_if(!longer, kernel, grid, a.unit / kBlkWords, 0, st, a, isect_ids, flatten_ids, p.counters);
         }
     } else {

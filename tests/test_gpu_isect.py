@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import DEV, n, t
+from gpu_util import DEV, launched, n, t
 
 pytestmark = pytest.mark.gpu
 
@@ -332,6 +332,39 @@ def test_lists_anywhere_in_memory(C, N, tw, th, ids_off, flat_off, long_lists, m
     n_tiles = C * tw * th
     assert torch.equal(starts[flat_off: flat_off + n_tiles], want[3].flatten()) and starts[flat_off + n_tiles] == n_isects
     for buffer, off, size in ((ids, ids_off, n_isects), (flat, flat_off, n_isects), (starts, flat_off, n_tiles + 1)):
+        assert (buffer[:off] == -7).all() and (buffer[off + size: off + size + 8] == -7).all()
+
+
+@pytest.mark.parametrize("ids_off,flat_off", [(0, 0), (1, 0), (2, 2), (2, 1)])
+@pytest.mark.parametrize("capacity,kernel", [(11_000_000, "tile_scatter_kernel"), (11_100_000, "tile_scatter_kernel"),
+                                             (41_900_000, "tile_scatter_kernel"), (42_000_000, "tile_scatter_kernel/1024")])
+def test_list_kernels_by_the_room_for_entries(capacity, kernel, ids_off, flat_off, monkeypatch):
+    """Plain stores, streaming stores, units of 1024 records: each side of the two lines, arrays aligned and not."""
+    from splatad_b200 import _lib, ops
+    C, N, tw, th = 2, 1400, 23, 17
+    g = torch.Generator().manual_seed(3)
+    means2d = torch.rand(C, N, 2, generator=g) * torch.tensor([16.0 * tw, 16.0 * th])
+    radii = (torch.rand(C, N, 2, generator=g) ** 3 * 90).to(torch.int32) + 1
+    depths = torch.rand(C, N, generator=g) * 30 + 0.5
+    want = _run_cam(means2d, radii, depths, 16, tw, th)
+    ids = torch.full((capacity + 8,), -7, dtype=torch.int64, device=DEV)
+    flat = torch.full((capacity + 8,), -7, dtype=torch.int32, device=DEV)
+    fill_ws = torch.empty(_lib.load().splatad_isect_fill_workspace_bytes(capacity), dtype=torch.uint8, device=DEV)
+    call = ops._call
+
+    def elsewhere(name, *args):
+        if name == "splatad_isect_tiles_fill":
+            *head, _, _, _, _, _, starts, host, stream = args
+            args = (*head, _lib.ptr(fill_ws), fill_ws.numel(), capacity, ids.data_ptr() + 8 * ids_off, flat.data_ptr() + 4 * flat_off,
+                    starts, host, stream)
+        return call(name, *args)
+
+    monkeypatch.setattr(ops, "_call", elsewhere)
+    _, names = launched(lambda: ops.isect_tiles(t(means2d), t(radii), t(depths), 16, tw, th))
+    assert kernel in names, names
+    for buffer, off, lists in ((ids, ids_off, want[1]), (flat, flat_off, want[2])):
+        size = lists.numel()
+        assert torch.equal(buffer[off: off + size], lists)
         assert (buffer[:off] == -7).all() and (buffer[off + size: off + size + 8] == -7).all()
 
 
