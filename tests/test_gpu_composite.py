@@ -479,10 +479,13 @@ def test_pixels_by_how_many_tiles_a_gaussian_covers(C, ts, channels, absgrad):
 @pytest.mark.parametrize("C,W,H,ts,channels,sigma_px,N,absgrad", [
     (30, 127, 133, 16, 3, (20.0, 90.0), 150, False), (84, 132, 131, 16, 4, (20.0, 90.0), 90, True), (30, 128, 128, 16, 1, (3.0, 60.0), 200, True),
     (84, 121, 120, 16, 2, (60.0, 400.0), 64, False), (24, 131, 129, 32, 4, (10.0, 90.0), 150, False), (110, 130, 130, 24, 3, (20.0, 90.0), 90, False),
-    (30, 127, 133, 16, 7, (20.0, 90.0), 90, True), (30, 132, 131, 16, 14, (10.0, 90.0), 90, False)])
+    (30, 127, 133, 16, 7, (20.0, 90.0), 90, True), (30, 132, 131, 16, 14, (10.0, 90.0), 90, False),
+    (30, 127, 133, 16, 5, (20.0, 90.0), 90, False), (24, 131, 130, 16, 7, (10.0, 90.0), 90, False), (30, 128, 131, 16, 8, (20.0, 90.0), 90, False),
+    (24, 132, 129, 16, 16, (20.0, 90.0), 90, True)])
 def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, absgrad):
     """Scenes of large Gaussians: entries that cover a patch go through without a test in the kernel for them, which the hint
-    chooses; images, alphas and last positions are those of the kernel without runs, bit for bit, and match the oracle, as the gradients do. Opaque
+    chooses - forward up to four channels, backward up to sixteen, and not where a tile's rows leave lanes over (24 pixels) -; images, alphas
+    and last positions are those of the kernel without runs, bit for bit, and match the oracle, as the gradients do. Opaque
     and capped entries, needles, a flat conic and ones that cover part of a patch among them."""
     from oracle import composite
     from splatad_b200 import _lib
@@ -512,7 +515,9 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, 
         image, alphas = torch.empty(C, H, W, channels, device=DEV), torch.empty(C, H, W, 1, device=DEV)
         last = torch.empty(C, H, W, dtype=torch.int32, device=DEV)
         lib.splatad_rasterize_set_spread_hint(spread, count)
-        _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last), _lib.stream_ptr(ids.device))
+        _, (name,) = launched(lambda: _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last),
+                                                _lib.stream_ptr(ids.device)))
+        assert name.endswith(",runs") == (spread > 0 and channels <= 4 and ts != 24), name
         if first is None:
             first = image, alphas, last
             assert_close("image", n(image), want["render_colors"], 1e-4, 1e-5, mask=ok[..., None])
@@ -522,8 +527,10 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, 
         v = {k: torch.zeros_like(dev[k]) for k in keys}
         v_abs = torch.zeros_like(dev["means2d"]) if absgrad else None
         lib.splatad_rasterize_set_spread_hint(spread, count)
-        _lib.call("splatad_rasterize_to_pixels_bwd", *head, p(alphas), p(last), p(cotangents[0]), p(cotangents[1]), p(v_abs),
-                  *(p(v[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")), _lib.stream_ptr(ids.device))
+        _, (name,) = launched(lambda: _lib.call(
+            "splatad_rasterize_to_pixels_bwd", *head, p(alphas), p(last), p(cotangents[0]), p(cotangents[1]), p(v_abs),
+            *(p(v[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")), _lib.stream_ptr(ids.device)))
+        assert name.endswith(",runs") == (spread > 0 and ts != 24), name
         for k in keys:
             _grad_check(f"spread {spread} v_{k}", v[k], ref["v_" + k].reshape(v[k].shape))
         if absgrad:
@@ -559,12 +566,43 @@ def test_runs_are_for_dense_lists_of_large_gaussians(C, W, H, ts, spread, per_ti
     assert [k.endswith("_kernel/8,runs") for k in names] == [forward, backward], names
 
 
-@pytest.mark.parametrize("what", ["colors", "means2d", "conics", "opacities", "flat", "cotangent"])
-def test_runs_with_values_that_are_not_finite(what):
-    """The kernels with runs and those without them agree on the pixels that a value which is not finite reaches, on the Gaussians that
-    get such a gradient, and on all others."""
+def test_runs_of_thousands_of_faint_entries():
+    """Every entry covers every patch with an alpha just above 1/255, so that some 2250 of them go by before a transmittance comes
+    near the limit, the longest sum that the bound of the transmittances is ever taken over: each pixel stops where it does
+    without runs, and the images are the same bit for bit."""
     from splatad_b200 import _lib
-    C, W, H, ts, channels, N = 30, 128, 127, 16, 3, 90
+    C, W, H, ts, N = 2, 480, 480, 16, 2600
+    g = torch.Generator().manual_seed(9)
+    tw, th = W // ts, H // ts
+    means2d, colors = torch.rand(C, N, 2, generator=g) * torch.tensor([W, H]), torch.rand(C, N, 3, generator=g)
+    conics = torch.tensor([2e-8, 0.0, 2e-8]).expand(C, N, 3).contiguous()
+    opacities = 1.005 / 255 * (1 + 0.08 * torch.rand(C, N, generator=g))
+    dev = [x.to(DEV) for x in (means2d, conics, colors, opacities, torch.zeros(C, N, 2), torch.zeros(C))]
+    offsets = (torch.arange(C * tw * th, dtype=torch.int32) * N).to(DEV)
+    ids = torch.arange(C * N, dtype=torch.int32).view(C, 1, N).expand(C, tw * th, N).contiguous().to(DEV)
+    lib, p, results = _lib.load(), _lib.ptr, []
+    for hint, runs in (((0.0, 0), False), ((100.0, 10**8), True)):
+        image, alphas = torch.empty(C, H, W, 3, device=DEV), torch.empty(C, H, W, 1, device=DEV)
+        last = torch.empty(C, H, W, dtype=torch.int32, device=DEV)
+        lib.splatad_rasterize_set_spread_hint(*hint)
+        _, (name,) = launched(lambda: _lib.call(
+            "splatad_rasterize_to_pixels_fwd", C, ids.numel(), *(p(x) for x in dev[:3]), 3, *(p(x) for x in dev[3:]), None, W, H, ts, tw, th,
+            p(offsets), p(ids), p(image), p(alphas), p(last), _lib.stream_ptr(ids.device)))
+        assert name.endswith(",runs") == runs, name
+        results.append((image, alphas, last))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    at = results[0][2].view(C, th, ts, tw, ts) % N   # (each tile's list has the N entries of its camera)
+    assert 2000 < int(at.min()) and int(at.max()) < N - 100
+
+
+@pytest.mark.parametrize("channels,absgrad", [(3, False), (8, False), (8, True), (14, False)])
+@pytest.mark.parametrize("what", ["colors", "means2d", "conics", "opacities", "flat", "cotangent"])
+def test_runs_with_values_that_are_not_finite(what, channels, absgrad):
+    """The kernels with runs (above four channels the backward ones) and those without them agree on the pixels that a value which is
+    not finite reaches, on the Gaussians that get such a gradient, and on all others."""
+    from splatad_b200 import _lib
+    C, W, H, ts, N = 30, 128, 127, 16, 90
     c = _camera_case(C, N, W, H, ts, channels, 77, sigma_px=(15.0, 80.0))
     if what == "flat": c["conics"][:, 5] = torch.tensor([1e-37, 0.0, 1e-37])
     elif what != "cotangent":
@@ -591,9 +629,13 @@ def test_runs_with_values_that_are_not_finite(what):
     v_c, v_a, gradients = torch.where(same, v_c, 0.0), torch.where(same, v_a, 0.0), []
     for hint, (_, alphas_h, last_h) in zip(hints, results):
         grads = {k: torch.zeros_like(dev[k]) for k in keys}
+        if absgrad:
+            grads["absgrad"] = torch.zeros_like(dev["means2d"])
         lib.splatad_rasterize_set_spread_hint(*hint)
-        _lib.call("splatad_rasterize_to_pixels_bwd", *head, p(alphas_h), p(last_h), p(v_c), p(v_a), None,
-                  *(p(grads[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")), _lib.stream_ptr(ids.device))
+        _, (name,) = launched(lambda: _lib.call(
+            "splatad_rasterize_to_pixels_bwd", *head, p(alphas_h), p(last_h), p(v_c), p(v_a), p(grads.get("absgrad")),
+            *(p(grads[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")), _lib.stream_ptr(ids.device)))
+        assert name.endswith(",runs") == (hint[1] > 0), name
         gradients.append(grads)
     v, v_r = gradients
     # pixels are worked out again patch by patch, and patches differ in size: a rounding, and a decision in a few thousand, may differ
@@ -602,7 +644,7 @@ def test_runs_with_values_that_are_not_finite(what):
     assert (image.isfinite() == image_r.isfinite()).float().mean() > 0.9999
     both = image.isfinite() & image_r.isfinite()
     assert_close("image", n(image_r), n(image), 1e-4, 1e-5, mask=n(both).astype(bool), max_bad_frac=1e-3)
-    for k in keys:
+    for k in v:
         assert (v[k].isfinite() == v_r[k].isfinite()).float().mean() > 0.999, k
         both = v[k].isfinite() & v_r[k].isfinite()
         _grad_check(k, torch.where(both, v_r[k], 0.0), n(torch.where(both, v[k], 0.0)), rel=5e-3)
