@@ -554,9 +554,9 @@ def roofline_stages(prof, cam_prof, n_gauss, n_vis, n_isects, n_rec, pairs, cam_
 # DRAM bytes (read + written) per launch on the headline frame, from the ncu captures summarised
 # under profiles/; kernels without a committed capture give null.
 NCU_TRAFFIC = {
-    "tile_scatter_kernel": (146_702_336, "profiles/lidar_training_step.md"),
+    "tile_scatter_kernel": (130_190_000, "profiles/lidar_training_step.md"),
     "blk_scatter_kernel": (8_276_224, "profiles/lidar_training_step.md"),
-    "rasterize_to_points_fwd_kernel": (4_691_200, "profiles/lidar_training_step.md"),
+    "rasterize_to_points_fwd_kernel": (4_910_000, "profiles/lidar_training_step.md"),
     "lidar_projection_fwd_kernel": (45_829_376, "profiles/lidar_projection_fwd_config2.md"),
     "depth_bucket_scatter_kernel": (11_567_616, "profiles/depth_bucket_kernels_config2.md"),
     "depth_bucket_count_kernel": (9_038_592, "profiles/depth_bucket_kernels_config2.md"),

@@ -426,7 +426,9 @@ int splatad_populate_image_from_points(
 /* No counterpart in the reference. Arms a one-shot hint for the NEXT camera compositing call of the calling
  * thread, forward or backward: list entries per Gaussian that the lists hold, as far as the caller knows
  * it (0: not known, the number of tiles decides alone), and how many entries there are in all (0: not known). It chooses how many pixels a lane draws
- * and whether entries that cover a patch go through in runs, and cannot change an image; gradients are the same sums in another order. */
+ * and whether entries that cover a patch go through in runs, and cannot change an image of finite values (a patch with one that is not
+ * finite is worked out again by itself, and patches differ in size: a rounding there, or a decision at a threshold, may differ); gradients
+ * are the same sums in another order. */
 int splatad_rasterize_set_spread_hint(float tiles_per_gaussian, int64_t n_isects);
 
 /* rasterize_to_pixels_fwd_tensor - gsplat/cuda/csrc/rasterization.cu:1520-2019, kernel

@@ -588,7 +588,7 @@ constexpr int pixels_fwd_regs(int cdim, int px, bool runs) {
 // batch -, which it reaches with one entry in 15 to 45. Such an entry, one that does not cover the patch and one that needs care are
 // looked at one by one. What bounds it then is the FP32 pipe, at 75 % of its rate within a run, and the batches. 1920 x 1080, 27 tiles per
 // Gaussian 104 M -> 82 M warp instructions, 145 -> 130 us, 54 tiles 119 -> 95, six cameras 584 -> 445. Where few entries cover their patch it
-// is slower by up to half: see covers_patches(). (Entries two by two: 144 us, for the registers; the next batch's entries loaded ahead: no change.)
+// is slower by up to half: see covers_patches(). (Entries two by two: 5 % slower, for the registers; the next batch's entries loaded ahead: no change.)
 //
 // kTogether: rows in 16-byte pieces, staged by copy_rows(). A kernel of its own: with both ways in one, 1920 x 1080 and 32 channels
 // take 648 us instead of 506.
