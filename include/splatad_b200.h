@@ -362,6 +362,12 @@ int splatad_isect_set_early_count(int64_t *host_pair, int64_t sequence);
  * count. NULL disarms. */
 int splatad_isect_set_listed_count(int64_t *host_word);
 
+/* No counterpart in the reference. Arms a one-shot request for the NEXT _fill call of the calling thread: *host_word, pinned (mapped)
+ * host memory, receives sequence << 32 | how many tiles one of the nearest Gaussians covers on the average, as the bit pattern of a
+ * float (0: not known), by a kernel of the fill early on or, where none reports it (lidar tiles, unsorted output, grids
+ * beyond the block split, an error), by the call itself. It is always answered. NULL disarms. */
+int splatad_isect_set_near_tiles(int64_t *host_word, uint32_t sequence);
+
 /* No counterpart in the reference. Arms a one-shot hint for the NEXT _plan call of the calling
  * thread with sort = 1: the depths of the elements it will list are expected within
  * [depth_lo, depth_hi], given as the bit patterns of two non-negative finite floats (the range the
@@ -430,6 +436,10 @@ int splatad_populate_image_from_points(
  * finite is worked out again by itself, and patches differ in size: a rounding there, or a decision at a threshold, may differ); gradients
  * are the same sums in another order. */
 int splatad_rasterize_set_spread_hint(float tiles_per_gaussian, int64_t n_isects);
+
+/* The same for how many tiles one of the nearest Gaussians covers (splatad_isect_set_near_tiles; 0: not known, and no entries go
+ * through in runs). */
+int splatad_rasterize_set_near_hint(float tiles_per_near_gaussian);
 
 /* rasterize_to_pixels_fwd_tensor - gsplat/cuda/csrc/rasterization.cu:1520-2019, kernel
  * 1360-1518. Inputs are [C,N,..] or packed [nnz,..] (flatten_ids index either);

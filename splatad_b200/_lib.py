@@ -13,6 +13,7 @@ import importlib.machinery
 import importlib.util
 import os
 import re
+import struct
 import subprocess
 import time
 from typing import Dict, List, Optional, Tuple
@@ -259,9 +260,12 @@ def acquire_pinned_slot(device: torch.device) -> torch.Tensor:
     asynchronously); give it back with :func:`release_pinned_slot` once it has been read. Slots are
     recycled per (device, stream): a plan copies its counters twice (the count early, everything at
     its end), and only work enqueued later on the same stream is ordered behind the second copy."""
-    free = _free_slots.get(_stream_key(device))
-    slot = free.pop() if free else torch.zeros(10, dtype=torch.int64).pin_memory()
-    slot._splatad_stream_key = _stream_key(device)
+    key = _stream_key(device)
+    free = _free_slots.get(key)
+    if free:
+        return free.pop()
+    slot = torch.zeros(10, dtype=torch.int64).pin_memory()
+    slot._splatad_stream_key, slot._splatad_words = key, memoryview(slot.numpy())
     return slot
 
 
@@ -280,7 +284,7 @@ def wait_for_count(slot: torch.Tensor, sequence: int, event: torch.cuda.Event, p
     plan copies at its end, [4..7] the early words {count, sequence, status, depth range}). Polls the triple for
     ``sequence`` - a kernel stores it there itself, long before the plan's own copy - and falls back to waiting for
     ``event`` (recorded behind the plan) when it does not show up within ``patience_s``."""
-    view = slot.numpy()
+    view = getattr(slot, "_splatad_words", None) or slot.numpy()
     if sequence:
         deadline = time.perf_counter() + patience_s
         while view[5] != sequence:
@@ -290,6 +294,35 @@ def wait_for_count(slot: torch.Tensor, sequence: int, event: torch.cuda.Event, p
             return int(view[4]), int(view[6])
     event.synchronize()
     return int(view[0]), int(view[2])
+
+
+_near_rings: Dict[int, tuple] = {}
+_float_of = struct.Struct("f").unpack_from
+
+
+class NearRequest:
+    """Has the next camera fill report how many tiles a near Gaussian covers (splatad_isect_set_near_tiles) and reads it. The
+    word is one of 64 per device that are never given back, so that nobody has to read it: one that a later
+    request has taken over, or that takes too long, reads as not known."""
+
+    __slots__ = ("words", "at", "sequence")
+
+    def __init__(self, device: torch.device):
+        ring = _near_rings.get(device.index)
+        if ring is None:
+            words = torch.zeros(64, dtype=torch.int64).pin_memory()
+            ring = _near_rings[device.index] = (words, words.data_ptr(), memoryview(words.numpy()))
+        self.sequence = next_sequence() & 0x7FFFFFFF
+        self.at, self.words = self.sequence & 63, ring[2]
+        load().splatad_isect_set_near_tiles(ring[1] + 8 * self.at, self.sequence)
+
+    def __call__(self, patience_s: float = 0.02) -> float:
+        word = self.words[self.at]
+        if word >> 32 < self.sequence:
+            deadline = time.perf_counter() + patience_s
+            while word >> 32 < self.sequence and time.perf_counter() < deadline:
+                word = self.words[self.at]
+        return _float_of((word & 0xFFFFFFFF).to_bytes(4, "little"))[0] if word >> 32 == self.sequence else 0.0
 
 
 def release_pinned_slot(slot: torch.Tensor) -> None:

@@ -2672,9 +2672,14 @@ static uint32_t pixels_that_fit(bool four, bool eight, uint32_t tile_size) {
 static bool many_entries(float spread, int64_t entries, int64_t line, float or_spread) {
     return !(spread > 0.f) || entries <= 0 || entries >= line || spread >= or_spread;
 }
-// Whether most entries that a camera kernel looks at cover their patches, so that runs pay (forward: eight pixels per lane, up to four channels): the
-// nearest Gaussians are the ones that count, and they are larger the more tiles the mean one covers and the more of them
-// a tile's list holds. By the product of the two; us without runs (the better of four and eight pixels) and with. Forward: 8160 tiles, 28 tiles per Gaussian and 74
+// Whether most entries that a camera kernel looks at cover their patches, so that runs pay (forward: eight pixels per lane, up to four channels). The
+// nearest Gaussians are the ones that count: how many tiles each of them covers (near: splatad_isect_set_near_tiles(); not known, no runs). Without runs and with, us, forward, by
+// near tiles: 8 (three million of 3 pixels before a sky of large ones, 7 tiles and 6790 entries on the average, 2040 tiles) 225 and 322; 18 (6 pixels) 119 and 167; 54 (sizes of
+// two pixels on the average and e^1.5 around it) 143 and 145; 79 141 and 145; 113 (24 pixels) 90 and 105; 203 108 and 105; 295 (48 pixels) 80 and 87; 350 and more 0.4 to 30 % less with runs in
+// all of 446 scenes, such as 404 56 and 47, 479 193 and 187, 582 259 and 237, 1039 41 and 33, 1961 195 and 155. Backward: 9 248 and 334; 26 435 and 475; 66 469 and 499; 117 221 and 227; 136 438 and
+// 446; 175 and more the same or less in all of 615, 202 149 and 141, 295 168 and 148, 533 236 and 232, 637 127 and 83. Neither the mean of all Gaussians, nor that of all entries, nor the
+// share of entries of large ones tells these apart: what lies far away is never composited.
+// Then by tiles per Gaussian times entries per tile, where near ones are large; us without runs (the better of four and eight pixels) and with. Forward: 8160 tiles, 28 tiles per Gaussian and 74
 // entries per tile (2 k) 87 and 117, 27 and 143 (4 k) 113 and 136, 16 and 682 (11 k) 162 and 158, 27 and 593 (16 k) 156 and 150, 27 and 1171 (32 k) 147 and 133, 129 and 5750 142
 // and 113; 16320, 26 and 198 (5 k) 246 and 271, 92 and 1307 (120 k) 225 and 180; 10800, 19 and 357 (7 k) 195 and 211, 45 and 1414 (64 k) 170 and 142; 5700, 12 and 507 (6 k) 125 and
 // 138, 20 and 1234 (25 k) 117 and 104. Fewer tiles: 3510, 13 and 564 (7 k) 78 and 91, 24 and 1066 (26 k) 78 and 80; 3600, 23 and 2296 (53 k) 85 and 78; 2040, 16 and 704 (11 k)
@@ -2687,10 +2692,10 @@ static bool many_entries(float spread, int64_t entries, int64_t line, float or_s
 // and 791 (48 k) 271 and 250; 3600, 14 and 1354 (19 k) 174 and 162; 2040, 9 and 1546 (14 k) 132 and 118, 35 and 629 (22 k) 124 and 109, 25 and 2252 (57 k) 104 and 86; 1840, 39 and 319 (13
 // k) 98 and 91; 1450, 13 and 995 (13 k) 108 and 72; 920, 9 and 3660 (34 k) 90 and 66. With 8 / 14 channels: 8160, 57 and 251 420 / 610 and 410 / 606, 60 and 791 425 / 608 and 397 / 591; 3600, 14 and 1354 250 /
 // 348 and 235 / 342; 2040, 9 and 1546 173 / 227 and 158 / 220, with absolute gradients 191 / 244 and 172 / 232 (fewer tiles take two pixels per lane and no runs).
-static bool covers_patches(uint64_t blocks, uint32_t tile_size, float spread, int64_t entries, bool backward) {
+static bool covers_patches(uint64_t blocks, uint32_t tile_size, float spread, int64_t entries, float near, bool backward) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
     const double product = (double)spread * (double)entries;   // times the tiles
-    if (entries <= 0 || tile_threads<8>(tile_size) % 32u != 0u) return false;
+    if (entries <= 0 || !(near >= (backward ? 175.f : 350.f)) || tile_threads<8>(tile_size) % 32u != 0u) return false;
     if (backward) return tiles >= 900u && product >= 12500.0 * tiles;
     if (tiles < 1800u || entries < 2200000) return false;
     return product >= (tiles < 5000u ? 30000.0 : entries < 400 * (int64_t)tiles ? 17000.0 : 12500.0) * tiles;
@@ -2719,10 +2724,11 @@ static bool pixels_bwd_other(uint64_t blocks, uint32_t tile_size, uint32_t chann
 // One-shot hint of the calling thread's next camera compositing call.
 static thread_local float t_spread_hint = 0.f;
 static thread_local int64_t t_entries_hint = 0;
-struct SplatHint { float spread; int64_t entries; };   // 0: not known
+static thread_local float t_near_hint = 0.f;
+struct SplatHint { float spread; int64_t entries; float near; };   // 0: not known
 static SplatHint take_spread_hint(uint32_t tile_size) {
-    const SplatHint hint = {spread_of_16(t_spread_hint, tile_size), t_entries_hint};
-    t_spread_hint = 0.f;
+    const SplatHint hint = {spread_of_16(t_spread_hint, tile_size), t_entries_hint, spread_of_16(t_near_hint, tile_size)};
+    t_spread_hint = t_near_hint = 0.f;
     t_entries_hint = 0;
     return hint;
 }
@@ -2782,6 +2788,11 @@ extern "C" int splatad_rasterize_set_spread_hint(float tiles_per_gaussian, int64
     return SPLATAD_OK;
 }
 
+extern "C" int splatad_rasterize_set_near_hint(float tiles_per_near_gaussian) {
+    t_near_hint = tiles_per_near_gaussian;
+    return SPLATAD_OK;
+}
+
 extern "C" int splatad_rasterize_to_pixels_fwd(
     uint32_t C, int64_t n_isects, const float *means2d, const float *conics, const float *colors,
     uint32_t channels, const float *opacities, const float *pix_vels,
@@ -2830,7 +2841,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     }
 #define CALL(D)                                                                                   \
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2)) else if (D <= 16 && px == 4) CALL_PX(D, (D <= 16 ? 4 : 2)) else CALL_PX(D, 2)
-    const bool runs = channels <= 4 && covers_patches(blocks, tile_size, hint.spread, hint.entries, false);
+    const bool runs = channels <= 4 && covers_patches(blocks, tile_size, hint.spread, hint.entries, hint.near, false);
     const uint32_t px = runs ? 8u : pixels_per_lane_fwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool vec = channels % 4u == 0u && (reinterpret_cast<uintptr_t>(colors) & 15u) == 0u;
     {
@@ -2905,7 +2916,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2), A) else if (D <= 20 && px == 4) CALL_PX(D, (D <= 20 ? 4 : 2), A) else CALL_PX(D, 2, A)
 #define CALL(D)                                                                                   \
     if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)
-    const bool runs = covers_patches(blocks, tile_size, hint.spread, hint.entries, true);
+    const bool runs = covers_patches(blocks, tile_size, hint.spread, hint.entries, hint.near, true);
     const uint32_t px = runs && channels <= 4 ? 8u : pixels_per_lane_bwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool other = pixels_bwd_other(blocks, tile_size, channels, px, hint.spread);
     {

@@ -42,7 +42,8 @@ using OptTensor = c10::optional<Tensor>;
     X(splatad_isect_plan_workspace_bytes) X(splatad_isect_fill_workspace_bytes) X(splatad_lidar_azimuth_tiles)           \
     X(splatad_isect_tiles_plan) X(splatad_isect_tiles_fill) X(splatad_isect_lidar_tiles_plan)                            \
     X(splatad_isect_lidar_tiles_fill) X(splatad_isect_set_early_count) X(splatad_isect_set_depth_range_hint)             \
-    X(splatad_isect_set_listed_count) X(splatad_rasterize_set_spread_hint) X(splatad_rasterize_set_rows_hint)            \
+    X(splatad_isect_set_listed_count) X(splatad_isect_set_near_tiles) X(splatad_rasterize_set_spread_hint)               \
+    X(splatad_rasterize_set_near_hint) X(splatad_rasterize_set_rows_hint)                                                \
     X(splatad_rasterize_expected_to_pixels_fwd) X(splatad_rasterize_expected_to_pixels_bwd)                              \
     X(splatad_lidar_frame_fwd) X(splatad_rasterize_to_points_fwd) X(splatad_rasterize_to_points_bwd) X(splatad_map_points_workspace_bytes)          \
     X(splatad_map_strided_points_to_lidar_tiles) X(splatad_points_mapping_offset_encode) X(splatad_populate_image_from_points)
@@ -555,7 +556,7 @@ struct CameraFrame : torch::CustomClassHolder {
     std::vector<int64_t> color_sizes;
     int64_t K = 0, D = 0, sh_degree = -1;     // spherical harmonics (K coefficients) or D plain channels
     bool packed = false, per_camera = false, depth = false, expected = false, absgrad = false;
-    float eps2d = 0.f, spread = 0.f;          // spread: tiles that a listed Gaussian covers on the average, 0: not known
+    float eps2d = 0.f, spread = 0.f, near = 0.f;   // spread, near: tiles that a listed or near Gaussian covers on the average, 0: not known
     Tensor camera_ids, gaussian_ids, radii, means2d, depths, conics, comps, pix_vels, tiles_per_gauss, campos;
     Tensor opacities, colors;                 // rows made for this frame (undefined: the parameters serve as they are)
     Tensor isect_ids, flatten_ids, offsets, render, alphas, last_ids;
@@ -565,7 +566,7 @@ struct CameraFrame : torch::CustomClassHolder {
         k->C = C; k->N = N; k->n = n; k->W = W; k->H = H; k->tile_size = tile_size; k->tile_w = tile_w; k->tile_h = tile_h;
         k->channels = channels; k->K = K; k->D = D; k->sh_degree = sh_degree; k->packed = packed; k->per_camera = per_camera;
         k->depth = depth; k->expected = expected; k->absgrad = absgrad; k->eps2d = eps2d; k->n_isects = n_isects;
-        k->spread = spread;
+        k->spread = spread; k->near = near;
         k->color_sizes = color_sizes;
         return k;
     }
@@ -692,6 +693,7 @@ struct CameraCompositeNode : torch::autograd::Function<CameraCompositeNode> {
         if (f->absgrad) zeros.add(v_abs, means2d.sizes());
         zeros.make(options);
         lib.splatad_rasterize_set_spread_hint(f->spread, f->n_isects);
+        lib.splatad_rasterize_set_near_hint(f->near);
         check(lib.splatad_rasterize_expected_to_pixels_bwd(
             (uint32_t)f->C, f->n_isects, F(means2d), F(conics), F(colors), (uint32_t)f->channels, F(opacities), F(pix_vels), F(saved[5]),
             F(saved[6]), (uint32_t)f->W, (uint32_t)f->H, (uint32_t)f->tile_size, (uint32_t)f->tile_w, (uint32_t)f->tile_h, I(saved[9]),
@@ -805,6 +807,11 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
             const PlanRequests requests(slot, sequence, last_range, true);
             check(grid(lib.splatad_isect_tiles_plan, plan_ws.data_ptr(), (size_t)plan_ws.numel(), (int64_t *)nullptr, stream.stream()));
         }
+        // who may take runs: whole warps of eight pixels per lane, many tiles, forward up to four channels, backward up to sixteen
+        const int64_t tiles_16 = C * tile_w * tile_h * tile_size * tile_size / 256;
+        const bool ask_near = tile_size % 16 == 0 && ((tiles_16 >= 1800 && channels <= 4) || (grad && tiles_16 >= 900 && channels <= 16));
+        slot.word[10] = 0;
+        if (ask_near) lib.splatad_isect_set_near_tiles(const_cast<int64_t *>(slot.word) + 10, (uint32_t)sequence);
         check(grid(lib.splatad_isect_tiles_fill, plan_ws.data_ptr(), fill_ws.data_ptr(), (size_t)fill_ws.numel(), capacity,
                    L(f->isect_ids), I(f->flatten_ids), I(f->offsets), (int64_t *)nullptr, stream.stream()));
         const float *o = F(opacities), *c = mode == 2 ? F(f->depths) : F(colors);
@@ -843,10 +850,18 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
                     if ((i & 4095u) == 4095u && stream.query()) break;
                 nnz = load_word(slot.word + 8);
             }
+            if (ask_near) {
+                int64_t word;
+                for (uint32_t i = 0; (uint32_t)((uint64_t)(word = load_word(slot.word + 10)) >> 32) != (uint32_t)sequence; ++i, pause())
+                    if ((i & 4095u) == 4095u && stream.query()) break;
+                const uint32_t bits = (uint32_t)word;
+                memcpy(&f->near, &bits, 4);
+            }
         }
         if (nnz <= 0 || nnz > rows_max || !usable(counts, capacity))
             return py::make_tuple(nnz, counts.n_isects, counts.status, counts.depth_range, counts.listed, py::none());
         lib.splatad_rasterize_set_spread_hint(counts.spread(), counts.n_isects);
+        lib.splatad_rasterize_set_near_hint(f->near);
         check(lib.splatad_rasterize_expected_to_pixels_fwd(
             (uint32_t)C, -1, F(f->means2d), F(f->conics), c, (uint32_t)channels, o, F(f->pix_vels), F(rs_t), F(bg), (uint32_t)W, (uint32_t)H,
             (uint32_t)tile_size, (uint32_t)tile_w, (uint32_t)tile_h, I(f->offsets), I(f->flatten_ids), expected, M(f->render), M(f->alphas),

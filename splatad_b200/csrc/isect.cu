@@ -1151,6 +1151,10 @@ struct BlkArgs {
     uint32_t *unit_cnt;           // [units][32] list entries per (unit, tile); scanned per block in place
     uint4 *unit_info;             // [units] {block, first record, end}
     uint32_t *tile_base;          // [C * n_tiles] totals, then first list position of every tile
+    float *near;                  // [1] tiles that a near entry covers, where asked for
+    volatile int64_t *near_host;  // who asks: sequence << 32 | the float's bits; may be null
+    uint32_t near_sequence;
+    uint32_t near_shift, near_step;   // 512s of each sensor that is looked at (log2), and every how manieth sensor is
 };
 
 // More intersections than output slots: the split is skipped altogether (the record arrays are sized
@@ -1260,12 +1264,51 @@ __device__ __forceinline__ uint32_t blk_row_cols(const BlkRect &b, uint32_t r) {
     return (r - b.sy) < b.ny ? b.nx : 0u;
 }
 
+// The mean number of tiles that one of the nearest Gaussians covers: of the first 4096 entries of one sensor, or of as many of
+// up to eight together, by 512 until they make 32 list entries per tile. Most of what compositing looks at is theirs. A block that starts
+// with the kernel and has little to count does it first, with one wait for all its loads (in the last block of 500 k Gaussians, which starts when the others
+// end: 2 to 3 us of the frame); the kernel behind it tells the host, whose link a longer kernel covers (2 us here, 4 with a fence).
+constexpr uint32_t kNearGroups = 8, kNearPerTile = 32, kNearCta = 300;
+__device__ __forceinline__ void find_near(const BlkArgs &a) {
+    __shared__ uint32_t s_near[kNearGroups], s_of[kNearGroups];   // tiles, entries
+    const uint32_t tid = threadIdx.x, sensors = min(a.C, kNearGroups);
+    if (tid < kNearGroups) s_near[tid] = 0u;
+    uint2 r[kNearGroups];
+#pragma unroll
+    for (uint32_t g = 0; g < kNearGroups; ++g) {
+        const uint32_t i = g >> a.near_shift, sensor = i < sensors ? i * a.near_step : 0u, k = g - (i << a.near_shift);
+        const uint32_t lo = __ldg(a.sensor_start + sensor) + k * kBlkThreads, end = __ldg(a.sensor_start + sensor + 1);
+        const uint32_t n = i < sensors && lo < end ? min(kBlkThreads, end - lo) : 0u;
+        r[g] = tid < n ? __ldg(a.rect + lo + tid) : make_uint2(0u, 0u);
+        if (tid == 0) s_of[g] = n;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t g = 0; g < kNearGroups; ++g) {
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, (r[g].x >> 16) * (r[g].y >> 16));
+        if ((tid & 31u) == 0u && sum) atomicAdd(&s_near[g], sum);
+    }
+    __syncthreads();
+    if (tid != 0) return;
+    float tiles = 0.f, of = 0.f;
+    for (uint32_t i = 0; i < sensors; ++i) {
+        uint32_t sum = 0;
+        for (uint32_t g = i << a.near_shift; g < (i + 1) << a.near_shift && sum < kNearPerTile * a.n_tiles; ++g) {
+            sum += s_near[g];
+            of += (float)s_of[g];
+        }
+        tiles += (float)sum;
+    }
+    *a.near = of > 0.f && !blk_overflow(a) ? tiles / of : 0.f;
+}
+
 template <bool kWrap>
-__global__ void __launch_bounds__(kBlkThreads)
+__global__ void __launch_bounds__(kBlkThreads, 4)
 blk_count_kernel(BlkArgs a) {
     chain_enter();
     extern __shared__ uint32_t s_cnt[];   // [blocks]
     const bool overflow = blk_overflow(a);
+    if (!kWrap && a.near_host != nullptr && blockIdx.x == min(gridDim.x - 1, kNearCta)) find_near(a);
     const BlkCta c = blk_cta(a);
     const uint2 rect = blk_load_rect(a, c.first + threadIdx.x);
     for (uint32_t k = threadIdx.x; k < a.blocks; k += kBlkThreads) s_cnt[k] = 0u;
@@ -1356,6 +1399,8 @@ blk_scatter_kernel(BlkArgs a) {
     uint32_t *s_base = s_dyn;              // [warps][rows][bx] position of the warp's first record
     uint32_t *s_mask = s_base + plane;     // (kWrap: 4 planes of) [warps][rows][bx] lanes with a record
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lt = (1u << lane) - 1u;
+    if (!kWrap && a.near_host != nullptr && tid == 0 && blockIdx.x == min(gridDim.x - 1, kNearCta) && blockIdx.y == 0)
+        *a.near_host = (int64_t)((uint64_t)a.near_sequence << 32 | __float_as_uint(*a.near));
     const bool overflow = blk_overflow(a);
     const BlkCta c = blk_cta(a);
     const uint32_t entry = c.first + tid;
@@ -1857,6 +1902,7 @@ struct BlkWs {
     uint32_t *rec_start, *unit_start, *unit_cnt, *tile_base;
     uint4 *unit_info;
     uint2 *rec;
+    float *near;
     size_t bytes;
 };
 
@@ -1871,6 +1917,7 @@ static BlkWs carve_blocks(void *ws, uint64_t cap) {
     // a record stands for at least one list entry; every block rounds its records up to whole units
     w.unit_cnt = (uint32_t *)take(sizeof(uint32_t) * 32 * (cap / kBlkUnitMin + kBlkMaxBlocks));
     w.unit_info = (uint4 *)take(sizeof(uint4) * (cap / kBlkUnitMin + kBlkMaxBlocks));
+    w.near = (float *)take(sizeof(float));
     w.rec = (uint2 *)take(sizeof(uint2) * cap);
     w.bytes = off;
     return w;
@@ -2138,7 +2185,29 @@ static int isect_plan(const IsectGeom &g, int32_t *tiles_per_gauss, int sort, vo
     return check_launch("isect plan");
 }
 
-static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int sort,
+// One-shot request of the calling thread's next fill (splatad_isect_set_near_tiles). Where no kernel is to answer it, it is
+// answered here: not known.
+static thread_local int64_t *t_near_host = nullptr;
+static thread_local uint32_t t_near_seq = 0;
+struct NearRequest {
+    int64_t *host = t_near_host;
+    const uint32_t sequence = t_near_seq;
+    NearRequest() { t_near_host = nullptr; }
+    ~NearRequest() {
+        if (host != nullptr) __atomic_store_n(host, (int64_t)((uint64_t)sequence << 32), __ATOMIC_RELEASE);
+    }
+    int64_t *take_on_device() {   // for a kernel that answers
+        void *dptr = nullptr;
+        if (host != nullptr && cudaHostGetDevicePointer(&dptr, host, 0) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        host = nullptr;
+        return (int64_t *)dptr;
+    }
+};
+
+static int isect_fill(const IsectGeom &g, NearRequest &near, const int32_t *tiles_per_gauss, int sort,
                       void *plan_workspace, void *fill_workspace, size_t fill_workspace_bytes,
                       int64_t capacity, int64_t *isect_ids, int32_t *flatten_ids,
                       int32_t *tile_offsets, int64_t *host_counts, cudaStream_t st) {
@@ -2195,6 +2264,10 @@ static int isect_fill(const IsectGeom &g, const int32_t *tiles_per_gauss, int so
         a.total = g.total;
         a.rec_start = w.rec_start; a.unit_start = w.unit_start;
         a.rec = w.rec;
+        a.near = w.near; a.near_host = g.lidar ? nullptr : near.take_on_device(); a.near_sequence = near.sequence;
+        const uint32_t near_sensors = min(g.C, kNearGroups);
+        a.near_shift = bit_length(kNearGroups / near_sensors) - 1;
+        a.near_step = g.C / near_sensors;
         a.unit_cnt = w.unit_cnt; a.unit_info = w.unit_info; a.tile_base = w.tile_base;
         const uint32_t ctas_a = div_up(g.total, kBlkThreads) + (g.C > 1 ? g.C : 0u);
         a.ctas = ctas_a;
@@ -2704,12 +2777,13 @@ extern "C" int splatad_isect_tiles_fill(
     uint32_t tile_height, int32_t sort, const int32_t *tiles_per_gauss, void *plan_workspace,
     void *fill_workspace, size_t fill_workspace_bytes, int64_t capacity, int64_t *isect_ids,
     int32_t *flatten_ids, int32_t *tile_offsets, int64_t *host_counts, void *stream) {
+    NearRequest near;
     if (total_elems == 0 || capacity <= 0) return SPLATAD_OK;
     IsectGeom g;
     int rc = make_cam_geom(g, C, N, total_elems, means2d, radii, depths, camera_ids, tile_size,
                            tile_width, tile_height);
     if (rc != SPLATAD_OK) return rc;
-    return isect_fill(g, tiles_per_gauss, sort, plan_workspace, fill_workspace,
+    return isect_fill(g, near, tiles_per_gauss, sort, plan_workspace, fill_workspace,
                       fill_workspace_bytes, capacity, isect_ids, flatten_ids, tile_offsets, host_counts,
                       (cudaStream_t)stream);
 }
@@ -2744,12 +2818,13 @@ extern "C" int splatad_isect_lidar_tiles_fill(
     const int32_t *tiles_per_gauss, void *plan_workspace, void *fill_workspace,
     size_t fill_workspace_bytes, int64_t capacity, int64_t *isect_ids, int32_t *flatten_ids,
     int32_t *tile_offsets, int64_t *host_counts, void *stream) {
+    NearRequest near;   // (lidar lists: not known)
     if (total_elems == 0 || capacity <= 0) return SPLATAD_OK;
     IsectGeom g;
     int rc = make_lidar_geom(g, C, N, total_elems, means2d, radii, depths, camera_ids,
                              elev_boundaries, n_boundaries, tile_azim_resolution, min_azim);
     if (rc != SPLATAD_OK) return rc;
-    return isect_fill(g, tiles_per_gauss, sort, plan_workspace, fill_workspace,
+    return isect_fill(g, near, tiles_per_gauss, sort, plan_workspace, fill_workspace,
                       fill_workspace_bytes, capacity, isect_ids, flatten_ids, tile_offsets, host_counts,
                       (cudaStream_t)stream);
 }
@@ -2762,6 +2837,12 @@ extern "C" int splatad_isect_set_early_count(int64_t *host_pair, int64_t sequenc
 
 extern "C" int splatad_isect_set_listed_count(int64_t *host_word) {
     t_listed_host = host_word;
+    return SPLATAD_OK;
+}
+
+extern "C" int splatad_isect_set_near_tiles(int64_t *host_word, uint32_t sequence) {
+    t_near_host = host_word;
+    t_near_seq = sequence;
     return SPLATAD_OK;
 }
 

@@ -981,10 +981,12 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
     def fill(capacity):
         isect_ids = torch.empty(capacity, dtype=torch.int64, device=dev)
         flatten_ids = torch.empty(capacity, dtype=torch.int32, device=dev)
-        offsets = None
+        offsets, near = None, float
         if capacity > 0:
             fill_ws = None
             if sort:
+                if kind == "tiles" and n_tiles_total * geom_args[0] ** 2 >= 900 * 256:   # fewer take no kernel that asks
+                    near = _lib.NearRequest(dev)
                 fill_bytes = lib.splatad_isect_fill_workspace_bytes(capacity)
                 fill_ws = _lib.workspace("isect_fill", fill_bytes, dev)
                 # the fill knows where every tile starts (and appends the total); kept for
@@ -994,7 +996,7 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
                   _lib.ptr(tiles_per_gauss), _lib.ptr(plan_ws), _lib.ptr(fill_ws),
                   fill_ws.numel() if fill_ws is not None else 0, capacity, _lib.ptr(isect_ids),
                   _lib.ptr(flatten_ids), _lib.ptr(offsets), None, stream)
-        return isect_ids, flatten_ids, offsets
+        return isect_ids, flatten_ids, offsets, near
 
     def read_count(slot=None, words=None, sequence=0, event=None):
         if slot is None:
@@ -1023,11 +1025,12 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
             plan()
             torch.cuda.current_stream(dev).synchronize()
             n_isects, listed = read_count()
-        isect_ids, flatten_ids, offsets = fill(n_isects)
+        isect_ids, flatten_ids, offsets, near = fill(n_isects)
         if offsets is not None:
             isect_ids._splatad_tile_offsets = (C, offsets[:n_tiles_total])
         if listed > 0:
             _spread_hint[key] = flatten_ids._splatad_spread = n_isects / listed
+            flatten_ids._splatad_counts = _ReadOnce(lambda: (n_isects, listed, near()))
         return tiles_per_gauss, isect_ids, flatten_ids
 
     if not deferred:
@@ -1042,7 +1045,7 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
     # behind the plan is the fallback
     sequence = _lib.next_sequence()
     lib.splatad_isect_set_early_count(slot.data_ptr() + 32, sequence)
-    words = slot.numpy()
+    words = slot._splatad_words
     words[9] = 0
     lib.splatad_isect_set_listed_count(slot.data_ptr() + 72)
     try:
@@ -1053,8 +1056,9 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
         raise
     counted = torch.cuda.Event()
     counted.record(torch.cuda.current_stream(dev))
-    isect_buf, flat_buf, offsets = fill(capacity)
-    count = flat_buf._splatad_counts = _ReadOnce(lambda: read_count(slot, words, sequence, counted))
+    isect_buf, flat_buf, offsets, near = fill(capacity)
+    count = _ReadOnce(lambda: (*read_count(slot, words, sequence, counted), near()))
+    flat_buf._splatad_counts = count
     return DeferredIsect(tiles_per_gauss, isect_buf, flat_buf, offsets, C, n_tiles_total, capacity, count, exact)
 
 
@@ -1067,7 +1071,8 @@ _depth_sort_mode: dict = {}   # same keys -> 2 once a frame of the shape needed 
 
 
 class _ReadOnce:
-    """(list entries, elements listed) of a plan, read when first asked for: whoever asks waits until they are there."""
+    """(list entries, elements listed, tiles that a near one covers) of a frame's lists, read when first asked for: whoever
+    asks waits until they are there."""
 
     def __init__(self, read):
         self._read, self._value = read, None
@@ -1439,7 +1444,8 @@ def rasterize_to_pixels(
     # when everything before it is enqueued); chooses the split of the work
     spread = getattr(flatten_ids, "_splatad_counts", None) or (
         getattr(flatten_ids, "_splatad_spread", 0.0),
-        getattr(flatten_ids, "_splatad_count", 0 if total_follows else flatten_ids.numel()))
+        getattr(flatten_ids, "_splatad_count", 0 if total_follows else flatten_ids.numel()),
+        getattr(flatten_ids, "_splatad_near", 0.0))
     tail = (image_width, image_height, tile_size, isect_offsets.contiguous(), flatten_ids.contiguous(),
             absgrad, total_follows, spread)
     if channels <= _lib.MAX_CHANNELS:
@@ -1457,10 +1463,18 @@ def rasterize_to_pixels(
     return torch.cat(renders, dim=-1), alphas
 
 
+def _hint_counts(spread: float, count: int, near: float) -> None:
+    """What the lists of this thread's next camera compositing call hold, as far as it is known."""
+    lib = _lib.load()
+    lib.splatad_rasterize_set_spread_hint(spread, count)
+    if near > 0.0:
+        lib.splatad_rasterize_set_near_hint(near)
+
+
 class _RasterizeToPixels(torch.autograd.Function):
     @staticmethod
     def forward(ctx, means2d, conics, colors, opacities, pix_vels, rolling_shutter_time, backgrounds,
-                width, height, tile_size, isect_offsets, flatten_ids, absgrad, total_follows=False, spread=(0.0, 0)):
+                width, height, tile_size, isect_offsets, flatten_ids, absgrad, total_follows=False, spread=(0.0, 0, 0.0)):
         dev = means2d.device
         assert means2d.dtype == torch.float32, means2d.dtype
         C, tile_h, tile_w = isect_offsets.shape
@@ -1474,10 +1488,10 @@ class _RasterizeToPixels(torch.autograd.Function):
         n_isects = _n_isects_arg(isect_offsets, flatten_ids, total_follows)
         _debug_check_lists("rasterize_to_pixels", flatten_ids, means2d.numel() // 2, isect_offsets, total_follows)
         if isinstance(spread, _ReadOnce):
-            count, listed = spread()
-            spread = (count / listed, count) if listed > 0 else (0.0, 0)
+            count, listed, near = spread()
+            spread = (count / listed, count, near) if listed > 0 else (0.0, 0, 0.0)
         ctx.n_isects_arg, ctx.spread = n_isects, spread
-        _lib.load().splatad_rasterize_set_spread_hint(*spread)
+        _hint_counts(*spread)
         _call(
             "splatad_rasterize_to_pixels_fwd", C, n_isects, _lib.ptr(means2d), _lib.ptr(conics_f),
             _lib.ptr(colors_f), channels, _lib.ptr(opac_f), _lib.ptr(vels_f), _lib.ptr(rs), _lib.ptr(bg),
@@ -1500,7 +1514,7 @@ class _RasterizeToPixels(torch.autograd.Function):
         v_render_alphas = _f(v_render_alphas)
         v_means2d, v_conics, v_colors, v_opacities, v_pix_vels, v_abs = _zeros_like_many(
             means2d, conics, colors, opacities, pix_vels, means2d if ctx.absgrad else None)
-        _lib.load().splatad_rasterize_set_spread_hint(*ctx.spread)
+        _hint_counts(*ctx.spread)
         _call(
             "splatad_rasterize_to_pixels_bwd", C, ctx.n_isects_arg, _lib.ptr(means2d),
             _lib.ptr(conics), _lib.ptr(colors), channels, _lib.ptr(opacities), _lib.ptr(pix_vels),

@@ -514,7 +514,7 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, 
     for spread, count in ((0.0, 0), (100.0, 10**8)):
         image, alphas = torch.empty(C, H, W, channels, device=DEV), torch.empty(C, H, W, 1, device=DEV)
         last = torch.empty(C, H, W, dtype=torch.int32, device=DEV)
-        lib.splatad_rasterize_set_spread_hint(spread, count)
+        lib.splatad_rasterize_set_spread_hint(spread, count), lib.splatad_rasterize_set_near_hint(4 * spread)
         _, (name,) = launched(lambda: _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last),
                                                 _lib.stream_ptr(ids.device)))
         assert name.endswith(",runs") == (spread > 0 and channels <= 4 and ts != 24), name
@@ -526,7 +526,7 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, 
             assert torch.equal(got, expect)
         v = {k: torch.zeros_like(dev[k]) for k in keys}
         v_abs = torch.zeros_like(dev["means2d"]) if absgrad else None
-        lib.splatad_rasterize_set_spread_hint(spread, count)
+        lib.splatad_rasterize_set_spread_hint(spread, count), lib.splatad_rasterize_set_near_hint(4 * spread)
         _, (name,) = launched(lambda: _lib.call(
             "splatad_rasterize_to_pixels_bwd", *head, p(alphas), p(last), p(cotangents[0]), p(cotangents[1]), p(v_abs),
             *(p(v[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")), _lib.stream_ptr(ids.device)))
@@ -537,14 +537,17 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, 
             _grad_check(f"spread {spread} absgrad", v_abs, ref["v_means2d_abs"].reshape(v_abs.shape))
 
 
-@pytest.mark.parametrize("C,W,H,ts,spread,per_tile,forward,backward", [
-    (2, 640, 360, 16, 68.0, 573, False, True), (2, 640, 360, 16, 38.0, 1400, True, True), (1, 1280, 720, 16, 59.0, 596, False, True),
-    (1, 1280, 720, 16, 23.0, 2296, True, True), (2, 1280, 720, 16, 81.0, 162, False, True), (2, 1280, 720, 16, 79.0, 316, True, True),
-    (3, 1440, 430, 16, 43.0, 372, False, True), (4, 640, 800, 16, 31.0, 439, True, True), (1, 1920, 1080, 16, 27.0, 1171, True, True),
-    (1, 1920, 1080, 16, 16.0, 682, False, False), (1, 640, 360, 16, 79.0, 3643, False, True), (1, 480, 270, 16, 79.0, 9000, False, False),
-    (1, 1280, 720, 24, 59.0, 5000, False, False), (1, 1280, 720, 32, 20.0, 5000, True, True)])
-def test_runs_are_for_dense_lists_of_large_gaussians(C, W, H, ts, spread, per_tile, forward, backward):
-    """Which camera kernels a hint chooses, on both sides of each line: sparse lists, few tiles, rows that leave lanes over."""
+@pytest.mark.parametrize("C,W,H,ts,spread,per_tile,near,forward,backward", [
+    (2, 640, 360, 16, 68.0, 573, 900, False, True), (2, 640, 360, 16, 38.0, 1400, 900, True, True), (1, 1280, 720, 16, 59.0, 596, 900, False, True),
+    (1, 1280, 720, 16, 23.0, 2296, 900, True, True), (2, 1280, 720, 16, 81.0, 162, 900, False, True), (2, 1280, 720, 16, 79.0, 316, 900, True, True),
+    (3, 1440, 430, 16, 43.0, 372, 900, False, True), (4, 640, 800, 16, 31.0, 439, 900, True, True), (1, 1920, 1080, 16, 27.0, 1171, 900, True, True),
+    (1, 1920, 1080, 16, 16.0, 682, 900, False, False), (1, 640, 360, 16, 79.0, 3643, 900, False, True), (1, 480, 270, 16, 79.0, 9000, 900, False, False),
+    (1, 1280, 720, 24, 59.0, 5000, 900, False, False), (1, 1280, 720, 32, 20.0, 5000, 300, True, True), (1, 1920, 1080, 16, 27.0, 1171, 349, False, True),
+    (1, 1920, 1080, 16, 27.0, 1171, 351, True, True), (1, 1920, 1080, 16, 37.0, 9673, 40, False, False), (1, 1920, 1080, 16, 27.0, 1171, 176, False, True),
+    (1, 1920, 1080, 16, 27.0, 1171, 0, False, False)])
+def test_runs_are_for_dense_lists_of_large_gaussians(C, W, H, ts, spread, per_tile, near, forward, backward):
+    """Which camera kernels the hints choose, on both sides of each line: near Gaussians that are small or of no known size, sparse lists, few
+    tiles, rows that leave lanes over."""
     from splatad_b200 import _lib
     lib, p = _lib.load(), _lib.ptr
     tw, th = -(-W // ts), -(-H // ts)
@@ -556,9 +559,9 @@ def test_runs_are_for_dense_lists_of_large_gaussians(C, W, H, ts, spread, per_ti
     entries = per_tile * C * tw * th
 
     def both():
-        lib.splatad_rasterize_set_spread_hint(spread, entries)
+        lib.splatad_rasterize_set_spread_hint(spread, entries), lib.splatad_rasterize_set_near_hint(near)
         _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last), _lib.stream_ptr(ids.device))
-        lib.splatad_rasterize_set_spread_hint(spread, entries)
+        lib.splatad_rasterize_set_spread_hint(spread, entries), lib.splatad_rasterize_set_near_hint(near)
         _lib.call("splatad_rasterize_to_pixels_bwd", *head, p(alphas), p(last), p(image), p(alphas), None, *(p(g) for g in grads),
                   _lib.stream_ptr(ids.device))
 
@@ -584,7 +587,7 @@ def test_runs_of_thousands_of_faint_entries():
     for hint, runs in (((0.0, 0), False), ((100.0, 10**8), True)):
         image, alphas = torch.empty(C, H, W, 3, device=DEV), torch.empty(C, H, W, 1, device=DEV)
         last = torch.empty(C, H, W, dtype=torch.int32, device=DEV)
-        lib.splatad_rasterize_set_spread_hint(*hint)
+        lib.splatad_rasterize_set_spread_hint(*hint), lib.splatad_rasterize_set_near_hint(4 * hint[0])
         _, (name,) = launched(lambda: _lib.call(
             "splatad_rasterize_to_pixels_fwd", C, ids.numel(), *(p(x) for x in dev[:3]), 3, *(p(x) for x in dev[3:]), None, W, H, ts, tw, th,
             p(offsets), p(ids), p(image), p(alphas), p(last), _lib.stream_ptr(ids.device)))
@@ -621,7 +624,7 @@ def test_runs_with_values_that_are_not_finite(what, channels, absgrad):
     for hint in hints:
         image, alphas = torch.empty(C, H, W, channels, device=DEV), torch.empty(C, H, W, 1, device=DEV)
         last = torch.empty(C, H, W, dtype=torch.int32, device=DEV)
-        lib.splatad_rasterize_set_spread_hint(*hint)
+        lib.splatad_rasterize_set_spread_hint(*hint), lib.splatad_rasterize_set_near_hint(4 * hint[0])
         _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last), _lib.stream_ptr(ids.device))
         results.append((image, alphas, last))
     (image, alphas, last), (image_r, alphas_r, last_r) = results
@@ -631,7 +634,7 @@ def test_runs_with_values_that_are_not_finite(what, channels, absgrad):
         grads = {k: torch.zeros_like(dev[k]) for k in keys}
         if absgrad:
             grads["absgrad"] = torch.zeros_like(dev["means2d"])
-        lib.splatad_rasterize_set_spread_hint(*hint)
+        lib.splatad_rasterize_set_spread_hint(*hint), lib.splatad_rasterize_set_near_hint(4 * hint[0])
         _, (name,) = launched(lambda: _lib.call(
             "splatad_rasterize_to_pixels_bwd", *head, p(alphas_h), p(last_h), p(v_c), p(v_a), p(grads.get("absgrad")),
             *(p(grads[k]) for k in ("means2d", "conics", "colors", "opacities", "pix_vels")), _lib.stream_ptr(ids.device)))

@@ -45,14 +45,16 @@ def test_a_frame_reports_how_many_tiles_its_gaussians_cover(packed):
 
 @pytest.mark.parametrize("packed,pose", [(False, False), (True, False), (False, True)])
 def test_a_frame_is_split_by_its_own_counts(packed, pose):
-    """Two scenes of one shape in turn, one of large Gaussians and one of small ones: each takes the compositing kernels it
-    takes by itself, forward and backward, in native frames and (with a pose that is optimised) by the ops."""
+    """Scenes of one shape in turn - Gaussians that are large where they are near, small ones, and ones that all cover 36 tiles or so, whose
+    lists are as long and whose patches few of them cover: each takes the compositing kernels it takes by itself, and only the first those
+    with runs, forward and backward, in native frames and (with a pose that is optimised) by the ops."""
     import splatad_b200
     from splatad_b200 import scenes
     g = _to_gpu(scenes.config1(N=150_011, packed=packed))
     if pose:
         g["viewmats"] = g["viewmats"].clone().requires_grad_(True)
-    scales = {"large": g["scales"] * 1.5, "small": g["scales"] * 0.25}
+    even = g["means"][:, 2:].clamp(min=0.3) * (12.0 / 1200.0)
+    scales = {"large": g["scales"] * 1.5, "small": g["scales"] * 0.25, "even": even.expand(-1, 3) * 1.0}
 
     def step(which):
         leaf = scales[which].clone().requires_grad_(True)
@@ -68,8 +70,9 @@ def test_a_frame_is_split_by_its_own_counts(packed, pose):
         _forget()
         for _ in range(3):
             alone[which] = kernels(which)
-    assert all(k.endswith(",runs") for k in alone["large"]) and not any(k.endswith(",runs") for k in alone["small"])
-    for which in ("large", "small", "large", "small", "small", "large"):
+    assert all(k.endswith(",runs") for k in alone["large"])
+    assert not any(k.endswith(",runs") for which in ("small", "even") for k in alone[which])
+    for which in ("large", "small", "large", "even", "small", "small", "even", "large"):
         assert kernels(which) == alone[which], which
 
 

@@ -368,6 +368,87 @@ def test_list_kernels_by_the_room_for_entries(capacity, kernel, ids_off, flat_of
         assert (buffer[:off] == -7).all() and (buffer[off + size: off + size + 8] == -7).all()
 
 
+@pytest.mark.parametrize("radix", [False, True])
+@pytest.mark.parametrize("C,N,tw,th,r", [(1, 5000, 60, 15, 9), (1, 300, 31, 30, 60), (1, 9000, 40, 30, 200), (2, 2600, 25, 18, 40), (3, 1500, 20, 15, 5),
+                                         (6, 700, 30, 20, 30), (9, 600, 12, 9, 25), (20, 520, 9, 5, 12), (1, 5000, 20, 13, 9)])
+def test_how_many_tiles_a_near_gaussian_covers(C, N, tw, th, r, radix, monkeypatch):
+    """What a fill reports about the first entries in depth order is what their rectangles say."""
+    from splatad_b200 import ops
+    g = torch.Generator().manual_seed(C * N)
+    means2d = (torch.rand(C, N, 2, generator=g) * 1.2 - 0.1) * torch.tensor([16.0 * tw, 16.0 * th])
+    radii = torch.randint(0, 2 * r, (C, N, 2), generator=g, dtype=torch.int32)
+    depths = torch.rand(C, N, generator=g) * 30 + 0.5
+    args = (t(means2d), t(radii, torch.int32), t(depths), 16, tw, th)
+    if radix:
+        monkeypatch.setattr(ops, "_depth_sort_mode", _AlwaysRadix())
+    tiles = n(ops.isect_tiles_deferred(*args).tiles_per_gauss).astype(np.int64)
+    n_isects, listed, near = ops.isect_tiles_deferred(*args).flatten_ids._splatad_counts()
+    if C * tw * th < 900:
+        assert near == 0.0   # (nobody asks)
+        return
+    assert n_isects == tiles.sum() and listed == (tiles > 0).sum()
+    sensors, total, of = min(C, 8), 0, 0
+    for i in range(sensors):
+        c = i * (C // sensors)
+        order = np.argsort(n(depths)[c], kind="stable")
+        order, seen = order[tiles[c][order] > 0], 0
+        for k in range({1: 8, 2: 4, 3: 2, 4: 2}.get(sensors, 1)):
+            group = order[512 * k: 512 * (k + 1)]
+            if seen >= 32 * tw * th:
+                break
+            seen, of = seen + tiles[c][group].sum(), of + len(group)
+        total += seen
+    assert near == pytest.approx(total / of, rel=1e-6)
+
+
+def test_near_tiles_are_always_answered(monkeypatch):
+    """Where no kernel reports them - lists that outgrow their room, a grid beyond the block split, unsorted output, lidar tiles, nothing to
+    list - the answer is 0, and a request is never left for the next call."""
+    from splatad_b200 import _lib, ops, scenes
+    lib = _lib.load()
+    words = torch.zeros(1, dtype=torch.int64).pin_memory()
+    monkeypatch.setattr(_lib, "NearRequest", lambda device: float)   # this test asks itself
+    g = torch.Generator().manual_seed(4)
+
+    def answered(sequence, call):
+        words[0] = -1
+        lib.splatad_isect_set_near_tiles(words.data_ptr(), sequence)
+        call()
+        torch.cuda.synchronize()
+        assert int(words[0]) >> 32 == sequence, sequence
+        return int(words[0]) & 0xFFFFFFFF
+
+    def cam(N=900, tw=20, th=10, **kw):
+        means2d = torch.rand(1, N, 2, generator=g) * torch.tensor([16.0 * tw, 16.0 * th])
+        radii = torch.randint(1, 30, (1, N, 2), generator=g, dtype=torch.int32)
+        return ops.isect_tiles(t(means2d), t(radii, torch.int32), t(torch.rand(1, N, generator=g)), 16, tw, th, **kw)
+
+    assert answered(1, cam) > 0
+    assert answered(2, lambda: cam(sort=False)) == 0
+    assert answered(3, lambda: cam(tw=256, th=136)) == 0
+    eb = scenes.elevation_boundaries(scenes.beams_128(), 8)
+    assert answered(4, lambda: _run_lidar(torch.rand(1, 500, 2, generator=g) * 20, torch.rand(1, 500, 2, generator=g) + 1, torch.rand(1, 500, generator=g),
+                                          eb, 6.4, -180.0)) == 0
+    call = ops._call
+
+    def short(name, *args):   # room for three entries
+        if name == "splatad_isect_tiles_fill":
+            args = (*args[:-6], 3, *args[-5:])
+        return call(name, *args)
+
+    with monkeypatch.context() as patch:
+        patch.setattr(ops, "_call", short)
+        assert answered(5, cam) == 0
+    p = _lib.ptr
+    one = torch.zeros(8, device=DEV)
+    assert answered(6, lambda: lib.splatad_isect_tiles_fill(1, 0, 0, *[p(one)] * 4, 16, 4, 4, 1, p(one), p(one), p(one), 32, 8, p(one), p(one), None, None,
+                                                            None)) == 0
+    words[0] = 0
+    cam()                                             # nothing is asked for any more
+    torch.cuda.synchronize()
+    assert int(words[0]) == 0
+
+
 @pytest.mark.parametrize("turns", [0.3, 0.99, 1.0, 1.01, 2.4, 4.5])
 def test_block_split_of_rectangles_around_the_turn(turns):
     """Lidar rectangles that wrap past the last azimuth tile, end just short of or just past a full
