@@ -365,7 +365,8 @@ int splatad_isect_set_listed_count(int64_t *host_word);
 /* No counterpart in the reference. Arms a one-shot request for the NEXT _fill call of the calling thread: *host_word, pinned (mapped)
  * host memory, receives sequence << 32 | how many tiles one of the nearest Gaussians covers on the average, as the bit pattern of a
  * float (0: not known), by a kernel of the fill early on or, where none reports it (lidar tiles, unsorted output, grids
- * beyond the block split, an error), by the call itself. It is always answered. NULL disarms. */
+ * beyond the block split, an error), by the call itself. Not answered where there are fewer than 10000 list entries per tile, counted
+ * n_isects * n_isects / listed elements: no compositing call asks then. NULL disarms. */
 int splatad_isect_set_near_tiles(int64_t *host_word, uint32_t sequence);
 
 /* No counterpart in the reference. Arms a one-shot hint for the NEXT _plan call of the calling

@@ -850,7 +850,9 @@ py::object camera_frame(const Tensor &means, const Tensor &quats, const Tensor &
                     if ((i & 4095u) == 4095u && stream.query()) break;
                 nnz = load_word(slot.word + 8);
             }
-            if (ask_near) {
+            // (with room to spare below what is told, and below what a kernel with runs wants)
+            if (ask_near && usable(counts, capacity) &&
+                (double)counts.n_isects * (double)counts.n_isects >= 11000. * (double)(C * tile_w * tile_h) * (double)std::max<int64_t>(counts.listed, 1)) {
                 int64_t word;
                 for (uint32_t i = 0; (uint32_t)((uint64_t)(word = load_word(slot.word + 10)) >> 32) != (uint32_t)sequence; ++i, pause())
                     if ((i & 4095u) == 4095u && stream.query()) break;

@@ -1154,6 +1154,7 @@ struct BlkArgs {
     float *near;                  // [1] tiles that a near entry covers, where asked for
     volatile int64_t *near_host;  // who asks: sequence << 32 | the float's bits; may be null
     uint32_t near_sequence;
+    float near_least;             // list entries squared per element listed from which on it is told
     uint32_t near_shift, near_step;   // 512s of each sensor that is looked at (log2), and every how manieth sensor is
 };
 
@@ -1399,8 +1400,11 @@ blk_scatter_kernel(BlkArgs a) {
     uint32_t *s_base = s_dyn;              // [warps][rows][bx] position of the warp's first record
     uint32_t *s_mask = s_base + plane;     // (kWrap: 4 planes of) [warps][rows][bx] lanes with a record
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lt = (1u << lane) - 1u;
-    if (!kWrap && a.near_host != nullptr && tid == 0 && blockIdx.x == min(gridDim.x - 1, kNearCta) && blockIdx.y == 0)
-        *a.near_host = (int64_t)((uint64_t)a.near_sequence << 32 | __float_as_uint(*a.near));
+    if (!kWrap && a.near_host != nullptr && tid == 0 && blockIdx.x == min(gridDim.x - 1, kNearCta) && blockIdx.y == 0) {
+        const float n = (float)a.counters[CNT_NISECT];   // short lists: nobody waits, and the store would outlast a short kernel (1 us)
+        if (n * n >= a.near_least * (float)a.counters[CNT_NVIS])
+            *a.near_host = (int64_t)((uint64_t)a.near_sequence << 32 | __float_as_uint(*a.near));
+    }
     const bool overflow = blk_overflow(a);
     const BlkCta c = blk_cta(a);
     const uint32_t entry = c.first + tid;
@@ -2265,6 +2269,7 @@ static int isect_fill(const IsectGeom &g, NearRequest &near, const int32_t *tile
         a.rec_start = w.rec_start; a.unit_start = w.unit_start;
         a.rec = w.rec;
         a.near = w.near; a.near_host = g.lidar ? nullptr : near.take_on_device(); a.near_sequence = near.sequence;
+        a.near_least = 10000.f * (float)(g.C * g.n_tiles);
         const uint32_t near_sensors = min(g.C, kNearGroups);
         a.near_shift = bit_length(kNearGroups / near_sensors) - 1;
         a.near_step = g.C / near_sensors;

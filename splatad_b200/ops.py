@@ -1016,6 +1016,10 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
             return -1, 0       # the depth buckets were too crowded: the order is not final
         return n_isects, listed if sort else 0
 
+    def with_near(n_isects, listed, near):
+        # told from 10000 on, of no use below 12500
+        return n_isects, listed, near() if n_isects * n_isects >= 11000 * n_tiles_total * max(listed, 1) else 0.0
+
     def exact():
         plan()
         torch.cuda.current_stream(dev).synchronize()
@@ -1030,7 +1034,7 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
             isect_ids._splatad_tile_offsets = (C, offsets[:n_tiles_total])
         if listed > 0:
             _spread_hint[key] = flatten_ids._splatad_spread = n_isects / listed
-            flatten_ids._splatad_counts = _ReadOnce(lambda: (n_isects, listed, near()))
+            flatten_ids._splatad_counts = _ReadOnce(lambda: with_near(n_isects, listed, near))
         return tiles_per_gauss, isect_ids, flatten_ids
 
     if not deferred:
@@ -1057,7 +1061,7 @@ def _isect_common(kind, means2d, radii, depths, packed, n_cameras, camera_ids, g
     counted = torch.cuda.Event()
     counted.record(torch.cuda.current_stream(dev))
     isect_buf, flat_buf, offsets, near = fill(capacity)
-    count = _ReadOnce(lambda: (*read_count(slot, words, sequence, counted), near()))
+    count = _ReadOnce(lambda: with_near(*read_count(slot, words, sequence, counted), near))
     flat_buf._splatad_counts = count
     return DeferredIsect(tiles_per_gauss, isect_buf, flat_buf, offsets, C, n_tiles_total, capacity, count, exact)
 

@@ -369,8 +369,8 @@ def test_list_kernels_by_the_room_for_entries(capacity, kernel, ids_off, flat_of
 
 
 @pytest.mark.parametrize("radix", [False, True])
-@pytest.mark.parametrize("C,N,tw,th,r", [(1, 5000, 60, 15, 9), (1, 300, 31, 30, 60), (1, 9000, 40, 30, 200), (2, 2600, 25, 18, 40), (3, 1500, 20, 15, 5),
-                                         (6, 700, 30, 20, 30), (9, 600, 12, 9, 25), (20, 520, 9, 5, 12), (1, 5000, 20, 13, 9)])
+@pytest.mark.parametrize("C,N,tw,th,r", [(1, 5000, 60, 15, 200), (1, 300, 31, 30, 300), (1, 9000, 40, 30, 200), (2, 2600, 25, 18, 140), (3, 1500, 20, 15, 130),
+                                         (6, 700, 30, 20, 300), (9, 600, 12, 9, 200), (20, 520, 9, 5, 250), (1, 5000, 20, 13, 90), (1, 5000, 60, 15, 9)])
 def test_how_many_tiles_a_near_gaussian_covers(C, N, tw, th, r, radix, monkeypatch):
     """What a fill reports about the first entries in depth order is what their rectangles say."""
     from splatad_b200 import ops
@@ -383,8 +383,8 @@ def test_how_many_tiles_a_near_gaussian_covers(C, N, tw, th, r, radix, monkeypat
         monkeypatch.setattr(ops, "_depth_sort_mode", _AlwaysRadix())
     tiles = n(ops.isect_tiles_deferred(*args).tiles_per_gauss).astype(np.int64)
     n_isects, listed, near = ops.isect_tiles_deferred(*args).flatten_ids._splatad_counts()
-    if C * tw * th < 900:
-        assert near == 0.0   # (nobody asks)
+    if C * tw * th < 900 or r < 50:
+        assert near == 0.0   # (few tiles, short lists: nobody asks)
         return
     assert n_isects == tiles.sum() and listed == (tiles > 0).sum()
     sensors, total, of = min(C, 8), 0, 0
@@ -403,7 +403,7 @@ def test_how_many_tiles_a_near_gaussian_covers(C, N, tw, th, r, radix, monkeypat
 
 def test_near_tiles_are_always_answered(monkeypatch):
     """Where no kernel reports them - lists that outgrow their room, a grid beyond the block split, unsorted output, lidar tiles, nothing to
-    list - the answer is 0, and a request is never left for the next call."""
+    list - the answer is 0, and a request is never left for the next call. (Short lists alone go without an answer.)"""
     from splatad_b200 import _lib, ops, scenes
     lib = _lib.load()
     words = torch.zeros(1, dtype=torch.int64).pin_memory()
@@ -418,9 +418,9 @@ def test_near_tiles_are_always_answered(monkeypatch):
         assert int(words[0]) >> 32 == sequence, sequence
         return int(words[0]) & 0xFFFFFFFF
 
-    def cam(N=900, tw=20, th=10, **kw):
+    def cam(N=900, tw=20, th=10, r=600, **kw):
         means2d = torch.rand(1, N, 2, generator=g) * torch.tensor([16.0 * tw, 16.0 * th])
-        radii = torch.randint(1, 30, (1, N, 2), generator=g, dtype=torch.int32)
+        radii = torch.randint(1, r, (1, N, 2), generator=g, dtype=torch.int32)
         return ops.isect_tiles(t(means2d), t(radii, torch.int32), t(torch.rand(1, N, generator=g)), 16, tw, th, **kw)
 
     assert answered(1, cam) > 0
@@ -444,6 +444,8 @@ def test_near_tiles_are_always_answered(monkeypatch):
     assert answered(6, lambda: lib.splatad_isect_tiles_fill(1, 0, 0, *[p(one)] * 4, 16, 4, 4, 1, p(one), p(one), p(one), 32, 8, p(one), p(one), None, None,
                                                             None)) == 0
     words[0] = 0
+    lib.splatad_isect_set_near_tiles(words.data_ptr(), 7)
+    cam(r=30)
     cam()                                             # nothing is asked for any more
     torch.cuda.synchronize()
     assert int(words[0]) == 0
