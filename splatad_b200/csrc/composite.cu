@@ -2692,11 +2692,13 @@ static bool many_entries(float spread, int64_t entries, int64_t line, float or_s
 // and 791 (48 k) 271 and 250; 3600, 14 and 1354 (19 k) 174 and 162; 2040, 9 and 1546 (14 k) 132 and 118, 35 and 629 (22 k) 124 and 109, 25 and 2252 (57 k) 104 and 86; 1840, 39 and 319 (13
 // k) 98 and 91; 1450, 13 and 995 (13 k) 108 and 72; 920, 9 and 3660 (34 k) 90 and 66. With 8 / 14 channels: 8160, 57 and 251 420 / 610 and 410 / 606, 60 and 791 425 / 608 and 397 / 591; 3600, 14 and 1354 250 /
 // 348 and 235 / 342; 2040, 9 and 1546 173 / 227 and 158 / 220, with absolute gradients 191 / 244 and 172 / 232 (fewer tiles take two pixels per lane and no runs).
-static bool covers_patches(uint64_t blocks, uint32_t tile_size, float spread, int64_t entries, float near, bool backward) {
+// Five to eight channels, backward: not where the warps without runs, twenty an SM, just fit at once and the sixteen with do not (1500 tiles 122 and 129,
+// 1550: 1.06 to 1.15 times as fast with runs in all of eighteen scenes).
+static bool covers_patches(uint64_t blocks, uint32_t tile_size, uint32_t channels, float spread, int64_t entries, float near, bool backward) {
     const uint32_t tiles = tiles_of_256(blocks, tile_size);
     const double product = (double)spread * (double)entries;   // times the tiles
     if (entries <= 0 || !(near >= (backward ? 175.f : 350.f)) || tile_threads<8>(tile_size) % 32u != 0u) return false;
-    if (backward) return tiles >= 900u && product >= 12500.0 * tiles;
+    if (backward) return tiles >= (channels > 4u && channels <= 8u ? 1530u : 900u) && product >= 12500.0 * tiles;
     if (tiles < 1800u || entries < 2200000) return false;
     return product >= (tiles < 5000u ? 30000.0 : entries < 400 * (int64_t)tiles ? 17000.0 : 12500.0) * tiles;
 }
@@ -2841,7 +2843,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_fwd(
     }
 #define CALL(D)                                                                                   \
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2)) else if (D <= 16 && px == 4) CALL_PX(D, (D <= 16 ? 4 : 2)) else CALL_PX(D, 2)
-    const bool runs = channels <= 4 && covers_patches(blocks, tile_size, hint.spread, hint.entries, hint.near, false);
+    const bool runs = channels <= 4 && covers_patches(blocks, tile_size, channels, hint.spread, hint.entries, hint.near, false);
     const uint32_t px = runs ? 8u : pixels_per_lane_fwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool vec = channels % 4u == 0u && (reinterpret_cast<uintptr_t>(colors) & 15u) == 0u;
     {
@@ -2916,7 +2918,7 @@ extern "C" int splatad_rasterize_expected_to_pixels_bwd(
     if (D <= 4 && px == 8) CALL_PX(D, (D <= 4 ? 8 : 2), A) else if (D <= 20 && px == 4) CALL_PX(D, (D <= 20 ? 4 : 2), A) else CALL_PX(D, 2, A)
 #define CALL(D)                                                                                   \
     if (v_means2d_abs) CALL_ABS(D, true) else CALL_ABS(D, false)
-    const bool runs = covers_patches(blocks, tile_size, hint.spread, hint.entries, hint.near, true);
+    const bool runs = covers_patches(blocks, tile_size, channels, hint.spread, hint.entries, hint.near, true);
     const uint32_t px = runs && channels <= 4 ? 8u : pixels_per_lane_bwd(blocks, tile_size, channels, hint.spread, hint.entries);
     const bool other = pixels_bwd_other(blocks, tile_size, channels, px, hint.spread);
     {

@@ -537,6 +537,35 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, 
             _grad_check(f"spread {spread} absgrad", v_abs, ref["v_means2d_abs"].reshape(v_abs.shape))
 
 
+def _chosen(C, W, H, ts, spread, per_tile, near, channels):
+    """Names of the forward and the backward kernel that hints choose; drawn are empty lists."""
+    from splatad_b200 import _lib
+    lib, p = _lib.load(), _lib.ptr
+    tw, th = -(-W // ts), -(-H // ts)
+    offsets, ids = torch.ones(C, th, tw, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)   # empty lists
+    image, alphas, one = torch.empty(C, H, W, channels, device=DEV), torch.zeros(C, H, W, 1, device=DEV), torch.zeros(32, device=DEV)
+    last, rs = torch.full((C, H, W), -1, dtype=torch.int32, device=DEV), torch.zeros(C, device=DEV)
+    head = (C, 1, p(one), p(one), p(one), channels, p(one), p(one), p(rs), None, W, H, ts, tw, th, p(offsets), p(ids))
+    grads = [torch.zeros(32, device=DEV) for _ in range(5)]
+    entries = per_tile * C * tw * th
+
+    def both():
+        lib.splatad_rasterize_set_spread_hint(spread, entries), lib.splatad_rasterize_set_near_hint(near)
+        _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last), _lib.stream_ptr(ids.device))
+        lib.splatad_rasterize_set_spread_hint(spread, entries), lib.splatad_rasterize_set_near_hint(near)
+        _lib.call("splatad_rasterize_to_pixels_bwd", *head, p(alphas), p(last), p(image), p(alphas), None, *(p(g) for g in grads),
+                  _lib.stream_ptr(ids.device))
+
+    return launched(both)[1]
+
+
+@pytest.mark.parametrize("W,H,channels,runs", [(960, 400, 8, False), (960, 400, 4, True), (960, 400, 14, True), (800, 496, 8, True), (800, 496, 5, True),
+                                              (800, 496, 17, False), (1200, 296, 8, False)])
+def test_backward_runs_by_channels(W, H, channels, runs):
+    """Up to sixteen channels; five to eight not where the warps without runs just fit at once."""
+    assert _chosen(1, W, H, 16, 20.0, 1800, 900, channels)[1].endswith(",runs") == runs
+
+
 @pytest.mark.parametrize("C,W,H,ts,spread,per_tile,near,forward,backward", [
     (2, 640, 360, 16, 68.0, 573, 900, False, True), (2, 640, 360, 16, 38.0, 1400, 900, True, True), (1, 1280, 720, 16, 59.0, 596, 900, False, True),
     (1, 1280, 720, 16, 23.0, 2296, 900, True, True), (2, 1280, 720, 16, 81.0, 162, 900, False, True), (2, 1280, 720, 16, 79.0, 316, 900, True, True),
@@ -548,24 +577,7 @@ def test_runs_of_entries_that_cover_a_patch(C, W, H, ts, channels, sigma_px, N, 
 def test_runs_are_for_dense_lists_of_large_gaussians(C, W, H, ts, spread, per_tile, near, forward, backward):
     """Which camera kernels the hints choose, on both sides of each line: near Gaussians that are small or of no known size, sparse lists, few
     tiles, rows that leave lanes over."""
-    from splatad_b200 import _lib
-    lib, p = _lib.load(), _lib.ptr
-    tw, th = -(-W // ts), -(-H // ts)
-    offsets, ids = torch.ones(C, th, tw, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)   # empty lists
-    image, alphas, one = torch.empty(C, H, W, 3, device=DEV), torch.zeros(C, H, W, 1, device=DEV), torch.zeros(8, device=DEV)
-    last, rs = torch.full((C, H, W), -1, dtype=torch.int32, device=DEV), torch.zeros(C, device=DEV)
-    head = (C, 1, p(one), p(one), p(one), 3, p(one), p(one), p(rs), None, W, H, ts, tw, th, p(offsets), p(ids))
-    grads = [torch.zeros(8, device=DEV) for _ in range(5)]
-    entries = per_tile * C * tw * th
-
-    def both():
-        lib.splatad_rasterize_set_spread_hint(spread, entries), lib.splatad_rasterize_set_near_hint(near)
-        _lib.call("splatad_rasterize_to_pixels_fwd", *head, p(image), p(alphas), p(last), _lib.stream_ptr(ids.device))
-        lib.splatad_rasterize_set_spread_hint(spread, entries), lib.splatad_rasterize_set_near_hint(near)
-        _lib.call("splatad_rasterize_to_pixels_bwd", *head, p(alphas), p(last), p(image), p(alphas), None, *(p(g) for g in grads),
-                  _lib.stream_ptr(ids.device))
-
-    names = launched(both)[1]
+    names = _chosen(C, W, H, ts, spread, per_tile, near, 3)
     assert [k.endswith("_kernel/8,runs") for k in names] == [forward, backward], names
 
 
